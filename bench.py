@@ -283,9 +283,9 @@ def time_step(timer, step, x, steps, warmup, use_graph):
 
     for _ in range(max(warmup, 3)):
         step()
-    n0 = _lib.launch_count
+    n0 = _lib.launches()
     step()
-    launches = _lib.launch_count - n0
+    launches = _lib.launches() - n0
     flush = input_bytes(x) < 2 * L2_BYTES
     graph = capture_graph(step) if use_graph else None
     fn = graph.replay if graph is not None else step

@@ -21,39 +21,18 @@ import os
 
 import torch
 
-from flashqla_b200 import cp, ops
-from flashqla_b200.ops import CHUNK_SIZE, SeqTables
-from flashqla_b200.utils import input_guard, l2norm_bwd, l2norm_fwd
+from flashqla_b200 import _lib, cp, ops
+from flashqla_b200.ops import CHUNK_SIZE
 
 
-def _state_in(x, state_v_first):
-    """User state -> kernel layout ([key dim][value dim], fp32, contiguous)."""
-    if x is None:
-        return None
-    if state_v_first:
-        x = x.transpose(-1, -2)
-    return x.to(torch.float32).contiguous()
+# bits of the native entry points' `flags` argument (csrc/host/module.cpp)
+FINAL_STATE, OUTPUT_H, AUTO_CP, V_FIRST, CACHE, SAVE_TILES, LEAD_IN, L2NORM = (
+    1 << i for i in range(8))
 
 
-def _state_out(x, state_v_first):
-    if x is None or not state_v_first:
-        return x
-    return x.transpose(-1, -2).contiguous()
-
-
-def _as_f32(g):
-    return g if g.dtype == torch.float32 else g.float()
-
-
-def _beta_in(beta):
-    return beta if beta.dtype in (torch.float32, torch.bfloat16) else beta.float()
-
-
-def _bf16(x):
-    """float16 inputs (which the reference accepts, ``chunk/__init__.py:364-367``) are computed
-    in bfloat16: the tensor cores of this build are fed bf16 operands only.  Results go back to
-    the caller's dtype."""
-    return x if x is None or x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
+def _switches(auto_cp, state_v_first) -> int:
+    return (AUTO_CP * bool(auto_cp) | V_FIRST * bool(state_v_first)
+            | SAVE_TILES * bool(SAVE_STATE_TILES) | LEAD_IN * bool(cp.LEAD_IN))
 
 
 # With the forward cache on (the training path), the forward also keeps what the backward would
@@ -105,7 +84,6 @@ def run_forward(q, k, v, A, g_cum, beta, scale, h0, tables, output_final_state=T
     return res, cp_cache
 
 
-@ops.on_tensor_device
 def chunk_gated_delta_rule_fwd(
     q: torch.Tensor,
     k: torch.Tensor,
@@ -126,27 +104,11 @@ def chunk_gated_delta_rule_fwd(
     consumed as-is by ``chunk_gated_delta_rule_bwd``."""
     if scale is None:
         scale = k.shape[-1] ** -0.5
-    in_dtype = q.dtype
-    q, k, v = _bf16(q).contiguous(), _bf16(k).contiguous(), _bf16(v).contiguous()
-    g = _as_f32(g).contiguous()
-    beta = _beta_in(beta).contiguous()
-    B, T, Hq, D = k.shape
-    tables = SeqTables(B, T, cu_seqlens)
-    g_cum, A = ops.kkt_solve(k, beta, g, cu_seqlens, raw_gate=True)  # cumsum fused into the kernel
-    h0 = _state_in(initial_state, state_v_first)
-
-    res, cp_cache = run_forward(q, k, v, A, g_cum, beta, scale, h0, tables, output_final_state,
-                                output_h, auto_cp, enable_fwd_cp_cache)
-    o = res["o"] if in_dtype == torch.bfloat16 else res["o"].to(in_dtype)
-    h = res.get("h")
-    if h is not None:
-        h = h.view(B, -1, *h.shape[1:]) if cu_seqlens is None else h.unsqueeze(0)
-        h = _state_out(h, state_v_first)
-    final_state = _state_out(res.get("ht"), state_v_first)
-    return g_cum, A, o, h, final_state, cp_cache
+    flags = (FINAL_STATE * bool(output_final_state) | OUTPUT_H * bool(output_h)
+             | _switches(auto_cp, state_v_first) | CACHE * bool(enable_fwd_cp_cache))
+    return _lib.host().forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, flags)
 
 
-@ops.on_tensor_device
 def chunk_gated_delta_rule_bwd(
     q: torch.Tensor,
     k: torch.Tensor,
@@ -167,53 +129,8 @@ def chunk_gated_delta_rule_bwd(
     ``(dq, dk, dv, db, dg, dh0)`` (``chunk/__init__.py:91-159``)."""
     if scale is None:
         scale = k.shape[-1] ** -0.5
-    in_dtype = q.dtype
-    q, k, v, do, A = (_bf16(x).contiguous() for x in (q, k, v, do, A))
-    g = _as_f32(g).contiguous()
-    beta_k = _beta_in(beta).contiguous()
-    B, T, Hq, D = k.shape
-    Hv = v.shape[2]
-    tables = SeqTables(B, T, cu_seqlens)
-    h0 = _state_in(initial_state, state_v_first)
-    dht_k = _state_in(dht, state_v_first)
-
-    cached = (tuple(cp_cache) if cp_cache is not None else ()) + (None, None, None, None)
-    plan = cp.plan_segments(tables, Hv, is_bwd=True, device=k.device) if auto_cp else None
-    lead = lead_out = None
-    if plan is not None:
-        if cached[0] is not None:
-            seg_h0, lead = cached[0], cached[3]
-        else:
-            seg_h0, lead = _segment_starts(plan, k, v, A, g, beta_k, scale, h0)
-        if cp.LEAD_IN and _tiles_ok(D):
-            seg_dht, lead_out = cp.backward_end(plan, q, k, v, A, g, beta_k, do, scale, dht_k)
-        else:
-            seg_dht = cp.backward_segment_states(plan, q, k, v, A, g, beta_k, do, scale, dht_k)
-        run_tables, run_h0, run_dht = plan.seg_tables, seg_h0, seg_dht
-    else:
-        run_tables, run_h0, run_dht = tables, h0, dht_k
-
-    # K = V = 128: the sequential kernels hand h, v_new, dh, du to the chunk-parallel kernel as
-    # ready-made operand tiles (written by TMA), not as row-major tensors
-    tiles = _tiles_ok(D)
-    if tiles and cached[1] is not None and cached[2] is not None:
-        fw = {"h": cached[1], "vnew": cached[2]}  # kept by the forward: no recomputation
-    else:
-        fw = ops.fwd_seq(None, k, v, A, g, beta_k, scale, run_h0, output_o=False, output_h=True,
-                         output_vnew=True, tables=run_tables, operand_tiles=tiles,
-                         lead_chunks=lead if tiles else None)
-    bw = ops.bwd_dh(q, k, A, g, beta_k, do, scale, run_dht, tables=run_tables,
-                    operand_tiles=tiles, lead_chunks=lead_out)
-    dq, dk, dv, db, dg = ops.bwd_main(q, k, v, fw["vnew"], A, g, beta_k, do, bw["du"], fw["h"],
-                                      bw["dh"], scale, tables=run_tables, operand_tiles=tiles)
-    dh0 = bw["dh0"]
-    if plan is not None:
-        dh0 = dh0[plan.first_seg_of_raw]
-    if initial_state is None:
-        dh0 = None
-    dh0 = _state_out(dh0, state_v_first)
-    dq, dk, dv, db, dg = finish_backward(dq, dk, dv, db, dg, Hq, beta.dtype, in_dtype, cu_seqlens)
-    return dq, dk, dv, db, dg, dh0
+    return _lib.host().backward(q, k, v, g, beta, A, do, dht, scale, initial_state, cu_seqlens,
+                                _switches(auto_cp, state_v_first), cp_cache, None)
 
 
 def finish_backward(dq, dk, dv, db, dg, Hq, beta_dtype, in_dtype, cu_seqlens):
@@ -230,9 +147,11 @@ def finish_backward(dq, dk, dv, db, dg, Hq, beta_dtype, in_dtype, cu_seqlens):
 
 
 class ChunkGatedDeltaRuleFunction(torch.autograd.Function):
+    """The autograd class of the reference, for callers that apply it themselves;
+    ``chunk_gated_delta_rule`` records the same two passes as a native autograd node
+    (``csrc/host/autograd.cpp``)."""
+
     @staticmethod
-    @input_guard
-    @torch.amp.custom_fwd(device_type="cuda")
     def forward(
         ctx,
         q: torch.Tensor,
@@ -249,50 +168,36 @@ class ChunkGatedDeltaRuleFunction(torch.autograd.Function):
         auto_cp: bool = True,
         enable_fwd_cp_cache: bool = True,
     ):
-        q_rstd, k_rstd = None, None
-        if use_qk_l2norm_in_kernel:
-            q, q_rstd = l2norm_fwd(q)
-            k, k_rstd = l2norm_fwd(k)
-        g_cum, A, o, _, final_state, cp_cache = chunk_gated_delta_rule_fwd(
-            q=q, k=k, v=v, g=g, beta=beta, scale=scale, initial_state=initial_state,
-            output_final_state=output_final_state, output_h=False, cu_seqlens=cu_seqlens,
-            state_v_first=state_v_first, auto_cp=auto_cp,
-            enable_fwd_cp_cache=enable_fwd_cp_cache,
-        )
-        cached = tuple(cp_cache) if cp_cache is not None else ()
-        ctx.save_for_backward(q, k, q_rstd, k_rstd, v, g_cum, beta, A, initial_state, cu_seqlens,
-                              *cached)
-        ctx.n_cached = len(cached)
+        if scale is None:
+            scale = k.shape[-1] ** -0.5
+        ctx.flags = _switches(auto_cp, state_v_first)
+        flags = (ctx.flags | FINAL_STATE * bool(output_final_state)
+                 | CACHE * bool(enable_fwd_cp_cache) | L2NORM * bool(use_qk_l2norm_in_kernel))
+        g_cum, A, o, _, final_state, cp_cache, *norm = _lib.host().forward(
+            q, k, v, g, beta, scale, initial_state, cu_seqlens, flags)
+        q_used, k_used = norm[:2] if norm else (q, k)
+        ctx.save_for_backward(q_used, k_used, v, g_cum, beta, A, initial_state, cu_seqlens, q, k,
+                              *norm[2:], *(cp_cache or ()))
+        ctx.has_norm, ctx.has_cache = bool(norm), cp_cache is not None
         ctx.g_dtype = g.dtype
         ctx.scale = scale
-        ctx.state_v_first = state_v_first
-        ctx.auto_cp = auto_cp
-        ctx.use_qk_l2norm_in_kernel = use_qk_l2norm_in_kernel
-        return o.to(q.dtype), final_state
+        return o, final_state
 
     @staticmethod
-    @input_guard
-    @torch.amp.custom_bwd(device_type="cuda")
     def backward(ctx, do: torch.Tensor, dht: torch.Tensor):
-        saved = ctx.saved_tensors
-        q, k, q_rstd, k_rstd, v, g_cum, beta, A, initial_state, cu_seqlens = saved[:10]
-        cp_cache = tuple(saved[10:]) if ctx.n_cached else None
-        dq, dk, dv, db, dg, dh0 = chunk_gated_delta_rule_bwd(
-            q=q, k=k, v=v, g=g_cum, beta=beta, A=A, do=do, dht=dht, scale=ctx.scale,
-            initial_state=initial_state, cu_seqlens=cu_seqlens,
-            state_v_first=ctx.state_v_first, auto_cp=ctx.auto_cp, cp_cache=cp_cache,
-        )
-        if ctx.use_qk_l2norm_in_kernel:
-            dq = l2norm_bwd(q, q_rstd, dq)
-            dk = l2norm_bwd(k, k_rstd, dk)
+        q_used, k_used, v, g_cum, beta, A, initial_state, cu_seqlens, q, k, *rest = ctx.saved_tensors
+        norm = (q, k, rest.pop(0), rest.pop(0)) if ctx.has_norm else None
+        dq, dk, dv, db, dg, dh0 = _lib.host().backward(
+            q_used, k_used, v, g_cum, beta, A, do, dht, ctx.scale, initial_state, cu_seqlens,
+            ctx.flags, tuple(rest) if ctx.has_cache else None, norm)
         return (
-            dq.to(q),
-            dk.to(k),
-            dv.to(v),
+            dq,
+            dk,
+            dv,
             dg.to(ctx.g_dtype),
-            db.to(beta),
+            db,
             None,
-            dh0 if initial_state is not None else None,
+            dh0,
             None,
             None,
             None,
@@ -327,27 +232,10 @@ def chunk_gated_delta_rule(
     packed variable-length input (batch must be 1); ``state_v_first`` stores states as ``[V,K]``.
     Returns ``(o [B,T,HV,V], final_state [N,HV,K,V] or None)``.
     """
-    assert q.dtype == k.dtype == v.dtype
-    assert q.dtype == torch.bfloat16 or q.dtype == torch.float16, (
-        "FlashQLA only supports bfloat16 and float16."
-    )
     assert not head_first, "head_first=True is not supported."
-    assert v.shape[2] % k.shape[2] == 0, "num_qk_heads must be divisible to num_v_heads."
-    if cu_seqlens is not None:
-        if q.shape[0] != 1:
-            raise ValueError(
-                f"The batch size is expected to be 1 rather than {q.shape[0]} when using "
-                f"`cu_seqlens`. Please flatten variable-length inputs before processing."
-            )
-        if initial_state is not None and initial_state.shape[0] != len(cu_seqlens) - 1:
-            raise ValueError(
-                f"The number of initial states is expected to be equal to the number of input "
-                f"sequences, i.e., {len(cu_seqlens) - 1} rather than {initial_state.shape[0]}."
-            )
-    if scale is None:
-        scale = k.shape[-1] ** -0.5
-    o, final_state = ChunkGatedDeltaRuleFunction.apply(
-        q, k, v, g, beta, scale, initial_state, output_final_state, cu_seqlens,
-        use_qk_l2norm_in_kernel, state_v_first, auto_cp, enable_fwd_cp_cache,
-    )
-    return o, final_state
+    return _lib.host().apply(
+        q, k, v, g, beta, scale, initial_state, cu_seqlens,
+        (FINAL_STATE if output_final_state else 0) | (AUTO_CP if auto_cp else 0)
+        | (V_FIRST if state_v_first else 0) | (CACHE if enable_fwd_cp_cache else 0)
+        | (SAVE_TILES if SAVE_STATE_TILES else 0) | (LEAD_IN if cp.LEAD_IN else 0)
+        | (L2NORM if use_qk_l2norm_in_kernel else 0))

@@ -26,6 +26,8 @@ SIGNATURES = {
     "fqla_merge_states": [P, P, P, P, P, P, P, I, I, I, I, LL, P],
     "fqla_l2norm_fwd": [P, P, P, LL, I, I, F, P],
     "fqla_l2norm_bwd": [P, P, P, P, LL, I, I, I, P],
+    "fqla_prepare_inputs": [P] * 8 + [LL, LL, I, I, I, F, P],
+    "fqla_finish_grads": [P] * 10 + [LL, I, I, I, P],
     "fqla_segment_scan": [P, I, I, P, I, P, I, F, I, P, P, P, P, P, P],
     "fqla_device_status": [P, I],
     "fqla_selftest_wait_timeout": [I, P],
@@ -33,6 +35,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class FqlaError(RuntimeError):
@@ -62,6 +65,28 @@ def load():
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+def host():
+    """The native host path (``csrc/host``, an extension module over PyTorch's C++ API), loaded
+    once."""
+    global _host
+    if _host is None:
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise FqlaError(
+                "flashqla_b200._host is missing: build the native code first "
+                f"(python -m flashqla_b200.build). There is no fallback. ({e})") from e
+        module.set_error_type(FqlaError)
+        _host = module
+    return _host
+
+
+def launches() -> int:
+    """Entry-point calls of the library that succeeded so far: this binding's and the native host
+    path's."""
+    return launch_count + (_host.launches() if _host is not None else 0)
 
 
 launch_count = 0  # kernels enqueued through this binding (one per successful entry-point call)

@@ -20,20 +20,17 @@ fixed-length input, which the reference never splits).
 
 from __future__ import annotations
 
-import math
 from dataclasses import dataclass
 
 import torch
 
-from . import ops
+from . import _lib, ops
 from .ops import CHUNK_SIZE, SeqTables
 from .utils import tensor_cache
 
 THRESHOLD = -10.0
 MIN_SEGMENT_CHUNKS = 8
 VALUE_SLICES = 1  # CTAs per (segment, head) of the tcgen05 forward kernel
-SEGMENT_OVERHEAD_CHUNKS = 2  # cost of a hand-off, in chunk steps of the main kernel
-CTA_START_CHUNKS = 2  # cost of starting a CTA (tensor-memory allocation, first loads), same unit
 # True: the tcgen05 recurrence kernels start a segment a few chunks early (forward,
 # ``forward_start``) or late (reverse, ``backward_end``) from a zero state; False: every segment's
 # start state comes from the separate state-only pass and the merge chain
@@ -56,87 +53,25 @@ class SegmentPlan:
     n_seg: int
 
 
-def _makespan(costs: list[int], copies: int, machines: int) -> int:
-    """Length of the schedule the hardware produces for CTAs of the given costs (each present
-    ``copies`` times, one per head) handed out longest first to ``machines`` SMs, one CTA per SM:
-    every CTA goes to the SM that frees up first."""
-    import heapq
-
-    items = sorted(costs, reverse=True)
-    n = len(items) * copies
-    if n <= machines:
-        return items[0] if items else 0
-    loads = [0] * machines
-    heapq.heapify(loads)
-    for c in items:
-        for _ in range(copies):
-            heapq.heappush(loads, heapq.heappop(loads) + c)
-    return max(loads)
-
-
 def split_sequences(bounds: list[int], num_heads: int, n_sm: int,
                     min_chunks: int = MIN_SEGMENT_CHUNKS, slices: int = VALUE_SLICES):
-    """Host-side segment planner.  ``bounds`` are the raw cumulative sequence lengths.
+    """Host-side segment planner (native: ``csrc/host/planner.cpp``).  ``bounds`` are the raw
+    cumulative sequence lengths.
 
     The sequential kernels keep one CTA per SM and walk their chunks in order; the CTAs of a
     launch are handed out longest first, each to the SM that frees up first.  The planner
-    evaluates that schedule (``_makespan``) for the unsplit batch and for every maximum segment
-    length ``ceil(longest / p)`` (sequences longer than the limit are cut into equal, chunk
-    aligned parts), charging ``CTA_START_CHUNKS`` per CTA and ``SEGMENT_OVERHEAD_CHUNKS`` more
-    per segment that needs a start state, and keeps the cheapest.  It therefore splits a single
-    long sequence to fill the GPU, splits only the few long documents of a ragged batch that
-    would otherwise be the tail of the launch, and leaves a batch alone that already keeps every
-    SM busy.
+    evaluates that schedule for the unsplit batch and for every maximum segment length
+    ``ceil(longest / p)`` (sequences longer than the limit are cut into equal, chunk aligned
+    parts), charging a fixed cost per CTA and another per segment that needs a start state, and
+    keeps the cheapest.  It therefore splits a single long sequence to fill the GPU, splits only
+    the few long documents of a ragged batch that would otherwise be the tail of the launch, and
+    leaves a batch alone that already keeps every SM busy.
 
     Returns ``None`` when no split beats the unsplit schedule by at least 3 %, else
     ``(seg_bounds, seg_begin)``: the cumulative lengths of the segments and, per raw sequence, the
     index of its first segment.
     """
-    lens = [e - s for s, e in zip(bounds[:-1], bounds[1:])]
-    chunks = [(n + CHUNK_SIZE - 1) // CHUNK_SIZE for n in lens]
-    longest = max(chunks) if chunks else 0
-    if longest < 2 * min_chunks:
-        return None
-    copies = num_heads * slices
-
-    def layout(limit):
-        parts = [max(1, math.ceil(c / limit)) for c in chunks]
-        per = [math.ceil(c / p) if c else 0 for c, p in zip(chunks, parts)]
-        costs = []
-        for c, p, pc in zip(chunks, parts, per):
-            for i in range(p):
-                seg = min(pc, c - i * pc)
-                if seg > 0:
-                    costs.append(seg + CTA_START_CHUNKS + (SEGMENT_OVERHEAD_CHUNKS if i else 0))
-        return parts, per, _makespan(costs, copies, n_sm)
-
-    _, _, unsplit = layout(longest)
-    tried, cands = set(), []
-    for p in range(2, longest // min_chunks + 1):
-        limit = math.ceil(longest / p)
-        if limit < min_chunks:
-            break
-        if limit in tried:
-            continue
-        tried.add(limit)
-        parts, per, cost = layout(limit)
-        cands.append((cost, parts, per))
-    if not cands:
-        return None
-    cheapest = min(c[0] for c in cands)
-    if cheapest > 0.97 * unsplit:
-        return None
-    # among near-ties the coarsest split: fewer CTAs, fewer hand-offs
-    best = next(c for c in cands if c[0] <= 1.03 * cheapest)
-    _, parts, per = best
-    seg_bounds, seg_begin = [], []
-    for s, np_, pc in zip(bounds[:-1], parts, per):
-        seg_begin.append(len(seg_bounds))
-        for i in range(np_):
-            seg_bounds.append(s + i * pc * CHUNK_SIZE)  # balanced, chunk aligned
-    seg_begin.append(len(seg_bounds))
-    seg_bounds.append(bounds[-1])
-    return seg_bounds, seg_begin
+    return _lib.host().split_sequences(bounds, num_heads, n_sm, min_chunks, slices)
 
 
 @tensor_cache

@@ -1,0 +1,121 @@
+#include "autograd.h"
+
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+
+namespace fqla_host {
+
+namespace ag = torch::autograd;
+
+namespace {
+
+struct GatedDeltaRuleBackward : public ag::Node {
+  // inputs as the kernels read them, the forward's results, what the forward kept
+  ag::SavedVariable q, k, v, g_cum, beta, A, initial_state, cu, seg_h0, h, vnew, lead;
+  // q, k before the normalisation, reciprocal norms (with l2norm)
+  ag::SavedVariable q_in, k_in, q_rstd, k_rstd;
+  double scale = 1.0;
+  Options opt;
+  at::ScalarType dtype = at::kBFloat16, beta_dtype = at::kFloat, g_dtype = at::kFloat,
+                 h0_dtype = at::kFloat;
+  bool has_h0 = false;
+  at::TensorOptions o_options;
+  std::vector<int64_t> o_sizes;
+
+  std::string name() const override { return "GatedDeltaRuleBackward"; }
+
+  void release_variables() override {
+    for (ag::SavedVariable* s : {&q, &k, &v, &g_cum, &beta, &A, &initial_state, &cu, &seg_h0, &h,
+                                 &vnew, &lead, &q_in, &k_in, &q_rstd, &k_rstd})
+      s->reset_data();
+  }
+
+  ag::variable_list apply(ag::variable_list&& grads) override {
+    auto get = [&](const ag::SavedVariable& s) { return s.unpack(); };
+    auto opt_get = [&](const ag::SavedVariable& s) -> OptTensor {
+      at::Tensor t = s.unpack();
+      return t.defined() ? OptTensor(t) : std::nullopt;
+    };
+    ag::variable_list out(6);
+    const OptTensor dht = grads.size() > 1 && grads[1].defined() ? OptTensor(grads[1]) : std::nullopt;
+    if (!grads[0].defined() && !dht) return out;
+    const at::Tensor dO = grads[0].defined() ? grads[0] : at::zeros(o_sizes, o_options);
+    const Cache cache{opt_get(seg_h0), opt_get(h), opt_get(vnew), opt_get(lead)};
+    Norm norm;
+    if (opt.l2norm) norm = Norm{get(q_in), get(k_in), get(q_rstd), get(k_rstd)};
+    const Backward r = backward(get(q), get(k), get(v), get(g_cum), get(beta), get(A), dO, dht, scale,
+                                opt_get(initial_state), opt_get(cu), opt, cache,
+                                opt.l2norm ? &norm : nullptr, dtype);
+    out[0] = r.dq;
+    out[1] = r.dk;
+    out[2] = r.dv;
+    out[3] = r.dg.scalar_type() == g_dtype ? r.dg : r.dg.to(g_dtype);
+    out[4] = r.db.scalar_type() == beta_dtype ? r.db : r.db.to(beta_dtype);
+    if (r.dh0) out[5] = r.dh0->scalar_type() == h0_dtype ? *r.dh0 : r.dh0->to(h0_dtype);
+    return out;
+  }
+};
+
+bool needs_grad(const at::Tensor& t) { return t.defined() && t.requires_grad(); }
+
+}  // namespace
+
+std::pair<at::Tensor, OptTensor> apply(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                                       const at::Tensor& g, const at::Tensor& beta, double scale,
+                                       const OptTensor& initial_state, const OptTensor& cu,
+                                       Options opt) {
+  const bool grad = c10::GradMode::is_enabled() &&
+                    (needs_grad(q) || needs_grad(k) || needs_grad(v) || needs_grad(g) ||
+                     needs_grad(beta) || (initial_state && needs_grad(*initial_state)));
+  opt.cache = opt.cache && grad;  // nothing will ask for it otherwise
+  opt.norm_grad = opt.l2norm && grad;
+  Forward r = forward(q, k, v, g, beta, scale, initial_state, cu, opt);
+  if (!grad) return {r.o, r.final_state};
+
+  auto node = std::shared_ptr<GatedDeltaRuleBackward>(new GatedDeltaRuleBackward(), ag::deleteNode);
+  const at::Tensor h0 = initial_state ? *initial_state : at::Tensor();
+  node->set_next_edges(ag::collect_next_edges(q, k, v, g, beta, h0));
+  node->scale = scale;
+  node->opt = opt;
+  node->dtype = q.scalar_type();
+  node->beta_dtype = beta.scalar_type();
+  node->g_dtype = g.scalar_type();
+  node->has_h0 = initial_state.has_value();
+  if (initial_state) node->h0_dtype = initial_state->scalar_type();
+  node->o_options = r.o.options();
+  node->o_sizes = r.o.sizes().vec();
+  auto save = [](ag::SavedVariable& s, const at::Tensor& t) {
+    if (t.defined()) s = ag::SavedVariable(t, false);
+  };
+  auto save_opt = [&](ag::SavedVariable& s, const OptTensor& t) {
+    if (t) save(s, *t);
+  };
+  save(node->q, r.q);
+  save(node->k, r.k);
+  save(node->v, r.v);
+  save(node->g_cum, r.g_cum);
+  save(node->beta, beta);
+  save(node->A, r.A);
+  save_opt(node->initial_state, initial_state);
+  save_opt(node->cu, cu);
+  save_opt(node->seg_h0, r.cache.seg_h0);
+  save_opt(node->h, r.cache.h);
+  save_opt(node->vnew, r.cache.vnew);
+  save_opt(node->lead, r.cache.lead);
+  if (opt.l2norm) {
+    save(node->q_in, q);
+    save(node->k_in, k);
+    save(node->q_rstd, r.q_rstd);
+    save(node->k_rstd, r.k_rstd);
+  }
+  ag::set_history(r.o, node);
+  if (r.final_state) {
+    at::Tensor ht = *r.final_state;
+    ag::set_history(ht, node);
+    r.final_state = ht;
+  }
+  return {r.o, r.final_state};
+}
+
+}  // namespace fqla_host

@@ -1,0 +1,205 @@
+#include "batch.h"
+
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAException.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+
+#include <algorithm>
+#include <list>
+#include <mutex>
+#include <numeric>
+#include <vector>
+
+#include "errors.h"
+#include "planner.h"
+
+namespace fqla_host {
+
+namespace {
+
+// Recent entries, least recently used first.  A step of a program uses a handful of batches
+// (micro-batches in flight between their forward and backward); an entry is a few hundred KB at
+// the most.  Shared by all threads; the tables are immutable once built.
+constexpr size_t MAX_ENTRIES = 16;
+std::list<std::shared_ptr<Batch>> entries;
+std::mutex entries_lock;
+
+bool capturing() {
+  return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+}
+
+std::vector<int64_t> read_bounds(const at::Tensor& cu) {
+  at::Tensor h = cu.cpu();
+  std::vector<int64_t> b((size_t)h.numel());
+  if (h.scalar_type() == at::kInt) {
+    const int* p = h.data_ptr<int>();
+    std::copy(p, p + b.size(), b.begin());
+  } else {
+    const int64_t* p = h.data_ptr<int64_t>();
+    std::copy(p, p + b.size(), b.begin());
+  }
+  return b;
+}
+
+// cu | chunk offsets | chunk (sequence, chunk in sequence) rows | longest-first order
+struct Tables {
+  size_t cu, offsets, indices, order;
+  int64_t num_chunks;
+};
+Tables add_tables(std::vector<int>& out, const std::vector<int64_t>& bounds) {
+  Tables t;
+  const size_t n = bounds.size() - 1;
+  t.cu = out.size();
+  out.insert(out.end(), bounds.begin(), bounds.end());
+  t.offsets = out.size();
+  int64_t sum = 0;
+  std::vector<int64_t> len(n);
+  for (size_t i = 0; i < n; ++i) {
+    len[i] = bounds[i + 1] - bounds[i];
+    out.push_back((int)sum);
+    sum += (len[i] + CHUNK - 1) / CHUNK;
+  }
+  out.push_back((int)sum);
+  t.num_chunks = sum;
+  t.indices = out.size();
+  for (size_t i = 0; i < n; ++i)
+    for (int64_t c = 0; c < (len[i] + CHUNK - 1) / CHUNK; ++c) {
+      out.push_back((int)i);
+      out.push_back((int)c);
+    }
+  t.order = out.size();
+  std::vector<int> order(n);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return len[a] > len[b]; });
+  out.insert(out.end(), order.begin(), order.end());
+  return t;
+}
+
+std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int64_t T, int64_t Hv,
+                             int device) {
+  auto b = std::make_shared<Batch>();
+  b->B = B;
+  b->T = T;
+  b->Hv = Hv;
+  b->device = device;
+  std::vector<int64_t> bounds;
+  std::vector<int> host;
+  Tables raw{};
+  const bool packed = cu.has_value();
+  if (packed) {
+    b->cu = *cu;
+    b->version = cu->is_inference() ? 0 : cu->_version();
+    bounds = read_bounds(*cu);
+    b->N = (int64_t)bounds.size() - 1;
+    raw = add_tables(host, bounds);
+    b->num_chunks = raw.num_chunks;
+    b->total = bounds.back();
+  } else {
+    b->N = B;
+    b->num_chunks = B * ((T + CHUNK - 1) / CHUNK);
+    b->total = B * T;
+    for (int64_t i = 0; i <= B; ++i) bounds.push_back(i * T);
+  }
+  const int n_sm = at::cuda::getDeviceProperties(device)->multiProcessorCount;
+  const auto split = split_sequences(bounds, Hv, n_sm);
+  Tables seg{};
+  size_t begin = 0, first = 0, last = 0, kf = 0, kb = 0;
+  if (split) {
+    seg = add_tables(host, split->seg_bounds);
+    b->n_seg = (int64_t)split->seg_bounds.size() - 1;
+    begin = host.size();
+    host.insert(host.end(), split->seg_begin.begin(), split->seg_begin.end());
+    first = host.size();
+    for (int64_t i = 0; i < b->N; ++i) host.push_back((int)split->seg_begin[i]);
+    last = host.size();
+    for (int64_t i = 0; i < b->N; ++i) host.push_back((int)split->seg_begin[i + 1] - 1);
+    // the last segment of a sequence hands nothing forward, the first nothing backward
+    std::vector<int> keep_f((size_t)b->n_seg, 1), keep_b((size_t)b->n_seg, 1);
+    for (int64_t i = 0; i < b->N; ++i)
+      if (split->seg_begin[i + 1] > split->seg_begin[i]) {
+        keep_b[(size_t)split->seg_begin[i]] = 0;
+        keep_f[(size_t)split->seg_begin[i + 1] - 1] = 0;
+      }
+    kf = host.size();
+    host.insert(host.end(), keep_f.begin(), keep_f.end());
+    kb = host.size();
+    host.insert(host.end(), keep_b.begin(), keep_b.end());
+  }
+  if (!host.empty()) {
+    b->stream = at::cuda::getCurrentCUDAStream(device);
+    b->store = at::detail::empty_cuda({(int64_t)host.size()}, at::kInt, c10::Device(c10::kCUDA, device),
+                                      std::nullopt);
+    // pageable source: the call returns once the data has been staged
+    C10_CUDA_CHECK(cudaMemcpyAsync(b->store.data_ptr(), host.data(), host.size() * sizeof(int),
+                                   cudaMemcpyHostToDevice, *b->stream));
+    // the entry may be used from another stream next
+    C10_CUDA_CHECK(cudaStreamSynchronize(*b->stream));
+  }
+  const int* d = host.empty() ? nullptr : b->store.data_ptr<int>();
+  if (packed) {
+    b->d_cu = d + raw.cu;
+    b->d_offsets = d + raw.offsets;
+    b->d_indices = d + raw.indices;
+    b->d_order = b->N < 2 ? nullptr : d + raw.order;
+  }
+  if (split) {
+    b->s_cu = d + seg.cu;
+    b->s_offsets = d + seg.offsets;
+    b->s_indices = d + seg.indices;
+    b->s_order = b->n_seg < 2 ? nullptr : d + seg.order;
+    b->s_begin = d + begin;
+    b->keep_fwd = d + kf;
+    b->keep_bwd = d + kb;
+    b->first_seg = b->store.narrow(0, (int64_t)first, b->N);
+    b->last_seg = b->store.narrow(0, (int64_t)last, b->N);
+  }
+  return b;
+}
+
+}  // namespace
+
+std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B, int64_t T,
+                                 int64_t Hv, int device) {
+  if (cu) {
+    if (cu->scalar_type() != at::kInt && cu->scalar_type() != at::kLong)
+      throw PyError(PyError::Type, "cu_seqlens must be int32 or int64");
+    if (B != 1) throw PyError(PyError::Value, "packed input (cu_seqlens) needs batch size 1");
+  }
+  const uint32_t version = cu && !cu->is_inference() ? cu->_version() : 0;
+  const bool cap = capturing();
+  std::lock_guard<std::mutex> hold(entries_lock);
+  for (auto it = entries.begin(); it != entries.end(); ++it) {
+    Batch& e = **it;
+    if (e.B != B || e.T != T || e.Hv != Hv || e.device != device) continue;
+    if (cu ? !(e.cu.defined() && e.cu.unsafeGetTensorImpl() == cu->unsafeGetTensorImpl() &&
+               e.version == version)
+           : e.cu.defined())
+      continue;
+    if (cap) e.pinned = true;
+    if (e.stream) {
+      // an evicted entry's tables must outlive the kernels of every stream that read them
+      const auto current = at::cuda::getCurrentCUDAStream(device);
+      if (current != *e.stream)
+        c10::cuda::CUDACachingAllocator::recordStream(e.store.storage().data_ptr(), current);
+    }
+    entries.splice(entries.end(), entries, it);
+    return entries.back();
+  }
+  // building a table needs a host round trip
+  if (cap) throw PyError(PyError::Assertion, "index tables of this batch were not built before CUDA graph capture");
+  auto b = build(cu, B, T, Hv, device);
+  size_t unpinned = 0;
+  for (auto& e : entries) unpinned += !e->pinned;
+  if (unpinned >= MAX_ENTRIES)
+    for (auto it = entries.begin(); it != entries.end(); ++it)
+      if (!(*it)->pinned) {
+        entries.erase(it);
+        break;
+      }
+  entries.push_back(b);
+  return b;
+}
+
+}  // namespace fqla_host

@@ -1,0 +1,39 @@
+// Index tables and split plan of one batch, built once and kept.
+#pragma once
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <cstdint>
+#include <memory>
+#include <optional>
+
+namespace fqla_host {
+
+struct Batch {
+  // what the entry was made for
+  at::Tensor cu;          // the caller's cu_seqlens (undefined: fixed length); kept alive by the entry
+  uint32_t version = 0;   // its version counter when the tables were read
+  int64_t B = 0, T = 0, Hv = 0;
+  int device = 0;
+  bool pinned = false;    // looked up during a stream capture: never evicted
+
+  at::Tensor store;       // all device tables, int32, allocated on `stream`
+  std::optional<c10::cuda::CUDAStream> stream;
+  int64_t N = 0, num_chunks = 0, total = 0;
+  // packed batches (null pointers for fixed-length ones)
+  const int *d_cu = nullptr, *d_offsets = nullptr, *d_indices = nullptr, *d_order = nullptr;
+  // the split plan, when there is one; segments are seen as a packed batch
+  int64_t n_seg = 0;
+  const int *s_cu = nullptr, *s_offsets = nullptr, *s_indices = nullptr, *s_order = nullptr;
+  const int *s_begin = nullptr;   // [N + 1] first segment of every raw sequence
+  const int *keep_fwd = nullptr, *keep_bwd = nullptr;  // [n_seg]
+  at::Tensor first_seg, last_seg;  // int32 [N], views of `store`
+};
+
+// Tables for a batch of `Hv` value heads; one host round trip (reads cu_seqlens, writes the
+// tables) the first time a cu_seqlens tensor (identity and version counter) or a fixed shape is
+// seen, none after that while the entry is kept.
+std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B, int64_t T,
+                                 int64_t Hv, int device);
+
+}  // namespace fqla_host

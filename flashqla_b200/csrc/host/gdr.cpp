@@ -1,0 +1,421 @@
+#include "gdr.h"
+
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/GradMode.h>
+#include <c10/cuda/CUDAGuard.h>
+
+#include <cstdlib>
+
+#include "../../../include/fqla.h"
+#include "batch.h"
+#include "errors.h"
+
+namespace fqla_host {
+
+std::atomic<long long> launch_count{0};
+
+namespace {
+
+constexpr int CHUNK = 64;
+constexpr float THRESHOLD = -10.f;  // log of what a truncated past may still weigh
+
+void check(int status, const char* what) {
+  launch_count.fetch_add(1, std::memory_order_relaxed);
+  if (status != FQLA_OK)
+    throw PyError(PyError::Fqla, std::string(what) + " failed with status " + std::to_string(status) +
+                                     ": " + fqla_status_string(status));
+}
+
+at::Tensor empty(at::IntArrayRef sizes, at::ScalarType dtype, c10::Device dev) {
+  return at::detail::empty_cuda(sizes, dtype, dev, std::nullopt);
+}
+
+template <typename T = void>
+const T* ptr(const OptTensor& t) {
+  return t ? static_cast<const T*>(t->data_ptr()) : nullptr;
+}
+template <typename T = void>
+T* mut(const OptTensor& t) {
+  return t ? static_cast<T*>(t->data_ptr()) : nullptr;
+}
+
+// The tensor-core kernels are fed bfloat16 only: other types are converted.  TMA and the 16-byte
+// accesses want aligned rows, which a contiguous view into a larger buffer need not have.
+at::Tensor aligned(const at::Tensor& x) {
+  at::Tensor y = x.contiguous();
+  return reinterpret_cast<uintptr_t>(y.data_ptr()) % 16 ? y.clone() : y;
+}
+at::Tensor as_bf16(const at::Tensor& x) {
+  return aligned(x.scalar_type() == at::kBFloat16 ? x : x.to(at::kBFloat16));
+}
+at::Tensor as_f32(const at::Tensor& x) {
+  return (x.scalar_type() == at::kFloat ? x : x.to(at::kFloat)).contiguous();
+}
+at::Tensor beta_in(const at::Tensor& b) {
+  if (b.scalar_type() == at::kFloat || b.scalar_type() == at::kBFloat16) return b.contiguous();
+  return b.to(at::kFloat).contiguous();
+}
+OptTensor state_in(const OptTensor& x, bool v_first) {
+  if (!x) return std::nullopt;
+  at::Tensor t = v_first ? x->transpose(-1, -2) : *x;
+  return as_f32(t);
+}
+OptTensor state_out(const OptTensor& x, bool v_first) {
+  if (!x || !v_first) return x;
+  return x->transpose(-1, -2).contiguous();
+}
+
+// One call's shapes, stream and index tables.
+struct Call {
+  c10::Device dev{c10::kCUDA, 0};
+  void* stream = nullptr;
+  int B, T, Hq, Hv, D;
+  float scale;
+  std::shared_ptr<Batch> batch;
+  bool split = false;  // run over the segments of the plan
+
+  // tables of the sequential kernels: the sequences themselves or the segments
+  const int* cu() const { return split ? batch->s_cu : batch->d_cu; }
+  const int* offsets() const { return split ? batch->s_offsets : batch->d_offsets; }
+  const int* indices() const { return split ? batch->s_indices : batch->d_indices; }
+  const int* order() const { return split ? batch->s_order : batch->d_order; }
+  int N() const { return (int)(split ? batch->n_seg : batch->N); }
+  // segments are a packed batch of all rows
+  int kB() const { return split ? 1 : B; }
+  int kT() const { return split ? B * T : T; }
+};
+
+Call make_call(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, double scale,
+               const OptTensor& cu, bool auto_cp) {
+  Call c;
+  c.dev = k.device();
+  c.stream = (void*)at::cuda::getCurrentCUDAStream(c.dev.index()).stream();
+  c.B = (int)k.size(0);
+  c.T = (int)k.size(1);
+  c.Hq = (int)k.size(2);
+  c.D = (int)k.size(3);
+  c.Hv = (int)v.size(2);
+  c.scale = (float)scale;
+  c.batch = batch_for(cu, c.B, c.T, c.Hv, c.dev.index());
+  c.split = auto_cp && c.batch->n_seg > 0;
+  return c;
+}
+
+void check_state(const OptTensor& s, const Call& c) {
+  if (!s) return;
+  if (s->dim() != 4 || s->size(0) != c.batch->N || s->size(1) != c.Hv || s->size(2) != c.D ||
+      s->size(3) != c.D)
+    throw PyError(PyError::Assertion,
+                  "initial_state must be [" + std::to_string(c.batch->N) + "," + std::to_string(c.Hv) +
+                      "," + std::to_string(c.D) + "," + std::to_string(c.D) + "]");
+}
+
+bool tiles_ok(int D) {
+  static const bool forced = std::getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
+  return D == 128 && !forced;
+}
+
+struct SeqIn {  // inputs of the sequential kernels
+  const at::Tensor &q, &k, &v, &A, &g, &beta;
+  int beta_f32;
+};
+
+void run_fwd(const Call& c, const SeqIn& in, bool with_q, const float* h0, const OptTensor& ht,
+             const OptTensor& o, const OptTensor& h, const OptTensor& vnew, const OptTensor& M,
+             const int* warm, const int* m_mask, const int* lead, bool tiles) {
+  check(fqla_fwd_seq(with_q ? in.q.data_ptr() : nullptr, in.k.data_ptr(), in.v.data_ptr(),
+                     in.A.data_ptr(), (const float*)in.g.data_ptr(), in.beta.data_ptr(), in.beta_f32,
+                     h0, mut<float>(ht), mut(o), mut(h), mut(vnew), mut<float>(M), warm, m_mask, lead,
+                     c.order(), nullptr, 1, c.kB(), c.kT(), c.Hq, c.Hv, c.D, c.scale, c.cu(),
+                     c.offsets(), 0, c.N(), tiles, c.stream),
+        "fwd_seq");
+}
+
+at::Tensor merge(const Call& c, const at::Tensor& local, const at::Tensor& M, const int* use_m,
+                 const OptTensor& raw, const int* any_fb, bool reverse) {
+  at::Tensor out = empty({c.batch->n_seg, c.Hv, c.D, c.D}, at::kFloat, c.dev);
+  check(fqla_merge_states((const float*)local.data_ptr(), (const float*)M.data_ptr(), use_m,
+                          ptr<float>(raw), c.batch->s_begin, any_fb, (float*)out.data_ptr(),
+                          (int)c.batch->N, c.Hv, c.D, reverse, 0, c.stream),
+        "merge_states");
+  return out;
+}
+
+// Per (segment, head) int32 tables of the scan: warm, fallback, lead, exact_warm, and any_fallback
+// per (sequence, head) behind them.
+struct Scan {
+  at::Tensor store;
+  int *warm, *fallback, *lead, *exact_warm, *any_fb;
+  at::Tensor lead_tensor;
+};
+Scan segment_scan(const Call& c, const at::Tensor& g, bool from_start) {
+  Scan s;
+  const int64_t n = c.batch->n_seg * c.Hv;
+  s.store = empty({4 * n + c.batch->N * c.Hv}, at::kInt, c.dev);
+  int* p = s.store.data_ptr<int>();
+  s.warm = p;
+  s.fallback = p + n;
+  s.lead = p + 2 * n;
+  s.exact_warm = p + 3 * n;
+  s.any_fb = p + 4 * n;
+  s.lead_tensor = s.store.narrow(0, 2 * n, n).view({c.batch->n_seg, c.Hv});
+  check(fqla_segment_scan((const float*)g.data_ptr(), c.kT(), c.Hv, c.batch->s_cu, 0,
+                          c.batch->s_begin, (int)c.batch->N, THRESHOLD, from_start, s.warm,
+                          s.fallback, s.lead, s.exact_warm, s.any_fb, c.stream),
+        "segment_scan");
+  return s;
+}
+// The scan of the explicit route: every segment takes a start state from the merge chain.
+Scan warmup_scan(const Call& c, const at::Tensor& g, bool from_start) {
+  Scan s{};
+  const int64_t n = c.batch->n_seg * c.Hv;
+  s.store = empty({2 * n}, at::kInt, c.dev);
+  s.warm = s.store.data_ptr<int>();
+  s.fallback = s.warm + n;
+  check(fqla_warmup_scan((const float*)g.data_ptr(), c.kT(), c.Hv, c.batch->s_cu, 0,
+                         (int)c.batch->n_seg, THRESHOLD, from_start,
+                         from_start ? c.batch->keep_bwd : c.batch->keep_fwd, s.warm, s.fallback,
+                         c.stream),
+        "warmup_scan");
+  return s;
+}
+
+// Start states of the segments (and lead-in counts) of a split plan.  Segments whose past dies out
+// inside the segment before them start themselves a few chunks early from a zero state; the exact
+// chain (state-only pass with the transition matrices, then the merge) returns at once for them.
+void segment_starts(const Call& c, const SeqIn& in, const OptTensor& h0, bool lead_in, Cache& out) {
+  const bool leads = lead_in && tiles_ok(c.D);
+  const Scan s = leads ? segment_scan(c, in.g, false) : warmup_scan(c, in.g, false);
+  at::Tensor local = empty({2, c.batch->n_seg, c.Hv, c.D, c.D}, at::kFloat, c.dev);
+  at::Tensor l = local.select(0, 0), M = local.select(0, 1);
+  run_fwd(c, in, false, nullptr, l, std::nullopt, std::nullopt, std::nullopt, M,
+          leads ? s.exact_warm : s.warm, s.fallback, nullptr, false);
+  out.seg_h0 = merge(c, l, M, s.fallback, h0, leads ? s.any_fb : nullptr, false);
+  if (leads) out.lead = s.lead_tensor;
+}
+
+void run_dh(const Call& c, const SeqIn& in, const at::Tensor& dO, const float* dht,
+            const OptTensor& dh, const OptTensor& du, const OptTensor& dh0, const int* warm,
+            const int* lead, bool tiles) {
+  check(fqla_bwd_dh(in.q.data_ptr(), in.k.data_ptr(), in.A.data_ptr(), (const float*)in.g.data_ptr(),
+                    in.beta.data_ptr(), in.beta_f32, dO.data_ptr(), dht, mut(dh), mut(du),
+                    mut<float>(dh0), warm, lead, c.order(), nullptr, 1, c.kB(), c.kT(), c.Hq, c.Hv,
+                    c.D, c.scale, c.cu(), c.offsets(), 0, c.N(), tiles, c.stream),
+        "bwd_dh");
+}
+
+// Mirror image of segment_starts for the state gradient.
+std::pair<at::Tensor, OptTensor> segment_ends(const Call& c, const SeqIn& in, const at::Tensor& dO,
+                                              const OptTensor& dht, bool lead_in, Scan& keep) {
+  const bool leads = lead_in && tiles_ok(c.D);
+  keep = leads ? segment_scan(c, in.g, true) : warmup_scan(c, in.g, true);
+  at::Tensor local = empty({2, c.batch->n_seg, c.Hv, c.D, c.D}, at::kFloat, c.dev);
+  at::Tensor l = local.select(0, 0), M = local.select(0, 1);
+  run_dh(c, in, dO, nullptr, std::nullopt, std::nullopt, l, leads ? keep.exact_warm : keep.warm,
+         nullptr, false);
+  run_fwd(c, in, false, nullptr, std::nullopt, std::nullopt, std::nullopt, std::nullopt, M, nullptr,
+          keep.fallback, nullptr, false);
+  at::Tensor ends = merge(c, l, M, keep.fallback, dht, leads ? keep.any_fb : nullptr, true);
+  return {ends, leads ? OptTensor(keep.lead_tensor) : std::nullopt};
+}
+
+constexpr double L2NORM_EPS = 1e-6;
+
+// q, k, v as the kernels read them: one launch where q, k are normalised or all three are float16,
+// none for bfloat16.
+void prepare(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor& v_in,
+             const Options& opt, Forward& r) {
+  const auto dt = q_in.scalar_type();
+  const bool f16 = dt == at::kHalf;
+  const bool one = k_in.scalar_type() == dt && v_in.scalar_type() == dt && (f16 || dt == at::kBFloat16);
+  if (!(one && (opt.l2norm || f16))) {
+    r.q = as_bf16(q_in);
+    r.k = as_bf16(k_in);
+    r.v = as_bf16(v_in);
+    if (!opt.l2norm) return;
+  }
+  const at::Tensor q = one ? aligned(q_in) : r.q, k = one ? aligned(k_in) : r.k;
+  const at::Tensor v = f16 && one ? aligned(v_in) : as_bf16(v_in);
+  const int64_t D = q.size(-1), rows = D ? q.numel() / D : 0;
+  r.q = empty(q.sizes(), at::kBFloat16, q.device());
+  r.k = empty(k.sizes(), at::kBFloat16, q.device());
+  r.v = f16 && one ? empty(v.sizes(), at::kBFloat16, q.device()) : v;
+  if (opt.norm_grad) {
+    r.q_rstd = empty({rows}, at::kFloat, q.device());
+    r.k_rstd = empty({rows}, at::kFloat, q.device());
+  }
+  check(fqla_prepare_inputs(q.data_ptr(), k.data_ptr(), v.data_ptr(), r.q.data_ptr(),
+                            r.k.data_ptr(), f16 && one ? r.v.data_ptr() : nullptr,
+                            opt.norm_grad ? (float*)r.q_rstd.data_ptr() : nullptr,
+                            opt.norm_grad ? (float*)r.k_rstd.data_ptr() : nullptr, rows,
+                            D ? v.numel() / D : 0, (int)D, f16 && one, opt.l2norm,
+                            (float)L2NORM_EPS,
+                            (void*)at::cuda::getCurrentCUDAStream(q.device().index()).stream()),
+        "prepare_inputs");
+}
+
+void require_cuda(std::initializer_list<const at::Tensor*> ts) {
+  for (const at::Tensor* t : ts)
+    if (!t->is_cuda())
+      throw PyError(PyError::Fqla, "flashqla_b200 kernels need CUDA tensors; there is no CPU fallback");
+}
+
+}  // namespace
+
+Forward forward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor& v_in,
+                const at::Tensor& g_in, const at::Tensor& beta_in_, double scale,
+                const OptTensor& initial_state, const OptTensor& cu, const Options& opt) {
+  require_cuda({&q_in, &k_in, &v_in, &g_in, &beta_in_});
+  c10::cuda::CUDAGuard guard(k_in.device());
+  c10::AutoGradMode no_grad(false);
+  Forward r;
+  const Call c = make_call(q_in, k_in, v_in, scale, cu, opt.auto_cp);
+  prepare(q_in, k_in, v_in, opt, r);
+  const at::Tensor &q = r.q, &k = r.k, &v = r.v;
+  const at::Tensor g = as_f32(g_in), beta = beta_in(beta_in_);
+  const OptTensor h0 = state_in(initial_state, opt.state_v_first);
+  check_state(h0, c);
+
+  // gate cumsum and A = (I + strict_lower(diag(beta) K K^T decay))^-1
+  r.g_cum = empty(g.sizes(), at::kFloat, c.dev);
+  r.A = empty({c.B, c.T, c.Hv, CHUNK}, at::kBFloat16, c.dev);
+  if (c.batch->total < (int64_t)c.B * c.T) r.g_cum.narrow(1, c.batch->total, c.T - c.batch->total).zero_();
+  const int beta_f32 = beta.scalar_type() == at::kFloat;
+  check(fqla_kkt_solve(k.data_ptr(), beta.data_ptr(), beta_f32, (const float*)g.data_ptr(),
+                       (float*)r.g_cum.data_ptr(), r.A.data_ptr(), c.B, c.T, c.Hq, c.Hv, c.D,
+                       c.batch->d_cu, 0, c.batch->d_indices, c.batch->num_chunks, c.stream),
+        "kkt_solve");
+
+  const SeqIn in{q, k, v, r.A, r.g_cum, beta, beta_f32};
+  const bool tiles = tiles_ok(c.D);
+  const bool keep = opt.cache && opt.save_tiles && !opt.output_h;
+  if (c.split) segment_starts(c, in, h0, opt.lead_in, r.cache);
+
+  r.o = empty(v.sizes(), at::kBFloat16, c.dev);
+  OptTensor h, vnew, ht;
+  if (keep || opt.output_h)
+    h = empty({c.batch->num_chunks, c.Hv, c.D, c.D}, at::kBFloat16, c.dev);
+  if (keep)
+    vnew = tiles ? empty({c.batch->num_chunks, c.Hv, c.D, CHUNK}, at::kBFloat16, c.dev)
+                 : empty(v.sizes(), at::kBFloat16, c.dev);
+  if (opt.output_final_state) ht = empty({c.N(), c.Hv, c.D, c.D}, at::kFloat, c.dev);
+  run_fwd(c, in, true, c.split ? ptr<float>(r.cache.seg_h0) : ptr<float>(h0), ht, r.o, h, vnew,
+          std::nullopt, nullptr, nullptr, ptr<int>(r.cache.lead), keep && tiles);
+  if (c.split && ht) ht = ht->index_select(0, c.batch->last_seg);
+  r.final_state = state_out(ht, opt.state_v_first);
+  if (q_in.scalar_type() != at::kBFloat16) r.o = r.o.to(q_in.scalar_type());
+  if (opt.output_h) {
+    at::Tensor x = cu ? h->unsqueeze(0) : h->view({c.B, -1, c.Hv, c.D, c.D});
+    r.h = state_out(x, opt.state_v_first);
+  }
+  if (keep) {
+    r.cache.h = h;
+    r.cache.vnew = vnew;
+  }
+  r.has_cache = opt.cache && (keep || c.split);
+  return r;
+}
+
+Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor& v_in,
+                  const at::Tensor& g_in, const at::Tensor& beta_in_, const at::Tensor& A_in,
+                  const at::Tensor& dO_in, const OptTensor& dht_in, double scale,
+                  const OptTensor& initial_state, const OptTensor& cu, const Options& opt,
+                  const Cache& cached, const Norm* norm, at::ScalarType dtype) {
+  require_cuda({&q_in, &k_in, &v_in, &g_in, &beta_in_, &A_in, &dO_in});
+  c10::cuda::CUDAGuard guard(k_in.device());
+  c10::AutoGradMode no_grad(false);
+  const at::Tensor q = as_bf16(q_in), k = as_bf16(k_in), v = as_bf16(v_in);
+  const at::Tensor dO = as_bf16(dO_in), A = as_bf16(A_in);
+  const at::Tensor g = as_f32(g_in), beta = beta_in(beta_in_);
+  const Call c = make_call(q, k, v, scale, cu, opt.auto_cp);
+  const OptTensor h0 = state_in(initial_state, opt.state_v_first);
+  const OptTensor dht = state_in(dht_in, opt.state_v_first);
+  check_state(h0, c);
+  check_state(dht, c);
+  const int beta_f32 = beta.scalar_type() == at::kFloat;
+  const SeqIn in{q, k, v, A, g, beta, beta_f32};
+  const bool tiles = tiles_ok(c.D);
+
+  // per-chunk states and v_new: kept by the forward, or recomputed
+  OptTensor h = cached.h, vnew = cached.vnew;
+  if (!h || !vnew) {
+    Cache starts{cached.seg_h0, std::nullopt, std::nullopt, cached.lead};
+    if (c.split && !starts.seg_h0) segment_starts(c, in, h0, opt.lead_in, starts);
+    h = empty({c.batch->num_chunks, c.Hv, c.D, c.D}, at::kBFloat16, c.dev);
+    vnew = tiles ? empty({c.batch->num_chunks, c.Hv, c.D, CHUNK}, at::kBFloat16, c.dev)
+                 : empty(v.sizes(), at::kBFloat16, c.dev);
+    run_fwd(c, in, false, c.split ? ptr<float>(starts.seg_h0) : ptr<float>(h0), std::nullopt,
+            std::nullopt, h, vnew, std::nullopt, nullptr, nullptr,
+            tiles ? ptr<int>(starts.lead) : nullptr, tiles);
+  }
+
+  // reverse recurrence of the state gradient
+  OptTensor ends = dht, lead_out;
+  Scan scan{};
+  if (c.split) {
+    auto [e, l] = segment_ends(c, in, dO, dht, opt.lead_in, scan);
+    ends = e;
+    lead_out = l;
+  }
+  at::Tensor dh = empty({c.batch->num_chunks, c.Hv, c.D, c.D}, at::kBFloat16, c.dev);
+  at::Tensor du = tiles ? empty({c.batch->num_chunks, c.Hv, c.D, CHUNK}, at::kBFloat16, c.dev)
+                        : empty(v.sizes(), at::kBFloat16, c.dev);
+  OptTensor dh0;
+  if (initial_state) dh0 = empty({c.N(), c.Hv, c.D, c.D}, at::kFloat, c.dev);
+  run_dh(c, in, dO, ptr<float>(ends), dh, du, dh0, nullptr, ptr<int>(lead_out), tiles);
+
+  // chunk-parallel part, per value head
+  Backward r;
+  const int64_t total = c.batch->total, rows = (int64_t)c.B * c.T;
+  r.dq = empty({c.B, c.T, c.Hv, c.D}, at::kBFloat16, c.dev);
+  r.dk = empty({c.B, c.T, c.Hv, c.D}, at::kBFloat16, c.dev);
+  r.dv = empty({c.B, c.T, c.Hv, c.D}, at::kBFloat16, c.dev);
+  r.db = empty({c.B, c.T, c.Hv}, at::kFloat, c.dev);
+  at::Tensor dg = empty({c.B, c.T, c.Hv}, at::kFloat, c.dev);
+  r.dg = empty({c.B, c.T, c.Hv}, at::kFloat, c.dev);
+  if (total < rows)  // rows past the last packed sequence are never written by the kernels
+    for (at::Tensor* t : {&r.dq, &r.dk, &r.dv, &r.db, &r.dg}) t->narrow(1, total, rows - total).zero_();
+  check(fqla_bwd_main(q.data_ptr(), k.data_ptr(), v.data_ptr(), vnew->data_ptr(), A.data_ptr(),
+                      (const float*)g.data_ptr(), beta.data_ptr(), beta_f32, dO.data_ptr(),
+                      du.data_ptr(), h->data_ptr(), dh.data_ptr(), r.dq.data_ptr(), r.dk.data_ptr(),
+                      r.dv.data_ptr(), (float*)r.db.data_ptr(), (float*)dg.data_ptr(), c.kB(), c.kT(),
+                      c.Hq, c.Hv, c.D, c.scale, c.cu(), c.offsets(), c.indices(), 0,
+                      c.batch->num_chunks, tiles, c.stream),
+        "bwd_main");
+  const bool f16 = dtype == at::kHalf;
+  if (c.Hq < c.Hv || norm || f16) {
+    const auto t = f16 ? at::kHalf : at::kBFloat16;
+    at::Tensor dq = empty({c.B, c.T, c.Hq, c.D}, t, c.dev), dk = empty({c.B, c.T, c.Hq, c.D}, t, c.dev);
+    at::Tensor dv = f16 ? empty(v.sizes(), t, c.dev) : r.dv;
+    // the gradient of the normalisation reads its inputs in the type of its outputs
+    at::Tensor nq, nk;
+    if (norm) {
+      nq = aligned(norm->q.scalar_type() == t ? norm->q : norm->q.to(t));
+      nk = aligned(norm->k.scalar_type() == t ? norm->k : norm->k.to(t));
+    }
+    check(fqla_finish_grads(r.dq.data_ptr(), r.dk.data_ptr(), f16 ? r.dv.data_ptr() : nullptr,
+                            norm ? nq.data_ptr() : nullptr, norm ? nk.data_ptr() : nullptr,
+                            norm ? (const float*)norm->q_rstd.data_ptr() : nullptr,
+                            norm ? (const float*)norm->k_rstd.data_ptr() : nullptr, dq.data_ptr(),
+                            dk.data_ptr(), f16 ? dv.data_ptr() : nullptr, rows * c.Hq, c.Hv / c.Hq,
+                            c.D, f16, c.stream),
+          "finish_grads");
+    r.dq = dq;
+    r.dk = dk;
+    r.dv = dv;
+  }
+  check(fqla_chunk_local_cumsum((const float*)dg.data_ptr(), (float*)r.dg.data_ptr(), c.B, c.T, c.Hv,
+                                c.batch->d_cu, 0, (int)c.batch->N, c.batch->d_indices,
+                                c.batch->num_chunks, 1, c.stream),
+        "chunk_local_cumsum");
+  if (!f16 && dtype != at::kBFloat16)
+    for (at::Tensor* t : {&r.dq, &r.dk, &r.dv}) *t = t->to(dtype);
+  if (dh0) {
+    if (c.split) dh0 = dh0->index_select(0, c.batch->first_seg);
+    r.dh0 = state_out(dh0, opt.state_v_first);
+  }
+  return r;
+}
+
+}  // namespace fqla_host

@@ -1,0 +1,63 @@
+// The forward and backward of the operator as sequences of launches of the C-ABI kernels.
+#pragma once
+#include <ATen/ATen.h>
+
+#include <atomic>
+#include <optional>
+
+namespace fqla_host {
+
+using OptTensor = std::optional<at::Tensor>;
+
+struct Options {
+  bool output_final_state = true;
+  bool output_h = false;
+  bool auto_cp = true;
+  bool state_v_first = false;
+  bool cache = false;       // hand the backward what it would recompute
+  bool save_tiles = true;   // ... the per-chunk states and v_new among it
+  bool l2norm = false;      // L2-normalise the rows of q and k first
+  bool norm_grad = false;   // ... and keep what its gradient needs
+  bool lead_in = true;      // segments of a split plan start themselves from a zero state
+};
+
+// What the forward keeps for the backward: start states of the segments of a split plan, per-chunk
+// states and v_new (operand tiles for K = V = 128, row-major for 64), lead-in chunk counts.
+struct Cache {
+  OptTensor seg_h0, h, vnew, lead;
+};
+
+// The L2 normalisation of q and k: the rows before it and their reciprocal norms.
+struct Norm {
+  at::Tensor q, k, q_rstd, k_rstd;
+};
+
+struct Forward {
+  at::Tensor g_cum, A, o;
+  OptTensor h, final_state;
+  bool has_cache = false;
+  Cache cache;
+  at::Tensor q, k, v;          // what the kernels read: bfloat16, normalised where asked for
+  at::Tensor q_rstd, k_rstd;   // with norm_grad
+};
+
+struct Backward {
+  at::Tensor dq, dk, dv, db, dg;
+  OptTensor dh0;
+};
+
+Forward forward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& g,
+                const at::Tensor& beta, double scale, const OptTensor& initial_state,
+                const OptTensor& cu, const Options& opt);
+
+// `g_cum` and `A` are the forward's; q, k the ones its kernels read.  With `norm` the gradients of q,
+// k are mapped back through the normalisation.  dq, dk, dv come in `dtype`, db and dg in float32.
+Backward backward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                  const at::Tensor& g_cum, const at::Tensor& beta, const at::Tensor& A,
+                  const at::Tensor& dO, const OptTensor& dht, double scale,
+                  const OptTensor& initial_state, const OptTensor& cu, const Options& opt,
+                  const Cache& cache, const Norm* norm, at::ScalarType dtype);
+
+extern std::atomic<long long> launch_count;  // kernels enqueued by this file
+
+}  // namespace fqla_host

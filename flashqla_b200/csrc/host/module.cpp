@@ -1,0 +1,262 @@
+// Python bindings of the native host path (flashqla_b200._host).
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/python_headers.h>
+
+#include <cmath>
+#include <string>
+
+#include "autograd.h"
+#include "errors.h"
+#include "gdr.h"
+#include "planner.h"
+
+namespace fqla_host {
+namespace {
+
+PyObject* fqla_error = nullptr;  // flashqla_b200._lib.FqlaError
+
+PyObject* raise(const std::exception& e) {
+  PyObject* type = PyExc_RuntimeError;
+  if (auto* p = dynamic_cast<const PyError*>(&e)) {
+    switch (p->kind) {
+      case PyError::Assertion: type = PyExc_AssertionError; break;
+      case PyError::Type: type = PyExc_TypeError; break;
+      case PyError::Value: type = PyExc_ValueError; break;
+      case PyError::NotImplemented: type = PyExc_NotImplementedError; break;
+      case PyError::Fqla: type = fqla_error ? fqla_error : PyExc_RuntimeError; break;
+    }
+  } else if (auto* c = dynamic_cast<const c10::OutOfMemoryError*>(&e)) {
+    // torch.OutOfMemoryError, as the caching allocator's failures surface everywhere else
+    PyObject* torch = PyImport_ImportModule("torch");
+    PyObject* oom = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
+    if (oom) PyErr_SetString(oom, c->what_without_backtrace());
+    Py_XDECREF(oom);
+    Py_XDECREF(torch);
+    return nullptr;
+  }
+  PyErr_SetString(type, e.what());
+  return nullptr;
+}
+
+at::Tensor tensor(PyObject* o, const char* name) {
+  if (!THPVariable_Check(o)) throw PyError(PyError::Type, std::string(name) + " must be a tensor");
+  return THPVariable_Unpack(o);
+}
+OptTensor opt_tensor(PyObject* o, const char* name) {
+  if (o == Py_None) return std::nullopt;
+  return tensor(o, name);
+}
+// other Python threads run while the host path works (it may wait for the device)
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+template <typename F>
+auto without_gil(F&& f) {
+  WithoutGil w;
+  return f();
+}
+
+PyObject* wrap(const at::Tensor& t) { return THPVariable_Wrap(t); }
+PyObject* wrap(const OptTensor& t) {
+  if (!t) Py_RETURN_NONE;
+  return THPVariable_Wrap(*t);
+}
+template <typename... Ts>
+PyObject* tuple_of(const Ts&... ts) {
+  PyObject* out = PyTuple_New(sizeof...(ts));
+  if (!out) return nullptr;
+  Py_ssize_t i = 0;
+  for (PyObject* x : {wrap(ts)...}) PyTuple_SET_ITEM(out, i++, x);
+  return out;
+}
+
+// bits of the `flags` argument; the operator module (flash_qla/ops/gated_delta_rule/chunk) has the same list
+enum { FINAL_STATE = 1, OUTPUT_H = 2, AUTO_CP = 4, V_FIRST = 8, CACHE = 16, SAVE_TILES = 32, LEAD_IN = 64,
+       L2NORM = 128 };
+
+Options options(PyObject* o) {
+  const long f = PyLong_AsLong(o);
+  if (f == -1 && PyErr_Occurred()) throw PyError(PyError::Type, "flags must be an int");
+  Options opt;
+  opt.output_final_state = f & FINAL_STATE;
+  opt.output_h = f & OUTPUT_H;
+  opt.auto_cp = f & AUTO_CP;
+  opt.state_v_first = f & V_FIRST;
+  opt.cache = f & CACHE;
+  opt.save_tiles = f & SAVE_TILES;
+  opt.lead_in = f & LEAD_IN;
+  opt.l2norm = opt.norm_grad = f & L2NORM;
+  return opt;
+}
+
+double number(PyObject* o) {
+  const double x = PyFloat_AsDouble(o);
+  if (x == -1.0 && PyErr_Occurred()) {
+    PyErr_Clear();
+    throw PyError(PyError::Type, "scale must be a number");
+  }
+  return x;
+}
+
+// apply(q, k, v, g, beta, scale or None, initial_state, cu_seqlens, flags) -> (o, final_state),
+// recorded for autograd.  The argument checks of the public operator are made here.
+PyObject* py_apply(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  try {
+    if (n != 9) throw PyError(PyError::Type, "apply takes 9 arguments");
+    const at::Tensor q = tensor(a[0], "q"), k = tensor(a[1], "k"), v = tensor(a[2], "v");
+    const OptTensor h0 = opt_tensor(a[6], "initial_state"), cu = opt_tensor(a[7], "cu_seqlens");
+    if (q.scalar_type() != k.scalar_type() || k.scalar_type() != v.scalar_type())
+      throw PyError(PyError::Assertion, "q, k and v must have one dtype");
+    if (q.scalar_type() != at::kBFloat16 && q.scalar_type() != at::kHalf)
+      throw PyError(PyError::Assertion, "FlashQLA only supports bfloat16 and float16.");
+    if (k.size(2) == 0 || v.size(2) % k.size(2) != 0)
+      throw PyError(PyError::Assertion, "num_qk_heads must be divisible to num_v_heads.");
+    if (cu) {
+      if (q.size(0) != 1)
+        throw PyError(PyError::Value,
+                      "The batch size is expected to be 1 rather than " + std::to_string(q.size(0)) +
+                          " when using `cu_seqlens`. Please flatten variable-length inputs before processing.");
+      if (h0 && h0->size(0) != cu->size(0) - 1)
+        throw PyError(PyError::Value,
+                      "The number of initial states is expected to be equal to the number of input "
+                      "sequences, i.e., " + std::to_string(cu->size(0) - 1) + " rather than " +
+                          std::to_string(h0->size(0)) + ".");
+    }
+    const double scale = a[5] == Py_None ? 1.0 / std::sqrt((double)k.size(-1)) : number(a[5]);
+    const at::Tensor g = tensor(a[3], "g"), beta = tensor(a[4], "beta");
+    const Options opt = options(a[8]);
+    const auto r = without_gil([&] { return apply(q, k, v, g, beta, scale, h0, cu, opt); });
+    return tuple_of(r.first, r.second);
+  } catch (const std::exception& e) {
+    return raise(e);
+  }
+}
+
+// forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, flags)
+//   -> (g_cum, A, o, h, final_state, cp_cache), with L2NORM also (q, k, q_rstd, k_rstd)
+PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  try {
+    if (n != 9) throw PyError(PyError::Type, "forward takes 9 arguments");
+    const at::Tensor q = tensor(a[0], "q"), k = tensor(a[1], "k"), v = tensor(a[2], "v"),
+                     g = tensor(a[3], "g"), beta = tensor(a[4], "beta");
+    const double scale = number(a[5]);
+    const OptTensor h0 = opt_tensor(a[6], "initial_state"), cu = opt_tensor(a[7], "cu_seqlens");
+    const Options opt = options(a[8]);
+    const Forward r = without_gil([&] { return forward(q, k, v, g, beta, scale, h0, cu, opt); });
+    PyObject* cache;
+    if (r.has_cache) {
+      cache = tuple_of(r.cache.seg_h0, r.cache.h, r.cache.vnew, r.cache.lead);
+    } else {
+      cache = Py_None;
+      Py_INCREF(cache);
+    }
+    const bool norm = r.q_rstd.defined();
+    PyObject* out = PyTuple_New(norm ? 10 : 6);
+    PyTuple_SET_ITEM(out, 0, wrap(r.g_cum));
+    PyTuple_SET_ITEM(out, 1, wrap(r.A));
+    PyTuple_SET_ITEM(out, 2, wrap(r.o));
+    PyTuple_SET_ITEM(out, 3, wrap(r.h));
+    PyTuple_SET_ITEM(out, 4, wrap(r.final_state));
+    PyTuple_SET_ITEM(out, 5, cache);
+    if (norm) {
+      PyTuple_SET_ITEM(out, 6, wrap(r.q));
+      PyTuple_SET_ITEM(out, 7, wrap(r.k));
+      PyTuple_SET_ITEM(out, 8, wrap(r.q_rstd));
+      PyTuple_SET_ITEM(out, 9, wrap(r.k_rstd));
+    }
+    return out;
+  } catch (const std::exception& e) {
+    return raise(e);
+  }
+}
+
+// backward(q, k, v, g_cum, beta, A, do, dht, scale, initial_state, cu_seqlens, flags, cp_cache, norm)
+//   -> (dq, dk, dv, db, dg, dh0);  norm: None or (q, k before the normalisation, q_rstd, k_rstd)
+PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  try {
+    if (n != 14) throw PyError(PyError::Type, "backward takes 14 arguments");
+    Cache cache;
+    if (a[12] != Py_None) {
+      if (!PyTuple_Check(a[12])) throw PyError(PyError::Type, "cp_cache must be a tuple or None");
+      OptTensor* slots[4] = {&cache.seg_h0, &cache.h, &cache.vnew, &cache.lead};
+      for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[12]) && i < 4; ++i)
+        *slots[i] = opt_tensor(PyTuple_GET_ITEM(a[12], i), "cp_cache entry");
+    }
+    Norm norm;
+    if (a[13] != Py_None) {
+      if (!PyTuple_Check(a[13]) || PyTuple_GET_SIZE(a[13]) != 4)
+        throw PyError(PyError::Type, "norm must be a tuple of four tensors or None");
+      at::Tensor* parts[4] = {&norm.q, &norm.k, &norm.q_rstd, &norm.k_rstd};
+      for (int i = 0; i < 4; ++i) *parts[i] = tensor(PyTuple_GET_ITEM(a[13], i), "norm entry");
+    }
+    const at::Tensor q = tensor(a[0], "q"), k = tensor(a[1], "k"), v = tensor(a[2], "v"),
+                     g = tensor(a[3], "g"), beta = tensor(a[4], "beta"), A = tensor(a[5], "A"),
+                     dO = tensor(a[6], "do");
+    const OptTensor dht = opt_tensor(a[7], "dht"), h0 = opt_tensor(a[9], "initial_state"),
+                    cu = opt_tensor(a[10], "cu_seqlens");
+    const double scale = number(a[8]);
+    const Options opt = options(a[11]);
+    const bool normed = a[13] != Py_None;
+    Backward r = without_gil([&] {
+      return backward(q, k, v, g, beta, A, dO, dht, scale, h0, cu, opt, cache, normed ? &norm : nullptr,
+                      (normed ? norm.q : q).scalar_type());
+    });
+    if (r.db.scalar_type() != beta.scalar_type()) r.db = r.db.to(beta.scalar_type());
+    return tuple_of(r.dq, r.dk, r.dv, r.db, r.dg, r.dh0);
+  } catch (const std::exception& e) {
+    return raise(e);
+  }
+}
+
+// split_sequences(bounds, heads, n_sm, min_chunks, slices) -> None or (seg_bounds, seg_begin)
+PyObject* py_split(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  try {
+    if (n != 5) throw PyError(PyError::Type, "split_sequences takes 5 arguments");
+    PyObject* seq = PySequence_Fast(a[0], "bounds must be a sequence of ints");
+    if (!seq) return nullptr;
+    std::vector<int64_t> bounds;
+    for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq); ++i)
+      bounds.push_back(PyLong_AsLongLong(PySequence_Fast_GET_ITEM(seq, i)));
+    Py_DECREF(seq);
+    long long x[4];
+    for (int i = 0; i < 4; ++i) x[i] = PyLong_AsLongLong(a[1 + i]);
+    if (PyErr_Occurred()) return nullptr;
+    const auto s = split_sequences(bounds, x[0], x[1], x[2], x[3]);
+    if (!s) Py_RETURN_NONE;
+    auto list = [](const std::vector<int64_t>& v) {
+      PyObject* l = PyList_New((Py_ssize_t)v.size());
+      for (size_t i = 0; i < v.size(); ++i) PyList_SET_ITEM(l, (Py_ssize_t)i, PyLong_FromLongLong(v[i]));
+      return l;
+    };
+    PyObject* out = PyTuple_New(2);
+    PyTuple_SET_ITEM(out, 0, list(s->seg_bounds));
+    PyTuple_SET_ITEM(out, 1, list(s->seg_begin));
+    return out;
+  } catch (const std::exception& e) {
+    return raise(e);
+  }
+}
+
+PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(launch_count.load()); }
+
+PyObject* py_set_error(PyObject*, PyObject* type) {
+  Py_XINCREF(type);
+  Py_XSETREF(fqla_error, type);
+  Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {
+    {"apply", (PyCFunction)(void*)py_apply, METH_FASTCALL, "the operator, recorded for autograd"},
+    {"forward", (PyCFunction)(void*)py_forward, METH_FASTCALL, "the whole forward"},
+    {"backward", (PyCFunction)(void*)py_backward, METH_FASTCALL, "the whole backward"},
+    {"split_sequences", (PyCFunction)(void*)py_split, METH_FASTCALL, "segment planner"},
+    {"launches", py_launches, METH_NOARGS, "kernels enqueued so far"},
+    {"set_error_type", py_set_error, METH_O, "exception type of failed launches"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods};
+
+}  // namespace
+}  // namespace fqla_host
+
+PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&fqla_host::module); }

@@ -164,6 +164,25 @@ int fqla_l2norm_fwd(const void* x, void* y, float* rstd, long long rows, int D, 
 int fqla_l2norm_bwd(const void* y, const float* rstd, const void* dy, float* dx, long long rows,
                     int D, int y_dtype, int dy_dtype, void* stream);
 
+/* One pass over the operator's inputs: q, k (optionally L2-normalised per row, eps as above) and,
+ * with v_out, v come out as bf16 from bf16 or (is_f16) fp16.  rows_qk rows of D in q and in k,
+ * rows_v in v; q_rstd, k_rstd (fp32 [rows_qk], optional) get the reciprocal norms.  D 64 or 128;
+ * q, k, v 16-byte aligned and contiguous.
+ * Replaces the two calls of l2norm_fwd in chunk/__init__.py:193-196 and the dtype casts. */
+int fqla_prepare_inputs(const void* q, const void* k, const void* v, void* q_out, void* k_out,
+                        void* v_out, float* q_rstd, float* k_rstd, long long rows_qk,
+                        long long rows_v, int D, int is_f16, int normalise, float eps,
+                        void* stream);
+/* One pass over the gradients of fqla_bwd_main: dq, dk = sum over the G value heads of a group of
+ * dq_v, dk_v (bf16), mapped back through the L2 normalisation when q_rstd, k_rstd are given (q, k:
+ * the operator's own inputs, before normalisation), written as bf16 or (is_f16) fp16; with dv_in,
+ * dv is converted too.  rows_qk rows of D per q/k head row.
+ * Replaces group_reduce_vector (ops/utils/group_reduce.py:60-79) and l2norm_bwd
+ * (utils/math.py:38-51) as the backward calls them. */
+int fqla_finish_grads(const void* dq_v, const void* dk_v, const void* dv_in, const void* q,
+                      const void* k, const float* q_rstd, const float* k_rstd, void* dq, void* dk,
+                      void* dv, long long rows_qk, int G, int D, int is_f16, void* stream);
+
 /* The scan of fqla_warmup_scan for a whole split plan in one launch, plus the decision how each
  * segment gets its start state.  seg_begin [n_raw+1] (int32): first segment of every raw
  * sequence.  Outputs, all int32: warm, fallback [n_seg,Hv] as for fqla_warmup_scan (the segment
