@@ -20,6 +20,9 @@ SIGNATURES = {
     "fqla_fwd_seq": [P] * 6 + [I] + [P] * 11 + [I] * 6 + [F, P, P, I, I, I, P],
     "fqla_bwd_dh": [P, P, P, P, P, I, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, P, P, I, I, I,
                     P],
+    "fqla_fwd_run": [P, P],
+    "fqla_bwd_dh_run": [P, P],
+    "fqla_bwd_main_run": [P, P],
     "fqla_bwd_main": [P] * 7 + [I] + [P] * 9 + [I, I, I, I, I, F, P, P, P, I, LL, I, P],
     "fqla_group_reduce": [P, P, LL, I, I, I, P],
     "fqla_warmup_scan": [P, I, I, P, I, I, F, I, P, P, P, P],

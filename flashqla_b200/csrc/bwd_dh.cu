@@ -27,7 +27,10 @@ struct BwdDhParams {
   const void* beta;
   int beta_is_f32;
   const bf16* dO;
-  const float* dht;  // [N, Hv, D, D] or null
+  const float* dht;  // [*, Hv, D, D] or null; the next four: see fqla_bwd_dh_args
+  const float* seg_dht;
+  const int *dht_row, *dh0_row;
+  int v_first;
   bf16* dh;          // [chunks, Hv, D, D] or null
   bf16* du;          // [rows, Hv, D] or null
   float* dh0;        // [N, Hv, D, D] or null
@@ -86,6 +89,7 @@ __global__ void __launch_bounds__(256, 1) bwd_dh_kernel(const BwdDhParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wm = warp & 3, wn = warp >> 2;
   const int hv = blockIdx.x % p.Hv;
+  pdl_wait();
   const int n = p.order ? p.order[blockIdx.x / p.Hv] : (int)(blockIdx.x / p.Hv);
   const int hq = hv / (p.Hv / p.Hq);
   const int v0 = blockIdx.y * BV;
@@ -99,7 +103,11 @@ __global__ void __launch_bounds__(256, 1) bwd_dh_kernel(const BwdDhParams p) {
   }
 
   float dS[MTS][NTV][4];
-  const long long state_off = ((long long)n * p.Hv + hv) * D * D;
+  const int dht_row = p.dht_row ? p.dht_row[n] : n;
+  const bool edge = dht_row >= 0;  // ends its sequence; else it is handed a gradient, if any
+  const float* dht = c_end != sp.n_chunks ? nullptr : edge ? p.dht : p.seg_dht;
+  if (dht) dht += ((long long)(edge ? dht_row : n) * p.Hv + hv) * D * D;
+  const bool dht_v_first = edge && p.v_first;
 #pragma unroll
   for (int mt = 0; mt < MTS; ++mt)
 #pragma unroll
@@ -108,8 +116,7 @@ __global__ void __launch_bounds__(256, 1) bwd_dh_kernel(const BwdDhParams p) {
       for (int e = 0; e < 4; ++e) {
         int r = (16 * MTS) * wm + mt * 16 + (lane >> 2) + (e >> 1) * 8;
         int c = v0 + (BV / 2) * wn + nt * 8 + (lane & 3) * 2 + (e & 1);
-        dS[mt][nt][e] =
-            (p.dht && c_end == sp.n_chunks) ? p.dht[state_off + (long long)r * D + c] : 0.f;
+        dS[mt][nt][e] = dht ? dht[dht_v_first ? (long long)c * D + r : (long long)r * D + c] : 0.f;
       }
   auto store_state_copy = [&]() {
 #pragma unroll
@@ -274,7 +281,9 @@ __global__ void __launch_bounds__(256, 1) bwd_dh_kernel(const BwdDhParams p) {
     store_state_copy();  // last read in phase A, two barriers ago
   }
 
-  if (p.dh0) {
+  const int dh0_row = p.dh0_row ? p.dh0_row[n] : n;
+  if (p.dh0 && dh0_row >= 0) {
+    float* dst = p.dh0 + ((long long)dh0_row * p.Hv + hv) * D * D;
 #pragma unroll
     for (int mt = 0; mt < MTS; ++mt)
 #pragma unroll
@@ -283,8 +292,13 @@ __global__ void __launch_bounds__(256, 1) bwd_dh_kernel(const BwdDhParams p) {
         for (int hh = 0; hh < 2; ++hh) {
           int r = (16 * MTS) * wm + mt * 16 + (lane >> 2) + hh * 8;
           int c = v0 + (BV / 2) * wn + nt * 8 + (lane & 3) * 2;
-          *reinterpret_cast<float2*>(p.dh0 + state_off + (long long)r * D + c) =
-              make_float2(dS[mt][nt][2 * hh], dS[mt][nt][2 * hh + 1]);
+          if (p.v_first) {
+            dst[(long long)c * D + r] = dS[mt][nt][2 * hh];
+            dst[(long long)(c + 1) * D + r] = dS[mt][nt][2 * hh + 1];
+          } else {
+            *reinterpret_cast<float2*>(dst + (long long)r * D + c) =
+                make_float2(dS[mt][nt][2 * hh], dS[mt][nt][2 * hh + 1]);
+          }
         }
   }
 }
@@ -293,23 +307,49 @@ template <int D>
 static int launch_bwd_dh(const BwdDhParams& p, cudaStream_t st) {
   constexpr int BV = 64;
   using L = BwdDhSmem<D, BV>;
-  int rc = configure_smem((const void*)bwd_dh_kernel<D, BV>, L::BYTES);
+  static std::atomic<unsigned long long> done;
+  int rc = configure_smem((const void*)bwd_dh_kernel<D, BV>, L::BYTES, done);
   if (rc != 0) return rc;
   dim3 grid((unsigned)(p.N * p.Hv), D / BV);
-  bwd_dh_kernel<D, BV><<<grid, 256, L::BYTES, st>>>(p);
-  return (int)cudaGetLastError();
+  return launch_pdl(bwd_dh_kernel<D, BV>, grid, dim3(256), L::BYTES, st, p);
 }
 
 // tcgen05 version for K = V = 128, full walks only (bwd_dh_tc.cu)
-int launch_bwd_dh_tc(const void* q, const void* k, const void* A, const float* g, const void* beta,
-                     int beta_is_f32, const void* dO, const float* dht, void* dh, void* du,
-                     float* dh0, int tiled, const int* lead, const int* order, const int* run_mask,
-                     int run_value, int N, int Hq, int Hv,
-                     long long T_rows, float scale, SeqLayout lay, cudaStream_t st);
+int launch_bwd_dh_tc(const fqla_bwd_dh_args& a, int N, SeqLayout lay, cudaStream_t st);
 
 }  // namespace fqla
 
 using namespace fqla;
+
+extern "C" int fqla_bwd_dh_run(const fqla_bwd_dh_args* args, void* stream) {
+  if (!args) return FQLA_ERR_INVALID_ARG;
+  const fqla_bwd_dh_args& a = *args;
+  if (!a.q || !a.k || !a.A || !a.g_cum || !a.beta || !a.dO || a.Hq <= 0 || a.Hv % a.Hq)
+    return FQLA_ERR_INVALID_ARG;
+  if (a.cu_seqlens && (!a.chunk_offsets || a.B != 1)) return FQLA_ERR_INVALID_ARG;
+  if (a.warm_chunks && (a.dh || a.du)) return FQLA_ERR_INVALID_ARG;
+  if (a.lead_chunks && a.warm_chunks) return FQLA_ERR_INVALID_ARG;
+  const int N = a.cu_seqlens ? a.N : a.B;
+  if (N <= 0) return FQLA_OK;
+  const SeqLayout lay{{a.cu_seqlens, a.idx_is64}, {a.chunk_offsets, a.idx_is64}, a.T};
+  cudaStream_t st = (cudaStream_t)stream;
+  static const bool force_legacy = getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
+  if (a.D == 128 && !a.warm_chunks && !force_legacy) return launch_bwd_dh_tc(a, N, lay, st);
+  // only the tcgen05 kernel writes tiles or leads out
+  if (a.operand_tiles || a.lead_chunks) return FQLA_ERR_UNSUPPORTED_DIM;
+  BwdDhParams p;
+  p.q = (const bf16*)a.q; p.k = (const bf16*)a.k; p.A = (const bf16*)a.A; p.g = a.g_cum;
+  p.beta = a.beta; p.beta_is_f32 = a.beta_is_f32; p.dO = (const bf16*)a.dO;
+  p.dht = a.dht; p.seg_dht = a.seg_dht; p.dht_row = a.dht_row; p.dh0_row = a.dh0_row;
+  p.v_first = a.state_v_first;
+  p.dh = (bf16*)a.dh; p.du = (bf16*)a.du; p.dh0 = a.dh0; p.warm = a.warm_chunks; p.order = a.seq_order;
+  p.run_mask = a.run_mask; p.run_value = a.run_value;
+  p.N = N; p.Hq = a.Hq; p.Hv = a.Hv; p.scale = a.scale;
+  p.lay = lay;
+  if (a.D == 128) return launch_bwd_dh<128>(p, st);
+  if (a.D == 64) return launch_bwd_dh<64>(p, st);
+  return FQLA_ERR_UNSUPPORTED_DIM;
+}
 
 extern "C" int fqla_bwd_dh(const void* q, const void* k, const void* A, const float* g_cum,
                            const void* beta, int beta_is_f32, const void* dO, const float* dht,
@@ -319,28 +359,12 @@ extern "C" int fqla_bwd_dh(const void* q, const void* k, const void* A, const fl
                            const void* cu_seqlens,
                            const void* chunk_offsets, int idx_is64, int N, int operand_tiles,
                            void* stream) {
-  if (!q || !k || !A || !g_cum || !beta || !dO || Hq <= 0 || Hv % Hq)
-    return FQLA_ERR_INVALID_ARG;
-  if (cu_seqlens && (!chunk_offsets || B != 1)) return FQLA_ERR_INVALID_ARG;
-  if (warm_chunks && (dh || du)) return FQLA_ERR_INVALID_ARG;
-  if (lead_chunks && warm_chunks) return FQLA_ERR_INVALID_ARG;
-  BwdDhParams p;
-  p.q = (const bf16*)q; p.k = (const bf16*)k; p.A = (const bf16*)A; p.g = g_cum;
-  p.beta = beta; p.beta_is_f32 = beta_is_f32; p.dO = (const bf16*)dO; p.dht = dht;
-  p.dh = (bf16*)dh; p.du = (bf16*)du; p.dh0 = dh0; p.warm = warm_chunks; p.order = seq_order;
-  p.run_mask = run_mask; p.run_value = run_value;
-  p.N = cu_seqlens ? N : B; p.Hq = Hq; p.Hv = Hv; p.scale = scale;
-  p.lay = SeqLayout{{cu_seqlens, idx_is64}, {chunk_offsets, idx_is64}, T};
-  if (p.N <= 0) return FQLA_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  static const bool force_legacy = getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
-  if (D == 128 && !warm_chunks && !force_legacy)
-    return launch_bwd_dh_tc(q, k, A, g_cum, beta, beta_is_f32, dO, dht, dh, du, dh0,
-                            operand_tiles, lead_chunks, seq_order, run_mask, run_value, p.N, Hq, Hv, (long long)B * T, scale, p.lay,
-                            st);
-  // only the tcgen05 kernel writes tiles or leads out
-  if (operand_tiles || lead_chunks) return FQLA_ERR_UNSUPPORTED_DIM;
-  if (D == 128) return launch_bwd_dh<128>(p, st);
-  if (D == 64) return launch_bwd_dh<64>(p, st);
-  return FQLA_ERR_UNSUPPORTED_DIM;
+  fqla_bwd_dh_args a = {};
+  a.q = q; a.k = k; a.A = A; a.g_cum = g_cum; a.beta = beta; a.beta_is_f32 = beta_is_f32;
+  a.dO = dO; a.dht = dht; a.dh = dh; a.du = du; a.dh0 = dh0; a.warm_chunks = warm_chunks;
+  a.lead_chunks = lead_chunks; a.seq_order = seq_order; a.run_mask = run_mask;
+  a.run_value = run_value; a.B = B; a.T = T; a.Hq = Hq; a.Hv = Hv; a.D = D; a.scale = scale;
+  a.cu_seqlens = cu_seqlens; a.chunk_offsets = chunk_offsets; a.idx_is64 = idx_is64; a.N = N;
+  a.operand_tiles = operand_tiles;
+  return fqla_bwd_dh_run(&a, stream);
 }

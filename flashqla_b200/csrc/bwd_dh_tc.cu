@@ -33,10 +33,13 @@ struct BwdDhTcParams {
   const float* g;
   const void* beta;
   int beta_is_f32;
-  const float* dht;  // [N, Hv, D, D] or null
+  const float* dht;  // [*, Hv, D, D] or null; the next four: see fqla_bwd_dh_args in include/fqla.h
+  const float* seg_dht;
+  const int *dht_row, *dh0_row;
+  int v_first;
   bf16* dh;          // [chunks, Hv, D, D] or null
   bf16* du;          // [rows, Hv, D] or null
-  float* dh0;        // [N, Hv, D, D] or null
+  float* dh0;        // [*, Hv, D, D] or null
   int N, Hq, Hv;
   float scale;
   SeqLayout lay;
@@ -99,15 +102,12 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int hv = blockIdx.x % p.Hv;
-  const int n = p.order ? p.order[blockIdx.x / p.Hv] : (int)(blockIdx.x / p.Hv);
+  auto sequence = [&] { return p.order ? p.order[blockIdx.x / p.Hv] : (int)(blockIdx.x / p.Hv); };
   const int hq = hv / (p.Hv / p.Hq);
-  if (p.run_mask && p.run_mask[n * p.Hv + hv] != p.run_value) return;  // uniform per CTA
-  const SeqSpan sp = p.lay.span(n);
-  // iteration `it` handles chunk n_it - 1 - it of the segment; chunks >= sp.n_chunks are the
-  // lead-out chunks (whole chunks, except possibly the very last one of the sequence)
-  const int lead = (p.lead && sp.n_chunks > 0) ? p.lead[n * p.Hv + hv] : 0;
-  const int n_it = sp.n_chunks + lead;
-  const int len_ext = sp.len + (lead > 0 ? min(lead * CHUNK, p.lay.span(n + 1).len) : 0);
+  if (p.run_mask) {
+    pdl_wait();
+    if (p.run_mask[sequence() * p.Hv + hv] != p.run_value) return;  // uniform per CTA
+  }
 
   if (tid == 0) {
     mbar_init(&bars[FULL0], 1);
@@ -144,27 +144,73 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     *reinterpret_cast<uint4*>(smem + OFF_P + i * 16) = make_uint4(0, 0, 0, 0);
   fence_proxy_async();
   if (warp == 0) tmem_alloc(tmem_slot, 512);
+  // everything above overlaps the tail of the kernel before: no global memory up to here
+  pdl_wait();
+  const int n = sequence();
+  const SeqSpan sp = p.lay.span(n);
+  // iteration `it` handles chunk n_it - 1 - it of the segment; chunks >= sp.n_chunks are the
+  // lead-out chunks (whole chunks, except possibly the very last one of the sequence)
+  const int lead = (p.lead && sp.n_chunks > 0) ? p.lead[n * p.Hv + hv] : 0;
+  const int n_it = sp.n_chunks + lead;
+  const int len_ext = sp.len + (lead > 0 ? min(lead * CHUNK, p.lay.span(n + 1).len) : 0);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
-  const long long state_off = ((long long)n * p.Hv + hv) * D * D;
   bool ok = true;
   auto WAIT = [&](int idx, uint32_t parity) { return mbar_wait(&bars[idx], parity, abort_flag); };
+
+  // End gradient -> tensor memory, dS^T[v][k]; zero without one and for a lead-out.  The three
+  // read-out groups share the columns 2 : 1 : 1: one memory latency (see fwd_tc.cu).
+  if (warp >= 4) {
+    const int dht_row = p.dht_row ? p.dht_row[n] : n;
+    const bool edge = dht_row >= 0;
+    const float* src = lead > 0 ? nullptr : edge ? p.dht : p.seg_dht;
+    if (src) src += ((long long)(edge ? dht_row : n) * p.Hv + hv) * D * D;
+    const int v = (warp & 3) * 32 + lane;
+    auto load32 = [&](int k0, float (&x)[32]) {
+      if (!src) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = 0.f;
+      } else if (edge && p.v_first) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const float4 t = *reinterpret_cast<const float4*>(src + (long long)v * D + k0 + j);
+          x[j] = t.x;
+          x[j + 1] = t.y;
+          x[j + 2] = t.z;
+          x[j + 3] = t.w;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = src[(long long)(k0 + j) * D + v];
+      }
+    };
+    float x[32];
+    if (warp < 8) {
+      float y[32];
+      load32(0, x);
+      load32(32, y);
+      tmem_st32(tmem + lane_sel + TM_S, x);
+      tmem_st32(tmem + lane_sel + TM_S + 32, y);
+    } else {
+      load32(warp < 12 ? 64 : 96, x);
+      tmem_st32(tmem + lane_sel + TM_S + (warp < 12 ? 64 : 96), x);
+    }
+    tmem_st_wait();
+    tc_fence_before();
+    if (warp < 8) {
+      asm volatile("bar.sync 2, 384;" ::: "memory");  // the state group waits for the other two
+      tc_fence_after();
+    } else {
+      asm volatile("bar.arrive 2, 384;" ::: "memory");
+    }
+  }
 
   if (warp >= 4 && warp < 8) {
     // =============================== state group ===============================
     const int v = tid - 128;
-#pragma unroll 1
-    for (int k0 = 0; k0 < D; k0 += 32) {
-      float x[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        x[j] = (p.dht && lead == 0) ? p.dht[state_off + (long long)(k0 + j) * D + v] : 0.f;
-      tmem_st32(tmem + lane_sel + TM_S + k0, x);
-    }
-    tmem_st_wait();
     for (int it = 0; it < n_it && ok; ++it) {
       const int s = it & 1, c = n_it - 1 - it;
       if (it > 0) ok = WAIT(S_DONE, (it - 1) & 1);
@@ -222,15 +268,24 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       mbar_arrive(&bars[S_DEC]);
     }
     if (ok && n_it > 0) ok = WAIT(S_DONE, (n_it - 1) & 1);
-    if (ok && p.dh0) {
+    const int dh0_row = p.dh0_row ? p.dh0_row[n] : n;
+    if (ok && p.dh0 && dh0_row >= 0) {
+      float* dst = p.dh0 + ((long long)dh0_row * p.Hv + hv) * D * D;
       tc_fence_after();
 #pragma unroll 1
       for (int k0 = 0; k0 < D; k0 += 32) {
         float x[32];
         tmem_ld32(tmem + lane_sel + TM_S + k0, x);
         tmem_ld_wait();
+        if (p.v_first) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) p.dh0[state_off + (long long)(k0 + j) * D + v] = x[j];
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(dst + (long long)v * D + k0 + j) =
+                make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) dst[(long long)(k0 + j) * D + v] = x[j];
+        }
       }
     }
   } else if (warp >= 8 && warp < 12) {
@@ -603,39 +658,39 @@ int bwd_dh_tc_status(int* out, int reset) {
 // ---- host side --------------------------------------------------------------------------------
 int make_tile_map(CUtensorMap* m, const void* ptr, long long rows, long long cols, int box_rows);
 
-int launch_bwd_dh_tc(const void* q, const void* k, const void* A, const float* g, const void* beta,
-                     int beta_is_f32, const void* dO, const float* dht, void* dh, void* du,
-                     float* dh0, int tiled, const int* lead, const int* order, const int* run_mask,
-                     int run_value, int N, int Hq, int Hv,
-                     long long T_rows, float scale, SeqLayout lay, cudaStream_t st) {
+int launch_bwd_dh_tc(const fqla_bwd_dh_args& a, int N, SeqLayout lay, cudaStream_t st) {
   using namespace bdtc;
   CUtensorMap mq, mk, mdo, ma, mdh, mdu;
+  const long long T_rows = (long long)a.B * a.T;
   int rc;
-  if ((rc = make_tile_map(&mq, q, T_rows, (long long)Hq * D, 64))) return rc;
-  if ((rc = make_tile_map(&mk, k, T_rows, (long long)Hq * D, 64))) return rc;
-  if ((rc = make_tile_map(&mdo, dO, T_rows, (long long)Hv * D, 64))) return rc;
-  if ((rc = make_tile_map(&ma, A, T_rows, (long long)Hv * CHUNK, 64))) return rc;
+  if ((rc = make_tile_map(&mq, a.q, T_rows, (long long)a.Hq * D, 64))) return rc;
+  if ((rc = make_tile_map(&mk, a.k, T_rows, (long long)a.Hq * D, 64))) return rc;
+  if ((rc = make_tile_map(&mdo, a.dO, T_rows, (long long)a.Hv * D, 64))) return rc;
+  if ((rc = make_tile_map(&ma, a.A, T_rows, (long long)a.Hv * CHUNK, 64))) return rc;
   mdh = mq;
   mdu = mq;
-  if (tiled) {
+  if (a.operand_tiles) {
     // an upper bound of the chunk count: the maps only have to cover what the kernel stores
     const long long max_chunks = (T_rows + CHUNK - 1) / CHUNK + N;
-    if (dh && (rc = make_tile_map(&mdh, dh, max_chunks * Hv * D, D, 128))) return rc;
-    if (du && (rc = make_tile_map(&mdu, du, max_chunks * Hv * D, CHUNK, 128))) return rc;
+    if (a.dh && (rc = make_tile_map(&mdh, a.dh, max_chunks * a.Hv * D, D, 128))) return rc;
+    if (a.du && (rc = make_tile_map(&mdu, a.du, max_chunks * a.Hv * D, CHUNK, 128))) return rc;
   }
   BwdDhTcParams p;
-  p.tiled = tiled;
-  p.order = order;
-  p.lead = lead;
-  p.run_mask = run_mask;
-  p.run_value = run_value;
-  p.g = g; p.beta = beta; p.beta_is_f32 = beta_is_f32; p.dht = dht;
-  p.dh = (bf16*)dh; p.du = (bf16*)du; p.dh0 = dh0;
-  p.N = N; p.Hq = Hq; p.Hv = Hv; p.scale = scale; p.lay = lay;
-  rc = configure_smem((const void*)bwd_dh_tc_kernel, SMEM_BYTES);
+  p.tiled = a.operand_tiles;
+  p.order = a.seq_order;
+  p.lead = a.lead_chunks;
+  p.run_mask = a.run_mask;
+  p.run_value = a.run_value;
+  p.g = a.g_cum; p.beta = a.beta; p.beta_is_f32 = a.beta_is_f32;
+  p.dht = a.dht; p.seg_dht = a.seg_dht; p.dht_row = a.dht_row; p.dh0_row = a.dh0_row;
+  p.v_first = a.state_v_first;
+  p.dh = (bf16*)a.dh; p.du = (bf16*)a.du; p.dh0 = a.dh0;
+  p.N = N; p.Hq = a.Hq; p.Hv = a.Hv; p.scale = a.scale; p.lay = lay;
+  static std::atomic<unsigned long long> done;
+  rc = configure_smem((const void*)bwd_dh_tc_kernel, SMEM_BYTES, done);
   if (rc != 0) return rc;
-  bwd_dh_tc_kernel<<<(unsigned)(N * Hv), 512, SMEM_BYTES, st>>>(p, mq, mk, mdo, ma, mdh, mdu);
-  return (int)cudaGetLastError();
+  return launch_pdl(bwd_dh_tc_kernel, dim3((unsigned)(N * a.Hv)), dim3(512), (size_t)SMEM_BYTES, st, p, mq,
+                    mk, mdo, ma, mdh, mdu);
 }
 
 }  // namespace fqla

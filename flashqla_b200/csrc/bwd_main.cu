@@ -37,8 +37,9 @@ struct BwdMainParams {
   bf16* dq;   // [rows, Hv, D]
   bf16* dk;   // [rows, Hv, D]
   bf16* dv;   // [rows, Hv, D]
-  float* db;  // [rows, Hv]
+  void* db;   // [rows, Hv], fp32 or (db_bf16) bf16
   float* dg;  // [rows, Hv]
+  int dg_cumsum, db_bf16;  // see fqla_bwd_main_args
   int Hq, Hv;
   float scale;
   SeqLayout lay;
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(256, 1) bwd_main_kernel(const BwdMainParams p)
   float* sDb = sDg + CHUNK;
   float* sDgLast = sDb + CHUNK;
 
+  pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wm = warp & 3, wn = warp >> 2;
   const int hv = blockIdx.y, hq = hv / (p.Hv / p.Hq);
@@ -458,31 +460,62 @@ __global__ void __launch_bounds__(256, 1) bwd_main_kernel(const BwdMainParams p)
                   dk[0][nt][2 * hh + 1]);
     }
   __syncthreads();
-  if (tid < valid) {
-    float dgv = sDg[tid];
+  if (tid < CHUNK) {
+    float dgv = tid < valid ? sDg[tid] : 0.f;
     if (tid == valid - 1) dgv += *sDgLast;
-    p.dg[(row0 + tid) * p.Hv + hv] = dgv;
-    p.db[(row0 + tid) * p.Hv + hv] = sDb[tid];
+    if (p.dg_cumsum) dgv = suffix_sum64(dgv, tid, sG);  // sG is dead
+    if (tid < valid) {
+      const long long i = (row0 + tid) * p.Hv + hv;
+      p.dg[i] = dgv;
+      if (p.db_bf16) reinterpret_cast<bf16*>(p.db)[i] = __float2bfloat16(sDb[tid]);
+      else reinterpret_cast<float*>(p.db)[i] = sDb[tid];
+    }
   }
 }
 
 template <int D>
 static int launch_bwd_main(const BwdMainParams& p, long long n_chunks, cudaStream_t st) {
   using L = BwdMainSmem<D>;
-  int rc = configure_smem((const void*)bwd_main_kernel<D>, L::BYTES);
+  static std::atomic<unsigned long long> done;
+  int rc = configure_smem((const void*)bwd_main_kernel<D>, L::BYTES, done);
   if (rc != 0) return rc;
-  bwd_main_kernel<D><<<dim3((unsigned)n_chunks, p.Hv), 256, L::BYTES, st>>>(p);
-  return (int)cudaGetLastError();
+  return launch_pdl(bwd_main_kernel<D>, dim3((unsigned)n_chunks, p.Hv), dim3(256), L::BYTES, st, p);
 }
 
 // tcgen05 version for K = V = 128 (bwd_main_tc.cu)
-int launch_bwd_main_tc(const void* q, const void* k, const void* v, const void* vnew, const void* A,
-                       const float* g, const void* beta, int beta_is_f32, const void* dO,
-                       const void* du, const void* h, const void* dh, void* dq, void* dk, void* dv,
-                       float* db, float* dg, int tiled, int Hq, int Hv, long long T_rows, long long n_chunks,
-                       float scale, SeqLayout lay, IndexTable chunk_indices, cudaStream_t st);
+int launch_bwd_main_tc(const fqla_bwd_main_args& a, long long n_chunks, SeqLayout lay, IndexTable chunk_indices,
+                       cudaStream_t st);
 }  // namespace fqla
 using namespace fqla;
+
+extern "C" int fqla_bwd_main_run(const fqla_bwd_main_args* args, void* stream) {
+  if (!args) return FQLA_ERR_INVALID_ARG;
+  const fqla_bwd_main_args& a = *args;
+  if (!a.q || !a.k || !a.v || !a.vnew || !a.A || !a.g_cum || !a.beta || !a.dO || !a.du || !a.h || !a.dh ||
+      !a.dq || !a.dk || !a.dv || !a.db || !a.dg || a.Hq <= 0 || a.Hv % a.Hq)
+    return FQLA_ERR_INVALID_ARG;
+  if (a.cu_seqlens && (!a.chunk_offsets || !a.chunk_indices || a.B != 1)) return FQLA_ERR_INVALID_ARG;
+  const SeqLayout lay{{a.cu_seqlens, a.idx_is64}, {a.chunk_offsets, a.idx_is64}, a.T};
+  const IndexTable ci{a.chunk_indices, a.idx_is64};
+  const long long n = a.cu_seqlens ? a.num_chunks : (long long)a.B * ((a.T + CHUNK - 1) / CHUNK);
+  if (n <= 0) return FQLA_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  static const bool force_legacy = getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
+  if (a.D == 128 && !force_legacy) return launch_bwd_main_tc(a, n, lay, ci, st);
+  if (a.operand_tiles) return FQLA_ERR_UNSUPPORTED_DIM;  // only the tcgen05 kernel reads tiles
+  BwdMainParams p;
+  p.q = (const bf16*)a.q; p.k = (const bf16*)a.k; p.v = (const bf16*)a.v;
+  p.vnew = (const bf16*)a.vnew; p.A = (const bf16*)a.A; p.g = a.g_cum; p.beta = a.beta;
+  p.beta_is_f32 = a.beta_is_f32; p.dO = (const bf16*)a.dO; p.du = (const bf16*)a.du;
+  p.h = (const bf16*)a.h; p.dh = (const bf16*)a.dh; p.dq = (bf16*)a.dq; p.dk = (bf16*)a.dk;
+  p.dv = (bf16*)a.dv; p.db = a.db; p.dg = a.dg; p.dg_cumsum = a.dg_cumsum; p.db_bf16 = a.db_is_bf16;
+  p.Hq = a.Hq; p.Hv = a.Hv; p.scale = a.scale;
+  p.lay = lay;
+  p.chunk_indices = ci;
+  if (a.D == 128) return launch_bwd_main<128>(p, n, st);
+  if (a.D == 64) return launch_bwd_main<64>(p, n, st);
+  return FQLA_ERR_UNSUPPORTED_DIM;
+}
 
 extern "C" int fqla_bwd_main(const void* q, const void* k, const void* v, const void* vnew,
                              const void* A, const float* g_cum, const void* beta,
@@ -492,28 +525,11 @@ extern "C" int fqla_bwd_main(const void* q, const void* k, const void* v, const 
                              const void* cu_seqlens, const void* chunk_offsets,
                              const void* chunk_indices, int idx_is64, long long num_chunks,
                              int operand_tiles, void* stream) {
-  if (!q || !k || !v || !vnew || !A || !g_cum || !beta || !dO || !du || !h || !dh || !dq ||
-      !dk || !dv || !db || !dg || Hq <= 0 || Hv % Hq)
-    return FQLA_ERR_INVALID_ARG;
-  if (cu_seqlens && (!chunk_offsets || !chunk_indices || B != 1)) return FQLA_ERR_INVALID_ARG;
-  BwdMainParams p;
-  p.q = (const bf16*)q; p.k = (const bf16*)k; p.v = (const bf16*)v;
-  p.vnew = (const bf16*)vnew; p.A = (const bf16*)A; p.g = g_cum; p.beta = beta;
-  p.beta_is_f32 = beta_is_f32; p.dO = (const bf16*)dO; p.du = (const bf16*)du;
-  p.h = (const bf16*)h; p.dh = (const bf16*)dh; p.dq = (bf16*)dq; p.dk = (bf16*)dk;
-  p.dv = (bf16*)dv; p.db = db; p.dg = dg; p.Hq = Hq; p.Hv = Hv; p.scale = scale;
-  p.lay = SeqLayout{{cu_seqlens, idx_is64}, {chunk_offsets, idx_is64}, T};
-  p.chunk_indices = IndexTable{chunk_indices, idx_is64};
-  long long n = cu_seqlens ? num_chunks : (long long)B * ((T + CHUNK - 1) / CHUNK);
-  if (n <= 0) return FQLA_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  static const bool force_legacy = getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
-  if (D == 128 && !force_legacy)
-    return launch_bwd_main_tc(q, k, v, vnew, A, g_cum, beta, beta_is_f32, dO, du, h, dh, dq, dk, dv,
-                              db, dg, operand_tiles, Hq, Hv, (long long)B * T, n, scale, p.lay,
-                              p.chunk_indices, st);
-  if (operand_tiles) return FQLA_ERR_UNSUPPORTED_DIM;  // only the tcgen05 kernel reads tiles
-  if (D == 128) return launch_bwd_main<128>(p, n, st);
-  if (D == 64) return launch_bwd_main<64>(p, n, st);
-  return FQLA_ERR_UNSUPPORTED_DIM;
+  fqla_bwd_main_args a = {};
+  a.q = q; a.k = k; a.v = v; a.vnew = vnew; a.A = A; a.g_cum = g_cum; a.beta = beta;
+  a.beta_is_f32 = beta_is_f32; a.dO = dO; a.du = du; a.h = h; a.dh = dh; a.dq = dq; a.dk = dk;
+  a.dv = dv; a.db = db; a.dg = dg; a.B = B; a.T = T; a.Hq = Hq; a.Hv = Hv; a.D = D; a.scale = scale;
+  a.cu_seqlens = cu_seqlens; a.chunk_offsets = chunk_offsets; a.chunk_indices = chunk_indices;
+  a.idx_is64 = idx_is64; a.num_chunks = num_chunks; a.operand_tiles = operand_tiles;
+  return fqla_bwd_main_run(&a, stream);
 }

@@ -41,8 +41,9 @@ struct BwdMainTcParams {
   bf16* dq;
   bf16* dk;
   bf16* dv;
-  float* db;
+  void* db;                // fp32 or (db_bf16) bf16
   float* dg;
+  int dg_cumsum, db_bf16;  // see fqla_bwd_main_args
   int Hq, Hv;
   float scale;
   SeqLayout lay;
@@ -69,7 +70,7 @@ constexpr int OFF_DW = OFF_DA + 8192;       // -du h^T
 // columns: 4 lane quarters x 64), of db (rows 4 x 64, two column terms 4 x 64 each) and of the
 // chunk total (16)
 constexpr int OFF_VEC = OFF_DW + ROW_TILE;
-constexpr int OFF_BAR = OFF_VEC + (4 * 64 + 5 * 256 + 512 + 16) * 4;
+constexpr int OFF_BAR = OFF_VEC + (4 * 64 + 5 * 256 + 512 + 18) * 4;
 constexpr int N_BARS = 20;
 constexpr int OFF_MISC = OFF_BAR + N_BARS * 8;
 constexpr int SMEM_BYTES = OFF_MISC + 16 + 1024;
@@ -190,6 +191,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(tmem_slot, 512);
+  pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -480,8 +482,9 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
     // would otherwise idle until the first wide products are complete)
     auto combine = [&](long long first, int n_rows) {  // first = row0 * Hv + hv of the item
       const int r = tid - N_EPI / 2;
-      if (r >= 0 && r < n_rows) {
-        float dgv = 0.f, dbv = 0.f;
+      if (r < 0 || r >= CHUNK) return;  // two whole warps go on
+      float dgv = 0.f, dbv = 0.f;
+      if (r < n_rows) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           dgv += sRowW[j * 64 + r] - sColDg[j * 64 + r];
@@ -493,8 +496,13 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 #pragma unroll
           for (int j = 0; j < 8; ++j) dgv += sLast[j];
         }
-        p.dg[first + (long long)r * p.Hv] = dgv;
-        p.db[first + (long long)r * p.Hv] = dbv;
+      }
+      if (p.dg_cumsum) dgv = suffix_sum64(dgv, r, sLast + 16);
+      if (r < n_rows) {
+        const long long i = first + (long long)r * p.Hv;
+        p.dg[i] = dgv;
+        if (p.db_bf16) reinterpret_cast<bf16*>(p.db)[i] = __float2bfloat16(dbv);
+        else reinterpret_cast<float*>(p.db)[i] = dbv;
       }
     };
     Item cur = decode(blockIdx.x);
@@ -880,35 +888,36 @@ int make_tile_map(CUtensorMap* m, const void* ptr, long long rows, long long col
   return 0;
 }
 
-int launch_bwd_main_tc(const void* q, const void* k, const void* v, const void* vnew, const void* A,
-                       const float* g, const void* beta, int beta_is_f32, const void* dO,
-                       const void* du, const void* h, const void* dh, void* dq, void* dk, void* dv,
-                       float* db, float* dg, int tiled, int Hq, int Hv, long long T_rows, long long n_chunks,
-                       float scale, SeqLayout lay, IndexTable chunk_indices, cudaStream_t st) {
+int launch_bwd_main_tc(const fqla_bwd_main_args& a, long long n_chunks, SeqLayout lay,
+                       IndexTable chunk_indices, cudaStream_t st) {
   using namespace bmtc;
   CUtensorMap mq, mk, mv, mvn, mdo, mdu, mh, mdh, ma;
+  const long long T_rows = (long long)a.B * a.T;
+  const int Hq = a.Hq, Hv = a.Hv;
   int rc;
-  if ((rc = make_tile_map(&mq, q, T_rows, (long long)Hq * D, 64))) return rc;
-  if ((rc = make_tile_map(&mk, k, T_rows, (long long)Hq * D, 64))) return rc;
-  if ((rc = make_tile_map(&mv, v, T_rows, (long long)Hv * D, 64))) return rc;
-  if (tiled) {
-    if ((rc = make_tile_map(&mvn, vnew, n_chunks * Hv * D, CHUNK, 128))) return rc;
-    if ((rc = make_tile_map(&mdu, du, n_chunks * Hv * D, CHUNK, 128))) return rc;
+  if ((rc = make_tile_map(&mq, a.q, T_rows, (long long)Hq * D, 64))) return rc;
+  if ((rc = make_tile_map(&mk, a.k, T_rows, (long long)Hq * D, 64))) return rc;
+  if ((rc = make_tile_map(&mv, a.v, T_rows, (long long)Hv * D, 64))) return rc;
+  if (a.operand_tiles) {
+    if ((rc = make_tile_map(&mvn, a.vnew, n_chunks * Hv * D, CHUNK, 128))) return rc;
+    if ((rc = make_tile_map(&mdu, a.du, n_chunks * Hv * D, CHUNK, 128))) return rc;
   } else {
-    if ((rc = make_tile_map(&mvn, vnew, T_rows, (long long)Hv * D, 64))) return rc;
-    if ((rc = make_tile_map(&mdu, du, T_rows, (long long)Hv * D, 64))) return rc;
+    if ((rc = make_tile_map(&mvn, a.vnew, T_rows, (long long)Hv * D, 64))) return rc;
+    if ((rc = make_tile_map(&mdu, a.du, T_rows, (long long)Hv * D, 64))) return rc;
   }
-  if ((rc = make_tile_map(&mdo, dO, T_rows, (long long)Hv * D, 64))) return rc;
-  if ((rc = make_tile_map(&mh, h, n_chunks * Hv * D, D, 128))) return rc;
-  if ((rc = make_tile_map(&mdh, dh, n_chunks * Hv * D, D, 128))) return rc;
-  if ((rc = make_tile_map(&ma, A, T_rows, (long long)Hv * CHUNK, 64))) return rc;
+  if ((rc = make_tile_map(&mdo, a.dO, T_rows, (long long)Hv * D, 64))) return rc;
+  if ((rc = make_tile_map(&mh, a.h, n_chunks * Hv * D, D, 128))) return rc;
+  if ((rc = make_tile_map(&mdh, a.dh, n_chunks * Hv * D, D, 128))) return rc;
+  if ((rc = make_tile_map(&ma, a.A, T_rows, (long long)Hv * CHUNK, 64))) return rc;
   BwdMainTcParams p;
-  p.g = g; p.beta = beta; p.beta_is_f32 = beta_is_f32;
-  p.dq = (bf16*)dq; p.dk = (bf16*)dk; p.dv = (bf16*)dv; p.db = db; p.dg = dg;
-  p.Hq = Hq; p.Hv = Hv; p.scale = scale; p.lay = lay; p.chunk_indices = chunk_indices;
+  p.g = a.g_cum; p.beta = a.beta; p.beta_is_f32 = a.beta_is_f32;
+  p.dq = (bf16*)a.dq; p.dk = (bf16*)a.dk; p.dv = (bf16*)a.dv; p.db = a.db; p.dg = a.dg;
+  p.dg_cumsum = a.dg_cumsum; p.db_bf16 = a.db_is_bf16;
+  p.Hq = Hq; p.Hv = Hv; p.scale = a.scale; p.lay = lay; p.chunk_indices = chunk_indices;
   p.n_chunks = n_chunks;
-  rc = configure_smem(tiled ? (const void*)bwd_main_tc_kernel<true> : (const void*)bwd_main_tc_kernel<false>,
-                      SMEM_BYTES);
+  static std::atomic<unsigned long long> done[2];
+  rc = configure_smem(a.operand_tiles ? (const void*)bwd_main_tc_kernel<true> : (const void*)bwd_main_tc_kernel<false>,
+                      SMEM_BYTES, done[a.operand_tiles ? 1 : 0]);
   if (rc != 0) return rc;
   int dev = 0, n_sm = 0;  // per launch: the current device may differ from call to call
   cudaGetDevice(&dev);
@@ -916,11 +925,8 @@ int launch_bwd_main_tc(const void* q, const void* k, const void* v, const void* 
   if (n_sm <= 0) n_sm = 148;
   const long long total = n_chunks * Hv;
   const unsigned grid = (unsigned)(total < n_sm ? total : n_sm);
-  if (tiled)
-    bwd_main_tc_kernel<true><<<grid, NT, SMEM_BYTES, st>>>(p, mq, mk, mv, mvn, mdo, mdu, mh, mdh, ma);
-  else
-    bwd_main_tc_kernel<false><<<grid, NT, SMEM_BYTES, st>>>(p, mq, mk, mv, mvn, mdo, mdu, mh, mdh, ma);
-  return (int)cudaGetLastError();
+  return launch_pdl(a.operand_tiles ? bwd_main_tc_kernel<true> : bwd_main_tc_kernel<false>, dim3(grid), dim3(NT),
+                    (size_t)SMEM_BYTES, st, p, mq, mk, mv, mvn, mdo, mdu, mh, mdh, ma);
 }
 
 }  // namespace fqla

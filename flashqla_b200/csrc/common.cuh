@@ -58,6 +58,14 @@ struct SeqLayout {
   }
 };
 
+// ---- programmatic dependent launch (see launch_pdl) -------------------------------------------
+// Block until every kernel this one depends on has completed and its writes are visible.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// No kernel signals its dependents early (griddepcontrol.launch_dependents): they start as the
+// blocks of the kernel before exit.  Signalled at block start they took SMs the kernel's own tail
+// and the kernel behind it needed: 335 instead of 311 us for the 4 x 8192 forward, 617 instead of
+// 593 us for 64 packed prompts (320 and 595 without dependent launches).
+
 // ---- small PTX wrappers ---------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -186,6 +194,19 @@ __device__ __forceinline__ void load_tile_async(bf16* s, const bf16* g, long lon
     const bf16* src = g + (long long)(ok ? r : 0) * g_stride + c;
     cp_async16(s + r * LDS + c, src, ok);
   }
+}
+
+// Suffix sum over the 64 rows of a chunk, one row per thread of two whole warps (row = 0..63); both
+// warps must call it, `slot` is one float of shared memory that nobody else touches meanwhile.
+__device__ __forceinline__ float suffix_sum64(float x, int row, float* slot) {
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const float y = __shfl_down_sync(0xffffffffu, x, d);
+    if ((row & 31) + d < 32) x += y;
+  }
+  if (row == 32) *slot = x;
+  asm volatile("bar.sync 3, 64;" ::: "memory");
+  return row < 32 ? x + *slot : x;
 }
 
 __device__ __forceinline__ float load_beta(const void* beta, int beta_is_f32, long long idx) {

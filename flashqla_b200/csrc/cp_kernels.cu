@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(128)
 warmup_scan_kernel(const float* __restrict__ g_cum, int Hv, SeqLayout lay, int n_seg,
                    float threshold, int from_start, const int* __restrict__ keep,
                    int* __restrict__ warm, int* __restrict__ fallback) {
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int item = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (item >= n_seg * Hv) return;
@@ -86,6 +87,7 @@ segment_scan_kernel(const float* __restrict__ g_cum, int Hv, SeqLayout lay,
                     const int* __restrict__ seg_begin, float threshold, int from_start,
                     int* __restrict__ warm, int* __restrict__ fallback, int* __restrict__ lead,
                     int* __restrict__ exact_warm, int* __restrict__ any_fb) {
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = blockIdx.x / Hv, hv = blockIdx.x % Hv;
   const int s0 = seg_begin[r], s1 = seg_begin[r + 1];
@@ -134,6 +136,7 @@ __global__ void __launch_bounds__(D) merge_kernel(const float* __restrict__ loca
   // one staging buffer: the local state of the step, then D x BK panels of M, forward [a][j]
   // (row stride BK+1), reverse [j][a]
   __shared__ float panel[D * (BK + 1)];
+  pdl_wait();
   const int a = threadIdx.x, lane = a & 31, warp = a >> 5;
   const int v0 = blockIdx.x * BV, hv = blockIdx.y, r = blockIdx.z;
   const int s0 = seg_begin[r], s1 = seg_begin[r + 1];  // segments [s0, s1)
@@ -226,9 +229,8 @@ extern "C" int fqla_warmup_scan(const float* g_cum, int T, int Hv, const void* s
   if (n_seg <= 0) return FQLA_OK;
   SeqLayout lay{{seg_cu_seqlens, idx_is64}, {seg_cu_seqlens, idx_is64}, T};
   const long long items = (long long)n_seg * Hv;
-  warmup_scan_kernel<<<(unsigned)((items + 3) / 4), 128, 0, (cudaStream_t)stream>>>(
+  return launch_pdl(warmup_scan_kernel, dim3((unsigned)((items + 3) / 4)), dim3(128), 0, (cudaStream_t)stream,
       g_cum, Hv, lay, n_seg, threshold, from_start, keep, warm, fallback);
-  return (int)cudaGetLastError();
 }
 
 extern "C" int fqla_segment_scan(const float* g_cum, int T, int Hv, const void* seg_cu_seqlens,
@@ -240,9 +242,8 @@ extern "C" int fqla_segment_scan(const float* g_cum, int T, int Hv, const void* 
     return FQLA_ERR_INVALID_ARG;
   if (n_raw <= 0) return FQLA_OK;
   SeqLayout lay{{seg_cu_seqlens, idx_is64}, {seg_cu_seqlens, idx_is64}, T};
-  segment_scan_kernel<<<(unsigned)(n_raw * Hv), 256, 0, (cudaStream_t)stream>>>(
+  return launch_pdl(segment_scan_kernel, dim3((unsigned)(n_raw * Hv)), dim3(256), 0, (cudaStream_t)stream,
       g_cum, Hv, lay, seg_begin, threshold, from_start, warm, fallback, lead, exact_warm, any_fb);
-  return (int)cudaGetLastError();
 }
 
 extern "C" int fqla_merge_states(const float* local, const float* M, const int* use_m,
@@ -253,15 +254,13 @@ extern "C" int fqla_merge_states(const float* local, const float* M, const int* 
   if (n_raw <= 0) return FQLA_OK;
   cudaStream_t st = (cudaStream_t)stream;
   if (D == 128) {
-    merge_kernel<128><<<dim3(128 / 32, Hv, n_raw), 128, 0, st>>>(
+    return launch_pdl(merge_kernel<128>, dim3(128 / 32, Hv, n_raw), dim3(128), 0, st,
         local, M, use_m, raw, seg_begin, any_fb, out, Hv, reverse,
         seg_stride ? seg_stride : (long long)Hv * D * D, seg_stride ? seg_stride : Hv);
   } else if (D == 64) {
-    merge_kernel<64><<<dim3(64 / 32, Hv, n_raw), 64, 0, st>>>(
+    return launch_pdl(merge_kernel<64>, dim3(64 / 32, Hv, n_raw), dim3(64), 0, st,
         local, M, use_m, raw, seg_begin, any_fb, out, Hv, reverse,
         seg_stride ? seg_stride : (long long)Hv * D * D, seg_stride ? seg_stride : Hv);
-  } else {
-    return FQLA_ERR_UNSUPPORTED_DIM;
   }
-  return (int)cudaGetLastError();
+  return FQLA_ERR_UNSUPPORTED_DIM;
 }

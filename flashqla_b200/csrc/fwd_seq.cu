@@ -24,11 +24,7 @@
 namespace fqla {
 
 // tcgen05 implementation of the full forward (fwd_tc.cu)
-int launch_fwd_tc(const void* q, const void* k, const void* v, const void* A, const float* g,
-                  const void* beta, int beta_is_f32, const float* h0, float* ht, void* o, void* h,
-                  void* vnew, int tiled, const int* lead, const int* order, const int* run_mask,
-                  int run_value, int N, int Hq, int Hv, long long T_rows, float scale,
-                  SeqLayout lay, cudaStream_t st);
+int launch_fwd_tc(const fqla_fwd_args& a, int N, SeqLayout lay, cudaStream_t st);
 
 struct FwdSeqParams {
   const bf16* q;      // may be null (state-only pass)
@@ -38,8 +34,11 @@ struct FwdSeqParams {
   const float* g;     // chunk-local cumsum
   const void* beta;
   int beta_is_f32;
-  const float* h0;    // [N, Hv, D, D] or null
-  float* ht;          // [N, Hv, D, D] or null
+  const float* h0;    // [*, Hv, D, D] or null; seg_h0, h0_row, ht_row, v_first: see fqla_fwd_args
+  const float* seg_h0;
+  const int *h0_row, *ht_row;
+  int v_first;
+  float* ht;          // [*, Hv, D, D] or null
   bf16* o;            // [rows, Hv, D] or null
   bf16* h;            // [chunks, Hv, D, D] or null
   bf16* vnew;         // [rows, Hv, D] or null
@@ -100,6 +99,7 @@ __global__ void __launch_bounds__(256, 1) fwd_seq_kernel(const FwdSeqParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wm = warp & 3, wn = warp >> 2;
   const int hv = blockIdx.x % p.Hv;
+  pdl_wait();
   const int n = p.order ? p.order[blockIdx.x / p.Hv] : (int)(blockIdx.x / p.Hv);
   const int hq = hv / (p.Hv / p.Hq);
   constexpr int V_SLICES = D / BV;
@@ -120,7 +120,11 @@ __global__ void __launch_bounds__(256, 1) fwd_seq_kernel(const FwdSeqParams p) {
 
   // ---- state in registers: rows 32*wm + mt*16 + ..., cols (BV/2)*wn + nt*8 + ...
   float S[MTS][NTV][4];
-  const long long state_off = ((long long)n * p.Hv + hv) * D * D;
+  const int h0_row = p.h0_row ? p.h0_row[n] : n;
+  const bool edge = h0_row >= 0;  // starts its sequence; else it is handed a state, if any
+  const float* h0 = c_begin != 0 ? nullptr : edge ? p.h0 : p.seg_h0;
+  if (h0) h0 += ((long long)(edge ? h0_row : n) * p.Hv + hv) * D * D;
+  const bool h0_v_first = edge && p.v_first;
 #pragma unroll
   for (int mt = 0; mt < MTS; ++mt)
 #pragma unroll
@@ -131,7 +135,7 @@ __global__ void __launch_bounds__(256, 1) fwd_seq_kernel(const FwdSeqParams p) {
         int c = v0 + (BV / 2) * wn + nt * 8 + (lane & 3) * 2 + (e & 1);
         float x = 0.f;
         if (m_slice) x = (r == c) ? 1.f : 0.f;
-        else if (p.h0 && c_begin == 0) x = p.h0[state_off + (long long)r * D + c];
+        else if (h0) x = h0[h0_v_first ? (long long)c * D + r : (long long)r * D + c];
         S[mt][nt][e] = x;
       }
   auto store_state_copy = [&]() {
@@ -310,8 +314,11 @@ __global__ void __launch_bounds__(256, 1) fwd_seq_kernel(const FwdSeqParams p) {
   }
 
   // ---- final state / transition matrix out (fp32)
+  const int ht_row = m_slice || !p.ht_row ? n : p.ht_row[n];
   float* dst = m_slice ? p.M : p.ht;
-  if (dst) {
+  if (dst && ht_row >= 0) {
+    dst += ((long long)ht_row * p.Hv + hv) * D * D;
+    const bool v_first = !m_slice && p.v_first;
 #pragma unroll
     for (int mt = 0; mt < MTS; ++mt)
 #pragma unroll
@@ -320,8 +327,13 @@ __global__ void __launch_bounds__(256, 1) fwd_seq_kernel(const FwdSeqParams p) {
         for (int hh = 0; hh < 2; ++hh) {
           int r = (16 * MTS) * wm + mt * 16 + (lane >> 2) + hh * 8;
           int c = v0 + (BV / 2) * wn + nt * 8 + (lane & 3) * 2;
-          *reinterpret_cast<float2*>(dst + state_off + (long long)r * D + c) =
-              make_float2(S[mt][nt][2 * hh], S[mt][nt][2 * hh + 1]);
+          if (v_first) {
+            dst[(long long)c * D + r] = S[mt][nt][2 * hh];
+            dst[(long long)(c + 1) * D + r] = S[mt][nt][2 * hh + 1];
+          } else {
+            *reinterpret_cast<float2*>(dst + (long long)r * D + c) =
+                make_float2(S[mt][nt][2 * hh], S[mt][nt][2 * hh + 1]);
+          }
         }
   }
   // rows of o past the last sequence's end come out zero
@@ -340,16 +352,54 @@ template <int D>
 static int launch_fwd_seq(const FwdSeqParams& p, cudaStream_t st) {
   constexpr int BV = 64;
   using L = FwdSeqSmem<D, BV>;
-  int rc = configure_smem((const void*)fwd_seq_kernel<D, BV>, L::BYTES);
+  static std::atomic<unsigned long long> done;
+  int rc = configure_smem((const void*)fwd_seq_kernel<D, BV>, L::BYTES, done);
   if (rc != 0) return rc;
   dim3 grid((unsigned)(p.N * p.Hv), (D / BV) * (p.M ? 2 : 1));
-  fwd_seq_kernel<D, BV><<<grid, 256, L::BYTES, st>>>(p);
-  return (int)cudaGetLastError();
+  return launch_pdl(fwd_seq_kernel<D, BV>, grid, dim3(256), L::BYTES, st, p);
 }
 
 }  // namespace fqla
 
 using namespace fqla;
+
+extern "C" int fqla_fwd_run(const fqla_fwd_args* args, void* stream) {
+  if (!args) return FQLA_ERR_INVALID_ARG;
+  const fqla_fwd_args& a = *args;
+  if (!a.k || !a.v || !a.A || !a.g_cum || !a.beta || a.Hq <= 0 || a.Hv % a.Hq) return FQLA_ERR_INVALID_ARG;
+  if (a.cu_seqlens && (!a.chunk_offsets || a.B != 1)) return FQLA_ERR_INVALID_ARG;
+  if (a.o && !a.q) return FQLA_ERR_INVALID_ARG;
+  if (a.warm_chunks && (a.q || a.h || a.vnew)) return FQLA_ERR_INVALID_ARG;
+  if (a.lead_chunks && (a.warm_chunks || a.M || a.m_mask)) return FQLA_ERR_INVALID_ARG;
+  const int N = a.cu_seqlens ? a.N : a.B;
+  if (N <= 0) return FQLA_OK;
+  const SeqLayout lay{{a.cu_seqlens, a.idx_is64}, {a.chunk_offsets, a.idx_is64}, a.T};
+  cudaStream_t st = (cudaStream_t)stream;
+  // The full forward (q and o present, K = V = 128) and the recomputation of the per-chunk
+  // states and v_new for the backward pass (neither q nor o) run on the tcgen05 kernel;
+  // state-only passes, transition matrices and D = 64 run on the mma.sync kernel in this file.
+  static const bool force_legacy = getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
+  const bool full = a.q && a.o, recompute = !a.q && !a.o && (a.h || a.vnew);
+  if (a.D == 128 && (full || recompute) && !a.M && !a.warm_chunks && !a.m_mask && !force_legacy)
+    return launch_fwd_tc(a, N, lay, st);
+  // tcgen05 kernel only
+  if (a.operand_tiles || a.lead_chunks || a.o_is_f16) return FQLA_ERR_UNSUPPORTED_DIM;
+  FwdSeqParams p;
+  p.q = (const bf16*)a.q; p.k = (const bf16*)a.k; p.v = (const bf16*)a.v; p.A = (const bf16*)a.A;
+  p.g = a.g_cum; p.beta = a.beta; p.beta_is_f32 = a.beta_is_f32;
+  p.h0 = a.h0; p.seg_h0 = a.seg_h0; p.h0_row = a.h0_row; p.ht_row = a.ht_row;
+  p.v_first = a.state_v_first; p.ht = a.ht;
+  p.o = (bf16*)a.o; p.h = (bf16*)a.h; p.vnew = (bf16*)a.vnew; p.M = a.M;
+  p.warm = a.warm_chunks; p.m_mask = a.m_mask; p.order = a.seq_order; p.run_mask = a.run_mask;
+  p.run_value = a.run_value;
+  p.N = N; p.Hq = a.Hq; p.Hv = a.Hv;
+  p.T_rows = (long long)a.B * a.T;
+  p.scale = a.scale;
+  p.lay = lay;
+  if (a.D == 128) return launch_fwd_seq<128>(p, st);
+  if (a.D == 64) return launch_fwd_seq<64>(p, st);
+  return FQLA_ERR_UNSUPPORTED_DIM;
+}
 
 extern "C" int fqla_fwd_seq(const void* q, const void* k, const void* v, const void* A,
                             const float* g_cum, const void* beta, int beta_is_f32,
@@ -359,37 +409,12 @@ extern "C" int fqla_fwd_seq(const void* q, const void* k, const void* v, const v
                             int Hq, int Hv, int D, float scale, const void* cu_seqlens,
                             const void* chunk_offsets, int idx_is64, int N, int operand_tiles,
                             void* stream) {
-  if (!k || !v || !A || !g_cum || !beta || Hq <= 0 || Hv % Hq) return FQLA_ERR_INVALID_ARG;
-  if (cu_seqlens && (!chunk_offsets || B != 1)) return FQLA_ERR_INVALID_ARG;
-  if (o && !q) return FQLA_ERR_INVALID_ARG;
-  if (warm_chunks && (q || h || vnew)) return FQLA_ERR_INVALID_ARG;
-  if (lead_chunks && (warm_chunks || M || m_mask)) return FQLA_ERR_INVALID_ARG;
-  FwdSeqParams p;
-  p.q = (const bf16*)q; p.k = (const bf16*)k; p.v = (const bf16*)v; p.A = (const bf16*)A;
-  p.g = g_cum; p.beta = beta; p.beta_is_f32 = beta_is_f32;
-  p.h0 = h0; p.ht = ht; p.o = (bf16*)o; p.h = (bf16*)h; p.vnew = (bf16*)vnew; p.M = M;
-  p.warm = warm_chunks;
-  p.m_mask = m_mask;
-  p.order = seq_order;
-  p.run_mask = run_mask;
-  p.run_value = run_value;
-  p.N = cu_seqlens ? N : B; p.Hq = Hq; p.Hv = Hv;
-  p.T_rows = (long long)B * T;
-  p.scale = scale;
-  p.lay = SeqLayout{{cu_seqlens, idx_is64}, {chunk_offsets, idx_is64}, T};
-  if (p.N <= 0) return FQLA_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  // The full forward (q and o present, K = V = 128) and the recomputation of the per-chunk
-  // states and v_new for the backward pass (neither q nor o) run on the tcgen05 kernel;
-  // state-only passes, transition matrices and D = 64 run on the mma.sync kernel in this file.
-  static const bool force_legacy = getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
-  const bool full = q && o, recompute = !q && !o && (h || vnew);
-  if (D == 128 && (full || recompute) && !M && !warm_chunks && !m_mask && !force_legacy)
-    return launch_fwd_tc(q, k, v, A, g_cum, beta, beta_is_f32, h0, ht, o, h, vnew, operand_tiles,
-                         lead_chunks, seq_order, run_mask, run_value, p.N, Hq, Hv, p.T_rows, scale,
-                         p.lay, st);
-  if (operand_tiles || lead_chunks) return FQLA_ERR_UNSUPPORTED_DIM;  // tcgen05 kernel only
-  if (D == 128) return launch_fwd_seq<128>(p, st);
-  if (D == 64) return launch_fwd_seq<64>(p, st);
-  return FQLA_ERR_UNSUPPORTED_DIM;
+  fqla_fwd_args a = {};
+  a.q = q; a.k = k; a.v = v; a.A = A; a.g_cum = g_cum; a.beta = beta; a.beta_is_f32 = beta_is_f32;
+  a.h0 = h0; a.ht = ht; a.o = o; a.h = h; a.vnew = vnew; a.M = M; a.warm_chunks = warm_chunks;
+  a.m_mask = m_mask; a.lead_chunks = lead_chunks; a.seq_order = seq_order; a.run_mask = run_mask;
+  a.run_value = run_value; a.B = B; a.T = T; a.Hq = Hq; a.Hv = Hv; a.D = D; a.scale = scale;
+  a.cu_seqlens = cu_seqlens; a.chunk_offsets = chunk_offsets; a.idx_is64 = idx_is64; a.N = N;
+  a.operand_tiles = operand_tiles;
+  return fqla_fwd_run(&a, stream);
 }

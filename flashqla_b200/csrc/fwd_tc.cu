@@ -38,6 +38,7 @@
 //     64-127  prep    : one thread per chunk row: A' and A'' tiles
 // Synchronisation is by mbarriers only; every wait is bounded and reports through a status word.
 #include <cuda.h>
+#include <cuda_fp16.h>
 
 #include <cstdlib>
 
@@ -81,6 +82,9 @@ struct FwdTcParams {
   const void* beta;
   int beta_is_f32;
   const float* h0;
+  const float* seg_h0;            // see fqla_fwd_args in include/fqla.h for these five
+  const int *h0_row, *ht_row;
+  int v_first;
   float* ht;
   bf16* o;
   bf16* h;
@@ -155,11 +159,21 @@ __device__ __forceinline__ uint32_t scale_bf16x2(uint32_t packed, float lo, floa
   return pack_bf16(f.x * lo, f.y * hi);
 }
 
+template <bool F16>
+__device__ __forceinline__ uint32_t pack_out(float lo, float hi) {
+  if constexpr (F16) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  } else {
+    return pack_bf16(lo, hi);
+  }
+}
+
 // EXTRA: per-chunk state and v_new outputs (compiled out of the common instantiation: the six
 // roles run six different code regions at once, and the kernel is sensitive to its
 // instruction-cache footprint).  NO_O: state-only walk (recomputation for the backward pass): no q,
-// no output products, the output warps stay idle.
-template <bool EXTRA, bool NO_O>
+// no output products, the output warps stay idle.  O_F16: o leaves as fp16 instead of bf16.
+template <bool EXTRA, bool NO_O, bool O_F16>
 __global__ void __launch_bounds__(512, 1)
 fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
               const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -176,13 +190,12 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int hv = blockIdx.x % p.Hv;
-  const int n = p.order ? p.order[blockIdx.x / p.Hv] : (int)(blockIdx.x / p.Hv);
+  auto sequence = [&] { return p.order ? p.order[blockIdx.x / p.Hv] : (int)(blockIdx.x / p.Hv); };
   const int hq = hv / (p.Hv / p.Hq);
-  if (p.run_mask && p.run_mask[n * p.Hv + hv] != p.run_value) return;  // uniform per CTA
-  const SeqSpan sp = p.lay.span(n);
-  // iteration j handles chunk c = j - lead of the sequence; c < 0 are the lead-in chunks
-  const int lead = p.lead ? p.lead[n * p.Hv + hv] : 0;
-  const int n_it = sp.n_chunks == 0 ? 0 : sp.n_chunks + lead;
+  if (p.run_mask) {
+    pdl_wait();
+    if (p.run_mask[sequence() * p.Hv + hv] != p.run_value) return;  // uniform per CTA
+  }
   const bool tile_h = EXTRA && p.tiled && p.h, tile_vn = EXTRA && p.tiled && p.vnew;
 
   if (tid == 0) FQLA_CHUNK_CLOCK(126);
@@ -228,15 +241,69 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     *reinterpret_cast<uint4*>(smem + OFF_P + i * 16) = make_uint4(0, 0, 0, 0);
   fence_proxy_async();
   if (warp == 0) tmem_alloc(tmem_slot, 512);
+  // everything above overlaps the tail of the kernel before: no global memory up to here
+  pdl_wait();
+  const int n = sequence();
+  const SeqSpan sp = p.lay.span(n);
+  // iteration j handles chunk c = j - lead of the sequence; c < 0 are the lead-in chunks
+  const int lead = p.lead ? p.lead[n * p.Hv + hv] : 0;
+  const int n_it = sp.n_chunks == 0 ? 0 : sp.n_chunks + lead;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;  // this warp's lane quarter
-  const long long state_off = ((long long)n * p.Hv + hv) * D * D;
   bool ok = true;
   auto WAIT = [&](int idx, uint32_t parity) { return mbar_wait(&bars[idx], parity, abort_flag); };
 
+  // Initial state -> tensor memory, S^T[v][k]; zero without one and for a lead-in.  The three
+  // read-out groups share the columns 2 : 1 : 1, each thread with its whole part in flight at once:
+  // one memory latency (four in turn, 3 us of an 11 us launch over two chunks, when the state group
+  // loaded 32 columns at a time by itself).
+  if (warp >= 4) {
+    const int h0_row = p.h0_row ? p.h0_row[n] : n;
+    const bool edge = h0_row >= 0;  // starts its sequence; else it is handed a state, if any
+    const float* src = lead > 0 ? nullptr : edge ? p.h0 : p.seg_h0;
+    if (src) src += ((long long)(edge ? h0_row : n) * p.Hv + hv) * D * D;
+    const int v = (warp & 3) * 32 + lane;
+    auto load32 = [&](int k0, float (&x)[32]) {
+      if (!src) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = 0.f;
+      } else if (edge && p.v_first) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const float4 t = *reinterpret_cast<const float4*>(src + (long long)v * D + k0 + j);
+          x[j] = t.x;
+          x[j + 1] = t.y;
+          x[j + 2] = t.z;
+          x[j + 3] = t.w;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = src[(long long)(k0 + j) * D + v];
+      }
+    };
+    float x[32];
+    if (warp < 8) {
+      float y[32];
+      load32(0, x);
+      load32(32, y);
+      tmem_st32(tmem + lane_sel + TM_S, x);
+      tmem_st32(tmem + lane_sel + TM_S + 32, y);
+    } else {
+      load32(warp < 12 ? 64 : 96, x);
+      tmem_st32(tmem + lane_sel + TM_S + (warp < 12 ? 64 : 96), x);
+    }
+    tmem_st_wait();
+    tc_fence_before();
+    if (warp < 8) {
+      asm volatile("bar.sync 2, 384;" ::: "memory");  // the state group waits for the other two
+      tc_fence_after();
+    } else {
+      asm volatile("bar.arrive 2, 384;" ::: "memory");
+    }
+  }
 
   // Role of each warp.  The MMA issuer is warp 0 and the producer warp 1 on purpose: among the
   // warps of one scheduler the oldest (lowest id) wins when several are ready, and these two
@@ -244,16 +311,6 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   if (warp >= 4 && warp < 8) {
     // =============================== S group ===============================
     const int v = tid - 128;  // lane of tensor memory = value index
-    // initial state -> tensor memory (S^T[v][k] = h0[k][v]); a lead-in starts from zero
-#pragma unroll 1
-    for (int k0 = 0; k0 < D; k0 += 32) {
-      float x[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        x[j] = (p.h0 && lead == 0) ? p.h0[state_off + (long long)(k0 + j) * D + v] : 0.f;
-      tmem_st32(tmem + lane_sel + TM_S + k0, x);
-    }
-    tmem_st_wait();
     for (int it = 0; it < n_it && ok; ++it) {
       const int s = it & 1;
       if (v == 0) FQLA_TRACE(0, 0);
@@ -340,15 +397,24 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       if (v == 0) FQLA_TRACE(0, 4);
     }
     if (ok && n_it > 0) ok = WAIT(S_DONE, (n_it - 1) & 1);
-    if (ok && p.ht) {
+    const int ht_row = p.ht_row ? p.ht_row[n] : n;
+    if (ok && p.ht && ht_row >= 0) {
+      float* dst = p.ht + ((long long)ht_row * p.Hv + hv) * D * D;
       tc_fence_after();
 #pragma unroll 1
       for (int k0 = 0; k0 < D; k0 += 32) {
         float x[32];
         tmem_ld32(tmem + lane_sel + TM_S + k0, x);
         tmem_ld_wait();
+        if (p.v_first) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) p.ht[state_off + (long long)(k0 + j) * D + v] = x[j];
+          for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(dst + (long long)v * D + k0 + j) =
+                make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) dst[(long long)(k0 + j) * D + v] = x[j];
+        }
       }
     }
   } else if (warp >= 8 && warp < 12) {
@@ -501,8 +567,8 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
             const float2 s2 = sgv[i + z];
             const float* aa = a + 4 * (i + z);
             const float* bb = b + 4 * (i + z);
-            w[2 * z] = pack_bf16(s2.x * aa[0] + bb[0], s2.y * aa[1] + bb[1]);
-            w[2 * z + 1] = pack_bf16(s2.x * aa[2] + bb[2], s2.y * aa[3] + bb[3]);
+            w[2 * z] = pack_out<O_F16>(s2.x * aa[0] + bb[0], s2.y * aa[1] + bb[1]);
+            w[2 * z + 1] = pack_out<O_F16>(s2.x * aa[2] + bb[2], s2.y * aa[3] + bb[3]);
           }
           stmatrix_x4_trans(base + (uint32_t)(i * 1024), w[0], w[1], w[2], w[3]);
         }
@@ -885,49 +951,49 @@ static int make_map(CUtensorMap* m, const void* ptr, long long rows, long long c
   return make_tile_map(m, ptr, rows, cols, 64);
 }
 
-int launch_fwd_tc(const void* q, const void* k, const void* v, const void* A, const float* g,
-                  const void* beta, int beta_is_f32, const float* h0, float* ht, void* o, void* h,
-                  void* vnew, int tiled, const int* lead, const int* order, const int* run_mask,
-                  int run_value, int N, int Hq, int Hv, long long T_rows, float scale,
-                  SeqLayout lay, cudaStream_t st) {
+int launch_fwd_tc(const fqla_fwd_args& a, int N, SeqLayout lay, cudaStream_t st) {
   using namespace fwdtc;
   CUtensorMap mq, mk, mv, ma, mh, mvn, mo;
+  const long long T_rows = (long long)a.B * a.T;
   int rc;
   // without q (recomputation of h and v_new for the backward pass) the state-only variant runs;
   // its q map is never used and only has to be a valid map
-  if ((rc = make_map(&mq, q ? q : k, T_rows, (long long)Hq * D))) return rc;
-  if ((rc = make_map(&mk, k, T_rows, (long long)Hq * D))) return rc;
-  if ((rc = make_map(&mv, v, T_rows, (long long)Hv * D))) return rc;
-  if ((rc = make_map(&ma, A, T_rows, (long long)Hv * CHUNK))) return rc;
+  if ((rc = make_map(&mq, a.q ? a.q : a.k, T_rows, (long long)a.Hq * D))) return rc;
+  if ((rc = make_map(&mk, a.k, T_rows, (long long)a.Hq * D))) return rc;
+  if ((rc = make_map(&mv, a.v, T_rows, (long long)a.Hv * D))) return rc;
+  if ((rc = make_map(&ma, a.A, T_rows, (long long)a.Hv * CHUNK))) return rc;
   mh = mq;
   mvn = mq;
   mo = mq;
-  if (o && (rc = make_map(&mo, o, T_rows, (long long)Hv * D))) return rc;
-  if (tiled) {
+  if (a.o && (rc = make_map(&mo, a.o, T_rows, (long long)a.Hv * D))) return rc;
+  if (a.operand_tiles) {
     // an upper bound of the chunk count: the maps only have to cover what the kernel stores
     const long long max_chunks = (T_rows + CHUNK - 1) / CHUNK + N;
-    if (h && (rc = make_tile_map(&mh, h, max_chunks * Hv * D, D, 128))) return rc;
-    if (vnew && (rc = make_tile_map(&mvn, vnew, max_chunks * Hv * D, CHUNK, 128))) return rc;
+    if (a.h && (rc = make_tile_map(&mh, a.h, max_chunks * a.Hv * D, D, 128))) return rc;
+    if (a.vnew && (rc = make_tile_map(&mvn, a.vnew, max_chunks * a.Hv * D, CHUNK, 128))) return rc;
   }
   FwdTcParams p;
-  p.tiled = tiled;
-  p.lead = lead;
-  p.order = order;
-  p.run_mask = run_mask;
-  p.run_value = run_value;
-  p.g = g; p.beta = beta; p.beta_is_f32 = beta_is_f32; p.h0 = h0; p.ht = ht;
-  p.o = (bf16*)o; p.h = (bf16*)h; p.vnew = (bf16*)vnew;
-  p.N = N; p.Hq = Hq; p.Hv = Hv; p.T_rows = T_rows; p.scale = scale; p.lay = lay;
-  const bool extra = h != nullptr || vnew != nullptr;
-  auto launch = [&](auto kernel, int smem_bytes) {
-    int err = configure_smem((const void*)kernel, smem_bytes);
+  p.g = a.g_cum; p.beta = a.beta; p.beta_is_f32 = a.beta_is_f32;
+  p.h0 = a.h0; p.seg_h0 = a.seg_h0; p.h0_row = a.h0_row; p.ht_row = a.ht_row;
+  p.v_first = a.state_v_first; p.ht = a.ht;
+  p.o = (bf16*)a.o; p.h = (bf16*)a.h; p.vnew = (bf16*)a.vnew;
+  p.N = N; p.Hq = a.Hq; p.Hv = a.Hv; p.T_rows = T_rows; p.scale = a.scale; p.lay = lay;
+  p.tiled = a.operand_tiles; p.lead = a.lead_chunks; p.run_mask = a.run_mask;
+  p.run_value = a.run_value; p.order = a.seq_order;
+  auto launch = [&](auto kernel, int smem_bytes, std::atomic<unsigned long long>& done) {
+    int err = configure_smem((const void*)kernel, smem_bytes, done);
     if (err != 0) return err;
-    kernel<<<(unsigned)(N * Hv), 512, smem_bytes, st>>>(p, mq, mk, mv, ma, mh, mvn, mo);
-    return (int)cudaGetLastError();
+    return launch_pdl(kernel, dim3((unsigned)(N * a.Hv)), dim3(512), (size_t)smem_bytes, st, p, mq, mk,
+                      mv, ma, mh, mvn, mo);
   };
-  if (!q && !o) return launch(fwd_tc_kernel<true, true>, SMEM_BYTES_EXTRA);  // recomputation of h, v_new
-  if (extra) return launch(fwd_tc_kernel<true, false>, SMEM_BYTES_EXTRA);
-  return launch(fwd_tc_kernel<false, false>, SMEM_BYTES);
+  static std::atomic<unsigned long long> done[5];
+  if (!a.q && !a.o)  // recomputation of h, v_new
+    return launch(fwd_tc_kernel<true, true, false>, SMEM_BYTES_EXTRA, done[0]);
+  if (a.h || a.vnew)
+    return a.o_is_f16 ? launch(fwd_tc_kernel<true, false, true>, SMEM_BYTES_EXTRA, done[1])
+                      : launch(fwd_tc_kernel<true, false, false>, SMEM_BYTES_EXTRA, done[2]);
+  return a.o_is_f16 ? launch(fwd_tc_kernel<false, false, true>, SMEM_BYTES, done[3])
+                    : launch(fwd_tc_kernel<false, false, false>, SMEM_BYTES, done[4]);
 }
 
 }  // namespace fqla

@@ -111,10 +111,15 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
     b->n_seg = (int64_t)split->seg_bounds.size() - 1;
     begin = host.size();
     host.insert(host.end(), split->seg_begin.begin(), split->seg_begin.end());
+    std::vector<int> rf((size_t)b->n_seg, -1), rl((size_t)b->n_seg, -1);
+    for (int64_t i = 0; i < b->N; ++i) {
+      rf[(size_t)split->seg_begin[i]] = (int)i;
+      rl[(size_t)split->seg_begin[i + 1] - 1] = (int)i;
+    }
     first = host.size();
-    for (int64_t i = 0; i < b->N; ++i) host.push_back((int)split->seg_begin[i]);
+    host.insert(host.end(), rf.begin(), rf.end());
     last = host.size();
-    for (int64_t i = 0; i < b->N; ++i) host.push_back((int)split->seg_begin[i + 1] - 1);
+    host.insert(host.end(), rl.begin(), rl.end());
     // the last segment of a sequence hands nothing forward, the first nothing backward
     std::vector<int> keep_f((size_t)b->n_seg, 1), keep_b((size_t)b->n_seg, 1);
     for (int64_t i = 0; i < b->N; ++i)
@@ -152,8 +157,8 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
     b->s_begin = d + begin;
     b->keep_fwd = d + kf;
     b->keep_bwd = d + kb;
-    b->first_seg = b->store.narrow(0, (int64_t)first, b->N);
-    b->last_seg = b->store.narrow(0, (int64_t)last, b->N);
+    b->raw_first = d + first;
+    b->raw_last = d + last;
   }
   return b;
 }

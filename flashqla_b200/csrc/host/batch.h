@@ -27,7 +27,8 @@ struct Batch {
   const int *s_cu = nullptr, *s_offsets = nullptr, *s_indices = nullptr, *s_order = nullptr;
   const int *s_begin = nullptr;   // [N + 1] first segment of every raw sequence
   const int *keep_fwd = nullptr, *keep_bwd = nullptr;  // [n_seg]
-  at::Tensor first_seg, last_seg;  // int32 [N], views of `store`
+  // [n_seg]: the sequence a segment starts (ends), -1 for segments inside
+  const int *raw_first = nullptr, *raw_last = nullptr;
 };
 
 // Tables for a batch of `Hv` value heads; one host round trip (reads cu_seqlens, writes the

@@ -56,14 +56,10 @@ at::Tensor beta_in(const at::Tensor& b) {
   if (b.scalar_type() == at::kFloat || b.scalar_type() == at::kBFloat16) return b.contiguous();
   return b.to(at::kFloat).contiguous();
 }
-OptTensor state_in(const OptTensor& x, bool v_first) {
+// states: float32, in the caller's own layout (the kernels read either)
+OptTensor state_in(const OptTensor& x) {
   if (!x) return std::nullopt;
-  at::Tensor t = v_first ? x->transpose(-1, -2) : *x;
-  return as_f32(t);
-}
-OptTensor state_out(const OptTensor& x, bool v_first) {
-  if (!x || !v_first) return x;
-  return x->transpose(-1, -2).contiguous();
+  return aligned(x->scalar_type() == at::kFloat ? *x : x->to(at::kFloat));
 }
 
 // One call's shapes, stream and index tables.
@@ -121,16 +117,38 @@ struct SeqIn {  // inputs of the sequential kernels
   int beta_f32;
 };
 
-void run_fwd(const Call& c, const SeqIn& in, bool with_q, const float* h0, const OptTensor& ht,
-             const OptTensor& o, const OptTensor& h, const OptTensor& vnew, const OptTensor& M,
-             const int* warm, const int* m_mask, const int* lead, bool tiles) {
-  check(fqla_fwd_seq(with_q ? in.q.data_ptr() : nullptr, in.k.data_ptr(), in.v.data_ptr(),
-                     in.A.data_ptr(), (const float*)in.g.data_ptr(), in.beta.data_ptr(), in.beta_f32,
-                     h0, mut<float>(ht), mut(o), mut(h), mut(vnew), mut<float>(M), warm, m_mask, lead,
-                     c.order(), nullptr, 1, c.kB(), c.kT(), c.Hq, c.Hv, c.D, c.scale, c.cu(),
-                     c.offsets(), 0, c.N(), tiles, c.stream),
-        "fwd_seq");
+fqla_fwd_args fwd_args(const Call& c, const SeqIn& in) {
+  fqla_fwd_args a = {};
+  a.k = in.k.data_ptr(); a.v = in.v.data_ptr(); a.A = in.A.data_ptr();
+  a.g_cum = (const float*)in.g.data_ptr(); a.beta = in.beta.data_ptr(); a.beta_is_f32 = in.beta_f32;
+  a.seq_order = c.order(); a.run_value = 1; a.B = c.kB(); a.T = c.kT(); a.Hq = c.Hq; a.Hv = c.Hv;
+  a.D = c.D; a.scale = c.scale; a.cu_seqlens = c.cu(); a.chunk_offsets = c.offsets(); a.N = c.N();
+  return a;
 }
+// where the sequences' own initial states go in and final states come out
+void fwd_states(const Call& c, fqla_fwd_args& a, const OptTensor& h0, const OptTensor& seg_h0,
+                const OptTensor& ht, bool v_first) {
+  a.h0 = ptr<float>(h0);
+  a.ht = mut<float>(ht);
+  a.state_v_first = v_first;
+  if (c.split) {
+    a.seg_h0 = ptr<float>(seg_h0);
+    a.h0_row = c.batch->raw_first;
+    a.ht_row = c.batch->raw_last;
+  }
+}
+void run_fwd(const Call& c, const fqla_fwd_args& a) { check(fqla_fwd_run(&a, c.stream), "fwd_seq"); }
+
+fqla_bwd_dh_args dh_args(const Call& c, const SeqIn& in, const at::Tensor& dO) {
+  fqla_bwd_dh_args a = {};
+  a.q = in.q.data_ptr(); a.k = in.k.data_ptr(); a.A = in.A.data_ptr();
+  a.g_cum = (const float*)in.g.data_ptr(); a.beta = in.beta.data_ptr(); a.beta_is_f32 = in.beta_f32;
+  a.dO = dO.data_ptr(); a.seq_order = c.order(); a.run_value = 1; a.B = c.kB(); a.T = c.kT();
+  a.Hq = c.Hq; a.Hv = c.Hv; a.D = c.D; a.scale = c.scale; a.cu_seqlens = c.cu();
+  a.chunk_offsets = c.offsets(); a.N = c.N();
+  return a;
+}
+void run_dh(const Call& c, const fqla_bwd_dh_args& a) { check(fqla_bwd_dh_run(&a, c.stream), "bwd_dh"); }
 
 at::Tensor merge(const Call& c, const at::Tensor& local, const at::Tensor& M, const int* use_m,
                  const OptTensor& raw, const int* any_fb, bool reverse) {
@@ -181,43 +199,46 @@ Scan warmup_scan(const Call& c, const at::Tensor& g, bool from_start) {
   return s;
 }
 
+// The merge chain reads the sequences' own states as [key][value].
+OptTensor key_first(const OptTensor& x, bool v_first) {
+  return x && v_first ? OptTensor(x->transpose(-1, -2).contiguous()) : x;
+}
+
 // Start states of the segments (and lead-in counts) of a split plan.  Segments whose past dies out
 // inside the segment before them start themselves a few chunks early from a zero state; the exact
 // chain (state-only pass with the transition matrices, then the merge) returns at once for them.
-void segment_starts(const Call& c, const SeqIn& in, const OptTensor& h0, bool lead_in, Cache& out) {
-  const bool leads = lead_in && tiles_ok(c.D);
+void segment_starts(const Call& c, const SeqIn& in, const OptTensor& h0, const Options& opt, Cache& out) {
+  const bool leads = opt.lead_in && tiles_ok(c.D);
   const Scan s = leads ? segment_scan(c, in.g, false) : warmup_scan(c, in.g, false);
   at::Tensor local = empty({2, c.batch->n_seg, c.Hv, c.D, c.D}, at::kFloat, c.dev);
   at::Tensor l = local.select(0, 0), M = local.select(0, 1);
-  run_fwd(c, in, false, nullptr, l, std::nullopt, std::nullopt, std::nullopt, M,
-          leads ? s.exact_warm : s.warm, s.fallback, nullptr, false);
-  out.seg_h0 = merge(c, l, M, s.fallback, h0, leads ? s.any_fb : nullptr, false);
+  fqla_fwd_args a = fwd_args(c, in);
+  a.ht = (float*)l.data_ptr();
+  a.M = (float*)M.data_ptr();
+  a.warm_chunks = leads ? s.exact_warm : s.warm;
+  a.m_mask = s.fallback;
+  run_fwd(c, a);
+  out.seg_h0 = merge(c, l, M, s.fallback, key_first(h0, opt.state_v_first), leads ? s.any_fb : nullptr, false);
   if (leads) out.lead = s.lead_tensor;
-}
-
-void run_dh(const Call& c, const SeqIn& in, const at::Tensor& dO, const float* dht,
-            const OptTensor& dh, const OptTensor& du, const OptTensor& dh0, const int* warm,
-            const int* lead, bool tiles) {
-  check(fqla_bwd_dh(in.q.data_ptr(), in.k.data_ptr(), in.A.data_ptr(), (const float*)in.g.data_ptr(),
-                    in.beta.data_ptr(), in.beta_f32, dO.data_ptr(), dht, mut(dh), mut(du),
-                    mut<float>(dh0), warm, lead, c.order(), nullptr, 1, c.kB(), c.kT(), c.Hq, c.Hv,
-                    c.D, c.scale, c.cu(), c.offsets(), 0, c.N(), tiles, c.stream),
-        "bwd_dh");
 }
 
 // Mirror image of segment_starts for the state gradient.
 std::pair<at::Tensor, OptTensor> segment_ends(const Call& c, const SeqIn& in, const at::Tensor& dO,
-                                              const OptTensor& dht, bool lead_in, Scan& keep) {
-  const bool leads = lead_in && tiles_ok(c.D);
-  keep = leads ? segment_scan(c, in.g, true) : warmup_scan(c, in.g, true);
+                                              const OptTensor& dht, const Options& opt) {
+  const bool leads = opt.lead_in && tiles_ok(c.D);
+  const Scan s = leads ? segment_scan(c, in.g, true) : warmup_scan(c, in.g, true);
   at::Tensor local = empty({2, c.batch->n_seg, c.Hv, c.D, c.D}, at::kFloat, c.dev);
   at::Tensor l = local.select(0, 0), M = local.select(0, 1);
-  run_dh(c, in, dO, nullptr, std::nullopt, std::nullopt, l, leads ? keep.exact_warm : keep.warm,
-         nullptr, false);
-  run_fwd(c, in, false, nullptr, std::nullopt, std::nullopt, std::nullopt, std::nullopt, M, nullptr,
-          keep.fallback, nullptr, false);
-  at::Tensor ends = merge(c, l, M, keep.fallback, dht, leads ? keep.any_fb : nullptr, true);
-  return {ends, leads ? OptTensor(keep.lead_tensor) : std::nullopt};
+  fqla_bwd_dh_args a = dh_args(c, in, dO);
+  a.dh0 = (float*)l.data_ptr();
+  a.warm_chunks = leads ? s.exact_warm : s.warm;
+  run_dh(c, a);
+  fqla_fwd_args m = fwd_args(c, in);
+  m.M = (float*)M.data_ptr();
+  m.m_mask = s.fallback;
+  run_fwd(c, m);
+  at::Tensor ends = merge(c, l, M, s.fallback, key_first(dht, opt.state_v_first), leads ? s.any_fb : nullptr, true);
+  return {ends, leads ? OptTensor(s.lead_tensor) : std::nullopt};
 }
 
 constexpr double L2NORM_EPS = 1e-6;
@@ -274,7 +295,7 @@ Forward forward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor
   prepare(q_in, k_in, v_in, opt, r);
   const at::Tensor &q = r.q, &k = r.k, &v = r.v;
   const at::Tensor g = as_f32(g_in), beta = beta_in(beta_in_);
-  const OptTensor h0 = state_in(initial_state, opt.state_v_first);
+  const OptTensor h0 = state_in(initial_state);
   check_state(h0, c);
 
   // gate cumsum and A = (I + strict_lower(diag(beta) K K^T decay))^-1
@@ -290,24 +311,33 @@ Forward forward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor
   const SeqIn in{q, k, v, r.A, r.g_cum, beta, beta_f32};
   const bool tiles = tiles_ok(c.D);
   const bool keep = opt.cache && opt.save_tiles && !opt.output_h;
-  if (c.split) segment_starts(c, in, h0, opt.lead_in, r.cache);
+  if (c.split) segment_starts(c, in, h0, opt, r.cache);
 
-  r.o = empty(v.sizes(), at::kBFloat16, c.dev);
-  OptTensor h, vnew, ht;
+  // the tcgen05 kernel writes o in the caller's float16 itself
+  const bool o_f16 = tiles && q_in.scalar_type() == at::kHalf;
+  r.o = empty(v.sizes(), o_f16 ? at::kHalf : at::kBFloat16, c.dev);
+  OptTensor h, vnew;
   if (keep || opt.output_h)
     h = empty({c.batch->num_chunks, c.Hv, c.D, c.D}, at::kBFloat16, c.dev);
   if (keep)
     vnew = tiles ? empty({c.batch->num_chunks, c.Hv, c.D, CHUNK}, at::kBFloat16, c.dev)
                  : empty(v.sizes(), at::kBFloat16, c.dev);
-  if (opt.output_final_state) ht = empty({c.N(), c.Hv, c.D, c.D}, at::kFloat, c.dev);
-  run_fwd(c, in, true, c.split ? ptr<float>(r.cache.seg_h0) : ptr<float>(h0), ht, r.o, h, vnew,
-          std::nullopt, nullptr, nullptr, ptr<int>(r.cache.lead), keep && tiles);
-  if (c.split && ht) ht = ht->index_select(0, c.batch->last_seg);
-  r.final_state = state_out(ht, opt.state_v_first);
-  if (q_in.scalar_type() != at::kBFloat16) r.o = r.o.to(q_in.scalar_type());
+  if (opt.output_final_state)
+    r.final_state = empty({c.batch->N, c.Hv, c.D, c.D}, at::kFloat, c.dev);
+  fqla_fwd_args a = fwd_args(c, in);
+  fwd_states(c, a, h0, r.cache.seg_h0, r.final_state, opt.state_v_first);
+  a.q = q.data_ptr();
+  a.o = r.o.data_ptr();
+  a.o_is_f16 = o_f16;
+  a.h = mut(h);
+  a.vnew = mut(vnew);
+  a.lead_chunks = ptr<int>(r.cache.lead);
+  a.operand_tiles = keep && tiles;
+  run_fwd(c, a);
+  if (q_in.scalar_type() != r.o.scalar_type()) r.o = r.o.to(q_in.scalar_type());
   if (opt.output_h) {
     at::Tensor x = cu ? h->unsqueeze(0) : h->view({c.B, -1, c.Hv, c.D, c.D});
-    r.h = state_out(x, opt.state_v_first);
+    r.h = key_first(x, opt.state_v_first);
   }
   if (keep) {
     r.cache.h = h;
@@ -329,8 +359,8 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
   const at::Tensor dO = as_bf16(dO_in), A = as_bf16(A_in);
   const at::Tensor g = as_f32(g_in), beta = beta_in(beta_in_);
   const Call c = make_call(q, k, v, scale, cu, opt.auto_cp);
-  const OptTensor h0 = state_in(initial_state, opt.state_v_first);
-  const OptTensor dht = state_in(dht_in, opt.state_v_first);
+  const OptTensor h0 = state_in(initial_state);
+  const OptTensor dht = state_in(dht_in);
   check_state(h0, c);
   check_state(dht, c);
   const int beta_f32 = beta.scalar_type() == at::kFloat;
@@ -341,48 +371,66 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
   OptTensor h = cached.h, vnew = cached.vnew;
   if (!h || !vnew) {
     Cache starts{cached.seg_h0, std::nullopt, std::nullopt, cached.lead};
-    if (c.split && !starts.seg_h0) segment_starts(c, in, h0, opt.lead_in, starts);
+    if (c.split && !starts.seg_h0) segment_starts(c, in, h0, opt, starts);
     h = empty({c.batch->num_chunks, c.Hv, c.D, c.D}, at::kBFloat16, c.dev);
     vnew = tiles ? empty({c.batch->num_chunks, c.Hv, c.D, CHUNK}, at::kBFloat16, c.dev)
                  : empty(v.sizes(), at::kBFloat16, c.dev);
-    run_fwd(c, in, false, c.split ? ptr<float>(starts.seg_h0) : ptr<float>(h0), std::nullopt,
-            std::nullopt, h, vnew, std::nullopt, nullptr, nullptr,
-            tiles ? ptr<int>(starts.lead) : nullptr, tiles);
+    fqla_fwd_args a = fwd_args(c, in);
+    fwd_states(c, a, h0, starts.seg_h0, std::nullopt, opt.state_v_first);
+    a.h = mut(h);
+    a.vnew = mut(vnew);
+    a.lead_chunks = tiles ? ptr<int>(starts.lead) : nullptr;
+    a.operand_tiles = tiles;
+    run_fwd(c, a);
   }
 
   // reverse recurrence of the state gradient
-  OptTensor ends = dht, lead_out;
-  Scan scan{};
+  OptTensor seg_dht, lead_out;
   if (c.split) {
-    auto [e, l] = segment_ends(c, in, dO, dht, opt.lead_in, scan);
-    ends = e;
+    auto [e, l] = segment_ends(c, in, dO, dht, opt);
+    seg_dht = e;
     lead_out = l;
   }
   at::Tensor dh = empty({c.batch->num_chunks, c.Hv, c.D, c.D}, at::kBFloat16, c.dev);
   at::Tensor du = tiles ? empty({c.batch->num_chunks, c.Hv, c.D, CHUNK}, at::kBFloat16, c.dev)
                         : empty(v.sizes(), at::kBFloat16, c.dev);
-  OptTensor dh0;
-  if (initial_state) dh0 = empty({c.N(), c.Hv, c.D, c.D}, at::kFloat, c.dev);
-  run_dh(c, in, dO, ptr<float>(ends), dh, du, dh0, nullptr, ptr<int>(lead_out), tiles);
+  Backward r;
+  if (initial_state) r.dh0 = empty({c.batch->N, c.Hv, c.D, c.D}, at::kFloat, c.dev);
+  fqla_bwd_dh_args d = dh_args(c, in, dO);
+  d.dht = ptr<float>(dht);
+  d.dh = dh.data_ptr();
+  d.du = du.data_ptr();
+  d.dh0 = mut<float>(r.dh0);
+  d.state_v_first = opt.state_v_first;
+  d.lead_chunks = ptr<int>(lead_out);
+  d.operand_tiles = tiles;
+  if (c.split) {
+    d.seg_dht = ptr<float>(seg_dht);
+    d.dht_row = c.batch->raw_last;
+    d.dh0_row = c.batch->raw_first;
+  }
+  run_dh(c, d);
 
   // chunk-parallel part, per value head
-  Backward r;
   const int64_t total = c.batch->total, rows = (int64_t)c.B * c.T;
+  const bool db_bf16 = beta_in_.scalar_type() == at::kBFloat16;
   r.dq = empty({c.B, c.T, c.Hv, c.D}, at::kBFloat16, c.dev);
   r.dk = empty({c.B, c.T, c.Hv, c.D}, at::kBFloat16, c.dev);
   r.dv = empty({c.B, c.T, c.Hv, c.D}, at::kBFloat16, c.dev);
-  r.db = empty({c.B, c.T, c.Hv}, at::kFloat, c.dev);
-  at::Tensor dg = empty({c.B, c.T, c.Hv}, at::kFloat, c.dev);
+  r.db = empty({c.B, c.T, c.Hv}, db_bf16 ? at::kBFloat16 : at::kFloat, c.dev);
   r.dg = empty({c.B, c.T, c.Hv}, at::kFloat, c.dev);
   if (total < rows)  // rows past the last packed sequence are never written by the kernels
     for (at::Tensor* t : {&r.dq, &r.dk, &r.dv, &r.db, &r.dg}) t->narrow(1, total, rows - total).zero_();
-  check(fqla_bwd_main(q.data_ptr(), k.data_ptr(), v.data_ptr(), vnew->data_ptr(), A.data_ptr(),
-                      (const float*)g.data_ptr(), beta.data_ptr(), beta_f32, dO.data_ptr(),
-                      du.data_ptr(), h->data_ptr(), dh.data_ptr(), r.dq.data_ptr(), r.dk.data_ptr(),
-                      r.dv.data_ptr(), (float*)r.db.data_ptr(), (float*)dg.data_ptr(), c.kB(), c.kT(),
-                      c.Hq, c.Hv, c.D, c.scale, c.cu(), c.offsets(), c.indices(), 0,
-                      c.batch->num_chunks, tiles, c.stream),
-        "bwd_main");
+  fqla_bwd_main_args m = {};
+  m.q = q.data_ptr(); m.k = k.data_ptr(); m.v = v.data_ptr(); m.vnew = vnew->data_ptr();
+  m.A = A.data_ptr(); m.g_cum = (const float*)g.data_ptr(); m.beta = beta.data_ptr();
+  m.beta_is_f32 = beta_f32; m.dO = dO.data_ptr(); m.du = du.data_ptr(); m.h = h->data_ptr();
+  m.dh = dh.data_ptr(); m.dq = r.dq.data_ptr(); m.dk = r.dk.data_ptr(); m.dv = r.dv.data_ptr();
+  m.db = r.db.data_ptr(); m.dg = (float*)r.dg.data_ptr(); m.B = c.kB(); m.T = c.kT(); m.Hq = c.Hq;
+  m.Hv = c.Hv; m.D = c.D; m.scale = c.scale; m.cu_seqlens = c.cu(); m.chunk_offsets = c.offsets();
+  m.chunk_indices = c.indices(); m.num_chunks = c.batch->num_chunks; m.operand_tiles = tiles;
+  m.dg_cumsum = 1; m.db_is_bf16 = db_bf16;
+  check(fqla_bwd_main_run(&m, c.stream), "bwd_main");
   const bool f16 = dtype == at::kHalf;
   if (c.Hq < c.Hv || norm || f16) {
     const auto t = f16 ? at::kHalf : at::kBFloat16;
@@ -405,16 +453,8 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
     r.dk = dk;
     r.dv = dv;
   }
-  check(fqla_chunk_local_cumsum((const float*)dg.data_ptr(), (float*)r.dg.data_ptr(), c.B, c.T, c.Hv,
-                                c.batch->d_cu, 0, (int)c.batch->N, c.batch->d_indices,
-                                c.batch->num_chunks, 1, c.stream),
-        "chunk_local_cumsum");
   if (!f16 && dtype != at::kBFloat16)
     for (at::Tensor* t : {&r.dq, &r.dk, &r.dv}) *t = t->to(dtype);
-  if (dh0) {
-    if (c.split) dh0 = dh0->index_select(0, c.batch->first_seg);
-    r.dh0 = state_out(dh0, opt.state_v_first);
-  }
   return r;
 }
 

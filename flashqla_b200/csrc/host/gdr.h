@@ -51,7 +51,8 @@ Forward forward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, c
                 const OptTensor& cu, const Options& opt);
 
 // `g_cum` and `A` are the forward's; q, k the ones its kernels read.  With `norm` the gradients of q,
-// k are mapped back through the normalisation.  dq, dk, dv come in `dtype`, db and dg in float32.
+// k are mapped back through the normalisation.  dq, dk, dv come in `dtype`, db
+// in bfloat16 or float32 (beta's type where it is one of them), dg in float32.
 Backward backward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
                   const at::Tensor& g_cum, const at::Tensor& beta, const at::Tensor& A,
                   const at::Tensor& dO, const OptTensor& dht, double scale,

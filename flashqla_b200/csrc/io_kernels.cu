@@ -74,6 +74,7 @@ struct PrepareParams {
 template <typename IN, int D>
 __global__ void __launch_bounds__(256) prepare_inputs_kernel(const PrepareParams p) {
   constexpr int LANES = D / 8;
+  pdl_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   const long long n_qk = p.rows_qk * LANES, n_v = p.v_out ? p.rows_v * LANES : 0;
   // which tensor, and the 16-byte piece of it (rows never straddle a warp: LANES divides 32)
@@ -111,6 +112,7 @@ struct FinishParams {
 template <typename OUT, int D>
 __global__ void __launch_bounds__(256) finish_grads_kernel(const FinishParams p) {
   constexpr int LANES = D / 8;
+  pdl_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   const long long n_qk = p.rows_qk * LANES, n_v = p.dv_in ? p.rows_v * LANES : 0;
   const bool is_q = i < n_qk, is_k = !is_q && i < 2 * n_qk;
@@ -168,13 +170,11 @@ extern "C" int fqla_prepare_inputs(const void* q, const void* k, const void* v, 
   const unsigned grid = (unsigned)((n + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
   if (D == 128) {
-    if (is_f16) prepare_inputs_kernel<F16x8, 128><<<grid, 256, 0, st>>>(p);
-    else prepare_inputs_kernel<Bf16x8, 128><<<grid, 256, 0, st>>>(p);
-  } else {
-    if (is_f16) prepare_inputs_kernel<F16x8, 64><<<grid, 256, 0, st>>>(p);
-    else prepare_inputs_kernel<Bf16x8, 64><<<grid, 256, 0, st>>>(p);
+    if (is_f16) return launch_pdl(prepare_inputs_kernel<F16x8, 128>, dim3(grid), dim3(256), 0, st, p);
+    return launch_pdl(prepare_inputs_kernel<Bf16x8, 128>, dim3(grid), dim3(256), 0, st, p);
   }
-  return (int)cudaGetLastError();
+  if (is_f16) return launch_pdl(prepare_inputs_kernel<F16x8, 64>, dim3(grid), dim3(256), 0, st, p);
+  return launch_pdl(prepare_inputs_kernel<Bf16x8, 64>, dim3(grid), dim3(256), 0, st, p);
 }
 
 extern "C" int fqla_finish_grads(const void* dq_v, const void* dk_v, const void* dv_in,
@@ -191,11 +191,9 @@ extern "C" int fqla_finish_grads(const void* dq_v, const void* dk_v, const void*
   const unsigned grid = (unsigned)((n + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
   if (D == 128) {
-    if (is_f16) finish_grads_kernel<F16x8, 128><<<grid, 256, 0, st>>>(p);
-    else finish_grads_kernel<Bf16x8, 128><<<grid, 256, 0, st>>>(p);
-  } else {
-    if (is_f16) finish_grads_kernel<F16x8, 64><<<grid, 256, 0, st>>>(p);
-    else finish_grads_kernel<Bf16x8, 64><<<grid, 256, 0, st>>>(p);
+    if (is_f16) return launch_pdl(finish_grads_kernel<F16x8, 128>, dim3(grid), dim3(256), 0, st, p);
+    return launch_pdl(finish_grads_kernel<Bf16x8, 128>, dim3(grid), dim3(256), 0, st, p);
   }
-  return (int)cudaGetLastError();
+  if (is_f16) return launch_pdl(finish_grads_kernel<F16x8, 64>, dim3(grid), dim3(256), 0, st, p);
+  return launch_pdl(finish_grads_kernel<Bf16x8, 64>, dim3(grid), dim3(256), 0, st, p);
 }

@@ -18,6 +18,7 @@ __global__ void __launch_bounds__(128) cumsum_kernel(const float* __restrict__ g
                                                      float* __restrict__ out, int H, int T_rows,
                                                      SeqLayout lay, IndexTable chunk_indices,
                                                      int N, int reverse) {
+  pdl_wait();
   int seq, ci;
   if (lay.cu.ptr) {
     seq = (int)chunk_indices[2 * blockIdx.x];
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(128, 6) kkt_solve_kernel(
 
   int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int hq = blockIdx.y, G = Hv / Hq;
+  pdl_wait();
   int seq, ci;
   if (lay.cu.ptr) {
     seq = (int)chunk_indices[2 * blockIdx.x];
@@ -277,6 +279,7 @@ __global__ void __launch_bounds__(128, 6) kkt_solve_kernel(
 __global__ void group_reduce_kernel(const bf16* __restrict__ in, bf16* __restrict__ out,
                                     long long n_vec, int G, int D8) {
   // one thread per 8-element (16-byte) segment of an output row
+  pdl_wait();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_vec) return;
   long long row_hq = i / D8;
@@ -312,9 +315,8 @@ extern "C" int fqla_chunk_local_cumsum(const float* g, float* out, int B, int T,
   SeqLayout lay{{cu_seqlens, idx_is64}, {nullptr, idx_is64}, T};
   long long n = cu_seqlens ? num_chunks : (long long)B * ((T + CHUNK - 1) / CHUNK);
   if (n <= 0) return FQLA_OK;
-  cumsum_kernel<<<(unsigned)n, 128, 0, (cudaStream_t)stream>>>(
+  return launch_pdl(cumsum_kernel, dim3((unsigned)n), dim3(128), 0, (cudaStream_t)stream,
       g, out, H, B * T, lay, IndexTable{chunk_indices, idx_is64}, cu_seqlens ? N : B, reverse);
-  return (int)cudaGetLastError();
 }
 
 template <int D>
@@ -323,11 +325,11 @@ static int launch_kkt(const void* k, const void* beta, int beta_is_f32, const fl
                       long long n, cudaStream_t st) {
   constexpr int k_tile = CHUNK * (D + 8) * 2, x_tile = CHUNK * (CHUNK + 4) * 4;
   constexpr int smem = (k_tile > x_tile ? k_tile : x_tile) + x_tile + 2 * CHUNK * 4;
-  int rc = configure_smem((const void*)kkt_solve_kernel<D>, smem);
+  static std::atomic<unsigned long long> done;
+  int rc = configure_smem((const void*)kkt_solve_kernel<D>, smem, done);
   if (rc != 0) return rc;
-  kkt_solve_kernel<D><<<dim3((unsigned)n, Hq), 128, smem, st>>>(
-      (const bf16*)k, beta, beta_is_f32, g, g_cum_out, (bf16*)A, Hq, Hv, lay, ci);
-  return (int)cudaGetLastError();
+  return launch_pdl(kkt_solve_kernel<D>, dim3((unsigned)n, Hq), dim3(128), (size_t)smem, st, (const bf16*)k,
+                    beta, beta_is_f32, g, g_cum_out, (bf16*)A, Hq, Hv, lay, ci);
 }
 
 extern "C" int fqla_kkt_solve(const void* k, const void* beta, int beta_is_f32,
@@ -352,7 +354,6 @@ extern "C" int fqla_group_reduce(const void* in, void* out, long long rows, int 
   if (!in || !out || G <= 0 || D % 8) return FQLA_ERR_INVALID_ARG;
   long long n_vec = rows * Hq * (D / 8);
   if (n_vec <= 0) return FQLA_OK;
-  group_reduce_kernel<<<(unsigned)((n_vec + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-      (const bf16*)in, (bf16*)out, n_vec, G, D / 8);
-  return (int)cudaGetLastError();
+  return launch_pdl(group_reduce_kernel, dim3((unsigned)((n_vec + 255) / 256)), dim3(256), 0,
+                    (cudaStream_t)stream, (const bf16*)in, (bf16*)out, n_vec, G, D / 8);
 }

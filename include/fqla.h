@@ -93,6 +93,35 @@ int fqla_fwd_seq(const void* q, const void* k, const void* v, const void* A, con
                  int B, int T, int Hq, int Hv, int D, float scale, const void* cu_seqlens,
                  const void* chunk_offsets, int idx_is64, int N, int operand_tiles, void* stream);
 
+/* fqla_fwd_seq with every argument in one structure, zero-initialised by the caller, plus what the
+ * positional form has no room for:
+ *   h0_row [N] (int32, optional): sequence n starts from h0[h0_row[n]] where that is >= 0, else from
+ *     seg_h0[n] (zero without seg_h0).  For the segments of a split plan h0 then stays in the order
+ *     of the sequences, and seg_h0 (the merge chain's output) is read only where a segment is handed
+ *     a state.  Without h0_row: h0[n].
+ *   ht_row [N] (int32, optional): the end state of sequence n goes to ht[ht_row[n]] where that is
+ *     >= 0 and nowhere otherwise.  Without ht_row: ht[n].
+ *   state_v_first: h0 and ht are [value dim][key dim] instead of [key dim][value dim] (seg_h0 and M
+ *     never are).
+ *   o_is_f16: o is written as fp16 (K = V = 128, tcgen05 kernel only). */
+typedef struct fqla_fwd_args {
+  const void *q, *k, *v, *A;
+  const float* g_cum;
+  const void* beta;
+  int beta_is_f32;
+  const float *h0, *seg_h0;
+  const int *h0_row, *ht_row;
+  float* ht;
+  void *o, *h, *vnew;
+  float* M;
+  const int *warm_chunks, *m_mask, *lead_chunks, *seq_order, *run_mask;
+  int run_value, B, T, Hq, Hv, D;
+  float scale;
+  const void *cu_seqlens, *chunk_offsets;
+  int idx_is64, N, operand_tiles, state_v_first, o_is_f16;
+} fqla_fwd_args;
+int fqla_fwd_run(const fqla_fwd_args* args, void* stream);
+
 /* Sequential reverse recurrence of the state gradient.  Optional outputs: per-chunk dh, du (the
  * gradient of vnew), dh0.  warm_chunks (optional, dh0-only calls): walk only the first
  * warm_chunks[n,hv] chunks from a zero gradient.  operand_tiles != 0 (K = V = 128, no
@@ -113,6 +142,28 @@ int fqla_bwd_dh(const void* q, const void* k, const void* A, const float* g_cum,
                 float scale, const void* cu_seqlens, const void* chunk_offsets, int idx_is64, int N,
                 int operand_tiles, void* stream);
 
+/* fqla_bwd_dh with every argument in one structure, zero-initialised by the caller.  dht_row [N]:
+ * sequence n starts from dht[dht_row[n]] where that is >= 0, else from seg_dht[n] (zero without
+ * seg_dht); dh0_row [N]: dh0 of sequence n goes to dh0[dh0_row[n]] where that is >= 0;
+ * state_v_first: dht and dh0 are [value dim][key dim].  As in fqla_fwd_args. */
+typedef struct fqla_bwd_dh_args {
+  const void *q, *k, *A;
+  const float* g_cum;
+  const void* beta;
+  int beta_is_f32;
+  const void* dO;
+  const float *dht, *seg_dht;
+  const int *dht_row, *dh0_row;
+  void *dh, *du;
+  float* dh0;
+  const int *warm_chunks, *lead_chunks, *seq_order, *run_mask;
+  int run_value, B, T, Hq, Hv, D;
+  float scale;
+  const void *cu_seqlens, *chunk_offsets;
+  int idx_is64, N, operand_tiles, state_v_first;
+} fqla_bwd_dh_args;
+int fqla_bwd_dh_run(const fqla_bwd_dh_args* args, void* stream);
+
 /* Chunk-parallel backward: dq, dk (per VALUE head, [B,T,Hv,D] bf16), dv, dbeta and the
  * pre-cumsum dg (both fp32 [B,T,Hv]) from h, dh, vnew and du.  operand_tiles != 0 (K = V = 128):
  * h, dh, vnew and du are in the operand layouts written by fqla_fwd_seq / fqla_bwd_dh with the
@@ -124,6 +175,26 @@ int fqla_bwd_main(const void* q, const void* k, const void* v, const void* vnew,
                   float* db, float* dg, int B, int T, int Hq, int Hv, int D, float scale,
                   const void* cu_seqlens, const void* chunk_offsets, const void* chunk_indices,
                   int idx_is64, long long num_chunks, int operand_tiles, void* stream);
+
+/* fqla_bwd_main with every argument in one structure, zero-initialised by the caller.  dg_cumsum: dg
+ * comes out after its reverse chunk-local cumulative sum (what fqla_chunk_local_cumsum, reverse,
+ * would make of it); db_is_bf16: db is bf16 instead of fp32. */
+typedef struct fqla_bwd_main_args {
+  const void *q, *k, *v, *vnew, *A;
+  const float* g_cum;
+  const void* beta;
+  int beta_is_f32;
+  const void *dO, *du, *h, *dh;
+  void *dq, *dk, *dv, *db;
+  float* dg;
+  int B, T, Hq, Hv, D;
+  float scale;
+  const void *cu_seqlens, *chunk_offsets, *chunk_indices;
+  int idx_is64;
+  long long num_chunks;
+  int operand_tiles, dg_cumsum, db_is_bf16;
+} fqla_bwd_main_args;
+int fqla_bwd_main_run(const fqla_bwd_main_args* args, void* stream);
 
 /* out[row, hq, :] = sum over the G value heads of group hq of in[row, hq*G + i, :] (bf16, fp32
  * accumulation).  Replaces group_reduce_vector, flash_qla/ops/utils/group_reduce.py:60-79. */
