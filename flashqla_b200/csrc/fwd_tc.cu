@@ -1040,6 +1040,7 @@ extern "C" int fqla_selftest_wait_timeout(int tries, void* stream) {
 namespace fqla {
 int bwd_main_tc_status(int* out, int reset);
 int bwd_dh_tc_status(int* out, int reset);
+int kkt_status(int* out, int reset);
 }
 
 extern "C" int fqla_device_status(int* out, int reset) {
@@ -1051,7 +1052,10 @@ extern "C" int fqla_device_status(int* out, int reset) {
   if (rc != 0) return rc;
   rc = fqla::bwd_dh_tc_status(&u, reset);
   if (rc != 0) return rc;
-  if (out) *out = v | w | u;
+  int x = 0;
+  rc = fqla::kkt_status(&x, reset);
+  if (rc != 0) return rc;
+  if (out) *out = v | w | u | x;
   if (reset && v != 0) {
     int z = 0;
     e = cudaMemcpyToSymbol(fqla::g_device_status, &z, sizeof(int));

@@ -4,11 +4,15 @@
 //   * sum of per-value-head dq/dk over each grouped-value-attention group
 // These replace the reference's ops/utils/cumsum.py:14-134, blackwell/kkt_solve.py:19-281 and
 // ops/utils/group_reduce.py:12-57.
-#include <type_traits>
+#include <cuda.h>
+
 #include "common.cuh"
 #include "fqla_internal.h"
+#include "tc05.cuh"
 
 namespace fqla {
+
+int make_tile_map(CUtensorMap* m, const void* ptr, long long rows, long long cols, int box_rows);
 
 // ------------------------------------------------------------------------------------------
 // Chunk-local cumsum.  One CTA per chunk, one warp per head (looping), two rows per lane.
@@ -58,75 +62,160 @@ __global__ void __launch_bounds__(128) cumsum_kernel(const float* __restrict__ g
   }
 }
 
-// C[16 x 8*NT] = A[16 x 8*KT] * B[8*KT x 8*NT], both row-major fp32 in shared memory, as
-// mma.m16n8k8 with tf32 inputs.  Fragment element (g = lane/4, t = lane%4): c[nt][0..3] =
-// C[g][8nt+2t], C[g][8nt+2t+1], C[g+8][8nt+2t], C[g+8][8nt+2t+1].
-__device__ __forceinline__ uint32_t to_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+// ------------------------------------------------------------------------------------------
+// kkt + solve:  A = (I + L)^-1,  L = strict_lower(diag(beta) K K^T exp(g_s - g_t)),  one 64 x 64
+// problem per (chunk, value head).
+//
+// ONE WARP solves one problem, in registers: there is no block-wide barrier on the way, and what
+// hides the latencies is that a dozen warps with a problem each sit on an SM.  (The form before
+// spread a problem over four warps and met eight block barriers per head with two of the four
+// warps idle in the forward substitution: 79 us for 8192 problems against 31 us of HBM time.)
+// A block is min(G, 4) warps sharing the K tile of one (chunk, q head); warp w takes the value
+// heads w, w + 4, ... of the group.
+//
+// All 64 x 64 matrices are 16 x 16 blocks in the fragment layout of mma.sync (lane l = 4 g + t:
+// element e of column half h is row g + 8 (e >> 1), column 8 h + 2 t + (e & 1)):
+//   1. K K^T: the 10 blocks on and below the diagonal (bf16 products, fp32 sums).  A fragment of
+//      rows loaded by ldmatrix serves as left operand and, for the transposed product, as right
+//      operand, so each is loaded once.
+//   2. L in place; the four 16 x 16 diagonal blocks go through shared memory.
+//   3. D_i = (I + L_ii)^-1 by forward substitution in fp32, a lane = one column of two blocks.
+//   4. The blocks of X = A below the diagonal, from  X_ij = -D_i (sum_{j<=k<i} L_ik X_kj),  are
+//      computed TRANSPOSED (Y_ji = X_ij^T = -(sum_k Y_jk L_ik^T) D_i^T, Y_jj = D_j^T): then every left
+//      operand is a result in fragment layout and every right operand L_ik^T, D_i^T is, read
+//      element for element, the fragment of L_ik, D_i: no shuffle, no shared memory.  tf32 inputs
+//      rounded to nearest, fp32 sums.  (tf32 k index t / t + 4 stands for column 2 t / 2 t + 1.)
+//   5. bf16 tile through shared memory (stmatrix undoes the transposition), one TMA store.
+// L is kept NEGATED throughout, so that every step is an addition.
+//
+// What bounds it: instruction issue and the latency of one warp's chain.  4 x 8192 tokens, 16 heads
+// (8192 problems): the four-warp form 79 us; this one with scalar fp32, cvt.rna and per-thread
+// copies 58 us (3090 instructions per problem); with packed fp32 pairs, TMA both ways and the
+// rounding add below KKT_NOW
+// ------------------------------------------------------------------------------------------
+// set to 1 when a block of kkt_solve_kernel abandoned its bounded wait; read through
+// fqla_device_status
+__device__ int g_kkt_status = 0;
+
+struct Block16 {  // 16 x 16 fp32 fragment
+  float c[2][4];
+};
+// the same block as tf32 operand.  Rounding to nearest (ties away) is adding half an ulp of the
+// 10-bit mantissa to the magnitude; the tensor core ignores the 13 bits below.
+struct Op16 {
+  uint32_t c[2][4];
+};
+__device__ __forceinline__ uint32_t to_tf32(float x) { return __float_as_uint(x) + 0x1000u; }
+__device__ __forceinline__ Op16 to_op(const Block16& b) {
+  Op16 o;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o.c[h][e] = to_tf32(b.c[h][e]);
+  return o;
+}
+// d (+)= a * b^T
+template <bool ADD>
+__device__ __forceinline__ void mma_abt(Block16& d, const Op16& a, const Op16& b) {
+#pragma unroll
+  for (int s = 0; s < 2; ++s)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (ADD || s > 0)
+        asm volatile(
+            "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+            "{%0,%1,%2,%3};"
+            : "+f"(d.c[h][0]), "+f"(d.c[h][1]), "+f"(d.c[h][2]), "+f"(d.c[h][3])
+            : "r"(a.c[s][0]), "r"(a.c[s][2]), "r"(a.c[s][1]), "r"(a.c[s][3]), "r"(b.c[s][2 * h]),
+              "r"(b.c[s][2 * h + 1]));
+      else
+        asm volatile(
+            "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+            "{%10,%10,%10,%10};"
+            : "=f"(d.c[h][0]), "=f"(d.c[h][1]), "=f"(d.c[h][2]), "=f"(d.c[h][3])
+            : "r"(a.c[s][0]), "r"(a.c[s][2]), "r"(a.c[s][1]), "r"(a.c[s][3]), "r"(b.c[s][2 * h]),
+              "r"(b.c[s][2 * h + 1]), "f"(0.f));
+    }
+}
+template <bool ADD>
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if (ADD)
+    mma_bf16_16816(d, a, b0, b1);
+  else
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+        "{%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// packed pairs of fp32 (one instruction for two lanes of arithmetic)
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "add.rn.ftz.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return r;
 }
-template <int NT, int KT>
-__device__ __forceinline__ void tf32_gemm(float (&c)[NT][4], const float* A, int lda, const float* B,
-                                          int ldb, int lane) {
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
-#pragma unroll
-  for (int kt = 0; kt < KT; ++kt) {
-    const uint32_t a0 = to_tf32(A[g * lda + 8 * kt + t]), a1 = to_tf32(A[(g + 8) * lda + 8 * kt + t]);
-    const uint32_t a2 = to_tf32(A[g * lda + 8 * kt + t + 4]), a3 = to_tf32(A[(g + 8) * lda + 8 * kt + t + 4]);
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-      const uint32_t b0 = to_tf32(B[(8 * kt + t) * ldb + 8 * nt + g]);
-      const uint32_t b1 = to_tf32(B[(8 * kt + t + 4) * ldb + 8 * nt + g]);
-      asm volatile(
-          "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-          "{%0,%1,%2,%3};"
-          : "+f"(c[nt][0]), "+f"(c[nt][1]), "+f"(c[nt][2]), "+f"(c[nt][3])
-          : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    }
-  }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "mul.rn.ftz.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
 }
-template <int NT>
-__device__ __forceinline__ void store_frag(float* C, int ldc, const float (&c)[NT][4], float sign,
-                                           int lane) {
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt) {
-    *reinterpret_cast<float2*>(C + g * ldc + 8 * nt + 2 * t) = make_float2(sign * c[nt][0], sign * c[nt][1]);
-    *reinterpret_cast<float2*>(C + (g + 8) * ldc + 8 * nt + 2 * t) = make_float2(sign * c[nt][2], sign * c[nt][3]);
-  }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, w, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 w, {%6, %7};\n\t"
+      "fma.rn.ftz.f32x2 z, x, y, w;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
 }
 
-// ------------------------------------------------------------------------------------------
-// kkt + solve.  One CTA (128 threads) per (chunk, q head): K K^T is computed once and kept in
-// registers, then scaled and inverted for each of the Hv / Hq value heads of the group in turn.
-//   1. K K^T (64x64xD) on tensor cores, 2. L = strict_lower(beta_s * KK^T * exp(g_s-g_t)) in fp32,
-//   3. X = (I+L)^-1 by blocked forward substitution in fp32, 4. bf16 rows out.
-// ------------------------------------------------------------------------------------------
+namespace kkt {
+constexpr int MAX_WARPS = 4;
+// The diagonal blocks 0 | 2 and 1 | 3 sit in shared memory as two matrices of pairs, so that one
+// packed operation serves both blocks.  Row stride 52 words (16-byte rows, at most two-way bank
+// conflicts for fragments and transposed fragments), pair stride 16 banks apart (the two
+// half-warps read one pair each).
+constexpr int LD_DIAG = 52, DIAG_STRIDE = 16 * LD_DIAG + 16;
+constexpr int WARP_BYTES = CHUNK * CHUNK * 2;  // 8192: the output tile, and before it the diagonal blocks
+constexpr int VEC_BYTES = 2 * CHUNK * 4;       // g, -beta of a warp's head
+static_assert(2 * DIAG_STRIDE * 4 <= WARP_BYTES, "diagonal blocks fit the output tile");
 template <int D>
-__global__ void __launch_bounds__(128, 6) kkt_solve_kernel(
-    const bf16* __restrict__ k, const void* __restrict__ beta, int beta_is_f32,
-    const float* __restrict__ g, float* __restrict__ g_cum_out, bf16* __restrict__ A, int Hq,
-    int Hv, SeqLayout lay, IndexTable chunk_indices) {
-  constexpr int LDK = D + 8;
-  constexpr int LDL = CHUNK + 4;  // floats; rows stay 16-byte aligned
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* sK = reinterpret_cast<bf16*>(smem_raw);
-  // the inverse X [64][LDL] is built over the K tile, dead once K K^T is in sL (5 CTAs per SM)
-  constexpr int REGION0 = CHUNK * LDK * 2 > CHUNK * LDL * 4 ? CHUNK * LDK * 2 : CHUNK * LDL * 4;
-  float* sX = reinterpret_cast<float*>(smem_raw);
-  float* sL = reinterpret_cast<float*>(smem_raw + REGION0);
-  float* sG = sL + CHUNK * LDL;
-  float* sB = sG + CHUNK;
-  // partial products [32][32]: they live in the rows 0-31, columns 32-63 of L, a part of its
-  // upper triangle that is neither written nor read (six CTAs per SM fit with that)
-  constexpr int LDY = LDL;
-  float* sY = sL + 32;
+constexpr int k_bytes() { return CHUNK * D * 2; }
+// a single-warp block builds its output over the K tile, dead by then; + barrier, + alignment
+template <int D>
+constexpr int smem_bytes(int warps) {
+  return k_bytes<D>() + warps * VEC_BYTES + (warps > 1 ? warps * WARP_BYTES : 0) + 16 + 1024;
+}
+}  // namespace kkt
 
-  int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+template <int D>
+__global__ void __launch_bounds__(32 * kkt::MAX_WARPS, 3) kkt_solve_kernel(
+    const void* __restrict__ beta, int beta_is_f32, const float* __restrict__ g,
+    float* __restrict__ g_cum_out, bf16* __restrict__ A, int Hq, int Hv, SeqLayout lay,
+    IndexTable chunk_indices, const __grid_constant__ CUtensorMap map_k,
+    const __grid_constant__ CUtensorMap map_a) {
+  using namespace kkt;
+  extern __shared__ unsigned char smem_dyn[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n_warps = blockDim.x >> 5;
+  // per-warp scratch (1024-byte aligned): diagonal blocks (fp32), then the output tile (bf16)
+  unsigned char* scratch = n_warps == 1 ? smem : smem + k_bytes<D>() + warp * WARP_BYTES;
+  float* sD = reinterpret_cast<float*>(scratch);
+  unsigned char* vecs = smem + k_bytes<D>() + (n_warps > 1 ? n_warps * WARP_BYTES : 0);
+  float* sG = reinterpret_cast<float*>(vecs + warp * VEC_BYTES);  // g log2(e)
+  float* sB = sG + CHUNK;                                         // -beta
+  uint64_t* bar = reinterpret_cast<uint64_t*>(vecs + n_warps * VEC_BYTES);
+  int* abort_flag = reinterpret_cast<int*>(bar + 1);
+  const int q8 = lane >> 2, t4 = lane & 3, l7 = lane & 7;  // fragment row, column pair; row mod 8
   const int hq = blockIdx.y, G = Hv / Hq;
+  if (tid == 0) {
+    tc::mbar_init(bar, 1);
+    *abort_flag = 0;
+    tc::fence_mbar_init();
+  }
   pdl_wait();
   int seq, ci;
   if (lay.cu.ptr) {
@@ -137,139 +226,252 @@ __global__ void __launch_bounds__(128, 6) kkt_solve_kernel(
     seq = blockIdx.x / per;
     ci = blockIdx.x % per;
   }
-  SeqSpan sp = lay.span(seq);
-  long long row0 = sp.bos + (long long)ci * CHUNK;
-  int valid = min(CHUNK, sp.len - ci * CHUNK);
+  const SeqSpan sp = lay.span(seq);
+  const long long row0 = sp.bos + (long long)ci * CHUNK;
+  const int valid = min(CHUNK, sp.len - ci * CHUNK);
+  if (n_warps > 1) __syncthreads();
+  else __syncwarp();
+  if (tid == 0) {
+    // rows past the end of the sequence hold other rows of k: what they give is masked below
+    tc::mbar_arrive_expect_tx(bar, k_bytes<D>());
+#pragma unroll
+    for (int b = 0; b < D / 64; ++b)
+      tc::tma_load_2d(smem + b * 8192, &map_k, hq * D + 64 * b, (int)row0, bar);
+  }
+  bool ok = true;
 
-  load_tile_async<D, LDK, 128>(sK, k + (row0 * Hq + hq) * D, (long long)Hq * D, valid, tid);
-  cp_async_commit();
-  float kkt[24];  // this thread's part of the lower blocks of K K^T
 #pragma unroll 1
-  for (int gi = 0; gi < G; ++gi) {
-  const int hv = hq * G + gi;
-  if (gi > 0) __syncthreads();  // the inverse of the head before has been written out
-  if (tid < CHUNK) {
-    sB[tid] = tid < valid ? load_beta(beta, beta_is_f32, (row0 + tid) * Hv + hv) : 0.f;
-    if (g_cum_out) {
-      // g is the raw log gate: chunk-local inclusive prefix sum over the valid rows (rows past
-      // the end repeat the last value, as the clamped read below does), done by the first two warps
-      float x = tid < valid ? g[(row0 + tid) * Hv + hv] : 0.f;
+  for (int gi = warp; gi < G && ok; gi += n_warps) {
+    const int hv = hq * G + gi;
+    {  // gates and beta of the rows lane, lane + 32
+      float x[2];
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const float y = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= d) x += y;
+      for (int z = 0; z < 2; ++z) {
+        const int r = lane + 32 * z;
+        const long long i = (row0 + min(r, valid - 1)) * Hv + hv;
+        x[z] = g[i];
+        sB[r] = r < valid ? -load_beta(beta, beta_is_f32, i) : 0.f;
       }
-      if (tid == 31) sL[0] = x;
-      asm volatile("bar.sync 1, 64;" ::: "memory");
-      if (tid >= 32) x += sL[0];
-      sG[tid] = x;
-      if (tid < valid) g_cum_out[(row0 + tid) * Hv + hv] = x;
+      if (g_cum_out) {
+        // g is the raw log gate: chunk-local inclusive prefix sum over the valid rows (rows past
+        // the end repeat the last value, as the clamped read does)
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          if (lane + 32 * z >= valid) x[z] = 0.f;
+#pragma unroll
+          for (int d = 1; d < 32; d <<= 1) {
+            const float y = __shfl_up_sync(0xffffffffu, x[z], d);
+            if (lane >= d) x[z] += y;
+          }
+        }
+        x[1] += __shfl_sync(0xffffffffu, x[0], 31);
+#pragma unroll
+        for (int z = 0; z < 2; ++z)
+          if (lane + 32 * z < valid) g_cum_out[(row0 + lane + 32 * z) * Hv + hv] = x[z];
+      }
+      sG[lane] = x[0] * 1.4426950408889634f;
+      sG[lane + 32] = x[1] * 1.4426950408889634f;
+    }
+    ok = tc::mbar_wait(bar, 0, abort_flag);
+    if (!ok) break;
+    __syncwarp();
+
+    // ---- 1. K K^T, lower blocks (rb, cb), index rb (rb + 1) / 2 + cb
+    Block16 L[10];
+    {
+      // 16-byte chunk c of row r of a 64-column block sits at chunk c ^ (r & 7)
+      const uint32_t frag = smem_u32(smem) + (uint32_t)((l7 + ((lane >> 3) & 1) * 8) * 128);
+      uint32_t col[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) col[i] = (uint32_t)(((2 * i + (lane >> 4)) ^ l7) << 4);
+#pragma unroll
+      for (int ks = 0; ks < D / 16; ++ks) {
+        uint32_t a[4][4];
+#pragma unroll
+        for (int rb = 0; rb < 4; ++rb)
+          ldmatrix_x4_addr(a[rb], frag + col[ks & 3] + (uint32_t)((ks >> 2) * 8192 + rb * 2048));
+#pragma unroll
+        for (int rb = 0; rb < 4; ++rb)
+#pragma unroll
+          for (int cb = 0; cb <= rb; ++cb) {
+            Block16& d = L[rb * (rb + 1) / 2 + cb];
+            if (ks == 0) {
+              mma_bf16<false>(d.c[0], a[rb], a[cb][0], a[cb][2]);
+              mma_bf16<false>(d.c[1], a[rb], a[cb][1], a[cb][3]);
+            } else {
+              mma_bf16<true>(d.c[0], a[rb], a[cb][0], a[cb][2]);
+              mma_bf16<true>(d.c[1], a[rb], a[cb][1], a[cb][3]);
+            }
+          }
+      }
+    }
+    // ---- 2. -L
+    {
+      float gr[8], br[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        gr[i] = sG[8 * i + q8];
+        br[i] = sB[8 * i + q8];
+      }
+      const bool below0 = q8 > 2 * t4, below1 = q8 > 2 * t4 + 1;  // inside an 8 x 8 diagonal block
+#pragma unroll
+      for (int cb = 0; cb < 4; ++cb)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float2 gc = *reinterpret_cast<const float2*>(sG + 16 * cb + 8 * h + 2 * t4);
+          const float2 ngc = make_float2(-gc.x, -gc.y);
+#pragma unroll
+          for (int rb = cb; rb < 4; ++rb)
+#pragma unroll
+            for (int z = 0; z < 2; ++z) {
+              float* c = L[rb * (rb + 1) / 2 + cb].c[h] + 2 * z;
+              if (rb == cb && h > z) {  // above the diagonal
+                c[0] = c[1] = 0.f;
+                continue;
+              }
+              const int ri = 2 * rb + z;
+              const float2 d = add2(make_float2(gr[ri], gr[ri]), ngc);
+              const float2 x = mul2(make_float2(c[0], c[1]), make_float2(br[ri], br[ri]));
+              const float2 v = mul2(x, make_float2(exp2f(d.x), exp2f(d.y)));
+              c[0] = v.x;
+              c[1] = v.y;
+              if (rb == cb && h == z) {
+                if (!below0) c[0] = 0.f;
+                if (!below1) c[1] = 0.f;
+              }
+            }
+        }
+      if (valid < CHUNK) {  // rows past the end: whatever their k holds, L is zero there
+#pragma unroll
+        for (int rb = 0; rb < 4; ++rb)
+#pragma unroll
+          for (int cb = 0; cb <= rb; ++cb)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (16 * rb + q8 + 8 * (e >> 1) >= valid) L[rb * (rb + 1) / 2 + cb].c[h][e] = 0.f;
+      }
+    }
+    // ---- 3. inverses of the diagonal blocks
+    // the K tile (single-warp blocks) and the output tile of the head before are dead
+    if (lane == 0) tc::tma_store_wait_read();
+    __syncwarp();
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          const float *lo = L[b * (b + 3) / 2].c[h] + 2 * z, *hi = L[(b + 2) * (b + 5) / 2].c[h] + 2 * z;
+          *reinterpret_cast<float4*>(sD + b * DIAG_STRIDE + (q8 + 8 * z) * LD_DIAG + 16 * h + 4 * t4) =
+              make_float4(lo[0], hi[0], lo[1], hi[1]);
+        }
+    __syncwarp();
+    {
+      const int c = lane & 15;  // column c of the blocks b, b + 2 with b = lane / 16
+      float* d = sD + (lane >> 4) * DIAG_STRIDE;
+      float2 x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float one = i == c ? 1.f : 0.f;
+        float2 s = make_float2(one, one), s1 = make_float2(0.f, 0.f);  // two chains
+#pragma unroll
+        for (int j = 0; j < i; j += 2) {
+          const float4 l = *reinterpret_cast<const float4*>(d + i * LD_DIAG + 2 * j);
+          s = fma2(make_float2(l.x, l.y), x[j], s);
+          if (j + 1 < i) s1 = fma2(make_float2(l.z, l.w), x[j + 1], s1);
+        }
+        x[i] = i > 1 ? add2(s, s1) : s;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 16; ++i) *reinterpret_cast<float2*>(d + i * LD_DIAG + 2 * c) = x[i];
+      __syncwarp();
+    }
+    // D_i and D_j^T as operands, D_i packed for the output
+    Op16 Dop[4], Y[4][4];  // Y[j][i], j <= i: X_ij^T
+    uint32_t dpack[4][4];
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          const float4 v = *reinterpret_cast<const float4*>(sD + b * DIAG_STRIDE + (q8 + 8 * z) * LD_DIAG + 16 * h + 4 * t4);
+          dpack[b][2 * h + z] = pack_bf16(v.x, v.z);
+          dpack[b + 2][2 * h + z] = pack_bf16(v.y, v.w);
+          Dop[b].c[h][2 * z] = to_tf32(v.x);
+          Dop[b].c[h][2 * z + 1] = to_tf32(v.z);
+          Dop[b + 2].c[h][2 * z] = to_tf32(v.y);
+          Dop[b + 2].c[h][2 * z + 1] = to_tf32(v.w);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float2 w = *reinterpret_cast<const float2*>(sD + b * DIAG_STRIDE + (8 * h + 2 * t4 + e) * LD_DIAG + 2 * (q8 + 8 * z));
+            Y[b][b].c[h][2 * z + e] = to_tf32(w.x);
+            Y[b + 2][b + 2].c[h][2 * z + e] = to_tf32(w.y);
+          }
+        }
+    __syncwarp();  // the diagonal blocks have been read: the output tile goes over them
+    // ---- 4. and 5.: blocks below the diagonal, row by row, each stored as soon as it is known
+    const uint32_t out = smem_u32(scratch);
+    const int mtx = lane >> 3;  // stmatrix: this lane addresses row l7 of matrix mtx
+#pragma unroll
+    for (int i = 1; i < 4; ++i) {
+      Op16 Lop[3];
+#pragma unroll
+      for (int kk = 0; kk < i; ++kk) Lop[kk] = to_op(L[i * (i + 1) / 2 + kk]);
+#pragma unroll
+      for (int j = 0; j < i; ++j) {
+        Block16 t, y;
+        mma_abt<false>(t, Y[j][j], Lop[j]);
+#pragma unroll
+        for (int kk = j + 1; kk < i; ++kk) mma_abt<true>(t, Y[j][kk], Lop[kk]);
+        mma_abt<false>(y, to_op(t), Dop[i]);
+        if (i < 3) Y[j][i] = to_op(y);
+        // 8 x 8 matrices (Y rows 8 a, columns 8 h; mtx = 2 h + a) go, transposed, to X rows 8 h,
+        // columns 8 a of the block
+        tc::stmatrix_x4_trans(
+            out + (uint32_t)((16 * i + 8 * (mtx >> 1) + l7) * 128 + (((2 * j + (mtx & 1)) ^ l7) << 4)),
+            pack_bf16(y.c[0][0], y.c[0][1]), pack_bf16(y.c[0][2], y.c[0][3]),
+            pack_bf16(y.c[1][0], y.c[1][1]), pack_bf16(y.c[1][2], y.c[1][3]));
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int z = 0; z < 2; ++z)
+          *reinterpret_cast<uint32_t*>(scratch + (16 * b + q8 + 8 * z) * 128 + (((2 * b + h) ^ q8) << 4) + 4 * t4) =
+              dpack[b][2 * h + z];
+    // blocks above the diagonal: zero (lane: row lane / 2 of the block, 16-byte half lane % 2)
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = i + 1; j < 4; ++j) {
+        const int r = 16 * i + (lane >> 1);
+        *reinterpret_cast<uint4*>(scratch + r * 128 + (((2 * j + (lane & 1)) ^ (r & 7)) << 4)) =
+            make_uint4(0, 0, 0, 0);
+      }
+    if (valid == CHUNK) {
+      tc::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) {
+        tc::tma_store_2d(&map_a, hv * CHUNK, (int)row0, scratch);
+        tc::tma_store_commit();
+      }
     } else {
-      int r = min(tid, valid - 1);
-      sG[tid] = g[(row0 + r) * Hv + hv];
-    }
-  }
-  if (gi == 0) cp_async_wait<0>();
-  __syncthreads();
-
-  // Only the 16 x 16 blocks on and below the diagonal of K K^T are needed (10 of 16); they are
-  // dealt to the four warps 3, 3, 2, 2.  rb = row block, [u0, u0 + NU) = 16-column blocks.
-  auto kkt_blocks = [&](auto nu_tag, auto off_tag, int rb, int u0) {
-    constexpr int NU = decltype(nu_tag)::value;
-    float (&acc)[1][2 * NU][4] = *reinterpret_cast<float (*)[1][2 * NU][4]>(kkt + decltype(off_tag)::value);
-    if (gi == 0) {  // the K tile is gone (the inverse is built over it) once the first head is done
-      zero_acc(acc);
-      warp_gemm<1, 2 * NU, D / 16, false, false>(acc, sK + rb * 16 * LDK, LDK, sK + u0 * 16 * LDK, LDK, lane);
-    }
-#pragma unroll
-    for (int hh = 0; hh < 2; ++hh) {
-      const int r = rb * 16 + (lane >> 2) + hh * 8;
-      const float br = sB[r], gr = sG[r];
-#pragma unroll
-      for (int nt = 0; nt < 2 * NU; ++nt) {
-        const int c = u0 * 16 + nt * 8 + (lane & 3) * 2;  // columns c, c + 1: one 8-byte store
-        const float2 gc = *reinterpret_cast<const float2*>(sG + c);
-        float2 v;
-        v.x = r > c ? br * acc[0][nt][2 * hh] * fast_exp(gr - gc.x) : 0.f;
-        v.y = r > c + 1 ? br * acc[0][nt][2 * hh + 1] * fast_exp(gr - gc.y) : 0.f;
-        *reinterpret_cast<float2*>(sL + r * LDL + c) = v;
+      __syncwarp();
+      for (int i = lane; i < valid * 8; i += 32) {
+        const int r = i >> 3, c = i & 7;
+        *reinterpret_cast<uint4*>(A + ((row0 + r) * Hv + hv) * CHUNK + 8 * c) =
+            *reinterpret_cast<const uint4*>(scratch + r * 128 + ((c ^ (r & 7)) << 4));
       }
     }
-  };
-  if (warp == 0) {
-    kkt_blocks(std::integral_constant<int, 3>{}, std::integral_constant<int, 0>{}, 3, 0);
-  } else if (warp == 1) {
-    kkt_blocks(std::integral_constant<int, 3>{}, std::integral_constant<int, 0>{}, 2, 0);
-  } else if (warp == 2) {
-    kkt_blocks(std::integral_constant<int, 1>{}, std::integral_constant<int, 0>{}, 3, 3);
-    kkt_blocks(std::integral_constant<int, 1>{}, std::integral_constant<int, 8>{}, 0, 0);
-  } else {
-    kkt_blocks(std::integral_constant<int, 2>{}, std::integral_constant<int, 0>{}, 1, 0);
-  }
-  __syncthreads();
-
-  // Inverse of the unit lower-triangular (I + L) by recursive halving:
-  //   [[P, 0], [C, Q]]^-1 = [[P^-1, 0], [-Q^-1 C P^-1, Q^-1]].
-  // The four 16 x 16 diagonal blocks come from forward substitution in fp32 (thread = one column
-  // of one block); the two 16 x 16 and then the one 32 x 32 off-diagonal blocks are two small
-  // products each, on tensor cores with tf32 inputs (round to nearest) and fp32 accumulation.
-  if (tid < CHUNK) {
-    const int b0 = (tid >> 4) * 16, c = tid & 15;
-    float x[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float s = (i == c) ? 1.f : 0.f;
-#pragma unroll
-      for (int jj = 0; jj < i; ++jj) s -= sL[(b0 + i) * LDL + b0 + jj] * x[jj];
-      x[i] = s;
-      sX[(b0 + i) * LDL + b0 + c] = s;
-    }
-  } else {
-    // the 16 x 16 blocks above the diagonal inside each 32 x 32 diagonal block are operands of
-    // the last two products: they must read as zero
-    const int t = tid - CHUNK, blk = t >> 5, r = (t >> 1) & 15, c0 = (t & 1) * 8;
-    float* z = sX + (32 * blk + r) * LDL + 32 * blk + 16 + c0;
-    *reinterpret_cast<float4*>(z) = make_float4(0.f, 0.f, 0.f, 0.f);
-    *reinterpret_cast<float4*>(z + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  __syncthreads();
-  {
-    // 32 x 32 diagonal blocks: pair p covers rows/cols [32p, 32p+32); warp = (pair, 8-column tile pair)
-    const int pr = warp >> 1, bi = 32 * pr + 16, bj = 32 * pr, n0 = 8 * (warp & 1);
-    float* y = sY + pr * 16 * LDY;
-    float c[1][4];
-    tf32_gemm<1, 2>(c, sL + bi * LDL + bj, LDL, sX + bj * LDL + bj + n0, LDL, lane);
-    store_frag<1>(y + n0, LDY, c, 1.f, lane);
-    __syncthreads();
-    tf32_gemm<1, 2>(c, sX + bi * LDL + bi, LDL, y + n0, LDY, lane);
-    store_frag<1>(sX + bi * LDL + bj + n0, LDL, c, -1.f, lane);
-    __syncthreads();
-  }
-  {
-    // the 32 x 32 block below the diagonal: warp = (16-row tile, 16-column half)
-    const int m0 = 16 * (warp >> 1), n0 = 16 * (warp & 1);
-    float c[2][4];
-    tf32_gemm<2, 4>(c, sL + (32 + m0) * LDL, LDL, sX + n0, LDL, lane);
-    store_frag<2>(sY + m0 * LDY + n0, LDY, c, 1.f, lane);
-    __syncthreads();
-    tf32_gemm<2, 4>(c, sX + (32 + m0) * LDL + 32, LDL, sY + n0, LDY, lane);
-    store_frag<2>(sX + (32 + m0) * LDL + n0, LDL, c, -1.f, lane);
-    __syncthreads();
-  }
-  // bf16 rows out, 16 bytes per store; blocks above the diagonal are zero
-  for (int i = tid; i < CHUNK * 8; i += 128) {
-    const int r = i >> 3, c0 = (i & 7) * 8;
-    if (r < valid) {
-      uint4 pk = make_uint4(0, 0, 0, 0);
-      if ((c0 >> 4) <= (r >> 4)) {
-        const float* xr = sX + r * LDL + c0;
-        pk = make_uint4(pack_bf16(xr[0], xr[1]), pack_bf16(xr[2], xr[3]), pack_bf16(xr[4], xr[5]),
-                        pack_bf16(xr[6], xr[7]));
-      }
-      *reinterpret_cast<uint4*>(A + ((row0 + r) * Hv + hv) * CHUNK + c0) = pk;
-    }
-  }
-  }  // value heads of the group
+  }  // value heads of this warp
+  if (lane == 0) tc::tma_store_wait_read();  // shared memory outlives the stores' reads
+  if (!ok && lane == 0) atomicCAS(&g_kkt_status, 0, 1);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -302,6 +504,18 @@ __global__ void group_reduce_kernel(const bf16* __restrict__ in, bf16* __restric
   *reinterpret_cast<uint4*>(out + i * 8) = res;
 }
 
+int kkt_status(int* out, int reset) {
+  int v = 0;
+  cudaError_t e = cudaMemcpyFromSymbol(&v, g_kkt_status, sizeof(int));
+  if (e != cudaSuccess) return (int)e;
+  *out = v;
+  if (reset && v != 0) {
+    int z = 0;
+    e = cudaMemcpyToSymbol(g_kkt_status, &z, sizeof(int));
+  }
+  return (int)e;
+}
+
 }  // namespace fqla
 
 using namespace fqla;
@@ -322,14 +536,17 @@ extern "C" int fqla_chunk_local_cumsum(const float* g, float* out, int B, int T,
 template <int D>
 static int launch_kkt(const void* k, const void* beta, int beta_is_f32, const float* g,
                       float* g_cum_out, void* A, int Hq, int Hv, SeqLayout lay, IndexTable ci,
-                      long long n, cudaStream_t st) {
-  constexpr int k_tile = CHUNK * (D + 8) * 2, x_tile = CHUNK * (CHUNK + 4) * 4;
-  constexpr int smem = (k_tile > x_tile ? k_tile : x_tile) + x_tile + 2 * CHUNK * 4;
+                      long long n, long long T_rows, cudaStream_t st) {
+  const int G = Hv / Hq, warps = G < kkt::MAX_WARPS ? G : kkt::MAX_WARPS;
   static std::atomic<unsigned long long> done;
-  int rc = configure_smem((const void*)kkt_solve_kernel<D>, smem, done);
+  int rc = configure_smem((const void*)kkt_solve_kernel<D>, kkt::smem_bytes<D>(kkt::MAX_WARPS), done);
   if (rc != 0) return rc;
-  return launch_pdl(kkt_solve_kernel<D>, dim3((unsigned)n, Hq), dim3(128), (size_t)smem, st, (const bf16*)k,
-                    beta, beta_is_f32, g, g_cum_out, (bf16*)A, Hq, Hv, lay, ci);
+  CUtensorMap mk, ma;
+  if ((rc = make_tile_map(&mk, k, T_rows, (long long)Hq * D, 64))) return rc;
+  if ((rc = make_tile_map(&ma, A, T_rows, (long long)Hv * CHUNK, 64))) return rc;
+  return launch_pdl(kkt_solve_kernel<D>, dim3((unsigned)n, Hq), dim3(32 * warps),
+                    (size_t)kkt::smem_bytes<D>(warps), st, beta, beta_is_f32, g, g_cum_out, (bf16*)A, Hq, Hv,
+                    lay, ci, mk, ma);
 }
 
 extern "C" int fqla_kkt_solve(const void* k, const void* beta, int beta_is_f32,
@@ -344,8 +561,8 @@ extern "C" int fqla_kkt_solve(const void* k, const void* beta, int beta_is_f32,
   long long n = cu_seqlens ? num_chunks : (long long)B * ((T + CHUNK - 1) / CHUNK);
   if (n <= 0) return FQLA_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (D == 128) return launch_kkt<128>(k, beta, beta_is_f32, g_cum, g_cum_out, A, Hq, Hv, lay, ci, n, st);
-  if (D == 64) return launch_kkt<64>(k, beta, beta_is_f32, g_cum, g_cum_out, A, Hq, Hv, lay, ci, n, st);
+  if (D == 128) return launch_kkt<128>(k, beta, beta_is_f32, g_cum, g_cum_out, A, Hq, Hv, lay, ci, n, (long long)B * T, st);
+  if (D == 64) return launch_kkt<64>(k, beta, beta_is_f32, g_cum, g_cum_out, A, Hq, Hv, lay, ci, n, (long long)B * T, st);
   return FQLA_ERR_UNSUPPORTED_DIM;
 }
 
