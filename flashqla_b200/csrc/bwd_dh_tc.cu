@@ -315,8 +315,9 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       mbar_arrive(&bars[W_READY]);
       return true;
     };
-    if (n_it > 0) ok = convert_w(0);
-    for (int it = 0; it < n_it && ok; ++it) {
+#pragma unroll 1
+    for (int it = -1; it < n_it && ok; ++it) {  // it = -1: only w of the first iteration
+     if (it >= 0) {
       const int c = n_it - 1 - it;
       const long long row0 = sp.bos + (long long)c * CHUNK;
       const int valid = min(CHUNK, len_ext - c * CHUNK);
@@ -356,6 +357,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
               p.du[((row0 + 32 * h + j) * p.Hv + hv) * D + v] = __float2bfloat16(x[j]);
         }
       }
+     }
       if (it + 1 < n_it) ok = convert_w(it + 1);
     }
   } else if (warp >= 12) {
@@ -396,93 +398,90 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     }
   } else if (warp == 0) {
     // =============================== MMA issuer ===============================
-    if (lane == 0) {
-      constexpr uint32_t ID_P = idesc_bf16(64, 64, 0, 0);
-      constexpr uint32_t ID_X1 = idesc_bf16(128, 64, 0, 0);
-      constexpr uint32_t ID_X2 = idesc_bf16(128, 64, 1, 1);
-      constexpr uint32_t ID_W = idesc_bf16(64, 128, 0, 1);
-      constexpr uint32_t ID_UPD_W = idesc_bf16(128, 128, 0, 1) | (1u << 13);  // A negated
-      constexpr uint32_t ID_UPD_Q = idesc_bf16(128, 128, 1, 1);
-      const uint32_t st_lo = desc_lo_kmajor(smem + OFF_ST), dvt_lo = desc_lo_kmajor(smem + OFF_DVT);
-      const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 8192), pmn_lo = desc_lo_mnmajor(smem + OFF_P, 8192);
-      const uint32_t app_lo = desc_lo_kmajor(smem + OFF_APP);
-      const uint32_t qsmn_lo = desc_lo_mnmajor(smem + OFF_QS, 8192);
-      const uint32_t q0_lo = desc_lo_kmajor(smem + OFF_STAGE);
-      const uint32_t k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE);
-      const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE, 8192);
-      const uint32_t domn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + 2 * TILE, 8192);
-      constexpr uint32_t STAGE_LO = STAGE_BYTES >> 4;
-      auto issue_w = [&](uint32_t so) {
-        umma_group<4, 2, 0, 128, 0, false>(tmem + TM_W, app_lo, kmn0_lo + so, ID_W);
-        umma_commit(&bars[W_DONE]);
-      };
-      auto issue_p = [&](uint32_t so) {
-        umma_group<8, 2, 512, 2, 512, false>(tmem + TM_P, q0_lo + so, k0_lo + so, ID_P);
-        umma_commit(&bars[P_DONE]);
-      };
-      auto issue_x2 = [&](uint32_t so) {
-        umma_group<4, 128, 0, 128, 0, false>(tmem + TM_X2, domn0_lo + so, pmn_lo, ID_X2);
-        umma_commit(&bars[X2_DONE]);
-      };
-      for (int it = 0; it < n_it && ok; ++it) {
-        const int s = it & 1;
-        const uint32_t so = s ? STAGE_LO : 0u, so_next = s ? 0u : STAGE_LO;
-        if (it == 0) {
-          ok = WAIT(FULL0, 0) && WAIT(AP_READY, 0);
-          if (!ok) break;
-          tc_fence_after();
-          issue_w(0);
-          issue_p(0);
-          ok = WAIT(P_READY, 0);
-          if (!ok) break;
-          tc_fence_after();
-          issue_x2(0);
-        }
-        ok = WAIT(S_COPY, it & 1);
+    // (the warp stays converged; see elect_one in tc05.cuh)
+    constexpr uint32_t ID_P = idesc_bf16(64, 64, 0, 0);
+    constexpr uint32_t ID_X1 = idesc_bf16(128, 64, 0, 0);
+    constexpr uint32_t ID_X2 = idesc_bf16(128, 64, 1, 1);
+    constexpr uint32_t ID_W = idesc_bf16(64, 128, 0, 1);
+    constexpr uint32_t ID_UPD_W = idesc_bf16(128, 128, 0, 1) | (1u << 13);  // A negated
+    constexpr uint32_t ID_UPD_Q = idesc_bf16(128, 128, 1, 1);
+    const uint32_t st_lo = desc_lo_kmajor(smem + OFF_ST), dvt_lo = desc_lo_kmajor(smem + OFF_DVT);
+    const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 8192), pmn_lo = desc_lo_mnmajor(smem + OFF_P, 8192);
+    const uint32_t app_lo = desc_lo_kmajor(smem + OFF_APP);
+    const uint32_t qsmn_lo = desc_lo_mnmajor(smem + OFF_QS, 8192);
+    const uint32_t q0_lo = desc_lo_kmajor(smem + OFF_STAGE);
+    const uint32_t k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE);
+    const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE, 8192);
+    const uint32_t domn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + 2 * TILE, 8192);
+    constexpr uint32_t STAGE_LO = STAGE_BYTES >> 4;
+    auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
+#pragma unroll 1
+    for (int it = -1; it < n_it && ok; ++it) {  // it = -1: only what prepares the first iteration
+      const int s = it & 1;
+      const uint32_t so = s ? STAGE_LO : 0u, so_next = s ? 0u : STAGE_LO;
+      const int y_tile = (int)(((sp.chunk_base + (n_it - 1 - it)) * p.Hv + hv) * D);
+      if (it >= 0) {
+        ok = WAITW(S_COPY, it & 1);
         if (!ok) break;
         tc_fence_after();
-        // X1^T = dS^T K^T   (on the chain)
-        umma_group<8, 2, 1024, 2, 512, false>(tmem + TM_X1, st_lo, k0_lo + so, ID_X1);
-        tma_store_wait_read();  // du^T of the chunk before has left its tile
-        umma_commit(&bars[X1_DONE]);
-        const int y_tile = (int)(((sp.chunk_base + (n_it - 1 - it)) * p.Hv + hv) * D);
-        if (p.tiled && p.dh && it >= lead) {  // the operand copy of dS^T is dh of this chunk
-          tma_store_2d(&map_dh, 0, y_tile, smem + OFF_ST);
-          tma_store_2d(&map_dh, 64, y_tile, smem + OFF_ST + 16384);
-          tma_store_commit();
-        }
-        if (it + 1 < n_it) {
-          ok = WAIT(FULL0 + (s ^ 1), ((it + 1) >> 1) & 1);
-          if (!ok) break;
-          issue_p(so_next);  // the Pg group has read P of this chunk (P_READY waited below/earlier)
-        }
-        ok = WAIT(W_READY, it & 1) && WAIT(QS_READY, it & 1) && WAIT(S_DEC, it & 1) &&
-             WAIT(DV_READY, it & 1);
-        if (!ok) break;
-        tc_fence_after();
-        // dS^T <- dS^T - dv^T w + dO^T (scale gamma q)
-        umma_group<4, 2, 0, 128, 0, true>(tmem + TM_S, dvt_lo, wmn_lo, ID_UPD_W);
-        umma_group<4, 128, 0, 128, 0, true>(tmem + TM_S, domn0_lo + so, qsmn_lo, ID_UPD_Q);
-        tma_store_wait_read();  // the dS^T tile may be rewritten after this
-        umma_commit(&bars[S_DONE]);
-        if (p.tiled && p.du && it >= lead) {
-          tma_store_2d(&map_du, 0, y_tile, smem + OFF_DVT);
-          tma_store_commit();
-        }
-        umma_commit(&bars[EMPTY0 + s]);
-        if (it + 1 < n_it) {
-          ok = WAIT(AP_READY, (it + 1) & 1);
-          if (!ok) break;
-          tc_fence_after();
-          issue_w(so_next);
-          ok = WAIT(P_READY, (it + 1) & 1);
-          if (!ok) break;
-          tc_fence_after();
-          issue_x2(so_next);
+        if (elect_one()) {
+          // X1^T = dS^T K^T   (on the chain)
+          umma_group<8, 2, 1024, 2, 512, false>(tmem + TM_X1, st_lo, k0_lo + so, ID_X1);
+          tma_store_wait_read();  // du^T of the chunk before has left its tile
+          umma_commit(&bars[X1_DONE]);
+          if (p.tiled && p.dh && it >= lead) {  // the operand copy of dS^T is dh of this chunk
+            tma_store_2d(&map_dh, 0, y_tile, smem + OFF_ST);
+            tma_store_2d(&map_dh, 64, y_tile, smem + OFF_ST + 16384);
+            tma_store_commit();
+          }
         }
       }
-      tma_store_wait_all();
+      if (it + 1 < n_it) {
+        // (the Pg group has read P of this chunk: P_READY was waited for an iteration ago)
+        ok = WAITW(FULL0 + (s ^ 1), ((it + 1) >> 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          umma_group<8, 2, 512, 2, 512, false>(tmem + TM_P, q0_lo + so_next, k0_lo + so_next, ID_P);
+          umma_commit(&bars[P_DONE]);
+        }
+      }
+      if (it >= 0) {
+        ok = WAITW(W_READY, it & 1) && WAITW(QS_READY, it & 1) && WAITW(S_DEC, it & 1) &&
+             WAITW(DV_READY, it & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          // dS^T <- dS^T - dv^T w + dO^T (scale gamma q)
+          umma_group<4, 2, 0, 128, 0, true>(tmem + TM_S, dvt_lo, wmn_lo, ID_UPD_W);
+          umma_group<4, 128, 0, 128, 0, true>(tmem + TM_S, domn0_lo + so, qsmn_lo, ID_UPD_Q);
+          tma_store_wait_read();  // the dS^T tile may be rewritten after this
+          umma_commit(&bars[S_DONE]);
+          if (p.tiled && p.du && it >= lead) {
+            tma_store_2d(&map_du, 0, y_tile, smem + OFF_DVT);
+            tma_store_commit();
+          }
+          umma_commit(&bars[EMPTY0 + s]);
+        }
+      }
+      if (it + 1 < n_it) {
+        ok = WAITW(AP_READY, (it + 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          umma_group<4, 2, 0, 128, 0, false>(tmem + TM_W, app_lo, kmn0_lo + so_next, ID_W);
+          umma_commit(&bars[W_DONE]);
+        }
+        ok = WAITW(P_READY, (it + 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          umma_group<4, 128, 0, 128, 0, false>(tmem + TM_X2, domn0_lo + so_next, pmn_lo, ID_X2);
+          umma_commit(&bars[X2_DONE]);
+        }
+      }
     }
+    if (elect_one()) tma_store_wait_all();
   } else if (warp == 1) {
     // =============================== producer ===============================
     float g_r[2] = {0.f, 0.f}, b_r[2] = {0.f, 0.f}, gl_r = 0.f;
@@ -498,89 +497,83 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         b_r[z] = r < valid ? load_beta(p.beta, p.beta_is_f32, (row0 + r) * p.Hv + hv) : 0.f;
       }
     };
-    // vectors and A tile of the chunk of iteration j (its stage's A buffer is free once the
-    // scaling warps have read it)
-    auto a_part = [&](int j) {
-      const int sj = j & 1, c = n_it - 1 - j;
-      const long long row0 = sp.bos + (long long)c * CHUNK;
-      const int valid = min(CHUNK, len_ext - c * CHUNK);
-      if (j >= 2 && !WAIT(EMPTYA0 + sj, ((j >> 1) - 1) & 1)) return false;
-      float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
-#pragma unroll
-      for (int z = 0; z < 2; ++z) {
-        int r = 2 * lane + z;
-        float gam = fast_exp(g_r[z]);
-        vs[V_G * CHUNK + r] = g_r[z];
-        vs[V_BG * CHUNK + r] = b_r[z] * gam;
-        vs[V_RHO * CHUNK + r] = fast_exp(gl_r - g_r[z]);
-        vs[V_SGAM * CHUNK + r] = p.scale * gam;
-      }
-      if (lane == 0) vs[V_GL * CHUNK] = fast_exp(gl_r);
+    auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
+    // zero the rows past the sequence end in n 8 KB blocks of 64 rows, then hand the tile on
+    auto zero_rows = [&](unsigned char* base, int n, int valid, uint64_t* full) {
+#pragma unroll 1
+      for (int i = lane; i < n * 512; i += 32)
+        if (((i >> 3) & 63) >= valid) *reinterpret_cast<uint4*>(base + i * 16) = make_uint4(0, 0, 0, 0);
+      fence_proxy_async();
       __syncwarp();
-      unsigned char* dst = smem + OFF_STAGE + sj * STAGE_BYTES + 3 * TILE;
-      const bool partial = valid < CHUNK;
-      uint64_t* bar = partial ? &bars[PRIVA] : &bars[FULLA0 + sj];
-      if (lane == 0) {
-        mbar_arrive_expect_tx(bar, TILE_A);
-        tma_load_2d(dst, &map_a, hv * CHUNK, (int)row0, bar);
-      }
-      if (partial) {
-        // only the last chunk of a sequence (the first one walked) can be partial: used once
-        if (!WAIT(PRIVA, 0)) return false;
-        for (int i = lane; i < (CHUNK - valid) * 8; i += 32)
-          *reinterpret_cast<uint4*>(dst + (valid + (i >> 3)) * 128 + ((i & 7) << 4)) = make_uint4(0, 0, 0, 0);
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[FULLA0 + sj]);
-      }
-      return true;
+      if (lane == 0) mbar_arrive(full);
     };
-    if (n_it > 0) {
-      fetch(0);
-      ok = a_part(0);
-      if (n_it > 1) fetch(1);
-    }
-    for (int it = 0; it < n_it && ok; ++it) {
-      const int s = it & 1, c = n_it - 1 - it;
-      const long long row0 = sp.bos + (long long)c * CHUNK;
-      const int valid = min(CHUNK, len_ext - c * CHUNK);
-      if (it >= 2) {
-        ok = WAIT(EMPTY0 + s, ((it >> 1) - 1) & 1);
-        if (!ok) break;
-      }
-      unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
-      const bool partial = valid < CHUNK;
-      uint64_t* bar = partial ? &bars[PRIV] : &bars[FULL0 + s];
-      if (lane == 0) {
-        mbar_arrive_expect_tx(bar, STAGE_BYTES - TILE_A);
-        const int y = (int)row0;
-        tma_load_2d(st + TILE, &map_k, hq * D, y, bar);
-        tma_load_2d(st + TILE + 8192, &map_k, hq * D + 64, y, bar);
-        tma_load_2d(st, &map_q, hq * D, y, bar);
-        tma_load_2d(st + 8192, &map_q, hq * D + 64, y, bar);
-        tma_load_2d(st + 2 * TILE, &map_do, hv * D, y, bar);
-        tma_load_2d(st + 2 * TILE + 8192, &map_do, hv * D + 64, y, bar);
-      }
-      if (partial) {
-        ok = WAIT(PRIV, 0);
-        if (!ok) break;
-        for (int blk = 0; blk < 6; ++blk) {
-          unsigned char* base = st + blk * 8192;
-          for (int i = lane; i < (CHUNK - valid) * 8; i += 32)
-            *reinterpret_cast<uint4*>(base + (valid + (i >> 3)) * 128 + ((i & 7) << 4)) =
-                make_uint4(0, 0, 0, 0);
+    // As in fwd_tc.cu: q, k, dO of iteration it; vectors and A tile of iteration it + 1; the gates of
+    // iteration it + 2 into registers.  Slot (it + 1) % 4 of the vectors was last read for iteration
+    // it - 3, which the wait on the stage of iteration it - 2 has seen finished.
+#pragma unroll 1
+    for (int it = -2; it < n_it && ok; ++it) {
+      if (it >= 0) {
+        const int s = it & 1, c = n_it - 1 - it;
+        const int y = (int)(sp.bos + (long long)c * CHUNK);
+        const int valid = min(CHUNK, len_ext - c * CHUNK);
+        const bool partial = valid < CHUNK;
+        if (it >= 2) {
+          ok = WAITW(EMPTY0 + s, ((it >> 1) - 1) & 1);
+          if (!ok) break;
         }
-        fence_proxy_async();
+        unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
+        uint64_t* bar = &bars[partial ? PRIV : FULL0 + s];
+        if (elect_one()) {
+          mbar_arrive_expect_tx(bar, STAGE_BYTES - TILE_A);
+          tma_load_2d(st + TILE, &map_k, hq * D, y, bar);
+          tma_load_2d(st + TILE + 8192, &map_k, hq * D + 64, y, bar);
+          tma_load_2d(st, &map_q, hq * D, y, bar);
+          tma_load_2d(st + 8192, &map_q, hq * D + 64, y, bar);
+          tma_load_2d(st + 2 * TILE, &map_do, hv * D, y, bar);
+          tma_load_2d(st + 2 * TILE + 8192, &map_do, hv * D + 64, y, bar);
+        }
+        if (partial) {
+          ok = WAITW(PRIV, 0);
+          if (!ok) break;
+          zero_rows(st, 6, valid, &bars[FULL0 + s]);
+        }
+      }
+      const int j = it + 1;
+      if (j >= 0 && j < n_it) {
+        const int sj = j & 1, c = n_it - 1 - j;
+        const int valid = min(CHUNK, len_ext - c * CHUNK);
+        const bool partial = valid < CHUNK;
+        // the stage's A buffer is free once the scaling warps have read it
+        if (j >= 2) {
+          ok = WAITW(EMPTYA0 + sj, ((j >> 1) - 1) & 1);
+          if (!ok) break;
+        }
+        float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          int r = 2 * lane + z;
+          float gam = fast_exp(g_r[z]);
+          vs[V_G * CHUNK + r] = g_r[z];
+          vs[V_BG * CHUNK + r] = b_r[z] * gam;
+          vs[V_RHO * CHUNK + r] = fast_exp(gl_r - g_r[z]);
+          vs[V_SGAM * CHUNK + r] = p.scale * gam;
+        }
+        if (lane == 0) vs[V_GL * CHUNK] = fast_exp(gl_r);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[FULL0 + s]);
+        unsigned char* dst = smem + OFF_STAGE + sj * STAGE_BYTES + 3 * TILE;
+        uint64_t* bar = &bars[partial ? PRIVA : FULLA0 + sj];
+        if (elect_one()) {
+          mbar_arrive_expect_tx(bar, TILE_A);
+          tma_load_2d(dst, &map_a, hv * CHUNK, (int)(sp.bos + (long long)c * CHUNK), bar);
+        }
+        if (partial) {
+          // only the last chunk of a sequence (the first one walked) can be partial: used once
+          ok = WAITW(PRIVA, 0);
+          if (!ok) break;
+          zero_rows(dst, 1, valid, &bars[FULLA0 + sj]);
+        }
       }
-      // the next chunk's vectors and A tile go out a whole chunk before its q, k, dO; slot
-      // (it + 1) % 4 of the vectors was last read for the chunk of iteration it - 3, which the wait
-      // on the stage of iteration it - 2 above has seen finished
-      if (it + 1 < n_it) {
-        ok = a_part(it + 1);
-        if (ok && it + 2 < n_it) fetch(it + 2);
-      }
+      if (it + 2 < n_it) fetch(it + 2);
     }
   } else {
     // =============================== scaling warps (2, 3) ===============================

@@ -158,19 +158,28 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
     long long row0, chunk_id;
     int valid, hv, hq;
   };
-  auto decode = [&](long long w) {
+  // item w = (chunk w / Hv, head w % Hv); a CTA steps by gridDim.x items: no division per item
+  const int step_c = (int)gridDim.x / p.Hv, step_h = (int)gridDim.x % p.Hv, group = p.Hv / p.Hq;
+  auto advance = [&](int& cidx, int& hv) {
+    cidx += step_c;
+    hv += step_h;
+    if (hv >= p.Hv) {
+      hv -= p.Hv;
+      ++cidx;
+    }
+  };
+  auto decode = [&](int cidx, int hv) {
     Item t;
-    const long long cidx = w / p.Hv;
-    t.hv = (int)(w % p.Hv);
-    t.hq = t.hv / (p.Hv / p.Hq);
+    t.hv = hv;
+    t.hq = hv / group;
     int seq, ci;
     if (p.lay.cu.ptr) {
       seq = (int)p.chunk_indices[2 * cidx];
       ci = (int)p.chunk_indices[2 * cidx + 1];
     } else {
       const int per = (p.lay.T + CHUNK - 1) / CHUNK;
-      seq = (int)(cidx / per);
-      ci = (int)(cidx % per);
+      seq = cidx / per;
+      ci = cidx % per;
     }
     const SeqSpan sp = p.lay.span(seq);
     t.row0 = sp.bos + (long long)ci * CHUNK;
@@ -200,9 +209,12 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 
   if (warp == N_EPI / 32) {
     // ====================== issue warp: TMA loads and every tcgen05.mma ======================
-    if (lane == 0) {
+    // (the warp stays converged; see elect_one in tc05.cuh)
+    {
+      auto WAIT = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
       auto load_a = [&](const Item& t, int kbuf) {
         const int y = (int)t.row0, ys = (int)((t.chunk_id * p.Hv + t.hv) * D);
+        if (!elect_one()) return;
         mbar_arrive_expect_tx(&bars[L_A], TX_A);
         tma_load_2d(smem + OFF_DU - ROW_TILE, &map_do, t.hv * D, y, &bars[L_A]);  // = OFF_DO
         tma_load_2d(smem + OFF_DO + 8192, &map_do, t.hv * D + 64, y, &bars[L_A]);
@@ -221,6 +233,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       };
       auto load_b = [&](const Item& t) {
         const int y = (int)t.row0;
+        if (!elect_one()) return;
         mbar_arrive_expect_tx(&bars[L_B], TX_B);
         if constexpr (TILED) {
           tma_load_2d(smem + OFF_DU, &map_du, 0, (int)((t.chunk_id * p.Hv + t.hv) * D), &bars[L_B]);
@@ -234,6 +247,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         tma_load_2d(smem + OFF_V + 8192, &map_v, t.hv * D + 64, y, &bars[L_B]);
       };
       auto load_c = [&](const Item& t) {
+        if (!elect_one()) return;
         mbar_arrive_expect_tx(&bars[L_C], TX_C);
         tma_load_2d(smem + OFF_A, &map_a, t.hv * CHUNK, (int)t.row0, &bars[L_C]);
       };
@@ -260,7 +274,8 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       constexpr uint32_t ID_MK_128 = idesc_bf16(64, 128, 1, 0);
       constexpr uint32_t KBUF_LO = ROW_TILE >> 4;
 
-      Item cur = decode(blockIdx.x);
+      int at_c = (int)blockIdx.x / p.Hv, at_h = (int)blockIdx.x % p.Hv;
+      Item cur = decode(at_c, at_h);
       load_a(cur, 0);
       load_b(cur);
       load_c(cur);
@@ -271,7 +286,10 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         const uint32_t ph = it & 1;
         const bool has_next = w + gridDim.x < total;
         Item nxt = cur;
-        if (has_next) nxt = decode(w + gridDim.x);
+        if (has_next) {
+          advance(at_c, at_h);
+          nxt = decode(at_c, at_h);
+        }
         const uint32_t k_lo = k_lo0 + (ph ? KBUF_LO : 0u), kmn_lo = kmn_lo0 + (ph ? KBUF_LO : 0u);
         // the read-out warps have finished the previous item (accumulators free) and have zeroed
         // the rows past the sequence end in this item's tiles (which also means: tiles landed)
@@ -284,43 +302,49 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         if (!ok) break;
         tc_fence_after();
         // ---- products that need only loaded tiles ----
-        if constexpr (TILED) {
-          umma_group<8, 128, 512, 128, 512, false>(tmem + T_DW, duT_lo, hT_lo, ID_MM_128);
-        } else {
-          umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DW, du_lo, h_lo, ID_KK_128);
+        if (elect_one()) {
+          if constexpr (TILED) {
+            umma_group<8, 128, 512, 128, 512, false>(tmem + T_DW, duT_lo, hT_lo, ID_MM_128);
+          } else {
+            umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DW, du_lo, h_lo, ID_KK_128);
+          }
+          umma_commit(&bars[C_DW]);
+          if constexpr (TILED) {
+            umma_group<8, 2, 512, 128, 512, false>(tmem + T_DS, do_lo, vnT_lo, ID_KM_64);
+          } else {
+            umma_group<8, 2, 512, 2, 512, false>(tmem + T_DS, do_lo, vn_lo, ID_KK_64);
+          }
+          umma_group<8, 2, 512, 2, 512, false>(tmem + T_QK, q_lo, k_lo, ID_KK_64);
+          umma_commit(&bars[C_DSQK]);
         }
-        umma_commit(&bars[C_DW]);
-        if constexpr (TILED) {
-          umma_group<8, 2, 512, 128, 512, false>(tmem + T_DS, do_lo, vnT_lo, ID_KM_64);
-        } else {
-          umma_group<8, 2, 512, 2, 512, false>(tmem + T_DS, do_lo, vn_lo, ID_KK_64);
-        }
-        umma_group<8, 2, 512, 2, 512, false>(tmem + T_QK, q_lo, k_lo, ID_KK_64);
-        umma_commit(&bars[C_DSQK]);
         // ---- dw is an operand now: the pieces of dA, and A^T dw, A^T du ----
         ok = WAIT(R_DW, ph);
         if (!ok) break;
         tc_fence_after();
-        umma_group<8, 2, 512, 2, 512, false>(tmem + T_X1, dw_lo, k_lo, ID_KK_64);
-        if constexpr (TILED) umma_group<8, 128, 512, 2, 512, false>(tmem + T_X2, duT_lo, v_lo, ID_MK_64);
-        else umma_group<8, 2, 512, 2, 512, false>(tmem + T_X2, du_lo, v_lo, ID_KK_64);
-        umma_commit(&bars[C_X]);
-        // products off the dependent chain go behind the ones the read-out is waiting for
-        if constexpr (TILED) {
-          umma_group<8, 2, 512, 128, 512, false>(tmem + T_DQ1, do_lo, hT_lo, ID_KM_128);
-          umma_group<8, 128, 512, 128, 512, false>(tmem + T_DK1, vnT_lo, dhT_lo, ID_MM_128);
-        } else {
-          umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DQ1, do_lo, h_lo, ID_KK_128);
-          umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DK1, vn_lo, dh_lo, ID_KK_128);
+        if (elect_one()) {
+          umma_group<8, 2, 512, 2, 512, false>(tmem + T_X1, dw_lo, k_lo, ID_KK_64);
+          if constexpr (TILED) umma_group<8, 128, 512, 2, 512, false>(tmem + T_X2, duT_lo, v_lo, ID_MK_64);
+          else umma_group<8, 2, 512, 2, 512, false>(tmem + T_X2, du_lo, v_lo, ID_KK_64);
+          umma_commit(&bars[C_X]);
+          // products off the dependent chain go behind the ones the read-out is waiting for
+          if constexpr (TILED) {
+            umma_group<8, 2, 512, 128, 512, false>(tmem + T_DQ1, do_lo, hT_lo, ID_KM_128);
+            umma_group<8, 128, 512, 128, 512, false>(tmem + T_DK1, vnT_lo, dhT_lo, ID_MM_128);
+          } else {
+            umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DQ1, do_lo, h_lo, ID_KK_128);
+            umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DK1, vn_lo, dh_lo, ID_KK_128);
+          }
+          umma_commit(&bars[C_1B]);
         }
-        umma_commit(&bars[C_1B]);
         // ---- ds is an operand now ----
         ok = WAIT(R_DS, ph);
         if (!ok) break;
         tc_fence_after();
-        umma_group<4, 2, 0, 128, 0, false>(tmem + T_DQ2, ds_lo, kmn_lo, ID_KM_128);
-        umma_group<4, 128, 0, 128, 0, false>(tmem + T_DK2, dsmn_lo, qmn_lo, ID_MM_128);
-        umma_group<8, 2, 512, 2, 512, false>(tmem + T_KK, k_lo, k_lo, ID_KK_64);  // qk has been read
+        if (elect_one()) {
+          umma_group<4, 2, 0, 128, 0, false>(tmem + T_DQ2, ds_lo, kmn_lo, ID_KM_128);
+          umma_group<4, 128, 0, 128, 0, false>(tmem + T_DK2, dsmn_lo, qmn_lo, ID_MM_128);
+          umma_group<8, 2, 512, 2, 512, false>(tmem + T_KK, k_lo, k_lo, ID_KK_64);  // qk has been read
+        }
         // h, dh, dO, v_new are dead once the first products are complete and the h.dh sum is done
         if (has_next) {
           ok = WAIT(C_1B, ph) && WAIT(R_HD, ph);
@@ -331,20 +355,24 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         ok = WAIT(R_DA, ph);
         if (!ok) break;
         tc_fence_after();
-        umma_group<4, 128, 0, 128, 0, false>(tmem + T_T, amn_lo, damn_lo, ID_MM_64);
-        umma_commit(&bars[C_T]);
-        // with A' = A diag(beta) and A'' = A diag(beta gamma) (written over the dead v tile):
-        // dk += A''^T dw (onto ds^T q), dv = A'^T du -- the row scalings ride on the operands
-        umma_group<4, 128, 0, 128, 0, true>(tmem + T_DK2, a2mn_lo, dwmn_lo, ID_MM_128);
-        if constexpr (TILED) umma_group<4, 128, 0, 2, 0, false>(tmem + T_T2, a1mn_lo, du_lo, ID_MK_128);
-        else umma_group<4, 128, 0, 128, 0, false>(tmem + T_T2, a1mn_lo, dumn_lo, ID_MM_128);
-        umma_commit(&bars[C_2B]);
+        if (elect_one()) {
+          umma_group<4, 128, 0, 128, 0, false>(tmem + T_T, amn_lo, damn_lo, ID_MM_64);
+          umma_commit(&bars[C_T]);
+          // with A' = A diag(beta) and A'' = A diag(beta gamma) (written over the dead v tile):
+          // dk += A''^T dw (onto ds^T q), dv = A'^T du -- the row scalings ride on the operands
+          umma_group<4, 128, 0, 128, 0, true>(tmem + T_DK2, a2mn_lo, dwmn_lo, ID_MM_128);
+          if constexpr (TILED) umma_group<4, 128, 0, 2, 0, false>(tmem + T_T2, a1mn_lo, du_lo, ID_MK_128);
+          else umma_group<4, 128, 0, 128, 0, false>(tmem + T_T2, a1mn_lo, dumn_lo, ID_MM_128);
+          umma_commit(&bars[C_2B]);
+        }
         // ---- T -> d3 = T A^T ----
         ok = WAIT(R_T, ph);
         if (!ok) break;
         tc_fence_after();
-        umma_group<4, 2, 0, 2, 0, false>(tmem + T_D3, da_lo, a_lo, ID_KK_64);
-        umma_commit(&bars[C_D3]);
+        if (elect_one()) {
+          umma_group<4, 2, 0, 2, 0, false>(tmem + T_D3, da_lo, a_lo, ID_KK_64);
+          umma_commit(&bars[C_D3]);
+        }
         // The bulk group is past its first read-out (always waited for: its threads combine the
         // partial sums of the previous item before that, and the last products of this item let
         // the group overwrite those sums).
@@ -364,9 +392,11 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         if (!ok) break;
         tc_fence_after();
         // dk += (beta dA3) K + (beta dA3)^T K, onto the same accumulator
-        umma_group<4, 2, 0, 128, 0, true>(tmem + T_DK2, ds_lo, kmn_lo, ID_KM_128);
-        umma_group<4, 128, 0, 128, 0, true>(tmem + T_DK2, dsmn_lo, kmn_lo, ID_MM_128);
-        umma_commit(&bars[C_5]);
+        if (elect_one()) {
+          umma_group<4, 2, 0, 128, 0, true>(tmem + T_DK2, ds_lo, kmn_lo, ID_KM_128);
+          umma_group<4, 128, 0, 128, 0, true>(tmem + T_DK2, dsmn_lo, kmn_lo, ID_MM_128);
+          umma_commit(&bars[C_5]);
+        }
         cur = nxt;
       }
       if (!ok) *abort_flag = 1;
@@ -505,7 +535,8 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         else reinterpret_cast<float*>(p.db)[i] = dbv;
       }
     };
-    Item cur = decode(blockIdx.x);
+    int at_c = (int)blockIdx.x / p.Hv, at_h = (int)blockIdx.x % p.Hv;
+    Item cur = decode(at_c, at_h);
     long long prev_first = 0;
     int prev_rows = 0;
     fetch_vectors(cur);
@@ -518,7 +549,10 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       const uint32_t ph = it & 1;
       const bool has_next = w + gridDim.x < total;
       Item nxt = cur;
-      if (has_next) nxt = decode(w + gridDim.x);
+      if (has_next) {
+        advance(at_c, at_h);
+        nxt = decode(at_c, at_h);
+      }
       const int valid = cur.valid;
       const int koff = OFF_K + (int)ph * ROW_TILE;
       const float* sG = ph ? sVec1 : sVec0;

@@ -32,10 +32,9 @@
 //     256-383 V group : Vn^T -> rho-scaled and plain bf16 operand copies (tensor memory);
 //                       w^T -> bf16 operand tile (shared memory)
 //     384-511 O group : P -> Pg (operand); output epilogue o = s gamma O1 + O2
-//     warp 0  : issues every tcgen05.mma (one elected lane)
-//     warp 1  : producer: per-chunk gate vectors (fetched one chunk ahead), TMA loads of the
+//     warp 0  : issues the products of the chain, warp 1 all others (one elected lane each)
+//     warp 2  : producer: per-chunk gate vectors (fetched one chunk ahead), TMA loads of the
 //               q, k, v, A tiles (2 stages), zero-fill of rows past the end of a partial chunk
-//     64-127  prep    : one thread per chunk row: A' and A'' tiles
 // Synchronisation is by mbarriers only; every wait is bounded and reports through a status word.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -443,8 +442,9 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       mbar_arrive(&bars[W_READY]);
       return true;
     };
-    if (n_it > 0) ok = convert_w(0);
-    for (int it = 0; it < n_it && ok; ++it) {
+#pragma unroll 1
+    for (int it = -1; it < n_it && ok; ++it) {  // it = -1: only w^T of the first iteration
+     if (it >= 0) {
       const int c = it - lead;
       const long long row0 = sp.bos + (long long)c * CHUNK;
       const int valid = c < 0 ? 0 : min(CHUNK, sp.len - c * CHUNK);  // 0: nothing is stored
@@ -504,6 +504,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           mbar_arrive(&bars[VN_READY]);
         }
       }
+     }
       if (it + 1 < n_it) ok = convert_w(it + 1);
       if (v == 0) FQLA_TRACE(1, 3);
     }
@@ -530,7 +531,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       const float* sg = vec + (it & 3) * VEC_SLOT_FLOATS + V_SGAM * CHUNK;
       const long long row0 = sp.bos + (long long)c * CHUNK;
       const int valid = min(CHUNK, sp.len - c * CHUNK);
-      if (v == 0) tma_store_wait_read();  // the store of the chunk before has read the tile
+      if (wq == 0 && elect_one()) tma_store_wait_read();  // the store of the chunk before has read the tile
       asm volatile("bar.sync 1, 128;" ::: "memory");
       // The accumulators hold o transposed ([value index][token]).  Read with the 16-lane shape, a
       // lane gets mma-style fragments: rows l/4 and l/4 + 8 of a 16-row half, token pairs
@@ -576,13 +577,14 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       fence_proxy_async();
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (valid == CHUNK) {
-        if (v == 0) {
+        if (wq == 0 && elect_one()) {
           tma_store_2d(&map_o, hv * D, (int)row0, smem + OFF_O);
           tma_store_2d(&map_o, hv * D + 64, (int)row0, smem + OFF_O + 8192);
           tma_store_commit();
         }
       } else {
         // 16 pieces of 16 bytes per row; piece pc of row r sits at pc ^ (r & 7) inside its box
+#pragma unroll 1
         for (int i = v; i < valid * 16; i += 128) {
           const int r = i >> 4, pc = i & 15;
           const uint4 w = *reinterpret_cast<const uint4*>(smem + OFF_O + (pc >> 3) * 8192 + r * 128 +
@@ -625,19 +627,21 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       return true;
     };
     const float log2_scale = log2f(p.scale);
-    if (n_it > 0) ok = scale_a(0);
-    for (int j = 0; j < n_it && ok; ++j) {
+    // every part appears once (the kernel streams its code through a shared instruction cache):
+    // j = -1 only scales A of the first iteration, j = n_it only writes out the last chunk
+#pragma unroll 1
+    for (int j = -1; j <= n_it && ok; ++j) {
       const int it = j - lead;  // chunk of the sequence; < 0: lead-in, no output
-      if (!NO_O && it >= 0) {
+      // the epilogue of the chunk before first: the issuing thread needs its accumulators free
+      // (O_FREE) for this chunk's first output product
+      if (!NO_O && it > 0 && n_it > 0) {
+        ok = WAIT(O_DONE, (it - 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        epilogue(it - 1);
+      }
+      if (!NO_O && it >= 0 && j >= 0 && j < n_it) {
         const float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
-        // the epilogue of the chunk before first: the issuing thread needs its accumulators free
-        // (O_FREE) for this chunk's first output product
-        if (it > 0) {
-          ok = WAIT(O_DONE, (it - 1) & 1);
-          if (!ok) break;
-          tc_fence_after();
-          epilogue(it - 1);
-        }
         ok = WAIT(FULL0 + (j & 1), (j >> 1) & 1) && WAIT(P_DONE, it & 1);
         if (!ok) break;
         tc_fence_after();
@@ -672,18 +676,11 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       if (j + 1 < n_it) ok = scale_a(j + 1);
     }
     if constexpr (!NO_O) {
-      const int n_out = n_it - lead;  // chunks with output
-      if (ok && n_out > 0) {
-        ok = WAIT(O_DONE, (n_out - 1) & 1);
-        if (ok) {
-          tc_fence_after();
-          epilogue(n_out - 1);
-        }
-      }
-      if (v == 0) tma_store_wait_all();
+      if (wq == 0 && elect_one()) tma_store_wait_all();
       // rows of o past the end of the last packed sequence come out zero
       if (p.o && p.lay.cu.ptr && n == p.N - 1) {
         const long long end = sp.bos + sp.len;
+#pragma unroll 1
         for (long long i = tid - 384; i < (p.T_rows - end) * 16; i += 128)
           *reinterpret_cast<uint4*>(p.o + ((end + (i >> 4)) * p.Hv + hv) * D + (i & 15) * 8) =
               make_uint4(0, 0, 0, 0);
@@ -691,8 +688,8 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     }
   } else if (warp == 0 || warp == 1) {
     // =============================== MMA issuers ===============================
-    // Two threads issue, each with its own waits and its own tcgen05.commit (a commit covers the
-    // MMAs of the committing thread only):
+    // Two warps issue, each with its own waits and, from one elected lane, its own products and
+    // tcgen05.commit (a commit covers the MMAs of the committing thread only):
     //   warp 0, the chain: Vn^T and the state update, nothing else: twelve MMAs per chunk;
     //   warp 1, everything off the chain: P, O1^T, O2^T and u^T / w^T of the next chunk.  It is the
     //           one that waits for the output group, so the chain never stands behind an epilogue.
@@ -704,114 +701,126 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     constexpr uint32_t ID_OT = idesc_bf16(128, 64, 0, 0);            // A from tensor memory
     constexpr uint32_t ID_S = idesc_bf16(128, 128, 0, 1);
     constexpr uint32_t STAGE_LO = STAGE_BYTES >> 4;
-    if (warp == 0 && lane == 0) {
-      auto SPIN = [&](int idx, uint32_t parity) { return mbar_wait_spin(&bars[idx], parity, abort_flag); };
+    if (warp == 0) {
+      auto SPIN = [&](int idx, uint32_t parity) { return mbar_wait_warp<true>(&bars[idx], parity, abort_flag); };
+      auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
       // low descriptor words of every operand tile (see umma_lo); steps are 32-bit adds
       const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 16384);
       const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE_QK, 8192);
-      auto store_vn = [&](int it) {  // after VN_READY: the v_new^T tile is complete
-        tma_store_2d(&map_vn, 0, (int)(((sp.chunk_base + (it - lead)) * p.Hv + hv) * D), smem + OFF_VNT);
-        tma_store_commit();
-      };
+#pragma unroll 1
       for (int it = 0; it < n_it && ok; ++it) {
         const int s = it & 1, c = it - lead;  // c < 0: lead-in chunk
         const uint32_t so = s ? STAGE_LO : 0u;
-        FQLA_TRACE(3, 0);
-        if (it < 126) FQLA_CHUNK_CLOCK(it);
+        if (lane == 0) FQLA_TRACE(3, 0);
+        if (lane == 0 && it < 126) FQLA_CHUNK_CLOCK(it);
         ok = SPIN(S_COPY, it & 1) && SPIN(W_READY, it & 1);
         if (!ok) break;
         tc_fence_after();
-        FQLA_TRACE(3, 1);
-        // Vn^T = u^T - S^T w^T   (accumulates onto u^T; A = packed S^T in tensor memory)
-        umma_ts_group<8, 8, 128, true>(tmem + TM_UV, tmem + TM_SB, wmn_lo, ID_VN);
-        if constexpr (EXTRA) tma_store_wait_read();  // v_new^T of the chunk before has left its tile
-        umma_commit(&bars[VN_DONE]);
-        FQLA_TRACE(3, 2);
+        if (lane == 0) FQLA_TRACE(3, 1);
+        if (elect_one()) {
+          // Vn^T = u^T - S^T w^T   (accumulates onto u^T; A = packed S^T in tensor memory)
+          umma_ts_group<8, 8, 128, true>(tmem + TM_UV, tmem + TM_SB, wmn_lo, ID_VN);
+          if constexpr (EXTRA) tma_store_wait_read();  // v_new^T of the chunk before has left its tile
+          umma_commit(&bars[VN_DONE]);
+        }
+        if (lane == 0) FQLA_TRACE(3, 2);
         if constexpr (EXTRA) {
           if (tile_h && c >= 0) {  // the state entering this chunk, as an operand tile
-            ok = WAIT(ST_READY, c & 1);
+            ok = WAITW(ST_READY, c & 1);
             if (!ok) break;
-            const int y = (int)(((sp.chunk_base + c) * p.Hv + hv) * D);
-            tma_store_2d(&map_h, 0, y, smem + OFF_ST);
-            tma_store_2d(&map_h, 64, y, smem + OFF_ST + 16384);
-            tma_store_commit();
+            if (elect_one()) {
+              const int y = (int)(((sp.chunk_base + c) * p.Hv + hv) * D);
+              tma_store_2d(&map_h, 0, y, smem + OFF_ST);
+              tma_store_2d(&map_h, 64, y, smem + OFF_ST + 16384);
+              tma_store_commit();
+            }
           }
         }
-        FQLA_TRACE(3, 3);
+        if (lane == 0) FQLA_TRACE(3, 3);
         ok = SPIN(VB_READY, it & 1) && SPIN(S_DEC, it & 1);
         if (!ok) break;
         tc_fence_after();
-        FQLA_TRACE(3, 4);
-        // S^T += (rho Vn)^T K      (A = packed rho Vn^T; B = K tile read MN-major)
-        umma_ts_group<4, 8, 128, true>(tmem + TM_S, tmem + TM_VRB, kmn0_lo + so, ID_S);
-        if constexpr (EXTRA) tma_store_wait_read();  // the S^T tile may be rewritten after this
-        umma_commit(&bars[S_DONE]);
-        umma_commit(&bars[EMPTY0 + s]);  // this thread's last product that reads the stage
-        FQLA_TRACE(3, 5);
+        if (lane == 0) FQLA_TRACE(3, 4);
+        if (elect_one()) {
+          // S^T += (rho Vn)^T K      (A = packed rho Vn^T; B = K tile read MN-major)
+          umma_ts_group<4, 8, 128, true>(tmem + TM_S, tmem + TM_VRB, kmn0_lo + so, ID_S);
+          if constexpr (EXTRA) tma_store_wait_read();  // the S^T tile may be rewritten after this
+          umma_commit(&bars[S_DONE]);
+          umma_commit(&bars[EMPTY0 + s]);  // this thread's last product that reads the stage
+        }
+        if (lane == 0) FQLA_TRACE(3, 5);
         if constexpr (EXTRA) {
           if (tile_vn && c >= 0) {
-            ok = WAIT(VN_READY, c & 1);
+            ok = WAITW(VN_READY, c & 1);
             if (!ok) break;
-            store_vn(it);
+            if (elect_one()) {  // the v_new^T tile is complete
+              tma_store_2d(&map_vn, 0, (int)(((sp.chunk_base + c) * p.Hv + hv) * D), smem + OFF_VNT);
+              tma_store_commit();
+            }
           }
         }
-        FQLA_TRACE(3, 8);
+        if (lane == 0) FQLA_TRACE(3, 8);
       }
-      if constexpr (EXTRA) tma_store_wait_all();
-    } else if (warp == 1 && lane == 0) {
+      if constexpr (EXTRA) {
+        if (elect_one()) tma_store_wait_all();
+      }
+    } else {
+      auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
       const uint32_t p_lo = desc_lo_kmajor(smem + OFF_P);
       const uint32_t q0_lo = desc_lo_kmajor(smem + OFF_STAGE);
       const uint32_t k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE_QK);
       const uint32_t ap_lo = desc_lo_kmajor(smem + OFF_AP), app_lo = desc_lo_kmajor(smem + OFF_APP);
       const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE_QK, 8192);
       const uint32_t vmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + 2 * TILE_QK, 8192);
-      auto issue_u_w = [&](uint32_t so) {  // so = stage offset in descriptor units
-        umma_group<4, 128, 0, 2, 0, false>(tmem + TM_UV, vmn0_lo + so, ap_lo, ID_UT);
-        umma_group<4, 128, 0, 2, 0, false>(tmem + TM_PW, kmn0_lo + so, app_lo, ID_UT);
-        umma_commit(&bars[W_DONE]);
-      };
-      if (n_it > 0) {
-        ok = WAIT(FULL0, 0) && WAIT(AP_READY, 0);
-        if (ok) {
-          tc_fence_after();
-          issue_u_w(0);
+      // u^T and w^T of iteration j (so = its stage's offset in descriptor units).  u^T overwrites Vn^T
+      // (read by the value group), w^T overwrites P (read by the output group): the waits below.
+      auto issue_u_w = [&](uint32_t so) {
+        if (elect_one()) {
+          umma_group<4, 128, 0, 2, 0, false>(tmem + TM_UV, vmn0_lo + so, ap_lo, ID_UT);
+          umma_group<4, 128, 0, 2, 0, false>(tmem + TM_PW, kmn0_lo + so, app_lo, ID_UT);
+          umma_commit(&bars[W_DONE]);
         }
-      }
-      for (int it = 0; it < n_it && ok; ++it) {
+      };
+#pragma unroll 1
+      for (int it = -1; it < n_it && ok; ++it) {  // it = -1: only u^T, w^T of the first iteration
         const int s = it & 1, c = it - lead;
         const uint32_t so = s ? STAGE_LO : 0u, so_next = s ? 0u : STAGE_LO;
-        const bool with_o = !NO_O && c >= 0;
+        const bool with_o = !NO_O && c >= 0 && it >= 0;
         if (with_o) {
           // P = Q K^T goes first: the output group turns it into Pg while everything else runs.
           // Its columns held w^T of this chunk until the value group made the operand tile of it.
-          ok = WAIT(W_READY, it & 1);
+          ok = WAITW(W_READY, it & 1);
           if (!ok) break;
           tc_fence_after();
-          umma_group<8, 2, 512, 2, 512, false>(tmem + TM_PW, q0_lo + so, k0_lo + so, ID_P);
-          umma_commit(&bars[P_DONE]);
+          if (elect_one()) {
+            umma_group<8, 2, 512, 2, 512, false>(tmem + TM_PW, q0_lo + so, k0_lo + so, ID_P);
+            umma_commit(&bars[P_DONE]);
+          }
           // O1^T = S^T Q^T   (A = packed S^T; B = q tile, K-major)
-          ok = WAIT(S_COPY, it & 1) && (c == 0 || WAIT(O_FREE, (c - 1) & 1));
+          ok = WAITW(S_COPY, it & 1) && (c == 0 || WAITW(O_FREE, (c - 1) & 1));
           if (!ok) break;
           tc_fence_after();
-          umma_ts_group_kmajor_b<8>(tmem + TM_O1, tmem + TM_SB, q0_lo + so, ID_OT);
-          umma_commit(&bars[SB_FREE]);
+          if (elect_one()) {
+            umma_ts_group_kmajor_b<8>(tmem + TM_O1, tmem + TM_SB, q0_lo + so, ID_OT);
+            umma_commit(&bars[SB_FREE]);
+          }
         }
         // this thread's products that read the stage (u^T, w^T of this chunk, issued a chunk ago,
         // and the two above) are all issued
-        umma_commit(&bars[EMPTY0 + s]);
+        if (it >= 0 && elect_one()) umma_commit(&bars[EMPTY0 + s]);
         if (with_o) {
           // O2^T = Vn^T Pg^T   (A = packed Vn^T; B = Pg, K-major)
-          ok = WAIT(P_READY, c & 1) && WAIT(VB_READY, it & 1);
+          ok = WAITW(P_READY, c & 1) && WAITW(VB_READY, it & 1);
           if (!ok) break;
           tc_fence_after();
-          umma_ts_group<4, 8, 2, false>(tmem + TM_O2, tmem + TM_VNB, p_lo, ID_OT);
-          umma_commit(&bars[O_DONE]);
+          if (elect_one()) {
+            umma_ts_group<4, 8, 2, false>(tmem + TM_O2, tmem + TM_VNB, p_lo, ID_OT);
+            umma_commit(&bars[O_DONE]);
+          }
         }
         if (it + 1 < n_it) {
-          // u^T and w^T of the next chunk: u^T overwrites Vn^T (read by the value group:
-          // VB_READY), w^T overwrites P (read by the output group: P_READY above)
-          ok = WAIT(FULL0 + (s ^ 1), ((it + 1) >> 1) & 1) && WAIT(AP_READY, (it + 1) & 1) &&
-               WAIT(VB_READY, it & 1);
+          ok = WAITW(FULL0 + (s ^ 1), ((it + 1) >> 1) & 1) && WAITW(AP_READY, (it + 1) & 1) &&
+               (it < 0 || WAITW(VB_READY, it & 1));
           if (!ok) break;
           tc_fence_after();
           issue_u_w(so_next);
@@ -834,94 +843,88 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         b_r[z] = r < valid ? load_beta(p.beta, p.beta_is_f32, (row0 + r) * p.Hv + hv) : 0.f;
       }
     };
-    // vectors and A tile of chunk j (its stage's A buffer is free once the prep warps have read it)
-    auto a_part = [&](int j) {
-      const int sj = j & 1, c = j - lead;
-      const long long row0 = sp.bos + (long long)c * CHUNK;
-      const int valid = c < 0 ? CHUNK : min(CHUNK, sp.len - c * CHUNK);
-      if (j >= 2 && !WAIT(EMPTYA0 + sj, ((j >> 1) - 1) & 1)) return false;
-      float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
-#pragma unroll
-      for (int z = 0; z < 2; ++z) {
-        int r = 2 * lane + z;
-        float gam = fast_exp(g_r[z]);
-        vs[V_G * CHUNK + r] = g_r[z];
-        vs[V_BETA * CHUNK + r] = b_r[z];
-        vs[V_BG * CHUNK + r] = b_r[z] * gam;
-        vs[V_RHO * CHUNK + r] = fast_exp(gl_r - g_r[z]);
-        vs[V_SGAM * CHUNK + r] = p.scale * gam;
-      }
-      if (lane == 0) vs[V_GL * CHUNK] = fast_exp(gl_r);
+    auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
+    // zero the rows past the sequence end in n 8 KB blocks of 64 rows (they belong to the next
+    // sequence), then hand the tile on
+    auto zero_rows = [&](unsigned char* base, int n, int valid, uint64_t* full) {
+#pragma unroll 1
+      for (int i = lane; i < n * 512; i += 32)
+        if (((i >> 3) & 63) >= valid) *reinterpret_cast<uint4*>(base + i * 16) = make_uint4(0, 0, 0, 0);
+      fence_proxy_async();
       __syncwarp();
-      unsigned char* dst = smem + OFF_STAGE + sj * STAGE_BYTES + 2 * TILE_QK + TILE_V;
-      const bool partial = valid < CHUNK;
-      uint64_t* bar = partial ? &bars[PRIVA] : &bars[FULLA0 + sj];
-      if (lane == 0) {
-        mbar_arrive_expect_tx(bar, TILE_A);
-        tma_load_2d(dst, &map_a, hv * CHUNK, (int)row0, bar);
-      }
-      if (partial) {
-        // rows past the sequence end belong to the next sequence: wait for the copy, zero them
-        // (only the last chunk of a sequence can be partial: the private barrier is used once)
-        if (!WAIT(PRIVA, 0)) return false;
-        for (int i = lane; i < (CHUNK - valid) * 8; i += 32)
-          *reinterpret_cast<uint4*>(dst + (valid + (i >> 3)) * 128 + ((i & 7) << 4)) = make_uint4(0, 0, 0, 0);
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[FULLA0 + sj]);
-      }
-      return true;
+      if (lane == 0) mbar_arrive(full);
     };
-    if (n_it > 0) {
-      fetch(0);
-      ok = a_part(0);
-      if (n_it > 1) fetch(1);
-    }
-    for (int it = 0; it < n_it && ok; ++it) {
-      const int s = it & 1, c = it - lead;
-      const long long row0 = sp.bos + (long long)c * CHUNK;
-      const int valid = c < 0 ? CHUNK : min(CHUNK, sp.len - c * CHUNK);
-      const bool with_q = !NO_O && c >= 0;
-      if (it >= 2) {
-        ok = WAIT(EMPTY0 + s, ((it >> 1) - 1) & 1);
-        if (!ok) break;
-      }
-      unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
-      const bool partial = valid < CHUNK;
-      uint64_t* bar = partial ? &bars[PRIV] : &bars[FULL0 + s];
-      if (lane == 0) {
-        mbar_arrive_expect_tx(bar, STAGE_BYTES - TILE_A - (with_q ? 0 : TILE_QK));
-        const int y = (int)row0;
-        tma_load_2d(st + TILE_QK, &map_k, hq * D, y, bar);
-        tma_load_2d(st + TILE_QK + 8192, &map_k, hq * D + 64, y, bar);
-        tma_load_2d(st + 2 * TILE_QK, &map_v, hv * D, y, bar);
-        tma_load_2d(st + 2 * TILE_QK + 8192, &map_v, hv * D + 64, y, bar);
-        if (with_q) {
-          tma_load_2d(st, &map_q, hq * D, y, bar);
-          tma_load_2d(st + 8192, &map_q, hq * D + 64, y, bar);
+    // Iteration `it`: q, k, v of chunk it; vectors and A tile of chunk it + 1, a whole chunk before
+    // its q, k, v (whose stage is still in use, but the prep warps can start on A early); the gates
+    // of chunk it + 2 into registers.  (Slot (it + 1) % 4 of the vectors was last read for chunk
+    // it - 3, which the wait on the stage of chunk it - 2 has seen finished.)
+#pragma unroll 1
+    for (int it = -2; it < n_it && ok; ++it) {
+      if (it >= 0) {
+        const int s = it & 1, c = it - lead;
+        const int y = (int)(sp.bos + (long long)c * CHUNK);
+        const int valid = c < 0 ? CHUNK : min(CHUNK, sp.len - c * CHUNK);
+        const bool with_q = !NO_O && c >= 0, partial = valid < CHUNK;
+        if (it >= 2) {
+          ok = WAITW(EMPTY0 + s, ((it >> 1) - 1) & 1);
+          if (!ok) break;
+        }
+        unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
+        uint64_t* bar = &bars[partial ? PRIV : FULL0 + s];
+        if (elect_one()) {
+          mbar_arrive_expect_tx(bar, STAGE_BYTES - TILE_A - (with_q ? 0 : TILE_QK));
+          tma_load_2d(st + TILE_QK, &map_k, hq * D, y, bar);
+          tma_load_2d(st + TILE_QK + 8192, &map_k, hq * D + 64, y, bar);
+          tma_load_2d(st + 2 * TILE_QK, &map_v, hv * D, y, bar);
+          tma_load_2d(st + 2 * TILE_QK + 8192, &map_v, hv * D + 64, y, bar);
+          if (with_q) {
+            tma_load_2d(st, &map_q, hq * D, y, bar);
+            tma_load_2d(st + 8192, &map_q, hq * D + 64, y, bar);
+          }
+        }
+        if (partial) {
+          ok = WAITW(PRIV, 0);
+          if (!ok) break;
+          zero_rows(st, 6, valid, &bars[FULL0 + s]);
         }
       }
-      if (partial) {
-        ok = WAIT(PRIV, 0);
-        if (!ok) break;
-        for (int blk = 0; blk < 6; ++blk) {
-          unsigned char* base = st + blk * 8192;
-          for (int i = lane; i < (CHUNK - valid) * 8; i += 32)
-            *reinterpret_cast<uint4*>(base + (valid + (i >> 3)) * 128 + ((i & 7) << 4)) =
-                make_uint4(0, 0, 0, 0);
+      const int j = it + 1;
+      if (j >= 0 && j < n_it) {
+        const int sj = j & 1, c = j - lead;
+        const int valid = c < 0 ? CHUNK : min(CHUNK, sp.len - c * CHUNK);
+        const bool partial = valid < CHUNK;
+        // the stage's A buffer is free once the prep warps have read it
+        if (j >= 2) {
+          ok = WAITW(EMPTYA0 + sj, ((j >> 1) - 1) & 1);
+          if (!ok) break;
         }
-        fence_proxy_async();
+        float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          int r = 2 * lane + z;
+          float gam = fast_exp(g_r[z]);
+          vs[V_G * CHUNK + r] = g_r[z];
+          vs[V_BETA * CHUNK + r] = b_r[z];
+          vs[V_BG * CHUNK + r] = b_r[z] * gam;
+          vs[V_RHO * CHUNK + r] = fast_exp(gl_r - g_r[z]);
+          vs[V_SGAM * CHUNK + r] = p.scale * gam;
+        }
+        if (lane == 0) vs[V_GL * CHUNK] = fast_exp(gl_r);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[FULL0 + s]);
+        unsigned char* dst = smem + OFF_STAGE + sj * STAGE_BYTES + 2 * TILE_QK + TILE_V;
+        uint64_t* bar = &bars[partial ? PRIVA : FULLA0 + sj];
+        if (elect_one()) {
+          mbar_arrive_expect_tx(bar, TILE_A);
+          tma_load_2d(dst, &map_a, hv * CHUNK, (int)(sp.bos + (long long)c * CHUNK), bar);
+        }
+        if (partial) {
+          // only the last chunk of a sequence can be partial: the private barrier is used once
+          ok = WAITW(PRIVA, 0);
+          if (!ok) break;
+          zero_rows(dst, 1, valid, &bars[FULLA0 + sj]);
+        }
       }
-      // The next chunk's vectors and A tile go out now, a whole chunk before its q, k, v: the
-      // q, k, v stage of chunk it + 1 is still in use, but the prep warps can start on A early.
-      // (Slot (it + 1) % 4 of the vectors was last read for chunk it - 3, which the wait on the
-      // stage of chunk it - 2 above has seen finished.)
-      if (it + 1 < n_it) {
-        ok = a_part(it + 1);
-        if (ok && it + 2 < n_it) fetch(it + 2);
-      }
+      if (it + 2 < n_it) fetch(it + 2);
     }
   }
 
@@ -1013,8 +1016,7 @@ extern "C" int fqla_debug_fwd_chunk_clock(long long* out256) {
 
 namespace fqla {
 // Self-test of the bounded-wait path: one thread waits on an mbarrier that nobody ever arrives
-// at, with a budget of `tries` suspended tries of at most 1 ms each.  The wait gives up, the
-// kernel sets the device status word exactly as a product kernel does, and returns.
+// at, with a budget of `tries` tries.  The wait gives up, the kernel sets the device status word exactly as a product kernel does, and returns.
 __global__ void wait_timeout_selftest_kernel(uint32_t tries) {
   __shared__ uint64_t bar;
   __shared__ int abort_flag;

@@ -45,23 +45,21 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                "r"(bytes)
                : "memory");
 }
-// One try: the thread is suspended by the hardware until the phase completes or the time hint
-// (nanoseconds) runs out; no instructions are issued meanwhile, so waiting warps do not take
-// issue slots from the warps they share a scheduler with.
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity, uint32_t hint_ns) {
+// One try: the thread may be suspended by the hardware until the phase completes or a (short,
+// about 0.2 us on B200) system limit runs out; no instructions are issued meanwhile.
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(s32(bar)), "r"(parity), "r"(hint_ns)
+      : "r"(s32(bar)), "r"(parity)
       : "memory");
   return ok != 0;
 }
 
-// Non-blocking test of a phase (about 13 cycles on B200 when the phase is complete; the bounded
-// loop around the suspending form was measured at about 200 cycles even then).
+// Non-blocking test of a phase (about 13 cycles on B200).
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -74,18 +72,21 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait: at most `budget` tries of up to 1 ms each.  Gives up as soon as *abort_flag
-// (shared memory) is set; on its own timeout it sets *abort_flag so that every other role of the
-// CTA leaves too.  Returns false when the wait was abandoned.
+// Bounded wait: at most `budget` tries (the default is some seconds).  Gives up as soon as
+// *abort_flag (shared memory) is set; on its own timeout it sets *abort_flag so that every other
+// role of the CTA leaves too.  Returns false when the wait was abandoned.
+// One loop around one instruction: a kernel has dozens of wait sites and is larger than the
+// instruction cache.  (A test first and then tries with a 1 ms suspend hint was 5-10 % more code
+// and woke up later: 802 against 787 us for a 262144-token forward, 2040 against 1997 us for 32768
+// packed training tokens.)
+constexpr uint32_t WAIT_TRIES = 1u << 24;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
-                                          volatile int* abort_flag, uint32_t budget = 2000) {
-  if (mbar_test_wait(bar, parity)) return true;  // fast path: the phase is already complete
-  // not unrolled: a kernel has dozens of wait sites and is larger than the instruction cache
+                                          volatile int* abort_flag, uint32_t budget = WAIT_TRIES) {
 #pragma unroll 1
-  for (uint32_t i = 0; i < budget; ++i) {
-    if (mbar_try_wait(bar, parity, 1000000u)) return true;
+  do {
+    if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
-  }
+  } while (--budget);
   *abort_flag = 1;
   return false;
 }
@@ -101,15 +102,33 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t saddr, uint32_t r0, u
                : "memory");
 }
 
-// The same bounded wait for a thread that is alone in its warp and on the critical path: it polls
-// (about 13 cycles per test) for a while before it lets the hardware suspend it, because waking
-// from the suspended form costs several hundred cycles.
-__device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity,
-                                               volatile int* abort_flag) {
+// ---- issuing warps -----------------------------------------------------------------------------
+// A warp that issues tcgen05 and TMA instructions stays CONVERGED: all its lanes run the loop and
+// the waits, and only the instructions themselves sit behind elect_one().  The compiler then keeps
+// descriptors in uniform registers: six instructions per MMA.  Inside a divergent `lane == 0` branch
+// it cannot know that one thread is active and emits a loop over distinct operand values for every
+// MMA, 49 instructions (790 bytes of code) each: 58 of the forward recurrence kernel's 93 KB,
+// streamed through instruction caches that the SMs of a GPC share (a chunk took 4.3 k cycles on an
+// otherwise idle GPC and 7.3 k with all its SMs busy).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+// Bounded wait of a whole converged warp: the result is the same in every lane.  SPIN: poll (about
+// 25 cycles a round) without looking at the abort flag in between, for the warp on the critical path.
+template <bool SPIN>
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  uint32_t n = WAIT_TRIES;
 #pragma unroll 1
-  for (int i = 0; i < 2048; ++i)
-    if (mbar_test_wait(bar, parity)) return true;
-  return mbar_wait(bar, parity, abort_flag);
+  do {
+    if (__all_sync(0xffffffffu, SPIN ? mbar_test_wait(bar, parity) : mbar_try_wait(bar, parity))) return true;
+    if (!SPIN && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
+  } while (--n);
+  *abort_flag = 1;
+  return false;
 }
 
 // ---- proxy / tcgen05 fences ------------------------------------------------------------------
