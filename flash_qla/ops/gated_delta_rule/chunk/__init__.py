@@ -233,9 +233,14 @@ def chunk_gated_delta_rule(
     Returns ``(o [B,T,HV,V], final_state [N,HV,K,V] or None)``.
     """
     assert not head_first, "head_first=True is not supported."
-    return _lib.host().apply(
+    out = _lib.host().apply(
         q, k, v, g, beta, scale, initial_state, cu_seqlens,
         (FINAL_STATE if output_final_state else 0) | (AUTO_CP if auto_cp else 0)
         | (V_FIRST if state_v_first else 0) | (CACHE if enable_fwd_cp_cache else 0)
         | (SAVE_TILES if SAVE_STATE_TILES else 0) | (LEAD_IN if cp.LEAD_IN else 0)
         | (L2NORM if use_qk_l2norm_in_kernel else 0))
+    if out is None:  # a trace, a functorch transform or a forward-mode tangent
+        out = ChunkGatedDeltaRuleFunction.apply(
+            q, k, v, g, beta, scale, initial_state, output_final_state, cu_seqlens,
+            use_qk_l2norm_in_kernel, state_v_first, auto_cp, enable_fwd_cp_cache)
+    return out

@@ -1,4 +1,6 @@
 // Python bindings of the native host path (flashqla_b200._host).
+#include <ATen/TracerMode.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/python_headers.h>
 
@@ -15,27 +17,27 @@ namespace {
 
 PyObject* fqla_error = nullptr;  // flashqla_b200._lib.FqlaError
 
-PyObject* raise(const std::exception& e) {
-  PyObject* type = PyExc_RuntimeError;
-  if (auto* p = dynamic_cast<const PyError*>(&e)) {
-    switch (p->kind) {
+// Runs a binding's body.  Errors of this module's own checks surface as the Python types the
+// operator documents; everything else (an exception raised in a saved-tensor hook, out of memory,
+// PyTorch's own errors) as PyTorch's bindings report it.
+template <typename F>
+PyObject* guarded(F&& body) {
+  HANDLE_TH_ERRORS
+  try {
+    return body();
+  } catch (const PyError& e) {
+    PyObject* type = PyExc_RuntimeError;
+    switch (e.kind) {
       case PyError::Assertion: type = PyExc_AssertionError; break;
       case PyError::Type: type = PyExc_TypeError; break;
       case PyError::Value: type = PyExc_ValueError; break;
       case PyError::NotImplemented: type = PyExc_NotImplementedError; break;
       case PyError::Fqla: type = fqla_error ? fqla_error : PyExc_RuntimeError; break;
     }
-  } else if (auto* c = dynamic_cast<const c10::OutOfMemoryError*>(&e)) {
-    // torch.OutOfMemoryError, as the caching allocator's failures surface everywhere else
-    PyObject* torch = PyImport_ImportModule("torch");
-    PyObject* oom = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
-    if (oom) PyErr_SetString(oom, c->what_without_backtrace());
-    Py_XDECREF(oom);
-    Py_XDECREF(torch);
+    PyErr_SetString(type, e.what());
     return nullptr;
   }
-  PyErr_SetString(type, e.what());
-  return nullptr;
+  END_HANDLE_TH_ERRORS
 }
 
 at::Tensor tensor(PyObject* o, const char* name) {
@@ -99,10 +101,22 @@ double number(PyObject* o) {
   return x;
 }
 
+// What only PyTorch's own function class deals with: a trace records the call by it, a functorch
+// transform or a forward-mode tangent is refused by it (the native node would drop the tangent).
+bool needs_function_class(std::initializer_list<const at::Tensor*> ts) {
+  if (at::tracer::impl::is_dispatch_enabled()) return true;
+  constexpr c10::DispatchKeySet transforms({c10::DispatchKey::FuncTorchBatched,
+                                            c10::DispatchKey::FuncTorchGradWrapper});
+  for (const at::Tensor* t : ts)
+    if (t->key_set().has_any(transforms) || t->_fw_grad(0).defined()) return true;
+  return false;
+}
+
 // apply(q, k, v, g, beta, scale or None, initial_state, cu_seqlens, flags) -> (o, final_state),
-// recorded for autograd.  The argument checks of the public operator are made here.
+// recorded for autograd; None where the call belongs to the function class (above).  The argument
+// checks of the public operator are made here.
 PyObject* py_apply(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  try {
+  return guarded([&]() -> PyObject* {
     if (n != 9) throw PyError(PyError::Type, "apply takes 9 arguments");
     const at::Tensor q = tensor(a[0], "q"), k = tensor(a[1], "k"), v = tensor(a[2], "v");
     const OptTensor h0 = opt_tensor(a[6], "initial_state"), cu = opt_tensor(a[7], "cu_seqlens");
@@ -126,17 +140,17 @@ PyObject* py_apply(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const double scale = a[5] == Py_None ? 1.0 / std::sqrt((double)k.size(-1)) : number(a[5]);
     const at::Tensor g = tensor(a[3], "g"), beta = tensor(a[4], "beta");
     const Options opt = options(a[8]);
+    if (needs_function_class({&q, &k, &v, &g, &beta}) || (h0 && needs_function_class({&*h0})))
+      Py_RETURN_NONE;
     const auto r = without_gil([&] { return apply(q, k, v, g, beta, scale, h0, cu, opt); });
     return tuple_of(r.first, r.second);
-  } catch (const std::exception& e) {
-    return raise(e);
-  }
+  });
 }
 
 // forward(q, k, v, g, beta, scale, initial_state, cu_seqlens, flags)
 //   -> (g_cum, A, o, h, final_state, cp_cache), with L2NORM also (q, k, q_rstd, k_rstd)
 PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  try {
+  return guarded([&]() -> PyObject* {
     if (n != 9) throw PyError(PyError::Type, "forward takes 9 arguments");
     const at::Tensor q = tensor(a[0], "q"), k = tensor(a[1], "k"), v = tensor(a[2], "v"),
                      g = tensor(a[3], "g"), beta = tensor(a[4], "beta");
@@ -166,15 +180,13 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
       PyTuple_SET_ITEM(out, 9, wrap(r.k_rstd));
     }
     return out;
-  } catch (const std::exception& e) {
-    return raise(e);
-  }
+  });
 }
 
 // backward(q, k, v, g_cum, beta, A, do, dht, scale, initial_state, cu_seqlens, flags, cp_cache, norm)
 //   -> (dq, dk, dv, db, dg, dh0);  norm: None or (q, k before the normalisation, q_rstd, k_rstd)
 PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  try {
+  return guarded([&]() -> PyObject* {
     if (n != 14) throw PyError(PyError::Type, "backward takes 14 arguments");
     Cache cache;
     if (a[12] != Py_None) {
@@ -204,14 +216,12 @@ PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
     if (r.db.scalar_type() != beta.scalar_type()) r.db = r.db.to(beta.scalar_type());
     return tuple_of(r.dq, r.dk, r.dv, r.db, r.dg, r.dh0);
-  } catch (const std::exception& e) {
-    return raise(e);
-  }
+  });
 }
 
 // split_sequences(bounds, heads, n_sm, min_chunks, slices) -> None or (seg_bounds, seg_begin)
 PyObject* py_split(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  try {
+  return guarded([&]() -> PyObject* {
     if (n != 5) throw PyError(PyError::Type, "split_sequences takes 5 arguments");
     PyObject* seq = PySequence_Fast(a[0], "bounds must be a sequence of ints");
     if (!seq) return nullptr;
@@ -233,9 +243,7 @@ PyObject* py_split(PyObject*, PyObject* const* a, Py_ssize_t n) {
     PyTuple_SET_ITEM(out, 0, list(s->seg_bounds));
     PyTuple_SET_ITEM(out, 1, list(s->seg_begin));
     return out;
-  } catch (const std::exception& e) {
-    return raise(e);
-  }
+  });
 }
 
 PyObject* py_launches(PyObject*, PyObject*) { return PyLong_FromLongLong(launch_count.load()); }
