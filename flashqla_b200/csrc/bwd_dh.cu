@@ -14,6 +14,8 @@
 // context parallelism, in blackwell/cp_bwd.py:16-589.
 //
 // mma.sync implementation, eight cooperating warps, cp.async double buffering.
+#include <climits>
+
 #include "common.cuh"
 #include "fqla_internal.h"
 
@@ -93,14 +95,12 @@ __global__ void __launch_bounds__(256, 1) bwd_dh_kernel(const BwdDhParams p) {
   const int n = p.order ? p.order[blockIdx.x / p.Hv] : (int)(blockIdx.x / p.Hv);
   const int hq = hv / (p.Hv / p.Hq);
   const int v0 = blockIdx.y * BV;
-  if (p.run_mask && p.run_mask[n * p.Hv + hv] != p.run_value) return;  // uniform per CTA
+  // what there is to do, before anything else is read (see fwd_seq.cu)
+  const int run = p.run_mask ? p.run_mask[n * p.Hv + hv] : p.run_value;
+  const int warm = p.warm ? p.warm[n * p.Hv + hv] : INT_MAX;  // < 0: no output is written
+  if (run != p.run_value || warm < 0) return;  // uniform per CTA
   const SeqSpan sp = p.lay.span(n);
-  int c_end = sp.n_chunks;  // exclusive
-  if (p.warm) {
-    const int w = p.warm[n * p.Hv + hv];
-    if (w < 0) return;  // nothing is wanted of this (sequence, head): no output is written
-    c_end = min(sp.n_chunks, w);
-  }
+  const int c_end = min(sp.n_chunks, warm);  // exclusive
 
   float dS[MTS][NTV][4];
   const int dht_row = p.dht_row ? p.dht_row[n] : n;

@@ -113,109 +113,211 @@ segment_scan_kernel(const float* __restrict__ g_cum, int Hv, SeqLayout lay,
   }
 }
 
-// Chain the segments of one raw sequence for one head and one 32-wide value slice.
-// grid = (D/32, Hv, n_raw), 128 threads for D = 128 (thread a owns row a of the slice).
-//   forward  (reverse = 0): out[first] = start_raw; out[i+1] = local[i] + useM[i] * M[i]   out[i]
-//   backward (reverse = 1): out[last]  = end_raw;   out[i-1] = local[i] + useM[i] * M[i]^T out[i]
+__device__ __forceinline__ void cp_async4(float* smem_dst, const float* gmem_src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src));
+}
+
+// Chain the segments of the raw sequences, per head:
+//   forward  (reverse = 0): out[first] = raw; out[i+1] = local[i] + useM[i] * M[i]   out[i]
+//   backward (reverse = 1): out[last]  = raw; out[i-1] = local[i] + useM[i] * M[i]^T out[i]
+// The steps of a chain are serial, its value columns are independent: a CTA walks one chain for
+// BV = 8 of them, and what bounds it is the latency of a step, a D x D x 8 product in fp32 (2 x 8
+// outputs per thread, the contraction split over KS groups of threads and summed through shared
+// memory; about 1000 cycles of fused multiply-adds at D = 128).  M arrives by cp.async two steps
+// ahead in three buffers whose padded rows (LDM = D + 4) keep both the row-wise 16-byte reads
+// (forward) and the column reads (reverse) free of bank conflicts.  32 columns per CTA with M
+// staged in panels inside the step took 16 us a step: the 18-segment chains of two heads of 32768
+// tokens 293 us, now 51.
+// Few CTAs (one per SM) take the (sequence, head) pairs in turn, gridDim.y apart, and only those
+// that have a chain at all (any_fb): usually none has, and a CTA then ends after one load.
 template <int D>
-__global__ void __launch_bounds__(D) merge_kernel(const float* __restrict__ local,
-                                                  const float* __restrict__ M,
-                                                  const int* __restrict__ use_m,
-                                                  const float* __restrict__ raw,
-                                                  const int* __restrict__ seg_begin,
-                                                  const int* __restrict__ any_fb,
-                                                  float* __restrict__ out, int Hv, int reverse,
-                                                  long long seg_stride, long long use_stride) {
-  // seg_stride / use_stride: distance in 4-byte words between the entries of consecutive
-  // segments in local and M / in use_m (packed tensors, or the records of a gathered buffer);
-  // raw and out are always packed
-  constexpr int BV = 32, BK = 32, LDC = BV + 1;
-  // all global traffic is one 128-byte row segment per warp instruction; the padded row stride
-  // keeps both the row-wise (warp = row) and the thread-owns-a-row accesses free of bank conflicts
-  __shared__ float cur[D * LDC];
-  // one staging buffer: the local state of the step, then D x BK panels of M, forward [a][j]
-  // (row stride BK+1), reverse [j][a]
-  __shared__ float panel[D * (BK + 1)];
+struct Merge {
+  static constexpr int BV = 8, NT = 256, KS = 2 * NT / D, KB = D / KS, LDM = D + 4;
+  static constexpr int M_FLOATS = D * LDM, PER = D * BV / NT;
+  static constexpr int SMEM_BYTES = (3 * M_FLOATS + D * BV + KS * D * BV) * 4;
+  static constexpr int CTAS_Y = D == 128 ? 9 : 54;  // x D / BV slices: all SMs, one or three CTAs each
+};
+struct MergeParams {
+  const float *local, *M;
+  const int* use_m;
+  const float* raw;
+  const int *seg_begin, *any_fb;
+  float* out;
+  int Hv, n_pairs, reverse, raw_v_first, vec16;
+  // distance in 4-byte words between the entries of consecutive segments in local and M / in use_m
+  // (packed tensors, or the records of a gathered buffer); raw and out are always packed
+  long long seg_stride, use_stride;
+};
+template <int D>
+__global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
+  using C = Merge<D>;
+  constexpr int BV = C::BV, NT = C::NT, KS = C::KS, KB = C::KB, LDM = C::LDM, PER = C::PER;
+  extern __shared__ __align__(16) float sm[];
+  __shared__ unsigned active[NT / 32];
+  float* cur = sm + 3 * C::M_FLOATS;   // [D][BV] state of the step
+  float* part = cur + D * BV;          // [KS][D][BV] partial products
   pdl_wait();
-  const int a = threadIdx.x, lane = a & 31, warp = a >> 5;
-  const int v0 = blockIdx.x * BV, hv = blockIdx.y, r = blockIdx.z;
-  const int s0 = seg_begin[r], s1 = seg_begin[r + 1];  // segments [s0, s1)
-  if (s1 <= s0) return;
-  auto state = [&](const float* base, int seg) {
-    return base + (((long long)seg * Hv + hv) * D) * D;
-  };
-  auto strided = [&](const float* base, int seg) {
-    return base + (long long)seg * seg_stride + ((long long)hv * D) * D;
-  };
-  if (any_fb && any_fb[r * Hv + hv] == 0) {
-    // no chain for this (sequence, head): the recurrence kernel leads in by itself; only the
-    // edge segment needs a state (the sequence's own initial state or final-state gradient)
-    const float* src = raw ? state(raw, r) : nullptr;
-    float* dst = const_cast<float*>(state(out, reverse ? s1 - 1 : s0));
-    for (int row = warp; row < D; row += D / 32)
-      dst[(long long)row * D + v0 + lane] = src ? src[(long long)row * D + v0 + lane] : 0.f;
-    return;
-  }
-  // initial value
-  {
-    const float* src = raw ? state(raw, r) : nullptr;
-    for (int row = warp; row < D; row += D / 32)
-      cur[row * LDC + lane] = src ? src[(long long)row * D + v0 + lane] : 0.f;
-  }
-  __syncthreads();
-  const int n = s1 - s0;
-  // the local state (and the flag) of the next step are fetched one step ahead into registers:
-  // the chain itself then only waits for shared memory
-  constexpr int RPW = D / (D / 32);  // rows per warp
-  float pre[RPW];
-  int pre_m = 0;
-  auto prefetch = [&](int step) {
-    const int i = reverse ? s1 - 1 - step : s0 + step;
-    const float* loc = strided(local, i);
-#pragma unroll
-    for (int t = 0; t < RPW; ++t) pre[t] = loc[(long long)(warp + t * (D / 32)) * D + v0 + lane];
-    pre_m = use_m == nullptr ? 1 : use_m[(long long)i * use_stride + hv];
-  };
-  if (n > 1) prefetch(0);
-  for (int step = 0; step < n; ++step) {
-    const int i = reverse ? s1 - 1 - step : s0 + step;
-    float* dst = const_cast<float*>(state(out, i));
-    for (int row = warp; row < D; row += D / 32) dst[(long long)row * D + v0 + lane] = cur[row * LDC + lane];
-    if (step == n - 1) break;
-#pragma unroll
-    for (int t = 0; t < RPW; ++t) panel[(warp + t * (D / 32)) * LDC + lane] = pre[t];
-    const bool with_m = pre_m != 0;
-    if (step + 1 < n - 1) prefetch(step + 1);
-    __syncthreads();
-    float acc[BV];
-#pragma unroll
-    for (int j = 0; j < BV; ++j) acc[j] = panel[a * LDC + j];
-    if (with_m) {
-      const float* m = strided(M, i);
-      for (int b0 = 0; b0 < D; b0 += BK) {
-        __syncthreads();  // the previous contents of the panel have been consumed
-        if (!reverse) {
-          // panel[a'][j] = M[a'][b0+j], one warp per row, coalesced
-          for (int row = warp; row < D; row += D / 32)
-            panel[row * (BK + 1) + lane] = m[(long long)row * D + b0 + lane];
-        } else {
-          // panel[j][a'] = M[b0+j][a']
-          for (int j = 0; j < BK; ++j) panel[j * D + a] = m[(long long)(b0 + j) * D + a];
-        }
-        __syncthreads();
+  const int t = threadIdx.x;
+  const int v0 = blockIdx.x * BV;
+  const int row = t * PER / BV, col = t * PER % BV;  // this thread's elements of the state
+  const int a = t % (D / 2), b0 = t / (D / 2) * KB;  // ... its rows a, a + D/2 and part of a product
+
+  auto chain = [&](int r, int hv) {
+    const int s0 = p.seg_begin[r], n = p.seg_begin[r + 1] - s0;
+    if (n <= 0) return;
+    auto seg = [&](int step) { return p.reverse ? s0 + n - 1 - step : s0 + step; };
+    auto strided = [&](const float* base, int step) {
+      return base + (long long)seg(step) * p.seg_stride + ((long long)hv * D) * D;
+    };
+    // the last step only stores: nothing of its segment is read
+    auto flag = [&](int step) {
+      return step >= n - 1 ? 0 : p.use_m ? p.use_m[(long long)seg(step) * p.use_stride + hv] : 1;
+    };
+    auto fetch_m = [&](int step, int with_m) {
+      if (with_m) {
+        const float* m = strided(p.M, step);
+        float* dst = sm + step % 3 * C::M_FLOATS;
+        if (p.vec16) {
 #pragma unroll 4
-        for (int j = 0; j < BK; ++j) {
-          float w = reverse ? panel[j * D + a] : panel[a * (BK + 1) + j];
-#pragma unroll
-          for (int vv = 0; vv < BV; ++vv) acc[vv] += w * cur[(b0 + j) * LDC + vv];
+          for (int i = t * 4; i < D * D; i += NT * 4) cp_async16(dst + i / D * LDM + i % D, m + i, true);
+        } else {
+#pragma unroll 4
+          for (int i = t; i < D * D; i += NT) cp_async4(dst + i / D * LDM + i % D, m + i);
         }
       }
-    }
-    __syncthreads();  // every read of cur (and of the panel) is done
+      cp_async_commit();
+    };
+    auto fetch_local = [&](int step, float (&x)[PER]) {
+      if (step >= n - 1) return;
+      const float* l = strided(p.local, step) + (long long)row * D + v0 + col;
 #pragma unroll
-    for (int j = 0; j < BV; ++j) cur[a * LDC + j] = acc[j];
+      for (int e = 0; e < PER; ++e) x[e] = l[e];
+    };
+    float own[PER], loc[PER], loc_next[PER];
+    const float* raw = p.raw ? p.raw + ((long long)r * p.Hv + hv) * D * D : nullptr;
+#pragma unroll
+    for (int e = 0; e < PER; ++e) {
+      const int v = v0 + col + e;
+      own[e] = !raw ? 0.f : raw[p.raw_v_first ? (long long)v * D + row : (long long)row * D + v];
+      loc[e] = loc_next[e] = 0.f;
+    }
+    int with_m = flag(0), with_m1 = flag(1), with_m2 = flag(2);
+    fetch_m(0, with_m);
+    fetch_m(1, with_m1);
+    fetch_local(0, loc);
+#pragma unroll 1
+    for (int step = 0; step < n; ++step) {
+      float* dst = p.out + (((long long)seg(step) * p.Hv + hv) * D + row) * D + v0 + col;
+#pragma unroll
+      for (int e = 0; e < PER; ++e) dst[e] = cur[row * BV + col + e] = own[e];
+      if (step == n - 1) break;
+      fetch_m(step + 2, with_m2);  // (its buffer was last read before the barrier that ended step - 1)
+      const int with_m3 = flag(step + 3);
+      fetch_local(step + 1, loc_next);
+      cp_async_wait<2>();
+      __syncthreads();
+      if (with_m) {
+        const float* m = sm + step % 3 * C::M_FLOATS;
+        float acc[2][BV] = {};
+#pragma unroll 2
+        for (int b = b0; b < b0 + KB; b += 4) {
+          float w[2][4];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (!p.reverse) {
+              const float4 x = *reinterpret_cast<const float4*>(m + (a + h * (D / 2)) * LDM + b);
+              w[h][0] = x.x; w[h][1] = x.y; w[h][2] = x.z; w[h][3] = x.w;
+            } else {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) w[h][j] = m[(b + j) * LDM + a + h * (D / 2)];
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float4 x = *reinterpret_cast<const float4*>(cur + (b + j) * BV);
+            const float4 y = *reinterpret_cast<const float4*>(cur + (b + j) * BV + 4);
+            const float c[BV] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+              for (int v = 0; v < BV; ++v) acc[h][v] += w[h][j] * c[v];
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float* q = part + ((t / (D / 2)) * D + a + h * (D / 2)) * BV;
+          *reinterpret_cast<float4*>(q) = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
+          *reinterpret_cast<float4*>(q + 4) = make_float4(acc[h][4], acc[h][5], acc[h][6], acc[h][7]);
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < PER; ++e) {
+        own[e] = loc[e];
+        if (with_m) {
+#pragma unroll
+          for (int k = 0; k < KS; ++k) own[e] += part[(k * D + row) * BV + col + e];
+        }
+        loc[e] = loc_next[e];
+      }
+      with_m = with_m1;
+      with_m1 = with_m2;
+      with_m2 = with_m3;
+    }
+    cp_async_wait<0>();
+    __syncthreads();  // the next chain of this CTA reuses every buffer
+  };
+
+  const int mine = (p.n_pairs - (int)blockIdx.y + (int)gridDim.y - 1) / (int)gridDim.y;
+#pragma unroll 1
+  for (int base = 0; base < mine; base += NT) {
+    const int i = base + t;
+    const bool on = i < mine && (!p.any_fb || p.any_fb[blockIdx.y + (long long)i * gridDim.y] != 0);
+    const unsigned bits = __ballot_sync(0xffffffffu, on);
+    if ((t & 31) == 0) active[t / 32] = bits;
+    __syncthreads();
+#pragma unroll 1
+    for (int w = 0; w < NT / 32; ++w)
+      for (unsigned left = active[w]; left; left &= left - 1) {
+        const int pair = (int)blockIdx.y + (base + 32 * w + __ffs(left) - 1) * (int)gridDim.y;
+        chain(pair / p.Hv, pair % p.Hv);
+      }
     __syncthreads();
   }
+}
+
+// The (sequence, head) pairs without a chain: only the edge segment's entry is written.
+template <int D>
+__global__ void __launch_bounds__(D) merge_edge_kernel(const MergeParams p) {
+  pdl_wait();
+  const int hv = blockIdx.y, r = blockIdx.z;
+  const int s0 = p.seg_begin[r], s1 = p.seg_begin[r + 1];
+  if (s1 <= s0 || p.any_fb[r * p.Hv + hv] != 0) return;
+  const float* src = p.raw ? p.raw + ((long long)r * p.Hv + hv) * D * D : nullptr;
+  float* dst = p.out + ((long long)(p.reverse ? s1 - 1 : s0) * p.Hv + hv) * D * D;
+  const int v = threadIdx.x;
+  for (int k = blockIdx.x; k < D; k += gridDim.x)
+    dst[(long long)k * D + v] = !src ? 0.f : src[p.raw_v_first ? (long long)v * D + k : (long long)k * D + v];
+}
+
+template <int D>
+static int launch_merge(const fqla_merge_args& a, cudaStream_t st) {
+  using C = Merge<D>;
+  MergeParams p;
+  p.local = a.local; p.M = a.M; p.use_m = a.use_m; p.raw = a.raw; p.seg_begin = a.seg_begin;
+  p.any_fb = a.any_fallback; p.out = a.out; p.Hv = a.Hv; p.n_pairs = a.n_raw * a.Hv;
+  p.reverse = a.reverse; p.raw_v_first = a.raw_v_first;
+  p.seg_stride = a.seg_stride ? a.seg_stride : (long long)a.Hv * D * D;
+  p.use_stride = a.seg_stride ? a.seg_stride : a.Hv;
+  p.vec16 = ((reinterpret_cast<uintptr_t>(a.M) | (unsigned long long)p.seg_stride * 4) & 15) == 0;
+  static std::atomic<unsigned long long> done;
+  int rc = configure_smem((const void*)merge_kernel<D>, C::SMEM_BYTES, done);
+  if (rc != 0) return rc;
+  const int y = p.n_pairs < C::CTAS_Y ? p.n_pairs : C::CTAS_Y;
+  rc = launch_pdl(merge_kernel<D>, dim3(D / C::BV, y), dim3(C::NT), C::SMEM_BYTES, st, p);
+  if (rc != 0 || !a.any_fallback || a.no_edges) return rc;
+  return launch_pdl(merge_edge_kernel<D>, dim3(8, a.Hv, a.n_raw), dim3(D), 0, st, p);
 }
 
 }  // namespace fqla
@@ -246,21 +348,23 @@ extern "C" int fqla_segment_scan(const float* g_cum, int T, int Hv, const void* 
       g_cum, Hv, lay, seg_begin, threshold, from_start, warm, fallback, lead, exact_warm, any_fb);
 }
 
+extern "C" int fqla_merge_run(const fqla_merge_args* args, void* stream) {
+  if (!args) return FQLA_ERR_INVALID_ARG;
+  const fqla_merge_args& a = *args;
+  if (!a.local || !a.M || !a.seg_begin || !a.out || a.Hv <= 0 || a.seg_stride < 0) return FQLA_ERR_INVALID_ARG;
+  if (a.n_raw <= 0) return FQLA_OK;
+  if (a.D == 128) return launch_merge<128>(a, (cudaStream_t)stream);
+  if (a.D == 64) return launch_merge<64>(a, (cudaStream_t)stream);
+  return FQLA_ERR_UNSUPPORTED_DIM;
+}
+
 extern "C" int fqla_merge_states(const float* local, const float* M, const int* use_m,
                                  const float* raw, const int* seg_begin, const int* any_fb,
                                  float* out, int n_raw, int Hv, int D, int reverse,
                                  long long seg_stride, void* stream) {
-  if (!local || !M || !seg_begin || !out || Hv <= 0 || seg_stride < 0) return FQLA_ERR_INVALID_ARG;
-  if (n_raw <= 0) return FQLA_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (D == 128) {
-    return launch_pdl(merge_kernel<128>, dim3(128 / 32, Hv, n_raw), dim3(128), 0, st,
-        local, M, use_m, raw, seg_begin, any_fb, out, Hv, reverse,
-        seg_stride ? seg_stride : (long long)Hv * D * D, seg_stride ? seg_stride : Hv);
-  } else if (D == 64) {
-    return launch_pdl(merge_kernel<64>, dim3(64 / 32, Hv, n_raw), dim3(64), 0, st,
-        local, M, use_m, raw, seg_begin, any_fb, out, Hv, reverse,
-        seg_stride ? seg_stride : (long long)Hv * D * D, seg_stride ? seg_stride : Hv);
-  }
-  return FQLA_ERR_UNSUPPORTED_DIM;
+  fqla_merge_args a = {};
+  a.local = local; a.M = M; a.use_m = use_m; a.raw = raw; a.seg_begin = seg_begin;
+  a.any_fallback = any_fb; a.out = out; a.n_raw = n_raw; a.Hv = Hv; a.D = D; a.reverse = reverse;
+  a.seg_stride = seg_stride;
+  return fqla_merge_run(&a, stream);
 }

@@ -16,6 +16,7 @@
 // This translation unit is the mma.sync (legacy tensor core) implementation: all eight warps
 // cooperate on each product in turn, operands staged by cp.async with the next chunk's tiles in
 // flight.  It supports D = 64 and D = 128.
+#include <climits>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -106,17 +107,16 @@ __global__ void __launch_bounds__(256, 1) fwd_seq_kernel(const FwdSeqParams p) {
   const bool m_slice = (int)blockIdx.y >= V_SLICES;  // transition-matrix slice
   const int v0 = (m_slice ? (int)blockIdx.y - V_SLICES : (int)blockIdx.y) * BV;
   const bool with_q = p.q != nullptr && !m_slice;
-  const SeqSpan sp = p.lay.span(n);
-  if (p.run_mask && p.run_mask[n * p.Hv + hv] != p.run_value) return;  // uniform per CTA
-  if (m_slice && p.m_mask && p.m_mask[n * p.Hv + hv] == 0) return;
+  // What there is to do, before anything else is read: in a split plan usually nothing (the whole
+  // launch is a few thousand CTAs that end here).
+  const int item = n * p.Hv + hv;
+  const int run = p.run_mask ? p.run_mask[item] : p.run_value;
+  const int warm = p.warm ? p.warm[item] : INT_MAX;  // < 0: no output is written
+  const int masked = m_slice && p.m_mask ? p.m_mask[item] : 1;
+  if (run != p.run_value || warm < 0 || masked == 0) return;          // uniform per CTA
   if (!m_slice && !p.ht && !p.o && !p.h && !p.vnew) return;          // nothing asked of this slice
-
-  int c_begin = 0;
-  if (p.warm) {
-    const int w = p.warm[n * p.Hv + hv];
-    if (w < 0) return;  // nothing is wanted of this (sequence, head): no output is written
-    c_begin = max(0, sp.n_chunks - w);
-  }
+  const SeqSpan sp = p.lay.span(n);
+  const int c_begin = max(0, sp.n_chunks - min(warm, sp.n_chunks));
 
   // ---- state in registers: rows 32*wm + mt*16 + ..., cols (BV/2)*wn + nt*8 + ...
   float S[MTS][NTV][4];

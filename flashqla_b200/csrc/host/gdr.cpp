@@ -150,13 +150,17 @@ fqla_bwd_dh_args dh_args(const Call& c, const SeqIn& in, const at::Tensor& dO) {
 }
 void run_dh(const Call& c, const fqla_bwd_dh_args& a) { check(fqla_bwd_dh_run(&a, c.stream), "bwd_dh"); }
 
+// Start states (reverse: end gradients) of the segments that are handed one.  The edges of a sequence
+// take raw itself (row maps), so the entries of pairs without a chain are left out.
 at::Tensor merge(const Call& c, const at::Tensor& local, const at::Tensor& M, const int* use_m,
-                 const OptTensor& raw, const int* any_fb, bool reverse) {
+                 const OptTensor& raw, bool raw_v_first, const int* any_fb, bool reverse) {
   at::Tensor out = empty({c.batch->n_seg, c.Hv, c.D, c.D}, at::kFloat, c.dev);
-  check(fqla_merge_states((const float*)local.data_ptr(), (const float*)M.data_ptr(), use_m,
-                          ptr<float>(raw), c.batch->s_begin, any_fb, (float*)out.data_ptr(),
-                          (int)c.batch->N, c.Hv, c.D, reverse, 0, c.stream),
-        "merge_states");
+  fqla_merge_args a = {};
+  a.local = (const float*)local.data_ptr(); a.M = (const float*)M.data_ptr(); a.use_m = use_m;
+  a.raw = ptr<float>(raw); a.seg_begin = c.batch->s_begin; a.any_fallback = any_fb;
+  a.out = (float*)out.data_ptr(); a.n_raw = (int)c.batch->N; a.Hv = c.Hv; a.D = c.D;
+  a.reverse = reverse; a.raw_v_first = raw_v_first; a.no_edges = 1;
+  check(fqla_merge_run(&a, c.stream), "merge_states");
   return out;
 }
 
@@ -199,11 +203,6 @@ Scan warmup_scan(const Call& c, const at::Tensor& g, bool from_start) {
   return s;
 }
 
-// The merge chain reads the sequences' own states as [key][value].
-OptTensor key_first(const OptTensor& x, bool v_first) {
-  return x && v_first ? OptTensor(x->transpose(-1, -2).contiguous()) : x;
-}
-
 // Start states of the segments (and lead-in counts) of a split plan.  Segments whose past dies out
 // inside the segment before them start themselves a few chunks early from a zero state; the exact
 // chain (state-only pass with the transition matrices, then the merge) returns at once for them.
@@ -218,7 +217,7 @@ void segment_starts(const Call& c, const SeqIn& in, const OptTensor& h0, const O
   a.warm_chunks = leads ? s.exact_warm : s.warm;
   a.m_mask = s.fallback;
   run_fwd(c, a);
-  out.seg_h0 = merge(c, l, M, s.fallback, key_first(h0, opt.state_v_first), leads ? s.any_fb : nullptr, false);
+  out.seg_h0 = merge(c, l, M, s.fallback, h0, opt.state_v_first, leads ? s.any_fb : nullptr, false);
   if (leads) out.lead = s.lead_tensor;
 }
 
@@ -237,7 +236,7 @@ std::pair<at::Tensor, OptTensor> segment_ends(const Call& c, const SeqIn& in, co
   m.M = (float*)M.data_ptr();
   m.m_mask = s.fallback;
   run_fwd(c, m);
-  at::Tensor ends = merge(c, l, M, s.fallback, key_first(dht, opt.state_v_first), leads ? s.any_fb : nullptr, true);
+  at::Tensor ends = merge(c, l, M, s.fallback, dht, opt.state_v_first, leads ? s.any_fb : nullptr, true);
   return {ends, leads ? OptTensor(s.lead_tensor) : std::nullopt};
 }
 
@@ -337,7 +336,7 @@ Forward forward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor
   if (q_in.scalar_type() != r.o.scalar_type()) r.o = r.o.to(q_in.scalar_type());
   if (opt.output_h) {
     at::Tensor x = cu ? h->unsqueeze(0) : h->view({c.B, -1, c.Hv, c.D, c.D});
-    r.h = key_first(x, opt.state_v_first);
+    r.h = opt.state_v_first ? x.transpose(-1, -2).contiguous() : x;
   }
   if (keep) {
     r.cache.h = h;

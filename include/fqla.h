@@ -225,6 +225,20 @@ int fqla_merge_states(const float* local, const float* M, const int* use_m, cons
                       const int* seg_begin, const int* any_fallback, float* out, int n_raw, int Hv,
                       int D, int reverse, long long seg_stride, void* stream);
 
+/* fqla_merge_states with every argument in one structure, zero-initialised by the caller.
+ * raw_v_first: raw is [value dim][key dim] (local, M and out never are); no_edges: with
+ * any_fallback, the edge entries of pairs without a chain are not written either. */
+typedef struct fqla_merge_args {
+  const float *local, *M;
+  const int* use_m;
+  const float* raw;
+  const int *seg_begin, *any_fallback;
+  float* out;
+  int n_raw, Hv, D, reverse, raw_v_first, no_edges;
+  long long seg_stride;
+} fqla_merge_args;
+int fqla_merge_run(const fqla_merge_args* args, void* stream);
+
 /* Row-wise L2 normalisation (the optional pre-op of q and k): y = x * rsqrt(sum x^2 + eps) in
  * the dtype of x, rstd [rows] fp32; and its gradient dx = (dy - <dy, y> y) * rstd, fp32.
  * Rows are contiguous, D even and <= 512.  dtype codes: 0 bf16, 1 fp16, 2 fp32.
