@@ -13,7 +13,7 @@
 //     w    = (Ac diag(beta gamma)) Kc   [tok][k]
 //     dS^T <- gamma_last dS^T - dv^T w + dOc^T (scale gamma .* Qc)
 // Six roles as in the forward kernel (fwd_tc.cu): warp 0 issues every tcgen05.mma, warp 1 runs the
-// TMA pipeline (two stages of q, k, dO, A) and the per-row vectors, warps 2-3 scale A and q,
+// TMA pipeline (two stages of q, k, dO, A) and the per-row vectors, warps 2-3 scale A and q (in place),
 // warps 4-7 own the state (operand copy, decay, dh / dh0 output), warps 8-11 turn X1, X2 and w
 // into operands (and write du), warps 12-15 build Pg.  All waits are bounded mbarrier waits.
 #include <cuda.h>
@@ -66,8 +66,7 @@ constexpr int OFF_DVT = OFF_ST + 32768;   // dv^T   [128 x 128B]
 constexpr int OFF_W = OFF_DVT + 16384;    // w      2 blocks of [64 x 128B]
 constexpr int OFF_P = OFF_W + 16384;      // Pg     [64 x 128B]
 constexpr int OFF_APP = OFF_P + 8192;     // A diag(beta gamma)
-constexpr int OFF_QS = OFF_APP + 8192;    // scale gamma .* q, 2 blocks of [64 x 128B]
-constexpr int OFF_VEC = OFF_QS + TILE;
+constexpr int OFF_VEC = OFF_APP + 8192;
 constexpr int VEC_SLOT_FLOATS = 5 * CHUNK;
 constexpr int OFF_BAR = OFF_VEC + 4 * VEC_SLOT_FLOATS * 4;
 constexpr int N_BARS = 24;
@@ -408,8 +407,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     const uint32_t st_lo = desc_lo_kmajor(smem + OFF_ST), dvt_lo = desc_lo_kmajor(smem + OFF_DVT);
     const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 8192), pmn_lo = desc_lo_mnmajor(smem + OFF_P, 8192);
     const uint32_t app_lo = desc_lo_kmajor(smem + OFF_APP);
-    const uint32_t qsmn_lo = desc_lo_mnmajor(smem + OFF_QS, 8192);
-    const uint32_t q0_lo = desc_lo_kmajor(smem + OFF_STAGE);
+    const uint32_t q0_lo = desc_lo_kmajor(smem + OFF_STAGE), qmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE, 8192);
     const uint32_t k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE);
     const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE, 8192);
     const uint32_t domn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + 2 * TILE, 8192);
@@ -447,14 +445,17 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         }
       }
       if (it >= 0) {
-        ok = WAITW(W_READY, it & 1) && WAITW(QS_READY, it & 1) && WAITW(S_DEC, it & 1) &&
-             WAITW(DV_READY, it & 1);
+        // dS^T <- dS^T + dO^T (scale gamma q) - dv^T w; the first product while dv is on its way
+        ok = WAITW(QS_READY, it & 1) && WAITW(S_DEC, it & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one())
+          umma_group<4, 128, 0, 128, 0, true>(tmem + TM_S, domn0_lo + so, qmn0_lo + so, ID_UPD_Q);
+        ok = WAITW(W_READY, it & 1) && WAITW(DV_READY, it & 1);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
-          // dS^T <- dS^T - dv^T w + dO^T (scale gamma q)
           umma_group<4, 2, 0, 128, 0, true>(tmem + TM_S, dvt_lo, wmn_lo, ID_UPD_W);
-          umma_group<4, 128, 0, 128, 0, true>(tmem + TM_S, domn0_lo + so, qsmn_lo, ID_UPD_Q);
           tma_store_wait_read();  // the dS^T tile may be rewritten after this
           umma_commit(&bars[S_DONE]);
           if (p.tiled && p.du && it >= lead) {
@@ -588,8 +589,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       if (ok && it > 0) ok = WAIT(W_DONE, (it - 1) & 1);  // w of the chunk before has been issued and is done
       if (!ok) break;
       const float* vs = vec + (it & 3) * VEC_SLOT_FLOATS;
-      const unsigned char* stg = smem + OFF_STAGE + s * STAGE_BYTES;
-      const unsigned char* src = stg + 3 * TILE;
+      const unsigned char* src = smem + OFF_STAGE + s * STAGE_BYTES + 3 * TILE;
       const float4 g0 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8);
       const float4 g1 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8 + 4);
 #pragma unroll 4
@@ -606,18 +606,17 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         mbar_arrive(&bars[AP_READY]);
         mbar_arrive(&bars[EMPTYA0 + s]);  // the A tile of this stage is no longer read
       }
-      // q' has one buffer: the state update of the chunk before must have read it; q has landed
-      ok = WAIT(FULL0 + s, (it >> 1) & 1);
-      if (ok && it > 0) ok = WAIT(S_DONE, (it - 1) & 1);
+      // q' goes over q, once P = Q K^T has read it: ready long before the state update wants it (a
+      // buffer of its own had to wait for the update of the chunk before)
+      ok = WAIT(FULL0 + s, (it >> 1) & 1) && WAIT(P_DONE, it & 1);
       if (!ok) break;
       const float sg = vs[V_SGAM * CHUNK + r];
-      unsigned char* qs = smem + OFF_QS;
-#pragma unroll 1
+      unsigned char* q = smem + OFF_STAGE + s * STAGE_BYTES + r * 128;
+#pragma unroll 2
       for (int q16 = 0; q16 < 16; ++q16) {
-        const int blk = q16 >> 3, pc = (q16 + r) & 7;
-        const uint4 a = *reinterpret_cast<const uint4*>(stg + blk * 8192 + r * 128 + pc * 16);
-        *reinterpret_cast<uint4*>(qs + blk * 8192 + r * 128 + pc * 16) =
-            make_uint4(scale2(a.x, sg, sg), scale2(a.y, sg, sg), scale2(a.z, sg, sg), scale2(a.w, sg, sg));
+        uint4* x = reinterpret_cast<uint4*>(q + (q16 >> 3) * 8192 + ((q16 + r) & 7) * 16);
+        const uint4 a = *x;
+        *x = make_uint4(scale2(a.x, sg, sg), scale2(a.y, sg, sg), scale2(a.z, sg, sg), scale2(a.w, sg, sg));
       }
       fence_proxy_async();
       __syncwarp();
