@@ -334,7 +334,7 @@ extern "C" int fqla_bwd_dh_run(const fqla_bwd_dh_args* args, void* stream) {
   const SeqLayout lay{{a.cu_seqlens, a.idx_is64}, {a.chunk_offsets, a.idx_is64}, a.T};
   cudaStream_t st = (cudaStream_t)stream;
   static const bool force_legacy = getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
-  if (a.D == 128 && !a.warm_chunks && !force_legacy) return launch_bwd_dh_tc(a, N, lay, st);
+  if (a.D == 128 && !(a.warm_chunks && a.operand_tiles) && !force_legacy) return launch_bwd_dh_tc(a, N, lay, st);
   // only the tcgen05 kernel writes tiles or leads out
   if (a.operand_tiles || a.lead_chunks) return FQLA_ERR_UNSUPPORTED_DIM;
   BwdDhParams p;

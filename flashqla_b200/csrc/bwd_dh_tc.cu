@@ -18,6 +18,8 @@
 // into operands (and write du), warps 12-15 build Pg.  All waits are bounded mbarrier waits.
 #include <cuda.h>
 
+#include <climits>
+
 #include "common.cuh"
 #include "fqla_internal.h"
 #include "tc05.cuh"
@@ -54,6 +56,9 @@ struct BwdDhTcParams {
   // [N, Hv] or null: a CTA whose entry differs from run_value returns at once
   const int* run_mask;
   int run_value;
+  // [N, Hv] or null (dh0 only): only the first warm[n,hv] chunks are walked, from a zero gradient
+  // (< 0: nothing is done)
+  const int* warm;
 };
 
 namespace bdtc {
@@ -107,6 +112,12 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     pdl_wait();
     if (p.run_mask[sequence() * p.Hv + hv] != p.run_value) return;  // uniform per CTA
   }
+  int warm = INT_MAX;
+  if (p.warm) {
+    pdl_wait();
+    warm = p.warm[sequence() * p.Hv + hv];
+    if (warm < 0) return;  // uniform per CTA
+  }
 
   if (tid == 0) {
     mbar_init(&bars[FULL0], 1);
@@ -149,7 +160,9 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
   const SeqSpan sp = p.lay.span(n);
   // iteration `it` handles chunk n_it - 1 - it of the segment; chunks >= sp.n_chunks are the
   // lead-out chunks (whole chunks, except possibly the very last one of the sequence)
-  const int lead = (p.lead && sp.n_chunks > 0) ? p.lead[n * p.Hv + hv] : 0;
+  // (lead < 0: the last -lead chunks are left out)
+  const int lead = p.warm ? min(warm, sp.n_chunks) - sp.n_chunks
+                          : (p.lead && sp.n_chunks > 0) ? p.lead[n * p.Hv + hv] : 0;
   const int n_it = sp.n_chunks + lead;
   const int len_ext = sp.len + (lead > 0 ? min(lead * CHUNK, p.lay.span(n + 1).len) : 0);
   tc_fence_before();
@@ -165,7 +178,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
   if (warp >= 4) {
     const int dht_row = p.dht_row ? p.dht_row[n] : n;
     const bool edge = dht_row >= 0;
-    const float* src = lead > 0 ? nullptr : edge ? p.dht : p.seg_dht;
+    const float* src = lead != 0 ? nullptr : edge ? p.dht : p.seg_dht;
     if (src) src += ((long long)(edge ? dht_row : n) * p.Hv + hv) * D * D;
     const int v = (warp & 3) * 32 + lane;
     auto load32 = [&](int k0, float (&x)[32]) {
@@ -673,6 +686,7 @@ int launch_bwd_dh_tc(const fqla_bwd_dh_args& a, int N, SeqLayout lay, cudaStream
   p.lead = a.lead_chunks;
   p.run_mask = a.run_mask;
   p.run_value = a.run_value;
+  p.warm = a.warm_chunks;
   p.g = a.g_cum; p.beta = a.beta; p.beta_is_f32 = a.beta_is_f32;
   p.dht = a.dht; p.seg_dht = a.seg_dht; p.dht_row = a.dht_row; p.dh0_row = a.dh0_row;
   p.v_first = a.state_v_first;

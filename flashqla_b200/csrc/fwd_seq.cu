@@ -375,13 +375,16 @@ extern "C" int fqla_fwd_run(const fqla_fwd_args* args, void* stream) {
   if (N <= 0) return FQLA_OK;
   const SeqLayout lay{{a.cu_seqlens, a.idx_is64}, {a.chunk_offsets, a.idx_is64}, a.T};
   cudaStream_t st = (cudaStream_t)stream;
-  // The full forward (q and o present, K = V = 128) and the recomputation of the per-chunk
-  // states and v_new for the backward pass (neither q nor o) run on the tcgen05 kernel;
-  // state-only passes, transition matrices and D = 64 run on the mma.sync kernel in this file.
+  // K = V = 128: the full forward (q and o present), the recomputation of the per-chunk states and
+  // v_new for the backward pass (neither q nor o) and the state-only pass with the transition
+  // matrices run on the tcgen05 kernel; D = 64 and other combinations of outputs on the mma.sync
+  // kernel in this file.  (End states and matrices of two heads of 32768 tokens, 18 segments: 78 us
+  // on the mma.sync kernel, 52 on the tcgen05 one; a pass that finds nothing to do, 4 us on either.)
   static const bool force_legacy = getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
   const bool full = a.q && a.o, recompute = !a.q && !a.o && (a.h || a.vnew);
-  if (a.D == 128 && (full || recompute) && !a.M && !a.warm_chunks && !a.m_mask && !force_legacy)
-    return launch_fwd_tc(a, N, lay, st);
+  const bool ends = !a.q && !a.o && !a.h && !a.vnew && (a.ht || a.M) && !a.operand_tiles && !a.lead_chunks;
+  const bool tc = ends || ((full || recompute) && !a.M && !a.warm_chunks && !a.m_mask);
+  if (a.D == 128 && tc && !force_legacy) return launch_fwd_tc(a, N, lay, st);
   // tcgen05 kernel only
   if (a.operand_tiles || a.lead_chunks || a.o_is_f16) return FQLA_ERR_UNSUPPORTED_DIM;
   FwdSeqParams p;

@@ -39,6 +39,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <climits>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -105,6 +106,13 @@ struct FwdTcParams {
   // [N] or null: the CTAs of block index i / Hv walk sequence order[i].  Blocks start in index
   // order, so a table that lists the longest sequences first shortens the tail of a ragged batch.
   const int* order;
+  // State-only variant: the blocks from m_first on compute the transition matrix M [N, Hv, D, D] (the
+  // same walk from the identity with v = 0), the ones before it the end state.  warm [N, Hv] or
+  // null: only the last warm[n,hv] chunks are walked, from a zero state (< 0: nothing is done);
+  // m_mask [N, Hv] or null: M only where non-zero.
+  float* M;
+  const int *warm, *m_mask;
+  int m_first;
 };
 
 namespace fwdtc {
@@ -170,8 +178,8 @@ __device__ __forceinline__ uint32_t pack_out(float lo, float hi) {
 
 // EXTRA: per-chunk state and v_new outputs (compiled out of the common instantiation: the six
 // roles run six different code regions at once, and the kernel is sensitive to its
-// instruction-cache footprint).  NO_O: state-only walk (recomputation for the backward pass): no q,
-// no output products, the output warps stay idle.  O_F16: o leaves as fp16 instead of bf16.
+// instruction-cache footprint).  NO_O: state-only walk, no q, no output products, the output warps
+// stay idle: with EXTRA the recomputation for the backward pass, without it end states and M.  O_F16: o leaves as fp16 instead of bf16.
 template <bool EXTRA, bool NO_O, bool O_F16>
 __global__ void __launch_bounds__(512, 1)
 fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
@@ -188,12 +196,23 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   float* vec = reinterpret_cast<float*>(smem + OFF_VEC);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int hv = blockIdx.x % p.Hv;
-  auto sequence = [&] { return p.order ? p.order[blockIdx.x / p.Hv] : (int)(blockIdx.x / p.Hv); };
+  constexpr bool STATE = NO_O && !EXTRA;
+  const bool m_pass = STATE && (int)blockIdx.x >= p.m_first;
+  const int block = m_pass ? (int)blockIdx.x - p.m_first : (int)blockIdx.x;
+  const int hv = block % p.Hv;
+  auto sequence = [&] { return p.order ? p.order[block / p.Hv] : block / p.Hv; };
   const int hq = hv / (p.Hv / p.Hq);
   if (p.run_mask) {
     pdl_wait();
     if (p.run_mask[sequence() * p.Hv + hv] != p.run_value) return;  // uniform per CTA
+  }
+  int warm = INT_MAX;
+  if (STATE && (p.warm || p.m_mask)) {
+    pdl_wait();
+    const int item = sequence() * p.Hv + hv;
+    const int masked = m_pass && p.m_mask ? p.m_mask[item] : 1;
+    if (p.warm) warm = p.warm[item];
+    if (warm < 0 || masked == 0) return;  // uniform per CTA
   }
   const bool tile_h = EXTRA && p.tiled && p.h, tile_vn = EXTRA && p.tiled && p.vnew;
 
@@ -238,6 +257,11 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   // groups that can be non-zero for its rows
   for (int i = tid; i < 8192 / 16; i += 512)
     *reinterpret_cast<uint4*>(smem + OFF_P + i * 16) = make_uint4(0, 0, 0, 0);
+  if (m_pass) {  // v stays zero: its tiles are never loaded
+    for (int i = tid; i < 2 * TILE_V / 16; i += 512)
+      *reinterpret_cast<uint4*>(smem + OFF_STAGE + 2 * TILE_QK + (i & 1023) * 16 + (i >> 10) * STAGE_BYTES) =
+          make_uint4(0, 0, 0, 0);
+  }
   fence_proxy_async();
   if (warp == 0) tmem_alloc(tmem_slot, 512);
   // everything above overlaps the tail of the kernel before: no global memory up to here
@@ -245,7 +269,8 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   const int n = sequence();
   const SeqSpan sp = p.lay.span(n);
   // iteration j handles chunk c = j - lead of the sequence; c < 0 are the lead-in chunks
-  const int lead = p.lead ? p.lead[n * p.Hv + hv] : 0;
+  // (lead < 0: the first -lead chunks are left out)
+  const int lead = STATE ? min(warm, sp.n_chunks) - sp.n_chunks : p.lead ? p.lead[n * p.Hv + hv] : 0;
   const int n_it = sp.n_chunks == 0 ? 0 : sp.n_chunks + lead;
   tc_fence_before();
   __syncthreads();
@@ -262,13 +287,13 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   if (warp >= 4) {
     const int h0_row = p.h0_row ? p.h0_row[n] : n;
     const bool edge = h0_row >= 0;  // starts its sequence; else it is handed a state, if any
-    const float* src = lead > 0 ? nullptr : edge ? p.h0 : p.seg_h0;
+    const float* src = (STATE ? lead != 0 || m_pass : lead > 0) ? nullptr : edge ? p.h0 : p.seg_h0;
     if (src) src += ((long long)(edge ? h0_row : n) * p.Hv + hv) * D * D;
     const int v = (warp & 3) * 32 + lane;
     auto load32 = [&](int k0, float (&x)[32]) {
       if (!src) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = 0.f;
+        for (int j = 0; j < 32; ++j) x[j] = m_pass && k0 + j == v ? 1.f : 0.f;
       } else if (edge && p.v_first) {
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
@@ -396,16 +421,17 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       if (v == 0) FQLA_TRACE(0, 4);
     }
     if (ok && n_it > 0) ok = WAIT(S_DONE, (n_it - 1) & 1);
-    const int ht_row = p.ht_row ? p.ht_row[n] : n;
-    if (ok && p.ht && ht_row >= 0) {
-      float* dst = p.ht + ((long long)ht_row * p.Hv + hv) * D * D;
+    const int ht_row = p.ht_row && !m_pass ? p.ht_row[n] : n;
+    float* end = m_pass ? p.M : p.ht;
+    if (ok && end && ht_row >= 0) {
+      float* dst = end + ((long long)ht_row * p.Hv + hv) * D * D;
       tc_fence_after();
 #pragma unroll 1
       for (int k0 = 0; k0 < D; k0 += 32) {
         float x[32];
         tmem_ld32(tmem + lane_sel + TM_S + k0, x);
         tmem_ld_wait();
-        if (p.v_first) {
+        if (p.v_first && !m_pass) {
 #pragma unroll
           for (int j = 0; j < 32; j += 4)
             *reinterpret_cast<float4*>(dst + (long long)v * D + k0 + j) =
@@ -872,11 +898,13 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
         uint64_t* bar = &bars[partial ? PRIV : FULL0 + s];
         if (elect_one()) {
-          mbar_arrive_expect_tx(bar, STAGE_BYTES - TILE_A - (with_q ? 0 : TILE_QK));
+          mbar_arrive_expect_tx(bar, STAGE_BYTES - TILE_A - (with_q ? 0 : TILE_QK) - (m_pass ? TILE_V : 0));
           tma_load_2d(st + TILE_QK, &map_k, hq * D, y, bar);
           tma_load_2d(st + TILE_QK + 8192, &map_k, hq * D + 64, y, bar);
-          tma_load_2d(st + 2 * TILE_QK, &map_v, hv * D, y, bar);
-          tma_load_2d(st + 2 * TILE_QK + 8192, &map_v, hv * D + 64, y, bar);
+          if (!m_pass) {
+            tma_load_2d(st + 2 * TILE_QK, &map_v, hv * D, y, bar);
+            tma_load_2d(st + 2 * TILE_QK + 8192, &map_v, hv * D + 64, y, bar);
+          }
           if (with_q) {
             tma_load_2d(st, &map_q, hq * D, y, bar);
             tma_load_2d(st + 8192, &map_q, hq * D + 64, y, bar);
@@ -983,13 +1011,22 @@ int launch_fwd_tc(const fqla_fwd_args& a, int N, SeqLayout lay, cudaStream_t st)
   p.N = N; p.Hq = a.Hq; p.Hv = a.Hv; p.T_rows = T_rows; p.scale = a.scale; p.lay = lay;
   p.tiled = a.operand_tiles; p.lead = a.lead_chunks; p.run_mask = a.run_mask;
   p.run_value = a.run_value; p.order = a.seq_order;
+  p.M = a.M; p.warm = a.warm_chunks; p.m_mask = a.m_mask; p.m_first = INT_MAX;
+  int blocks = N * a.Hv;
   auto launch = [&](auto kernel, int smem_bytes, std::atomic<unsigned long long>& done) {
     int err = configure_smem((const void*)kernel, smem_bytes, done);
     if (err != 0) return err;
-    return launch_pdl(kernel, dim3((unsigned)(N * a.Hv)), dim3(512), (size_t)smem_bytes, st, p, mq, mk,
+    return launch_pdl(kernel, dim3((unsigned)blocks), dim3(512), (size_t)smem_bytes, st, p, mq, mk,
                       mv, ma, mh, mvn, mo);
   };
-  static std::atomic<unsigned long long> done[5];
+  static std::atomic<unsigned long long> done[6];
+  if (!a.q && !a.o && !a.h && !a.vnew) {  // end states and transition matrices
+    if (a.M) {
+      p.m_first = a.ht ? blocks : 0;
+      blocks += p.m_first;
+    }
+    return launch(fwd_tc_kernel<false, true, false>, SMEM_BYTES, done[5]);
+  }
   if (!a.q && !a.o)  // recomputation of h, v_new
     return launch(fwd_tc_kernel<true, true, false>, SMEM_BYTES_EXTRA, done[0]);
   if (a.h || a.vnew)
