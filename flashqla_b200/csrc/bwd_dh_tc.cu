@@ -59,6 +59,7 @@ struct BwdDhTcParams {
   // [N, Hv] or null (dh0 only): only the first warm[n,hv] chunks are walked, from a zero gradient
   // (< 0: nothing is done)
   const int* warm;
+  int* zero_word;  // or null: set to zero (a counter of the kernel behind this one)
 };
 
 namespace bdtc {
@@ -156,6 +157,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
   if (warp == 0) tmem_alloc(tmem_slot, 512);
   // everything above overlaps the tail of the kernel before: no global memory up to here
   pdl_wait();
+  if (p.zero_word && blockIdx.x == 0 && tid == 0) *p.zero_word = 0;
   const int n = sequence();
   const SeqSpan sp = p.lay.span(n);
   // iteration `it` handles chunk n_it - 1 - it of the segment; chunks >= sp.n_chunks are the
@@ -687,6 +689,7 @@ int launch_bwd_dh_tc(const fqla_bwd_dh_args& a, int N, SeqLayout lay, cudaStream
   p.run_mask = a.run_mask;
   p.run_value = a.run_value;
   p.warm = a.warm_chunks;
+  p.zero_word = a.zero_word;
   p.g = a.g_cum; p.beta = a.beta; p.beta_is_f32 = a.beta_is_f32;
   p.dht = a.dht; p.seg_dht = a.seg_dht; p.dht_row = a.dht_row; p.dh0_row = a.dh0_row;
   p.v_first = a.state_v_first;

@@ -44,6 +44,7 @@ struct BwdMainTcParams {
   void* db;                // fp32 or (db_bf16) bf16
   float* dg;
   int dg_cumsum, db_bf16;  // see fqla_bwd_main_args
+  int* next_item;          // zero at launch, or null: see the walk of the items below
   int Hq, Hv;
   float scale;
   SeqLayout lay;
@@ -71,9 +72,11 @@ constexpr int OFF_DW = OFF_DA + 8192;       // -du h^T
 // chunk total (16)
 constexpr int OFF_VEC = OFF_DW + ROW_TILE;
 constexpr int OFF_BAR = OFF_VEC + (4 * 64 + 5 * 256 + 512 + 18) * 4;
-constexpr int N_BARS = 20;
+constexpr int N_BARS = 22;
 constexpr int OFF_MISC = OFF_BAR + N_BARS * 8;
-constexpr int SMEM_BYTES = OFF_MISC + 16 + 1024;
+constexpr int OFF_ITEM = OFF_MISC + 32;  // ring of four items, published by the issue warp
+constexpr int SMEM_BYTES = OFF_ITEM + 4 * 32 + 1024;
+static_assert(SMEM_BYTES <= 232448, "one CTA's shared memory");
 // the operand tiles of one item arrive in three groups, in the order their buffers become free
 constexpr uint32_t TX_A = 2 * SQ_TILE + 3 * ROW_TILE;  // h, dh, dO, v_new, k (other buffer)
 constexpr uint32_t TX_B = 3 * ROW_TILE;                // du, q, v
@@ -91,7 +94,9 @@ enum {
   C_DW, C_DSQK, C_1B, C_X, C_2B, C_T, C_D3, C_5,           // product groups complete (commit)
   R_ZERO, R_END,                     // all 16 read-out warps -> issue warp
   R_DW, R_DS, R_DA, R_T, R_D3,       // the 8 warps of the chain group -> issue warp
-  R_HD, R_E4                         // the 8 warps of the bulk group -> issue warp
+  R_HD, R_E4,                        // the 8 warps of the bulk group -> issue warp
+  R_CH,                              // the 8 warps of the chain group -> bulk group: item finished
+  I_NEXT                             // issue warp -> read-out warps: the next item is in the ring
 };
 }  // namespace bmtc
 
@@ -120,9 +125,19 @@ __device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, float (&v)[8]) {
 __device__ __forceinline__ void epi_barrier() {  // the 16 read-out warps only
   asm volatile("bar.sync 1, 512;" ::: "memory");
 }
+__device__ __forceinline__ void chain_barrier() {  // warps 0-7
+  asm volatile("bar.sync 4, 256;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_barrier() {  // warps 8-15
+  asm volatile("bar.sync 5, 256;" ::: "memory");
+}
 
-// Persistent: CTA b handles work items b, b + gridDim.x, ...; item w = (chunk w / Hv, head w % Hv),
-// so neighbouring CTAs share q and k of a grouped-value-attention group through L2.
+// Persistent: CTA b starts with work item b and takes the next one that nobody has (next_item counts
+// them out; without it b + gridDim.x, ...); item w = (chunk w / Hv, head w % Hv), so neighbouring CTAs
+// share q and k of a grouped-value-attention group through L2.  SMs differ in speed by a fifth
+// (instruction fetch), and with a fixed share each the fast ones run away: a tail, and CTAs working
+// far apart in memory.  262144 tokens x 8 heads, 7.1 GB: 1479 us (4.8 TB/s) counted out, 1970-2090 us
+// with a fixed share, 1650 us with a fixed share and the 16 warps in step (see the end of an item).
 // TILED: h, dh, vnew and du arrive in the operand layouts written by the sequential kernels
 // (h^T, dh^T as [V][K] per chunk; vnew^T, du^T as [V][64] per chunk) instead of row-major.
 template <bool TILED>
@@ -139,7 +154,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_MISC);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + OFF_MISC + 4);
-  volatile int* stop_flag = reinterpret_cast<volatile int*>(smem + OFF_MISC + 8);  // [2], by item parity
+  volatile int* stop_flag = reinterpret_cast<volatile int*>(smem + OFF_MISC + 8);  // [group][item parity]
   // per-row vectors g, gamma, rho, beta of an item: two buffers (item parity), the second one
   // behind the column sums
   float* sVec0 = reinterpret_cast<float*>(smem + OFF_VEC);
@@ -158,45 +173,54 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
     long long row0, chunk_id;
     int valid, hv, hq;
   };
-  // item w = (chunk w / Hv, head w % Hv); a CTA steps by gridDim.x items: no division per item
-  const int step_c = (int)gridDim.x / p.Hv, step_h = (int)gridDim.x % p.Hv, group = p.Hv / p.Hq;
-  auto advance = [&](int& cidx, int& hv) {
-    cidx += step_c;
-    hv += step_h;
-    if (hv >= p.Hv) {
-      hv -= p.Hv;
-      ++cidx;
+  Item* ring = reinterpret_cast<Item*>(smem + OFF_ITEM);
+  const int group = p.Hv / p.Hq;
+  // Claiming an item and reading the tables of a packed batch are three dependent loads.  The issue
+  // warp spreads them over the waits of the item before, the low words (row numbers fit) straight
+  // into the registers they stay in, and hands the item to the read-out warps through a ring in
+  // shared memory: read where the item begins the tables cost every warp 1500 of 14500 cycles.
+  struct Raw {
+    int seq, ci, begin, end, base;
+  };
+  auto low = [](const IndexTable& t, int i) { return reinterpret_cast<const int*>(t.ptr)[t.is64 ? 2 * i : i]; };
+  auto load_index = [&](int cidx, Raw& r) {
+    if (p.lay.cu.ptr) {
+      r.seq = low(p.chunk_indices, 2 * cidx);
+      r.ci = low(p.chunk_indices, 2 * cidx + 1);
+    } else {
+      const int per = (p.lay.T + CHUNK - 1) / CHUNK;
+      r.seq = cidx / per;
+      r.ci = cidx % per;
     }
   };
-  auto decode = [&](int cidx, int hv) {
+  auto load_span = [&](Raw& r) {
+    if (p.lay.cu.ptr) {
+      r.begin = low(p.lay.cu, r.seq);
+      r.end = low(p.lay.cu, r.seq + 1);
+      r.base = low(p.lay.chunk_offsets, r.seq);
+    }
+  };
+  auto finish = [&](const Raw& r, int hv) {
     Item t;
     t.hv = hv;
     t.hq = hv / group;
-    int seq, ci;
-    if (p.lay.cu.ptr) {
-      seq = (int)p.chunk_indices[2 * cidx];
-      ci = (int)p.chunk_indices[2 * cidx + 1];
-    } else {
-      const int per = (p.lay.T + CHUNK - 1) / CHUNK;
-      seq = cidx / per;
-      ci = cidx % per;
-    }
-    const SeqSpan sp = p.lay.span(seq);
-    t.row0 = sp.bos + (long long)ci * CHUNK;
+    const bool packed = p.lay.cu.ptr != nullptr;
+    const long long bos = packed ? r.begin : (long long)r.seq * p.lay.T;
+    const int len = packed ? r.end - r.begin : p.lay.T;
+    t.row0 = bos + (long long)r.ci * CHUNK;
     // clamped: a table row that does not belong to its sequence must not index outside the tiles
-    t.valid = max(1, min(CHUNK, sp.len - ci * CHUNK));
-    t.chunk_id = sp.chunk_base + ci;
+    t.valid = max(1, min(CHUNK, len - r.ci * CHUNK));
+    t.chunk_id = (packed ? r.base : (long long)r.seq * ((p.lay.T + CHUNK - 1) / CHUNK)) + r.ci;
     return t;
   };
-
   if (tid == 0) {
     for (int i = L_A; i <= C_5; ++i) mbar_init(&bars[i], 1);
     mbar_init(&bars[R_ZERO], N_EPI / 32);
     mbar_init(&bars[R_END], N_EPI / 32);
-    for (int i = R_DW; i <= R_E4; ++i) mbar_init(&bars[i], N_EPI / 64);
+    for (int i = R_DW; i <= R_CH; ++i) mbar_init(&bars[i], N_EPI / 64);
+    mbar_init(&bars[I_NEXT], 1);
     *abort_flag = 0;
-    stop_flag[0] = 0;
-    stop_flag[1] = 0;
+    for (int i = 0; i < 4; ++i) stop_flag[i] = 0;
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(tmem_slot, 512);
@@ -274,29 +298,30 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       constexpr uint32_t ID_MK_128 = idesc_bf16(64, 128, 1, 0);
       constexpr uint32_t KBUF_LO = ROW_TILE >> 4;
 
-      int at_c = (int)blockIdx.x / p.Hv, at_h = (int)blockIdx.x % p.Hv;
-      Item cur = decode(at_c, at_h);
+      Raw raw = {};
+      int claimed = (int)blockIdx.x;  // in lane 0
+      auto claim = [&] {
+        if (lane == 0) claimed = p.next_item ? (int)gridDim.x + atomicAdd(p.next_item, 1) : claimed + (int)gridDim.x;
+      };
+      load_index((int)blockIdx.x / p.Hv, raw);
+      load_span(raw);
+      Item cur = finish(raw, (int)blockIdx.x % p.Hv);
       load_a(cur, 0);
       load_b(cur);
       load_c(cur);
       bool ok = true;
       uint32_t it = 0;
 #pragma unroll 1
-      for (long long w = blockIdx.x; w < total && ok; w += gridDim.x, ++it) {
+      for (bool has_next = true; has_next && ok; ++it) {
         const uint32_t ph = it & 1;
-        const bool has_next = w + gridDim.x < total;
-        Item nxt = cur;
-        if (has_next) {
-          advance(at_c, at_h);
-          nxt = decode(at_c, at_h);
-        }
+        claim();
         const uint32_t k_lo = k_lo0 + (ph ? KBUF_LO : 0u), kmn_lo = kmn_lo0 + (ph ? KBUF_LO : 0u);
         // the read-out warps have finished the previous item (accumulators free) and have zeroed
         // the rows past the sequence end in this item's tiles (which also means: tiles landed)
         // A full chunk needs no zero fill: its first products start as soon as its tiles have
         // landed, while the bulk group still finishes the previous item (the accumulators they
-        // write were last read by the chain group, whose R_D3 this thread has seen; dq1 | dk1 come
-        // after R_DW of this item, which the read-out warps only give after the previous item).
+        // write were last read by the chain group, whose R_D3 this thread has seen; dq1 | dk1 and
+        // what follows wait for R_END of the previous item).
         if (cur.valid == CHUNK) ok = WAIT(L_A, ph) && WAIT(L_B, ph);
         else ok = (it == 0 || WAIT(R_END, (it - 1) & 1)) && WAIT(R_ZERO, ph);
         if (!ok) break;
@@ -326,7 +351,14 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           if constexpr (TILED) umma_group<8, 128, 512, 2, 512, false>(tmem + T_X2, duT_lo, v_lo, ID_MK_64);
           else umma_group<8, 2, 512, 2, 512, false>(tmem + T_X2, du_lo, v_lo, ID_KK_64);
           umma_commit(&bars[C_X]);
-          // products off the dependent chain go behind the ones the read-out is waiting for
+        }
+        // products off the dependent chain go behind the ones the read-out is waiting for
+        if (it > 0) {
+          ok = WAIT(R_END, (it - 1) & 1);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        if (elect_one()) {
           if constexpr (TILED) {
             umma_group<8, 2, 512, 128, 512, false>(tmem + T_DQ1, do_lo, hT_lo, ID_KM_128);
             umma_group<8, 128, 512, 128, 512, false>(tmem + T_DK1, vnT_lo, dhT_lo, ID_MM_128);
@@ -336,6 +368,10 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           }
           umma_commit(&bars[C_1B]);
         }
+        const int w_next = __shfl_sync(0xffffffffu, claimed, 0);
+        has_next = w_next < (int)total;
+        const int h_next = has_next ? w_next % p.Hv : 0;
+        if (has_next) load_index(w_next / p.Hv, raw);
         // ---- ds is an operand now ----
         ok = WAIT(R_DS, ph);
         if (!ok) break;
@@ -345,11 +381,20 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           umma_group<4, 128, 0, 128, 0, false>(tmem + T_DK2, dsmn_lo, qmn_lo, ID_MM_128);
           umma_group<8, 2, 512, 2, 512, false>(tmem + T_KK, k_lo, k_lo, ID_KK_64);  // qk has been read
         }
+        if (has_next) load_span(raw);
         // h, dh, dO, v_new are dead once the first products are complete and the h.dh sum is done
+        ok = WAIT(C_1B, ph) && WAIT(R_HD, ph);
+        if (!ok) break;
+        Item nxt = cur;
         if (has_next) {
-          ok = WAIT(C_1B, ph) && WAIT(R_HD, ph);
-          if (!ok) break;
+          nxt = finish(raw, h_next);
           load_a(nxt, (int)(ph ^ 1));
+        } else {
+          nxt.valid = 0;  // the read-out warps stop
+        }
+        if (lane == 0) {
+          ring[(it + 1) & 3] = nxt;
+          mbar_arrive(&bars[I_NEXT]);
         }
         // ---- dA -> T = A^T dA (and K K^T) ----
         ok = WAIT(R_DA, ph);
@@ -535,24 +580,19 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         else reinterpret_cast<float*>(p.db)[i] = dbv;
       }
     };
-    int at_c = (int)blockIdx.x / p.Hv, at_h = (int)blockIdx.x % p.Hv;
-    Item cur = decode(at_c, at_h);
+    Raw raw = {};
+    load_index((int)blockIdx.x / p.Hv, raw);
+    load_span(raw);
+    Item cur = finish(raw, (int)blockIdx.x % p.Hv);
     long long prev_first = 0;
     int prev_rows = 0;
     fetch_vectors(cur);
     write_vectors(cur, sVec0);
     epi_barrier();
     uint32_t it = 0;
-    bool stopped = false;
 #pragma unroll 1
-    for (long long w = blockIdx.x; w < total; w += gridDim.x, ++it) {
+    for (;; ++it) {
       const uint32_t ph = it & 1;
-      const bool has_next = w + gridDim.x < total;
-      Item nxt = cur;
-      if (has_next) {
-        advance(at_c, at_h);
-        nxt = decode(at_c, at_h);
-      }
       const int valid = cur.valid;
       const int koff = OFF_K + (int)ph * ROW_TILE;
       const float* sG = ph ? sVec1 : sVec0;
@@ -570,7 +610,12 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         }
       }
       signal(R_ZERO);
-      if (has_next) fetch_vectors(nxt);
+      Item nxt;
+      // the next item, from the middle of this one on
+      auto take_next = [&] {
+        ok = ok && WAIT(I_NEXT, ph);
+        nxt = ring[(it + 1) & 3];
+      };
       float acc_last = 0.f;
 
       if (chain) {
@@ -665,6 +710,8 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           }
         }
         signal(R_DA);
+        take_next();
+        if (ok && nxt.valid > 0) fetch_vectors(nxt);
 
         // ---- E5: T = A^T dA as an operand tile (over dA, which the product has consumed) ----
         ok = ok && WAIT(C_T, ph);
@@ -714,7 +761,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         signal(R_D3);
         signal(R_END);  // this group no longer touches the accumulators or the tiles of the item
         // The partial-sum slots were read for the previous item by threads of the bulk group, which
-        // arrive on R_E4 of this item only after that: long complete by now.
+        // arrive on R_E4 of this item only after that.
         ok = ok && WAIT(R_E4, ph);
         // one reduction per quantity, one plain store per (warp, row or column): no atomics
         acc_dg_a = quad_sum(acc_dg_a);
@@ -832,22 +879,37 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         for (int d = 16; d > 0; d >>= 1) acc_last += __shfl_xor_sync(0xffffffffu, acc_last, d);
         if (lane == 0) sLast[gw] = acc_last;
       }
-      // One barrier per item: every contribution to dg, db of this item is in, and the vectors of
-      // the next item are in place (other buffer).  The stop flag alternates as well, so that it
-      // is read by all before it can be written again.
-      if (has_next) write_vectors(nxt, ph ? sVec0 : sVec1);
+      // The chain group goes on to the next item as soon as it is through; the bulk group, which
+      // ends an item with the wide read-outs, follows at most an item behind (R_E4) and finds the
+      // chain group's contributions to dg, db and the vectors of the next item (other buffer)
+      // behind R_CH.  (One barrier of all sixteen warps here held the chain group for the last
+      // wide read-out, 1600 of 14500 cycles per item.)  Each group has a stop flag of its own, by
+      // item parity, so that it is read by the whole group before it can be written again.
+      if (chain) {
+        if (nxt.valid > 0) write_vectors(nxt, ph ? sVec0 : sVec1);
+      } else {
+        take_next();
+        ok = ok && WAIT(R_CH, ph);
+      }
       if (!ok) *abort_flag = 1;
-      if (tid == 0) stop_flag[ph] = *abort_flag;
-      epi_barrier();
+      volatile int* stop = stop_flag + (chain ? 0 : 2) + ph;
+      if ((tid & 255) == 0) *stop = *abort_flag ? 1 : nxt.valid > 0 ? 0 : 2;
+      if (chain) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars[R_CH]);
+        chain_barrier();
+      } else {
+        bulk_barrier();
+      }
       prev_first = cur.row0 * p.Hv + cur.hv;
       prev_rows = cur.valid;
       cur = nxt;
-      if (stop_flag[ph]) {  // written before the barrier by one thread: uniform
-        stopped = true;
+      const int how = *stop;  // written before the barrier by one thread: uniform in the group
+      if (how) {
+        if (how == 2) combine(prev_first, prev_rows);  // (1: some wait was given up)
         break;
       }
     }
-    if (it > 0 && !stopped) combine(prev_first, prev_rows);
   }
   tc_fence_before();
   __syncthreads();
@@ -949,6 +1011,7 @@ int launch_bwd_main_tc(const fqla_bwd_main_args& a, long long n_chunks, SeqLayou
   p.dg_cumsum = a.dg_cumsum; p.db_bf16 = a.db_is_bf16;
   p.Hq = Hq; p.Hv = Hv; p.scale = a.scale; p.lay = lay; p.chunk_indices = chunk_indices;
   p.n_chunks = n_chunks;
+  p.next_item = a.next_item;
   static std::atomic<unsigned long long> done[2];
   rc = configure_smem(a.operand_tiles ? (const void*)bwd_main_tc_kernel<true> : (const void*)bwd_main_tc_kernel<false>,
                       SMEM_BYTES, done[a.operand_tiles ? 1 : 0]);

@@ -403,6 +403,11 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
   d.state_v_first = opt.state_v_first;
   d.lead_chunks = ptr<int>(lead_out);
   d.operand_tiles = tiles;
+  at::Tensor counter;  // hands out the items of the chunk-parallel kernel
+  if (tiles) {
+    counter = empty({1}, at::kInt, c.dev);
+    d.zero_word = counter.data_ptr<int>();
+  }
   if (c.split) {
     d.seg_dht = ptr<float>(seg_dht);
     d.dht_row = c.batch->raw_last;
@@ -429,6 +434,7 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
   m.Hv = c.Hv; m.D = c.D; m.scale = c.scale; m.cu_seqlens = c.cu(); m.chunk_offsets = c.offsets();
   m.chunk_indices = c.indices(); m.num_chunks = c.batch->num_chunks; m.operand_tiles = tiles;
   m.dg_cumsum = 1; m.db_is_bf16 = db_bf16;
+  if (tiles) m.next_item = counter.data_ptr<int>();
   check(fqla_bwd_main_run(&m, c.stream), "bwd_main");
   const bool f16 = dtype == at::kHalf;
   if (c.Hq < c.Hv || norm || f16) {

@@ -145,7 +145,8 @@ int fqla_bwd_dh(const void* q, const void* k, const void* A, const float* g_cum,
 /* fqla_bwd_dh with every argument in one structure, zero-initialised by the caller.  dht_row [N]:
  * sequence n starts from dht[dht_row[n]] where that is >= 0, else from seg_dht[n] (zero without
  * seg_dht); dh0_row [N]: dh0 of sequence n goes to dh0[dh0_row[n]] where that is >= 0;
- * state_v_first: dht and dh0 are [value dim][key dim].  As in fqla_fwd_args. */
+ * state_v_first: dht and dh0 are [value dim][key dim].  As in fqla_fwd_args.  zero_word (optional, K =
+ * V = 128, tcgen05 kernel only): one int that is set to zero (next_item of fqla_bwd_main_args). */
 typedef struct fqla_bwd_dh_args {
   const void *q, *k, *A;
   const float* g_cum;
@@ -161,6 +162,7 @@ typedef struct fqla_bwd_dh_args {
   float scale;
   const void *cu_seqlens, *chunk_offsets;
   int idx_is64, N, operand_tiles, state_v_first;
+  int* zero_word;
 } fqla_bwd_dh_args;
 int fqla_bwd_dh_run(const fqla_bwd_dh_args* args, void* stream);
 
@@ -178,7 +180,9 @@ int fqla_bwd_main(const void* q, const void* k, const void* v, const void* vnew,
 
 /* fqla_bwd_main with every argument in one structure, zero-initialised by the caller.  dg_cumsum: dg
  * comes out after its reverse chunk-local cumulative sum (what fqla_chunk_local_cumsum, reverse,
- * would make of it); db_is_bf16: db is bf16 instead of fp32. */
+ * would make of it); db_is_bf16: db is bf16 instead of fp32; next_item (optional, D = 128): one int,
+ * zero when the kernel starts, of which the launch is the only user: its CTAs then take the
+ * (chunk, head) items as they go instead of a fixed share each. */
 typedef struct fqla_bwd_main_args {
   const void *q, *k, *v, *vnew, *A;
   const float* g_cum;
@@ -193,6 +197,7 @@ typedef struct fqla_bwd_main_args {
   int idx_is64;
   long long num_chunks;
   int operand_tiles, dg_cumsum, db_is_bf16;
+  int* next_item;
 } fqla_bwd_main_args;
 int fqla_bwd_main_run(const fqla_bwd_main_args* args, void* stream);
 
