@@ -1022,8 +1022,23 @@ int launch_bwd_main_tc(const fqla_bwd_main_args& a, long long n_chunks, SeqLayou
   if (n_sm <= 0) n_sm = 148;
   const long long total = n_chunks * Hv;
   const unsigned grid = (unsigned)(total < n_sm ? total : n_sm);
-  return launch_pdl(a.operand_tiles ? bwd_main_tc_kernel<true> : bwd_main_tc_kernel<false>, dim3(grid), dim3(NT),
-                    (size_t)SMEM_BYTES, st, p, mq, mk, mv, mvn, mdo, mdu, mh, mdh, ma);
+  // A caller without a counter gets one for this launch, in stream order (also under capture); where
+  // that cannot be had, or with a handful of items per CTA, each CTA takes its fixed share.
+  void* own = nullptr;
+  if (!p.next_item && total > 4ll * n_sm) {
+    if (cudaMallocAsync(&own, sizeof(int), st) == cudaSuccess &&
+        cudaMemsetAsync(own, 0, sizeof(int), st) == cudaSuccess)
+      p.next_item = (int*)own;
+    else
+      cudaGetLastError();
+  }
+  rc = launch_pdl(a.operand_tiles ? bwd_main_tc_kernel<true> : bwd_main_tc_kernel<false>, dim3(grid), dim3(NT),
+                  (size_t)SMEM_BYTES, st, p, mq, mk, mv, mvn, mdo, mdu, mh, mdh, ma);
+  if (own) {
+    const int freed = (int)cudaFreeAsync(own, st);
+    if (rc == 0) rc = freed;
+  }
+  return rc;
 }
 
 }  // namespace fqla

@@ -181,8 +181,8 @@ int fqla_bwd_main(const void* q, const void* k, const void* v, const void* vnew,
 /* fqla_bwd_main with every argument in one structure, zero-initialised by the caller.  dg_cumsum: dg
  * comes out after its reverse chunk-local cumulative sum (what fqla_chunk_local_cumsum, reverse,
  * would make of it); db_is_bf16: db is bf16 instead of fp32; next_item (optional, D = 128): one int,
- * zero when the kernel starts, of which the launch is the only user: its CTAs then take the
- * (chunk, head) items as they go instead of a fixed share each. */
+ * zero when the kernel starts, of which the launch is the only user: its CTAs take the
+ * (chunk, head) items as they go.  Without it a large launch allocates one in stream order. */
 typedef struct fqla_bwd_main_args {
   const void *q, *k, *v, *vnew, *A;
   const float* g_cum;
