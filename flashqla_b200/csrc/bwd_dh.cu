@@ -303,15 +303,21 @@ __global__ void __launch_bounds__(256, 1) bwd_dh_kernel(const BwdDhParams p) {
   }
 }
 
-template <int D>
-static int launch_bwd_dh(const BwdDhParams& p, cudaStream_t st) {
-  constexpr int BV = 64;
+template <int D, int BV>
+static int launch_slices(const BwdDhParams& p, cudaStream_t st) {
   using L = BwdDhSmem<D, BV>;
   static std::atomic<unsigned long long> done;
   int rc = configure_smem((const void*)bwd_dh_kernel<D, BV>, L::BYTES, done);
   if (rc != 0) return rc;
   dim3 grid((unsigned)(p.N * p.Hv), D / BV);
   return launch_pdl(bwd_dh_kernel<D, BV>, grid, dim3(256), L::BYTES, st, p);
+}
+template <int D>
+static int launch_bwd_dh(const BwdDhParams& p, cudaStream_t st) {
+  // narrower slices while every CTA has an SM of its own (see fwd_seq.cu; 512 tokens x 4 heads,
+  // D = 64: MEASURED_DH)
+  if (D == 64 && (long long)p.N * p.Hv * 2 <= sm_count()) return launch_slices<D, 32>(p, st);
+  return launch_slices<D, 64>(p, st);
 }
 
 // tcgen05 version for K = V = 128, full walks only (bwd_dh_tc.cu)

@@ -24,6 +24,14 @@ inline int configure_smem(const void* func, int bytes, std::atomic<unsigned long
   return (int)e;
 }
 
+// SMs of the current device (which may differ from call to call)
+inline int sm_count() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n > 0 ? n : 148;
+}
+
 // Launch with programmatic stream serialisation: the kernel's blocks may start while the kernel
 // before it in the stream drains, and its set-up (barriers, tensor memory, descriptor prefetch)
 // overlaps that tail and the launch latency.  Every such kernel executes pdl_wait() in every

@@ -348,15 +348,22 @@ __global__ void __launch_bounds__(256, 1) fwd_seq_kernel(const FwdSeqParams p) {
   }
 }
 
-template <int D>
-static int launch_fwd_seq(const FwdSeqParams& p, cudaStream_t st) {
-  constexpr int BV = 64;
+template <int D, int BV>
+static int launch_slices(const FwdSeqParams& p, cudaStream_t st) {
   using L = FwdSeqSmem<D, BV>;
   static std::atomic<unsigned long long> done;
   int rc = configure_smem((const void*)fwd_seq_kernel<D, BV>, L::BYTES, done);
   if (rc != 0) return rc;
   dim3 grid((unsigned)(p.N * p.Hv), (D / BV) * (p.M ? 2 : 1));
   return launch_pdl(fwd_seq_kernel<D, BV>, grid, dim3(256), L::BYTES, st, p);
+}
+template <int D>
+static int launch_fwd_seq(const FwdSeqParams& p, cudaStream_t st) {
+  // Columns of the state are independent.  While every CTA still has an SM of its own, slices half as
+  // wide shorten the chain of a chunk (512 tokens x 4 heads, D = 64: MEASURED_FWD); past that
+  // they would only repeat Q K^T and the loads of q, k, A.
+  if (D == 64 && (long long)p.N * p.Hv * (p.M ? 4 : 2) <= sm_count()) return launch_slices<D, 32>(p, st);
+  return launch_slices<D, 64>(p, st);
 }
 
 }  // namespace fqla
