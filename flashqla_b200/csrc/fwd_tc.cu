@@ -35,6 +35,15 @@
 //     warp 0  : issues the products of the chain, warp 1 all others (one elected lane each)
 //     warp 2  : producer: per-chunk gate vectors (fetched one chunk ahead), TMA loads of the
 //               q, k, v, A tiles (2 stages), zero-fill of rows past the end of a partial chunk
+//
+// The state-only pass of the exact hand-off (end states and transition matrices of segments) is a
+// chain of its own, because its roundings go into every segment behind the hand-off: A diag(beta),
+// A diag(beta gamma) and w, each rounded to bf16, are not formed.  Instead
+//     U^T [v x tok] = S^T K^T,  W^T = beta (V^T - gamma U^T),  Vn^T = W^T A^T
+// three products deep, W^T and rho Vn^T made by the V and the O group together (32 tokens each), warp 0
+// issuing everything.  W^T goes into its product as bf16; as the diagonal of A is one, what that rounding
+// left out is simply added to Vn^T.  (Error of o of the heads that never forget, against 64 bits, 8192 to
+// 16384 tokens: see the figures at the dispatch in fwd_seq.cu.)
 // Synchronisation is by mbarriers only; every wait is bounded and reports through a status word.
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -148,6 +157,10 @@ constexpr uint32_t TM_O2 = 384;   // O2^T fp32                      64 columns
 // same columns: w^T is issued only after the output group has read P, and the next P only after
 // the value group has turned w^T into its operand tile (the chain's first product waits for it).
 constexpr uint32_t TM_PW = 448;
+// state-only pass
+constexpr uint32_t TM_U = TM_UV;    // U^T fp32                   64 columns
+constexpr uint32_t TM_WB = TM_VNB;  // W^T bf16 (A operand)       32 columns
+constexpr uint32_t TM_VN = TM_O1;   // Vn^T fp32                  64 columns
 // barrier indices
 enum { FULL0 = 0, FULL1, EMPTY0, EMPTY1, S_COPY, S_DEC, VN_DONE, S_DONE, P_DONE, O_DONE, W_DONE,
        VB_READY, W_READY, P_READY, O_FREE, AP_READY, PRIV,
@@ -156,8 +169,11 @@ enum { FULL0 = 0, FULL1, EMPTY0, EMPTY1, S_COPY, S_DEC, VN_DONE, S_DONE, P_DONE,
        // tile outputs: the shared-memory copies of S^T / Vn^T are complete
        ST_READY, VN_READY,
        // the output product that reads the packed copy of S^T has completed
-       SB_FREE };
-// vectors inside a slot; V_GL holds gamma_last at [0]
+       SB_FREE,
+       // state-only pass: U^T is complete; W^T, made by the V and the O group, is (its name there)
+       U_DONE = P_DONE, WB_READY = P_READY };
+// vectors inside a slot; V_GL holds gamma_last at [0], V_BG gamma instead of beta gamma in the
+// state-only pass
 enum { V_G = 0, V_BETA = 1, V_BG = 2, V_RHO = 3, V_SGAM = 4, V_GL = 5 };
 }  // namespace fwdtc
 
@@ -178,8 +194,9 @@ __device__ __forceinline__ uint32_t pack_out(float lo, float hi) {
 
 // EXTRA: per-chunk state and v_new outputs (compiled out of the common instantiation: the six
 // roles run six different code regions at once, and the kernel is sensitive to its
-// instruction-cache footprint).  NO_O: state-only walk, no q, no output products, the output warps
-// stay idle: with EXTRA the recomputation for the backward pass, without it end states and M.  O_F16: o leaves as fp16 instead of bf16.
+// instruction-cache footprint).  NO_O: state-only walk, no q, no output products: with EXTRA the
+// recomputation for the backward pass (the output warps only scale A), without it (STATE) the end states
+// and M of the exact hand-off.  O_F16: o leaves as fp16 instead of bf16.
 template <bool EXTRA, bool NO_O, bool O_F16>
 __global__ void __launch_bounds__(512, 1)
 fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
@@ -223,13 +240,14 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   if (tid == 0) {
     mbar_init(&bars[FULL0], 1);
     mbar_init(&bars[FULL1], 1);
-    mbar_init(&bars[EMPTY0], 2);  // MMA commits of the two issuing threads
-    mbar_init(&bars[EMPTY1], 2);
+    mbar_init(&bars[EMPTY0], STATE ? 1 : 2);  // MMA commits of the issuing threads
+    mbar_init(&bars[EMPTY1], STATE ? 1 : 2);
     mbar_init(&bars[SB_FREE], 1);
     mbar_init(&bars[FULLA0], 1);
     mbar_init(&bars[FULLA1], 1);
-    mbar_init(&bars[EMPTYA0], 128);  // the output group, the only reader of the raw A tile
-    mbar_init(&bars[EMPTYA1], 128);
+    // the only reader of the raw A tile: the output group, or (STATE) a product
+    mbar_init(&bars[EMPTYA0], STATE ? 1 : 128);
+    mbar_init(&bars[EMPTYA1], STATE ? 1 : 128);
     mbar_init(&bars[PRIVA], 1);
     mbar_init(&bars[S_COPY], 128);
     mbar_init(&bars[S_DEC], 128);
@@ -238,9 +256,9 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     mbar_init(&bars[P_DONE], 1);
     mbar_init(&bars[O_DONE], 1);
     mbar_init(&bars[W_DONE], 1);
-    mbar_init(&bars[VB_READY], 128);
+    mbar_init(&bars[VB_READY], STATE ? 256 : 128);
     mbar_init(&bars[W_READY], 128);
-    mbar_init(&bars[P_READY], 128);
+    mbar_init(&bars[P_READY], STATE ? 256 : 128);
     mbar_init(&bars[O_FREE], 128);
     mbar_init(&bars[AP_READY], 128);
     mbar_init(&bars[PRIV], 1);
@@ -441,6 +459,64 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           for (int j = 0; j < 32; ++j) dst[(long long)(k0 + j) * D + v] = x[j];
         }
       }
+    }
+  } else if (STATE && warp >= 8) {
+    // =============================== V and O group, state-only pass ===============================
+    // Each takes 32 tokens of a chunk: U^T -> W^T = beta (V^T - gamma U^T), Vn^T -> rho Vn^T, both bf16
+    // operands in tensor memory.
+    const int v = (warp & 3) * 32 + lane;  // tensor-memory lane = value index
+    const int t0 = warp < 12 ? 0 : 32;
+    for (int it = 0; it < n_it && ok; ++it) {
+      const int s = it & 1;
+      ok = WAIT(FULL0 + s, (it >> 1) & 1);
+      if (!ok) break;
+      const float* vs = vec + (it & 3) * VEC_SLOT_FLOATS + t0;
+      // off the chain: this thread's value index of its 32 tokens
+      const unsigned char* vt = smem + OFF_STAGE + s * STAGE_BYTES + 2 * TILE_QK + (v >> 6) * 8192;
+      float x[32], y[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        y[j] = __bfloat162float(*reinterpret_cast<const bf16*>(vt + sw128_offset(t0 + j, v & 63)));
+      ok = WAIT(U_DONE, it & 1);
+      if (!ok) break;
+      tc_fence_after();
+      tmem_ld32(tmem + lane_sel + TM_U + t0, x);
+      tmem_ld_wait();
+      uint32_t pk[16];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 b = *reinterpret_cast<const float4*>(vs + V_BETA * CHUNK + 4 * i);
+        const float4 g = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 4 * i);
+        y[4 * i] = b.x * (y[4 * i] - g.x * x[4 * i]);
+        y[4 * i + 1] = b.y * (y[4 * i + 1] - g.y * x[4 * i + 1]);
+        y[4 * i + 2] = b.z * (y[4 * i + 2] - g.z * x[4 * i + 2]);
+        y[4 * i + 3] = b.w * (y[4 * i + 3] - g.w * x[4 * i + 3]);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {  // operand, and in y what its rounding left out
+        pk[i] = pack_bf16(y[2 * i], y[2 * i + 1]);
+        y[2 * i] -= __uint_as_float(pk[i] << 16);
+        y[2 * i + 1] -= __uint_as_float(pk[i] & 0xffff0000u);
+      }
+      tmem_st16(tmem + lane_sel + TM_WB + (t0 >> 1), pk);
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(&bars[WB_READY]);
+      ok = WAIT(VN_DONE, it & 1);
+      if (!ok) break;
+      tc_fence_after();
+      tmem_ld32(tmem + lane_sel + TM_VN + t0, x);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 r = *reinterpret_cast<const float4*>(vs + V_RHO * CHUNK + 4 * i);
+        pk[2 * i] = pack_bf16(r.x * (x[4 * i] + y[4 * i]), r.y * (x[4 * i + 1] + y[4 * i + 1]));
+        pk[2 * i + 1] = pack_bf16(r.z * (x[4 * i + 2] + y[4 * i + 2]), r.w * (x[4 * i + 3] + y[4 * i + 3]));
+      }
+      tmem_st16(tmem + lane_sel + TM_VRB + (t0 >> 1), pk);
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(&bars[VB_READY]);
     }
   } else if (warp >= 8 && warp < 12) {
     // =============================== V group ===============================
@@ -727,7 +803,43 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     constexpr uint32_t ID_OT = idesc_bf16(128, 64, 0, 0);            // A from tensor memory
     constexpr uint32_t ID_S = idesc_bf16(128, 128, 0, 1);
     constexpr uint32_t STAGE_LO = STAGE_BYTES >> 4;
-    if (warp == 0) {
+    if constexpr (STATE) {
+      auto SPIN = [&](int idx, uint32_t parity) { return mbar_wait_warp<true>(&bars[idx], parity, abort_flag); };
+      const uint32_t k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE_QK);
+      const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE_QK, 8192);
+      const uint32_t a0_lo = desc_lo_kmajor(smem + OFF_STAGE + 2 * TILE_QK + TILE_V);
+#pragma unroll 1
+      for (int it = 0; it < n_it && ok && warp == 0; ++it) {
+        const int s = it & 1, ph = (it >> 1) & 1;
+        const uint32_t so = s ? STAGE_LO : 0u;
+        ok = SPIN(FULL0 + s, ph) && SPIN(S_COPY, it & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          // U^T = S^T K^T   (A = packed S^T; B = K tile, K-major)
+          umma_ts_group_kmajor_b<8>(tmem + TM_U, tmem + TM_SB, k0_lo + so, ID_OT);
+          umma_commit(&bars[U_DONE]);
+        }
+        ok = SPIN(FULLA0 + s, ph) && SPIN(WB_READY, it & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          // Vn^T = W^T A^T   (A = packed W^T; B = A tile, K-major)
+          umma_ts_group<4, 8, 2, false>(tmem + TM_VN, tmem + TM_WB, a0_lo + so, ID_OT);
+          umma_commit(&bars[VN_DONE]);
+          umma_commit(&bars[EMPTYA0 + s]);
+        }
+        ok = SPIN(VB_READY, it & 1) && SPIN(S_DEC, it & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          // S^T += (rho Vn)^T K
+          umma_ts_group<4, 8, 128, true>(tmem + TM_S, tmem + TM_VRB, kmn0_lo + so, ID_S);
+          umma_commit(&bars[S_DONE]);
+          umma_commit(&bars[EMPTY0 + s]);
+        }
+      }
+    } else if (warp == 0) {
       auto SPIN = [&](int idx, uint32_t parity) { return mbar_wait_warp<true>(&bars[idx], parity, abort_flag); };
       auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
       // low descriptor words of every operand tile (see umma_lo); steps are 32-bit adds
@@ -933,7 +1045,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           float gam = fast_exp(g_r[z]);
           vs[V_G * CHUNK + r] = g_r[z];
           vs[V_BETA * CHUNK + r] = b_r[z];
-          vs[V_BG * CHUNK + r] = b_r[z] * gam;
+          vs[V_BG * CHUNK + r] = STATE ? gam : b_r[z] * gam;
           vs[V_RHO * CHUNK + r] = fast_exp(gl_r - g_r[z]);
           vs[V_SGAM * CHUNK + r] = p.scale * gam;
         }
