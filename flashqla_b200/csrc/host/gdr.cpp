@@ -107,6 +107,11 @@ void check_state(const OptTensor& s, const Call& c) {
                       "," + std::to_string(c.D) + "," + std::to_string(c.D) + "]");
 }
 
+void check_segments(const at::Tensor& t, const Call& c, const char* what) {
+  if (t.dim() < 2 || t.size(0) != c.batch->n_seg || t.size(1) != c.Hv)
+    throw PyError(PyError::Value, std::string("cp_cache: its ") + what + " belong to another batch");
+}
+
 bool tiles_ok(int D) {
   static const bool forced = std::getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
   return D == 128 && !forced;
@@ -369,8 +374,19 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
   // per-chunk states and v_new: kept by the forward, or recomputed
   OptTensor h = cached.h, vnew = cached.vnew;
   if (!h || !vnew) {
-    Cache starts{cached.seg_h0, std::nullopt, std::nullopt, cached.lead};
-    if (c.split && !starts.seg_h0) segment_starts(c, in, h0, opt, starts);
+    // start states and lead-in counts are per segment: of use only where this call runs over the
+    // segments they were made for (the forward may have been split where this call is not)
+    Cache starts;
+    if (c.split) {
+      if (cached.seg_h0) {
+        check_segments(*cached.seg_h0, c, "start states");
+        if (cached.lead) check_segments(*cached.lead, c, "lead-in counts");
+        starts.seg_h0 = cached.seg_h0;
+        starts.lead = cached.lead;
+      } else {
+        segment_starts(c, in, h0, opt, starts);
+      }
+    }
     h = empty({c.batch->num_chunks, c.Hv, c.D, c.D}, at::kBFloat16, c.dev);
     vnew = tiles ? empty({c.batch->num_chunks, c.Hv, c.D, CHUNK}, at::kBFloat16, c.dev)
                  : empty(v.sizes(), at::kBFloat16, c.dev);

@@ -1,0 +1,53 @@
+"""What the forward hands the backward (``cp_cache``) where the two calls are split differently, and
+where the per-chunk states are recomputed: same gradients as without a cache."""
+
+import pytest
+import torch
+
+from oracle import gdr_oracle as orc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("D", [128, 64])
+@pytest.mark.parametrize("fwd_cp,bwd_cp", [(True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("cu", [[0, 70, 4166, 6300], None], ids=["packed", "fixed"])
+def test_recomputation_takes_segment_tables_only_over_segments(D, fwd_cp, bwd_cp, cu, monkeypatch):
+    """Every sequence long enough is cut into segments; without the split the lead-in counts of
+    segments must not be read as those of sequences."""
+    import flash_qla.ops.gated_delta_rule.chunk as chunk
+    import flashqla_b200 as fq
+
+    B, T = (1, cu[-1]) if cu else (2, 3000)
+    x = orc.make_inputs(B, T, 1, 2, D, D, seed=9, cu_seqlens=torch.tensor(cu) if cu else None, with_h0=True)
+    d = {n: (x[n].bfloat16() if n in ("q", "k", "v", "beta", "do") else x[n]).to(DEV)
+         for n in ("q", "k", "v", "g", "beta", "h0", "do", "dht")}
+    cu_t = torch.tensor(cu, dtype=torch.int32, device=DEV) if cu else None
+    monkeypatch.setattr(chunk, "SAVE_STATE_TILES", False)
+    g_cum, A, _, _, _, cache = fq.chunk_gated_delta_rule_fwd(
+        d["q"], d["k"], d["v"], d["g"], d["beta"], None, d["h0"], cu_t, auto_cp=fwd_cp,
+        enable_fwd_cp_cache=True)
+    assert (cache is not None) == fwd_cp  # the batch is split
+    args = (d["q"], d["k"], d["v"], g_cum, d["beta"], A, d["do"], d["dht"], None, d["h0"], cu_t)
+    got = fq.chunk_gated_delta_rule_bwd(*args, auto_cp=bwd_cp, cp_cache=cache)
+    want = fq.chunk_gated_delta_rule_bwd(*args, auto_cp=bwd_cp)
+    for a, b in zip(got, want):  # the D = 64 kernel sums dg, dbeta with shared-memory atomics
+        assert torch.equal(a, b) or (D == 64 and orc.rel_err(a, b) < 1e-5)
+
+
+def test_a_cache_of_another_batch_is_refused(monkeypatch):
+    import flash_qla.ops.gated_delta_rule.chunk as chunk
+    import flashqla_b200 as fq
+
+    monkeypatch.setattr(chunk, "SAVE_STATE_TILES", False)
+
+    def forward(T):
+        x = orc.make_inputs(1, T, 1, 2, 128, 128, seed=2)
+        d = [x[n].bfloat16().to(DEV) for n in ("q", "k", "v")] + [x["g"].to(DEV), x["beta"].to(DEV)]
+        return d, fq.chunk_gated_delta_rule_fwd(*d, enable_fwd_cp_cache=True)
+
+    (q, k, v, _, beta), (g_cum, A, o, _, _, _) = forward(4096)
+    other = forward(2048)[1][5]
+    with pytest.raises(ValueError, match="another batch"):
+        fq.chunk_gated_delta_rule_bwd(q, k, v, g_cum, beta, A, o, cp_cache=other)
