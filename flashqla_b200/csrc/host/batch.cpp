@@ -19,11 +19,16 @@ namespace fqla_host {
 
 namespace {
 
-// Recent entries, least recently used first.  A step of a program uses a handful of batches
-// (micro-batches in flight between their forward and backward); an entry is a few hundred KB at
-// the most.  Shared by all threads; the tables are immutable once built.
-constexpr size_t MAX_ENTRIES = 16;
-std::list<std::shared_ptr<Batch>> entries;
+// Recent entries, least recently used first.  A step of a program uses a handful of packed batches
+// (micro-batches in flight between their forward and backward); an entry keeps the caller's
+// cu_seqlens and a few hundred KB of tables at the most.  Fixed shapes hold nothing of the caller's,
+// and tables (some KB) only where they are split: a program that warms up all the shapes it will
+// capture finds them again.  Shared by all threads; the tables are immutable once built.
+struct Entries {
+  const size_t most;
+  std::list<std::shared_ptr<Batch>> list;
+};
+Entries packed_entries{16, {}}, fixed_entries{1024, {}};
 std::mutex entries_lock;
 
 bool capturing() {
@@ -78,7 +83,12 @@ Tables add_tables(std::vector<int>& out, const std::vector<int64_t>& bounds) {
 }
 
 std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int64_t T, int64_t Hv,
-                             int device) {
+                             int device, bool plan, bool cap) {
+  // reading cu_seqlens and writing tables are host round trips
+  auto needs_round_trip = [&] {
+    if (cap)
+      throw PyError(PyError::Assertion, "index tables of this batch were not built before CUDA graph capture");
+  };
   auto b = std::make_shared<Batch>();
   b->B = B;
   b->T = T;
@@ -89,6 +99,7 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
   Tables raw{};
   const bool packed = cu.has_value();
   if (packed) {
+    needs_round_trip();
     b->cu = *cu;
     b->version = cu->is_inference() ? 0 : cu->_version();
     bounds = read_bounds(*cu);
@@ -103,7 +114,7 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
     for (int64_t i = 0; i <= B; ++i) bounds.push_back(i * T);
   }
   const int n_sm = at::cuda::getDeviceProperties(device)->multiProcessorCount;
-  const auto split = split_sequences(bounds, Hv, n_sm);
+  const auto split = plan ? split_sequences(bounds, Hv, n_sm) : std::nullopt;
   Tables seg{};
   size_t begin = 0, first = 0, last = 0, kf = 0, kb = 0;
   if (split) {
@@ -133,6 +144,7 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
     host.insert(host.end(), keep_b.begin(), keep_b.end());
   }
   if (!host.empty()) {
+    needs_round_trip();
     b->stream = at::cuda::getCurrentCUDAStream(device);
     b->store = at::detail::empty_cuda({(int64_t)host.size()}, at::kInt, c10::Device(c10::kCUDA, device),
                                       std::nullopt);
@@ -166,7 +178,7 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
 }  // namespace
 
 std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B, int64_t T,
-                                 int64_t Hv, int device) {
+                                 int64_t Hv, int device, bool auto_cp) {
   if (cu) {
     if (cu->scalar_type() != at::kInt && cu->scalar_type() != at::kLong)
       throw PyError(PyError::Type, "cu_seqlens must be int32 or int64");
@@ -174,16 +186,16 @@ std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B,
   }
   const uint32_t version = cu && !cu->is_inference() ? cu->_version() : 0;
   const bool cap = capturing();
+  if (!cu && !auto_cp) return build(cu, B, T, Hv, device, false, cap);  // nothing to look up
   std::lock_guard<std::mutex> hold(entries_lock);
-  for (auto it = entries.begin(); it != entries.end(); ++it) {
-    Batch& e = **it;
-    if (e.B != B || e.T != T || e.Hv != Hv || e.device != device) continue;
-    if (cu ? !(e.cu.defined() && e.cu.unsafeGetTensorImpl() == cu->unsafeGetTensorImpl() &&
-               e.version == version)
-           : e.cu.defined())
-      continue;
-    if (cap) e.pinned = true;
+  auto& [most, entries] = cu ? packed_entries : fixed_entries;
+  for (auto it = entries.end(); it != entries.begin();) {  // most recent first
+    Batch& e = **--it;
+    if (e.B != B || e.T != T || e.device != device) continue;
+    if (e.Hv != Hv && auto_cp) continue;  // only the plan depends on the heads
+    if (cu && !(e.cu.unsafeGetTensorImpl() == cu->unsafeGetTensorImpl() && e.version == version)) continue;
     if (e.stream) {
+      if (cap) e.pinned = true;
       // an evicted entry's tables must outlive the kernels of every stream that read them
       const auto current = at::cuda::getCurrentCUDAStream(device);
       if (current != *e.stream)
@@ -192,12 +204,10 @@ std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B,
     entries.splice(entries.end(), entries, it);
     return entries.back();
   }
-  // building a table needs a host round trip
-  if (cap) throw PyError(PyError::Assertion, "index tables of this batch were not built before CUDA graph capture");
-  auto b = build(cu, B, T, Hv, device);
+  auto b = build(cu, B, T, Hv, device, true, cap);
   size_t unpinned = 0;
   for (auto& e : entries) unpinned += !e->pinned;
-  if (unpinned >= MAX_ENTRIES)
+  if (unpinned >= most)
     for (auto it = entries.begin(); it != entries.end(); ++it)
       if (!(*it)->pinned) {
         entries.erase(it);

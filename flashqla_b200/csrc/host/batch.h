@@ -15,7 +15,7 @@ struct Batch {
   uint32_t version = 0;   // its version counter when the tables were read
   int64_t B = 0, T = 0, Hv = 0;
   int device = 0;
-  bool pinned = false;    // looked up during a stream capture: never evicted
+  bool pinned = false;    // its device tables were looked up during a stream capture: never evicted
 
   at::Tensor store;       // all device tables, int32, allocated on `stream`
   std::optional<c10::cuda::CUDAStream> stream;
@@ -31,10 +31,12 @@ struct Batch {
   const int *raw_first = nullptr, *raw_last = nullptr;
 };
 
-// Tables for a batch of `Hv` value heads; one host round trip (reads cu_seqlens, writes the
-// tables) the first time a cu_seqlens tensor (identity and version counter) or a fixed shape is
-// seen, none after that while the entry is kept.
+// Tables for a batch of `Hv` value heads (with auto_cp off its plan is not to be used).  One host round
+// trip (reads cu_seqlens, writes the tables) the first time a cu_seqlens tensor (identity and version
+// counter) or a fixed shape is seen, none after that while the entry is kept.  A fixed shape that is not
+// split, or one without auto_cp, has no tables and needs no round trip: it may be met for the first time
+// during a stream capture, where everything else that is not kept is an error.
 std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B, int64_t T,
-                                 int64_t Hv, int device);
+                                 int64_t Hv, int device, bool auto_cp);
 
 }  // namespace fqla_host

@@ -93,7 +93,7 @@ Call make_call(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, do
   c.D = (int)k.size(3);
   c.Hv = (int)v.size(2);
   c.scale = (float)scale;
-  c.batch = batch_for(cu, c.B, c.T, c.Hv, c.dev.index());
+  c.batch = batch_for(cu, c.B, c.T, c.Hv, c.dev.index(), auto_cp);
   c.split = auto_cp && c.batch->n_seg > 0;
   return c;
 }

@@ -1,0 +1,96 @@
+"""The operator under CUDA graph capture: which shapes may be captured, and that a replay computes what
+the call does."""
+
+import pytest
+import torch
+
+from oracle import gdr_oracle as orc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+HV = 2
+
+
+def _inputs(T, seed=1, cu=None):
+    x = orc.make_inputs(1, T, 1, HV, 128, 128, seed=seed, cu_seqlens=cu)
+    return [x[n].bfloat16().to(DEV) for n in ("q", "k", "v")] + [x["g"].to(DEV), x["beta"].to(DEV)]
+
+
+def _call(args, cu=None, auto_cp=True):
+    import flashqla_b200 as fq
+
+    with torch.no_grad():
+        return fq.chunk_gated_delta_rule(*args, output_final_state=True, cu_seqlens=cu, auto_cp=auto_cp)
+
+
+def _captured(args, **kw):
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = _call(args, **kw)
+    return graph, out
+
+
+def _replay_agrees(args, **kw):
+    graph, out = _captured(args, **kw)
+    for a, b in zip(args, _inputs(args[0].shape[1], seed=2, cu=None)):
+        a.copy_(b)  # other values in the same buffers
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(out, _call(args, **kw)):
+        assert torch.equal(a, b)
+
+
+def test_an_unsplit_fixed_shape_needs_no_call_before_its_capture():
+    _call(_inputs(64))  # loads the kernels
+    _replay_agrees(_inputs(331))
+    _replay_agrees(_inputs(4099), auto_cp=False)
+
+
+def test_every_shape_that_was_warmed_up_can_be_captured():
+    shapes = [1500 + 64 * i for i in range(24)]  # split: they have tables
+    for T in shapes:
+        _call(_inputs(T))
+    _replay_agrees(_inputs(shapes[0]))
+
+
+def test_a_split_or_packed_batch_without_tables_is_refused():
+    _call(_inputs(64))
+    for T, cu in ((5003, None), (200, torch.tensor([0, 77, 200], device=DEV))):
+        args = _inputs(T)
+        with pytest.raises(AssertionError, match="before CUDA graph capture"):
+            _captured(args, cu=cu)
+        torch.cuda.synchronize()
+        _call(args, cu=cu)
+        _captured(args, cu=cu)
+
+
+def test_twenty_packed_batches_in_turn():
+    """More batches than are kept: tables are rebuilt, one kept by a graph stays valid."""
+    args = _inputs(2000)
+    cus = [torch.tensor([0, 50 + i, 1300 + 3 * i, 2000], dtype=torch.int32, device=DEV) for i in range(20)]
+    want = [_call(args, cu=c) for c in cus]
+    graph, out = _captured(args, cu=cus[-1])
+    for _ in range(2):
+        for c, w in zip(cus, want):
+            for a, b in zip(_call(args, cu=c), w):
+                assert torch.equal(a, b)
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(out, want[-1]):
+        assert torch.equal(a, b)
+
+
+def test_one_batch_from_two_streams():
+    args = _inputs(6000)
+    cu = torch.tensor([0, 3000, 6000], dtype=torch.int32, device=DEV)
+    want = _call(args, cu=cu)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    out = []
+    for i in range(6):
+        with torch.cuda.stream(streams[i % 2]):
+            out.append(_call(args, cu=cu))
+    torch.cuda.synchronize()
+    for o in out:
+        for a, b in zip(o, want):
+            assert torch.equal(a, b)
