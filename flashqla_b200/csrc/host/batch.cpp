@@ -83,7 +83,7 @@ Tables add_tables(std::vector<int>& out, const std::vector<int64_t>& bounds) {
 }
 
 std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int64_t T, int64_t Hv,
-                             int device, bool plan, bool cap) {
+                             int device, bool plan, bool cap, const std::vector<int64_t>& read) {
   // reading cu_seqlens and writing tables are host round trips
   auto needs_round_trip = [&] {
     if (cap)
@@ -102,7 +102,8 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
     needs_round_trip();
     b->cu = *cu;
     b->version = cu->is_inference() ? 0 : cu->_version();
-    bounds = read_bounds(*cu);
+    bounds = read.empty() ? read_bounds(*cu) : read;
+    if (cu->is_inference()) b->bounds = bounds;
     b->N = (int64_t)bounds.size() - 1;
     raw = add_tables(host, bounds);
     b->num_chunks = raw.num_chunks;
@@ -186,7 +187,9 @@ std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B,
   }
   const uint32_t version = cu && !cu->is_inference() ? cu->_version() : 0;
   const bool cap = capturing();
-  if (!cu && !auto_cp) return build(cu, B, T, Hv, device, false, cap);  // nothing to look up
+  if (!cu && !auto_cp) return build(cu, B, T, Hv, device, false, cap, {});  // nothing to look up
+  std::vector<int64_t> read;
+  if (cu && cu->is_inference() && !cap) read = read_bounds(*cu);
   std::lock_guard<std::mutex> hold(entries_lock);
   auto& [most, entries] = cu ? packed_entries : fixed_entries;
   for (auto it = entries.end(); it != entries.begin();) {  // most recent first
@@ -194,6 +197,7 @@ std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B,
     if (e.B != B || e.T != T || e.device != device) continue;
     if (e.Hv != Hv && auto_cp) continue;  // only the plan depends on the heads
     if (cu && !(e.cu.unsafeGetTensorImpl() == cu->unsafeGetTensorImpl() && e.version == version)) continue;
+    if (!read.empty() && e.bounds != read) continue;
     if (e.stream) {
       if (cap) e.pinned = true;
       // an evicted entry's tables must outlive the kernels of every stream that read them
@@ -204,7 +208,7 @@ std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B,
     entries.splice(entries.end(), entries, it);
     return entries.back();
   }
-  auto b = build(cu, B, T, Hv, device, true, cap);
+  auto b = build(cu, B, T, Hv, device, true, cap, read);
   size_t unpinned = 0;
   for (auto& e : entries) unpinned += !e->pinned;
   if (unpinned >= most)

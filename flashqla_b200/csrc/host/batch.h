@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <memory>
 #include <optional>
+#include <vector>
 
 namespace fqla_host {
 
@@ -13,6 +14,7 @@ struct Batch {
   // what the entry was made for
   at::Tensor cu;          // the caller's cu_seqlens (undefined: fixed length); kept alive by the entry
   uint32_t version = 0;   // its version counter when the tables were read
+  std::vector<int64_t> bounds;  // its values (inference tensors, which have no version counter)
   int64_t B = 0, T = 0, Hv = 0;
   int device = 0;
   bool pinned = false;    // its device tables were looked up during a stream capture: never evicted
@@ -35,7 +37,9 @@ struct Batch {
 // trip (reads cu_seqlens, writes the tables) the first time a cu_seqlens tensor (identity and version
 // counter) or a fixed shape is seen, none after that while the entry is kept.  A fixed shape that is not
 // split, or one without auto_cp, has no tables and needs no round trip: it may be met for the first time
-// during a stream capture, where everything else that is not kept is an error.
+// during a stream capture, where everything else that is not kept is an error.  A cu_seqlens made in
+// inference mode has no version counter: it is read again at every call, and its tables are rebuilt where
+// it has changed (a capture, which cannot read it, takes the tables of the call before).
 std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B, int64_t T,
                                  int64_t Hv, int device, bool auto_cp);
 
