@@ -48,6 +48,16 @@ std::vector<int64_t> read_bounds(const at::Tensor& cu) {
   return b;
 }
 
+// The kernels' plain loads and stores follow the bounds: what does not lie inside the rows is refused
+// here, where the values are at hand.
+void check_bounds(const std::vector<int64_t>& b, int64_t rows) {
+  bool ok = !b.empty() && b.front() >= 0 && b.back() <= rows;
+  for (size_t i = 1; ok && i < b.size(); ++i) ok = b[i - 1] <= b[i];
+  if (!ok)
+    throw PyError(PyError::Value, "cu_seqlens must hold at least one value, start at 0 or above, not descend, and "
+                                  "end within the " + std::to_string(rows) + " rows of the input");
+}
+
 // cu | chunk offsets | chunk (sequence, chunk in sequence) rows | longest-first order
 struct Tables {
   size_t cu, offsets, indices, order;
@@ -103,6 +113,7 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
     b->cu = *cu;
     b->version = cu->is_inference() ? 0 : cu->_version();
     bounds = read.empty() ? read_bounds(*cu) : read;
+    check_bounds(bounds, T);
     if (cu->is_inference()) b->bounds = bounds;
     b->N = (int64_t)bounds.size() - 1;
     raw = add_tables(host, bounds);

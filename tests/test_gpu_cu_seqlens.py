@@ -1,4 +1,5 @@
-"""``cu_seqlens`` that changes between calls: the index tables follow its values, however it was made."""
+"""``cu_seqlens`` that changes between calls: the index tables follow its values, however it was made;
+and values outside the rows, which are refused before anything is launched."""
 
 import pytest
 import torch
@@ -50,3 +51,23 @@ def test_inference_tensor_under_capture():
         torch.cuda.synchronize()
         for a, b in zip(out, want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("values", [[], [-1, 3000], [0, 3001], [0, 1600, 1500, 3000], [0, 2 ** 33]], ids=str)
+def test_bounds_outside_the_rows_are_refused(values):
+    args = _args()
+    cu = torch.tensor(values, dtype=torch.int64, device=DEV)
+    with pytest.raises(ValueError, match="cu_seqlens"):
+        _call(args, cu)
+
+
+@pytest.mark.parametrize("values", [[0], [0, 0, 2000], [64, 2500]], ids=str)
+def test_bounds_inside_the_rows_are_taken(values):
+    """No sequence, an empty one, rows before the first and behind the last."""
+    args = _args()
+    o, ht = _call(args, torch.tensor(values, dtype=torch.int64, device=DEV))
+    assert ht.shape[0] == len(values) - 1
+    for i, (a, b) in enumerate(zip(values[:-1], values[1:])):
+        if a < b:
+            alone = _call([t[:, a:b].contiguous() for t in args], None)
+            assert orc.rel_err(o[:, a:b], alone[0]) < 5e-3 and orc.rel_err(ht[i], alone[1][0]) < 5e-3
