@@ -90,8 +90,8 @@ __global__ void __launch_bounds__(128) cumsum_kernel(const float* __restrict__ g
 //
 // What bounds it: instruction issue and the latency of one warp's chain.  4 x 8192 tokens, 16 heads
 // (8192 problems): the four-warp form 79 us; this one with scalar fp32, cvt.rna and per-thread
-// copies 58 us (3090 instructions per problem); with packed fp32 pairs, TMA both ways and the
-// rounding add below KKT_NOW
+// copies 58 us (3090 instructions per problem); with packed fp32 pairs, TMA both ways and cvt.rn
+// 46 us.
 // ------------------------------------------------------------------------------------------
 // set to 1 when a block of kkt_solve_kernel abandoned its bounded wait; read through
 // fqla_device_status
@@ -100,12 +100,17 @@ __device__ int g_kkt_status = 0;
 struct Block16 {  // 16 x 16 fp32 fragment
   float c[2][4];
 };
-// the same block as tf32 operand.  Rounding to nearest (ties away) is adding half an ulp of the
-// 10-bit mantissa to the magnitude; the tensor core ignores the 13 bits below.
+// the same block as tf32 operand.  The conversion keeps infinities and NaN; adding half an ulp to the bits,
+// which rounds as well and takes as long, makes -0 of the NaN of arithmetic (0x7fffffff).
+// (cvt.rna, ties away instead of to even: 3 us of 46 more on the 8192 problems below.)
 struct Op16 {
   uint32_t c[2][4];
 };
-__device__ __forceinline__ uint32_t to_tf32(float x) { return __float_as_uint(x) + 0x1000u; }
+__device__ __forceinline__ uint32_t to_tf32(float x) {
+  uint32_t r;
+  asm("cvt.rn.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return r;
+}
 __device__ __forceinline__ Op16 to_op(const Block16& b) {
   Op16 o;
 #pragma unroll
