@@ -20,10 +20,11 @@
 // one are dead (k has two buffers).
 #include <cuda.h>
 
-#include "common.cuh"
-#include "fqla_internal.h"
+#include <climits>
 #include <mutex>
 
+#include "common.cuh"
+#include "fqla_internal.h"
 #include "tc05.cuh"
 
 namespace fqla {
@@ -44,7 +45,7 @@ struct BwdMainTcParams {
   void* db;                // fp32 or (db_bf16) bf16
   float* dg;
   int dg_cumsum, db_bf16;  // see fqla_bwd_main_args
-  int* next_item;          // zero at launch, or null: see the walk of the items below
+  int* next_item;          // !CLC: zero at launch; see the walk of the items below
   int Hq, Hv;
   float scale;
   SeqLayout lay;
@@ -72,10 +73,11 @@ constexpr int OFF_DW = OFF_DA + 8192;       // -du h^T
 // chunk total (16)
 constexpr int OFF_VEC = OFF_DW + ROW_TILE;
 constexpr int OFF_BAR = OFF_VEC + (4 * 64 + 5 * 256 + 512 + 18) * 4;
-constexpr int N_BARS = 22;
+constexpr int N_BARS = 23;
 constexpr int OFF_MISC = OFF_BAR + N_BARS * 8;
 constexpr int OFF_ITEM = OFF_MISC + 32;  // ring of four items, published by the issue warp
-constexpr int SMEM_BYTES = OFF_ITEM + 4 * 32 + 1024;
+constexpr int OFF_CLAIM = (OFF_ITEM + 4 * 32 + 15) / 16 * 16;  // CLC: two answers of 16 bytes
+constexpr int SMEM_BYTES = OFF_CLAIM + 2 * 16 + 1024;
 static_assert(SMEM_BYTES <= 232448, "one CTA's shared memory");
 // the operand tiles of one item arrive in three groups, in the order their buffers become free
 constexpr uint32_t TX_A = 2 * SQ_TILE + 3 * ROW_TILE;  // h, dh, dO, v_new, k (other buffer)
@@ -96,7 +98,8 @@ enum {
   R_DW, R_DS, R_DA, R_T, R_D3,       // the 8 warps of the chain group -> issue warp
   R_HD, R_E4,                        // the 8 warps of the bulk group -> issue warp
   R_CH,                              // the 8 warps of the chain group -> bulk group: item finished
-  I_NEXT                             // issue warp -> read-out warps: the next item is in the ring
+  I_NEXT,                            // issue warp -> read-out warps: the next item is in the ring
+  I_CLAIM                            // CLC: the answer with the next item has arrived
 };
 }  // namespace bmtc
 
@@ -132,15 +135,17 @@ __device__ __forceinline__ void bulk_barrier() {  // warps 8-15
   asm volatile("bar.sync 5, 256;" ::: "memory");
 }
 
-// Persistent: CTA b starts with work item b and takes the next one that nobody has (next_item counts
-// them out; without it b + gridDim.x, ...); item w = (chunk w / Hv, head w % Hv), so neighbouring CTAs
-// share q and k of a grouped-value-attention group through L2.  SMs differ in speed by a fifth
-// (instruction fetch), and with a fixed share each the fast ones run away: a tail, and CTAs working
-// far apart in memory.  262144 tokens x 8 heads, 7.1 GB: 1479 us (4.8 TB/s) counted out, 1970-2090 us
-// with a fixed share, 1650 us with a fixed share and the 16 warps in step (see the end of an item).
+// Persistent: CTA b starts with work item b and takes the next one that nobody has; item w = (chunk
+// w / Hv, head w % Hv), so neighbouring CTAs share q and k of a grouped-value-attention group through
+// L2.  SMs differ in speed by a fifth (instruction fetch), and with a fixed share each the fast ones run
+// away: a tail, and CTAs working far apart in memory.  262144 tokens x 8 heads, 7.1 GB: 1472 us (4.8 TB/s)
+// counted out by next_item; 1492 us where the caller brings no counter and the grid has a block for every
+// item, those that run taking the items of those that have not started (CLC, cluster launch control: the
+// answer takes longer than that of an atomic); 1970-2090 us with a fixed share, 1650 us with a fixed share
+// and the 16 warps in step (see the end of an item).
 // TILED: h, dh, vnew and du arrive in the operand layouts written by the sequential kernels
 // (h^T, dh^T as [V][K] per chunk; vnew^T, du^T as [V][64] per chunk) instead of row-major.
-template <bool TILED>
+template <bool TILED, bool CLC>
 __global__ void __launch_bounds__(bmtc::NT, 1)
 bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap map_q,
                    const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -219,6 +224,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
     mbar_init(&bars[R_END], N_EPI / 32);
     for (int i = R_DW; i <= R_CH; ++i) mbar_init(&bars[i], N_EPI / 64);
     mbar_init(&bars[I_NEXT], 1);
+    if (CLC) mbar_init(&bars[I_CLAIM], 1);
     *abort_flag = 0;
     for (int i = 0; i < 4; ++i) stop_flag[i] = 0;
     fence_mbar_init();
@@ -300,9 +306,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 
       Raw raw = {};
       int claimed = (int)blockIdx.x;  // in lane 0
-      auto claim = [&] {
-        if (lane == 0) claimed = p.next_item ? (int)gridDim.x + atomicAdd(p.next_item, 1) : claimed + (int)gridDim.x;
-      };
+      unsigned char* answers = smem + OFF_CLAIM;  // two slots, by item parity
       load_index((int)blockIdx.x / p.Hv, raw);
       load_span(raw);
       Item cur = finish(raw, (int)blockIdx.x % p.Hv);
@@ -314,7 +318,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 #pragma unroll 1
       for (bool has_next = true; has_next && ok; ++it) {
         const uint32_t ph = it & 1;
-        claim();
+        if (!CLC && lane == 0) claimed = (int)gridDim.x + atomicAdd(p.next_item, 1);
         const uint32_t k_lo = k_lo0 + (ph ? KBUF_LO : 0u), kmn_lo = kmn_lo0 + (ph ? KBUF_LO : 0u);
         // the read-out warps have finished the previous item (accumulators free) and have zeroed
         // the rows past the sequence end in this item's tiles (which also means: tiles landed)
@@ -341,6 +345,10 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           }
           umma_group<8, 2, 512, 2, 512, false>(tmem + T_QK, q_lo, k_lo, ID_KK_64);
           umma_commit(&bars[C_DSQK]);
+          if constexpr (CLC) {
+            mbar_arrive_expect_tx(&bars[I_CLAIM], 16);
+            clc_try_cancel(answers + 16 * ph, &bars[I_CLAIM]);
+          }
         }
         // ---- dw is an operand now: the pieces of dA, and A^T dw, A^T du ----
         ok = WAIT(R_DW, ph);
@@ -368,8 +376,17 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           }
           umma_commit(&bars[C_1B]);
         }
-        const int w_next = __shfl_sync(0xffffffffu, claimed, 0);
-        has_next = w_next < (int)total;
+        int w_next;
+        if constexpr (CLC) {
+          ok = WAIT(I_CLAIM, ph);
+          if (!ok) break;
+          w_next = clc_block(answers + 16 * ph);
+          fence_proxy_async();  // read before the request after the next one writes the slot
+          has_next = w_next >= 0;
+        } else {
+          w_next = __shfl_sync(0xffffffffu, claimed, 0);
+          has_next = w_next < (int)total;
+        }
         const int h_next = has_next ? w_next % p.Hv : 0;
         if (has_next) load_index(w_next / p.Hv, raw);
         // ---- ds is an operand now ----
@@ -1012,33 +1029,21 @@ int launch_bwd_main_tc(const fqla_bwd_main_args& a, long long n_chunks, SeqLayou
   p.Hq = Hq; p.Hv = Hv; p.scale = a.scale; p.lay = lay; p.chunk_indices = chunk_indices;
   p.n_chunks = n_chunks;
   p.next_item = a.next_item;
-  static std::atomic<unsigned long long> done[2];
-  rc = configure_smem(a.operand_tiles ? (const void*)bwd_main_tc_kernel<true> : (const void*)bwd_main_tc_kernel<false>,
-                      SMEM_BYTES, done[a.operand_tiles ? 1 : 0]);
-  if (rc != 0) return rc;
-  int dev = 0, n_sm = 0;  // per launch: the current device may differ from call to call
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-  if (n_sm <= 0) n_sm = 148;
   const long long total = n_chunks * Hv;
-  const unsigned grid = (unsigned)(total < n_sm ? total : n_sm);
-  // A caller without a counter gets one for this launch, in stream order (also under capture); where
-  // that cannot be had, or with a handful of items per CTA, each CTA takes its fixed share.
-  void* own = nullptr;
-  if (!p.next_item && total > 4ll * n_sm) {
-    if (cudaMallocAsync(&own, sizeof(int), st) == cudaSuccess &&
-        cudaMemsetAsync(own, 0, sizeof(int), st) == cudaSuccess)
-      p.next_item = (int*)own;
-    else
-      cudaGetLastError();
-  }
-  rc = launch_pdl(a.operand_tiles ? bwd_main_tc_kernel<true> : bwd_main_tc_kernel<false>, dim3(grid), dim3(NT),
-                  (size_t)SMEM_BYTES, st, p, mq, mk, mv, mvn, mdo, mdu, mh, mdh, ma);
-  if (own) {
-    const int freed = (int)cudaFreeAsync(own, st);
-    if (rc == 0) rc = freed;
-  }
-  return rc;
+  if (total > INT_MAX) return FQLA_ERR_TOO_LARGE;
+  auto launch = [&](auto kernel, std::atomic<unsigned long long>& done, long long blocks) {
+    int err = configure_smem((const void*)kernel, SMEM_BYTES, done);
+    if (err != 0) return err;
+    return launch_pdl(kernel, dim3((unsigned)blocks), dim3(NT), (size_t)SMEM_BYTES, st, p, mq, mk, mv, mvn, mdo,
+                      mdu, mh, mdh, ma);
+  };
+  static std::atomic<unsigned long long> done[4];
+  if (!p.next_item)
+    return a.operand_tiles ? launch(bwd_main_tc_kernel<true, true>, done[0], total)
+                           : launch(bwd_main_tc_kernel<false, true>, done[1], total);
+  const long long n_sm = sm_count(), blocks = total < n_sm ? total : n_sm;
+  return a.operand_tiles ? launch(bwd_main_tc_kernel<true, false>, done[2], blocks)
+                         : launch(bwd_main_tc_kernel<false, false>, done[3], blocks);
 }
 
 }  // namespace fqla

@@ -131,6 +131,33 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   return false;
 }
 
+// ---- cluster launch control ----------------------------------------------------------------------
+// Asks for a block of this grid that has not started yet.  It then never starts, and the block that asked
+// does its work: dynamic hand-out of a grid without a counter in memory.  The answer (16 bytes, written
+// by the async proxy) lands in `slot` and counts on `bar`, which expects 16 bytes.  After an answer
+// without a block a CTA must not ask again.
+__device__ __forceinline__ void clc_try_cancel(void* slot, uint64_t* bar) {
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+          s32(slot)),
+      "r"(s32(bar))
+      : "memory");
+}
+// The answer: the block's index in a one-dimensional grid, or -1.
+__device__ __forceinline__ int clc_block(const void* slot) {
+  uint32_t found, x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 answer;\n\t"
+      "ld.shared.b128 answer, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, answer;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, answer;\n\t}"
+      : "=r"(found), "=r"(x)
+      : "r"(s32(slot))
+      : "memory");
+  return found ? (int)x : -1;
+}
+
 // ---- proxy / tcgen05 fences ------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

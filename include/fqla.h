@@ -146,7 +146,8 @@ int fqla_bwd_dh(const void* q, const void* k, const void* A, const float* g_cum,
  * sequence n starts from dht[dht_row[n]] where that is >= 0, else from seg_dht[n] (zero without
  * seg_dht); dh0_row [N]: dh0 of sequence n goes to dh0[dh0_row[n]] where that is >= 0;
  * state_v_first: dht and dh0 are [value dim][key dim].  As in fqla_fwd_args.  zero_word (optional, K =
- * V = 128, tcgen05 kernel only): one int that is set to zero (next_item of fqla_bwd_main_args). */
+ * V = 128, tcgen05 kernel only, no run_mask, no warm_chunks): one int that is set to zero (next_item of
+ * fqla_bwd_main_args). */
 typedef struct fqla_bwd_dh_args {
   const void *q, *k, *A;
   const float* g_cum;
@@ -182,7 +183,8 @@ int fqla_bwd_main(const void* q, const void* k, const void* v, const void* vnew,
  * comes out after its reverse chunk-local cumulative sum (what fqla_chunk_local_cumsum, reverse,
  * would make of it); db_is_bf16: db is bf16 instead of fp32; next_item (optional, D = 128): one int,
  * zero when the kernel starts, of which the launch is the only user: its CTAs take the
- * (chunk, head) items as they go.  Without it a large launch allocates one in stream order. */
+ * (chunk, head) items as they go.  Without it they take them by cluster launch control, 1 to 2 %
+ * slower. */
 typedef struct fqla_bwd_main_args {
   const void *q, *k, *v, *vnew, *A;
   const float* g_cum;
