@@ -176,17 +176,18 @@ class ChunkGatedDeltaRuleFunction(torch.autograd.Function):
         g_cum, A, o, _, final_state, cp_cache, *norm = _lib.host().forward(
             q, k, v, g, beta, scale, initial_state, cu_seqlens, flags)
         q_used, k_used = norm[:2] if norm else (q, k)
-        ctx.save_for_backward(q_used, k_used, v, g_cum, beta, A, initial_state, cu_seqlens, q, k,
+        ctx.save_for_backward(q_used, k_used, v, g_cum, beta, A, initial_state, cu_seqlens,
                               *norm[2:], *(cp_cache or ()))
         ctx.has_norm, ctx.has_cache = bool(norm), cp_cache is not None
+        ctx.f16 = q.dtype == torch.float16
         ctx.g_dtype = g.dtype
         ctx.scale = scale
         return o, final_state
 
     @staticmethod
     def backward(ctx, do: torch.Tensor, dht: torch.Tensor):
-        q_used, k_used, v, g_cum, beta, A, initial_state, cu_seqlens, q, k, *rest = ctx.saved_tensors
-        norm = (q, k, rest.pop(0), rest.pop(0)) if ctx.has_norm else None
+        q_used, k_used, v, g_cum, beta, A, initial_state, cu_seqlens, *rest = ctx.saved_tensors
+        norm = (rest.pop(0), rest.pop(0), ctx.f16) if ctx.has_norm else None
         dq, dk, dv, db, dg, dh0 = _lib.host().backward(
             q_used, k_used, v, g_cum, beta, A, do, dht, ctx.scale, initial_state, cu_seqlens,
             ctx.flags, tuple(rest) if ctx.has_cache else None, norm)

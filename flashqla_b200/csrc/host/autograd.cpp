@@ -13,8 +13,7 @@ namespace {
 struct GatedDeltaRuleBackward : public ag::Node {
   // inputs as the kernels read them, the forward's results, what the forward kept
   ag::SavedVariable q, k, v, g_cum, beta, A, initial_state, cu, seg_h0, h, vnew, lead;
-  // q, k before the normalisation, reciprocal norms (with l2norm)
-  ag::SavedVariable q_in, k_in, q_rstd, k_rstd;
+  ag::SavedVariable q_rstd, k_rstd;  // with l2norm; q, k above are then normalised
   double scale = 1.0;
   Options opt;
   at::ScalarType dtype = at::kBFloat16, beta_dtype = at::kFloat, g_dtype = at::kFloat,
@@ -27,7 +26,7 @@ struct GatedDeltaRuleBackward : public ag::Node {
 
   void release_variables() override {
     for (ag::SavedVariable* s : {&q, &k, &v, &g_cum, &beta, &A, &initial_state, &cu, &seg_h0, &h,
-                                 &vnew, &lead, &q_in, &k_in, &q_rstd, &k_rstd})
+                                 &vnew, &lead, &q_rstd, &k_rstd})
       s->reset_data();
   }
 
@@ -43,7 +42,7 @@ struct GatedDeltaRuleBackward : public ag::Node {
     const at::Tensor dO = grads[0].defined() ? grads[0] : at::zeros(o_sizes, o_options);
     const Cache cache{opt_get(seg_h0), opt_get(h), opt_get(vnew), opt_get(lead)};
     Norm norm;
-    if (opt.l2norm) norm = Norm{get(q_in), get(k_in), get(q_rstd), get(k_rstd)};
+    if (opt.l2norm) norm = Norm{get(q_rstd), get(k_rstd)};
     const Backward r = backward(get(q), get(k), get(v), get(g_cum), get(beta), get(A), dO, dht, scale,
                                 opt_get(initial_state), opt_get(cu), opt, cache,
                                 opt.l2norm ? &norm : nullptr, dtype);
@@ -104,8 +103,6 @@ std::pair<at::Tensor, OptTensor> apply(const at::Tensor& q, const at::Tensor& k,
   save_opt(node->vnew, r.cache.vnew);
   save_opt(node->lead, r.cache.lead);
   if (opt.l2norm) {
-    save(node->q_in, q);
-    save(node->k_in, k);
     save(node->q_rstd, r.q_rstd);
     save(node->k_rstd, r.k_rstd);
   }

@@ -457,18 +457,12 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
     const auto t = f16 ? at::kHalf : at::kBFloat16;
     at::Tensor dq = empty({c.B, c.T, c.Hq, c.D}, t, c.dev), dk = empty({c.B, c.T, c.Hq, c.D}, t, c.dev);
     at::Tensor dv = f16 ? empty(v.sizes(), t, c.dev) : r.dv;
-    // the gradient of the normalisation reads its inputs in the type of its outputs
-    at::Tensor nq, nk;
-    if (norm) {
-      nq = aligned(norm->q.scalar_type() == t ? norm->q : norm->q.to(t));
-      nk = aligned(norm->k.scalar_type() == t ? norm->k : norm->k.to(t));
-    }
     check(fqla_finish_grads(r.dq.data_ptr(), r.dk.data_ptr(), f16 ? r.dv.data_ptr() : nullptr,
-                            norm ? nq.data_ptr() : nullptr, norm ? nk.data_ptr() : nullptr,
+                            norm ? q.data_ptr() : nullptr, norm ? k.data_ptr() : nullptr,
                             norm ? (const float*)norm->q_rstd.data_ptr() : nullptr,
                             norm ? (const float*)norm->k_rstd.data_ptr() : nullptr, dq.data_ptr(),
                             dk.data_ptr(), f16 ? dv.data_ptr() : nullptr, rows * c.Hq, c.Hv / c.Hq,
-                            c.D, f16, c.stream),
+                            c.D, (f16 ? FQLA_GRADS_F16 : 0) | FQLA_ROWS_NORMALISED, c.stream),
           "finish_grads");
     r.dq = dq;
     r.dk = dk;

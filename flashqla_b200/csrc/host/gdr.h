@@ -27,9 +27,9 @@ struct Cache {
   OptTensor seg_h0, h, vnew, lead;
 };
 
-// The L2 normalisation of q and k: the rows before it and their reciprocal norms.
+// Reciprocal norms of the rows of q and k before their L2 normalisation.
 struct Norm {
-  at::Tensor q, k, q_rstd, k_rstd;
+  at::Tensor q_rstd, k_rstd;
 };
 
 struct Forward {
@@ -50,8 +50,9 @@ Forward forward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, c
                 const at::Tensor& beta, double scale, const OptTensor& initial_state,
                 const OptTensor& cu, const Options& opt);
 
-// `g_cum` and `A` are the forward's; q, k the ones its kernels read.  With `norm` the gradients of q,
-// k are mapped back through the normalisation.  dq, dk, dv come in `dtype`, db
+// `g_cum` and `A` are the forward's; q, k the ones its kernels read.  With `norm` (those are
+// normalised) the gradients of q, k are mapped back through the normalisation, which needs nothing of
+// the tensors before it: they may be freed or changed.  dq, dk, dv come in `dtype`, db
 // in bfloat16 or float32 (beta's type where it is one of them), dg in float32.
 Backward backward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
                   const at::Tensor& g_cum, const at::Tensor& beta, const at::Tensor& A,

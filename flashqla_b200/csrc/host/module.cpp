@@ -184,7 +184,8 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // backward(q, k, v, g_cum, beta, A, do, dht, scale, initial_state, cu_seqlens, flags, cp_cache, norm)
-//   -> (dq, dk, dv, db, dg, dh0);  norm: None or (q, k before the normalisation, q_rstd, k_rstd)
+//   -> (dq, dk, dv, db, dg, dh0);  norm: None, or where q, k are normalised (q_rstd, k_rstd, whether the
+//   operator's q, k, v were float16): dq, dk belong to the rows before the normalisation
 PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
     if (n != 14) throw PyError(PyError::Type, "backward takes 14 arguments");
@@ -196,11 +197,13 @@ PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         *slots[i] = opt_tensor(PyTuple_GET_ITEM(a[12], i), "cp_cache entry");
     }
     Norm norm;
+    bool norm_f16 = false;
     if (a[13] != Py_None) {
-      if (!PyTuple_Check(a[13]) || PyTuple_GET_SIZE(a[13]) != 4)
-        throw PyError(PyError::Type, "norm must be a tuple of four tensors or None");
-      at::Tensor* parts[4] = {&norm.q, &norm.k, &norm.q_rstd, &norm.k_rstd};
-      for (int i = 0; i < 4; ++i) *parts[i] = tensor(PyTuple_GET_ITEM(a[13], i), "norm entry");
+      if (!PyTuple_Check(a[13]) || PyTuple_GET_SIZE(a[13]) != 3)
+        throw PyError(PyError::Type, "norm must be (q_rstd, k_rstd, float16) or None");
+      norm.q_rstd = tensor(PyTuple_GET_ITEM(a[13], 0), "q_rstd");
+      norm.k_rstd = tensor(PyTuple_GET_ITEM(a[13], 1), "k_rstd");
+      norm_f16 = PyTuple_GET_ITEM(a[13], 2) == Py_True;
     }
     const at::Tensor q = tensor(a[0], "q"), k = tensor(a[1], "k"), v = tensor(a[2], "v"),
                      g = tensor(a[3], "g"), beta = tensor(a[4], "beta"), A = tensor(a[5], "A"),
@@ -212,7 +215,7 @@ PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool normed = a[13] != Py_None;
     Backward r = without_gil([&] {
       return backward(q, k, v, g, beta, A, dO, dht, scale, h0, cu, opt, cache, normed ? &norm : nullptr,
-                      (normed ? norm.q : q).scalar_type());
+                      !normed ? q.scalar_type() : norm_f16 ? at::kHalf : at::kBFloat16);
     });
     if (r.db.scalar_type() != beta.scalar_type()) r.db = r.db.to(beta.scalar_type());
     return tuple_of(r.dq, r.dk, r.dv, r.db, r.dg, r.dh0);

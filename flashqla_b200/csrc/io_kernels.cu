@@ -102,8 +102,9 @@ __global__ void __launch_bounds__(256) prepare_inputs_kernel(const PrepareParams
 
 struct FinishParams {
   const void *dq_v, *dk_v, *dv_in;  // bf16, per value head; dv_in null: dv is not converted
-  const void *q, *k;                // the operator's inputs (type of the outputs), for the normalisation
+  const void *q, *k;                // rows of the normalisation: its outputs (bf16) or inputs (type of dq)
   const float *q_rstd, *k_rstd;     // null: no normalisation
+  int normalised;                   // q, k are outputs
   void *dq, *dk, *dv;
   long long rows_qk, rows_v;
   int G;                            // value heads per q/k head
@@ -136,13 +137,17 @@ __global__ void __launch_bounds__(256) finish_grads_kernel(const FinishParams p)
     // y = x_in * rstd;  d x_in = (dy - <dy, y> y) * rstd
     const bool qk = in && (is_q || is_k);
     float y[8], dot = 0.f;
-    OUT::unpack(qk ? reinterpret_cast<const uint4*>(is_q ? p.q : p.k)[j] : make_uint4(0, 0, 0, 0), y);
+    const uint4 raw = qk ? reinterpret_cast<const uint4*>(is_q ? p.q : p.k)[j] : make_uint4(0, 0, 0, 0);
     const float r = qk ? (is_q ? p.q_rstd : p.k_rstd)[row] : 1.f;
+    if (p.normalised) {
+      Bf16x8::unpack(raw, y);
+    } else {
+      OUT::unpack(raw, y);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      y[e] *= r;
-      dot += x[e] * y[e];
+      for (int e = 0; e < 8; ++e) y[e] *= r;
     }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) dot += x[e] * y[e];
     dot = row_sum<LANES>(dot);
     if (qk) {
 #pragma unroll
@@ -180,14 +185,16 @@ extern "C" int fqla_prepare_inputs(const void* q, const void* k, const void* v, 
 extern "C" int fqla_finish_grads(const void* dq_v, const void* dk_v, const void* dv_in,
                                  const void* q, const void* k, const float* q_rstd,
                                  const float* k_rstd, void* dq, void* dk, void* dv,
-                                 long long rows_qk, int G, int D, int is_f16, void* stream) {
+                                 long long rows_qk, int G, int D, int types, void* stream) {
+  const int is_f16 = types & FQLA_GRADS_F16;
   if (!dq_v || !dk_v || !dq || !dk || (dv_in && !dv) || G <= 0 || rows_qk < 0)
     return FQLA_ERR_INVALID_ARG;
   if (q_rstd && (!k_rstd || !q || !k)) return FQLA_ERR_INVALID_ARG;
   if (D != 64 && D != 128) return FQLA_ERR_UNSUPPORTED_DIM;
   const long long rows_v = rows_qk * G, n = (2 * rows_qk + (dv_in ? rows_v : 0)) * (D / 8);
   if (n == 0) return FQLA_OK;
-  const FinishParams p{dq_v, dk_v, dv_in, q, k, q_rstd, k_rstd, dq, dk, dv, rows_qk, rows_v, G};
+  const FinishParams p{dq_v, dk_v, dv_in, q, k, q_rstd, k_rstd, types & FQLA_ROWS_NORMALISED, dq, dk, dv,
+                       rows_qk, rows_v, G};
   const unsigned grid = (unsigned)((n + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
   if (D == 128) {

@@ -266,14 +266,17 @@ int fqla_prepare_inputs(const void* q, const void* k, const void* v, void* q_out
                         long long rows_v, int D, int is_f16, int normalise, float eps,
                         void* stream);
 /* One pass over the gradients of fqla_bwd_main: dq, dk = sum over the G value heads of a group of
- * dq_v, dk_v (bf16), mapped back through the L2 normalisation when q_rstd, k_rstd are given (q, k:
- * the operator's own inputs, before normalisation), written as bf16 or (is_f16) fp16; with dv_in,
- * dv is converted too.  rows_qk rows of D per q/k head row.
+ * dq_v, dk_v (bf16), mapped back through the L2 normalisation when q_rstd, k_rstd are given, written
+ * as bf16 or (FQLA_GRADS_F16 in `types`) fp16; with dv_in, dv is converted too.  q, k: the rows before
+ * the normalisation, in the type of dq, or (FQLA_ROWS_NORMALISED in `types`) after it, bf16.  rows_qk
+ * rows of D per q/k head row.
  * Replaces group_reduce_vector (ops/utils/group_reduce.py:60-79) and l2norm_bwd
  * (utils/math.py:38-51) as the backward calls them. */
 int fqla_finish_grads(const void* dq_v, const void* dk_v, const void* dv_in, const void* q,
                       const void* k, const float* q_rstd, const float* k_rstd, void* dq, void* dk,
-                      void* dv, long long rows_qk, int G, int D, int is_f16, void* stream);
+                      void* dv, long long rows_qk, int G, int D, int types, void* stream);
+#define FQLA_GRADS_F16 1
+#define FQLA_ROWS_NORMALISED 2
 
 /* The scan of fqla_warmup_scan for a whole split plan in one launch, plus the decision how each
  * segment gets its start state.  seg_begin [n_raw+1] (int32): first segment of every raw

@@ -1,0 +1,55 @@
+"""What the operator keeps for its backward: with the normalisation in the operator, q and k after it and
+their reciprocal norms, nothing of the tensors before it."""
+
+import pytest
+import torch
+
+from oracle import gdr_oracle as orc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _inputs(T, dtype, seed=6):
+    x = orc.make_inputs(1, T, 2, 4, 128, 128, seed=seed)
+    d = [3.0 * x["q"], 0.5 * x["k"], x["v"]]
+    return [t.to(DEV, dtype).requires_grad_() for t in d] + [x["g"].to(DEV), x["beta"].to(DEV)]
+
+
+@pytest.mark.parametrize("apply_class", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_q_and_k_may_change_and_go_between_the_passes(dtype, apply_class):
+    from flash_qla.ops.gated_delta_rule.chunk import ChunkGatedDeltaRuleFunction, chunk_gated_delta_rule
+
+    def call(q, k, v, g, beta):
+        if apply_class:
+            return ChunkGatedDeltaRuleFunction.apply(q, k, v, g, beta, None, None, False, None, True)[0]
+        return chunk_gated_delta_rule(q, k, v, g, beta, use_qk_l2norm_in_kernel=True)[0]
+
+    leaves = _inputs(200, dtype)
+    want = torch.autograd.grad(call(*leaves).float().square().sum(), leaves[:3])
+    q, k = leaves[0] * 1, leaves[1] * 1  # not leaves: may be changed in place
+    o = call(q, k, *leaves[2:])
+    with torch.no_grad():
+        q.zero_()
+        k.fill_(float("nan"))
+    for a, b in zip(torch.autograd.grad(o.float().square().sum(), leaves[:3]), want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_bytes_kept(dtype):
+    from flash_qla import chunk_gated_delta_rule
+
+    T = 4096
+    leaves = _inputs(T, dtype)
+    held = {}
+
+    def pack(t):
+        held[t.data_ptr()] = t.numel() * t.element_size()
+        return t
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+        chunk_gated_delta_rule(*leaves, use_qk_l2norm_in_kernel=True, auto_cp=False, enable_fwd_cp_cache=False)
+    rows = 2 * T * 2  # of q and of k
+    assert sum(held.values()) <= rows * (128 * 2 + 4) + 4 * T * (128 * 2 + 64 * 2 + 4 + 4)  # q k rstd; v A g beta
