@@ -23,6 +23,7 @@ import torch
 
 from flashqla_b200 import _lib, cp, ops
 from flashqla_b200.ops import CHUNK_SIZE
+from flashqla_b200.utils import l2norm_bwd, l2norm_fwd
 
 
 # bits of the native entry points' `flags` argument (csrc/host/module.cpp)
@@ -170,6 +171,13 @@ class ChunkGatedDeltaRuleFunction(torch.autograd.Function):
     ):
         if scale is None:
             scale = k.shape[-1] ** -0.5
+        # the one-pass kernels take bfloat16 and float16; other types are normalised as they are, ahead
+        native = q.dtype == k.dtype == v.dtype and q.dtype in (torch.bfloat16, torch.float16)
+        ahead = ()
+        if use_qk_l2norm_in_kernel and not native:
+            q, q_rstd = l2norm_fwd(q)
+            k, k_rstd = l2norm_fwd(k)
+            ahead, use_qk_l2norm_in_kernel = (q_rstd, k_rstd), False
         ctx.flags = _switches(auto_cp, state_v_first)
         flags = (ctx.flags | FINAL_STATE * bool(output_final_state)
                  | CACHE * bool(enable_fwd_cp_cache) | L2NORM * bool(use_qk_l2norm_in_kernel))
@@ -177,8 +185,8 @@ class ChunkGatedDeltaRuleFunction(torch.autograd.Function):
             q, k, v, g, beta, scale, initial_state, cu_seqlens, flags)
         q_used, k_used = norm[:2] if norm else (q, k)
         ctx.save_for_backward(q_used, k_used, v, g_cum, beta, A, initial_state, cu_seqlens,
-                              *norm[2:], *(cp_cache or ()))
-        ctx.has_norm, ctx.has_cache = bool(norm), cp_cache is not None
+                              *ahead, *norm[2:], *(cp_cache or ()))
+        ctx.has_norm, ctx.has_cache, ctx.norm_ahead = bool(norm), cp_cache is not None, bool(ahead)
         ctx.f16 = q.dtype == torch.float16
         ctx.g_dtype = g.dtype
         ctx.scale = scale
@@ -187,10 +195,14 @@ class ChunkGatedDeltaRuleFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do: torch.Tensor, dht: torch.Tensor):
         q_used, k_used, v, g_cum, beta, A, initial_state, cu_seqlens, *rest = ctx.saved_tensors
+        q_rstd, k_rstd = (rest.pop(0), rest.pop(0)) if ctx.norm_ahead else (None, None)
         norm = (rest.pop(0), rest.pop(0), ctx.f16) if ctx.has_norm else None
         dq, dk, dv, db, dg, dh0 = _lib.host().backward(
             q_used, k_used, v, g_cum, beta, A, do, dht, ctx.scale, initial_state, cu_seqlens,
             ctx.flags, tuple(rest) if ctx.has_cache else None, norm)
+        if ctx.norm_ahead:
+            dq = l2norm_bwd(q_used, q_rstd, dq).to(q_used)
+            dk = l2norm_bwd(k_used, k_rstd, dk).to(k_used)
         return (
             dq,
             dk,

@@ -254,28 +254,27 @@ void prepare(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor& v
   const auto dt = q_in.scalar_type();
   const bool f16 = dt == at::kHalf;
   const bool one = k_in.scalar_type() == dt && v_in.scalar_type() == dt && (f16 || dt == at::kBFloat16);
+  if (opt.l2norm && !one) throw PyError(PyError::Type, "q, k, v must be bfloat16 or float16 to be normalised here");
   if (!(one && (opt.l2norm || f16))) {
     r.q = as_bf16(q_in);
     r.k = as_bf16(k_in);
     r.v = as_bf16(v_in);
-    if (!opt.l2norm) return;
+    return;
   }
-  const at::Tensor q = one ? aligned(q_in) : r.q, k = one ? aligned(k_in) : r.k;
-  const at::Tensor v = f16 && one ? aligned(v_in) : as_bf16(v_in);
+  const at::Tensor q = aligned(q_in), k = aligned(k_in), v = aligned(v_in);
   const int64_t D = q.size(-1), rows = D ? q.numel() / D : 0;
   r.q = empty(q.sizes(), at::kBFloat16, q.device());
   r.k = empty(k.sizes(), at::kBFloat16, q.device());
-  r.v = f16 && one ? empty(v.sizes(), at::kBFloat16, q.device()) : v;
+  r.v = f16 ? empty(v.sizes(), at::kBFloat16, q.device()) : v;
   if (opt.norm_grad) {
     r.q_rstd = empty({rows}, at::kFloat, q.device());
     r.k_rstd = empty({rows}, at::kFloat, q.device());
   }
-  check(fqla_prepare_inputs(q.data_ptr(), k.data_ptr(), v.data_ptr(), r.q.data_ptr(),
-                            r.k.data_ptr(), f16 && one ? r.v.data_ptr() : nullptr,
+  check(fqla_prepare_inputs(q.data_ptr(), k.data_ptr(), v.data_ptr(), r.q.data_ptr(), r.k.data_ptr(),
+                            f16 ? r.v.data_ptr() : nullptr,
                             opt.norm_grad ? (float*)r.q_rstd.data_ptr() : nullptr,
                             opt.norm_grad ? (float*)r.k_rstd.data_ptr() : nullptr, rows,
-                            D ? v.numel() / D : 0, (int)D, f16 && one, opt.l2norm,
-                            (float)L2NORM_EPS,
+                            D ? v.numel() / D : 0, (int)D, f16, opt.l2norm, (float)L2NORM_EPS,
                             (void*)at::cuda::getCurrentCUDAStream(q.device().index()).stream()),
         "prepare_inputs");
 }

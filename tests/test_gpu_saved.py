@@ -53,3 +53,21 @@ def test_bytes_kept(dtype):
         chunk_gated_delta_rule(*leaves, use_qk_l2norm_in_kernel=True, auto_cp=False, enable_fwd_cp_cache=False)
     rows = 2 * T * 2  # of q and of k
     assert sum(held.values()) <= rows * (128 * 2 + 4) + 4 * T * (128 * 2 + 64 * 2 + 4 + 4)  # q k rstd; v A g beta
+
+
+def test_the_class_normalises_float32_as_it_is():
+    """``ChunkGatedDeltaRuleFunction`` takes q, k, v of other types too: the normalisation and its gradient
+    stay in float32, only what the kernels read is bfloat16."""
+    from flash_qla.ops.gated_delta_rule.chunk import ChunkGatedDeltaRuleFunction
+    from flashqla_b200.utils import l2norm
+
+    leaves = _inputs(150, torch.float32)
+    q, k, v, g, beta = leaves
+    got = []
+    for in_op in (True, False):
+        qk = (q, k) if in_op else (l2norm(q), l2norm(k))
+        o = ChunkGatedDeltaRuleFunction.apply(*qk, v, g, beta, None, None, False, None, in_op)[0]
+        assert o.dtype == torch.float32
+        got.append([o, *torch.autograd.grad(o.square().sum(), leaves[:3])])
+    for a, b in zip(*got):
+        assert a.dtype == torch.float32 and torch.equal(a, b)
