@@ -130,7 +130,11 @@ __device__ __forceinline__ void cp_async4(float* smem_dst, const float* gmem_src
 // staged in panels inside the step took 16 us a step: the 18-segment chains of two heads of 32768
 // tokens 293 us, now 51.
 // Few CTAs (one per SM) take the (sequence, head) pairs in turn, gridDim.y apart, and only those
-// that have a chain at all (any_fb): usually none has, and a CTA then ends after one load.
+// that have a chain at all: usually none has, and a CTA then ends after a few loads.  Pairs that apply no
+// M (all of them, where the gates forget) are copies and left to merge_plain_kernel, whose blocks need
+// no SM of their own: beside a recurrence that leaves 16 SMs free, the start states of eight GPUs' shards
+// took 90 us here for 8 heads and 170 for 16, one CTA per SM in eight and nine rounds; now 37 and 55 (27 and
+// 35 with CTAs of 33 KB, whose chains with M took 254 and 311 us there against 225 and 258).
 template <int D>
 struct Merge {
   static constexpr int BV = 8, NT = 256, KS = 2 * NT / D, KB = D / KS, LDM = D + 4;
@@ -149,6 +153,18 @@ struct MergeParams {
   // (packed tensors, or the records of a gathered buffer); raw and out are always packed
   long long seg_stride, use_stride;
 };
+// Whether the chain of a (sequence, head) applies M in some step (looking at every `stride`-th one from
+// `first` on).  The last step of a chain applies nothing, and its segment's flag need not exist.
+__device__ __forceinline__ bool applies_m(const MergeParams& p, int pair, int first, int stride) {
+  const int r = pair / p.Hv, hv = pair % p.Hv;
+  const int s0 = p.seg_begin[r], n = p.seg_begin[r + 1] - s0;
+  if (!p.use_m) return n > 1;
+  const int begin = p.reverse ? s0 + 1 : s0;  // of the n - 1 segments that hand a state on
+  int any = 0;
+#pragma unroll 8
+  for (int i = first; i < n - 1; i += stride) any |= p.use_m[(long long)(begin + i) * p.use_stride + hv];
+  return any != 0;
+}
 template <int D>
 __global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
   using C = Merge<D>;
@@ -273,7 +289,8 @@ __global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
 #pragma unroll 1
   for (int base = 0; base < mine; base += NT) {
     const int i = base + t;
-    const bool on = i < mine && (!p.any_fb || p.any_fb[blockIdx.y + (long long)i * gridDim.y] != 0);
+    const long long item = blockIdx.y + (long long)i * gridDim.y;
+    const bool on = i < mine && (p.any_fb ? p.any_fb[item] != 0 : applies_m(p, (int)item, 0, 1));
     const unsigned bits = __ballot_sync(0xffffffffu, on);
     if ((t & 31) == 0) active[t / 32] = bits;
     __syncthreads();
@@ -287,18 +304,45 @@ __global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
   }
 }
 
-// The (sequence, head) pairs without a chain: only the edge segment's entry is written.
+// The (sequence, head) pairs without a chain: the edge segment's entry is raw, and (without any_fb, which
+// says that nobody reads them) the others are the local states next to them.  A copy, PLAIN_ROWS rows of
+// the pair's states per block: 9 records of 8 heads, 9.4 MB moved, together with the launch of merge_kernel
+// that then finds nothing 11 us (14 in its chains).
+constexpr int PLAIN_ROWS = 8;
 template <int D>
-__global__ void __launch_bounds__(D) merge_edge_kernel(const MergeParams p) {
+__global__ void __launch_bounds__(256) merge_plain_kernel(const MergeParams p) {
   pdl_wait();
-  const int hv = blockIdx.y, r = blockIdx.z;
+  const int pair = blockIdx.x, r = pair / p.Hv, hv = pair % p.Hv;
   const int s0 = p.seg_begin[r], s1 = p.seg_begin[r + 1];
-  if (s1 <= s0 || p.any_fb[r * p.Hv + hv] != 0) return;
-  const float* src = p.raw ? p.raw + ((long long)r * p.Hv + hv) * D * D : nullptr;
-  float* dst = p.out + ((long long)(p.reverse ? s1 - 1 : s0) * p.Hv + hv) * D * D;
-  const int v = threadIdx.x;
-  for (int k = blockIdx.x; k < D; k += gridDim.x)
-    dst[(long long)k * D + v] = !src ? 0.f : src[p.raw_v_first ? (long long)v * D + k : (long long)k * D + v];
+  if (s1 <= s0) return;
+  if (p.any_fb ? p.any_fb[pair] != 0 : __syncthreads_or(applies_m(p, pair, threadIdx.x, 256))) return;
+  const int row0 = blockIdx.y * PLAIN_ROWS, first = p.reverse ? s1 - 1 : s0;
+  const float* raw = p.raw ? p.raw + (long long)pair * D * D : nullptr;
+  auto out = [&](int seg) { return p.out + (((long long)seg * p.Hv + hv) * D + row0) * D; };
+  for (int i = threadIdx.x; i < PLAIN_ROWS * D; i += 256) {
+    const int k = row0 + i / D, v = i % D;
+    out(first)[i] = !raw ? 0.f : raw[p.raw_v_first ? (long long)v * D + k : (long long)k * D + v];
+  }
+  if (p.any_fb) return;
+  // all steps at once: they are independent
+  const int step = p.reverse ? -1 : 1;
+  const float* local = p.local + ((long long)hv * D + row0) * D;
+  if (p.vec16) {
+    constexpr int PER = PLAIN_ROWS * D / 4;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < (s1 - s0 - 1) * PER; i += 256) {
+      const int seg = first + step * (i / PER);
+      reinterpret_cast<float4*>(out(seg + step))[i % PER] =
+          reinterpret_cast<const float4*>(local + (long long)seg * p.seg_stride)[i % PER];
+    }
+  } else {
+    constexpr int PER = PLAIN_ROWS * D;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < (s1 - s0 - 1) * PER; i += 256) {
+      const int seg = first + step * (i / PER);
+      out(seg + step)[i % PER] = local[(long long)seg * p.seg_stride + i % PER];
+    }
+  }
 }
 
 template <int D>
@@ -310,14 +354,19 @@ static int launch_merge(const fqla_merge_args& a, cudaStream_t st) {
   p.reverse = a.reverse; p.raw_v_first = a.raw_v_first;
   p.seg_stride = a.seg_stride ? a.seg_stride : (long long)a.Hv * D * D;
   p.use_stride = a.seg_stride ? a.seg_stride : a.Hv;
-  p.vec16 = ((reinterpret_cast<uintptr_t>(a.M) | (unsigned long long)p.seg_stride * 4) & 15) == 0;
+  p.vec16 = ((reinterpret_cast<uintptr_t>(a.M) | reinterpret_cast<uintptr_t>(a.local) |
+              reinterpret_cast<uintptr_t>(a.out) | (unsigned long long)p.seg_stride * 4) & 15) == 0;
   static std::atomic<unsigned long long> done;
   int rc = configure_smem((const void*)merge_kernel<D>, C::SMEM_BYTES, done);
   if (rc != 0) return rc;
+  // With any_fallback and no_edges nothing is asked of pairs without a chain; always applying M, every
+  // sequence of two segments has one.
+  if (!(a.any_fallback && a.no_edges)) {
+    rc = launch_pdl(merge_plain_kernel<D>, dim3(p.n_pairs, D / PLAIN_ROWS), dim3(256), 0, st, p);
+    if (rc != 0) return rc;
+  }
   const int y = p.n_pairs < C::CTAS_Y ? p.n_pairs : C::CTAS_Y;
-  rc = launch_pdl(merge_kernel<D>, dim3(D / C::BV, y), dim3(C::NT), C::SMEM_BYTES, st, p);
-  if (rc != 0 || !a.any_fallback || a.no_edges) return rc;
-  return launch_pdl(merge_edge_kernel<D>, dim3(8, a.Hv, a.n_raw), dim3(D), 0, st, p);
+  return launch_pdl(merge_kernel<D>, dim3(D / C::BV, y), dim3(C::NT), C::SMEM_BYTES, st, p);
 }
 
 }  // namespace fqla
