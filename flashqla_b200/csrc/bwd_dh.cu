@@ -316,7 +316,8 @@ template <int D>
 static int launch_bwd_dh(const BwdDhParams& p, cudaStream_t st) {
   // narrower slices while every CTA has an SM of its own (see fwd_seq.cu; 512 tokens x 4 heads,
   // D = 64: 32 -> 25 us)
-  if (D == 64 && (long long)p.N * p.Hv * 2 <= sm_count()) return launch_slices<D, 32>(p, st);
+  if constexpr (D == 64)
+    if ((long long)p.N * p.Hv * 2 <= sm_count()) return launch_slices<D, 32>(p, st);
   return launch_slices<D, 64>(p, st);
 }
 

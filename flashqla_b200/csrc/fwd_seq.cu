@@ -362,7 +362,8 @@ static int launch_fwd_seq(const FwdSeqParams& p, cudaStream_t st) {
   // Columns of the state are independent.  While every CTA still has an SM of its own, slices half as
   // wide shorten the chain of a chunk (512 tokens x 4 heads, D = 64: 32 -> 24 us); past that they
   // would only repeat Q K^T and the loads of q, k, A.
-  if (D == 64 && (long long)p.N * p.Hv * (p.M ? 4 : 2) <= sm_count()) return launch_slices<D, 32>(p, st);
+  if constexpr (D == 64)
+    if ((long long)p.N * p.Hv * (p.M ? 4 : 2) <= sm_count()) return launch_slices<D, 32>(p, st);
   return launch_slices<D, 64>(p, st);
 }
 

@@ -18,7 +18,6 @@ struct GatedDeltaRuleBackward : public ag::Node {
   Options opt;
   at::ScalarType dtype = at::kBFloat16, beta_dtype = at::kFloat, g_dtype = at::kFloat,
                  h0_dtype = at::kFloat;
-  bool has_h0 = false;
   at::TensorOptions o_options;
   std::vector<int64_t> o_sizes;
 
@@ -80,7 +79,6 @@ std::pair<at::Tensor, OptTensor> apply(const at::Tensor& q, const at::Tensor& k,
   node->dtype = q.scalar_type();
   node->beta_dtype = beta.scalar_type();
   node->g_dtype = g.scalar_type();
-  node->has_h0 = initial_state.has_value();
   if (initial_state) node->h0_dtype = initial_state->scalar_type();
   node->o_options = r.o.options();
   node->o_sizes = r.o.sizes().vec();

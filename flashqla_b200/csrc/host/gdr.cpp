@@ -21,10 +21,10 @@ constexpr int CHUNK = 64;
 constexpr float THRESHOLD = -10.f;  // log of what a truncated past may still weigh
 
 void check(int status, const char* what) {
-  launch_count.fetch_add(1, std::memory_order_relaxed);
   if (status != FQLA_OK)
     throw PyError(PyError::Fqla, std::string(what) + " failed with status " + std::to_string(status) +
                                      ": " + fqla_status_string(status));
+  launch_count.fetch_add(1, std::memory_order_relaxed);
 }
 
 at::Tensor empty(at::IntArrayRef sizes, at::ScalarType dtype, c10::Device dev) {
