@@ -6,13 +6,16 @@ unchanged signatures (``chunk_gated_delta_rule_fwd`` ``:33-88``, ``chunk_gated_d
 file (not behind an alias) so that source-level checks written against the reference, such as
 its ``tests/test_function_signature.py``, find the class where they look for it.
 
-Pipeline (all launches on the current CUDA stream):
+Pipeline (``csrc/host/gdr.cpp``; all launches on the current CUDA stream):
 
-* forward:  chunk-local cumsum of g -> kkt + triangular solve (A) -> [segment planning and
-  state hand-off when a sequence is split for context parallelism] -> sequential recurrence
-  (o, optional h, final state).
-* backward: recompute h and v_new -> reverse recurrence of the state gradient (dh, du, dh0)
-  -> chunk-parallel dq/dk/dv/dbeta/dg -> GVA group sum -> reverse cumsum of dg.
+* forward:  [L2 normalisation of q, k and conversion of float16, one launch] -> chunk-local cumsum
+  of g, kkt and triangular solve (g_cum, A; one launch) -> [scan, exact state pass and merge chain
+  where a sequence is split into segments] -> sequential recurrence (o, optional h, final state; with
+  the cache on also the per-chunk states and v_new).
+* backward: [h and v_new recomputed where the forward kept none] -> [scan, exact passes, chain] ->
+  reverse recurrence of the state gradient (dh, du, dh0) -> chunk-parallel dq/dk/dv/dbeta/dg with
+  the reverse cumsum of dg -> [sum over the value heads of a group, gradient of the normalisation
+  and conversion, one launch].
 """
 
 from __future__ import annotations
@@ -38,8 +41,8 @@ def _switches(auto_cp, state_v_first) -> int:
 
 # With the forward cache on (the training path), the forward also keeps what the backward would
 # otherwise recompute with a second pass of the recurrence: the state entering every chunk and
-# v_new, as the operand tiles the chunk-parallel backward reads (768 bytes per token and value
-# head).  Set to False to trade that memory for the recomputation.
+# v_new.  K = V = 128: as the operand tiles the chunk-parallel backward reads, 768 bytes per token and
+# value head; K = V = 64: as rows, 256 bytes.  Set to False to trade that memory for the recomputation.
 SAVE_STATE_TILES = True
 
 
