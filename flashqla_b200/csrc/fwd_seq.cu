@@ -387,7 +387,7 @@ extern "C" int fqla_fwd_run(const fqla_fwd_args* args, void* stream) {
   // v_new for the backward pass (neither q nor o) and the state-only pass with the transition
   // matrices run on the tcgen05 kernel; D = 64 and other combinations of outputs on the mma.sync
   // kernel in this file.  (End states and matrices of two heads of 32768 tokens, 18 segments: 78 us
-  // on the mma.sync kernel, 61 on the tcgen05 one; a pass that finds nothing to do, 4 us on either.
+  // on the mma.sync kernel, 54 on the tcgen05 one; a pass that finds nothing to do, 4 us on either.
   // Relative error of o in the heads that never forget, against 64 bits, 8192 tokens with fp32 beta /
   // 16384 with bf16 beta: 4.09e-3 / 3.72e-3 with the mma.sync pass, 3.95e-3 / 3.57e-3 with this one;
   // with w = A diag(beta gamma) K as the full walk forms it, 54 us and 4.16e-3 / 3.62e-3.)

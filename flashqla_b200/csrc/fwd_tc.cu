@@ -172,8 +172,8 @@ enum { FULL0 = 0, FULL1, EMPTY0, EMPTY1, S_COPY, S_DEC, VN_DONE, S_DONE, P_DONE,
        SB_FREE,
        // state-only pass: U^T is complete; W^T, made by the V and the O group, is (its name there)
        U_DONE = P_DONE, WB_READY = P_READY };
-// vectors inside a slot; V_GL holds gamma_last at [0], V_BG gamma instead of beta gamma in the
-// state-only pass
+// vectors inside a slot; V_GL holds gamma_last at [0], V_BG -beta gamma instead of beta gamma in
+// the state-only pass
 enum { V_G = 0, V_BETA = 1, V_BG = 2, V_RHO = 3, V_SGAM = 4, V_GL = 5 };
 }  // namespace fwdtc
 
@@ -471,12 +471,18 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       ok = WAIT(FULL0 + s, (it >> 1) & 1);
       if (!ok) break;
       const float* vs = vec + (it & 3) * VEC_SLOT_FLOATS + t0;
-      // off the chain: this thread's value index of its 32 tokens
+      // off the chain: beta V^T, this thread's value index of its 32 tokens, and -beta gamma
       const unsigned char* vt = smem + OFF_STAGE + s * STAGE_BYTES + 2 * TILE_QK + (v >> 6) * 8192;
-      float x[32], y[32];
+      auto load32 = [&](const float* src, float (&a)[32]) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(a + 4 * i) = *reinterpret_cast<const float4*>(src + 4 * i);
+      };
+      float x[32], y[32], f[32];
+      load32(vs + V_BETA * CHUNK, y);
+      load32(vs + V_BG * CHUNK, f);
 #pragma unroll
       for (int j = 0; j < 32; ++j)
-        y[j] = __bfloat162float(*reinterpret_cast<const bf16*>(vt + sw128_offset(t0 + j, v & 63)));
+        y[j] *= __bfloat162float(*reinterpret_cast<const bf16*>(vt + sw128_offset(t0 + j, v & 63)));
       ok = WAIT(U_DONE, it & 1);
       if (!ok) break;
       tc_fence_after();
@@ -484,35 +490,28 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       tmem_ld_wait();
       uint32_t pk[16];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 b = *reinterpret_cast<const float4*>(vs + V_BETA * CHUNK + 4 * i);
-        const float4 g = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 4 * i);
-        y[4 * i] = b.x * (y[4 * i] - g.x * x[4 * i]);
-        y[4 * i + 1] = b.y * (y[4 * i + 1] - g.y * x[4 * i + 1]);
-        y[4 * i + 2] = b.z * (y[4 * i + 2] - g.z * x[4 * i + 2]);
-        y[4 * i + 3] = b.w * (y[4 * i + 3] - g.w * x[4 * i + 3]);
-      }
+      for (int j = 0; j < 32; ++j) y[j] += f[j] * x[j];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {  // operand, and in y what its rounding left out
-        pk[i] = pack_bf16(y[2 * i], y[2 * i + 1]);
-        y[2 * i] -= __uint_as_float(pk[i] << 16);
-        y[2 * i + 1] -= __uint_as_float(pk[i] & 0xffff0000u);
-      }
+      for (int i = 0; i < 16; ++i) pk[i] = pack_bf16(y[2 * i], y[2 * i + 1]);
       tmem_st16(tmem + lane_sel + TM_WB + (t0 >> 1), pk);
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&bars[WB_READY]);
+      // off the chain: rho, and rho times what the rounding of the operand left out
+      load32(vs + V_RHO * CHUNK, f);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        y[2 * i] = f[2 * i] * (y[2 * i] - __uint_as_float(pk[i] << 16));
+        y[2 * i + 1] = f[2 * i + 1] * (y[2 * i + 1] - __uint_as_float(pk[i] & 0xffff0000u));
+      }
       ok = WAIT(VN_DONE, it & 1);
       if (!ok) break;
       tc_fence_after();
       tmem_ld32(tmem + lane_sel + TM_VN + t0, x);
       tmem_ld_wait();
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 r = *reinterpret_cast<const float4*>(vs + V_RHO * CHUNK + 4 * i);
-        pk[2 * i] = pack_bf16(r.x * (x[4 * i] + y[4 * i]), r.y * (x[4 * i + 1] + y[4 * i + 1]));
-        pk[2 * i + 1] = pack_bf16(r.z * (x[4 * i + 2] + y[4 * i + 2]), r.w * (x[4 * i + 3] + y[4 * i + 3]));
-      }
+      for (int i = 0; i < 16; ++i)
+        pk[i] = pack_bf16(f[2 * i] * x[2 * i] + y[2 * i], f[2 * i + 1] * x[2 * i + 1] + y[2 * i + 1]);
       tmem_st16(tmem + lane_sel + TM_VRB + (t0 >> 1), pk);
       tmem_st_wait();
       tc_fence_before();
@@ -1045,7 +1044,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           float gam = fast_exp(g_r[z]);
           vs[V_G * CHUNK + r] = g_r[z];
           vs[V_BETA * CHUNK + r] = b_r[z];
-          vs[V_BG * CHUNK + r] = STATE ? gam : b_r[z] * gam;
+          vs[V_BG * CHUNK + r] = STATE ? -b_r[z] * gam : b_r[z] * gam;
           vs[V_RHO * CHUNK + r] = fast_exp(gl_r - g_r[z]);
           vs[V_SGAM * CHUNK + r] = p.scale * gam;
         }
