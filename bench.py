@@ -373,8 +373,8 @@ def dominant_kernel_roofline(timer, x, bwd, steps):
         # dq,dk,dv,dg,db out
         min_bytes = 2 * 256 / G + 2 * 256 + 128 + 6 + 3 * 256 + 8
         kernel_bytes = bwd_main_kernel_bytes(G)
-        # 16 tile products per chunk: 3 of 64x128x128, 5 of 64x64x128, 6 of 64x128x64, 2 of 64x64x64
-        flop_per_pair = 2 * (3 * 128 * 128 + 5 * 64 * 128 + 6 * 128 * 64 + 2 * 64 * 64)
+        # 11 tile products per chunk: 3 of 64x128x128, 4 of 64x64x128, 4 of 64x128x64
+        flop_per_pair = 2 * (3 * 128 * 128 + 4 * 64 * 128 + 4 * 128 * 64)
     for _ in range(3):
         dominant()
     k_ms = timer.run(dominant, steps, input_bytes(x) < 2 * L2_BYTES)

@@ -2,22 +2,27 @@
 //
 // Same mathematics and same outputs as bwd_main.cu (the reference's tests/ref_gdr.py:427-600,
 // evaluated by the reference kernels inside blackwell/fused_bwd.py:595-862).  Persistent CTAs
-// (one per SM) walk the work items (chunk, value head).  All sixteen tile products are
-// tcgen05.mma with M = 64 (rows = tokens) and fp32 accumulators in tensor memory; two M = 64
-// accumulators share each column range (lanes +0 and +16 of every 32-lane quarter).
+// (one per SM) walk the work items (chunk, value head).  With v_new = A W, W = beta (V - gamma K S):
+//     dW = A^T du,   dL = -dW v_new^T below the diagonal (A = (I + L)^-1: the gradient through the inverse
+//                    needs no product with A but the one in dW),   X = beta G dL,   Y = dW h^T
+//     ds = scale G (dO v_new^T)
+//     dq = scale gamma dO h^T + ds K,   dv = beta dW
+//     dk = rho v_new dh^T - beta gamma Y + ds^T q + (X + X^T) K
+// and dg, dbeta from row and column sums of q dq1, k dk1, k Y, v dW, ds (Q K^T), dL (K K^T).  (As the chain
+// dA = -(du h^T) (beta gamma K)^T + du (beta V)^T, dL = -A^T dA A^T it was sixteen products and six
+// read-outs in a row instead of eleven and three: 262144 tokens x 8 heads 1484 us, now 1380.)
+// All tile products are tcgen05.mma with M = 64 (rows = tokens) and fp32 accumulators in tensor memory;
+// two M = 64 accumulators share each column range (lanes +0 and +16 of every 32-lane quarter).
 //
 // Roles: warp 16 issues every product and every TMA load (one elected thread).  Warps 0-7 (chain
-// group) read the 64-wide accumulators (16-lane shape) and write the intermediate operands (dw,
-// ds, dA, T, dA3) back to shared memory as bf16 tiles; warps 8-15 (bulk group) do what is off the
-// dependent chain: the h.dh sum, dq1 | dk1 (scaled in place in tensor memory), dv and the final
-// dq | dk, read in the 32-lane shape with 16-byte shared and global accesses.  The sides are
-// coupled by one mbarrier per product group (commit -> read-out) and one per operand tile
-// (written -> may be multiplied), so that the chain
-//     dw -> dA -> T = A^T dA -> dA3 -> (beta dA3) K, (beta dA3)^T K
-// never waits for the bulk work.  Row scalings ride on operands where they can (A diag(beta),
-// A diag(beta gamma) are written over the dead v tile; dk is one accumulator fed by four
-// products).  Operand tiles of the next item are fetched as soon as the buffers of the current
-// one are dead (k has two buffers).
+// group) make operands of accumulators (dW, ds, X + X^T as bf16 tiles in shared memory), read in the
+// 16-lane shape, and dv; warps 8-15 (bulk group) do what is off the dependent chain: the h.dh sum, the row
+// sums of dq1 and dk1, and the final dq | dk, read in the 32-lane shape with 16-byte shared and global
+// accesses.  The sides are coupled by one mbarrier per product group (commit -> read-out) and one per
+// operand tile (written -> may be multiplied), so that the chain
+//     dW -> D3 = dW v_new^T -> (X + X^T) K
+// never waits for the bulk work.  Operand tiles of the next item are fetched as soon as the buffers of the
+// current one are dead (k has two buffers).
 #include <cuda.h>
 
 #include <climits>
@@ -65,41 +70,40 @@ constexpr int OFF_VN = OFF_V + ROW_TILE, OFF_DO = OFF_VN + ROW_TILE, OFF_DU = OF
 constexpr int OFF_H = OFF_DU + ROW_TILE;
 constexpr int OFF_DH = OFF_H + SQ_TILE;
 constexpr int OFF_A = OFF_DH + SQ_TILE;
-constexpr int OFF_DS = OFF_A + 8192;        // ds, later diag(beta) dA3
-constexpr int OFF_DA = OFF_DS + 8192;       // dA, then T = A^T dA, then dA3
-constexpr int OFF_DW = OFF_DA + 8192;       // -du h^T
-// g, gamma, rho, beta (64 floats each); per-warp partial sums of dg (rows: 4 column quarters x 64,
-// columns: 4 lane quarters x 64), of db (rows 4 x 64, two column terms 4 x 64 each) and of the
-// chunk total (16)
+constexpr int OFF_DS = OFF_A + 8192;
+constexpr int OFF_X = OFF_DS + 8192;        // X + X^T, X = beta dL
+constexpr int OFF_DW = OFF_X + 8192;        // dW = A^T du
+// g, gamma, rho, beta of an item (64 floats each; two buffers); partial sums: of dg by row (chain group:
+// 2 x 64; bulk group: 4 x 64) and by column (4 x 64), of db by row (chain and bulk group 2 x 64 each), of
+// the chunk total (8) and what suffix_sum64 needs (2)
 constexpr int OFF_VEC = OFF_DW + ROW_TILE;
-constexpr int OFF_BAR = OFF_VEC + (4 * 64 + 5 * 256 + 512 + 18) * 4;
-constexpr int N_BARS = 23;
+constexpr int OFF_BAR = OFF_VEC + (2 * 256 + 128 + 3 * 256 + 18) * 4;
+constexpr int N_BARS = 20;
 constexpr int OFF_MISC = OFF_BAR + N_BARS * 8;
 constexpr int OFF_ITEM = OFF_MISC + 32;  // ring of four items, published by the issue warp
 constexpr int OFF_CLAIM = (OFF_ITEM + 4 * 32 + 15) / 16 * 16;  // CLC: two answers of 16 bytes
 constexpr int SMEM_BYTES = OFF_CLAIM + 2 * 16 + 1024;
 static_assert(SMEM_BYTES <= 232448, "one CTA's shared memory");
-// the operand tiles of one item arrive in three groups, in the order their buffers become free
-constexpr uint32_t TX_A = 2 * SQ_TILE + 3 * ROW_TILE;  // h, dh, dO, v_new, k (other buffer)
-constexpr uint32_t TX_B = 3 * ROW_TILE;                // du, q, v
-constexpr uint32_t TX_C = 8192;                        // A
-// tensor memory: (column, lane half) of every accumulator
+// the operand tiles of one item arrive in four groups
+constexpr uint32_t TX_D = 8192 + 2 * ROW_TILE;  // A, du, v
+constexpr uint32_t TX_A = 3 * ROW_TILE;         // dO, v_new, k (other buffer)
+constexpr uint32_t TX_H = 2 * SQ_TILE;          // h, dh
+// tensor memory: (column, lane half) of every accumulator; each has a place of its own
 constexpr uint32_t HI = 16u << 16;
-constexpr uint32_t T_DQ1 = 0, T_DK1 = 0 + HI, T_DW = 256;   // dq1 | dk1 share columns (lane halves)
-constexpr uint32_t T_DQ2 = 128, T_DK2 = 128 + HI;        // ds K | the four-product dk sum share columns
-constexpr uint32_t T_T2 = 256 + HI, T_DS = 384 + HI, T_QK = 448 + HI;
-constexpr uint32_t T_X1 = 256, T_X2 = 320;            // after dw has been read
-constexpr uint32_t T_T = 384 + HI, T_KK = 448 + HI;    // after ds, qk have been read
-constexpr uint32_t T_D3 = 256;                         // after x1 has been read
+constexpr uint32_t T_DQ1 = 0, T_DK1 = 0 + HI;      // dO h^T | v_new dh^T
+constexpr uint32_t T_DQ2 = 128, T_DK2 = 128 + HI;  // ds K | ds^T q + (X + X^T) K
+constexpr uint32_t T_DW = 256, T_Y = 256 + HI;     // A^T du | dW h^T
+constexpr uint32_t T_DS = 384, T_D3 = 384 + HI;    // dO v_new^T | dW v_new^T
+constexpr uint32_t T_QK = 448, T_KK = 448 + HI;
 enum {
-  L_A = 0, L_B, L_C,                                       // TMA groups landed
-  C_DW, C_DSQK, C_1B, C_X, C_2B, C_T, C_D3, C_5,           // product groups complete (commit)
-  R_ZERO, R_END,                     // all 16 read-out warps -> issue warp
-  R_DW, R_DS, R_DA, R_T, R_D3,       // the 8 warps of the chain group -> issue warp
-  R_HD, R_E4,                        // the 8 warps of the bulk group -> issue warp
-  R_CH,                              // the 8 warps of the chain group -> bulk group: item finished
-  I_NEXT,                            // issue warp -> read-out warps: the next item is in the ring
-  I_CLAIM                            // CLC: the answer with the next item has arrived
+  L_D = 0, L_A, L_H, L_Q,                // TMA groups landed
+  C_DW, C_DSQK, C_D3, C_1B, C_2, C_5,    // product groups complete (commit)
+  R_ZERO,                                // all 16 read-out warps -> issue warp (partial chunks only)
+  R_DW, R_DS, R_D3,                      // the 8 warps of the chain group -> issue warp
+  R_CH,                                  // ... -> bulk group: item finished
+  R_HD, R_E4, R_END,                     // the 8 warps of the bulk group -> issue warp
+  I_NEXT,                                // issue warp -> read-out warps: the next item is in the ring
+  I_CLAIM                                // CLC: the answer with the next item has arrived
 };
 }  // namespace bmtc
 
@@ -164,12 +168,11 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
   // behind the column sums
   float* sVec0 = reinterpret_cast<float*>(smem + OFF_VEC);
   float* sRowDg = sVec0 + 256;
-  float* sColDg = sRowDg + 256;
+  float* sColDg = sRowDg + 128;
   float* sRowDb = sColDg + 256;
-  float* sColC1 = sRowDb + 256;
-  float* sVec1 = sColC1 + 256;
-  float* sRowW = sVec1 + 256;  // row terms of the 128-wide steps: [column quarter x lane half][row]
-  float* sLast = sRowW + 512;
+  float* sVec1 = sRowDb + 256;
+  float* sRowW = sVec1 + 256;  // row terms of the 128-wide steps: [column half x lane half][row]
+  float* sLast = sRowW + 256;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long total = p.n_chunks * p.Hv;
@@ -219,10 +222,9 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
     return t;
   };
   if (tid == 0) {
-    for (int i = L_A; i <= C_5; ++i) mbar_init(&bars[i], 1);
+    for (int i = L_D; i <= C_5; ++i) mbar_init(&bars[i], 1);
     mbar_init(&bars[R_ZERO], N_EPI / 32);
-    mbar_init(&bars[R_END], N_EPI / 32);
-    for (int i = R_DW; i <= R_CH; ++i) mbar_init(&bars[i], N_EPI / 64);
+    for (int i = R_DW; i <= R_END; ++i) mbar_init(&bars[i], N_EPI / 64);
     mbar_init(&bars[I_NEXT], 1);
     if (CLC) mbar_init(&bars[I_CLAIM], 1);
     *abort_flag = 0;
@@ -242,14 +244,28 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
     // (the warp stays converged; see elect_one in tc05.cuh)
     {
       auto WAIT = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
+      // Four groups, in the order in which their buffers become free (A and du are dead after the first
+      // product of an item, q only after the bulk group has read it).
+      auto load_d = [&](const Item& t) {
+        const int y = (int)t.row0;
+        if (!elect_one()) return;
+        mbar_arrive_expect_tx(&bars[L_D], TX_D);
+        tma_load_2d(smem + OFF_A, &map_a, t.hv * CHUNK, y, &bars[L_D]);
+        if constexpr (TILED) {
+          tma_load_2d(smem + OFF_DU, &map_du, 0, (int)((t.chunk_id * p.Hv + t.hv) * D), &bars[L_D]);
+        } else {
+          tma_load_2d(smem + OFF_DU, &map_du, t.hv * D, y, &bars[L_D]);
+          tma_load_2d(smem + OFF_DU + 8192, &map_du, t.hv * D + 64, y, &bars[L_D]);
+        }
+        tma_load_2d(smem + OFF_V, &map_v, t.hv * D, y, &bars[L_D]);
+        tma_load_2d(smem + OFF_V + 8192, &map_v, t.hv * D + 64, y, &bars[L_D]);
+      };
       auto load_a = [&](const Item& t, int kbuf) {
         const int y = (int)t.row0, ys = (int)((t.chunk_id * p.Hv + t.hv) * D);
         if (!elect_one()) return;
         mbar_arrive_expect_tx(&bars[L_A], TX_A);
-        tma_load_2d(smem + OFF_DU - ROW_TILE, &map_do, t.hv * D, y, &bars[L_A]);  // = OFF_DO
+        tma_load_2d(smem + OFF_DO, &map_do, t.hv * D, y, &bars[L_A]);
         tma_load_2d(smem + OFF_DO + 8192, &map_do, t.hv * D + 64, y, &bars[L_A]);
-        tma_load_2d(smem + OFF_H, &map_h, 0, ys, &bars[L_A]);
-        tma_load_2d(smem + OFF_H + 16384, &map_h, 64, ys, &bars[L_A]);
         if constexpr (TILED) {
           tma_load_2d(smem + OFF_VN, &map_vn, 0, ys, &bars[L_A]);
         } else {
@@ -258,50 +274,33 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         }
         tma_load_2d(smem + OFF_K + kbuf * ROW_TILE, &map_k, t.hq * D, y, &bars[L_A]);
         tma_load_2d(smem + OFF_K + kbuf * ROW_TILE + 8192, &map_k, t.hq * D + 64, y, &bars[L_A]);
-        tma_load_2d(smem + OFF_DH, &map_dh, 0, ys, &bars[L_A]);
-        tma_load_2d(smem + OFF_DH + 16384, &map_dh, 64, ys, &bars[L_A]);
+        mbar_arrive_expect_tx(&bars[L_H], TX_H);
+        tma_load_2d(smem + OFF_H, &map_h, 0, ys, &bars[L_H]);
+        tma_load_2d(smem + OFF_H + 16384, &map_h, 64, ys, &bars[L_H]);
+        tma_load_2d(smem + OFF_DH, &map_dh, 0, ys, &bars[L_H]);
+        tma_load_2d(smem + OFF_DH + 16384, &map_dh, 64, ys, &bars[L_H]);
       };
-      auto load_b = [&](const Item& t) {
-        const int y = (int)t.row0;
+      auto load_q = [&](const Item& t) {
         if (!elect_one()) return;
-        mbar_arrive_expect_tx(&bars[L_B], TX_B);
-        if constexpr (TILED) {
-          tma_load_2d(smem + OFF_DU, &map_du, 0, (int)((t.chunk_id * p.Hv + t.hv) * D), &bars[L_B]);
-        } else {
-          tma_load_2d(smem + OFF_DU, &map_du, t.hv * D, y, &bars[L_B]);
-          tma_load_2d(smem + OFF_DU + 8192, &map_du, t.hv * D + 64, y, &bars[L_B]);
-        }
-        tma_load_2d(smem + OFF_Q, &map_q, t.hq * D, y, &bars[L_B]);
-        tma_load_2d(smem + OFF_Q + 8192, &map_q, t.hq * D + 64, y, &bars[L_B]);
-        tma_load_2d(smem + OFF_V, &map_v, t.hv * D, y, &bars[L_B]);
-        tma_load_2d(smem + OFF_V + 8192, &map_v, t.hv * D + 64, y, &bars[L_B]);
-      };
-      auto load_c = [&](const Item& t) {
-        if (!elect_one()) return;
-        mbar_arrive_expect_tx(&bars[L_C], TX_C);
-        tma_load_2d(smem + OFF_A, &map_a, t.hv * CHUNK, (int)t.row0, &bars[L_C]);
+        mbar_arrive_expect_tx(&bars[L_Q], ROW_TILE);
+        tma_load_2d(smem + OFF_Q, &map_q, t.hq * D, (int)t.row0, &bars[L_Q]);
+        tma_load_2d(smem + OFF_Q + 8192, &map_q, t.hq * D + 64, (int)t.row0, &bars[L_Q]);
       };
       // descriptors (low words)
-      const uint32_t q_lo = desc_lo_kmajor(smem + OFF_Q), v_lo = desc_lo_kmajor(smem + OFF_V);
+      const uint32_t q_lo = desc_lo_kmajor(smem + OFF_Q), qmn_lo = desc_lo_mnmajor(smem + OFF_Q, 8192);
       const uint32_t k_lo0 = desc_lo_kmajor(smem + OFF_K), kmn_lo0 = desc_lo_mnmajor(smem + OFF_K, 8192);
-      const uint32_t vn_lo = desc_lo_kmajor(smem + OFF_VN);
+      const uint32_t vn_lo = desc_lo_kmajor(smem + OFF_VN), dumn_lo = desc_lo_mnmajor(smem + OFF_DU, 8192);
       const uint32_t do_lo = desc_lo_kmajor(smem + OFF_DO), du_lo = desc_lo_kmajor(smem + OFF_DU);
       const uint32_t h_lo = desc_lo_kmajor(smem + OFF_H), dh_lo = desc_lo_kmajor(smem + OFF_DH);
-      const uint32_t a_lo = desc_lo_kmajor(smem + OFF_A), ds_lo = desc_lo_kmajor(smem + OFF_DS);
-      const uint32_t da_lo = desc_lo_kmajor(smem + OFF_DA), dw_lo = desc_lo_kmajor(smem + OFF_DW);
-      const uint32_t qmn_lo = desc_lo_mnmajor(smem + OFF_Q, 8192);
-      const uint32_t dumn_lo = desc_lo_mnmajor(smem + OFF_DU, 8192), dwmn_lo = desc_lo_mnmajor(smem + OFF_DW, 8192);
-      const uint32_t amn_lo = desc_lo_mnmajor(smem + OFF_A, 8192), dsmn_lo = desc_lo_mnmajor(smem + OFF_DS, 8192);
-      const uint32_t damn_lo = desc_lo_mnmajor(smem + OFF_DA, 8192);
-      const uint32_t a1mn_lo = desc_lo_mnmajor(smem + OFF_V, 8192), a2mn_lo = desc_lo_mnmajor(smem + OFF_V + 8192, 8192);
+      const uint32_t amn_lo = desc_lo_mnmajor(smem + OFF_A, 8192), dw_lo = desc_lo_kmajor(smem + OFF_DW);
+      const uint32_t ds_lo = desc_lo_kmajor(smem + OFF_DS), dsmn_lo = desc_lo_mnmajor(smem + OFF_DS, 8192);
+      const uint32_t x_lo = desc_lo_kmajor(smem + OFF_X);
       // operand-tile layouts: [V rows][K or token columns], read MN-major, contraction over rows
       const uint32_t hT_lo = desc_lo_mnmajor(smem + OFF_H, 16384), dhT_lo = desc_lo_mnmajor(smem + OFF_DH, 16384);
-      const uint32_t vnT_lo = desc_lo_mnmajor(smem + OFF_VN, 16384), duT_lo = desc_lo_mnmajor(smem + OFF_DU, 16384);
+      const uint32_t vnT_lo = desc_lo_mnmajor(smem + OFF_VN, 16384);
       constexpr uint32_t ID_KK_128 = idesc_bf16(64, 128, 0, 0), ID_KK_64 = idesc_bf16(64, 64, 0, 0);
       constexpr uint32_t ID_KM_128 = idesc_bf16(64, 128, 0, 1), ID_MM_128 = idesc_bf16(64, 128, 1, 1);
-      constexpr uint32_t ID_MM_64 = idesc_bf16(64, 64, 1, 1);
-      constexpr uint32_t ID_KM_64 = idesc_bf16(64, 64, 0, 1), ID_MK_64 = idesc_bf16(64, 64, 1, 0);
-      constexpr uint32_t ID_MK_128 = idesc_bf16(64, 128, 1, 0);
+      constexpr uint32_t ID_KM_64 = idesc_bf16(64, 64, 0, 1), ID_MK_128 = idesc_bf16(64, 128, 1, 0);
       constexpr uint32_t KBUF_LO = ROW_TILE >> 4;
 
       Raw raw = {};
@@ -310,71 +309,72 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       load_index((int)blockIdx.x / p.Hv, raw);
       load_span(raw);
       Item cur = finish(raw, (int)blockIdx.x % p.Hv);
+      load_d(cur);
       load_a(cur, 0);
-      load_b(cur);
-      load_c(cur);
+      load_q(cur);
       bool ok = true;
-      uint32_t it = 0;
+      uint32_t it = 0, zero_ph = 0;
+      // An accumulator or an operand tile is written again only behind a barrier that says it has been
+      // read: what the chain group reads (dW, ds, qk, KK, D3) behind its own arrivals on the tiles it makes
+      // of them, what the bulk group reads (dq, dk, Y) behind R_END of the item before.
 #pragma unroll 1
       for (bool has_next = true; has_next && ok; ++it) {
         const uint32_t ph = it & 1;
         if (!CLC && lane == 0) claimed = (int)gridDim.x + atomicAdd(p.next_item, 1);
         const uint32_t k_lo = k_lo0 + (ph ? KBUF_LO : 0u), kmn_lo = kmn_lo0 + (ph ? KBUF_LO : 0u);
-        // the read-out warps have finished the previous item (accumulators free) and have zeroed
-        // the rows past the sequence end in this item's tiles (which also means: tiles landed)
-        // A full chunk needs no zero fill: its first products start as soon as its tiles have
-        // landed, while the bulk group still finishes the previous item (the accumulators they
-        // write were last read by the chain group, whose R_D3 this thread has seen; dq1 | dk1 and
-        // what follows wait for R_END of the previous item).
-        if (cur.valid == CHUNK) ok = WAIT(L_A, ph) && WAIT(L_B, ph);
-        else ok = (it == 0 || WAIT(R_END, (it - 1) & 1)) && WAIT(R_ZERO, ph);
+        // A partial chunk waits until the read-out warps have zeroed the rows past the sequence end (which
+        // also means that all its tiles have landed).
+        const bool partial = cur.valid != CHUNK;
+        if (partial) {
+          if (it > 0) {  // q of this item, below for a full chunk
+            ok = WAIT(C_2, ph ^ 1) && WAIT(R_E4, ph ^ 1);
+            if (!ok) break;
+            load_q(cur);
+          }
+          ok = WAIT(R_ZERO, zero_ph);
+          zero_ph ^= 1;
+        } else {
+          ok = WAIT(L_D, ph);
+        }
         if (!ok) break;
         tc_fence_after();
-        // ---- products that need only loaded tiles ----
+        // ---- dW = A^T du: needs nothing but A and du ----
         if (elect_one()) {
-          if constexpr (TILED) {
-            umma_group<8, 128, 512, 128, 512, false>(tmem + T_DW, duT_lo, hT_lo, ID_MM_128);
-          } else {
-            umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DW, du_lo, h_lo, ID_KK_128);
-          }
+          if constexpr (TILED) umma_group<4, 128, 0, 2, 0, false>(tmem + T_DW, amn_lo, du_lo, ID_MK_128);
+          else umma_group<4, 128, 0, 128, 0, false>(tmem + T_DW, amn_lo, dumn_lo, ID_MM_128);
           umma_commit(&bars[C_DW]);
-          if constexpr (TILED) {
-            umma_group<8, 2, 512, 128, 512, false>(tmem + T_DS, do_lo, vnT_lo, ID_KM_64);
-          } else {
-            umma_group<8, 2, 512, 2, 512, false>(tmem + T_DS, do_lo, vn_lo, ID_KK_64);
-          }
-          umma_group<8, 2, 512, 2, 512, false>(tmem + T_QK, q_lo, k_lo, ID_KK_64);
-          umma_commit(&bars[C_DSQK]);
           if constexpr (CLC) {
             mbar_arrive_expect_tx(&bars[I_CLAIM], 16);
             clc_try_cancel(answers + 16 * ph, &bars[I_CLAIM]);
           }
         }
-        // ---- dw is an operand now: the pieces of dA, and A^T dw, A^T du ----
+        if (!partial) {
+          if (it > 0) {
+            // q of the item before is dead: its product is complete, the bulk group has used it
+            ok = WAIT(C_2, ph ^ 1) && WAIT(R_E4, ph ^ 1);
+            if (!ok) break;
+            load_q(cur);
+          }
+          ok = WAIT(L_A, ph) && WAIT(L_Q, ph);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        // ---- ds, q k^T, K K^T ----
+        if (elect_one()) {
+          if constexpr (TILED) umma_group<8, 2, 512, 128, 512, false>(tmem + T_DS, do_lo, vnT_lo, ID_KM_64);
+          else umma_group<8, 2, 512, 2, 512, false>(tmem + T_DS, do_lo, vn_lo, ID_KK_64);
+          umma_group<8, 2, 512, 2, 512, false>(tmem + T_QK, q_lo, k_lo, ID_KK_64);
+          umma_commit(&bars[C_DSQK]);
+          umma_group<8, 2, 512, 2, 512, false>(tmem + T_KK, k_lo, k_lo, ID_KK_64);
+        }
+        // ---- dW is an operand now: D3 = dW v_new^T ----
         ok = WAIT(R_DW, ph);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
-          umma_group<8, 2, 512, 2, 512, false>(tmem + T_X1, dw_lo, k_lo, ID_KK_64);
-          if constexpr (TILED) umma_group<8, 128, 512, 2, 512, false>(tmem + T_X2, duT_lo, v_lo, ID_MK_64);
-          else umma_group<8, 2, 512, 2, 512, false>(tmem + T_X2, du_lo, v_lo, ID_KK_64);
-          umma_commit(&bars[C_X]);
-        }
-        // products off the dependent chain go behind the ones the read-out is waiting for
-        if (it > 0) {
-          ok = WAIT(R_END, (it - 1) & 1);
-          if (!ok) break;
-          tc_fence_after();
-        }
-        if (elect_one()) {
-          if constexpr (TILED) {
-            umma_group<8, 2, 512, 128, 512, false>(tmem + T_DQ1, do_lo, hT_lo, ID_KM_128);
-            umma_group<8, 128, 512, 128, 512, false>(tmem + T_DK1, vnT_lo, dhT_lo, ID_MM_128);
-          } else {
-            umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DQ1, do_lo, h_lo, ID_KK_128);
-            umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DK1, vn_lo, dh_lo, ID_KK_128);
-          }
-          umma_commit(&bars[C_1B]);
+          if constexpr (TILED) umma_group<8, 2, 512, 128, 512, false>(tmem + T_D3, dw_lo, vnT_lo, ID_KM_64);
+          else umma_group<8, 2, 512, 2, 512, false>(tmem + T_D3, dw_lo, vn_lo, ID_KK_64);
+          umma_commit(&bars[C_D3]);
         }
         int w_next;
         if constexpr (CLC) {
@@ -389,6 +389,23 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         }
         const int h_next = has_next ? w_next % p.Hv : 0;
         if (has_next) load_index(w_next / p.Hv, raw);
+        // ---- Y = dW h^T, dq1, dk1: off the chain ----
+        ok = WAIT(L_H, ph) && (it == 0 || WAIT(R_END, ph ^ 1));
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          if constexpr (TILED) {
+            umma_group<8, 2, 512, 128, 512, false>(tmem + T_Y, dw_lo, hT_lo, ID_KM_128);
+            umma_group<8, 2, 512, 128, 512, false>(tmem + T_DQ1, do_lo, hT_lo, ID_KM_128);
+            umma_group<8, 128, 512, 128, 512, false>(tmem + T_DK1, vnT_lo, dhT_lo, ID_MM_128);
+          } else {
+            umma_group<8, 2, 512, 2, 1024, false>(tmem + T_Y, dw_lo, h_lo, ID_KK_128);
+            umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DQ1, do_lo, h_lo, ID_KK_128);
+            umma_group<8, 2, 512, 2, 1024, false>(tmem + T_DK1, vn_lo, dh_lo, ID_KK_128);
+          }
+          umma_commit(&bars[C_1B]);
+        }
+        if (has_next) load_span(raw);
         // ---- ds is an operand now ----
         ok = WAIT(R_DS, ph);
         if (!ok) break;
@@ -396,16 +413,12 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         if (elect_one()) {
           umma_group<4, 2, 0, 128, 0, false>(tmem + T_DQ2, ds_lo, kmn_lo, ID_KM_128);
           umma_group<4, 128, 0, 128, 0, false>(tmem + T_DK2, dsmn_lo, qmn_lo, ID_MM_128);
-          umma_group<8, 2, 512, 2, 512, false>(tmem + T_KK, k_lo, k_lo, ID_KK_64);  // qk has been read
+          umma_commit(&bars[C_2]);
         }
-        if (has_next) load_span(raw);
-        // h, dh, dO, v_new are dead once the first products are complete and the h.dh sum is done
-        ok = WAIT(C_1B, ph) && WAIT(R_HD, ph);
-        if (!ok) break;
         Item nxt = cur;
         if (has_next) {
           nxt = finish(raw, h_next);
-          load_a(nxt, (int)(ph ^ 1));
+          load_d(nxt);  // A, du and v are dead: the chain group made dW, dv and what follows of them
         } else {
           nxt.valid = 0;  // the read-out warps stop
         }
@@ -413,51 +426,20 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           ring[(it + 1) & 3] = nxt;
           mbar_arrive(&bars[I_NEXT]);
         }
-        // ---- dA -> T = A^T dA (and K K^T) ----
-        ok = WAIT(R_DA, ph);
-        if (!ok) break;
-        tc_fence_after();
-        if (elect_one()) {
-          umma_group<4, 128, 0, 128, 0, false>(tmem + T_T, amn_lo, damn_lo, ID_MM_64);
-          umma_commit(&bars[C_T]);
-          // with A' = A diag(beta) and A'' = A diag(beta gamma) (written over the dead v tile):
-          // dk += A''^T dw (onto ds^T q), dv = A'^T du -- the row scalings ride on the operands
-          umma_group<4, 128, 0, 128, 0, true>(tmem + T_DK2, a2mn_lo, dwmn_lo, ID_MM_128);
-          if constexpr (TILED) umma_group<4, 128, 0, 2, 0, false>(tmem + T_T2, a1mn_lo, du_lo, ID_MK_128);
-          else umma_group<4, 128, 0, 128, 0, false>(tmem + T_T2, a1mn_lo, dumn_lo, ID_MM_128);
-          umma_commit(&bars[C_2B]);
-        }
-        // ---- T -> d3 = T A^T ----
-        ok = WAIT(R_T, ph);
-        if (!ok) break;
-        tc_fence_after();
-        if (elect_one()) {
-          umma_group<4, 2, 0, 2, 0, false>(tmem + T_D3, da_lo, a_lo, ID_KK_64);
-          umma_commit(&bars[C_D3]);
-        }
-        // The bulk group is past its first read-out (always waited for: its threads combine the
-        // partial sums of the previous item before that, and the last products of this item let
-        // the group overwrite those sums).
-        ok = WAIT(R_E4, ph);
-        if (!ok) break;
-        if (has_next) {
-          // du, q, v are dead once their products are complete and the bulk group has used q
-          ok = WAIT(C_2B, ph);
-          if (!ok) break;
-          load_b(nxt);
-          ok = WAIT(C_D3, ph);  // last product that reads A
-          if (!ok) break;
-          load_c(nxt);
-        }
-        // ---- beta dA3 is an operand now ----
+        // ---- dk += (X + X^T) K with X = beta dL, onto ds^T q ----
         ok = WAIT(R_D3, ph);
         if (!ok) break;
         tc_fence_after();
-        // dk += (beta dA3) K + (beta dA3)^T K, onto the same accumulator
         if (elect_one()) {
-          umma_group<4, 2, 0, 128, 0, true>(tmem + T_DK2, ds_lo, kmn_lo, ID_KM_128);
-          umma_group<4, 128, 0, 128, 0, true>(tmem + T_DK2, dsmn_lo, kmn_lo, ID_MM_128);
+          umma_group<4, 2, 0, 128, 0, true>(tmem + T_DK2, x_lo, kmn_lo, ID_KM_128);
           umma_commit(&bars[C_5]);
+        }
+        // h, dh, dO, v_new are dead once their products are complete and the h.dh sum is done; the other
+        // k buffer belonged to the item before, which R_END above has seen finished
+        if (has_next) {
+          ok = WAIT(C_1B, ph) && WAIT(R_HD, ph);
+          if (!ok) break;
+          load_a(nxt, (int)(ph ^ 1));
         }
         cur = nxt;
       }
@@ -465,12 +447,10 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
     }
   } else {
     // ====================== read-out warps ======================
-    // Two groups of eight warps.  The CHAIN group (warps 0-7) serves the dependent chain
-    // dw -> dA -> T -> dA3 (plus ds, which it gets for free from the same kind of tile): it reads
-    // the 64-wide accumulators in the 16-lane shape (lane l of warp (qd, half) owns rows
-    // 16 qd + l/4 (+8), column pairs 32 half + 8 i + 2 (l%4)).  The BULK group (warps 8-15) does
-    // everything that is off the chain: the h.dh sum, the scaling of dq1 | dk1 (written back to
-    // tensor memory), dv, and the final dq | dk.  It reads the 128-wide accumulators in the
+    // Two groups of eight warps.  The CHAIN group (warps 0-7) serves the dependent chain (plus ds, which
+    // it gets from the same kind of tile): it reads accumulators in the 16-lane shape (lane l of warp
+    // (qd, half) owns rows 16 qd + l/4 (+8), column pairs 8 i + 2 (l%4) of half the columns).  The BULK
+    // group (warps 8-15) does everything that is off the chain.  It reads the 128-wide accumulators in the
     // 32-lane shape, which returns the accumulator at lanes +0 and the one at lanes +16 of the
     // same columns at once: lane l owns row 16 qd + l%16 of the lower (l < 16) or upper one, 32
     // consecutive columns per pass; shared and global memory are touched 16 bytes at a time.
@@ -496,21 +476,15 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       x += __shfl_xor_sync(0xffffffffu, x, 16);
       return x;
     };
-    auto st_tile64 = [&](int off, int row, int col, float lo, float hi2) {
-      *reinterpret_cast<uint32_t*>(smem + off + sw128_offset(row, col)) = pack_bf16(lo, hi2);
-    };
     auto pack8 = [&](const float* x) {
       return make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
     };
-    // 32 consecutive columns of this thread's output row (x, fp32) go out as bf16. A thread owns a
+    // 32 consecutive columns of this thread's output row (bf16) go out. A thread owns a
     // row, so a plain 16-byte store per thread would touch 32 lines per instruction; the four
     // lanes of a quad first exchange their 16-byte pieces (a 4 x 4 transpose, two butterfly
     // steps), after which each store instruction writes 64 contiguous bytes of 8 rows.
     // base = offset of the row of lane 0 of the quad (+ the 32-column block), row_q = that row.
-    auto store_rows = [&](bf16* out, long long base, int row_q, int valid_rows, const float* x) {  // whole warp
-      uint4 pc[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) pc[j] = pack8(x + 8 * j);
+    auto store_rows = [&](bf16* out, long long base, int row_q, int valid_rows, uint4 (&pc)[4]) {  // whole warp
       const bool b0 = lane & 1, b1 = lane & 2;
       auto xchg = [&](uint4& keep_if0, uint4& keep_if1, bool bit, int mask) {
         // lanes with bit clear keep keep_if0 and send keep_if1; lanes with bit set the reverse
@@ -580,10 +554,9 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           dgv += sRowW[j * 64 + r] - sColDg[j * 64 + r];
-          dbv += sColC1[j * 64 + r];
+          dbv += sRowDb[j * 64 + r];
         }
         dgv += sRowDg[r] + sRowDg[64 + r];
-        dbv += sRowDb[r] + sRowDb[64 + r];
         if (r == n_rows - 1) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) dgv += sLast[j];
@@ -614,19 +587,18 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       const int koff = OFF_K + (int)ph * ROW_TILE;
       const float* sG = ph ? sVec1 : sVec0;
       const float *sGam = sG + 64, *sRho = sG + 128, *sBeta = sG + 192;
-      bool ok = WAIT(L_A, ph) && WAIT(L_B, ph) && WAIT(L_C, ph);
-      if (ok && valid < CHUNK) {
-        zero_rows(OFF_Q, 2, valid);
-        zero_rows(koff, 2, valid);
-        zero_rows(OFF_A, 1, valid);
-        if constexpr (TILED) {  // the transposed tiles already hold zeros past the sequence end
-          zero_rows(OFF_V, 2, valid);
-          zero_rows(OFF_DO, 2, valid);
-        } else {
-          zero_rows(OFF_V, 8, valid);  // v, v_new, dO, du
+      bool ok = true;
+      if (valid < CHUNK) {
+        ok = WAIT(L_D, ph) && WAIT(L_A, ph) && WAIT(L_H, ph) && WAIT(L_Q, ph);
+        if (ok) {
+          zero_rows(OFF_Q, 2, valid);
+          zero_rows(koff, 2, valid);
+          zero_rows(OFF_A, 1, valid);
+          if constexpr (TILED) zero_rows(OFF_DO, 2, valid);  // the transposed tiles already hold zeros
+          else zero_rows(OFF_VN, 6, valid);                  // v_new, dO, du
         }
+        signal(R_ZERO);
       }
-      signal(R_ZERO);
       Item nxt;
       // the next item, from the middle of this one on
       auto take_next = [&] {
@@ -637,42 +609,72 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 
       if (chain) {
         // ===================== chain group =====================
-        const float g_a = sG[row_a], g_b = sG[row_b];
         const float beta_a = sBeta[row_a], beta_b = sBeta[row_b];
-        // row sums (dg, db) and column sums (dg; the two column terms that come from A^T dw and
-        // A^T du) of this thread; reduced across lanes once, at the end of the item
+        // row sums (dg, db) and column sums (dg) of this thread; reduced across lanes once, at the end
+        // of the item
         float acc_dg_a = 0.f, acc_dg_b = 0.f, acc_db_a = 0.f, acc_db_b = 0.f;
-        float acc_col[8], acc_dbc[8];  // per column: dg terms (to subtract), db terms
+        float acc_col[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc_col[j] = acc_dbc[j] = 0.f;
+        for (int j = 0; j < 8; ++j) acc_col[j] = 0.f;
 
-        // ---- E1: dw = -du h^T as an operand tile (lower lanes of the 32-lane shape) ----
-        ok = ok && WAIT(C_DW, ph);
+        // ---- E1: dW = A^T du as an operand tile; dv = beta dW, made of v in place; db += dW v ----
+        // the products that read the operand tile of the item before are complete (C_1B)
+        ok = ok && WAIT(C_DW, ph) && (it == 0 || WAIT(C_1B, ph ^ 1)) && WAIT(L_D, ph);
         if (ok) {
           tc_fence_after();
-#pragma unroll 1
-          for (int pass = 0; pass < 2; ++pass) {
-            float x[32];
-            tmem_ld32(tmem + lanes + T_DW + c128 + 32 * pass, x);
-            tmem_ld_wait();
-            if (!hi) {
+          float x[32];
+          tmem_ld_16x64(tmem + lanes + T_DW + 64 * half, x);
+          tmem_ld_wait();
+          // 16-byte pieces 2 j, 2 j + 1 of rows 0-7 and 8-15 of this warp's [16 x 64] block: one
+          // stmatrix / ldmatrix with the addresses of lane's row
+          const uint32_t line = (uint32_t)(half * 8192 + (16 * qd + 8 * ((lane >> 3) & 1) + (lane & 7)) * 128);
+          auto at = [&](int j) { return line + (uint32_t)(((2 * j + (lane >> 4)) ^ (lane & 7)) << 4); };
 #pragma unroll
-              for (int j = 0; j < 32; ++j) x[j] = -x[j];
+          for (int j = 0; j < 4; ++j)
+            stmatrix_x4(s32(smem + OFF_DW) + at(j), pack_bf16(x[8 * j], x[8 * j + 1]), pack_bf16(x[8 * j + 2], x[8 * j + 3]),
+                        pack_bf16(x[8 * j + 4], x[8 * j + 5]), pack_bf16(x[8 * j + 6], x[8 * j + 7]));
+          signal(R_DW);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(smem + OFF_DW + piece(pass, j)) = pack8(x + 8 * j);
+          for (int j = 0; j < 4; ++j) {
+            uint32_t vr[4];
+            ldmatrix_x4_addr(vr, s32(smem + OFF_V) + at(j));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 t = __bfloat1622float2(*reinterpret_cast<const bf162*>(&vr[e]));
+              const float x0 = x[8 * j + 2 * e], x1 = x[8 * j + 2 * e + 1];
+              if (e & 1) acc_db_b += x0 * t.x + x1 * t.y;
+              else acc_db_a += x0 * t.x + x1 * t.y;
+              const float b = e & 1 ? beta_b : beta_a;
+              vr[e] = pack_bf16(b * x0, b * x1);
             }
+            stmatrix_x4(s32(smem + OFF_V) + at(j), vr[0], vr[1], vr[2], vr[3]);
           }
+          __syncwarp();
+          // out again as whole lines: eight threads write 128 contiguous bytes of a row
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int row = 16 * qd + 4 * j + (lane >> 3);
+            const uint4 w = *reinterpret_cast<const uint4*>(smem + OFF_V + half * 8192 + row * 128 +
+                                                            (((lane & 7) ^ (row & 7)) << 4));
+            if (row < valid)
+              *reinterpret_cast<uint4*>(p.dv + ((cur.row0 + row) * p.Hv + cur.hv) * D + 64 * half + 8 * (lane & 7)) = w;
+          }
+        } else {
+          signal(R_DW);
         }
-        signal(R_DW);
 
         // ---- E2: ds = scale * G * (dO Vn^T); ds2 = ds * (Q K^T) ----
-        ok = ok && WAIT(C_DSQK, ph);
+        ok = ok && WAIT(C_DSQK, ph) && (it == 0 || WAIT(C_2, ph ^ 1));
+        const float g_a = sG[row_a], g_b = sG[row_b];
+        // address of this lane's row in a [16 x 32] block of a 64-column tile, 16-byte piece 4 half + i
+        const uint32_t line = (uint32_t)((16 * qd + 8 * ((lane >> 3) & 1) + (lane & 7)) * 128);
         if (ok) {
           tc_fence_after();
           float ds[16], qk[16];
           tmem_ld_16x32(tmem + lanes + T_DS + c64, ds);
           tmem_ld_16x32(tmem + lanes + T_QK + c64, qk);
           tmem_ld_wait();
+          uint32_t w[8];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int col = c64 + 8 * i + cp;
@@ -681,90 +683,43 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
             const float a1 = col + 1 <= row_a ? p.scale * ds[4 * i + 1] * fast_exp(g_a - gc1) : 0.f;
             const float b0 = col <= row_b ? p.scale * ds[4 * i + 2] * fast_exp(g_b - gc0) : 0.f;
             const float b1 = col + 1 <= row_b ? p.scale * ds[4 * i + 3] * fast_exp(g_b - gc1) : 0.f;
-            st_tile64(OFF_DS, row_a, col, a0, a1);
-            st_tile64(OFF_DS, row_b, col, b0, b1);
+            w[2 * i] = pack_bf16(a0, a1);
+            w[2 * i + 1] = pack_bf16(b0, b1);
             const float s0 = a0 * qk[4 * i], s1 = a1 * qk[4 * i + 1], s2 = b0 * qk[4 * i + 2], s3 = b1 * qk[4 * i + 3];
             acc_dg_a += s0 + s1;
             acc_dg_b += s2 + s3;
             acc_col[2 * i] += s0 + s2;
             acc_col[2 * i + 1] += s1 + s3;
           }
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            stmatrix_x4(s32(smem + OFF_DS) + line + (uint32_t)(((4 * half + 2 * i + (lane >> 4)) ^ (lane & 7)) << 4),
+                        w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
         }
         signal(R_DS);
 
-        // ---- E3: dA = strict_lower(beta_c (gamma_c x1 + x2)); A' = A diag(beta), A'' = A diag(beta gamma) ----
-        ok = ok && WAIT(C_X, ph);
-        if (ok) {
-          tc_fence_after();
-          float x1[16], x2[16];
-          tmem_ld_16x32(tmem + lanes + T_X1 + c64, x1);
-          tmem_ld_16x32(tmem + lanes + T_X2 + c64, x2);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int col = c64 + 8 * i + cp;
-            const float b0 = sBeta[col], b1 = sBeta[col + 1], g0 = sGam[col], g1 = sGam[col + 1];
-            st_tile64(OFF_DA, row_a, col, col < row_a ? b0 * (g0 * x1[4 * i] + x2[4 * i]) : 0.f,
-                      col + 1 < row_a ? b1 * (g1 * x1[4 * i + 1] + x2[4 * i + 1]) : 0.f);
-            st_tile64(OFF_DA, row_b, col, col < row_b ? b0 * (g0 * x1[4 * i + 2] + x2[4 * i + 2]) : 0.f,
-                      col + 1 < row_b ? b1 * (g1 * x1[4 * i + 3] + x2[4 * i + 3]) : 0.f);
-            // rowsum((A^T dw) k)[r] = sum_s A[s][r] x1[s][r], rowsum((A^T du) v)[r] = sum_s A[s][r] x2[s][r]
-            const float2 A_a = ld_bf16x2(reinterpret_cast<const bf16*>(smem + OFF_A + sw128_offset(row_a, col)));
-            const float2 A_b = ld_bf16x2(reinterpret_cast<const bf16*>(smem + OFF_A + sw128_offset(row_b, col)));
-            // column r: db += gamma_r c1 + c2, dg += beta_r gamma_r c1 (entered with a minus sign
-            // into the column sums, which the final step subtracts)
-            const float c1a = A_a.x * x1[4 * i] + A_b.x * x1[4 * i + 2];
-            const float c1b = A_a.y * x1[4 * i + 1] + A_b.y * x1[4 * i + 3];
-            acc_dbc[2 * i] += g0 * c1a + A_a.x * x2[4 * i] + A_b.x * x2[4 * i + 2];
-            acc_dbc[2 * i + 1] += g1 * c1b + A_a.y * x2[4 * i + 1] + A_b.y * x2[4 * i + 3];
-            acc_col[2 * i] -= b0 * g0 * c1a;
-            acc_col[2 * i + 1] -= b1 * g1 * c1b;
-            // the v tile is dead (its product is part of this group): A' and A'' go there
-            st_tile64(OFF_V, row_a, col, A_a.x * b0, A_a.y * b1);
-            st_tile64(OFF_V, row_b, col, A_b.x * b0, A_b.y * b1);
-            st_tile64(OFF_V + 8192, row_a, col, A_a.x * b0 * g0, A_a.y * b1 * g1);
-            st_tile64(OFF_V + 8192, row_b, col, A_b.x * b0 * g0, A_b.y * b1 * g1);
-          }
-        }
-        signal(R_DA);
-        take_next();
-        if (ok && nxt.valid > 0) fetch_vectors(nxt);
-
-        // ---- E5: T = A^T dA as an operand tile (over dA, which the product has consumed) ----
-        ok = ok && WAIT(C_T, ph);
-        if (ok) {
-          tc_fence_after();
-          float t[16];
-          tmem_ld_16x32(tmem + lanes + T_T + c64, t);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int col = c64 + 8 * i + cp;
-            st_tile64(OFF_DA, row_a, col, t[4 * i], t[4 * i + 1]);
-            st_tile64(OFF_DA, row_b, col, t[4 * i + 2], t[4 * i + 3]);
-          }
-        }
-        signal(R_T);
-
-        // ---- E7: beta dA3 = -beta G d3 (over ds) as an operand tile; its dg and db terms ----
-        ok = ok && WAIT(C_D3, ph);
+        // ---- E7: X = beta dL, dL = -G D3 below the diagonal, D3 = dW v_new^T; X + X^T as an operand
+        //      tile; the dg and db terms of dL * (K K^T) ----
+        ok = ok && WAIT(C_D3, ph) && (it == 0 || WAIT(C_5, ph ^ 1));
         if (ok) {
           tc_fence_after();
           float d3[16], kk[16];
           tmem_ld_16x32(tmem + lanes + T_D3 + c64, d3);
           tmem_ld_16x32(tmem + lanes + T_KK + c64, kk);
           tmem_ld_wait();
+          const uint32_t tile = s32(smem + OFF_X);
+          const int r8 = lane & 7, second = (lane >> 3) & 1;  // which of two matrices this lane addresses
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
+            const int cb = 4 * half + i;  // 8-column block; this warp's 8-row blocks are 2 qd, 2 qd + 1
+            if (cb > 2 * qd + 1) continue;  // above the diagonal: written by the warp of the mirrored block
             const int col = c64 + 8 * i + cp;
             const float gc0 = sG[col], gc1 = sG[col + 1];
             const float a0 = col < row_a ? -d3[4 * i] * fast_exp(g_a - gc0) : 0.f;
             const float a1 = col + 1 < row_a ? -d3[4 * i + 1] * fast_exp(g_a - gc1) : 0.f;
             const float b0 = col < row_b ? -d3[4 * i + 2] * fast_exp(g_b - gc0) : 0.f;
             const float b1 = col + 1 < row_b ? -d3[4 * i + 3] * fast_exp(g_b - gc1) : 0.f;
-            st_tile64(OFF_DS, row_a, col, beta_a * a0, beta_a * a1);
-            st_tile64(OFF_DS, row_b, col, beta_b * b0, beta_b * b1);
-            // db += rowsum((dA3 K) k) = rowsum(dA3 * (K K^T)); the dg terms carry the beta factor
+            // db += rowsum((dL K) k) = rowsum(dL * (K K^T)); the dg terms carry the beta factor
             const float u0 = a0 * kk[4 * i], u1 = a1 * kk[4 * i + 1], u2 = b0 * kk[4 * i + 2], u3 = b1 * kk[4 * i + 3];
             acc_db_a += u0 + u1;
             acc_db_b += u2 + u3;
@@ -773,10 +728,25 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
             acc_dg_b += s2 + s3;
             acc_col[2 * i] += s0 + s2;
             acc_col[2 * i + 1] += s1 + s3;
+            // blocks (2 qd, cb) and (2 qd + 1, cb), and mirrored (cb, 2 qd) and (cb, 2 qd + 1)
+            uint32_t wa = pack_bf16(col < row_a ? beta_a * a0 : 0.f, col + 1 < row_a ? beta_a * a1 : 0.f);
+            uint32_t wb = pack_bf16(col < row_b ? beta_b * b0 : 0.f, col + 1 < row_b ? beta_b * b1 : 0.f);
+            const uint32_t straight = tile + (uint32_t)((16 * qd + 8 * second + r8) * 128 + ((cb ^ r8) << 4));
+            const uint32_t mirrored = tile + (uint32_t)((8 * cb + r8) * 128 + (((2 * qd + second) ^ r8) << 4));
+            if (cb < 2 * qd) {
+              stmatrix_x2(straight, wa, wb);
+              stmatrix_x2_trans(mirrored, wa, wb);
+            } else if (cb == 2 * qd) {  // the upper one of the two lies on the diagonal
+              stmatrix_x2(straight, wa | movmatrix_trans(wa), wb);
+              stmatrix_x1_trans(tile + (uint32_t)((8 * cb + r8) * 128 + (((2 * qd + 1) ^ r8) << 4)), wb);
+            } else {  // the upper one lies above the diagonal, the lower one on it
+              stmatrix_x1(tile + (uint32_t)((16 * qd + 8 + r8) * 128 + ((cb ^ r8) << 4)), wb | movmatrix_trans(wb));
+            }
           }
         }
         signal(R_D3);
-        signal(R_END);  // this group no longer touches the accumulators or the tiles of the item
+        take_next();
+        if (ok && nxt.valid > 0) fetch_vectors(nxt);
         // The partial-sum slots were read for the previous item by threads of the bulk group, which
         // arrive on R_E4 of this item only after that.
         ok = ok && WAIT(R_E4, ph);
@@ -794,16 +764,12 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float c = col_sum(acc_col[j]);
-          const float c1 = col_sum(acc_dbc[j]);
-          if (lane < 4) {
-            const int col = c64 + 8 * (j >> 1) + cp + (j & 1);
-            sColDg[qd * 64 + col] = c;
-            sColC1[qd * 64 + col] = c1;
-          }
+          if (lane < 4) sColDg[qd * 64 + c64 + 8 * (j >> 1) + cp + (j & 1)] = c;
         }
       } else {
         // ===================== bulk group =====================
         // gamma_last * sum(h * dh) over the whole 128 x 128 tiles (plain shared-memory reads)
+        ok = ok && WAIT(L_A, ph) && WAIT(L_H, ph);
         if (ok) {
           float hd = 0.f;
           for (int i = tid - N_EPI / 2; i < SQ_TILE / 16; i += N_EPI / 2) {
@@ -828,9 +794,9 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         const long long out_q = ((cur.row0 + row_q) * p.Hv + cur.hv) * D + c128;
         float acc_w = 0.f;
 
-        // ---- E4: dq1 = scale gamma (dO h^T) on the lower lanes, dk1 = rho (Vn dh^T) on the upper;
-        //      scaled in place (written back to tensor memory), with their dg terms ----
-        ok = ok && WAIT(C_1B, ph);
+        // ---- E4: the dg terms of dq1 = scale gamma (dO h^T) on the lower lanes, dk1 = rho (Vn dh^T) on
+        //      the upper ----
+        ok = ok && WAIT(C_1B, ph) && WAIT(L_Q, ph);
         if (ok) {
           tc_fence_after();
           const unsigned char* tile = smem + (hi ? koff : OFF_Q);
@@ -847,48 +813,57 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 const float2 t = __bfloat1622float2(*reinterpret_cast<const bf162*>(&pr[e]));
-                x[8 * j + 2 * e] *= f_w;
-                x[8 * j + 2 * e + 1] *= f_w;
                 s += t.x * x[8 * j + 2 * e] + t.y * x[8 * j + 2 * e + 1];
               }
             }
-            tmem_st32(tmem + lanes + T_DQ1 + c128 + 32 * pass, x);
             // dg += rowsum(q dq1) - rowsum(k dk1); the chunk total gets + sum(k dk1)
+            s *= f_w;
             acc_w += hi ? -s : s;
             if (hi) acc_last += s;
           }
-          tmem_st_wait();
         }
-        signal(R_E4);  // q (and this item's k for this group) are no longer read from shared memory
+        signal(R_E4);  // q is no longer read from shared memory
+        take_next();   // (before R_END: the item after the next is published only behind that)
 
-        // ---- E6: dv = A'^T du (upper lanes), already row-scaled by beta ----
-        ok = ok && WAIT(C_2B, ph);
-        if (ok) {
-          tc_fence_after();
-#pragma unroll 1
-          for (int pass = 0; pass < 2; ++pass) {
-            float x[32];
-            tmem_ld32(tmem + lanes + (T_T2 & 0xFFFFu) + c128 + 32 * pass, x);
-            tmem_ld_wait();
-            store_rows(p.dv, out_q + 32 * pass, row_q, hi ? valid : 0, x);  // dv sits on the upper lanes
-          }
-        }
-
-        // ---- E8: dq = dq1 + ds K (lower lanes); dk = dk1 + [ds^T q + A''^T dw + (beta dA3) K + (beta dA3)^T K] ----
+        // ---- E8: dq = dq1 + ds K (lower lanes); dk = dk1 - beta gamma Y + [ds^T q + (X + X^T) K] (upper
+        //      lanes), and the dg and db terms of Y = dW h^T ----
         ok = ok && WAIT(C_5, ph);
         if (ok) {
           tc_fence_after();
           bf16* out = hi ? p.dk : p.dq;
+          const float f_y = hi ? -sBeta[row_w] * sGam[row_w] : 0.f;
+          float s = 0.f;
 #pragma unroll 1
           for (int pass = 0; pass < 2; ++pass) {
-            float x[32], y[32];
-            tmem_ld32(tmem + lanes + T_DQ1 + c128 + 32 * pass, x);
-            tmem_ld32(tmem + lanes + T_DQ2 + c128 + 32 * pass, y);
-            tmem_ld_wait();
+            uint4 pc[4];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] += y[j];
-            store_rows(out, out_q + 32 * pass, row_q, valid, x);
+            for (int z = 0; z < 2; ++z) {
+              float x[16], y[16], w[16];
+              const uint32_t col = c128 + 32 * pass + 16 * z;
+              tmem_ld16(tmem + lanes + T_DQ1 + col, x);
+              tmem_ld16(tmem + lanes + T_DQ2 + col, y);
+              tmem_ld16(tmem + lanes + T_DW + col, w);  // upper lanes: Y; lower lanes: dW, not used
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                const uint4 raw = *reinterpret_cast<const uint4*>(smem + koff + piece(pass, 2 * z + j));
+                const uint32_t* pr = &raw.x;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float2 t = __bfloat1622float2(*reinterpret_cast<const bf162*>(&pr[e]));
+                  const int c = 8 * j + 2 * e;
+                  const float w0 = hi ? w[c] : 0.f, w1 = hi ? w[c + 1] : 0.f;
+                  s += t.x * w0 + t.y * w1;
+                  x[c] = f_w * x[c] + y[c] + f_y * w0;
+                  x[c + 1] = f_w * x[c + 1] + y[c + 1] + f_y * w1;
+                }
+                pc[2 * z + j] = pack8(x + 8 * j);
+              }
+            }
+            store_rows(out, out_q + 32 * pass, row_q, valid, pc);
           }
+          acc_w += f_y * s;
+          if (hi) sRowDb[128 + half * 64 + row_w] = -sGam[row_w] * s;
         }
         signal(R_END);  // accumulators and k of this item are free
         sRowW[(2 * half + (hi ? 1 : 0)) * 64 + row_w] = acc_w;
@@ -905,7 +880,6 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       if (chain) {
         if (nxt.valid > 0) write_vectors(nxt, ph ? sVec0 : sVec1);
       } else {
-        take_next();
         ok = ok && WAIT(R_CH, ph);
       }
       if (!ok) *abort_flag = 1;

@@ -102,6 +102,33 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t saddr, uint32_t r0, u
                : "memory");
 }
 
+// One, two or four 8 x 8 matrices as they are, or one or two transposed; lane 8 i + r gives the address of
+// row r of matrix i.
+__device__ __forceinline__ void stmatrix_x4(uint32_t saddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(r0), "r"(r1),
+               "r"(r2), "r"(r3)
+               : "memory");
+}
+__device__ __forceinline__ void stmatrix_x2(uint32_t saddr, uint32_t r0, uint32_t r1) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x2.shared.b16 [%0], {%1, %2};" ::"r"(saddr), "r"(r0), "r"(r1) : "memory");
+}
+__device__ __forceinline__ void stmatrix_x1(uint32_t saddr, uint32_t r0) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x1.shared.b16 [%0], {%1};" ::"r"(saddr), "r"(r0) : "memory");
+}
+__device__ __forceinline__ void stmatrix_x2_trans(uint32_t saddr, uint32_t r0, uint32_t r1) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x2.trans.shared.b16 [%0], {%1, %2};" ::"r"(saddr), "r"(r0), "r"(r1)
+               : "memory");
+}
+__device__ __forceinline__ void stmatrix_x1_trans(uint32_t saddr, uint32_t r0) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x1.trans.shared.b16 [%0], {%1};" ::"r"(saddr), "r"(r0) : "memory");
+}
+// an 8 x 8 matrix in fragment form, transposed across the warp
+__device__ __forceinline__ uint32_t movmatrix_trans(uint32_t r) {
+  uint32_t t;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(t) : "r"(r));
+  return t;
+}
+
 // ---- issuing warps -----------------------------------------------------------------------------
 // A warp that issues tcgen05 and TMA instructions stays CONVERGED: all its lanes run the loop and
 // the waits, and only the instructions themselves sit behind elect_one().  The compiler then keeps
