@@ -93,7 +93,8 @@ Tables add_tables(std::vector<int>& out, const std::vector<int64_t>& bounds) {
 }
 
 std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int64_t T, int64_t Hv,
-                             int device, bool plan, bool cap, const std::vector<int64_t>& read) {
+                             int device, bool plan, bool leads, bool cap,
+                             const std::vector<int64_t>& read) {
   // reading cu_seqlens and writing tables are host round trips
   auto needs_round_trip = [&] {
     if (cap)
@@ -104,6 +105,7 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
   b->T = T;
   b->Hv = Hv;
   b->device = device;
+  b->leads = leads;
   std::vector<int64_t> bounds;
   std::vector<int> host;
   Tables raw{};
@@ -126,7 +128,13 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
     for (int64_t i = 0; i <= B; ++i) bounds.push_back(i * T);
   }
   const int n_sm = at::cuda::getDeviceProperties(device)->multiProcessorCount;
-  const auto split = plan ? split_sequences(bounds, Hv, n_sm) : std::nullopt;
+  // a fixed shape met for the first time during a capture can be given no tables: it runs unsplit where the
+  // coarser rule leaves it so (and is planned again by the first call that can)
+  b->provisional = cap && !packed && leads && plan;
+  if (b->provisional) leads = false;
+  const auto split = !plan ? std::nullopt
+                     : leads ? split_sequences(bounds, Hv, n_sm, LEAD_MIN_SEGMENT_CHUNKS, 1, LEAD_SPLIT_CHUNKS)
+                             : split_sequences(bounds, Hv, n_sm);
   Tables seg{};
   size_t begin = 0, first = 0, last = 0, kf = 0, kb = 0;
   if (split) {
@@ -190,7 +198,7 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
 }  // namespace
 
 std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B, int64_t T,
-                                 int64_t Hv, int device, bool auto_cp) {
+                                 int64_t Hv, int device, bool auto_cp, bool leads) {
   if (cu) {
     if (cu->scalar_type() != at::kInt && cu->scalar_type() != at::kLong)
       throw PyError(PyError::Type, "cu_seqlens must be int32 or int64");
@@ -198,7 +206,7 @@ std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B,
   }
   const uint32_t version = cu && !cu->is_inference() ? cu->_version() : 0;
   const bool cap = capturing();
-  if (!cu && !auto_cp) return build(cu, B, T, Hv, device, false, cap, {});  // nothing to look up
+  if (!cu && !auto_cp) return build(cu, B, T, Hv, device, false, leads, cap, {});  // nothing to look up
   std::vector<int64_t> read;
   if (cu && cu->is_inference() && !cap) read = read_bounds(*cu);
   std::lock_guard<std::mutex> hold(entries_lock);
@@ -206,7 +214,7 @@ std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B,
   for (auto it = entries.end(); it != entries.begin();) {  // most recent first
     Batch& e = **--it;
     if (e.B != B || e.T != T || e.device != device) continue;
-    if (e.Hv != Hv && auto_cp) continue;  // only the plan depends on the heads
+    if ((e.Hv != Hv || e.leads != leads) && auto_cp) continue;  // only the plan depends on these
     if (cu && !(e.cu.unsafeGetTensorImpl() == cu->unsafeGetTensorImpl() && e.version == version)) continue;
     if (!read.empty() && e.bounds != read) continue;
     if (e.stream) {
@@ -219,7 +227,8 @@ std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B,
     entries.splice(entries.end(), entries, it);
     return entries.back();
   }
-  auto b = build(cu, B, T, Hv, device, true, cap, read);
+  auto b = build(cu, B, T, Hv, device, true, leads, cap, read);
+  if (b->provisional) return b;
   size_t unpinned = 0;
   for (auto& e : entries) unpinned += !e->pinned;
   if (unpinned >= most)

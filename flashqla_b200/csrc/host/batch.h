@@ -16,7 +16,9 @@ struct Batch {
   uint32_t version = 0;   // its version counter when the tables were read
   std::vector<int64_t> bounds;  // its values (inference tensors, which have no version counter)
   int64_t B = 0, T = 0, Hv = 0;
+  bool leads = false;     // planned for kernels whose segments can start early
   int device = 0;
+  bool provisional = false;  // planned by the coarser rule during a capture: not kept
   bool pinned = false;    // its device tables were looked up during a stream capture: never evicted
 
   at::Tensor store;       // all device tables, int32, allocated on `stream`
@@ -33,14 +35,16 @@ struct Batch {
   const int *raw_first = nullptr, *raw_last = nullptr;
 };
 
-// Tables for a batch of `Hv` value heads (with auto_cp off its plan is not to be used).  One host round
+// Tables for a batch of `Hv` value heads (with auto_cp off its plan is not to be used), planned for kernels
+// whose segments start a few chunks early (`leads`) or always need a state handed to them.  One host round
 // trip (reads cu_seqlens, writes the tables) the first time a cu_seqlens tensor (identity and version
 // counter) or a fixed shape is seen, none after that while the entry is kept.  A fixed shape that is not
 // split, or one without auto_cp, has no tables and needs no round trip: it may be met for the first time
-// during a stream capture, where everything else that is not kept is an error.  A cu_seqlens made in
+// during a stream capture, where everything else that is not kept is an error (a shape that only the finer
+// plan of `leads` would split runs unsplit in such a capture).  A cu_seqlens made in
 // inference mode has no version counter: it is read again at every call, and its tables are rebuilt where
 // it has changed (a capture, which cannot read it, takes the tables of the call before).
 std::shared_ptr<Batch> batch_for(const std::optional<at::Tensor>& cu, int64_t B, int64_t T,
-                                 int64_t Hv, int device, bool auto_cp);
+                                 int64_t Hv, int device, bool auto_cp, bool leads);
 
 }  // namespace fqla_host

@@ -82,8 +82,13 @@ struct Call {
   int kT() const { return split ? B * T : T; }
 };
 
+bool tiles_ok(int D) {
+  static const bool forced = std::getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
+  return D == 128 && !forced;
+}
+
 Call make_call(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, double scale,
-               const OptTensor& cu, bool auto_cp) {
+               const OptTensor& cu, const Options& opt) {
   Call c;
   c.dev = k.device();
   c.stream = (void*)at::cuda::getCurrentCUDAStream(c.dev.index()).stream();
@@ -93,8 +98,8 @@ Call make_call(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, do
   c.D = (int)k.size(3);
   c.Hv = (int)v.size(2);
   c.scale = (float)scale;
-  c.batch = batch_for(cu, c.B, c.T, c.Hv, c.dev.index(), auto_cp);
-  c.split = auto_cp && c.batch->n_seg > 0;
+  c.batch = batch_for(cu, c.B, c.T, c.Hv, c.dev.index(), opt.auto_cp, opt.lead_in && tiles_ok(c.D));
+  c.split = opt.auto_cp && c.batch->n_seg > 0;
   return c;
 }
 
@@ -110,11 +115,6 @@ void check_state(const OptTensor& s, const Call& c) {
 void check_segments(const at::Tensor& t, const Call& c, const char* what) {
   if (t.dim() < 2 || t.size(0) != c.batch->n_seg || t.size(1) != c.Hv)
     throw PyError(PyError::Value, std::string("cp_cache: its ") + what + " belong to another batch");
-}
-
-bool tiles_ok(int D) {
-  static const bool forced = std::getenv("FQLA_FORCE_MMA_SYNC") != nullptr;
-  return D == 128 && !forced;
 }
 
 struct SeqIn {  // inputs of the sequential kernels
@@ -294,7 +294,7 @@ Forward forward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor
   c10::cuda::CUDAGuard guard(k_in.device());
   c10::AutoGradMode no_grad(false);
   Forward r;
-  const Call c = make_call(q_in, k_in, v_in, scale, cu, opt.auto_cp);
+  const Call c = make_call(q_in, k_in, v_in, scale, cu, opt);
   prepare(q_in, k_in, v_in, opt, r);
   const at::Tensor &q = r.q, &k = r.k, &v = r.v;
   const at::Tensor g = as_f32(g_in), beta = beta_in(beta_in_);
@@ -361,7 +361,7 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
   const at::Tensor q = as_bf16(q_in), k = as_bf16(k_in), v = as_bf16(v_in);
   const at::Tensor dO = as_bf16(dO_in), A = as_bf16(A_in);
   const at::Tensor g = as_f32(g_in), beta = beta_in(beta_in_);
-  const Call c = make_call(q, k, v, scale, cu, opt.auto_cp);
+  const Call c = make_call(q, k, v, scale, cu, opt);
   const OptTensor h0 = state_in(initial_state);
   const OptTensor dht = state_in(dht_in);
   check_state(h0, c);

@@ -222,20 +222,20 @@ PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// split_sequences(bounds, heads, n_sm, min_chunks, slices) -> None or (seg_bounds, seg_begin)
+// split_sequences(bounds, heads, n_sm, min_chunks, slices[, split_cost]) -> None or (seg_bounds, seg_begin)
 PyObject* py_split(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    if (n != 5) throw PyError(PyError::Type, "split_sequences takes 5 arguments");
+    if (n != 5 && n != 6) throw PyError(PyError::Type, "split_sequences takes 5 or 6 arguments");
     PyObject* seq = PySequence_Fast(a[0], "bounds must be a sequence of ints");
     if (!seq) return nullptr;
     std::vector<int64_t> bounds;
     for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq); ++i)
       bounds.push_back(PyLong_AsLongLong(PySequence_Fast_GET_ITEM(seq, i)));
     Py_DECREF(seq);
-    long long x[4];
-    for (int i = 0; i < 4; ++i) x[i] = PyLong_AsLongLong(a[1 + i]);
+    long long x[5] = {};
+    for (int i = 0; i + 1 < n; ++i) x[i] = PyLong_AsLongLong(a[1 + i]);
     if (PyErr_Occurred()) return nullptr;
-    const auto s = split_sequences(bounds, x[0], x[1], x[2], x[3]);
+    const auto s = split_sequences(bounds, x[0], x[1], x[2], x[3], x[4]);
     if (!s) Py_RETURN_NONE;
     auto list = [](const std::vector<int64_t>& v) {
       PyObject* l = PyList_New((Py_ssize_t)v.size());

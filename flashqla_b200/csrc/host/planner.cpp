@@ -30,7 +30,7 @@ int64_t makespan(std::vector<int64_t> costs, int64_t copies, int64_t machines, i
 }
 
 std::optional<Split> split_sequences(const std::vector<int64_t>& bounds, int64_t heads, int64_t n_sm,
-                                     int64_t min_chunks, int64_t slices) {
+                                     int64_t min_chunks, int64_t slices, int64_t split_cost) {
   const size_t n = bounds.empty() ? 0 : bounds.size() - 1;
   std::vector<int64_t> chunks(n);
   int64_t longest = 0;
@@ -69,7 +69,7 @@ std::optional<Split> split_sequences(const std::vector<int64_t>& bounds, int64_t
     cands.emplace_back(limit, cost);
     cheapest = std::min(cheapest, cost);
   }
-  if (cands.empty() || (double)cheapest > 0.97 * (double)unsplit) return std::nullopt;
+  if (cands.empty() || (double)(cheapest + split_cost) > 0.97 * (double)unsplit) return std::nullopt;
   int64_t limit = 0;
   for (auto& c : cands)
     if ((double)c.second <= 1.03 * (double)cheapest) {
