@@ -28,7 +28,8 @@
 //
 // Warp roles (thread ranges):
 //     128-255 S group : fp32 master state in tensor memory; per chunk packs the bf16 operand copy
-//                       of S^T into tensor memory (on the chain), then decays S^T in place
+//                       of S^T into tensor memory (on the chain), then decays S^T in place and
+//                       scales A of the next chunk (A', A'')
 //     256-383 V group : Vn^T -> rho-scaled and plain bf16 operand copies (tensor memory);
 //                       w^T -> bf16 operand tile (shared memory)
 //     384-511 O group : P -> Pg (operand); output epilogue o = s gamma O1 + O2
@@ -353,7 +354,45 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   if (warp >= 4 && warp < 8) {
     // =============================== S group ===============================
     const int v = tid - 128;  // lane of tensor memory = value index
-    for (int it = 0; it < n_it && ok; ++it) {
+    // Off the chain: A' = A diag(beta), A'' = A diag(beta gamma) of iteration j, the scaled tiles the issuing
+    // thread needs for u^T, w^T.  Thread t owns the 8 columns 8 (t%8) .. of the rows t/8 + 16 i: its 16
+    // scale factors stay in registers, and the eight threads of a row touch the eight 16-byte pieces of that
+    // row (one 128-byte line per access, conflict-free).  Here and not in the output group, whose epilogue
+    // (1780 cycles), Pg (780) and this (1060) were the 4350 cycles of a chunk, while this group waits 2600 of
+    // them: 4 x 8192 tokens x 16 heads 160 -> 152 us, 262144 x 8 532 -> 511.
+    auto scale_a = [&](int j) {
+      const int sj = j & 1, c8 = v & 7, r0 = v >> 3;
+      const int pc = c8 ^ (r0 & 7);  // physical piece: rows r0 + 16 i all have (row & 7) == r0 & 7
+      if (!WAIT(FULLA0 + sj, (j >> 1) & 1)) return false;
+      if (j > 0 && !WAIT(W_DONE, (j - 1) & 1)) return false;  // u, w of the chunk before are done
+      const float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
+      const float4 b0 = *reinterpret_cast<const float4*>(vs + V_BETA * CHUNK + 8 * c8);
+      const float4 b1 = *reinterpret_cast<const float4*>(vs + V_BETA * CHUNK + 8 * c8 + 4);
+      const float4 g0 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8);
+      const float4 g1 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8 + 4);
+      const unsigned char* src = smem + OFF_STAGE + sj * STAGE_BYTES + 2 * TILE_QK + TILE_V;
+      uint4 a[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        a[i] = *reinterpret_cast<const uint4*>(src + (r0 + 16 * i) * 128 + pc * 16);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int off = (r0 + 16 * i) * 128 + pc * 16;
+        *reinterpret_cast<uint4*>(smem + OFF_AP + off) =
+            make_uint4(scale_bf16x2(a[i].x, b0.x, b0.y), scale_bf16x2(a[i].y, b0.z, b0.w),
+                       scale_bf16x2(a[i].z, b1.x, b1.y), scale_bf16x2(a[i].w, b1.z, b1.w));
+        *reinterpret_cast<uint4*>(smem + OFF_APP + off) =
+            make_uint4(scale_bf16x2(a[i].x, g0.x, g0.y), scale_bf16x2(a[i].y, g0.z, g0.w),
+                       scale_bf16x2(a[i].z, g1.x, g1.y), scale_bf16x2(a[i].w, g1.z, g1.w));
+      }
+      fence_proxy_async();
+      mbar_arrive(&bars[AP_READY]);
+      mbar_arrive(&bars[EMPTYA0 + sj]);  // the A tile of this stage is no longer read here
+      return true;
+    };
+#pragma unroll 1
+    for (int it = STATE ? 0 : -1; it < n_it && ok; ++it) {  // it = -1: only A of the first iteration
+     if (it >= 0) {
       const int s = it & 1;
       if (v == 0) FQLA_TRACE(0, 0);
       if (it > 0) ok = WAIT(S_DONE, (it - 1) & 1);
@@ -437,6 +476,11 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       tc_fence_before();
       mbar_arrive(&bars[S_DEC]);
       if (v == 0) FQLA_TRACE(0, 4);
+     }
+      if constexpr (!STATE) {
+        if (it + 1 < n_it) ok = scale_a(it + 1);
+      }
+      if (v == 0) FQLA_TRACE(0, 5);
     }
     if (ok && n_it > 0) ok = WAIT(S_DONE, (n_it - 1) & 1);
     const int ht_row = p.ht_row && !m_pass ? p.ht_row[n] : n;
@@ -611,9 +655,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     }
   } else if (warp >= 12) {
     // =============================== O group ===============================
-    // Per chunk: the epilogue of the chunk before, Pg of this chunk, and A' = A diag(beta),
-    // A'' = A diag(beta gamma) of the NEXT chunk (the scaled tiles the issuing thread needs for
-    // u^T, w^T at the end of this chunk).  The state-only variant keeps only the last part.
+    // Per chunk: the epilogue of the chunk before, then Pg of this chunk.
     // P is an M = 64 accumulator read with the 16-lane shape: lane l of warp q owns rows
     // 16q + l/4 and 16q + l/4 + 8, and in every group of 8 columns the pair 2*(l%4), +1.
     const int wq = warp & 3;
@@ -694,54 +736,21 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         }
       }
     };
-    // A', A'': thread t owns the 8 columns 8 (t%8) .. of the rows t/8 + 16 i: its 16 scale factors
-    // stay in registers, and the eight threads of a row touch the eight 16-byte pieces of that row
-    // (one 128-byte line per access, conflict-free)
-    auto scale_a = [&](int j) {
-      const int sj = j & 1, c8 = v & 7, r0 = v >> 3;
-      const int pc = c8 ^ (r0 & 7);  // physical piece: rows r0 + 16 i all have (row & 7) == r0 & 7
-      if (!WAIT(FULLA0 + sj, (j >> 1) & 1)) return false;
-      if (j > 0 && !WAIT(W_DONE, (j - 1) & 1)) return false;  // u, w of the chunk before are done
-      const float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
-      const float4 b0 = *reinterpret_cast<const float4*>(vs + V_BETA * CHUNK + 8 * c8);
-      const float4 b1 = *reinterpret_cast<const float4*>(vs + V_BETA * CHUNK + 8 * c8 + 4);
-      const float4 g0 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8);
-      const float4 g1 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8 + 4);
-      const unsigned char* src = smem + OFF_STAGE + sj * STAGE_BYTES + 2 * TILE_QK + TILE_V;
-      uint4 a[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        a[i] = *reinterpret_cast<const uint4*>(src + (r0 + 16 * i) * 128 + pc * 16);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int off = (r0 + 16 * i) * 128 + pc * 16;
-        *reinterpret_cast<uint4*>(smem + OFF_AP + off) =
-            make_uint4(scale_bf16x2(a[i].x, b0.x, b0.y), scale_bf16x2(a[i].y, b0.z, b0.w),
-                       scale_bf16x2(a[i].z, b1.x, b1.y), scale_bf16x2(a[i].w, b1.z, b1.w));
-        *reinterpret_cast<uint4*>(smem + OFF_APP + off) =
-            make_uint4(scale_bf16x2(a[i].x, g0.x, g0.y), scale_bf16x2(a[i].y, g0.z, g0.w),
-                       scale_bf16x2(a[i].z, g1.x, g1.y), scale_bf16x2(a[i].w, g1.z, g1.w));
-      }
-      fence_proxy_async();
-      mbar_arrive(&bars[AP_READY]);
-      mbar_arrive(&bars[EMPTYA0 + sj]);  // the A tile of this stage is no longer read here
-      return true;
-    };
     const float log2_scale = log2f(p.scale);
     // every part appears once (the kernel streams its code through a shared instruction cache):
-    // j = -1 only scales A of the first iteration, j = n_it only writes out the last chunk
+    // j = n_it only writes out the last chunk
 #pragma unroll 1
-    for (int j = -1; j <= n_it && ok; ++j) {
-      const int it = j - lead;  // chunk of the sequence; < 0: lead-in, no output
+    for (int j = max(lead, 0); !NO_O && j <= n_it && n_it > 0 && ok; ++j) {
+      const int it = j - lead;  // chunk of the sequence
       // the epilogue of the chunk before first: the issuing thread needs its accumulators free
       // (O_FREE) for this chunk's first output product
-      if (!NO_O && it > 0 && n_it > 0) {
+      if (it > 0) {
         ok = WAIT(O_DONE, (it - 1) & 1);
         if (!ok) break;
         tc_fence_after();
         epilogue(it - 1);
       }
-      if (!NO_O && it >= 0 && j >= 0 && j < n_it) {
+      if (j < n_it) {
         const float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
         ok = WAIT(FULL0 + (j & 1), (j >> 1) & 1) && WAIT(P_DONE, it & 1);
         if (!ok) break;
@@ -774,7 +783,6 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         fence_proxy_async();
         mbar_arrive(&bars[P_READY]);
       }
-      if (j + 1 < n_it) ok = scale_a(j + 1);
     }
     if constexpr (!NO_O) {
       if (wq == 0 && elect_one()) tma_store_wait_all();
