@@ -124,22 +124,41 @@ __device__ __forceinline__ void cp_async4(float* smem_dst, const float* gmem_src
 // The steps of a chain are serial, its value columns are independent: a CTA walks one chain for
 // BV = 8 of them, and what bounds it is the latency of a step, a D x D x 8 product in fp32 (2 x 8
 // outputs per thread, the contraction split over KS groups of threads and summed through shared
-// memory; about 1000 cycles of fused multiply-adds at D = 128).  M arrives by cp.async two steps
-// ahead in three buffers whose padded rows (LDM = D + 4) keep both the row-wise 16-byte reads
-// (forward) and the column reads (reverse) free of bank conflicts.  32 columns per CTA with M
-// staged in panels inside the step took 16 us a step: the 18-segment chains of two heads of 32768
-// tokens 293 us, now 51.
+// memory; about 1000 cycles of fused multiply-adds at D = 128).  Nothing of a step waits for global memory:
+// M and the local state arrive by cp.async two steps ahead in three buffers, the flags are read 512 steps
+// at a time.  (The flags and local states loaded into registers a step or three ahead were waited for at the
+// end of every step, where the registers move on: 18-segment chains of two heads of 32768 tokens 50 us, of
+// which 27 with neither the product nor M; now 40, of which 16.)  16-byte piece c of row r of M sits at c ^ (r & 7): both
+// the row-wise 16-byte reads (forward) and the column reads (reverse) are free of bank conflicts.  4 columns
+// per CTA instead of 8 read M twice as often from L2 (71 instead of 50 us then).
 // Few CTAs (one per SM) take the (sequence, head) pairs in turn, gridDim.y apart, and only those
 // that have a chain at all: usually none has, and a CTA then ends after a few loads.  Pairs that apply no
 // M (all of them, where the gates forget) are copies and left to merge_plain_kernel, whose blocks need
 // no SM of their own: beside a recurrence that leaves 16 SMs free, the start states of eight GPUs' shards
 // took 90 us here for 8 heads and 170 for 16, one CTA per SM in eight and nine rounds; now 37 and 55 (27 and
 // 35 with CTAs of 33 KB, whose chains with M took 254 and 311 us there against 225 and 258).
+// PER consecutive floats at once (in shared memory)
+template <int PER>
+__device__ __forceinline__ void load_floats(float (&x)[PER], const float* p) {
+  static_assert(PER == 2 || PER == 4, "one 8- or 16-byte access");
+  if constexpr (PER == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+  } else {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    x[0] = v.x; x[1] = v.y;
+  }
+}
+template <int PER>
+__device__ __forceinline__ void store_floats(float* p, const float (&x)[PER]) {
+  if constexpr (PER == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+  else *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+}
 template <int D>
 struct Merge {
-  static constexpr int BV = 8, NT = 256, KS = 2 * NT / D, KB = D / KS, LDM = D + 4;
-  static constexpr int M_FLOATS = D * LDM, PER = D * BV / NT;
-  static constexpr int SMEM_BYTES = (3 * M_FLOATS + D * BV + KS * D * BV) * 4;
+  static constexpr int BV = 8, NT = 256, KS = 2 * NT / D, KB = D / KS;
+  static constexpr int M_FLOATS = D * D, L_FLOATS = D * BV, PER = D * BV / NT;
+  static constexpr int SMEM_BYTES = (3 * M_FLOATS + 3 * L_FLOATS + D * BV + KS * D * BV) * 4;
   static constexpr int CTAS_Y = D == 128 ? 9 : 54;  // x D / BV slices: all SMs, one or three CTAs each
 };
 struct MergeParams {
@@ -168,10 +187,12 @@ __device__ __forceinline__ bool applies_m(const MergeParams& p, int pair, int fi
 template <int D>
 __global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
   using C = Merge<D>;
-  constexpr int BV = C::BV, NT = C::NT, KS = C::KS, KB = C::KB, LDM = C::LDM, PER = C::PER;
+  constexpr int BV = C::BV, NT = C::NT, KS = C::KS, KB = C::KB, PER = C::PER;
   extern __shared__ __align__(16) float sm[];
-  __shared__ unsigned active[NT / 32];
-  float* cur = sm + 3 * C::M_FLOATS;   // [D][BV] state of the step
+  constexpr int FLAGS = 512;           // steps whose flags are read at a time
+  __shared__ unsigned active[NT / 32], apply[2 * FLAGS / 32];
+  float* loc = sm + 3 * C::M_FLOATS;   // 3 x [D][BV] local states
+  float* cur = loc + 3 * C::L_FLOATS;  // [D][BV] state of the step
   float* part = cur + D * BV;          // [KS][D][BV] partial products
   pdl_wait();
   const int t = threadIdx.x;
@@ -186,53 +207,72 @@ __global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
     auto strided = [&](const float* base, int step) {
       return base + (long long)seg(step) * p.seg_stride + ((long long)hv * D) * D;
     };
-    // the last step only stores: nothing of its segment is read
-    auto flag = [&](int step) {
-      return step >= n - 1 ? 0 : p.use_m ? p.use_m[(long long)seg(step) * p.use_stride + hv] : 1;
+    // Flags of the steps from `first` on (whole CTA).  The last step only stores: nothing of its segment is
+    // read, and its flag is 0.
+    auto read_flags = [&](int first) {
+      __syncthreads();
+      for (int i = t; i < FLAGS; i += NT) {
+        const int step = first + i;
+        const bool on = step < n - 1 && (!p.use_m || p.use_m[(long long)seg(step) * p.use_stride + hv] != 0);
+        const unsigned bits = __ballot_sync(0xffffffffu, on);
+        if ((t & 31) == 0) apply[step / 32 % (2 * FLAGS / 32)] = bits;
+      }
+      __syncthreads();
     };
-    auto fetch_m = [&](int step, int with_m) {
-      if (with_m) {
-        const float* m = strided(p.M, step);
-        float* dst = sm + step % 3 * C::M_FLOATS;
+    auto flag = [&](int step) { return apply[step / 32 % (2 * FLAGS / 32)] >> (step & 31) & 1; };
+    // M and the local state of a step (a group of asynchronous copies, empty behind the end of the chain)
+    auto fetch = [&](int step) {
+      if (step < n - 1) {
+        const float* l = strided(p.local, step) + v0;
+        float* dl = loc + step % 3 * C::L_FLOATS;
         if (p.vec16) {
-#pragma unroll 4
-          for (int i = t * 4; i < D * D; i += NT * 4) cp_async16(dst + i / D * LDM + i % D, m + i, true);
+          for (int i = t * 4; i < D * BV; i += NT * 4) cp_async16(dl + i, l + (long long)(i / BV) * D + i % BV, true);
         } else {
+          for (int i = t; i < D * BV; i += NT) cp_async4(dl + i, l + (long long)(i / BV) * D + i % BV);
+        }
+        if (flag(step)) {
+          const float* m = strided(p.M, step);
+          float* dst = sm + step % 3 * C::M_FLOATS;
+          auto at = [](int i) { return i / D * D + (((i % D >> 2) ^ (i / D & 7)) << 2) + i % 4; };
+          if (p.vec16) {
 #pragma unroll 4
-          for (int i = t; i < D * D; i += NT) cp_async4(dst + i / D * LDM + i % D, m + i);
+            for (int i = t * 4; i < D * D; i += NT * 4) cp_async16(dst + at(i), m + i, true);
+          } else {
+#pragma unroll 4
+            for (int i = t; i < D * D; i += NT) cp_async4(dst + at(i), m + i);
+          }
         }
       }
       cp_async_commit();
     };
-    auto fetch_local = [&](int step, float (&x)[PER]) {
-      if (step >= n - 1) return;
-      const float* l = strided(p.local, step) + (long long)row * D + v0 + col;
-#pragma unroll
-      for (int e = 0; e < PER; ++e) x[e] = l[e];
-    };
-    float own[PER], loc[PER], loc_next[PER];
+    float own[PER];
     const float* raw = p.raw ? p.raw + ((long long)r * p.Hv + hv) * D * D : nullptr;
 #pragma unroll
     for (int e = 0; e < PER; ++e) {
       const int v = v0 + col + e;
       own[e] = !raw ? 0.f : raw[p.raw_v_first ? (long long)v * D + row : (long long)row * D + v];
-      loc[e] = loc_next[e] = 0.f;
     }
-    int with_m = flag(0), with_m1 = flag(1), with_m2 = flag(2);
-    fetch_m(0, with_m);
-    fetch_m(1, with_m1);
-    fetch_local(0, loc);
+    read_flags(0);
+    fetch(0);
+    fetch(1);
 #pragma unroll 1
     for (int step = 0; step < n; ++step) {
       float* dst = p.out + (((long long)seg(step) * p.Hv + hv) * D + row) * D + v0 + col;
+      store_floats(cur + row * BV + col, own);
+      if (p.vec16) {
+        store_floats(dst, own);
+      } else {
 #pragma unroll
-      for (int e = 0; e < PER; ++e) dst[e] = cur[row * BV + col + e] = own[e];
+        for (int e = 0; e < PER; ++e) dst[e] = own[e];
+      }
       if (step == n - 1) break;
-      fetch_m(step + 2, with_m2);  // (its buffer was last read before the barrier that ended step - 1)
-      const int with_m3 = flag(step + 3);
-      fetch_local(step + 1, loc_next);
+      const int with_m = flag(step);
+      if ((step + 2) % FLAGS == 0) read_flags(step + 2);  // (the other half holds this step's and the next one's)
+      fetch(step + 2);  // (its buffers were last read before the barrier that ended step - 1)
       cp_async_wait<2>();
       __syncthreads();
+      // (read here, ahead of the barrier behind which its buffer is filled again)
+      load_floats(own, loc + step % 3 * C::L_FLOATS + row * BV + col);
       if (with_m) {
         const float* m = sm + step % 3 * C::M_FLOATS;
         float acc[2][BV] = {};
@@ -242,11 +282,12 @@ __global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             if (!p.reverse) {
-              const float4 x = *reinterpret_cast<const float4*>(m + (a + h * (D / 2)) * LDM + b);
+              const float4 x = *reinterpret_cast<const float4*>(m + (a + h * (D / 2)) * D + (((b >> 2) ^ (a & 7)) << 2));
               w[h][0] = x.x; w[h][1] = x.y; w[h][2] = x.z; w[h][3] = x.w;
             } else {
 #pragma unroll
-              for (int j = 0; j < 4; ++j) w[h][j] = m[(b + j) * LDM + a + h * (D / 2)];
+              for (int j = 0; j < 4; ++j)
+                w[h][j] = m[(b + j) * D + ((((a + h * (D / 2)) >> 2) ^ ((b + j) & 7)) << 2) + (a & 3)];
             }
           }
 #pragma unroll
@@ -263,23 +304,27 @@ __global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           float* q = part + ((t / (D / 2)) * D + a + h * (D / 2)) * BV;
-          *reinterpret_cast<float4*>(q) = make_float4(acc[h][0], acc[h][1], acc[h][2], acc[h][3]);
-          *reinterpret_cast<float4*>(q + 4) = make_float4(acc[h][4], acc[h][5], acc[h][6], acc[h][7]);
+          // the halves of a row in the order that keeps eight lanes (32 bytes apart) off each other's banks
+          const bool odd = a >> 2 & 1;
+#pragma unroll
+          for (int z = 0; z < 2; ++z) {
+            const bool up = odd != (z == 1);
+            *reinterpret_cast<float4*>(q + (up ? 4 : 0)) =
+                make_float4(up ? acc[h][4] : acc[h][0], up ? acc[h][5] : acc[h][1], up ? acc[h][6] : acc[h][2],
+                            up ? acc[h][7] : acc[h][3]);
+          }
         }
       }
       __syncthreads();
+      if (with_m) {
 #pragma unroll
-      for (int e = 0; e < PER; ++e) {
-        own[e] = loc[e];
-        if (with_m) {
+        for (int k = 0; k < KS; ++k) {
+          float x[PER];
+          load_floats(x, part + (k * D + row) * BV + col);
 #pragma unroll
-          for (int k = 0; k < KS; ++k) own[e] += part[(k * D + row) * BV + col + e];
+          for (int e = 0; e < PER; ++e) own[e] += x[e];
         }
-        loc[e] = loc_next[e];
       }
-      with_m = with_m1;
-      with_m1 = with_m2;
-      with_m2 = with_m3;
     }
     cp_async_wait<0>();
     __syncthreads();  // the next chain of this CTA reuses every buffer
