@@ -132,7 +132,9 @@ std::shared_ptr<Batch> build(const std::optional<at::Tensor>& cu, int64_t B, int
   // coarser rule leaves it so (and is planned again by the first call that can)
   b->provisional = cap && !packed && leads && plan;
   if (b->provisional) leads = false;
-  const auto split = !plan ? std::nullopt
+  int64_t longest = 0;
+  for (size_t i = 1; i < bounds.size(); ++i) longest = std::max(longest, bounds[i] - bounds[i - 1]);
+  const auto split = !plan || (leads && longest <= (LEAD_MIN_CHUNKS - 1) * CHUNK) ? std::nullopt
                      : leads ? split_sequences(bounds, Hv, n_sm, LEAD_MIN_SEGMENT_CHUNKS, 1, LEAD_SPLIT_CHUNKS)
                              : split_sequences(bounds, Hv, n_sm);
   Tables seg{};

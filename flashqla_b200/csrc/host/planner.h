@@ -10,8 +10,10 @@ constexpr int CHUNK = 64;
 constexpr int MIN_SEGMENT_CHUNKS = 8;
 // K = V = 128, where most segments start a few chunks early and need no state from a pass of its own:
 // shorter segments pay.  LEAD_SPLIT_CHUNKS: what a split costs in any case, the three launches that find
-// out whether a state has to be handed over (9 us forward, 11 backward).
-constexpr int LEAD_MIN_SEGMENT_CHUNKS = 4, LEAD_SPLIT_CHUNKS = 4;
+// out whether a state has to be handed over (9 us forward, 11 backward).  Batches whose longest sequence has
+// less than LEAD_MIN_CHUNKS stay whole: there the launches cost a training step, which waits for the host,
+// more than the shorter chains give.
+constexpr int LEAD_MIN_SEGMENT_CHUNKS = 4, LEAD_SPLIT_CHUNKS = 4, LEAD_MIN_CHUNKS = 2 * MIN_SEGMENT_CHUNKS;
 // costs, in chunk steps of the recurrence kernel
 constexpr int SEGMENT_OVERHEAD_CHUNKS = 2;  // handing a start state to a segment
 constexpr int CTA_START_CHUNKS = 2;         // starting a CTA (tensor-memory allocation, first loads)
