@@ -21,6 +21,7 @@ SIGNATURES = {
     "fqla_bwd_dh": [P, P, P, P, P, I, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, P, P, I, I, I,
                     P],
     "fqla_fwd_run": [P, P],
+    "fqla_segment_scan_run": [P, P],
     "fqla_merge_run": [P, P],
     "fqla_bwd_dh_run": [P, P],
     "fqla_bwd_main_run": [P, P],

@@ -82,11 +82,14 @@ warmup_scan_kernel(const float* __restrict__ g_cum, int Hv, SeqLayout lay, int n
 //     exact_warm = -1 tells the separate state-only pass to skip the segment;
 //   * otherwise (any_fb = 1) lead = 0 everywhere and exact_warm = warm: the state-only pass,
 //     the transition matrices and the merge chain produce the exact start states.
+// make_m, have_m: see fqla_scan_args in include/fqla.h.  A training step computes each matrix once: the
+// pass of the backward over the segments of 2 x 8111 tokens, two of eight heads without decay, took 34 us.
 __global__ void __launch_bounds__(256)
 segment_scan_kernel(const float* __restrict__ g_cum, int Hv, SeqLayout lay,
                     const int* __restrict__ seg_begin, float threshold, int from_start,
                     int* __restrict__ warm, int* __restrict__ fallback, int* __restrict__ lead,
-                    int* __restrict__ exact_warm, int* __restrict__ any_fb) {
+                    int* __restrict__ exact_warm, int* __restrict__ any_fb, int* __restrict__ make_m,
+                    const int* __restrict__ have_m) {
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r = blockIdx.x / Hv, hv = blockIdx.x % Hv;
@@ -96,12 +99,15 @@ segment_scan_kernel(const float* __restrict__ g_cum, int Hv, SeqLayout lay,
     const bool hands_on = from_start ? seg > s0 : seg + 1 < s1;
     int n = 0;
     bool reached = true;
-    if (hands_on) n = scan_segment(g_cum, Hv, hv, lay.span(seg), threshold, from_start, lane, reached);
+    if (hands_on || (make_m && !have_m))
+      n = scan_segment(g_cum, Hv, hv, lay.span(seg), threshold, from_start, lane, reached);
     if (lane == 0) {
-      warm[seg * Hv + hv] = n;
-      fallback[seg * Hv + hv] = reached ? 0 : 1;
+      const int have = !reached && have_m && have_m[seg * Hv + hv];
+      warm[seg * Hv + hv] = hands_on || !reached ? n : 0;
+      fallback[seg * Hv + hv] = reached || !hands_on ? 0 : 1 + have;
+      if (make_m) make_m[seg * Hv + hv] = !reached && !have;
     }
-    fb_any |= reached ? 0 : 1;
+    fb_any |= reached || !hands_on ? 0 : 1;
   }
   const int any = __syncthreads_or(fb_any);  // also orders the writes above for the reads below
   if (threadIdx.x == 0) any_fb[r * Hv + hv] = any;
@@ -110,6 +116,7 @@ segment_scan_kernel(const float* __restrict__ g_cum, int Hv, SeqLayout lay,
     const bool has = from_start ? giver < s1 : giver >= s0;
     lead[seg * Hv + hv] = (!any && has) ? warm[giver * Hv + hv] : 0;
     exact_warm[seg * Hv + hv] = any ? warm[seg * Hv + hv] : -1;
+    if (make_m && !any) make_m[seg * Hv + hv] = 0;
   }
 }
 
@@ -162,7 +169,7 @@ struct Merge {
   static constexpr int CTAS_Y = D == 128 ? 9 : 54;  // x D / BV slices: all SMs, one or three CTAs each
 };
 struct MergeParams {
-  const float *local, *M;
+  const float *local, *M, *M_alt;
   const int* use_m;
   const float* raw;
   const int *seg_begin, *any_fb;
@@ -190,7 +197,7 @@ __global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
   constexpr int BV = C::BV, NT = C::NT, KS = C::KS, KB = C::KB, PER = C::PER;
   extern __shared__ __align__(16) float sm[];
   constexpr int FLAGS = 512;           // steps whose flags are read at a time
-  __shared__ unsigned active[NT / 32], apply[2 * FLAGS / 32];
+  __shared__ unsigned active[NT / 32], apply[2 * FLAGS / 32], other[2 * FLAGS / 32];
   float* loc = sm + 3 * C::M_FLOATS;   // 3 x [D][BV] local states
   float* cur = loc + 3 * C::L_FLOATS;  // [D][BV] state of the step
   float* part = cur + D * BV;          // [KS][D][BV] partial products
@@ -213,9 +220,12 @@ __global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
       __syncthreads();
       for (int i = t; i < FLAGS; i += NT) {
         const int step = first + i;
-        const bool on = step < n - 1 && (!p.use_m || p.use_m[(long long)seg(step) * p.use_stride + hv] != 0);
-        const unsigned bits = __ballot_sync(0xffffffffu, on);
-        if ((t & 31) == 0) apply[step / 32 % (2 * FLAGS / 32)] = bits;
+        const int use = step >= n - 1 ? 0 : p.use_m ? p.use_m[(long long)seg(step) * p.use_stride + hv] : 1;
+        const unsigned bits = __ballot_sync(0xffffffffu, use != 0), alt = __ballot_sync(0xffffffffu, use == 2);
+        if ((t & 31) == 0) {
+          apply[step / 32 % (2 * FLAGS / 32)] = bits;
+          other[step / 32 % (2 * FLAGS / 32)] = alt;
+        }
       }
       __syncthreads();
     };
@@ -231,7 +241,8 @@ __global__ void __launch_bounds__(256, 1) merge_kernel(const MergeParams p) {
           for (int i = t; i < D * BV; i += NT) cp_async4(dl + i, l + (long long)(i / BV) * D + i % BV);
         }
         if (flag(step)) {
-          const float* m = strided(p.M, step);
+          const bool alt = other[step / 32 % (2 * FLAGS / 32)] >> (step & 31) & 1;
+          const float* m = strided(alt ? p.M_alt : p.M, step);
           float* dst = sm + step % 3 * C::M_FLOATS;
           auto at = [](int i) { return i / D * D + (((i % D >> 2) ^ (i / D & 7)) << 2) + i % 4; };
           if (p.vec16) {
@@ -394,12 +405,12 @@ template <int D>
 static int launch_merge(const fqla_merge_args& a, cudaStream_t st) {
   using C = Merge<D>;
   MergeParams p;
-  p.local = a.local; p.M = a.M; p.use_m = a.use_m; p.raw = a.raw; p.seg_begin = a.seg_begin;
+  p.local = a.local; p.M = a.M; p.M_alt = a.M_alt ? a.M_alt : a.M; p.use_m = a.use_m; p.raw = a.raw; p.seg_begin = a.seg_begin;
   p.any_fb = a.any_fallback; p.out = a.out; p.Hv = a.Hv; p.n_pairs = a.n_raw * a.Hv;
   p.reverse = a.reverse; p.raw_v_first = a.raw_v_first;
   p.seg_stride = a.seg_stride ? a.seg_stride : (long long)a.Hv * D * D;
   p.use_stride = a.seg_stride ? a.seg_stride : a.Hv;
-  p.vec16 = ((reinterpret_cast<uintptr_t>(a.M) | reinterpret_cast<uintptr_t>(a.local) |
+  p.vec16 = ((reinterpret_cast<uintptr_t>(a.M) | reinterpret_cast<uintptr_t>(p.M_alt) | reinterpret_cast<uintptr_t>(a.local) |
               reinterpret_cast<uintptr_t>(a.out) | (unsigned long long)p.seg_stride * 4) & 15) == 0;
   static std::atomic<unsigned long long> done;
   int rc = configure_smem((const void*)merge_kernel<D>, C::SMEM_BYTES, done);
@@ -429,17 +440,28 @@ extern "C" int fqla_warmup_scan(const float* g_cum, int T, int Hv, const void* s
       g_cum, Hv, lay, n_seg, threshold, from_start, keep, warm, fallback);
 }
 
+extern "C" int fqla_segment_scan_run(const fqla_scan_args* args, void* stream) {
+  if (!args) return FQLA_ERR_INVALID_ARG;
+  const fqla_scan_args& a = *args;
+  if (!a.g_cum || !a.seg_cu_seqlens || !a.seg_begin || !a.warm || !a.fallback || !a.lead || !a.exact_warm ||
+      !a.any_fallback || a.Hv <= 0 || (a.have_m && !a.make_m))
+    return FQLA_ERR_INVALID_ARG;
+  if (a.n_raw <= 0) return FQLA_OK;
+  SeqLayout lay{{a.seg_cu_seqlens, a.idx_is64}, {a.seg_cu_seqlens, a.idx_is64}, a.T};
+  return launch_pdl(segment_scan_kernel, dim3((unsigned)(a.n_raw * a.Hv)), dim3(256), 0, (cudaStream_t)stream,
+      a.g_cum, a.Hv, lay, a.seg_begin, a.threshold, a.from_start, a.warm, a.fallback, a.lead, a.exact_warm,
+      a.any_fallback, a.make_m, a.have_m);
+}
+
 extern "C" int fqla_segment_scan(const float* g_cum, int T, int Hv, const void* seg_cu_seqlens,
                                  int idx_is64, const int* seg_begin, int n_raw, float threshold,
                                  int from_start, int* warm, int* fallback, int* lead,
                                  int* exact_warm, int* any_fb, void* stream) {
-  if (!g_cum || !seg_cu_seqlens || !seg_begin || !warm || !fallback || !lead || !exact_warm ||
-      !any_fb || Hv <= 0)
-    return FQLA_ERR_INVALID_ARG;
-  if (n_raw <= 0) return FQLA_OK;
-  SeqLayout lay{{seg_cu_seqlens, idx_is64}, {seg_cu_seqlens, idx_is64}, T};
-  return launch_pdl(segment_scan_kernel, dim3((unsigned)(n_raw * Hv)), dim3(256), 0, (cudaStream_t)stream,
-      g_cum, Hv, lay, seg_begin, threshold, from_start, warm, fallback, lead, exact_warm, any_fb);
+  fqla_scan_args a = {};
+  a.g_cum = g_cum; a.T = T; a.Hv = Hv; a.seg_cu_seqlens = seg_cu_seqlens; a.idx_is64 = idx_is64;
+  a.seg_begin = seg_begin; a.n_raw = n_raw; a.threshold = threshold; a.from_start = from_start;
+  a.warm = warm; a.fallback = fallback; a.lead = lead; a.exact_warm = exact_warm; a.any_fallback = any_fb;
+  return fqla_segment_scan_run(&a, stream);
 }
 
 extern "C" int fqla_merge_run(const fqla_merge_args* args, void* stream) {

@@ -12,7 +12,8 @@ namespace {
 
 struct GatedDeltaRuleBackward : public ag::Node {
   // inputs as the kernels read them, the forward's results, what the forward kept
-  ag::SavedVariable q, k, v, g_cum, beta, A, initial_state, cu, seg_h0, h, vnew, lead;
+  ag::SavedVariable q, k, v, g_cum, beta, A, initial_state, cu;
+  ag::SavedVariable kept[6];  // Cache, in its own order
   ag::SavedVariable q_rstd, k_rstd;  // with l2norm; q, k above are then normalised
   double scale = 1.0;
   Options opt;
@@ -24,9 +25,9 @@ struct GatedDeltaRuleBackward : public ag::Node {
   std::string name() const override { return "GatedDeltaRuleBackward"; }
 
   void release_variables() override {
-    for (ag::SavedVariable* s : {&q, &k, &v, &g_cum, &beta, &A, &initial_state, &cu, &seg_h0, &h,
-                                 &vnew, &lead, &q_rstd, &k_rstd})
+    for (ag::SavedVariable* s : {&q, &k, &v, &g_cum, &beta, &A, &initial_state, &cu, &q_rstd, &k_rstd})
       s->reset_data();
+    for (ag::SavedVariable& s : kept) s.reset_data();
   }
 
   ag::variable_list apply(ag::variable_list&& grads) override {
@@ -39,7 +40,9 @@ struct GatedDeltaRuleBackward : public ag::Node {
     const OptTensor dht = grads.size() > 1 && grads[1].defined() ? OptTensor(grads[1]) : std::nullopt;
     if (!grads[0].defined() && !dht) return out;
     const at::Tensor dO = grads[0].defined() ? grads[0] : at::zeros(o_sizes, o_options);
-    const Cache cache{opt_get(seg_h0), opt_get(h), opt_get(vnew), opt_get(lead)};
+    Cache cache;
+    int entry = 0;
+    Cache::each(cache, [&](OptTensor& t) { t = opt_get(kept[entry++]); });
     Norm norm;
     if (opt.l2norm) norm = Norm{get(q_rstd), get(k_rstd)};
     const Backward r = backward(get(q), get(k), get(v), get(g_cum), get(beta), get(A), dO, dht, scale,
@@ -96,10 +99,8 @@ std::pair<at::Tensor, OptTensor> apply(const at::Tensor& q, const at::Tensor& k,
   save(node->A, r.A);
   save_opt(node->initial_state, initial_state);
   save_opt(node->cu, cu);
-  save_opt(node->seg_h0, r.cache.seg_h0);
-  save_opt(node->h, r.cache.h);
-  save_opt(node->vnew, r.cache.vnew);
-  save_opt(node->lead, r.cache.lead);
+  int entry = 0;
+  Cache::each(r.cache, [&](OptTensor& t) { save_opt(node->kept[entry++], t); });
   if (opt.l2norm) {
     save(node->q_rstd, r.q_rstd);
     save(node->k_rstd, r.k_rstd);

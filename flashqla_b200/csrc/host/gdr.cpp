@@ -157,11 +157,12 @@ void run_dh(const Call& c, const fqla_bwd_dh_args& a) { check(fqla_bwd_dh_run(&a
 
 // Start states (reverse: end gradients) of the segments that are handed one.  The edges of a sequence
 // take raw itself (row maps), so the entries of pairs without a chain are left out.
-at::Tensor merge(const Call& c, const at::Tensor& local, const at::Tensor& M, const int* use_m,
+at::Tensor merge(const Call& c, const float* local, const float* M, const OptTensor& M_alt, const int* use_m,
                  const OptTensor& raw, bool raw_v_first, const int* any_fb, bool reverse) {
   at::Tensor out = empty({c.batch->n_seg, c.Hv, c.D, c.D}, at::kFloat, c.dev);
   fqla_merge_args a = {};
-  a.local = (const float*)local.data_ptr(); a.M = (const float*)M.data_ptr(); a.use_m = use_m;
+  a.local = local; a.M = M; a.use_m = use_m;
+  a.M_alt = ptr<float>(M_alt);
   a.raw = ptr<float>(raw); a.seg_begin = c.batch->s_begin; a.any_fallback = any_fb;
   a.out = (float*)out.data_ptr(); a.n_raw = (int)c.batch->N; a.Hv = c.Hv; a.D = c.D;
   a.reverse = reverse; a.raw_v_first = raw_v_first; a.no_edges = 1;
@@ -169,29 +170,38 @@ at::Tensor merge(const Call& c, const at::Tensor& local, const at::Tensor& M, co
   return out;
 }
 
-// Per (segment, head) int32 tables of the scan: warm, fallback, lead, exact_warm, and any_fallback
-// per (sequence, head) behind them.
+// Per (segment, head) int32 tables of the scan: warm, fallback, lead, exact_warm, make_m, and any_fallback
+// per (sequence, head) behind them.  m_mask: where matrices have to be made.
 struct Scan {
   at::Tensor store;
   int *warm, *fallback, *lead, *exact_warm, *any_fb;
-  at::Tensor lead_tensor;
+  const int* m_mask;
 };
-Scan segment_scan(const Call& c, const at::Tensor& g, bool from_start) {
+// keep: the matrices will be kept for the backward; have: which ones were
+Scan segment_scan(const Call& c, const at::Tensor& g, bool from_start, bool keep, const OptTensor& have) {
   Scan s;
   const int64_t n = c.batch->n_seg * c.Hv;
-  s.store = empty({4 * n + c.batch->N * c.Hv}, at::kInt, c.dev);
+  s.store = empty({5 * n + c.batch->N * c.Hv}, at::kInt, c.dev);
   int* p = s.store.data_ptr<int>();
   s.warm = p;
   s.fallback = p + n;
   s.lead = p + 2 * n;
   s.exact_warm = p + 3 * n;
-  s.any_fb = p + 4 * n;
-  s.lead_tensor = s.store.narrow(0, 2 * n, n).view({c.batch->n_seg, c.Hv});
-  check(fqla_segment_scan((const float*)g.data_ptr(), c.kT(), c.Hv, c.batch->s_cu, 0,
-                          c.batch->s_begin, (int)c.batch->N, THRESHOLD, from_start, s.warm,
-                          s.fallback, s.lead, s.exact_warm, s.any_fb, c.stream),
-        "segment_scan");
+  int* make = p + 4 * n;
+  s.any_fb = p + 5 * n;
+  s.m_mask = keep || have ? make : s.fallback;
+  fqla_scan_args a = {};
+  a.g_cum = (const float*)g.data_ptr(); a.T = c.kT(); a.Hv = c.Hv; a.seg_cu_seqlens = c.batch->s_cu;
+  a.seg_begin = c.batch->s_begin; a.n_raw = (int)c.batch->N; a.threshold = THRESHOLD;
+  a.from_start = from_start; a.warm = s.warm; a.fallback = s.fallback; a.lead = s.lead;
+  a.exact_warm = s.exact_warm; a.any_fallback = s.any_fb; a.make_m = keep || have ? make : nullptr;
+  a.have_m = ptr<int>(have);
+  check(fqla_segment_scan_run(&a, c.stream), "segment_scan");
   return s;
+}
+// One table of a scan as [segments, heads]
+at::Tensor scan_table(const Call& c, const Scan& s, const int* table) {
+  return s.store.as_strided({c.batch->n_seg, c.Hv}, {c.Hv, 1}, table - s.store.data_ptr<int>());
 }
 // The scan of the explicit route: every segment takes a start state from the merge chain.
 Scan warmup_scan(const Call& c, const at::Tensor& g, bool from_start) {
@@ -200,6 +210,7 @@ Scan warmup_scan(const Call& c, const at::Tensor& g, bool from_start) {
   s.store = empty({2 * n}, at::kInt, c.dev);
   s.warm = s.store.data_ptr<int>();
   s.fallback = s.warm + n;
+  s.m_mask = s.fallback;
   check(fqla_warmup_scan((const float*)g.data_ptr(), c.kT(), c.Hv, c.batch->s_cu, 0,
                          (int)c.batch->n_seg, THRESHOLD, from_start,
                          from_start ? c.batch->keep_bwd : c.batch->keep_fwd, s.warm, s.fallback,
@@ -211,38 +222,57 @@ Scan warmup_scan(const Call& c, const at::Tensor& g, bool from_start) {
 // Start states of the segments (and lead-in counts) of a split plan.  Segments whose past dies out
 // inside the segment before them start themselves a few chunks early from a zero state; the exact
 // chain (state-only pass with the transition matrices, then the merge) returns at once for them.
-void segment_starts(const Call& c, const SeqIn& in, const OptTensor& h0, const Options& opt, Cache& out) {
+// keep: the matrices, too, go to `out`.
+void segment_starts(const Call& c, const SeqIn& in, const OptTensor& h0, const Options& opt, bool keep,
+                    Cache& out) {
   const bool leads = opt.lead_in && tiles_ok(c.D);
-  const Scan s = leads ? segment_scan(c, in.g, false) : warmup_scan(c, in.g, false);
-  at::Tensor local = empty({2, c.batch->n_seg, c.Hv, c.D, c.D}, at::kFloat, c.dev);
-  at::Tensor l = local.select(0, 0), M = local.select(0, 1);
+  keep = keep && leads;
+  const Scan s = leads ? segment_scan(c, in.g, false, keep, std::nullopt) : warmup_scan(c, in.g, false);
+  at::Tensor l = empty({c.batch->n_seg, c.Hv, c.D, c.D}, at::kFloat, c.dev), M = empty(l.sizes(), at::kFloat, c.dev);
+  const float *lp = (const float*)l.data_ptr(), *Mp = (const float*)M.data_ptr();
   fqla_fwd_args a = fwd_args(c, in);
-  a.ht = (float*)l.data_ptr();
-  a.M = (float*)M.data_ptr();
+  a.ht = (float*)lp;
+  a.M = (float*)Mp;
   a.warm_chunks = leads ? s.exact_warm : s.warm;
-  a.m_mask = s.fallback;
+  a.m_mask = s.m_mask;
   run_fwd(c, a);
-  out.seg_h0 = merge(c, l, M, s.fallback, h0, opt.state_v_first, leads ? s.any_fb : nullptr, false);
-  if (leads) out.lead = s.lead_tensor;
+  out.seg_h0 = merge(c, lp, Mp, std::nullopt, s.fallback, h0, opt.state_v_first, leads ? s.any_fb : nullptr, false);
+  if (leads) out.lead = scan_table(c, s, s.lead);
+  if (keep) {
+    out.seg_m = M;
+    out.have_m = scan_table(c, s, s.m_mask);
+  }
 }
 
-// Mirror image of segment_starts for the state gradient.
-std::pair<at::Tensor, OptTensor> segment_ends(const Call& c, const SeqIn& in, const at::Tensor& dO,
-                                              const OptTensor& dht, const Options& opt) {
+// Mirror image of segment_starts for the state gradient; `kept`: what the forward kept, if anything.
+struct Ends {
+  at::Tensor ends;
+  at::Tensor tables;          // keeps what lead points to
+  const int* lead = nullptr;
+};
+Ends segment_ends(const Call& c, const SeqIn& in, const at::Tensor& dO,
+                  const OptTensor& dht, const Options& opt, const Cache& kept) {
   const bool leads = opt.lead_in && tiles_ok(c.D);
-  const Scan s = leads ? segment_scan(c, in.g, true) : warmup_scan(c, in.g, true);
+  OptTensor have, M_kept;
+  // (of use only where this call runs over the segments they were made for)
+  if (leads && kept.seg_m && kept.have_m && kept.seg_m->dim() == 4 && kept.seg_m->size(0) == c.batch->n_seg &&
+      kept.seg_m->size(1) == c.Hv && kept.have_m->numel() == c.batch->n_seg * c.Hv) {
+    M_kept = kept.seg_m;
+    have = kept.have_m;
+  }
+  const Scan s = leads ? segment_scan(c, in.g, true, false, have) : warmup_scan(c, in.g, true);
   at::Tensor local = empty({2, c.batch->n_seg, c.Hv, c.D, c.D}, at::kFloat, c.dev);
-  at::Tensor l = local.select(0, 0), M = local.select(0, 1);
+  float *l = (float*)local.data_ptr(), *M = l + local.numel() / 2;
   fqla_bwd_dh_args a = dh_args(c, in, dO);
-  a.dh0 = (float*)l.data_ptr();
+  a.dh0 = l;
   a.warm_chunks = leads ? s.exact_warm : s.warm;
   run_dh(c, a);
   fqla_fwd_args m = fwd_args(c, in);
-  m.M = (float*)M.data_ptr();
-  m.m_mask = s.fallback;
+  m.M = M;
+  m.m_mask = s.m_mask;
   run_fwd(c, m);
-  at::Tensor ends = merge(c, l, M, s.fallback, dht, opt.state_v_first, leads ? s.any_fb : nullptr, true);
-  return {ends, leads ? OptTensor(s.lead_tensor) : std::nullopt};
+  at::Tensor ends = merge(c, l, M, M_kept, s.fallback, dht, opt.state_v_first, leads ? s.any_fb : nullptr, true);
+  return {ends, s.store, leads ? s.lead : nullptr};
 }
 
 constexpr double L2NORM_EPS = 1e-6;
@@ -314,7 +344,7 @@ Forward forward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor
   const SeqIn in{q, k, v, r.A, r.g_cum, beta, beta_f32};
   const bool tiles = tiles_ok(c.D);
   const bool keep = opt.cache && opt.save_tiles && !opt.output_h;
-  if (c.split) segment_starts(c, in, h0, opt, r.cache);
+  if (c.split) segment_starts(c, in, h0, opt, opt.cache, r.cache);
 
   // the tcgen05 kernel writes o in the caller's float16 itself
   const bool o_f16 = tiles && q_in.scalar_type() == at::kHalf;
@@ -383,7 +413,7 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
         starts.seg_h0 = cached.seg_h0;
         starts.lead = cached.lead;
       } else {
-        segment_starts(c, in, h0, opt, starts);
+        segment_starts(c, in, h0, opt, false, starts);
       }
     }
     h = empty({c.batch->num_chunks, c.Hv, c.D, c.D}, at::kBFloat16, c.dev);
@@ -399,12 +429,8 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
   }
 
   // reverse recurrence of the state gradient
-  OptTensor seg_dht, lead_out;
-  if (c.split) {
-    auto [e, l] = segment_ends(c, in, dO, dht, opt);
-    seg_dht = e;
-    lead_out = l;
-  }
+  Ends ends;
+  if (c.split) ends = segment_ends(c, in, dO, dht, opt, cached);
   at::Tensor dh = empty({c.batch->num_chunks, c.Hv, c.D, c.D}, at::kBFloat16, c.dev);
   at::Tensor du = tiles ? empty({c.batch->num_chunks, c.Hv, c.D, CHUNK}, at::kBFloat16, c.dev)
                         : empty(v.sizes(), at::kBFloat16, c.dev);
@@ -416,7 +442,7 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
   d.du = du.data_ptr();
   d.dh0 = mut<float>(r.dh0);
   d.state_v_first = opt.state_v_first;
-  d.lead_chunks = ptr<int>(lead_out);
+  d.lead_chunks = ends.lead;
   d.operand_tiles = tiles;
   at::Tensor counter;  // hands out the items of the chunk-parallel kernel
   if (tiles) {
@@ -424,7 +450,7 @@ Backward backward(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tens
     d.zero_word = counter.data_ptr<int>();
   }
   if (c.split) {
-    d.seg_dht = ptr<float>(seg_dht);
+    d.seg_dht = (const float*)ends.ends.data_ptr();
     d.dht_row = c.batch->raw_last;
     d.dh0_row = c.batch->raw_first;
   }

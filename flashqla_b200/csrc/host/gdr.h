@@ -22,9 +22,14 @@ struct Options {
 };
 
 // What the forward keeps for the backward: start states of the segments of a split plan, per-chunk
-// states and v_new (operand tiles for K = V = 128, row-major for 64), lead-in chunk counts.
+// states and v_new (operand tiles for K = V = 128, row-major for 64), lead-in chunk counts, and the
+// transition matrices of the segments that have one (flags in have_m; the backward applies the same ones).
 struct Cache {
-  OptTensor seg_h0, h, vnew, lead;
+  OptTensor seg_h0, h, vnew, lead, seg_m, have_m;
+  template <typename Self, typename F>
+  static void each(Self& c, F&& f) {
+    for (auto* t : {&c.seg_h0, &c.h, &c.vnew, &c.lead, &c.seg_m, &c.have_m}) f(*t);
+  }
 };
 
 // Reciprocal norms of the rows of q and k before their L2 normalisation.

@@ -160,7 +160,7 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Forward r = without_gil([&] { return forward(q, k, v, g, beta, scale, h0, cu, opt); });
     PyObject* cache;
     if (r.has_cache) {
-      cache = tuple_of(r.cache.seg_h0, r.cache.h, r.cache.vnew, r.cache.lead);
+      cache = tuple_of(r.cache.seg_h0, r.cache.h, r.cache.vnew, r.cache.lead, r.cache.seg_m, r.cache.have_m);
     } else {
       cache = Py_None;
       Py_INCREF(cache);
@@ -192,9 +192,10 @@ PyObject* py_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Cache cache;
     if (a[12] != Py_None) {
       if (!PyTuple_Check(a[12])) throw PyError(PyError::Type, "cp_cache must be a tuple or None");
-      OptTensor* slots[4] = {&cache.seg_h0, &cache.h, &cache.vnew, &cache.lead};
-      for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(a[12]) && i < 4; ++i)
-        *slots[i] = opt_tensor(PyTuple_GET_ITEM(a[12], i), "cp_cache entry");
+      Py_ssize_t i = 0;
+      Cache::each(cache, [&](OptTensor& t) {
+        if (i < PyTuple_GET_SIZE(a[12])) t = opt_tensor(PyTuple_GET_ITEM(a[12], i++), "cp_cache entry");
+      });
     }
     Norm norm;
     bool norm_f16 = false;

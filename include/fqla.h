@@ -234,7 +234,8 @@ int fqla_merge_states(const float* local, const float* M, const int* use_m, cons
 
 /* fqla_merge_states with every argument in one structure, zero-initialised by the caller.
  * raw_v_first: raw is [value dim][key dim] (local, M and out never are); no_edges: with
- * any_fallback, the edge entries of pairs without a chain are not written either. */
+ * any_fallback, the edge entries of pairs without a chain are not written either; M_alt (optional,
+ * laid out as M): where use_m is 2 the matrix is taken from here. */
 typedef struct fqla_merge_args {
   const float *local, *M;
   const int* use_m;
@@ -243,6 +244,7 @@ typedef struct fqla_merge_args {
   float* out;
   int n_raw, Hv, D, reverse, raw_v_first, no_edges;
   long long seg_stride;
+  const float* M_alt;
 } fqla_merge_args;
 int fqla_merge_run(const fqla_merge_args* args, void* stream);
 
@@ -293,6 +295,27 @@ int fqla_finish_grads(const void* dq_v, const void* dk_v, const void* dv_in, con
 int fqla_segment_scan(const float* g_cum, int T, int Hv, const void* seg_cu_seqlens, int idx_is64,
                       const int* seg_begin, int n_raw, float threshold, int from_start, int* warm,
                       int* fallback, int* lead, int* exact_warm, int* any_fallback, void* stream);
+
+/* fqla_segment_scan with every argument in one structure, zero-initialised by the caller, plus make_m
+ * [n_seg,Hv] (optional, int32): the segments whose transition matrix has to be computed (m_mask of the
+ * state-only pass).  Without have_m these are the ones with fallback set and, of (sequence, head) pairs
+ * with any_fallback, the one that hands nothing on, where it does not reach the threshold either (its
+ * exact_warm is then its length): all that the scan of the other direction will ask for.  have_m [n_seg,Hv]
+ * (optional, with make_m) says which matrices the other direction has computed: where fallback would be 1
+ * it is then 2, and make_m 0. */
+typedef struct fqla_scan_args {
+  const float* g_cum;
+  int T, Hv;
+  const void* seg_cu_seqlens;
+  int idx_is64;
+  const int* seg_begin;
+  int n_raw;
+  float threshold;
+  int from_start;
+  int *warm, *fallback, *lead, *exact_warm, *any_fallback, *make_m;
+  const int* have_m;
+} fqla_scan_args;
+int fqla_segment_scan_run(const fqla_scan_args* args, void* stream);
 
 /* Forward (o and, optionally, the final state ht) for hosts that cannot allocate device memory
  * where they call this library: an inference engine that gave all device memory to its own arena
