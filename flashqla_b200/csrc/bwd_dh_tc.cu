@@ -12,10 +12,13 @@
 //     dv^T = rho .* X1^T + X2^T                        -> bf16 operand, emitted as du
 //     w    = (Ac diag(beta gamma)) Kc   [tok][k]
 //     dS^T <- gamma_last dS^T - dv^T w + dOc^T (scale gamma .* Qc)
-// Six roles as in the forward kernel (fwd_tc.cu): warp 0 issues every tcgen05.mma, warp 1 runs the
-// TMA pipeline (two stages of q, k, dO, A) and the per-row vectors, warps 2-3 scale A and q (in place),
-// warps 4-7 own the state (operand copy, decay, dh / dh0 output), warps 8-11 turn X1, X2 and w
-// into operands (and write du), warps 12-15 build Pg.  All waits are bounded mbarrier waits.
+// Roles: warp 0 issues the products that dS depends on (X1, the update), warp 3 the others (P, w, X2), warp 1
+// runs the TMA pipeline (two stages of q, k, dO, A) and the per-row vectors, warp 2 scales A, warps 4-7 own
+// the state (operand copy, decay, dh / dh0 output), warps 8-11 turn X1, X2 and w into operands (and write
+// du), warps 12-15 build Pg and scale q (in place).  All waits are bounded mbarrier waits.
+// (One thread issued everything before, 32 instructions of some 50 cycles a chunk, and two warps scaled both A
+// and q and took longer over q than the chain over a chunk: 262144 tokens x 8 heads 674 -> 587 us, 32768 packed
+// x 32 heads 384 -> 360, 4096 x 8 heads 22.6 -> 21.7; with A scaled by the state group 618, 362 and 21.9.)
 #include <cuda.h>
 
 #include <climits>
@@ -123,8 +126,8 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
   if (tid == 0) {
     mbar_init(&bars[FULL0], 1);
     mbar_init(&bars[FULL1], 1);
-    mbar_init(&bars[EMPTY0], 1 + 2);  // MMA commit + the two scaling warps
-    mbar_init(&bars[EMPTY1], 1 + 2);
+    mbar_init(&bars[EMPTY0], 2);  // MMA commits of the two issuing threads
+    mbar_init(&bars[EMPTY1], 2);
     mbar_init(&bars[S_COPY], 128);
     mbar_init(&bars[S_DEC], 128);
     mbar_init(&bars[X1_DONE], 1);
@@ -135,13 +138,13 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     mbar_init(&bars[DV_READY], 128);
     mbar_init(&bars[W_READY], 128);
     mbar_init(&bars[P_READY], 128);
-    mbar_init(&bars[AP_READY], 2);
-    mbar_init(&bars[QS_READY], 2);
+    mbar_init(&bars[AP_READY], 1);
+    mbar_init(&bars[QS_READY], 128);
     mbar_init(&bars[PRIV], 1);
     mbar_init(&bars[FULLA0], 1);
     mbar_init(&bars[FULLA1], 1);
-    mbar_init(&bars[EMPTYA0], 2);  // the two scaling warps, the only readers of the raw A tile
-    mbar_init(&bars[EMPTYA1], 2);
+    mbar_init(&bars[EMPTYA0], 1);  // the scaling warp, the only reader of the raw A tile
+    mbar_init(&bars[EMPTYA1], 1);
     mbar_init(&bars[PRIVA], 1);
     *abort_flag = 0;
     fence_mbar_init();
@@ -308,7 +311,8 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     const int wq = warp & 3;
     const int tok_w = 16 * wq + lane;  // lanes 0-15 of each quarter hold a row of w
     auto convert_w = [&](int it) {
-      if (!WAIT(W_DONE, it & 1)) return false;
+      // ... and the state update that reads the tile of the chunk before is complete
+      if (!WAIT(W_DONE, it & 1) || (it > 0 && !WAIT(S_DONE, (it - 1) & 1))) return false;
       tc_fence_after();
 #pragma unroll 1
       for (int c0 = 0; c0 < D; c0 += 32) {
@@ -375,7 +379,10 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       if (it + 1 < n_it) ok = convert_w(it + 1);
     }
   } else if (warp >= 12) {
-    // =============================== Pg group ===============================
+    // =============================== Pg and q group ===============================
+    // Pg, then q' = scale gamma .* q (rows) over q, once P = Q K^T has read it: ready long before the state
+    // update wants it.  Two threads per row, in rotated order.
+    const int qr = (tid - 384) >> 1, qh = tid & 1;
     const int wq = warp & 3;
     const int row_a = 16 * wq + (lane >> 2), row_b = row_a + 8, cp = 2 * (lane & 3);
     const uint32_t lanes_p = (uint32_t)(wq * 32) << 16;
@@ -409,32 +416,43 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       fence_proxy_async();
       tc_fence_before();
       mbar_arrive(&bars[P_READY]);
+      // (not before the update of the chunk before has been issued: its thread waits for that chunk's q)
+      if (it > 0) ok = WAIT(S_DONE, (it - 1) & 1);
+      if (!ok) break;
+      const float sg = vs[V_SGAM * CHUNK + qr];
+      unsigned char* q = smem + OFF_STAGE + (it & 1) * STAGE_BYTES + qh * 8192 + qr * 128;
+#pragma unroll 4
+      for (int q8 = 0; q8 < 8; ++q8) {
+        uint4* x8 = reinterpret_cast<uint4*>(q + ((q8 + qr) & 7) * 16);
+        const uint4 a = *x8;
+        *x8 = make_uint4(scale2(a.x, sg, sg), scale2(a.y, sg, sg), scale2(a.z, sg, sg), scale2(a.w, sg, sg));
+      }
+      fence_proxy_async();
+      mbar_arrive(&bars[QS_READY]);
     }
-  } else if (warp == 0) {
-    // =============================== MMA issuer ===============================
-    // (the warp stays converged; see elect_one in tc05.cuh)
+  } else if (warp == 0 || warp == 3) {
+    // =============================== MMA issuers ===============================
+    // (the warps stay converged; see elect_one in tc05.cuh)  Warp 0 issues what the state gradient depends
+    // on: X1 and the two products of the update; warp 3 the rest (P, w, X2 of the next iteration).
     constexpr uint32_t ID_P = idesc_bf16(64, 64, 0, 0);
     constexpr uint32_t ID_X1 = idesc_bf16(128, 64, 0, 0);
     constexpr uint32_t ID_X2 = idesc_bf16(128, 64, 1, 1);
     constexpr uint32_t ID_W = idesc_bf16(64, 128, 0, 1);
     constexpr uint32_t ID_UPD_W = idesc_bf16(128, 128, 0, 1) | (1u << 13);  // A negated
     constexpr uint32_t ID_UPD_Q = idesc_bf16(128, 128, 1, 1);
-    const uint32_t st_lo = desc_lo_kmajor(smem + OFF_ST), dvt_lo = desc_lo_kmajor(smem + OFF_DVT);
-    const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 8192), pmn_lo = desc_lo_mnmajor(smem + OFF_P, 8192);
-    const uint32_t app_lo = desc_lo_kmajor(smem + OFF_APP);
-    const uint32_t q0_lo = desc_lo_kmajor(smem + OFF_STAGE), qmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE, 8192);
-    const uint32_t k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE);
-    const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE, 8192);
+    const uint32_t q0_lo = desc_lo_kmajor(smem + OFF_STAGE), k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE);
     const uint32_t domn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + 2 * TILE, 8192);
     constexpr uint32_t STAGE_LO = STAGE_BYTES >> 4;
     auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
+    if (warp == 0) {
+      const uint32_t st_lo = desc_lo_kmajor(smem + OFF_ST), dvt_lo = desc_lo_kmajor(smem + OFF_DVT);
+      const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 8192), qmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE, 8192);
 #pragma unroll 1
-    for (int it = -1; it < n_it && ok; ++it) {  // it = -1: only what prepares the first iteration
-      const int s = it & 1;
-      const uint32_t so = s ? STAGE_LO : 0u, so_next = s ? 0u : STAGE_LO;
-      const int y_tile = (int)(((sp.chunk_base + (n_it - 1 - it)) * p.Hv + hv) * D);
-      if (it >= 0) {
-        ok = WAITW(S_COPY, it & 1);
+      for (int it = 0; it < n_it && ok; ++it) {
+        const int s = it & 1;
+        const uint32_t so = s ? STAGE_LO : 0u;
+        const int y_tile = (int)(((sp.chunk_base + (n_it - 1 - it)) * p.Hv + hv) * D);
+        ok = WAITW(FULL0 + s, (it >> 1) & 1) && WAITW(S_COPY, it & 1);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
@@ -448,18 +466,6 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
             tma_store_commit();
           }
         }
-      }
-      if (it + 1 < n_it) {
-        // (the Pg group has read P of this chunk: P_READY was waited for an iteration ago)
-        ok = WAITW(FULL0 + (s ^ 1), ((it + 1) >> 1) & 1);
-        if (!ok) break;
-        tc_fence_after();
-        if (elect_one()) {
-          umma_group<8, 2, 512, 2, 512, false>(tmem + TM_P, q0_lo + so_next, k0_lo + so_next, ID_P);
-          umma_commit(&bars[P_DONE]);
-        }
-      }
-      if (it >= 0) {
         // dS^T <- dS^T + dO^T (scale gamma q) - dv^T w; the first product while dv is on its way
         ok = WAITW(QS_READY, it & 1) && WAITW(S_DEC, it & 1);
         if (!ok) break;
@@ -480,24 +486,41 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
           umma_commit(&bars[EMPTY0 + s]);
         }
       }
-      if (it + 1 < n_it) {
-        ok = WAITW(AP_READY, (it + 1) & 1);
+      if (elect_one()) tma_store_wait_all();
+    } else {
+      const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE, 8192);
+      const uint32_t app_lo = desc_lo_kmajor(smem + OFF_APP), pmn_lo = desc_lo_mnmajor(smem + OFF_P, 8192);
+#pragma unroll 1
+      for (int it = 0; it < n_it && ok; ++it) {
+        const int s = it & 1;
+        const uint32_t so = s ? STAGE_LO : 0u;
+        // (the Pg group has read P of the chunk before: P_READY was waited for)
+        ok = WAITW(FULL0 + s, (it >> 1) & 1);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
-          umma_group<4, 2, 0, 128, 0, false>(tmem + TM_W, app_lo, kmn0_lo + so_next, ID_W);
+          umma_group<8, 2, 512, 2, 512, false>(tmem + TM_P, q0_lo + so, k0_lo + so, ID_P);
+          umma_commit(&bars[P_DONE]);
+        }
+        // w, whose accumulator the dv / w group has read for the chunk before
+        ok = WAITW(AP_READY, it & 1) && (it == 0 || WAITW(W_READY, (it - 1) & 1));
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          umma_group<4, 2, 0, 128, 0, false>(tmem + TM_W, app_lo, kmn0_lo + so, ID_W);
           umma_commit(&bars[W_DONE]);
         }
-        ok = WAITW(P_READY, (it + 1) & 1);
+        // X2^T = dO^T Pg, likewise
+        ok = WAITW(P_READY, it & 1) && (it == 0 || WAITW(DV_READY, (it - 1) & 1));
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
-          umma_group<4, 128, 0, 128, 0, false>(tmem + TM_X2, domn0_lo + so_next, pmn_lo, ID_X2);
+          umma_group<4, 128, 0, 128, 0, false>(tmem + TM_X2, domn0_lo + so, pmn_lo, ID_X2);
           umma_commit(&bars[X2_DONE]);
+          umma_commit(&bars[EMPTY0 + s]);
         }
       }
     }
-    if (elect_one()) tma_store_wait_all();
   } else if (warp == 1) {
     // =============================== producer ===============================
     float g_r[2] = {0.f, 0.f}, b_r[2] = {0.f, 0.f}, gl_r = 0.f;
@@ -592,12 +615,11 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       if (it + 2 < n_it) fetch(it + 2);
     }
   } else {
-    // =============================== scaling warps (2, 3) ===============================
+    // =============================== scaling warp (2) ===============================
     // A'' = A diag(beta gamma) (columns): thread t owns the 8 columns 8 (t%8) .. of the rows
-    // t/8 + 8 i, its scale factors stay in registers and the eight threads of a row touch one
-    // 128-byte line per access.  q' = scale gamma .* q (rows): one thread per row, rotated order.
-    const int r = tid - 64;
-    const int c8 = r & 7, r0 = r >> 3, pc_a = c8 ^ r0;
+    // t/8 + 4 i, its scale factors stay in registers and the eight threads of a row touch one
+    // 128-byte line per access.
+    const int c8 = lane & 7, r0 = lane >> 3;
     for (int it = 0; it < n_it && ok; ++it) {
       const int s = it & 1;
       ok = WAIT(FULLA0 + s, (it >> 1) & 1);
@@ -608,8 +630,8 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       const float4 g0 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8);
       const float4 g1 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8 + 4);
 #pragma unroll 4
-      for (int i = 0; i < 8; ++i) {
-        const int off = (r0 + 8 * i) * 128 + pc_a * 16;
+      for (int i = 0; i < 16; ++i) {
+        const int row = r0 + 4 * i, off = row * 128 + (c8 ^ (row & 7)) * 16;
         const uint4 a = *reinterpret_cast<const uint4*>(src + off);
         *reinterpret_cast<uint4*>(smem + OFF_APP + off) =
             make_uint4(scale2(a.x, g0.x, g0.y), scale2(a.y, g0.z, g0.w), scale2(a.z, g1.x, g1.y),
@@ -620,24 +642,6 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       if (lane == 0) {
         mbar_arrive(&bars[AP_READY]);
         mbar_arrive(&bars[EMPTYA0 + s]);  // the A tile of this stage is no longer read
-      }
-      // q' goes over q, once P = Q K^T has read it: ready long before the state update wants it (a
-      // buffer of its own had to wait for the update of the chunk before)
-      ok = WAIT(FULL0 + s, (it >> 1) & 1) && WAIT(P_DONE, it & 1);
-      if (!ok) break;
-      const float sg = vs[V_SGAM * CHUNK + r];
-      unsigned char* q = smem + OFF_STAGE + s * STAGE_BYTES + r * 128;
-#pragma unroll 2
-      for (int q16 = 0; q16 < 16; ++q16) {
-        uint4* x = reinterpret_cast<uint4*>(q + (q16 >> 3) * 8192 + ((q16 + r) & 7) * 16);
-        const uint4 a = *x;
-        *x = make_uint4(scale2(a.x, sg, sg), scale2(a.y, sg, sg), scale2(a.z, sg, sg), scale2(a.w, sg, sg));
-      }
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&bars[QS_READY]);
-        mbar_arrive(&bars[EMPTY0 + s]);
       }
     }
   }
