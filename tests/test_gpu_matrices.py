@@ -1,4 +1,4 @@
-"""The transition matrices that the forward keeps for the backward (entries five and six of its cache): the
+"""The transition matrices that the forward keeps for the backward (attributes of its cache): the
 gradients are bit for bit those of a backward that makes its own.  Segments that never forget, gates that
 rise again (where the scans of the two directions decide differently, so that each side has matrices the other
 lacks), ragged ends, several sequences, one of them unsplit."""
@@ -33,9 +33,9 @@ def test_kept_matrices_change_nothing(lens, gate):
     cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device="cuda")
     g_cum, A, *_, cache = fq.chunk_gated_delta_rule_fwd(q, k, v, g, beta, None, h0, cu, output_final_state=True,
                                                         enable_fwd_cp_cache=True)
-    assert len(cache) == 6 and cache[4] is not None
+    assert len(cache) == 4 and cache.seg_m is not None
     args = (q, k, v, g_cum, beta, A, do, dht, None, h0, cu)
-    own = fq.chunk_gated_delta_rule_bwd(*args, cp_cache=cache[:4])
+    own = fq.chunk_gated_delta_rule_bwd(*args, cp_cache=tuple(cache))
     for _ in range(2):
         for a, b in zip(fq.chunk_gated_delta_rule_bwd(*args, cp_cache=cache), own):
             assert torch.equal(a, b)
