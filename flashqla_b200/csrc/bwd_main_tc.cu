@@ -10,7 +10,7 @@
 //     dk = rho v_new dh^T - beta gamma Y + ds^T q + (X + X^T) K
 // and dg, dbeta from row and column sums of q dq1, k dk1, k Y, v dW, ds (Q K^T), dL (K K^T).  (As the chain
 // dA = -(du h^T) (beta gamma K)^T + du (beta V)^T, dL = -A^T dA A^T it was sixteen products and six
-// read-outs in a row instead of eleven and three: 262144 tokens x 8 heads 1484 us, now 1380.)
+// read-outs in a row instead of eleven and three: 262144 tokens x 8 heads 1471 us, now 1340 to 1358.)
 // All tile products are tcgen05.mma with M = 64 (rows = tokens) and fp32 accumulators in tensor memory;
 // two M = 64 accumulators share each column range (lanes +0 and +16 of every 32-lane quarter).
 //
@@ -142,11 +142,11 @@ __device__ __forceinline__ void bulk_barrier() {  // warps 8-15
 // Persistent: CTA b starts with work item b and takes the next one that nobody has; item w = (chunk
 // w / Hv, head w % Hv), so neighbouring CTAs share q and k of a grouped-value-attention group through
 // L2.  SMs differ in speed by a fifth (instruction fetch), and with a fixed share each the fast ones run
-// away: a tail, and CTAs working far apart in memory.  262144 tokens x 8 heads, 7.1 GB: 1472 us (4.8 TB/s)
-// counted out by next_item; 1492 us where the caller brings no counter and the grid has a block for every
-// item, those that run taking the items of those that have not started (CLC, cluster launch control: the
-// answer takes longer than that of an atomic); 1970-2090 us with a fixed share, 1650 us with a fixed share
-// and the 16 warps in step (see the end of an item).
+// away: a tail, and CTAs working far apart in memory.  262144 tokens x 8 heads, 7.1 GB, before the
+// present algebra: 1472 us (4.8 TB/s) counted out by next_item; 1492 us where the caller brings no counter
+// and the grid has a block for every item, those that run taking the items of those that have not started
+// (CLC, cluster launch control: the answer takes longer than that of an atomic); 1970-2090 us with a fixed
+// share, 1650 us with a fixed share and the 16 warps in step (see the end of an item).
 // TILED: h, dh, vnew and du arrive in the operand layouts written by the sequential kernels
 // (h^T, dh^T as [V][K] per chunk; vnew^T, du^T as [V][64] per chunk) instead of row-major.
 template <bool TILED, bool CLC>
