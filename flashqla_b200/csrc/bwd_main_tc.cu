@@ -107,19 +107,6 @@ enum {
 };
 }  // namespace bmtc
 
-// 16 lanes x 32 (x4) or 16 (x2) columns: register 4i+e of lane l holds row l/4 + 8*(e>>1),
-// column 8i + 2(l%4) + (e&1)
-__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, float (&v)[16]) {
-  uint32_t* r = reinterpret_cast<uint32_t*>(v);
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
 __device__ __forceinline__ void epi_barrier() {  // the 16 read-out warps only
   asm volatile("bar.sync 1, 512;" ::: "memory");
 }

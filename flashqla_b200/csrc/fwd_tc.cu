@@ -1,15 +1,16 @@
 // Sequential forward recurrence of the gated delta rule on Blackwell tensor cores:
 // TMA-fed tcgen05.mma with all accumulators in tensor memory, warp-specialised.
 //
-// One CTA (512 threads) walks the chunks of one (sequence or segment, value head), K = V = 128.
+// One CTA (640 threads; 512 without outputs) walks the chunks of one (sequence or segment, value head),
+// K = V = 128.
 // Per chunk, with S [K x V] the fp32 state entering the chunk, A the gated inverse from
 // kkt_solve, g the chunk-local cumulative log gate (gamma = exp g, rho = exp(g_last - g)):
 //
 //   off the serial chain, prepared one chunk ahead (WY form, FLA's w and u):
-//     A'  = A diag(beta),  A'' = A diag(beta gamma)                               (prep warps)
+//     A'  = A diag(beta),  A'' = A diag(beta gamma)                               (prep group)
 //     u^T [v x tok] = V^T A'^T          (A operand = V tile read MN-major)        -> TM_UV
-//     w^T [k x tok] = K^T A''^T         (A operand = K tile read MN-major)        -> TM_PW -> smem
-//     P   [tok x tok'] = Q K^T,  Pg = s P exp(g_tok - g_tok') for tok >= tok'     (O group)
+//     w^T [k x tok] = K^T A''^T         (A operand = K tile read MN-major)        -> TM_W -> smem
+//     P   [tok x tok'] = Q K^T,  Pg = s P exp(g_tok - g_tok') for tok >= tok'     (prep group)
 //   on the chain (two products):
 //     Vn^T [v x tok] = u^T - S^T w^T    (A = bf16 copy of S^T, negated; accumulates onto u^T)
 //     S^T  [v x k]   = gamma_last S^T + (rho Vn)^T K     (B = K tile read MN-major)
@@ -26,16 +27,26 @@
 // reference's blackwell/fused_fwd.py:349-596 (and the X/Y form of prepare_h.py:312-318) with the
 // gate folded into A.
 //
-// Warp roles (thread ranges):
-//     128-255 S group : fp32 master state in tensor memory; per chunk packs the bf16 operand copy
-//                       of S^T into tensor memory (on the chain), then decays S^T in place and
-//                       scales A of the next chunk (A', A'')
-//     256-383 V group : Vn^T -> rho-scaled and plain bf16 operand copies (tensor memory);
-//                       w^T -> bf16 operand tile (shared memory)
-//     384-511 O group : P -> Pg (operand); output epilogue o = s gamma O1 + O2
-//     warp 0  : issues the products of the chain, warp 1 all others (one elected lane each)
-//     warp 2  : producer: per-chunk gate vectors (fetched one chunk ahead), TMA loads of the
-//               q, k, v, A tiles (2 stages), zero-fill of rows past the end of a partial chunk
+// Warp roles:
+//     warps 4-7,   S group : fp32 master state in tensor memory; per chunk packs the bf16 operand copy of S^T
+//                            into tensor memory (on the chain), then decays S^T in place
+//     warps 8-11,  V group : Vn^T -> rho-scaled and plain bf16 operand copies (tensor memory, on the chain);
+//                            w^T -> bf16 operand tile (shared memory)
+//     warps 12-15, O group : output epilogue o = s gamma O1 + O2
+//     warps 16-19, prep group : A', A'' of the next chunk, P -> Pg   (warps 12-15 where nothing is output)
+//     warp 0 issues the two products of the chain, warp 1 those of the output, warp 3 u^T and w^T
+//     warp 2, producer: per-chunk gate vectors (fetched one chunk ahead), TMA loads of the q, k, v, A tiles
+//                       (2 stages), zero-fill of rows past the end of a partial chunk
+//
+// What bounds it: the chain of a chunk (3230 cycles on an idle chip: state copy 530, Vn^T 770, its read-out 780,
+// state update 700, and the arrivals between them) and, with all SMs at work, HBM: 262144 tokens x 8 heads 462 us,
+// 5.3 TB/s.  Two things had made it 4830 and 526 us (4 x 8192 x 16 heads 152 -> 132 us, 32768 packed x 32 heads with
+// tiles 391 -> 358).  (1) Roles that waited for one another in a ring: one thread that issued everything off the
+// chain, and an output group that built Pg between two epilogues.  No role waits here for another one's work off the
+// chain, and w^T and P, which share their columns, are read out of them at once.  (2) Code: the instruction cache of
+// an SM holds some 28 KB (straight code of one warp per scheduler, measured: full speed up to there, 2.5 cycles an
+// instruction beyond, 10 with all SMs at it), and a chunk runs every role's loop once.  So loops are rolled to
+// rounds of one tensor-memory load, and a wait is five instructions (tc05.cuh): 57 -> 47 KB, with tiles 72 -> 52.
 //
 // The state-only pass of the exact hand-off (end states and transition matrices of segments) is a
 // chain of its own, because its roundings go into every segment behind the hand-off: A diag(beta),
@@ -128,6 +139,7 @@ struct FwdTcParams {
 
 namespace fwdtc {
 constexpr int D = 128;
+constexpr int threads(bool no_o) { return no_o ? 512 : 640; }
 constexpr int TILE_QK = 16384, TILE_V = 16384, TILE_A = 8192;
 constexpr int STAGE_BYTES = 2 * TILE_QK + TILE_V + TILE_A;  // 57344
 constexpr int OFF_STAGE = 0;
@@ -155,16 +167,17 @@ constexpr uint32_t TM_VNB = 256;  // Vn^T bf16 (A operand, K = 64)  32 columns
 constexpr uint32_t TM_VRB = 288;  // rho Vn^T bf16                  32 columns
 constexpr uint32_t TM_O1 = 320;   // O1^T fp32                      64 columns
 constexpr uint32_t TM_O2 = 384;   // O2^T fp32                      64 columns
-// P (M = 64: lanes 0-15 of each quarter) and w^T of the NEXT chunk (M = 128) take turns in the
-// same columns: w^T is issued only after the output group has read P, and the next P only after
-// the value group has turned w^T into its operand tile (the chain's first product waits for it).
-constexpr uint32_t TM_PW = 448;
+// w^T of a chunk (M = 128) and, once the value group has made its operand tile of it, P (M = 64: lanes
+// 0-15 of each quarter) take turns in the same columns.
+constexpr uint32_t TM_W = 448, TM_P = TM_W;
 // state-only pass
 constexpr uint32_t TM_U = TM_UV;    // U^T fp32                   64 columns
 constexpr uint32_t TM_WB = TM_VNB;  // W^T bf16 (A operand)       32 columns
 constexpr uint32_t TM_VN = TM_O1;   // Vn^T fp32                  64 columns
 // barrier indices
-enum { FULL0 = 0, FULL1, EMPTY0, EMPTY1, S_COPY, S_DEC, VN_DONE, S_DONE, P_DONE, O_DONE, W_DONE,
+enum { FULL0 = 0, FULL1, EMPTY0, EMPTY1, S_COPY, S_DEC, VN_DONE, S_DONE, P_DONE, O_DONE,
+       // w^T, u^T of a chunk are complete (state-only pass: U^T)
+       W_DONE, U_DONE,
        VB_READY, W_READY, P_READY, O_FREE, AP_READY, PRIV,
        // the A tile and the per-row vectors of a chunk travel one chunk ahead of q, k, v
        FULLA0, FULLA1, EMPTYA0, EMPTYA1, PRIVA,
@@ -172,8 +185,10 @@ enum { FULL0 = 0, FULL1, EMPTY0, EMPTY1, S_COPY, S_DEC, VN_DONE, S_DONE, P_DONE,
        ST_READY, VN_READY,
        // the output product that reads the packed copy of S^T has completed
        SB_FREE,
-       // state-only pass: U^T is complete; W^T, made by the V and the O group, is (its name there)
-       U_DONE = P_DONE, WB_READY = P_READY };
+       // P has been read
+       P_FREE,
+       // state-only pass: W^T, made by the V and the O group, is there
+       WB_READY = P_READY };
 // vectors inside a slot; V_GL holds gamma_last at [0], V_BG -beta gamma instead of beta gamma in
 // the state-only pass
 enum { V_G = 0, V_BETA = 1, V_BG = 2, V_RHO = 3, V_SGAM = 4, V_GL = 5 };
@@ -194,13 +209,12 @@ __device__ __forceinline__ uint32_t pack_out(float lo, float hi) {
   }
 }
 
-// EXTRA: per-chunk state and v_new outputs (compiled out of the common instantiation: the six
-// roles run six different code regions at once, and the kernel is sensitive to its
-// instruction-cache footprint).  NO_O: state-only walk, no q, no output products: with EXTRA the
+// EXTRA: per-chunk state and v_new outputs (compiled out of the common instantiation, whose code
+// does not fit the instruction cache as it is).  NO_O: state-only walk, no q, no output products: with EXTRA the
 // recomputation for the backward pass (the output warps have nothing to do), without it (STATE) the end states
 // and M of the exact hand-off.  O_F16: o leaves as fp16 instead of bf16.
 template <bool EXTRA, bool NO_O, bool O_F16>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(fwdtc::threads(NO_O), 1)
 fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
               const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
               const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_h,
@@ -216,11 +230,8 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr bool STATE = NO_O && !EXTRA;
-  // What is off the chain goes in smaller rounds in the variants with per-chunk outputs.  Their code is a third
-  // larger, and code that is fetched once and runs two to four times costs fewer instruction fetches than it
-  // costs round trips to tensor memory: 262144 tokens x 8 heads 684 -> 658 us, 2 x 8111 x 8 heads 60.1 -> 55.7.
-  // Without the outputs (4 x 8192 x 16) the smaller rounds take 154.7 instead of 152.9.
-  constexpr int ROUNDS = EXTRA ? 2 : 1;
+  constexpr int NT = threads(NO_O);
+  constexpr int PREP = NO_O ? 12 : 16;  // first warp of the prep group
   const bool m_pass = STATE && (int)blockIdx.x >= p.m_first;
   const int block = m_pass ? (int)blockIdx.x - p.m_first : (int)blockIdx.x;
   const int hv = block % p.Hv;
@@ -248,9 +259,11 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   if (tid == 0) {
     mbar_init(&bars[FULL0], 1);
     mbar_init(&bars[FULL1], 1);
-    mbar_init(&bars[EMPTY0], STATE ? 1 : 2);  // MMA commits of the issuing threads
-    mbar_init(&bars[EMPTY1], STATE ? 1 : 2);
+    mbar_init(&bars[EMPTY0], STATE ? 1 : 3);  // MMA commits of the issuing threads
+    mbar_init(&bars[EMPTY1], STATE ? 1 : 3);
     mbar_init(&bars[SB_FREE], 1);
+    mbar_init(&bars[P_FREE], 128);
+    mbar_init(&bars[U_DONE], 1);
     mbar_init(&bars[FULLA0], 1);
     mbar_init(&bars[FULLA1], 1);
     // the only reader of the raw A tile: the state group, or (STATE) a product
@@ -281,10 +294,10 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   }
   // Pg is lower triangular: its tile is zeroed once, the O group only ever rewrites the column
   // groups that can be non-zero for its rows
-  for (int i = tid; i < 8192 / 16; i += 512)
+  for (int i = tid; i < 8192 / 16; i += NT)
     *reinterpret_cast<uint4*>(smem + OFF_P + i * 16) = make_uint4(0, 0, 0, 0);
   if (m_pass) {  // v stays zero: its tiles are never loaded
-    for (int i = tid; i < 2 * TILE_V / 16; i += 512)
+    for (int i = tid; i < 2 * TILE_V / 16; i += NT)
       *reinterpret_cast<uint4*>(smem + OFF_STAGE + 2 * TILE_QK + (i & 1023) * 16 + (i >> 10) * STAGE_BYTES) =
           make_uint4(0, 0, 0, 0);
   }
@@ -304,14 +317,19 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;  // this warp's lane quarter
-  bool ok = true;
-  auto WAIT = [&](int idx, uint32_t parity) { return mbar_wait(&bars[idx], parity, abort_flag); };
+  int tries = WAIT_TRIES;  // see mbar_wait; `more`: none was given up, on to the next pass of a role's loop
+  auto WAIT = [&](int idx, uint32_t parity) { mbar_wait(&bars[idx], parity, tries); };
+  auto more = [&] {
+    const bool ok = tries > 0;
+    if (ok) tries = WAIT_TRIES;
+    return ok;
+  };
 
   // Initial state -> tensor memory, S^T[v][k]; zero without one and for a lead-in.  The three
   // read-out groups share the columns 2 : 1 : 1, each thread with its whole part in flight at once:
   // one memory latency (four in turn, 3 us of an 11 us launch over two chunks, when the state group
   // loaded 32 columns at a time by itself).
-  if (warp >= 4) {
+  if (warp >= 4 && warp < 16) {
     int h0_row = p.h0_row ? p.h0_row[n] : n;
     if (lead_in < 0) h0_row = ~h0_row;
     const bool edge = h0_row >= 0;  // starts its sequence; else it is handed a state, if any
@@ -357,60 +375,18 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     }
   }
 
-  // Role of each warp.  The MMA issuer is warp 0 and the producer warp 1 on purpose: among the
-  // warps of one scheduler the oldest (lowest id) wins when several are ready, and these two
-  // single-thread roles must never queue behind the arithmetic of the compute groups.
+  // The single-thread roles are warps 0 to 3 on purpose: among the warps of one scheduler the oldest
+  // (lowest id) wins when several are ready, and these must never queue behind the compute groups.
   if (warp >= 4 && warp < 8) {
     // =============================== S group ===============================
     const int v = tid - 128;  // lane of tensor memory = value index
-    // Off the chain: A' = A diag(beta), A'' = A diag(beta gamma) of iteration j, the scaled tiles the issuing
-    // thread needs for u^T, w^T.  Thread t owns the 8 columns 8 (t%8) .. of the rows t/8 + 16 i: its 16
-    // scale factors stay in registers, and the eight threads of a row touch the eight 16-byte pieces of that
-    // row (one 128-byte line per access, conflict-free).  Here and not in the output group, whose epilogue
-    // (1780 cycles), Pg (780) and this (1060) were the 4350 cycles of a chunk, while this group waits 2600 of
-    // them: 4 x 8192 tokens x 16 heads 160 -> 152 us, 262144 x 8 532 -> 511.
-    auto scale_a = [&](int j) {
-      const int sj = j & 1, c8 = v & 7, r0 = v >> 3;
-      const int pc = c8 ^ (r0 & 7);  // physical piece: rows r0 + 16 i all have (row & 7) == r0 & 7
-      if (!WAIT(FULLA0 + sj, (j >> 1) & 1)) return false;
-      if (j > 0 && !WAIT(W_DONE, (j - 1) & 1)) return false;  // u, w of the chunk before are done
-      const float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
-      const float4 b0 = *reinterpret_cast<const float4*>(vs + V_BETA * CHUNK + 8 * c8);
-      const float4 b1 = *reinterpret_cast<const float4*>(vs + V_BETA * CHUNK + 8 * c8 + 4);
-      const float4 g0 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8);
-      const float4 g1 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8 + 4);
-      const unsigned char* src = smem + OFF_STAGE + sj * STAGE_BYTES + 2 * TILE_QK + TILE_V;
-      constexpr int N = EXTRA ? 1 : 4;  // rows a round
 #pragma unroll 1
-      for (int i0 = 0; i0 < 4; i0 += N) {
-        const int first = (r0 + 16 * i0) * 128 + pc * 16;
-        uint4 a[N];
-#pragma unroll
-        for (int i = 0; i < N; ++i) a[i] = *reinterpret_cast<const uint4*>(src + first + 2048 * i);
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-          *reinterpret_cast<uint4*>(smem + OFF_AP + first + 2048 * i) =
-              make_uint4(scale_bf16x2(a[i].x, b0.x, b0.y), scale_bf16x2(a[i].y, b0.z, b0.w),
-                         scale_bf16x2(a[i].z, b1.x, b1.y), scale_bf16x2(a[i].w, b1.z, b1.w));
-          *reinterpret_cast<uint4*>(smem + OFF_APP + first + 2048 * i) =
-              make_uint4(scale_bf16x2(a[i].x, g0.x, g0.y), scale_bf16x2(a[i].y, g0.z, g0.w),
-                         scale_bf16x2(a[i].z, g1.x, g1.y), scale_bf16x2(a[i].w, g1.z, g1.w));
-        }
-      }
-      fence_proxy_async();
-      mbar_arrive(&bars[AP_READY]);
-      mbar_arrive(&bars[EMPTYA0 + sj]);  // the A tile of this stage is no longer read here
-      return true;
-    };
-#pragma unroll 1
-    for (int it = STATE ? 0 : -1; it < n_it && ok; ++it) {  // it = -1: only A of the first iteration
-     if (it >= 0) {
+    for (int it = 0; it < n_it && more(); ++it) {
       const int s = it & 1;
       if (v == 0) FQLA_TRACE(0, 0);
-      if (it > 0) ok = WAIT(S_DONE, (it - 1) & 1);
+      if (it > 0) WAIT(S_DONE, (it - 1) & 1);
       // the output product of the chunk before, issued by the other thread, has read the copy
-      if (!NO_O && ok && it - 1 >= lead) ok = WAIT(SB_FREE, (it - 1 - lead) & 1);
-      if (!ok) break;
+      if (!NO_O && it - 1 >= lead) WAIT(SB_FREE, (it - 1 - lead) & 1);
       tc_fence_after();
       if (v == 0) FQLA_TRACE(0, 1);
       // on the chain: the bf16 operand copy of S^T, packed back into tensor memory.  (The products
@@ -431,74 +407,53 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       mbar_arrive(&bars[S_COPY]);
       if (v == 0) FQLA_TRACE(0, 2);
       if constexpr (EXTRA) {
-        // off the chain: the state entering this chunk as an output
+        // off the chain: the state entering this chunk as an output, from the operand copy
         if (p.h && it >= lead) {
-          bf16* hdst = p.h + ((sp.chunk_base + (it - lead)) * p.Hv + hv) * (long long)D * D;
+          unsigned char* row = smem + OFF_ST + v * 128;
 #pragma unroll 1
           for (int kb = 0; kb < 2; ++kb) {  // 64 columns (one operand block) per round
-            float x[32], y[32];
-            tmem_ld32(tmem + lane_sel + TM_S + kb * 64, x);
-            tmem_ld32(tmem + lane_sel + TM_S + kb * 64 + 32, y);
+            float x[32];
+            tmem_ld32(tmem + lane_sel + TM_SB + kb * 32, x);
             tmem_ld_wait();
-            if (p.tiled) {
-              unsigned char* row = smem + OFF_ST + kb * 16384 + v * 128;
 #pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                *reinterpret_cast<uint4*>(row + ((c ^ (v & 7)) << 4)) =
-                    make_uint4(pack_bf16(x[8 * c + 0], x[8 * c + 1]), pack_bf16(x[8 * c + 2], x[8 * c + 3]),
-                               pack_bf16(x[8 * c + 4], x[8 * c + 5]), pack_bf16(x[8 * c + 6], x[8 * c + 7]));
-                *reinterpret_cast<uint4*>(row + (((c + 4) ^ (v & 7)) << 4)) =
-                    make_uint4(pack_bf16(y[8 * c + 0], y[8 * c + 1]), pack_bf16(y[8 * c + 2], y[8 * c + 3]),
-                               pack_bf16(y[8 * c + 4], y[8 * c + 5]), pack_bf16(y[8 * c + 6], y[8 * c + 7]));
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                hdst[(long long)(kb * 64 + j) * D + v] = __float2bfloat16(x[j]);
-                hdst[(long long)(kb * 64 + 32 + j) * D + v] = __float2bfloat16(y[j]);
-              }
-            }
+            for (int c = 0; c < 8; ++c)
+              *reinterpret_cast<float4*>(row + kb * 16384 + ((c ^ (v & 7)) << 4)) =
+                  make_float4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
           }
           if (p.tiled) {
             fence_proxy_async();
             mbar_arrive(&bars[ST_READY]);
+          } else {  // row-major [k][v]: column v, from this thread's own row
+            bf16* hdst = p.h + ((sp.chunk_base + (it - lead)) * p.Hv + hv) * (long long)D * D + v;
+#pragma unroll 1
+            for (int k = 0; k < D; ++k)
+              hdst[(long long)k * D] =
+                  *reinterpret_cast<const bf16*>(smem + OFF_ST + (k >> 6) * 16384 + sw128_offset(v, k & 63));
           }
         }
       }
       // off the chain: decay in place, needed only by the state update at the end of the chunk
-      ok = WAIT(FULL0 + s, (it >> 1) & 1);
-      if (!ok) break;
+      WAIT(FULL0 + s, (it >> 1) & 1);
       if (v == 0) FQLA_TRACE(0, 3);
       const float gl = vec[(it & 3) * VEC_SLOT_FLOATS + V_GL * CHUNK];
-      constexpr int N = 2 / ROUNDS;  // pieces of 32 columns a round
 #pragma unroll 1
-      for (int k0 = 0; k0 < D; k0 += 32 * N) {
-        float x[N][32];
-#pragma unroll
-        for (int i = 0; i < N; ++i) tmem_ld32(tmem + lane_sel + TM_S + k0 + 32 * i, x[i]);
+      for (int k0 = 0; k0 < D; k0 += 32) {
+        float x[32];
+        tmem_ld32(tmem + lane_sel + TM_S + k0, x);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) x[i][j] *= gl;
-        }
-#pragma unroll
-        for (int i = 0; i < N; ++i) tmem_st32(tmem + lane_sel + TM_S + k0 + 32 * i, x[i]);
+        for (int j = 0; j < 32; ++j) x[j] *= gl;
+        tmem_st32(tmem + lane_sel + TM_S + k0, x);
       }
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&bars[S_DEC]);
       if (v == 0) FQLA_TRACE(0, 4);
-     }
-      if constexpr (!STATE) {
-        if (it + 1 < n_it) ok = scale_a(it + 1);
-      }
-      if (v == 0) FQLA_TRACE(0, 5);
     }
-    if (ok && n_it > 0) ok = WAIT(S_DONE, (n_it - 1) & 1);
+    if (tries > 0 && n_it > 0) WAIT(S_DONE, (n_it - 1) & 1);
     const int ht_row = p.ht_row && !m_pass ? p.ht_row[n] : n;
     float* end = m_pass ? p.M : p.ht;
-    if (ok && end && ht_row >= 0) {
+    if (tries > 0 && end && ht_row >= 0) {
       float* dst = end + ((long long)ht_row * p.Hv + hv) * D * D;
       tc_fence_after();
 #pragma unroll 1
@@ -523,10 +478,9 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     // operands in tensor memory.
     const int v = (warp & 3) * 32 + lane;  // tensor-memory lane = value index
     const int t0 = warp < 12 ? 0 : 32;
-    for (int it = 0; it < n_it && ok; ++it) {
+    for (int it = 0; it < n_it && more(); ++it) {
       const int s = it & 1;
-      ok = WAIT(FULL0 + s, (it >> 1) & 1);
-      if (!ok) break;
+      WAIT(FULL0 + s, (it >> 1) & 1);
       const float* vs = vec + (it & 3) * VEC_SLOT_FLOATS + t0;
       // off the chain: beta V^T, this thread's value index of its 32 tokens, and -beta gamma
       const unsigned char* vt = smem + OFF_STAGE + s * STAGE_BYTES + 2 * TILE_QK + (v >> 6) * 8192;
@@ -539,15 +493,14 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       load32(vs + V_BG * CHUNK, f);
 #pragma unroll
       for (int j = 0; j < 32; ++j)
-        y[j] *= __bfloat162float(*reinterpret_cast<const bf16*>(vt + sw128_offset(t0 + j, v & 63)));
-      ok = WAIT(U_DONE, it & 1);
-      if (!ok) break;
+        y[j] = __fmul_rn(y[j], __bfloat162float(*reinterpret_cast<const bf16*>(vt + sw128_offset(t0 + j, v & 63))));
+      WAIT(U_DONE, it & 1);
       tc_fence_after();
       tmem_ld32(tmem + lane_sel + TM_U + t0, x);
       tmem_ld_wait();
       uint32_t pk[16];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) y[j] += f[j] * x[j];
+      for (int j = 0; j < 32; ++j) y[j] = __fmaf_rn(f[j], x[j], y[j]);
 #pragma unroll
       for (int i = 0; i < 16; ++i) pk[i] = pack_bf16(y[2 * i], y[2 * i + 1]);
       tmem_st16(tmem + lane_sel + TM_WB + (t0 >> 1), pk);
@@ -561,8 +514,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         y[2 * i] = f[2 * i] * (y[2 * i] - __uint_as_float(pk[i] << 16));
         y[2 * i + 1] = f[2 * i + 1] * (y[2 * i + 1] - __uint_as_float(pk[i] & 0xffff0000u));
       }
-      ok = WAIT(VN_DONE, it & 1);
-      if (!ok) break;
+      WAIT(VN_DONE, it & 1);
       tc_fence_after();
       tmem_ld32(tmem + lane_sel + TM_VN + t0, x);
       tmem_ld_wait();
@@ -579,44 +531,33 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     const int v = tid - 256;  // tensor-memory lane: value index for Vn^T, key index for w^T
     // w^T of chunk `it` (tensor memory, [k][tok]) -> bf16 operand tile, row k = 64 tokens
     auto convert_w = [&](int it) {
-      if (!WAIT(W_DONE, it & 1)) return false;
+      WAIT(W_DONE, it & 1);
       tc_fence_after();
       unsigned char* row = smem + OFF_W + v * 128;
-      constexpr int N = 2 / ROUNDS;  // pieces of 32 columns a round
 #pragma unroll 1
-      for (int h = 0; h < 2; h += N) {
-        float x[N][32];
-#pragma unroll
-        for (int i = 0; i < N; ++i) tmem_ld32(tmem + lane_sel + TM_PW + 32 * (h + i), x[i]);
+      for (int h = 0; h < 8; h += 4) {  // 32 tokens, four 16-byte pieces per round
+        float x[32];
+        tmem_ld32(tmem + lane_sel + TM_W + 8 * h, x);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < N; ++i)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float* y = x[i] + 8 * c;
-            *reinterpret_cast<uint4*>(row + (((4 * (h + i) + c) ^ (v & 7)) << 4)) =
-                make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
-          }
+        for (int c = 0; c < 4; ++c)
+          *reinterpret_cast<uint4*>(row + (((h + c) ^ (v & 7)) << 4)) =
+              make_uint4(pack_bf16(x[8 * c], x[8 * c + 1]), pack_bf16(x[8 * c + 2], x[8 * c + 3]),
+                         pack_bf16(x[8 * c + 4], x[8 * c + 5]), pack_bf16(x[8 * c + 6], x[8 * c + 7]));
       }
       tc_fence_before();
       fence_proxy_async();
       mbar_arrive(&bars[W_READY]);
-      return true;
     };
 #pragma unroll 1
-    for (int it = -1; it < n_it && ok; ++it) {  // it = -1: only w^T of the first iteration
+    for (int it = -1; it < n_it && more(); ++it) {  // it = -1: only w^T of the first iteration
      if (it >= 0) {
       const int c = it - lead;
-      const long long row0 = sp.bos + (long long)c * CHUNK;
-      const int valid = c < 0 ? 0 : min(CHUNK, sp.len - c * CHUNK);  // 0: nothing is stored
       if (v == 0) FQLA_TRACE(1, 0);
-      ok = WAIT(FULL0 + (it & 1), (it >> 1) & 1) && WAIT(VN_DONE, it & 1);
-      if (!ok) break;
+      WAIT(FULL0 + (it & 1), (it >> 1) & 1);
+      WAIT(VN_DONE, it & 1);
       // the output product that reads Vn^T of the chunk before is issued by the other thread
-      if (!NO_O && c >= 1 && !WAIT(O_DONE, (c - 1) & 1)) {
-        ok = false;
-        break;
-      }
+      if (!NO_O && c >= 1) WAIT(O_DONE, (c - 1) & 1);
       tc_fence_after();
       if (v == 0) FQLA_TRACE(1, 1);
       const float* rho = vec + (it & 3) * VEC_SLOT_FLOATS + V_RHO * CHUNK;
@@ -626,58 +567,58 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       for (int t0 = 0; t0 < CHUNK; t0 += 32) {
         float x[32];
         tmem_ld32(tmem + lane_sel + TM_UV + t0, x);
+        float4 r[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = *reinterpret_cast<const float4*>(rho + t0 + 4 * i);
         tmem_ld_wait();
         uint32_t pr[16], pn[16];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const float4 r = *reinterpret_cast<const float4*>(rho + t0 + 4 * i);
-          pr[2 * i] = pack_bf16(r.x * x[4 * i], r.y * x[4 * i + 1]);
-          pr[2 * i + 1] = pack_bf16(r.z * x[4 * i + 2], r.w * x[4 * i + 3]);
+          pr[2 * i] = pack_bf16(r[i].x * x[4 * i], r[i].y * x[4 * i + 1]);
+          pr[2 * i + 1] = pack_bf16(r[i].z * x[4 * i + 2], r[i].w * x[4 * i + 3]);
           pn[2 * i] = pack_bf16(x[4 * i], x[4 * i + 1]);
           pn[2 * i + 1] = pack_bf16(x[4 * i + 2], x[4 * i + 3]);
         }
         tmem_st16(tmem + lane_sel + TM_VRB + (t0 >> 1), pr);
         tmem_st16(tmem + lane_sel + TM_VNB + (t0 >> 1), pn);
-        if constexpr (EXTRA) {
-          if (p.vnew && c >= 0) {
-            if (p.tiled) {  // the tile of the TMA store (the store of the chunk before has read it)
-              unsigned char* row = smem + OFF_VNT + v * 128;
-#pragma unroll
-              for (int q4 = 0; q4 < 4; ++q4)
-                *reinterpret_cast<uint4*>(row + ((((t0 >> 3) + q4) ^ (v & 7)) << 4)) =
-                    make_uint4(pn[4 * q4], pn[4 * q4 + 1], pn[4 * q4 + 2], pn[4 * q4 + 3]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (t0 + j < valid)
-                  p.vnew[((row0 + t0 + j) * p.Hv + hv) * D + v] = __float2bfloat16(x[j]);
-            }
-          }
-        }
       }
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(&bars[VB_READY]);
       if (v == 0) FQLA_TRACE(1, 2);
       if constexpr (EXTRA) {
-        if (tile_vn && c >= 0) {
-          fence_proxy_async();
-          mbar_arrive(&bars[VN_READY]);
+        // off the chain: v_new as an output, from the operand copy (the store of the chunk before has
+        // read the tile: the thread that issued this chunk's Vn^T waited for it)
+        if (p.vnew && c >= 0) {
+          unsigned char* row = smem + OFF_VNT + v * 128;
+          float x[32];
+          tmem_ld32(tmem + lane_sel + TM_VNB, x);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            *reinterpret_cast<float4*>(row + ((q ^ (v & 7)) << 4)) =
+                make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+          if (p.tiled) {
+            fence_proxy_async();
+            mbar_arrive(&bars[VN_READY]);
+          } else {  // row-major [row][v]: column v, from this thread's own row
+            const long long row0 = sp.bos + (long long)c * CHUNK;
+            const int valid = min(CHUNK, sp.len - c * CHUNK);
+            bf16* dst = p.vnew + (row0 * p.Hv + hv) * D + v;
+#pragma unroll 1
+            for (int j = 0; j < valid; ++j)
+              dst[(long long)j * p.Hv * D] = *reinterpret_cast<const bf16*>(smem + OFF_VNT + sw128_offset(v, j));
+          }
         }
       }
      }
-      if (it + 1 < n_it) ok = convert_w(it + 1);
+      if (it + 1 < n_it) convert_w(it + 1);
       if (v == 0) FQLA_TRACE(1, 3);
     }
-  } else if (warp >= 12) {
+  } else if (!NO_O && warp >= 12 && warp < 16) {
     // =============================== O group ===============================
-    // Per chunk: the epilogue of the chunk before, then Pg of this chunk.
-    // P is an M = 64 accumulator read with the 16-lane shape: lane l of warp q owns rows
-    // 16q + l/4 and 16q + l/4 + 8, and in every group of 8 columns the pair 2*(l%4), +1.
     const int wq = warp & 3;
     const int v = tid - 384;
-    const int row_a = 16 * wq + (lane >> 2), row_b = row_a + 8, cp = 2 * (lane & 3);
-    const uint32_t lanes_p = (uint32_t)(wq * 32) << 16;  // P: lanes 0-15 of the quarter
     // c counts the chunks of the sequence itself; the lead-in chunks (iterations j < lead) have no
     // output products, so the barriers of this group's products are phased by c, while stages and
     // vector slots follow the iteration j = c + lead
@@ -697,38 +638,37 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       // 8 i + 2 (l%4), +1.  stmatrix with .trans writes each 8 x 8 fragment block transposed, i.e.
       // as eight 16-byte pieces "8 value indices of one token": the tile comes out token-major
       // without a single shuffle.
+      // Rounds of 16 lanes (value indices) x 32 tokens.
       const int l4 = lane & 3, mtx = lane >> 3, r8 = lane & 7;
-      float2 sgv[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) sgv[i] = *reinterpret_cast<const float2*>(sg + 8 * i + 2 * l4);
 #pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        if (v == 0) FQLA_TRACE(2, h ? 7 : 5);
-        const uint32_t lanes = (uint32_t)(wq * 32 + 16 * h) << 16;
-        float a[32], b[32];
-        tmem_ld_16x64(tmem + lanes + TM_O1, a);
-        tmem_ld_16x64(tmem + lanes + TM_O2, b);
+      for (int h = 0; h < 4; ++h) {
+        const int t0 = 32 * (h & 1);
+        const uint32_t at = tmem + ((uint32_t)(wq * 32 + 8 * (h & 2)) << 16) + (uint32_t)t0;
+        float a[16], b[16];
+        tmem_ld_16x32(at + TM_O1, a);
+        tmem_ld_16x32(at + TM_O2, b);
+        float2 s2[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s2[i] = *reinterpret_cast<const float2*>(sg + t0 + 8 * i + 2 * l4);
         tmem_ld_wait();
-        if (v == 0) FQLA_TRACE(2, h ? 8 : 6);
-        if (h == 1) {  // all tensor-memory reads of this chunk's output are done
+        if (h == 3) {  // all tensor-memory reads of this chunk's output are done
           tc_fence_before();
           mbar_arrive(&bars[O_FREE]);
         }
         // this lane supplies the address of row r8 of matrix mtx of every store: matrices 0, 1 are
         // the two 8-row blocks of token block i, matrices 2, 3 those of token block i + 1
-        const int pv = ((wq & 1) * 32 + 16 * h) >> 3;  // 16-byte piece of rows 0-7 inside the box
+        const int pv = (wq & 1) * 4 + (h & 2);  // 16-byte piece of rows 0-7 inside the box
         const uint32_t base = s32(smem + OFF_O + (wq >> 1) * 8192) +
-                              (uint32_t)((8 * (mtx >> 1) + r8) * 128 + (((pv + (mtx & 1)) ^ r8) << 4));
+                              (uint32_t)((t0 + 8 * (mtx >> 1) + r8) * 128 + (((pv + (mtx & 1)) ^ r8) << 4));
 #pragma unroll
-        for (int i = 0; i < 8; i += 2) {
+        for (int i = 0; i < 4; i += 2) {
           uint32_t w[4];
 #pragma unroll
           for (int z = 0; z < 2; ++z) {
-            const float2 s2 = sgv[i + z];
             const float* aa = a + 4 * (i + z);
             const float* bb = b + 4 * (i + z);
-            w[2 * z] = pack_out<O_F16>(s2.x * aa[0] + bb[0], s2.y * aa[1] + bb[1]);
-            w[2 * z + 1] = pack_out<O_F16>(s2.x * aa[2] + bb[2], s2.y * aa[3] + bb[3]);
+            w[2 * z] = pack_out<O_F16>(s2[i + z].x * aa[0] + bb[0], s2[i + z].y * aa[1] + bb[1]);
+            w[2 * z + 1] = pack_out<O_F16>(s2[i + z].x * aa[2] + bb[2], s2[i + z].y * aa[3] + bb[3]);
           }
           stmatrix_x4_trans(base + (uint32_t)(i * 1024), w[0], w[1], w[2], w[3]);
         }
@@ -752,74 +692,111 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         }
       }
     };
-    const float log2_scale = log2f(p.scale);
-    // every part appears once (the kernel streams its code through a shared instruction cache):
-    // j = n_it only writes out the last chunk
 #pragma unroll 1
-    for (int j = max(lead, 0); !NO_O && j <= n_it && n_it > 0 && ok; ++j) {
-      const int it = j - lead;  // chunk of the sequence
-      // the epilogue of the chunk before first: the issuing thread needs its accumulators free
-      // (O_FREE) for this chunk's first output product
-      if (it > 0) {
-        ok = WAIT(O_DONE, (it - 1) & 1);
-        if (!ok) break;
-        tc_fence_after();
-        epilogue(it - 1);
+    for (int c = max(-lead, 0); c < n_it - lead && more(); ++c) {
+      if (v == 0) { const int it = c + lead; FQLA_TRACE(2, 0); }
+      WAIT(O_DONE, c & 1);
+      if (tries <= 0) break;  // nothing is stored of what is not complete
+      tc_fence_after();
+      if (v == 0) { const int it = c + lead; FQLA_TRACE(2, 1); }
+      epilogue(c);
+      if (v == 0) { const int it = c + lead; FQLA_TRACE(2, 2); }
+    }
+    if (wq == 0 && elect_one()) tma_store_wait_all();
+    // rows of o past the end of the last packed sequence come out zero
+    if (p.o && p.lay.cu.ptr && n == p.N - 1) {
+      const long long end = sp.bos + sp.len;
+#pragma unroll 1
+      for (long long i = tid - 384; i < (p.T_rows - end) * 16; i += 128)
+        *reinterpret_cast<uint4*>(p.o + ((end + (i >> 4)) * p.Hv + hv) * D + (i & 15) * 8) =
+            make_uint4(0, 0, 0, 0);
+    }
+  } else if (!STATE && warp >= PREP && warp < PREP + 4) {
+    // =============================== prep group ===============================
+    // A' = A diag(beta), A'' = A diag(beta gamma) of the next chunk, then Pg of this one.
+    const int v = tid - 32 * PREP, wq = warp & 3;
+    // A', A'': thread t owns the 8 columns 8 (t%8) .. of the rows t/8 + 16 i: its 16 scale factors stay in
+    // registers, and the eight threads of a row touch the eight 16-byte pieces of that row (one 128-byte line
+    // per access, conflict-free).
+    const int c8 = v & 7, r0 = v >> 3;
+    // Pg: P is an M = 64 accumulator read with the 16-lane shape: lane l of warp q owns rows
+    // 16q + l/4 and 16q + l/4 + 8, and in every group of 8 columns the pair 2*(l%4), +1.
+    const int row_a = 16 * wq + (lane >> 2), row_b = row_a + 8, cp = 2 * (lane & 3);
+    const uint32_t lanes_p = (uint32_t)(wq * 32) << 16;  // lanes 0-15 of the quarter
+    const float log2_scale = log2f(p.scale);
+#pragma unroll 1
+    for (int it = -1; it < n_it && more(); ++it) {  // it = -1: only A of the first iteration
+      if (v == 0) FQLA_TRACE(2, 3);
+      if (it + 1 < n_it) {
+        const int j = it + 1, sj = j & 1;
+        WAIT(FULLA0 + sj, (j >> 1) & 1);
+        if (j > 0) WAIT(U_DONE, (j - 1) & 1);  // u of the chunk before, and w ahead of it, are done
+        const float* vs = vec + (j & 3) * VEC_SLOT_FLOATS + 8 * c8;
+        const float4 b0 = *reinterpret_cast<const float4*>(vs + V_BETA * CHUNK);
+        const float4 b1 = *reinterpret_cast<const float4*>(vs + V_BETA * CHUNK + 4);
+        const float4 g0 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK);
+        const float4 g1 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 4);
+        // physical piece: rows r0 + 16 i all have (row & 7) == r0 & 7
+        unsigned char* dst = smem + OFF_AP + r0 * 128 + (c8 ^ (r0 & 7)) * 16;
+        const unsigned char* src = dst + (OFF_STAGE + 2 * TILE_QK + TILE_V - OFF_AP) + sj * STAGE_BYTES;
+        uint4 next = *reinterpret_cast<const uint4*>(src);
+#pragma unroll 1
+        for (int i = 0; i < 4 * 2048; i += 2048) {
+          const uint4 a = next;
+          next = *reinterpret_cast<const uint4*>(src + ((i + 2048) & 0x1fff));
+          *reinterpret_cast<uint4*>(dst + i) =
+              make_uint4(scale_bf16x2(a.x, b0.x, b0.y), scale_bf16x2(a.y, b0.z, b0.w),
+                         scale_bf16x2(a.z, b1.x, b1.y), scale_bf16x2(a.w, b1.z, b1.w));
+          *reinterpret_cast<uint4*>(dst + (OFF_APP - OFF_AP) + i) =
+              make_uint4(scale_bf16x2(a.x, g0.x, g0.y), scale_bf16x2(a.y, g0.z, g0.w),
+                         scale_bf16x2(a.z, g1.x, g1.y), scale_bf16x2(a.w, g1.z, g1.w));
+        }
+        fence_proxy_async();
+        mbar_arrive(&bars[AP_READY]);
+        mbar_arrive(&bars[EMPTYA0 + sj]);  // the A tile of this stage is no longer read here
       }
-      if (j < n_it) {
-        const float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
-        ok = WAIT(FULL0 + (j & 1), (j >> 1) & 1) && WAIT(P_DONE, it & 1);
-        if (!ok) break;
+      if (v == 0) FQLA_TRACE(2, 4);
+      if (!NO_O && it >= 0 && it >= lead) {
+        const float* vs = vec + (it & 3) * VEC_SLOT_FLOATS + V_G * CHUNK;
+        WAIT(P_DONE, (it - lead) & 1);
+        if (it > lead) WAIT(O_DONE, (it - lead - 1) & 1);  // the tile of the chunk before has been read
         tc_fence_after();
-        // Pg = s P exp(g_row - g_col) = P exp2((g_row - g_col) log2e + log2 s), col <= row
-        {
-          const float ga2 = vs[V_G * CHUNK + row_a] * 1.4426950408889634f + log2_scale;
-          const float gb2 = vs[V_G * CHUNK + row_b] * 1.4426950408889634f + log2_scale;
-          float x[32];
-          tmem_ld_16x64(tmem + lanes_p + TM_PW, x);
-          tmem_ld_wait();
-          tc_fence_before();
-          unsigned char* pa = smem + OFF_P + row_a * 128 + cp * 2;
-          unsigned char* pb = smem + OFF_P + row_b * 128 + cp * 2;
-          // column groups entirely above this warp's rows stay zero (written once at start)
+        if (v == 0) FQLA_TRACE(2, 5);
+        // Pg = s P exp(g_row - g_col) = P exp2((g_row - g_col) log2e + log2 s), col <= row; 16 columns a
+        // round (column groups entirely above this warp's rows stay zero, written once at start)
+        const float ga2 = vs[row_a] * 1.4426950408889634f + log2_scale;
+        const float gb2 = vs[row_b] * 1.4426950408889634f + log2_scale;
+        unsigned char* pa = smem + OFF_P + row_a * 128 + cp * 2;  // rows b: 8 rows below, the same swizzle
+        float x[32];
+        tmem_ld_16x64(tmem + lanes_p + TM_P, x);
+        tmem_ld_wait();
+        tc_fence_before();
+        mbar_arrive(&bars[P_FREE]);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            if (i > 2 * wq + 1) continue;
-            const float2 gc = *reinterpret_cast<const float2*>(vs + V_G * CHUNK + 8 * i + cp);
-            const int col = 8 * i + cp;
-            const float e0 = -1.4426950408889634f * gc.x, e1 = -1.4426950408889634f * gc.y;
-            const float a0 = col <= row_a ? x[4 * i] * exp2f(e0 + ga2) : 0.f;
-            const float a1 = col + 1 <= row_a ? x[4 * i + 1] * exp2f(e1 + ga2) : 0.f;
-            const float b0 = col <= row_b ? x[4 * i + 2] * exp2f(e0 + gb2) : 0.f;
-            const float b1 = col + 1 <= row_b ? x[4 * i + 3] * exp2f(e1 + gb2) : 0.f;
-            *reinterpret_cast<uint32_t*>(pa + ((i ^ (row_a & 7)) << 4)) = pack_bf16(a0, a1);
-            *reinterpret_cast<uint32_t*>(pb + ((i ^ (row_b & 7)) << 4)) = pack_bf16(b0, b1);
-          }
+        for (int i = 0; i < 8; ++i) {
+          if (i > 2 * wq + 1) continue;
+          const int col = 8 * i + cp;
+          const float2 gc = *reinterpret_cast<const float2*>(vs + col);
+          const float e0 = -1.4426950408889634f * gc.x, e1 = -1.4426950408889634f * gc.y;
+          const float a0 = col <= row_a ? x[4 * i] * exp2f(e0 + ga2) : 0.f;
+          const float a1 = col + 1 <= row_a ? x[4 * i + 1] * exp2f(e1 + ga2) : 0.f;
+          const float b0 = col <= row_b ? x[4 * i + 2] * exp2f(e0 + gb2) : 0.f;
+          const float b1 = col + 1 <= row_b ? x[4 * i + 3] * exp2f(e1 + gb2) : 0.f;
+          unsigned char* at = pa + ((i ^ (row_a & 7)) << 4);
+          *reinterpret_cast<uint32_t*>(at) = pack_bf16(a0, a1);
+          *reinterpret_cast<uint32_t*>(at + 1024) = pack_bf16(b0, b1);
         }
         fence_proxy_async();
         mbar_arrive(&bars[P_READY]);
+        if (v == 96) FQLA_TRACE(2, 6);
       }
     }
-    if constexpr (!NO_O) {
-      if (wq == 0 && elect_one()) tma_store_wait_all();
-      // rows of o past the end of the last packed sequence come out zero
-      if (p.o && p.lay.cu.ptr && n == p.N - 1) {
-        const long long end = sp.bos + sp.len;
-#pragma unroll 1
-        for (long long i = tid - 384; i < (p.T_rows - end) * 16; i += 128)
-          *reinterpret_cast<uint4*>(p.o + ((end + (i >> 4)) * p.Hv + hv) * D + (i & 15) * 8) =
-              make_uint4(0, 0, 0, 0);
-      }
-    }
-  } else if (warp == 0 || warp == 1) {
+  } else if (warp == 0 || warp == 1 || (!STATE && warp == 3)) {
     // =============================== MMA issuers ===============================
-    // Two warps issue, each with its own waits and, from one elected lane, its own products and
-    // tcgen05.commit (a commit covers the MMAs of the committing thread only):
-    //   warp 0, the chain: Vn^T and the state update, nothing else: twelve MMAs per chunk;
-    //   warp 1, everything off the chain: P, O1^T, O2^T and u^T / w^T of the next chunk.  It is the
-    //           one that waits for the output group, so the chain never stands behind an epilogue.
-    // The tensor pipe runs products in issue order whoever issued them; the extra barriers
-    // (SB_FREE, the O_DONE wait of the value group) cover what one thread's program order would.
+    // Three warps issue, each with its own waits and, from one elected lane, its own products and
+    // tcgen05.commit (a commit covers the MMAs of the committing thread only).  The tensor pipe runs products
+    // in the order in which they come, whoever issued them: what is off the chain is issued behind the
+    // chain's product of the moment and runs while the read-out groups work on that one's result.
     constexpr uint32_t ID_P = idesc_bf16(64, 64, 0, 0);
     constexpr uint32_t ID_UT = idesc_bf16(128, 64, 1, 0);            // A = V / K tile, MN-major
     constexpr uint32_t ID_VN = idesc_bf16(128, 64, 0, 1) | (1u << 13);  // A negated; B = w^T tile
@@ -827,24 +804,23 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     constexpr uint32_t ID_S = idesc_bf16(128, 128, 0, 1);
     constexpr uint32_t STAGE_LO = STAGE_BYTES >> 4;
     if constexpr (STATE) {
-      auto SPIN = [&](int idx, uint32_t parity) { return mbar_wait_warp<true>(&bars[idx], parity, abort_flag); };
       const uint32_t k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE_QK);
       const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE_QK, 8192);
       const uint32_t a0_lo = desc_lo_kmajor(smem + OFF_STAGE + 2 * TILE_QK + TILE_V);
 #pragma unroll 1
-      for (int it = 0; it < n_it && ok && warp == 0; ++it) {
+      for (int it = 0; it < n_it && warp == 0 && more(); ++it) {
         const int s = it & 1, ph = (it >> 1) & 1;
         const uint32_t so = s ? STAGE_LO : 0u;
-        ok = SPIN(FULL0 + s, ph) && SPIN(S_COPY, it & 1);
-        if (!ok) break;
+        WAIT(FULL0 + s, ph);
+        WAIT(S_COPY, it & 1);
         tc_fence_after();
         if (elect_one()) {
           // U^T = S^T K^T   (A = packed S^T; B = K tile, K-major)
           umma_ts_group_kmajor_b<8>(tmem + TM_U, tmem + TM_SB, k0_lo + so, ID_OT);
           umma_commit(&bars[U_DONE]);
         }
-        ok = SPIN(FULLA0 + s, ph) && SPIN(WB_READY, it & 1);
-        if (!ok) break;
+        WAIT(FULLA0 + s, ph);
+        WAIT(WB_READY, it & 1);
         tc_fence_after();
         if (elect_one()) {
           // Vn^T = W^T A^T   (A = packed W^T; B = A tile, K-major)
@@ -852,8 +828,8 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           umma_commit(&bars[VN_DONE]);
           umma_commit(&bars[EMPTYA0 + s]);
         }
-        ok = SPIN(VB_READY, it & 1) && SPIN(S_DEC, it & 1);
-        if (!ok) break;
+        WAIT(VB_READY, it & 1);
+        WAIT(S_DEC, it & 1);
         tc_fence_after();
         if (elect_one()) {
           // S^T += (rho Vn)^T K
@@ -863,19 +839,17 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         }
       }
     } else if (warp == 0) {
-      auto SPIN = [&](int idx, uint32_t parity) { return mbar_wait_warp<true>(&bars[idx], parity, abort_flag); };
-      auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
       // low descriptor words of every operand tile (see umma_lo); steps are 32-bit adds
       const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 16384);
       const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE_QK, 8192);
 #pragma unroll 1
-      for (int it = 0; it < n_it && ok; ++it) {
+      for (int it = 0; it < n_it && more(); ++it) {
         const int s = it & 1, c = it - lead;  // c < 0: lead-in chunk
         const uint32_t so = s ? STAGE_LO : 0u;
         if (lane == 0) FQLA_TRACE(3, 0);
-        if (lane == 0 && it < 126) FQLA_CHUNK_CLOCK(it);
-        ok = SPIN(S_COPY, it & 1) && SPIN(W_READY, it & 1);
-        if (!ok) break;
+        WAIT(U_DONE, it & 1);
+        WAIT(W_READY, it & 1);
+        WAIT(S_COPY, it & 1);
         tc_fence_after();
         if (lane == 0) FQLA_TRACE(3, 1);
         if (elect_one()) {
@@ -887,8 +861,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         if (lane == 0) FQLA_TRACE(3, 2);
         if constexpr (EXTRA) {
           if (tile_h && c >= 0) {  // the state entering this chunk, as an operand tile
-            ok = WAITW(ST_READY, c & 1);
-            if (!ok) break;
+            WAIT(ST_READY, c & 1);
             if (elect_one()) {
               const int y = (int)(((sp.chunk_base + c) * p.Hv + hv) * D);
               tma_store_2d(&map_h, 0, y, smem + OFF_ST);
@@ -898,8 +871,8 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           }
         }
         if (lane == 0) FQLA_TRACE(3, 3);
-        ok = SPIN(VB_READY, it & 1) && SPIN(S_DEC, it & 1);
-        if (!ok) break;
+        WAIT(VB_READY, it & 1);
+        WAIT(S_DEC, it & 1);
         tc_fence_after();
         if (lane == 0) FQLA_TRACE(3, 4);
         if (elect_one()) {
@@ -912,8 +885,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         if (lane == 0) FQLA_TRACE(3, 5);
         if constexpr (EXTRA) {
           if (tile_vn && c >= 0) {
-            ok = WAITW(VN_READY, c & 1);
-            if (!ok) break;
+            WAIT(VN_READY, c & 1);
             if (elect_one()) {  // the v_new^T tile is complete
               tma_store_2d(&map_vn, 0, (int)(((sp.chunk_base + c) * p.Hv + hv) * D), smem + OFF_VNT);
               tma_store_commit();
@@ -925,86 +897,90 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       if constexpr (EXTRA) {
         if (elect_one()) tma_store_wait_all();
       }
-    } else {
-      auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
+    } else if (warp == 1) {
       const uint32_t p_lo = desc_lo_kmajor(smem + OFF_P);
       const uint32_t q0_lo = desc_lo_kmajor(smem + OFF_STAGE);
       const uint32_t k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE_QK);
-      const uint32_t ap_lo = desc_lo_kmajor(smem + OFF_AP), app_lo = desc_lo_kmajor(smem + OFF_APP);
-      const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE_QK, 8192);
-      const uint32_t vmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + 2 * TILE_QK, 8192);
-      // u^T and w^T of iteration j (so = its stage's offset in descriptor units).  u^T overwrites Vn^T
-      // (read by the value group), w^T overwrites P (read by the output group): the waits below.
-      auto issue_u_w = [&](uint32_t so) {
-        if (elect_one()) {
-          umma_group<4, 128, 0, 2, 0, false>(tmem + TM_UV, vmn0_lo + so, ap_lo, ID_UT);
-          umma_group<4, 128, 0, 2, 0, false>(tmem + TM_PW, kmn0_lo + so, app_lo, ID_UT);
-          umma_commit(&bars[W_DONE]);
-        }
-      };
+      // (what is waited for by iteration is waited for in a lead-in, too: a parity tells a phase from its
+      // neighbours only)
 #pragma unroll 1
-      for (int it = -1; it < n_it && ok; ++it) {  // it = -1: only u^T, w^T of the first iteration
+      for (int it = 0; it < n_it && more(); ++it) {
         const int s = it & 1, c = it - lead;
-        const uint32_t so = s ? STAGE_LO : 0u, so_next = s ? 0u : STAGE_LO;
-        const bool with_o = !NO_O && c >= 0 && it >= 0;
+        const uint32_t so = s ? STAGE_LO : 0u;
+        const bool with_o = !NO_O && c >= 0;
+        if (lane == 0) FQLA_TRACE(4, 0);
+        WAIT(FULL0 + s, (it >> 1) & 1);
+        WAIT(W_READY, it & 1);
+        // P = Q K^T, over w^T; the prep group turns it into Pg
         if (with_o) {
-          // P = Q K^T goes first: the output group turns it into Pg while everything else runs.
-          // Its columns held w^T of this chunk until the value group made the operand tile of it.
-          ok = WAITW(W_READY, it & 1);
-          if (!ok) break;
           tc_fence_after();
+          if (lane == 0) FQLA_TRACE(4, 1);
           if (elect_one()) {
-            umma_group<8, 2, 512, 2, 512, false>(tmem + TM_PW, q0_lo + so, k0_lo + so, ID_P);
+            umma_loop<2, 2, 512, 2, 512>(tmem + TM_P, q0_lo + so, k0_lo + so, ID_P);
             umma_commit(&bars[P_DONE]);
           }
-          // O1^T = S^T Q^T   (A = packed S^T; B = q tile, K-major)
-          ok = WAITW(S_COPY, it & 1) && (c == 0 || WAITW(O_FREE, (c - 1) & 1));
-          if (!ok) break;
+        }
+        // O1^T = S^T Q^T   (A = packed S^T; B = q tile, K-major), behind Vn^T of the chain
+        if (lane == 0) FQLA_TRACE(4, 2);
+        WAIT(VN_DONE, it & 1);
+        if (with_o) {
+          if (c > 0) WAIT(O_FREE, (c - 1) & 1);
           tc_fence_after();
+          if (lane == 0) FQLA_TRACE(4, 3);
           if (elect_one()) {
-            umma_ts_group_kmajor_b<8>(tmem + TM_O1, tmem + TM_SB, q0_lo + so, ID_OT);
+            umma_ts_loop8<2, 512, false>(tmem + TM_O1, tmem + TM_SB, q0_lo + so, ID_OT);
             umma_commit(&bars[SB_FREE]);
           }
         }
-        // this thread's products that read the stage (u^T, w^T of this chunk, issued a chunk ago,
-        // and the two above) are all issued
-        if (it >= 0 && elect_one()) umma_commit(&bars[EMPTY0 + s]);
+        if (elect_one()) umma_commit(&bars[EMPTY0 + s]);  // this thread's products that read the stage
+        if (lane == 0) FQLA_TRACE(4, 4);
+        WAIT(VB_READY, it & 1);
+        // O2^T = Vn^T Pg^T   (A = packed Vn^T; B = Pg, K-major)
         if (with_o) {
-          // O2^T = Vn^T Pg^T   (A = packed Vn^T; B = Pg, K-major)
-          ok = WAITW(P_READY, c & 1) && WAITW(VB_READY, it & 1);
-          if (!ok) break;
+          WAIT(P_READY, c & 1);
           tc_fence_after();
+          if (lane == 0) FQLA_TRACE(4, 5);
           if (elect_one()) {
             umma_ts_group<4, 8, 2, false>(tmem + TM_O2, tmem + TM_VNB, p_lo, ID_OT);
             umma_commit(&bars[O_DONE]);
           }
         }
-        if (it + 1 < n_it) {
-          ok = WAITW(FULL0 + (s ^ 1), ((it + 1) >> 1) & 1) && WAITW(AP_READY, (it + 1) & 1) &&
-               (it < 0 || WAITW(VB_READY, it & 1));
-          if (!ok) break;
-          tc_fence_after();
-          issue_u_w(so_next);
+        if (lane == 0) FQLA_TRACE(4, 6);
+      }
+    } else {
+      // w^T of iteration it + 1, behind Vn^T of iteration `it`, which stands on the chain (and for which w^T of
+      // `it` has been made an operand), and behind Pg, made of P in the same columns.
+      const uint32_t ap_lo = desc_lo_kmajor(smem + OFF_AP), app_lo = desc_lo_kmajor(smem + OFF_APP);
+      const uint32_t vmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + 2 * TILE_QK, 8192);
+      const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE_QK, 8192);
+#pragma unroll 1
+      for (int it = -1; it + 1 < n_it && more(); ++it) {
+        const int s = (it + 1) & 1;
+        WAIT(FULL0 + s, ((it + 1) >> 1) & 1);
+        WAIT(AP_READY, (it + 1) & 1);
+        if (it >= 0) WAIT(VN_DONE, it & 1);
+        if (!NO_O && it >= 0 && it >= lead) WAIT(P_FREE, (it - lead) & 1);
+        tc_fence_after();
+        if (lane == 0) FQLA_TRACE(5, 0);
+        if (elect_one()) {
+          umma_group<4, 128, 0, 2, 0, false>(tmem + TM_W, kmn0_lo + (s ? STAGE_LO : 0u), app_lo, ID_UT);
+          umma_commit(&bars[W_DONE]);
         }
+        if (lane == 0) FQLA_TRACE(5, 1);
+        // u^T over Vn^T, which has been read, behind the state update
+        if (it >= 0) WAIT(S_DONE, it & 1);
+        tc_fence_after();
+        if (lane == 0) FQLA_TRACE(5, 2);
+        if (elect_one()) {
+          umma_group<4, 128, 0, 2, 0, false>(tmem + TM_UV, vmn0_lo + (s ? STAGE_LO : 0u), ap_lo, ID_UT);
+          umma_commit(&bars[U_DONE]);
+          umma_commit(&bars[EMPTY0 + s]);
+        }
+        if (lane == 0) FQLA_TRACE(5, 3);
       }
     }
   } else if (warp == 2) {
     // =============================== producer ===============================
-    float g_r[2] = {0.f, 0.f}, b_r[2] = {0.f, 0.f}, gl_r = 0.f;
-    // (lead-in chunks, c < 0, are whole chunks of the rows before the sequence)
-    auto fetch = [&](int it) {
-      const int c = it - lead;
-      const long long row0 = sp.bos + (long long)c * CHUNK;
-      const int valid = c < 0 ? CHUNK : min(CHUNK, sp.len - c * CHUNK);
-      gl_r = p.g[(row0 + valid - 1) * p.Hv + hv];
-#pragma unroll
-      for (int z = 0; z < 2; ++z) {
-        int r = 2 * lane + z, rc = min(r, valid - 1);
-        g_r[z] = p.g[(row0 + rc) * p.Hv + hv];
-        b_r[z] = r < valid ? load_beta(p.beta, p.beta_is_f32, (row0 + r) * p.Hv + hv) : 0.f;
-      }
-    };
-    auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
     // zero the rows past the sequence end in n 8 KB blocks of 64 rows (they belong to the next
     // sequence), then hand the tile on
     auto zero_rows = [&](unsigned char* base, int n, int valid, uint64_t* full) {
@@ -1019,17 +995,15 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     // its q, k, v (whose stage is still in use, but the prep warps can start on A early); the gates
     // of chunk it + 2 into registers.  (Slot (it + 1) % 4 of the vectors was last read for chunk
     // it - 3, which the wait on the stage of chunk it - 2 has seen finished.)
+    float g_r[2] = {0.f, 0.f}, b_r[2] = {0.f, 0.f}, gl_r = 0.f;
 #pragma unroll 1
-    for (int it = -2; it < n_it && ok; ++it) {
+    for (int it = -2; it < n_it && more(); ++it) {
       if (it >= 0) {
         const int s = it & 1, c = it - lead;
-        const int y = (int)(sp.bos + (long long)c * CHUNK);
+        const int y = (int)sp.bos + c * CHUNK;
         const int valid = c < 0 ? CHUNK : min(CHUNK, sp.len - c * CHUNK);
         const bool with_q = !NO_O && c >= 0, partial = valid < CHUNK;
-        if (it >= 2) {
-          ok = WAITW(EMPTY0 + s, ((it >> 1) - 1) & 1);
-          if (!ok) break;
-        }
+        if (it >= 2) WAIT(EMPTY0 + s, ((it >> 1) - 1) & 1);
         unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
         uint64_t* bar = &bars[partial ? PRIV : FULL0 + s];
         if (elect_one()) {
@@ -1046,8 +1020,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           }
         }
         if (partial) {
-          ok = WAITW(PRIV, 0);
-          if (!ok) break;
+          WAIT(PRIV, 0);
           zero_rows(st, 6, valid, &bars[FULL0 + s]);
         }
       }
@@ -1057,42 +1030,50 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         const int valid = c < 0 ? CHUNK : min(CHUNK, sp.len - c * CHUNK);
         const bool partial = valid < CHUNK;
         // the stage's A buffer is free once the prep warps have read it
-        if (j >= 2) {
-          ok = WAITW(EMPTYA0 + sj, ((j >> 1) - 1) & 1);
-          if (!ok) break;
-        }
-        float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
+        if (j >= 2) WAIT(EMPTYA0 + sj, ((j >> 1) - 1) & 1);
+        float* vs = vec + (j & 3) * VEC_SLOT_FLOATS + lane;
 #pragma unroll
         for (int z = 0; z < 2; ++z) {
-          int r = 2 * lane + z;
-          float gam = fast_exp(g_r[z]);
-          vs[V_G * CHUNK + r] = g_r[z];
-          vs[V_BETA * CHUNK + r] = b_r[z];
-          vs[V_BG * CHUNK + r] = STATE ? -b_r[z] * gam : b_r[z] * gam;
-          vs[V_RHO * CHUNK + r] = fast_exp(gl_r - g_r[z]);
-          vs[V_SGAM * CHUNK + r] = p.scale * gam;
+          const float gam = fast_exp(g_r[z]);
+          vs[V_G * CHUNK + 32 * z] = g_r[z];
+          vs[V_BETA * CHUNK + 32 * z] = b_r[z];
+          vs[V_BG * CHUNK + 32 * z] = STATE ? -b_r[z] * gam : b_r[z] * gam;
+          vs[V_RHO * CHUNK + 32 * z] = fast_exp(gl_r - g_r[z]);
+          vs[V_SGAM * CHUNK + 32 * z] = p.scale * gam;
         }
-        if (lane == 0) vs[V_GL * CHUNK] = fast_exp(gl_r);
+        vs[V_GL * CHUNK] = fast_exp(gl_r);
         __syncwarp();
         unsigned char* dst = smem + OFF_STAGE + sj * STAGE_BYTES + 2 * TILE_QK + TILE_V;
         uint64_t* bar = &bars[partial ? PRIVA : FULLA0 + sj];
         if (elect_one()) {
           mbar_arrive_expect_tx(bar, TILE_A);
-          tma_load_2d(dst, &map_a, hv * CHUNK, (int)(sp.bos + (long long)c * CHUNK), bar);
+          tma_load_2d(dst, &map_a, hv * CHUNK, (int)sp.bos + c * CHUNK, bar);
         }
         if (partial) {
           // only the last chunk of a sequence can be partial: the private barrier is used once
-          ok = WAITW(PRIVA, 0);
-          if (!ok) break;
+          WAIT(PRIVA, 0);
           zero_rows(dst, 1, valid, &bars[FULLA0 + sj]);
         }
       }
-      if (it + 2 < n_it) fetch(it + 2);
+      if (it + 2 < n_it) {
+        // (lead-in chunks, c < 0, are whole chunks of the rows before the sequence)
+        const int c = it + 2 - lead, last = (c < 0 ? CHUNK : min(CHUNK, sp.len - c * CHUNK)) - 1;
+        const long long at = (sp.bos + (long long)c * CHUNK) * p.Hv + hv;
+        gl_r = p.g[at + last * p.Hv];
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          const int r = lane + 32 * z;
+          const long long i = at + min(r, last) * p.Hv;
+          g_r[z] = p.g[i];
+          b_r[z] = load_beta(p.beta, p.beta_is_f32, i);
+          if (r > last) b_r[z] = 0.f;
+        }
+      }
     }
   }
 
   // ---- teardown: everybody meets, then the allocating warp frees tensor memory
-  if (!ok) *abort_flag = 1;
+  if (tries <= 0) *abort_flag = 1;
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);
@@ -1148,10 +1129,11 @@ int launch_fwd_tc(const fqla_fwd_args& a, int N, SeqLayout lay, cudaStream_t st)
   p.run_value = a.run_value; p.order = a.seq_order;
   p.M = a.M; p.warm = a.warm_chunks; p.m_mask = a.m_mask; p.m_first = INT_MAX;
   int blocks = N * a.Hv;
+  const bool no_o = !a.q && !a.o;
   auto launch = [&](auto kernel, int smem_bytes, std::atomic<unsigned long long>& done) {
     int err = configure_smem((const void*)kernel, smem_bytes, done);
     if (err != 0) return err;
-    return launch_pdl(kernel, dim3((unsigned)blocks), dim3(512), (size_t)smem_bytes, st, p, mq, mk,
+    return launch_pdl(kernel, dim3((unsigned)blocks), dim3(threads(no_o)), (size_t)smem_bytes, st, p, mq, mk,
                       mv, ma, mh, mvn, mo);
   };
   static std::atomic<unsigned long long> done[6];
@@ -1189,25 +1171,23 @@ extern "C" int fqla_debug_fwd_chunk_clock(long long* out256) {
 namespace fqla {
 // Self-test of the bounded-wait path: one thread waits on an mbarrier that nobody ever arrives
 // at, with a budget of `tries` tries.  The wait gives up, the kernel sets the device status word exactly as a product kernel does, and returns.
-__global__ void wait_timeout_selftest_kernel(uint32_t tries) {
+__global__ void wait_timeout_selftest_kernel(int tries) {
   __shared__ uint64_t bar;
-  __shared__ int abort_flag;
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
-    abort_flag = 0;
     fence_mbar_init();
   }
   __syncthreads();
-  bool ok = true;
-  if (threadIdx.x == 0) ok = mbar_wait(&bar, 0, &abort_flag, tries);
-  __syncthreads();
-  if (threadIdx.x == 0 && (!ok || abort_flag)) atomicCAS(&g_device_status, 0, 1);
+  if (threadIdx.x == 0) {
+    mbar_wait(&bar, 0, tries);
+    if (tries <= 0) atomicCAS(&g_device_status, 0, 1);
+  }
 }
 }  // namespace fqla
 
 extern "C" int fqla_selftest_wait_timeout(int tries, void* stream) {
   if (tries < 1 || tries > 100) return FQLA_ERR_INVALID_ARG;
-  fqla::wait_timeout_selftest_kernel<<<1, 32, 0, (cudaStream_t)stream>>>((uint32_t)tries);
+  fqla::wait_timeout_selftest_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(tries);
   return (int)cudaGetLastError();
 }
 

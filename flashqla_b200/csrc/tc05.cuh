@@ -79,9 +79,8 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 // instruction cache.  (A test first and then tries with a 1 ms suspend hint was 5-10 % more code
 // and woke up later: 802 against 787 us for a 262144-token forward, 2040 against 1997 us for 32768
 // packed training tokens.)
-constexpr uint32_t WAIT_TRIES = 1u << 24;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
-                                          volatile int* abort_flag, uint32_t budget = WAIT_TRIES) {
+                                          volatile int* abort_flag, uint32_t budget = 1u << 24) {
 #pragma unroll 1
   do {
     if (mbar_try_wait(bar, parity)) return true;
@@ -89,6 +88,27 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   } while (--budget);
   *abort_flag = 1;
   return false;
+}
+
+// Bounded wait.  `tries` is the thread's own count, WAIT_TRIES (about a second and more) at the start of each
+// pass of its loop; a wait that uses it up falls through, and so does every wait after it, until the loop looks
+// at the count and ends: one look a pass instead of a result at each of the dozens of wait sites, which were a
+// third of the kernels' code.  What a pass does after a wait was given up touches only the memory that it would
+// have touched anyway; its values are lost (the kernel sets its status word).  The thread is suspended by the
+// hardware meanwhile; polling with test_wait instead, or once before it, takes issue slots from the warps that
+// have work (262144-token forward recurrence: 467 us, 484 with a test at the waits that are mostly over).
+constexpr int WAIT_TRIES = 1 << 24;
+__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int& tries) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n"
+      "W%=:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra D%=;\n\t"
+      "add.s32 %0, %0, -1;\n\tsetp.gt.s32 p, %0, 0;\n\t@p bra W%=;\n"
+      "D%=:\n\t}"
+      : "+r"(tries)
+      : "r"(s32(bar)), "r"(parity)
+      : "memory");
 }
 
 // Four 8 x 8 bf16 matrices from registers to shared memory, each stored TRANSPOSED: register i of
@@ -148,7 +168,7 @@ __device__ __forceinline__ bool elect_one() {
 // 25 cycles a round) without looking at the abort flag in between, for the warp on the critical path.
 template <bool SPIN>
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  uint32_t n = WAIT_TRIES;
+  uint32_t n = 1u << 24;
 #pragma unroll 1
   do {
     if (__all_sync(0xffffffffu, SPIN ? mbar_test_wait(bar, parity) : mbar_try_wait(bar, parity))) return true;
@@ -274,6 +294,25 @@ __device__ __forceinline__ void tmem_ld_16x64(uint32_t taddr, float (&v)[32]) {
       : "r"(taddr)
       : "memory");
 }
+// The same over 32 (x4) and 16 (x2) columns.
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, float (&v)[16]) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, float (&v)[8]) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
 // 32 lanes x 16 consecutive columns -> 16 registers per thread
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t* r = reinterpret_cast<uint32_t*>(v);
@@ -389,6 +428,16 @@ __device__ __forceinline__ void umma_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t
         : "memory");
   }
 }
+// ... onto the accumulator where acc is not zero
+__device__ __forceinline__ void umma_acc(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, int acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(DESC_HI), "r"(idesc), "r"(acc)
+      : "memory");
+}
 // One product: NK K-steps; operand low words advance by A_STEP / B_STEP (units of 16 bytes) per
 // step, plus A_BLK / B_BLK after every fourth step (next 64-column block of a K-major operand).
 template <int NK, int A_STEP, int A_BLK, int B_STEP, int B_BLK, bool ACC_FIRST>
@@ -400,6 +449,19 @@ __device__ __forceinline__ void umma_group(uint32_t d_tmem, uint32_t a_lo, uint3
     const uint32_t b = b_lo + (uint32_t)((j & 3) * B_STEP + (j >> 2) * B_BLK);
     if (j == 0 && !ACC_FIRST) umma_lo<false>(d_tmem, a, b, idesc);
     else umma_lo<true>(d_tmem, a, b, idesc);
+  }
+}
+
+// The same as NB passes of a loop over four unrolled steps: the operand words advance by A_BLK / B_BLK a pass.
+template <int NB, int A_STEP, int A_BLK, int B_STEP, int B_BLK>
+__device__ __forceinline__ void umma_loop(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+#pragma unroll 1
+  for (int b = 0; b < NB; ++b) {
+    umma_acc(d_tmem, a_lo, b_lo, idesc, b);
+#pragma unroll
+    for (int j = 1; j < 4; ++j) umma_lo<true>(d_tmem, a_lo + (uint32_t)(j * A_STEP), b_lo + (uint32_t)(j * B_STEP), idesc);
+    a_lo += A_BLK;
+    b_lo += B_BLK;
   }
 }
 
@@ -428,6 +490,29 @@ __device__ __forceinline__ void umma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uin
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
         "r"(a_tmem), "r"(b_lo), "r"(DESC_HI), "r"(idesc)
         : "memory");
+  }
+}
+// Eight K-steps as two passes of a loop: B advances by B_STEP a step, by B_BLK a pass.
+template <int B_STEP, int B_BLK, bool ACC_FIRST>
+__device__ __forceinline__ void umma_ts_loop8(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc) {
+#pragma unroll 1
+  for (int b = 0; b < 2; ++b) {
+    if (ACC_FIRST) {
+      umma_ts_lo<true>(d_tmem, a_tmem, b_lo, idesc);
+    } else {
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+          "setp.ne.b32 p, %5, 0;\n\t"
+          "mov.b64 db, {%2, %3};\n\t"
+          "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
+          "r"(a_tmem), "r"(b_lo), "r"(DESC_HI), "r"(idesc), "r"(b)
+          : "memory");
+    }
+#pragma unroll
+    for (int j = 1; j < 4; ++j)
+      umma_ts_lo<true>(d_tmem, a_tmem + (uint32_t)(8 * j), b_lo + (uint32_t)(j * B_STEP), idesc);
+    a_tmem += 32;
+    b_lo += B_BLK;
   }
 }
 // NK K-steps; A advances A_COLS columns per step, B by B_STEP descriptor units (16 bytes) per step
