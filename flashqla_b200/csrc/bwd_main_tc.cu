@@ -10,7 +10,9 @@
 //     dk = rho v_new dh^T - beta gamma Y + ds^T q + (X + X^T) K
 // and dg, dbeta from row and column sums of q dq1, k dk1, k Y, v dW, ds (Q K^T), dL (K K^T).  (As the chain
 // dA = -(du h^T) (beta gamma K)^T + du (beta V)^T, dL = -A^T dA A^T it was sixteen products and six
-// read-outs in a row instead of eleven and three: 262144 tokens x 8 heads 1471 us, now 1340 to 1358.)
+// read-outs in a row instead of eleven and three: 262144 tokens x 8 heads 1471 -> 1340 us.  With waits that pause
+// between two tries (mbar_wait in tc05.cuh) 1260 to 1280, 5.7 TB/s; 32768 packed x 32 heads 686 -> 650, 4096 x 8
+// heads 30.9 -> 29.0.)
 // All tile products are tcgen05.mma with M = 64 (rows = tokens) and fp32 accumulators in tensor memory;
 // two M = 64 accumulators share each column range (lanes +0 and +16 of every 32-lane quarter).
 //
@@ -215,13 +217,14 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  auto WAIT = [&](int idx, uint32_t parity) { return mbar_wait(&bars[idx], parity, abort_flag); };
+  int tries = WAIT_TRIES;  // see mbar_wait; filled up for each item
+  auto WAIT = [&](int idx, uint32_t parity) { mbar_wait(&bars[idx], parity, tries); };
 
   if (warp == N_EPI / 32) {
     // ====================== issue warp: TMA loads and every tcgen05.mma ======================
     // (the warp stays converged; see elect_one in tc05.cuh)
     {
-      auto WAIT = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
+      auto WAIT = [&](int idx, uint32_t parity) { mbar_wait_uniform(&bars[idx], parity, tries); };
       // Four groups, in the order in which their buffers become free (A and du are dead after the first
       // product of an item, q only after the bulk group has read it).
       auto load_d = [&](const Item& t) {
@@ -290,13 +293,13 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       load_d(cur);
       load_a(cur, 0);
       load_q(cur);
-      bool ok = true;
       uint32_t it = 0, zero_ph = 0;
       // An accumulator or an operand tile is written again only behind a barrier that says it has been
       // read: what the chain group reads (dW, ds, qk, KK, D3) behind its own arrivals on the tiles it makes
       // of them, what the bulk group reads (dq, dk, Y) behind R_END of the item before.
 #pragma unroll 1
-      for (bool has_next = true; has_next && ok; ++it) {
+      for (bool has_next = true; has_next && tries > 0; ++it) {
+        tries = WAIT_TRIES;
         const uint32_t ph = it & 1;
         if (!CLC && lane == 0) claimed = (int)gridDim.x + atomicAdd(p.next_item, 1);
         const uint32_t k_lo = k_lo0 + (ph ? KBUF_LO : 0u), kmn_lo = kmn_lo0 + (ph ? KBUF_LO : 0u);
@@ -305,16 +308,15 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         const bool partial = cur.valid != CHUNK;
         if (partial) {
           if (it > 0) {  // q of this item, below for a full chunk
-            ok = WAIT(C_2, ph ^ 1) && WAIT(R_E4, ph ^ 1);
-            if (!ok) break;
+            WAIT(C_2, ph ^ 1);
+            WAIT(R_E4, ph ^ 1);
             load_q(cur);
           }
-          ok = WAIT(R_ZERO, zero_ph);
+          WAIT(R_ZERO, zero_ph);
           zero_ph ^= 1;
         } else {
-          ok = WAIT(L_D, ph);
+          WAIT(L_D, ph);
         }
-        if (!ok) break;
         tc_fence_after();
         // ---- dW = A^T du: needs nothing but A and du ----
         if (elect_one()) {
@@ -329,12 +331,12 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         if (!partial) {
           if (it > 0) {
             // q of the item before is dead: its product is complete, the bulk group has used it
-            ok = WAIT(C_2, ph ^ 1) && WAIT(R_E4, ph ^ 1);
-            if (!ok) break;
+            WAIT(C_2, ph ^ 1);
+            WAIT(R_E4, ph ^ 1);
             load_q(cur);
           }
-          ok = WAIT(L_A, ph) && WAIT(L_Q, ph);
-          if (!ok) break;
+          WAIT(L_A, ph);
+          WAIT(L_Q, ph);
           tc_fence_after();
         }
         // ---- ds, q k^T, K K^T ----
@@ -346,8 +348,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           umma_group<8, 2, 512, 2, 512, false>(tmem + T_KK, k_lo, k_lo, ID_KK_64);
         }
         // ---- dW is an operand now: D3 = dW v_new^T ----
-        ok = WAIT(R_DW, ph);
-        if (!ok) break;
+        WAIT(R_DW, ph);
         tc_fence_after();
         if (elect_one()) {
           if constexpr (TILED) umma_group<8, 2, 512, 128, 512, false>(tmem + T_D3, dw_lo, vnT_lo, ID_KM_64);
@@ -356,8 +357,8 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         }
         int w_next;
         if constexpr (CLC) {
-          ok = WAIT(I_CLAIM, ph);
-          if (!ok) break;
+          WAIT(I_CLAIM, ph);
+          if (tries <= 0) break;  // (no item to look up)
           w_next = clc_block(answers + 16 * ph);
           fence_proxy_async();  // read before the request after the next one writes the slot
           has_next = w_next >= 0;
@@ -368,8 +369,8 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         const int h_next = has_next ? w_next % p.Hv : 0;
         if (has_next) load_index(w_next / p.Hv, raw);
         // ---- Y = dW h^T, dq1, dk1: off the chain ----
-        ok = WAIT(L_H, ph) && (it == 0 || WAIT(R_END, ph ^ 1));
-        if (!ok) break;
+        WAIT(L_H, ph);
+        if (it > 0) WAIT(R_END, ph ^ 1);
         tc_fence_after();
         if (elect_one()) {
           if constexpr (TILED) {
@@ -385,8 +386,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         }
         if (has_next) load_span(raw);
         // ---- ds is an operand now ----
-        ok = WAIT(R_DS, ph);
-        if (!ok) break;
+        WAIT(R_DS, ph);
         tc_fence_after();
         if (elect_one()) {
           umma_group<4, 2, 0, 128, 0, false>(tmem + T_DQ2, ds_lo, kmn_lo, ID_KM_128);
@@ -405,8 +405,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           mbar_arrive(&bars[I_NEXT]);
         }
         // ---- dk += (X + X^T) K with X = beta dL, onto ds^T q ----
-        ok = WAIT(R_D3, ph);
-        if (!ok) break;
+        WAIT(R_D3, ph);
         tc_fence_after();
         if (elect_one()) {
           umma_group<4, 2, 0, 128, 0, true>(tmem + T_DK2, x_lo, kmn_lo, ID_KM_128);
@@ -415,13 +414,13 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         // h, dh, dO, v_new are dead once their products are complete and the h.dh sum is done; the other
         // k buffer belonged to the item before, which R_END above has seen finished
         if (has_next) {
-          ok = WAIT(C_1B, ph) && WAIT(R_HD, ph);
-          if (!ok) break;
+          WAIT(C_1B, ph);
+          WAIT(R_HD, ph);
           load_a(nxt, (int)(ph ^ 1));
         }
         cur = nxt;
       }
-      if (!ok) *abort_flag = 1;
+      if (tries <= 0) *abort_flag = 1;
     }
   } else {
     // ====================== read-out warps ======================
@@ -567,23 +566,25 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       const int koff = OFF_K + (int)ph * ROW_TILE;
       const float* sG = ph ? sVec1 : sVec0;
       const float *sGam = sG + 64, *sRho = sG + 128, *sBeta = sG + 192;
-      bool ok = true;
+      tries = WAIT_TRIES;
       if (valid < CHUNK) {
-        ok = WAIT(L_D, ph) && WAIT(L_A, ph) && WAIT(L_H, ph) && WAIT(L_Q, ph);
-        if (ok) {
-          zero_rows(OFF_Q, 2, valid);
-          zero_rows(koff, 2, valid);
-          zero_rows(OFF_A, 1, valid);
-          if constexpr (TILED) zero_rows(OFF_DO, 2, valid);  // the transposed tiles already hold zeros
-          else zero_rows(OFF_VN, 6, valid);                  // v_new, dO, du
-        }
+        WAIT(L_D, ph);
+        WAIT(L_A, ph);
+        WAIT(L_H, ph);
+        WAIT(L_Q, ph);
+        zero_rows(OFF_Q, 2, valid);
+        zero_rows(koff, 2, valid);
+        zero_rows(OFF_A, 1, valid);
+        if constexpr (TILED) zero_rows(OFF_DO, 2, valid);  // the transposed tiles already hold zeros
+        else zero_rows(OFF_VN, 6, valid);                  // v_new, dO, du
         signal(R_ZERO);
       }
       Item nxt;
       // the next item, from the middle of this one on
       auto take_next = [&] {
-        ok = ok && WAIT(I_NEXT, ph);
+        WAIT(I_NEXT, ph);
         nxt = ring[(it + 1) & 3];
+        if (tries <= 0) nxt.valid = 0;  // not there: nothing more
       };
       float acc_last = 0.f;
 
@@ -599,8 +600,10 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 
         // ---- E1: dW = A^T du as an operand tile; dv = beta dW, made of v in place; db += dW v ----
         // the products that read the operand tile of the item before are complete (C_1B)
-        ok = ok && WAIT(C_DW, ph) && (it == 0 || WAIT(C_1B, ph ^ 1)) && WAIT(L_D, ph);
-        if (ok) {
+        WAIT(C_DW, ph);
+        if (it > 0) WAIT(C_1B, ph ^ 1);
+        WAIT(L_D, ph);
+        {
           tc_fence_after();
           float x[32];
           tmem_ld_16x64(tmem + lanes + T_DW + 64 * half, x);
@@ -639,16 +642,15 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
             if (row < valid)
               *reinterpret_cast<uint4*>(p.dv + ((cur.row0 + row) * p.Hv + cur.hv) * D + 64 * half + 8 * (lane & 7)) = w;
           }
-        } else {
-          signal(R_DW);
         }
 
         // ---- E2: ds = scale * G * (dO Vn^T); ds2 = ds * (Q K^T) ----
-        ok = ok && WAIT(C_DSQK, ph) && (it == 0 || WAIT(C_2, ph ^ 1));
+        WAIT(C_DSQK, ph);
+        if (it > 0) WAIT(C_2, ph ^ 1);
         const float g_a = sG[row_a], g_b = sG[row_b];
         // address of this lane's row in a [16 x 32] block of a 64-column tile, 16-byte piece 4 half + i
         const uint32_t line = (uint32_t)((16 * qd + 8 * ((lane >> 3) & 1) + (lane & 7)) * 128);
-        if (ok) {
+        {
           tc_fence_after();
           float ds[16], qk[16];
           tmem_ld_16x32(tmem + lanes + T_DS + c64, ds);
@@ -680,8 +682,9 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 
         // ---- E7: X = beta dL, dL = -G D3 below the diagonal, D3 = dW v_new^T; X + X^T as an operand
         //      tile; the dg and db terms of dL * (K K^T) ----
-        ok = ok && WAIT(C_D3, ph) && (it == 0 || WAIT(C_5, ph ^ 1));
-        if (ok) {
+        WAIT(C_D3, ph);
+        if (it > 0) WAIT(C_5, ph ^ 1);
+        {
           tc_fence_after();
           float d3[16], kk[16];
           tmem_ld_16x32(tmem + lanes + T_D3 + c64, d3);
@@ -726,10 +729,10 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         }
         signal(R_D3);
         take_next();
-        if (ok && nxt.valid > 0) fetch_vectors(nxt);
+        if (nxt.valid > 0) fetch_vectors(nxt);
         // The partial-sum slots were read for the previous item by two warps of the bulk group (combine), which
         // arrive on R_E4 of this item only after that: both groups wait for it before they write theirs.
-        ok = ok && WAIT(R_E4, ph);
+        WAIT(R_E4, ph);
         // one reduction per quantity, one plain store per (warp, row or column): no atomics
         acc_dg_a = quad_sum(acc_dg_a);
         acc_dg_b = quad_sum(acc_dg_b);
@@ -749,8 +752,9 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       } else {
         // ===================== bulk group =====================
         // gamma_last * sum(h * dh) over the whole 128 x 128 tiles (plain shared-memory reads)
-        ok = ok && WAIT(L_A, ph) && WAIT(L_H, ph);
-        if (ok) {
+        WAIT(L_A, ph);
+        WAIT(L_H, ph);
+        {
           float hd = 0.f;
 #pragma unroll 2  // (unrolled as far as the compiler goes: 1 to 2 % of small launches in instruction fetches)
           for (int i = tid - N_EPI / 2; i < SQ_TILE / 16; i += N_EPI / 2) {
@@ -777,8 +781,9 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
 
         // ---- E4: the dg terms of dq1 = scale gamma (dO h^T) on the lower lanes, dk1 = rho (Vn dh^T) on
         //      the upper ----
-        ok = ok && WAIT(C_1B, ph) && WAIT(L_Q, ph);
-        if (ok) {
+        WAIT(C_1B, ph);
+        WAIT(L_Q, ph);
+        {
           tc_fence_after();
           const unsigned char* tile = smem + (hi ? koff : OFF_Q);
 #pragma unroll 1
@@ -809,8 +814,9 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         // ---- E8: dq = dq1 + ds K (lower lanes); dk = dk1 - beta gamma Y + [ds^T q + (X + X^T) K] (upper
         //      lanes), and the dg and db terms of Y = dW h^T ----
         // (R_E4: the two warps of combine have read the sums of the item before, see the chain group)
-        ok = ok && WAIT(R_E4, ph) && WAIT(C_5, ph);
-        if (ok) {
+        WAIT(R_E4, ph);
+        WAIT(C_5, ph);
+        {
           tc_fence_after();
           bf16* out = hi ? p.dk : p.dq;
           const float f_y = hi ? -sBeta[row_w] * sGam[row_w] : 0.f;
@@ -862,9 +868,9 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       if (chain) {
         if (nxt.valid > 0) write_vectors(nxt, ph ? sVec0 : sVec1);
       } else {
-        ok = ok && WAIT(R_CH, ph);
+        WAIT(R_CH, ph);
       }
-      if (!ok) *abort_flag = 1;
+      if (tries <= 0) *abort_flag = 1;
       volatile int* stop = stop_flag + (chain ? 0 : 2) + ph;
       if ((tid & 255) == 0) *stop = *abort_flag ? 1 : nxt.valid > 0 ? 0 : 2;
       if (chain) {

@@ -95,8 +95,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
 // at the count and ends: one look a pass instead of a result at each of the dozens of wait sites, which were a
 // third of the kernels' code.  What a pass does after a wait was given up touches only the memory that it would
 // have touched anyway; its values are lost (the kernel sets its status word).  The thread is suspended by the
-// hardware meanwhile; polling with test_wait instead, or once before it, takes issue slots from the warps that
-// have work (262144-token forward recurrence: 467 us, 484 with a test at the waits that are mostly over).
+// hardware meanwhile, but comes back early and often: trying again at once takes issue slots from the warps that
+// have work, hence the pause (chunk-parallel backward, 262144 tokens x 8 heads: 1510 us without it, 1260 with,
+// whether 20 or 400 ns; 1340 with a look at an abort flag in its place).  Polling with test_wait instead, or once
+// before it, costs more (forward recurrence 467 us, 484 with a test at the waits that are mostly over).
 constexpr int WAIT_TRIES = 1 << 24;
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int& tries) {
   asm volatile(
@@ -104,11 +106,18 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int& t
       "W%=:\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "@p bra D%=;\n\t"
-      "add.s32 %0, %0, -1;\n\tsetp.gt.s32 p, %0, 0;\n\t@p bra W%=;\n"
+      "nanosleep.u32 20;\n\tadd.s32 %0, %0, -1;\n\tsetp.gt.s32 p, %0, 0;\n\t@p bra W%=;\n"
       "D%=:\n\t}"
       : "+r"(tries)
       : "r"(s32(bar)), "r"(parity)
       : "memory");
+}
+
+// The same for a warp that issues products: it stays converged in the compiler's eyes, which keeps what is
+// computed between its waits in uniform registers.
+__device__ __forceinline__ void mbar_wait_uniform(uint64_t* bar, uint32_t parity, int& tries) {
+#pragma unroll 1
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity)) && --tries > 0) __nanosleep(20);
 }
 
 // Four 8 x 8 bf16 matrices from registers to shared memory, each stored TRANSPOSED: register i of
@@ -294,7 +303,7 @@ __device__ __forceinline__ void tmem_ld_16x64(uint32_t taddr, float (&v)[32]) {
       : "r"(taddr)
       : "memory");
 }
-// The same over 32 (x4) and 16 (x2) columns.
+// The same over 32 columns (x4).
 __device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, float (&v)[16]) {
   uint32_t* r = reinterpret_cast<uint32_t*>(v);
   asm volatile(
@@ -305,13 +314,6 @@ __device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, float (&v)[16]) {
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
-}
-__device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, float (&v)[8]) {
-  uint32_t* r = reinterpret_cast<uint32_t*>(v);
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr)
-               : "memory");
 }
 // 32 lanes x 16 consecutive columns -> 16 registers per thread
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
