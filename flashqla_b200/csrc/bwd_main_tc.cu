@@ -218,7 +218,10 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   int tries = WAIT_TRIES;  // see mbar_wait; filled up for each item
-  auto WAIT = [&](int idx, uint32_t parity) { mbar_wait(&bars[idx], parity, tries); };
+  auto WAIT = [&](int idx, uint32_t parity) {
+    mbar_wait(&bars[idx], parity, tries);
+    return tries > 0;
+  };
 
   if (warp == N_EPI / 32) {
     // ====================== issue warp: TMA loads and every tcgen05.mma ======================
@@ -865,12 +868,13 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       // behind R_CH.  (One barrier of all sixteen warps here held the chain group for the last
       // wide read-out, 1600 of 14500 cycles per item.)  Each group has a stop flag of its own, by
       // item parity, so that it is read by the whole group before it can be written again.
+      bool ok = tries > 0;
       if (chain) {
         if (nxt.valid > 0) write_vectors(nxt, ph ? sVec0 : sVec1);
       } else {
-        WAIT(R_CH, ph);
+        ok = ok && WAIT(R_CH, ph);
       }
-      if (tries <= 0) *abort_flag = 1;
+      if (!ok) *abort_flag = 1;
       volatile int* stop = stop_flag + (chain ? 0 : 2) + ph;
       if ((tid & 255) == 0) *stop = *abort_flag ? 1 : nxt.valid > 0 ? 0 : 2;
       if (chain) {
