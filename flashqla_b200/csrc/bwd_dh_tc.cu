@@ -18,7 +18,9 @@
 // du), warps 12-15 build Pg and scale q (in place).  All waits are bounded mbarrier waits.
 // (One thread issued everything before, 32 instructions of some 50 cycles a chunk, and two warps scaled both A
 // and q and took longer over q than the chain over a chunk: 262144 tokens x 8 heads 674 -> 587 us, 32768 packed
-// x 32 heads 384 -> 360, 4096 x 8 heads 22.6 -> 21.7; with A scaled by the state group 618, 362 and 21.9.)
+// x 32 heads 384 -> 360, 4096 x 8 heads 22.6 -> 21.7; with A scaled by the state group 618, 362 and 21.9.  With
+// waits that pause between two tries and row-major outputs made in rolled loops (69 -> 56 KB of code) 604 -> 584 and
+// 361 -> 353.)
 #include <cuda.h>
 
 #include <climits>
@@ -182,8 +184,20 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
-  bool ok = true;
-  auto WAIT = [&](int idx, uint32_t parity) { return mbar_wait(&bars[idx], parity, abort_flag); };
+  int tries = WAIT_TRIES;  // see mbar_wait; `more`: none was given up, on to the next pass of a role's loop
+  auto WAIT = [&](int idx, uint32_t parity) { mbar_wait(&bars[idx], parity, tries); };
+  // (of the issuing warps: see mbar_wait_uniform; 262144 tokens x 8 heads 584 us, 590 with the plain ones)
+  auto WAITU = [&](int idx, uint32_t parity) { mbar_wait_uniform(&bars[idx], parity, tries); };
+  auto more_u = [&] {
+    const bool ok = __all_sync(0xffffffffu, tries > 0);
+    if (ok) tries = WAIT_TRIES;
+    return ok;
+  };
+  auto more = [&] {
+    const bool ok = tries > 0;
+    if (ok) tries = WAIT_TRIES;
+    return ok;
+  };
 
   // End gradient -> tensor memory, dS^T[v][k]; zero without one and for a lead-out.  The three
   // read-out groups share the columns 2 : 1 : 1: one memory latency (see fwd_tc.cu).
@@ -236,10 +250,9 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
   if (warp >= 4 && warp < 8) {
     // =============================== state group ===============================
     const int v = tid - 128;
-    for (int it = 0; it < n_it && ok; ++it) {
+    for (int it = 0; it < n_it && more(); ++it) {
       const int s = it & 1, c = n_it - 1 - it;
-      if (it > 0) ok = WAIT(S_DONE, (it - 1) & 1);
-      if (!ok) break;
+      if (it > 0) WAIT(S_DONE, (it - 1) & 1);
       tc_fence_after();
       bf16* hdst = (p.dh && it >= lead)
                        ? p.dh + ((sp.chunk_base + c) * p.Hv + hv) * (long long)D * D : nullptr;
@@ -259,20 +272,18 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
               make_uint4(pack_bf16(y[8 * cc + 0], y[8 * cc + 1]), pack_bf16(y[8 * cc + 2], y[8 * cc + 3]),
                          pack_bf16(y[8 * cc + 4], y[8 * cc + 5]), pack_bf16(y[8 * cc + 6], y[8 * cc + 7]));
         }
-        if (hdst && !p.tiled) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            hdst[(long long)(kb * 64 + j) * D + v] = __float2bfloat16(x[j]);
-            hdst[(long long)(kb * 64 + 32 + j) * D + v] = __float2bfloat16(y[j]);
-          }
-        }
       }
       fence_proxy_async();
       tc_fence_before();
       mbar_arrive(&bars[S_COPY]);
+      if (hdst && !p.tiled) {  // row-major [k][v]: column v, from this thread's own row of the copy
+#pragma unroll 1
+        for (int k = 0; k < D; ++k)
+          hdst[(long long)k * D + v] =
+              *reinterpret_cast<const bf16*>(smem + OFF_ST + (k >> 6) * 16384 + sw128_offset(v, k & 63));
+      }
       // off the chain: decay in place
-      ok = WAIT(FULL0 + s, (it >> 1) & 1);
-      if (!ok) break;
+      WAIT(FULL0 + s, (it >> 1) & 1);
       const float gl = vec[(it & 3) * VEC_SLOT_FLOATS + V_GL * CHUNK];
 #pragma unroll 1
       for (int kb = 0; kb < 2; ++kb) {
@@ -292,9 +303,9 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       tc_fence_before();
       mbar_arrive(&bars[S_DEC]);
     }
-    if (ok && n_it > 0) ok = WAIT(S_DONE, (n_it - 1) & 1);
+    if (tries > 0 && n_it > 0) WAIT(S_DONE, (n_it - 1) & 1);
     const int dh0_row = p.dh0_row ? p.dh0_row[n] : n;
-    if (ok && p.dh0 && dh0_row >= 0) {
+    if (tries > 0 && p.dh0 && dh0_row >= 0) {
       float* dst = p.dh0 + ((long long)dh0_row * p.Hv + hv) * D * D;
       tc_fence_after();
 #pragma unroll 1
@@ -320,7 +331,8 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     const int tok_w = 16 * wq + lane;  // lanes 0-15 of each quarter hold a row of w
     auto convert_w = [&](int it) {
       // ... and the state update that reads the tile of the chunk before is complete
-      if (!WAIT(W_DONE, it & 1) || (it > 0 && !WAIT(S_DONE, (it - 1) & 1))) return false;
+      WAIT(W_DONE, it & 1);
+      if (it > 0) WAIT(S_DONE, (it - 1) & 1);
       tc_fence_after();
 #pragma unroll 1
       for (int c0 = 0; c0 < D; c0 += 32) {
@@ -339,16 +351,16 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       fence_proxy_async();
       tc_fence_before();
       mbar_arrive(&bars[W_READY]);
-      return true;
     };
 #pragma unroll 1
-    for (int it = -1; it < n_it && ok; ++it) {  // it = -1: only w of the first iteration
+    for (int it = -1; it < n_it && more(); ++it) {  // it = -1: only w of the first iteration
      if (it >= 0) {
       const int c = n_it - 1 - it;
       const long long row0 = sp.bos + (long long)c * CHUNK;
       const int valid = min(CHUNK, len_ext - c * CHUNK);
-      ok = WAIT(FULL0 + (it & 1), (it >> 1) & 1) && WAIT(X2_DONE, it & 1) && WAIT(X1_DONE, it & 1);
-      if (!ok) break;
+      WAIT(FULL0 + (it & 1), (it >> 1) & 1);
+      WAIT(X2_DONE, it & 1);
+      WAIT(X1_DONE, it & 1);
       tc_fence_after();
       const float* rho = vec + (it & 3) * VEC_SLOT_FLOATS + V_RHO * CHUNK;
       unsigned char* row = smem + OFF_DVT + v * 128;
@@ -371,20 +383,19 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
           *reinterpret_cast<uint4*>(row + (((4 * h + cc) ^ (v & 7)) << 4)) =
               make_uint4(pack_bf16(x[8 * cc + 0], x[8 * cc + 1]), pack_bf16(x[8 * cc + 2], x[8 * cc + 3]),
                          pack_bf16(x[8 * cc + 4], x[8 * cc + 5]), pack_bf16(x[8 * cc + 6], x[8 * cc + 7]));
-        if (h == 1) {  // operand complete, accumulators read: hand over before the global stores
-          fence_proxy_async();
-          tc_fence_before();
-          mbar_arrive(&bars[DV_READY]);
-        }
-        if (p.du && !p.tiled && it >= lead) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (32 * h + j < valid)
-              p.du[((row0 + 32 * h + j) * p.Hv + hv) * D + v] = __float2bfloat16(x[j]);
-        }
+      }
+      // operand complete, accumulators read: hand over before the global stores
+      fence_proxy_async();
+      tc_fence_before();
+      mbar_arrive(&bars[DV_READY]);
+      if (p.du && !p.tiled && it >= lead) {  // row-major: column v, from this thread's own row
+        bf16* dst = p.du + (row0 * p.Hv + hv) * D + v;
+#pragma unroll 1
+        for (int j = 0; j < valid; ++j)
+          dst[(long long)j * p.Hv * D] = *reinterpret_cast<const bf16*>(smem + OFF_DVT + sw128_offset(v, j));
       }
      }
-      if (it + 1 < n_it) ok = convert_w(it + 1);
+      if (it + 1 < n_it) convert_w(it + 1);
     }
   } else if (warp >= 12) {
     // =============================== Pg and q group ===============================
@@ -395,11 +406,11 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     const int row_a = 16 * wq + (lane >> 2), row_b = row_a + 8, cp = 2 * (lane & 3);
     const uint32_t lanes_p = (uint32_t)(wq * 32) << 16;
     const float log2_scale = log2f(p.scale);
-    for (int it = 0; it < n_it && ok; ++it) {
+    for (int it = 0; it < n_it && more(); ++it) {
       const float* vs = vec + (it & 3) * VEC_SLOT_FLOATS;
-      ok = WAIT(FULL0 + (it & 1), (it >> 1) & 1) && WAIT(P_DONE, it & 1);
-      if (ok && it > 0) ok = WAIT(X2_DONE, (it - 1) & 1);  // the previous Pg tile has been consumed
-      if (!ok) break;
+      WAIT(FULL0 + (it & 1), (it >> 1) & 1);
+      WAIT(P_DONE, it & 1);
+      if (it > 0) WAIT(X2_DONE, (it - 1) & 1);  // the previous Pg tile has been consumed
       tc_fence_after();
       const float ga2 = vs[V_G * CHUNK + row_a] * 1.4426950408889634f + log2_scale;
       const float gb2 = vs[V_G * CHUNK + row_b] * 1.4426950408889634f + log2_scale;
@@ -425,8 +436,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       tc_fence_before();
       mbar_arrive(&bars[P_READY]);
       // (not before the update of the chunk before has been issued: its thread waits for that chunk's q)
-      if (it > 0) ok = WAIT(S_DONE, (it - 1) & 1);
-      if (!ok) break;
+      if (it > 0) WAIT(S_DONE, (it - 1) & 1);
       const float sg = vs[V_SGAM * CHUNK + qr];
       unsigned char* q = smem + OFF_STAGE + (it & 1) * STAGE_BYTES + qh * 8192 + qr * 128;
 #pragma unroll 4
@@ -451,17 +461,16 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     const uint32_t q0_lo = desc_lo_kmajor(smem + OFF_STAGE), k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE);
     const uint32_t domn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + 2 * TILE, 8192);
     constexpr uint32_t STAGE_LO = STAGE_BYTES >> 4;
-    auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
     if (warp == 0) {
       const uint32_t st_lo = desc_lo_kmajor(smem + OFF_ST), dvt_lo = desc_lo_kmajor(smem + OFF_DVT);
       const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 8192), qmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE, 8192);
 #pragma unroll 1
-      for (int it = 0; it < n_it && ok; ++it) {
+      for (int it = 0; it < n_it && more_u(); ++it) {
         const int s = it & 1;
         const uint32_t so = s ? STAGE_LO : 0u;
         const int y_tile = (int)(((sp.chunk_base + (n_it - 1 - it)) * p.Hv + hv) * D);
-        ok = WAITW(FULL0 + s, (it >> 1) & 1) && WAITW(S_COPY, it & 1);
-        if (!ok) break;
+        WAITU(FULL0 + s, (it >> 1) & 1);
+        WAITU(S_COPY, it & 1);
         tc_fence_after();
         if (elect_one()) {
           // X1^T = dS^T K^T   (on the chain)
@@ -475,13 +484,13 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
           }
         }
         // dS^T <- dS^T + dO^T (scale gamma q) - dv^T w; the first product while dv is on its way
-        ok = WAITW(QS_READY, it & 1) && WAITW(S_DEC, it & 1);
-        if (!ok) break;
+        WAITU(QS_READY, it & 1);
+        WAITU(S_DEC, it & 1);
         tc_fence_after();
         if (elect_one())
           umma_group<4, 128, 0, 128, 0, true>(tmem + TM_S, domn0_lo + so, qmn0_lo + so, ID_UPD_Q);
-        ok = WAITW(W_READY, it & 1) && WAITW(DV_READY, it & 1);
-        if (!ok) break;
+        WAITU(W_READY, it & 1);
+        WAITU(DV_READY, it & 1);
         tc_fence_after();
         if (elect_one()) {
           umma_group<4, 2, 0, 128, 0, true>(tmem + TM_S, dvt_lo, wmn_lo, ID_UPD_W);
@@ -499,28 +508,27 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE, 8192);
       const uint32_t app_lo = desc_lo_kmajor(smem + OFF_APP), pmn_lo = desc_lo_mnmajor(smem + OFF_P, 8192);
 #pragma unroll 1
-      for (int it = 0; it < n_it && ok; ++it) {
+      for (int it = 0; it < n_it && more_u(); ++it) {
         const int s = it & 1;
         const uint32_t so = s ? STAGE_LO : 0u;
         // (the Pg group has read P of the chunk before: P_READY was waited for)
-        ok = WAITW(FULL0 + s, (it >> 1) & 1);
-        if (!ok) break;
+        WAITU(FULL0 + s, (it >> 1) & 1);
         tc_fence_after();
         if (elect_one()) {
           umma_group<8, 2, 512, 2, 512, false>(tmem + TM_P, q0_lo + so, k0_lo + so, ID_P);
           umma_commit(&bars[P_DONE]);
         }
         // w, whose accumulator the dv / w group has read for the chunk before
-        ok = WAITW(AP_READY, it & 1) && (it == 0 || WAITW(W_READY, (it - 1) & 1));
-        if (!ok) break;
+        WAITU(AP_READY, it & 1);
+        if (it > 0) WAITU(W_READY, (it - 1) & 1);
         tc_fence_after();
         if (elect_one()) {
           umma_group<4, 2, 0, 128, 0, false>(tmem + TM_W, app_lo, kmn0_lo + so, ID_W);
           umma_commit(&bars[W_DONE]);
         }
         // X2^T = dO^T Pg, likewise
-        ok = WAITW(P_READY, it & 1) && (it == 0 || WAITW(DV_READY, (it - 1) & 1));
-        if (!ok) break;
+        WAITU(P_READY, it & 1);
+        if (it > 0) WAITU(DV_READY, (it - 1) & 1);
         tc_fence_after();
         if (elect_one()) {
           umma_group<4, 128, 0, 128, 0, false>(tmem + TM_X2, domn0_lo + so, pmn_lo, ID_X2);
@@ -544,7 +552,6 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         b_r[z] = r < valid ? load_beta(p.beta, p.beta_is_f32, (row0 + r) * p.Hv + hv) : 0.f;
       }
     };
-    auto WAITW = [&](int idx, uint32_t parity) { return mbar_wait_warp<false>(&bars[idx], parity, abort_flag); };
     // zero the rows past the sequence end in n 8 KB blocks of 64 rows, then hand the tile on
     auto zero_rows = [&](unsigned char* base, int n, int valid, uint64_t* full) {
 #pragma unroll 1
@@ -558,15 +565,14 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     // iteration it + 2 into registers.  Slot (it + 1) % 4 of the vectors was last read for iteration
     // it - 3, which the wait on the stage of iteration it - 2 has seen finished.
 #pragma unroll 1
-    for (int it = -2; it < n_it && ok; ++it) {
+    for (int it = -2; it < n_it && more(); ++it) {
       if (it >= 0) {
         const int s = it & 1, c = n_it - 1 - it;
         const int y = (int)(sp.bos + (long long)c * CHUNK);
         const int valid = min(CHUNK, len_ext - c * CHUNK);
         const bool partial = valid < CHUNK;
         if (it >= 2) {
-          ok = WAITW(EMPTY0 + s, ((it >> 1) - 1) & 1);
-          if (!ok) break;
+          WAIT(EMPTY0 + s, ((it >> 1) - 1) & 1);
         }
         unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
         uint64_t* bar = &bars[partial ? PRIV : FULL0 + s];
@@ -580,8 +586,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
           tma_load_2d(st + 2 * TILE + 8192, &map_do, hv * D + 64, y, bar);
         }
         if (partial) {
-          ok = WAITW(PRIV, 0);
-          if (!ok) break;
+          WAIT(PRIV, 0);
           zero_rows(st, 6, valid, &bars[FULL0 + s]);
         }
       }
@@ -592,8 +597,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         const bool partial = valid < CHUNK;
         // the stage's A buffer is free once the scaling warps have read it
         if (j >= 2) {
-          ok = WAITW(EMPTYA0 + sj, ((j >> 1) - 1) & 1);
-          if (!ok) break;
+          WAIT(EMPTYA0 + sj, ((j >> 1) - 1) & 1);
         }
         float* vs = vec + (j & 3) * VEC_SLOT_FLOATS;
 #pragma unroll
@@ -615,8 +619,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         }
         if (partial) {
           // only the last chunk of a sequence (the first one walked) can be partial: used once
-          ok = WAITW(PRIVA, 0);
-          if (!ok) break;
+          WAIT(PRIVA, 0);
           zero_rows(dst, 1, valid, &bars[FULLA0 + sj]);
         }
       }
@@ -628,11 +631,10 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     // t/8 + 4 i, its scale factors stay in registers and the eight threads of a row touch one
     // 128-byte line per access.
     const int c8 = lane & 7, r0 = lane >> 3;
-    for (int it = 0; it < n_it && ok; ++it) {
+    for (int it = 0; it < n_it && more(); ++it) {
       const int s = it & 1;
-      ok = WAIT(FULLA0 + s, (it >> 1) & 1);
-      if (ok && it > 0) ok = WAIT(W_DONE, (it - 1) & 1);  // w of the chunk before has been issued and is done
-      if (!ok) break;
+      WAIT(FULLA0 + s, (it >> 1) & 1);
+      if (it > 0) WAIT(W_DONE, (it - 1) & 1);  // w of the chunk before has been issued and is done
       const float* vs = vec + (it & 3) * VEC_SLOT_FLOATS;
       const unsigned char* src = smem + OFF_STAGE + s * STAGE_BYTES + 3 * TILE;
       const float4 g0 = *reinterpret_cast<const float4*>(vs + V_BG * CHUNK + 8 * c8);
@@ -655,7 +657,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
   }
 
   // ---- teardown ----
-  if (!ok) *abort_flag = 1;
+  if (tries <= 0) *abort_flag = 1;
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);

@@ -213,12 +213,10 @@ __global__ void __launch_bounds__(32 * kkt::MAX_WARPS, 3) kkt_solve_kernel(
   float* sG = reinterpret_cast<float*>(vecs + warp * VEC_BYTES);  // g log2(e)
   float* sB = sG + CHUNK;                                         // -beta
   uint64_t* bar = reinterpret_cast<uint64_t*>(vecs + n_warps * VEC_BYTES);
-  int* abort_flag = reinterpret_cast<int*>(bar + 1);
   const int q8 = lane >> 2, t4 = lane & 3, l7 = lane & 7;  // fragment row, column pair; row mod 8
   const int hq = blockIdx.y, G = Hv / Hq;
   if (tid == 0) {
     tc::mbar_init(bar, 1);
-    *abort_flag = 0;
     tc::fence_mbar_init();
   }
   pdl_wait();
@@ -243,10 +241,10 @@ __global__ void __launch_bounds__(32 * kkt::MAX_WARPS, 3) kkt_solve_kernel(
     for (int b = 0; b < D / 64; ++b)
       tc::tma_load_2d(smem + b * 8192, &map_k, hq * D + 64 * b, (int)row0, bar);
   }
-  bool ok = true;
+  int tries = tc::WAIT_TRIES;
 
 #pragma unroll 1
-  for (int gi = warp; gi < G && ok; gi += n_warps) {
+  for (int gi = warp; gi < G && tries > 0; gi += n_warps) {
     const int hv = hq * G + gi;
     {  // gates and beta of the rows lane, lane + 32
       float x[2];
@@ -277,8 +275,8 @@ __global__ void __launch_bounds__(32 * kkt::MAX_WARPS, 3) kkt_solve_kernel(
       sG[lane] = x[0] * 1.4426950408889634f;
       sG[lane + 32] = x[1] * 1.4426950408889634f;
     }
-    ok = tc::mbar_wait(bar, 0, abort_flag);
-    if (!ok) break;
+    tc::mbar_wait(bar, 0, tries);
+    if (tries <= 0) break;
     __syncwarp();
 
     // ---- 1. K K^T, lower blocks (rb, cb), index rb (rb + 1) / 2 + cb
@@ -476,7 +474,7 @@ __global__ void __launch_bounds__(32 * kkt::MAX_WARPS, 3) kkt_solve_kernel(
     }
   }  // value heads of this warp
   if (lane == 0) tc::tma_store_wait_read();  // shared memory outlives the stores' reads
-  if (!ok && lane == 0) atomicCAS(&g_kkt_status, 0, 1);
+  if (tries <= 0 && lane == 0) atomicCAS(&g_kkt_status, 0, 1);
 }
 
 // ------------------------------------------------------------------------------------------

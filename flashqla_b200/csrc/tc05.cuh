@@ -59,37 +59,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Non-blocking test of a phase (about 13 cycles on B200).
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(s32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait: at most `budget` tries (the default is some seconds).  Gives up as soon as
-// *abort_flag (shared memory) is set; on its own timeout it sets *abort_flag so that every other
-// role of the CTA leaves too.  Returns false when the wait was abandoned.
-// One loop around one instruction: a kernel has dozens of wait sites and is larger than the
-// instruction cache.  (A test first and then tries with a 1 ms suspend hint was 5-10 % more code
-// and woke up later: 802 against 787 us for a 262144-token forward, 2040 against 1997 us for 32768
-// packed training tokens.)
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
-                                          volatile int* abort_flag, uint32_t budget = 1u << 24) {
-#pragma unroll 1
-  do {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-  } while (--budget);
-  *abort_flag = 1;
-  return false;
-}
-
 // Bounded wait.  `tries` is the thread's own count, WAIT_TRIES (about a second and more) at the start of each
 // pass of its loop; a wait that uses it up falls through, and so does every wait after it, until the loop looks
 // at the count and ends: one look a pass instead of a result at each of the dozens of wait sites, which were a
@@ -173,20 +142,6 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(p));
   return p != 0;
 }
-// Bounded wait of a whole converged warp: the result is the same in every lane.  SPIN: poll (about
-// 25 cycles a round) without looking at the abort flag in between, for the warp on the critical path.
-template <bool SPIN>
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  uint32_t n = 1u << 24;
-#pragma unroll 1
-  do {
-    if (__all_sync(0xffffffffu, SPIN ? mbar_test_wait(bar, parity) : mbar_try_wait(bar, parity))) return true;
-    if (!SPIN && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
-  } while (--n);
-  *abort_flag = 1;
-  return false;
-}
-
 // ---- cluster launch control ----------------------------------------------------------------------
 // Asks for a block of this grid that has not started yet.  It then never starts, and the block that asked
 // does its work: dynamic hand-out of a grid without a counter in memory.  The answer (16 bytes, written
