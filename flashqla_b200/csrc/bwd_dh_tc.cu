@@ -247,7 +247,8 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     }
   }
 
-  if (warp >= 4 && warp < 8) {
+  switch (warp >> 2) {  // (and not a chain of ifs: see fwd_tc.cu)
+  case 1: {
     // =============================== state group ===============================
     const int v = tid - 128;
     for (int it = 0; it < n_it && more(); ++it) {
@@ -324,7 +325,8 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         }
       }
     }
-  } else if (warp >= 8 && warp < 12) {
+  } break;
+  case 2: {
     // =============================== dv / w group ===============================
     const int v = tid - 256;
     const int wq = warp & 3;
@@ -397,7 +399,8 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
      }
       if (it + 1 < n_it) convert_w(it + 1);
     }
-  } else if (warp >= 12) {
+  } break;
+  case 3: {
     // =============================== Pg and q group ===============================
     // Pg, then q' = scale gamma .* q (rows) over q, once P = Q K^T has read it: ready long before the state
     // update wants it.  Two threads per row, in rotated order.
@@ -448,7 +451,8 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       fence_proxy_async();
       mbar_arrive(&bars[QS_READY]);
     }
-  } else if (warp == 0 || warp == 3) {
+  } break;
+  default: if (warp == 0 || warp == 3) {
     // =============================== MMA issuers ===============================
     // (the warps stay converged; see elect_one in tc05.cuh)  Warp 0 issues what the state gradient depends
     // on: X1 and the two products of the update; warp 3 the rest (P, w, X2 of the next iteration).
@@ -564,32 +568,37 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     // As in fwd_tc.cu: q, k, dO of iteration it; vectors and A tile of iteration it + 1; the gates of
     // iteration it + 2 into registers.  Slot (it + 1) % 4 of the vectors was last read for iteration
     // it - 3, which the wait on the stage of iteration it - 2 has seen finished.
+    // (A whole first chunk's q, k, dO go out at once, ahead of its gates, as in fwd_tc.cu.)
+    const bool early = n_it > 0 && len_ext >= n_it * CHUNK;
+    auto load = [&](int it) {
+      const int s = it & 1, c = n_it - 1 - it;
+      const int y = (int)(sp.bos + (long long)c * CHUNK);
+      const int valid = min(CHUNK, len_ext - c * CHUNK);
+      const bool partial = valid < CHUNK;
+      if (it >= 2) {
+        WAIT(EMPTY0 + s, ((it >> 1) - 1) & 1);
+      }
+      unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
+      uint64_t* bar = &bars[partial ? PRIV : FULL0 + s];
+      if (elect_one()) {
+        mbar_expect_tx(bar, STAGE_BYTES - TILE_A);
+        if (it > 0 || !early) mbar_arrive(bar);
+        tma_load_2d(st + TILE, &map_k, hq * D, y, bar);
+        tma_load_2d(st + TILE + 8192, &map_k, hq * D + 64, y, bar);
+        tma_load_2d(st, &map_q, hq * D, y, bar);
+        tma_load_2d(st + 8192, &map_q, hq * D + 64, y, bar);
+        tma_load_2d(st + 2 * TILE, &map_do, hv * D, y, bar);
+        tma_load_2d(st + 2 * TILE + 8192, &map_do, hv * D + 64, y, bar);
+      }
+      if (partial) {
+        WAIT(PRIV, 0);
+        zero_rows(st, 6, valid, &bars[FULL0 + s]);
+      }
+    };
 #pragma unroll 1
     for (int it = -2; it < n_it && more(); ++it) {
-      if (it >= 0) {
-        const int s = it & 1, c = n_it - 1 - it;
-        const int y = (int)(sp.bos + (long long)c * CHUNK);
-        const int valid = min(CHUNK, len_ext - c * CHUNK);
-        const bool partial = valid < CHUNK;
-        if (it >= 2) {
-          WAIT(EMPTY0 + s, ((it >> 1) - 1) & 1);
-        }
-        unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
-        uint64_t* bar = &bars[partial ? PRIV : FULL0 + s];
-        if (elect_one()) {
-          mbar_arrive_expect_tx(bar, STAGE_BYTES - TILE_A);
-          tma_load_2d(st + TILE, &map_k, hq * D, y, bar);
-          tma_load_2d(st + TILE + 8192, &map_k, hq * D + 64, y, bar);
-          tma_load_2d(st, &map_q, hq * D, y, bar);
-          tma_load_2d(st + 8192, &map_q, hq * D + 64, y, bar);
-          tma_load_2d(st + 2 * TILE, &map_do, hv * D, y, bar);
-          tma_load_2d(st + 2 * TILE + 8192, &map_do, hv * D + 64, y, bar);
-        }
-        if (partial) {
-          WAIT(PRIV, 0);
-          zero_rows(st, 6, valid, &bars[FULL0 + s]);
-        }
-      }
+      if (it > 0 || it == (early ? -2 : 0)) load(max(it, 0));
+      else if (it == 0 && lane == 0) mbar_arrive(&bars[FULL0]);
       const int j = it + 1;
       if (j >= 0 && j < n_it) {
         const int sj = j & 1, c = n_it - 1 - j;
@@ -655,6 +664,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       }
     }
   }
+  }  // switch
 
   // ---- teardown ----
   if (tries <= 0) *abort_flag = 1;
