@@ -39,14 +39,14 @@
 //                       (2 stages), zero-fill of rows past the end of a partial chunk
 //
 // What bounds it: the chain of a chunk (3230 cycles on an idle chip: state copy 530, Vn^T 770, its read-out 780,
-// state update 700, and the arrivals between them) and, with all SMs at work, HBM: 262144 tokens x 8 heads 462 us,
-// 5.3 TB/s.  Two things had made it 4830 and 526 us (4 x 8192 x 16 heads 152 -> 132 us, 32768 packed x 32 heads with
-// tiles 391 -> 358).  (1) Roles that waited for one another in a ring: one thread that issued everything off the
+// state update 700, and the arrivals between them) and, with all SMs at work, HBM: 262144 tokens x 8 heads 455 us,
+// 5.3 TB/s.  Two things had made it 4830 and 516 us (4 x 8192 x 16 heads 151 -> 131 us, 32768 packed x 32 heads with
+// tiles 392 -> 353).  (1) Roles that waited for one another in a ring: one thread that issued everything off the
 // chain, and an output group that built Pg between two epilogues.  No role waits here for another one's work off the
 // chain, and w^T and P, which share their columns, are read out of them at once.  (2) Code: the instruction cache of
 // an SM holds some 28 KB (straight code of one warp per scheduler, measured: full speed up to there, 2.5 cycles an
 // instruction beyond, 10 with all SMs at it), and a chunk runs every role's loop once.  So loops are rolled to
-// rounds of one tensor-memory load, and a wait is five instructions (tc05.cuh): 57 -> 47 KB, with tiles 72 -> 52.
+// rounds of one tensor-memory load, and a wait is six instructions (tc05.cuh): 57 -> 47 KB, with tiles 72 -> 52.
 //
 // The state-only pass of the exact hand-off (end states and transition matrices of segments) is a
 // chain of its own, because its roundings go into every segment behind the hand-off: A diag(beta),
@@ -937,7 +937,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           tc_fence_after();
           if (lane == 0) FQLA_TRACE(4, 3);
           if (elect_one()) {
-            umma_ts_loop8<2, 512, false>(tmem + TM_O1, tmem + TM_SB, q0_lo + so, ID_OT);
+            umma_ts_loop8<2, 512>(tmem + TM_O1, tmem + TM_SB, q0_lo + so, ID_OT);
             umma_commit(&bars[SB_FREE]);
           }
         }

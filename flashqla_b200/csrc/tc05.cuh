@@ -65,7 +65,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait.  `tries` is the thread's own count, WAIT_TRIES (about a second and more) at the start of each
 // pass of its loop; a wait that uses it up falls through, and so does every wait after it, until the loop looks
 // at the count and ends: one look a pass instead of a result at each of the dozens of wait sites, which were a
-// third of the kernels' code.  What a pass does after a wait was given up touches only the memory that it would
+// fifth of the kernels' code.  What a pass does after a wait was given up touches only the memory that it would
 // have touched anyway; its values are lost (the kernel sets its status word).  The thread is suspended by the
 // hardware meanwhile, but comes back early and often: trying again at once takes issue slots from the warps that
 // have work, hence the pause (chunk-parallel backward, 262144 tokens x 8 heads: 1510 us without it, 1260 with,
@@ -452,22 +452,18 @@ __device__ __forceinline__ void umma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uin
         : "memory");
   }
 }
-// Eight K-steps as two passes of a loop: B advances by B_STEP a step, by B_BLK a pass.
-template <int B_STEP, int B_BLK, bool ACC_FIRST>
+// Eight K-steps as two passes of a loop, fresh accumulator: B advances by B_STEP a step, by B_BLK a pass.
+template <int B_STEP, int B_BLK>
 __device__ __forceinline__ void umma_ts_loop8(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc) {
 #pragma unroll 1
   for (int b = 0; b < 2; ++b) {
-    if (ACC_FIRST) {
-      umma_ts_lo<true>(d_tmem, a_tmem, b_lo, idesc);
-    } else {
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-          "setp.ne.b32 p, %5, 0;\n\t"
-          "mov.b64 db, {%2, %3};\n\t"
-          "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
-          "r"(a_tmem), "r"(b_lo), "r"(DESC_HI), "r"(idesc), "r"(b)
-          : "memory");
-    }
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(b_lo), "r"(DESC_HI), "r"(idesc), "r"(b)
+        : "memory");
 #pragma unroll
     for (int j = 1; j < 4; ++j)
       umma_ts_lo<true>(d_tmem, a_tmem + (uint32_t)(8 * j), b_lo + (uint32_t)(j * B_STEP), idesc);
