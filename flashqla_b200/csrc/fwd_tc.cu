@@ -259,8 +259,8 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   if (tid == 0) {
     mbar_init(&bars[FULL0], 1);
     mbar_init(&bars[FULL1], 1);
-    mbar_init(&bars[EMPTY0], STATE ? 1 : 3);  // MMA commits of the issuing threads
-    mbar_init(&bars[EMPTY1], STATE ? 1 : 3);
+    mbar_init(&bars[EMPTY0], STATE ? 1 : NO_O ? 2 : 3);  // MMA commits of the issuing threads
+    mbar_init(&bars[EMPTY1], STATE ? 1 : NO_O ? 2 : 3);
     mbar_init(&bars[SB_FREE], 1);
     mbar_init(&bars[P_FREE], 128);
     mbar_init(&bars[U_DONE], 1);
@@ -389,8 +389,9 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       const int s = it & 1;
       if (v == 0) FQLA_TRACE(0, 0);
       if (it > 0) WAIT(S_DONE, (it - 1) & 1);
-      // the output product of the chunk before, issued by the other thread, has read the copy
-      if (!NO_O && it - 1 >= lead) WAIT(SB_FREE, (it - 1 - lead) & 1);
+      // the output product of the chunk before, issued by another thread, has read the copy (in a lead-in
+      // there is none, but its issuer signals all the same: see there)
+      if (!NO_O && it > 0) WAIT(SB_FREE, (it - 1) & 1);
       tc_fence_after();
       if (v == 0) FQLA_TRACE(0, 1);
       // on the chain: the bf16 operand copy of S^T, packed back into tensor memory.  (The products
@@ -907,21 +908,23 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         if (elect_one()) tma_store_wait_all();
       }
     } else if (warp == 1) {
+     if constexpr (!NO_O) {
       const uint32_t p_lo = desc_lo_kmajor(smem + OFF_P);
       const uint32_t q0_lo = desc_lo_kmajor(smem + OFF_STAGE);
       const uint32_t k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE_QK);
-      // (what is waited for by iteration is waited for in a lead-in, too: a parity tells a phase from its
-      // neighbours only)
+      // A parity tells a phase from its neighbours only, so nothing may run two chunks ahead of this warp.  Its
+      // products see to that; in a lead-in, where it has none, SB_FREE does, which the next state copy waits for,
+      // and it waits only for VN_DONE, which that copy comes before (and which implies W_READY of the same chunk
+      // and VB_READY of the one before).
 #pragma unroll 1
       for (int it = 0; it < n_it && more(); ++it) {
         const int s = it & 1, c = it - lead;
         const uint32_t so = s ? STAGE_LO : 0u;
-        const bool with_o = !NO_O && c >= 0;
         if (lane == 0) FQLA_TRACE(4, 0);
-        WAIT(FULL0 + s, (it >> 1) & 1);
-        WAIT(W_READY, it & 1);
         // P = Q K^T, over w^T; the prep group turns it into Pg
-        if (with_o) {
+        if (c >= 0) {
+          WAIT(FULL0 + s, (it >> 1) & 1);
+          WAIT(W_READY, it & 1);
           tc_fence_after();
           if (lane == 0) FQLA_TRACE(4, 1);
           if (elect_one()) {
@@ -932,20 +935,18 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         // O1^T = S^T Q^T   (A = packed S^T; B = q tile, K-major), behind Vn^T of the chain
         if (lane == 0) FQLA_TRACE(4, 2);
         WAIT(VN_DONE, it & 1);
-        if (with_o) {
-          if (c > 0) WAIT(O_FREE, (c - 1) & 1);
-          tc_fence_after();
-          if (lane == 0) FQLA_TRACE(4, 3);
-          if (elect_one()) {
-            umma_ts_loop8<2, 512>(tmem + TM_O1, tmem + TM_SB, q0_lo + so, ID_OT);
-            umma_commit(&bars[SB_FREE]);
-          }
+        if (c > 0) WAIT(O_FREE, (c - 1) & 1);
+        tc_fence_after();
+        if (lane == 0) FQLA_TRACE(4, 3);
+        if (elect_one()) {
+          if (c >= 0) umma_ts_loop8<2, 512>(tmem + TM_O1, tmem + TM_SB, q0_lo + so, ID_OT);
+          umma_commit(&bars[SB_FREE]);
+          umma_commit(&bars[EMPTY0 + s]);  // this thread's products that read the stage
         }
-        if (elect_one()) umma_commit(&bars[EMPTY0 + s]);  // this thread's products that read the stage
         if (lane == 0) FQLA_TRACE(4, 4);
-        WAIT(VB_READY, it & 1);
         // O2^T = Vn^T Pg^T   (A = packed Vn^T; B = Pg, K-major)
-        if (with_o) {
+        if (c >= 0) {
+          WAIT(VB_READY, it & 1);
           WAIT(P_READY, c & 1);
           tc_fence_after();
           if (lane == 0) FQLA_TRACE(4, 5);
@@ -956,6 +957,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         }
         if (lane == 0) FQLA_TRACE(4, 6);
       }
+     }
     } else {
       // w^T of iteration it + 1, behind Vn^T of iteration `it`, which stands on the chain (and for which w^T of
       // `it` has been made an operand), and behind Pg, made of P in the same columns.

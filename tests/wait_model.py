@@ -1,0 +1,436 @@
+"""A block of a warp-specialised kernel as its warps see it: who waits for which barrier, who arrives on it and
+who issues something asynchronous, read from the kernel's source and played on the CPU.
+
+``Kernel`` takes the part of the source between the first bounded wait's count and the teardown, and walks it
+once per warp: control flow, integers and lambdas are followed, everything else is passed over (a condition
+that an event depends on and that cannot be evaluated is an error).  ``nominal`` plays the warps in turn,
+``skipped_or_early`` says which waits a parity alone does not keep to their phase."""
+
+import itertools
+import os
+import re
+from types import SimpleNamespace
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "flashqla_b200", "csrc")
+EVENT = re.compile(r"\b(mbar_wait(?:_uniform)?|mbar_arrive(?:_expect_tx)?|umma_\w+|tma_(?:load|store)_2d|clc_try_cancel|"
+                   r"bar_all)\b|bar\.(?:sync|arrive)")
+BARRIER = re.compile(r"&bars\[(.*?)\]|^(\w+)$")
+
+
+def _close(text, at):
+    """index behind the bracket that opens at `at`"""
+    depth = 0
+    for i in range(at, len(text)):
+        depth += {"(": 1, "{": 1, "[": 1, ")": -1, "}": -1, "]": -1}.get(text[i], 0)
+        if depth == 0:
+            return i + 1
+    raise ValueError(text[at:at + 80])
+
+
+def _split(text, sep=","):
+    """at separators outside of brackets"""
+    parts, depth, start = [], 0, 0
+    for i, ch in enumerate(text):
+        depth += {"(": 1, "{": 1, "[": 1, ")": -1, "}": -1, "]": -1}.get(ch, 0)
+        if ch == sep and depth == 0:
+            parts.append(text[start:i])
+            start = i + 1
+    return [s.strip() for s in parts + [text[start:]]]
+
+
+def _statement(text, at):
+    """(node, index behind it)"""
+    rest = text[at:]
+    if m := re.match(r"(if|for|switch|while)\s*(constexpr)?\s*(?=\()", rest):
+        end = _close(text, at + m.end())
+        head = text[at + m.end() + 1:end - 1]
+        body, end = _next(text, end)
+        if m[1] != "if":
+            return (m[1], head, body), end
+        more = re.match(r"\s*else\b", text[end:])
+        other, end = _next(text, end + more.end()) if more else (None, end)
+        return ("if", head, body, other), end
+    if rest[0] == "{":
+        end = _close(text, at)
+        return ("block", _parse(text[at + 1:end - 1])), end
+    if m := re.match(r"(case\s+\w+|default)\s*:", rest):
+        return ("label", m[1].replace("case", "").strip()), at + m.end()
+    end = at
+    while text[end] != ";":
+        end = _close(text, end) if text[end] in "({[" else end + 1
+    return ("do", text[at:end].strip()), end + 1
+
+
+def _next(text, at):
+    return _statement(text, at + len(text[at:]) - len(text[at:].lstrip()))
+
+
+def _parse(text):
+    nodes, at = [], 0
+    while text[at:].strip():
+        node, at = _next(text, at)
+        nodes.append(node)
+    return nodes
+
+
+def _python(expr):
+    """A C++ expression over integers as a Python one."""
+    expr = re.sub(r"\((?:int|uint32_t|long long|bool)\)", "", expr.strip())
+    expr = re.sub(r"\b(0x[0-9a-f]+|\d+)u\b", r"\1", expr)
+    expr = re.sub(r"bar_all<(\d+), (\d+)>", r"bar_all", expr)
+    for open_ in reversed([m.start() for m in re.finditer(r"\(", expr)]):  # ternaries inside brackets first
+        end = _close(expr, open_)
+        inner = expr[open_ + 1:end - 1]
+        if "?" in inner:
+            expr = expr[:open_] + "(" + ", ".join(map(_python, _split(inner))) + ")" + expr[end:]
+    at = _split(expr, "?")
+    if len(at) > 1:
+        rest = "?".join(at[1:])
+        yes = _split(rest, ":")[0]
+        return f"(({_python(yes)}) if ({_python(at[0])}) else ({_python(rest[len(yes) + 1:].lstrip(': '))}))"
+    expr = expr.replace("&&", " and ").replace("||", " or ").replace(" / ", " // ")
+    return re.sub(r"!(?!=)", " not ", re.sub(r"\btrue\b", "True", re.sub(r"\bfalse\b", "False", expr))).strip()
+
+
+class Kernel:
+    """One block: `config` holds what the source's names stand for (template arguments, parameters)."""
+
+    def __init__(self, file, threads, config, text=None):
+        src = text if text is not None else open(os.path.join(CSRC, file)).read()
+        src = re.sub(r"//[^\n]*|^[ \t]*#[^\n]*", "", src, flags=re.M)
+        src = re.sub(r"(if \([^()]*\) )?(\{ const int it = [^;]*; )?FQLA_TRACE\([^;]*;( \})?", "", src)
+        self.names = {}
+        for body in re.findall(r"\benum \{(.*?)\}", src, flags=re.S):
+            value = -1
+            for item in _split(body):
+                name, _, same = (x.strip() for x in item.partition("="))
+                value = (self.names[same] if same in self.names else int(same)) if same else value + 1
+                self.names[name] = value
+        self.config, self.warps = dict(config), threads // 32
+        self.counts = {}
+        env = {**self.names, **self.config}
+        for head, bar, count in re.findall(r"(for \([^)]*\) )?mbar_init\(&bars\[(\w+)\], ([^;]+)\);", src):
+            if head:
+                first, last = re.search(r"= (\w+); i <= (\w+);", head).groups()
+                for b in range(self.names[first], self.names[last] + 1):
+                    self.counts[b] = eval(_python(count), {}, env)
+            elif bar in self.names:
+                self.counts[self.names[bar]] = eval(_python(count), {}, env)
+        at = src.index("int tries = WAIT_TRIES;")
+        self.nodes = _parse(src[at:src.index("tc_fence_before();\n  __syncthreads();\n  if (warp == 0) tmem_dealloc", at)])
+
+    # ---- one warp ---------------------------------------------------------------------------------------
+    def warp(self, index, shared):
+        """Generator of the warp's events: sends back what a wait (False: it ran out) or a vote gives."""
+        env = {**self.names, **self.config, **shared, "warp": index, "lane": 0, "tid": 32 * index, "tries": 1,
+               "WAIT_TRIES": 1, "elect_one": lambda: True, "__all_sync": lambda mask, x: x, "min": min, "max": max,
+               "abs": abs, "__shfl_sync": lambda mask, x, lane: x, "INT_MAX": 2**31 - 1}
+        lambdas = {}
+        yield from self._run(self.nodes, env, lambdas, False)
+
+    def _has_event(self, node, lambdas):
+        if node is None:
+            return False
+        if node[0] in ("block",):
+            return any(self._has_event(n, lambdas) for n in node[1])
+        if node[0] == "label":
+            return False
+        text = node[1]
+        if EVENT.search(text) and "= [&]" not in text:
+            return True
+        if node[0] == "do" and re.fullmatch(r"break|return|continue", text):
+            return True
+        if any(n in lambdas and lambdas[n][2] for n in re.findall(r"\b(\w+)\(", text)):
+            return True
+        return any(self._has_event(n, lambdas) for n in node[2:])
+
+    def _value(self, expr, env, lambdas):
+        """(a generator: an expression may hold a vote or call a lambda)"""
+        if m := re.search(r"bar_all<(\d+), (\d+)>\(", expr):
+            end = _close(expr, m.end() - 1)
+            mine = yield from self._value(expr[m.end():end - 1], env, lambdas)
+            result = yield "bar", int(m[1]), int(m[2]), bool(mine)
+            return eval(_python(expr[:m.start()] + str(result) + expr[end:]), {}, env)
+        for name in re.findall(r"\b(\w+)\(", expr):
+            if name in lambdas and name not in env:
+                at = re.search(rf"\b{name}\(", expr)
+                end = _close(expr, at.end() - 1)
+                args = [a for a in _split(expr[at.end():end - 1]) if a]
+                result = yield from self._call(name, args, env, lambdas, False)
+                expr = expr[:at.start()] + repr(result) + expr[end:]
+        return eval(_python(expr), {}, env)
+
+    def _call(self, name, args, env, lambdas, one):
+        params, body, _ = lambdas[name]
+        values = []
+        for a in args:
+            m = BARRIER.match(a)
+            try:
+                values.append(eval(_python(m[1] if m and m[1] else a), {}, env))
+            except NameError:  # an address
+                values.append(None)
+        old = {p: env.get(p) for p in params}
+        env.update(zip(params, values))
+        result = yield from self._run(body, env, lambdas, one)
+        env.update(old)
+        return result[1] if result and result[0] == "return" else None
+
+    def _run(self, nodes, env, lambdas, one):
+        """(`one`: inside a branch that a single lane takes.)  Returns why the walk ended early, or None."""
+        for node in nodes:
+            kind = node[0]
+            if kind == "block":
+                out = yield from self._run(node[1], env, lambdas, one)
+                if out:
+                    return out
+            elif kind == "if":
+                if not (self._has_event(node[2], lambdas) or self._has_event(node[3], lambdas)
+                        or EVENT.search(node[1])):
+                    # an assignment under a condition counts if both can be followed
+                    try:
+                        branch = node[2] if eval(_python(node[1]), {}, env) else node[3]
+                    except Exception:
+                        continue
+                    if branch:
+                        yield from self._run([branch], env, lambdas, one)
+                    continue
+                cond = yield from self._value(node[1], env, lambdas)
+                single = one or bool(re.search(r"elect_one\(\)|lane == 0|issuing\(\)", node[1]))
+                branch = node[2] if cond else node[3]
+                if branch:
+                    out = yield from self._run([branch], env, lambdas, single if cond else one)
+                    if out:
+                        return out
+            elif kind == "for":
+                if not self._has_event(node[2], lambdas):
+                    continue
+                init, cond, step = _split(node[1], ";")
+                if init:
+                    self._assign(re.sub(r"^(?:int|bool|uint32_t) ", "", init), env)
+                while not cond or (yield from self._value(cond, env, lambdas)):
+                    out = yield from self._run([node[2]], env, lambdas, one)
+                    if out and out[0] == "break":
+                        break
+                    if out and out[0] != "continue":
+                        return out
+                    if step:
+                        self._assign(step, env)
+            elif kind == "switch":
+                want = str((yield from self._value(node[1], env, lambdas)))
+                body = node[2][1]
+                labels = [i for i, n in enumerate(body) if n[0] == "label"]
+                at = next((i for i in labels if body[i][1] == want), None)
+                if at is None:
+                    at = next(i for i in labels if body[i][1] == "default")
+                out = yield from self._run([n for n in body[at + 1:] if n[0] != "label"], env, lambdas, one)
+                if out and out[0] == "return":
+                    return out
+            elif kind == "do":
+                out = yield from self._do(node[1], env, lambdas, one)
+                if out:
+                    return out
+        return None
+
+    def _assign(self, text, env):
+        m = re.match(r"(?:\+\+(\w+)|([\w.]+(?:\[.*?\])?) ([\^+|-]?)= (.*))$", text, flags=re.S)
+        if not m:
+            return
+        if m[1]:
+            env[m[1]] += 1
+            return
+        value = _python(m[4] if not m[3] else f"{m[2]} {m[3]} ({m[4]})")
+        if re.fullmatch(r"\w+", m[2]):
+            env[m[2]] = eval(value, {}, env)
+        else:
+            exec(f"{m[2]} = {value}", {}, env)
+
+    def _do(self, text, env, lambdas, one):
+        if text in ("break", "continue"):
+            return (text,)
+        if m := re.match(r"return\b(.*)", text, flags=re.S):
+            return "return", (yield from self._value(m[1], env, lambdas)) if m[1].strip() else None
+        if m := re.match(r"auto (\w+) = \[&\]\s*(?:\((.*?)\))?\s*(?=\{)", text, flags=re.S):
+            params = [re.split(r"[\s&*]+", p)[-1] for p in _split(m[2] or "") if p]
+            body = _parse(text[m.end() + 1:_close(text, m.end()) - 1])
+            lambdas[m[1]] = (params, body, False)
+            lambdas[m[1]] = (params, body, any(self._has_event(n, lambdas) for n in body))
+            return None
+        if m := re.match(r'asm volatile\("bar\.(sync|arrive) (\d+), (\d+);"', text):
+            yield ("bar" if m[1] == "sync" else "bar_arrive"), int(m[2]), int(m[3]), True
+            return None
+        if m := re.match(r"(\w+)(?:<.*?>)?\((.*)\)$", text, flags=re.S):
+            name, args = m[1], [a for a in _split(m[2]) if a]
+            if name.startswith("mbar_wait"):
+                bar = eval(_python(BARRIER.match(args[0])[1]), {}, env)
+                ok = yield "wait", bar, eval(_python(args[1]), {}, env) & 1
+                if not ok:
+                    env["tries"] = 0
+                return None
+            if name in ("mbar_arrive", "mbar_arrive_expect_tx", "umma_commit"):
+                b = BARRIER.match(args[0])
+                bar = eval(_python(b[1] or b[2]), {}, env)
+                yield "arrive", bar, 1 if one or name != "mbar_arrive" else 32
+                return None
+            if EVENT.match(name):
+                yield "issue", name, None
+                return None
+            if name in lambdas and name not in env:
+                if lambdas[name][2]:
+                    yield from self._call(name, args, env, lambdas, one)
+                return None
+        if m := re.match(r"uint64_t\* (\w+) = &bars\[(.*)\]$", text, flags=re.S):
+            env[m[1]] = eval(_python(m[2]), {}, env)
+            return None
+        m = re.match(r"(?:const |constexpr )?(?:int|bool|uint32_t|long long|Item) (.*)$", text, flags=re.S)
+        for part in _split(m[1] if m else text):
+            try:
+                if m and "=" in part and any(n in lambdas for n in re.findall(r"\b(\w+)\(", part)):
+                    name, _, expr = part.partition("=")
+                    env[name.strip()] = yield from self._value(expr.strip(), env, lambdas)
+                else:
+                    self._assign(part, env)
+            except Exception:  # not an integer that can be followed
+                pass
+        return None
+
+
+# ---- several warps --------------------------------------------------------------------------------------
+class _Block:
+    """The barriers of a block while its warps are played."""
+
+    def __init__(self, kernel, shared=dict):
+        self.kernel, self.done, self.pending, self.arrived = kernel, {}, dict(kernel.counts), {}
+        shared = shared()
+        self.warps = [kernel.warp(w, shared) for w in range(kernel.warps)]
+        self.at = [next(g, None) for g in self.warps]  # the event each warp stands at
+
+    def phase(self, bar, parity):
+        """the phase that a wait for `parity` sees completed, or None"""
+        done = self.done.get(bar, 0)
+        return done - 1 if (done - 1) & 1 == parity else None
+
+    def arrive(self, bar, n):
+        """the phase that it counts for"""
+        phase = self.done.get(bar, 0)
+        self.pending[bar] -= n
+        assert self.pending[bar] >= 0, f"barrier {bar}: more arrivals than its count"
+        if self.pending[bar] == 0:
+            self.done[bar], self.pending[bar] = phase + 1, self.kernel.counts[bar]
+        return phase
+
+    def go_on(self, w, value=None):
+        try:
+            self.at[w] = self.warps[w].send(value)
+        except StopIteration:
+            self.at[w] = None
+
+
+def nominal(kernel, shared=dict):
+    """[(warp, event, phase)] in an order in which the warps take turns; raises if they stop."""
+    block, log, named = _Block(kernel, shared), [], {}
+    while any(e is not None for e in block.at):
+        moved = False
+        for w, e in enumerate(block.at):
+            if e is None or (e[0] == "bar" and (w in named.get(e[1], {}))):
+                continue
+            value, phase = None, None
+            if e[0] == "wait":
+                phase = block.phase(e[1], e[2])
+                if phase is None:
+                    continue
+                value = True
+            elif e[0] == "arrive":
+                phase = block.arrive(e[1], e[2])
+            elif e[0].startswith("bar"):
+                here = named.setdefault(e[1], {})
+                here[w] = e
+                moved = True
+                if 32 * len(here) < e[2]:
+                    if e[0] == "bar_arrive":
+                        log.append((w, e, len(log)))
+                        block.go_on(w)
+                    continue
+                phase = len(log)
+                for other, ev in here.items():
+                    if ev[0] == "bar":
+                        log.append((other, ev, phase))
+                        block.go_on(other, all(x[3] for x in here.values()))
+                named[e[1]] = {}
+                continue
+            log.append((w, e, phase))
+            block.go_on(w, value)
+            moved = True
+        if not moved:
+            raise AssertionError(f"the warps stop: {[(w, e) for w, e in enumerate(block.at) if e]}")
+    return log
+
+
+def order(log):
+    """(follows, waits, arrivals): follows(a, b) says whether event b of the log comes after event a in every
+    run, by program order and by arrivals that a wait has seen complete; named barriers order nothing here."""
+    nodes = {}  # (warp, n-th event) in program order
+    seen, waits, arrivals = {}, [], {}
+    for i, (w, e, phase) in enumerate(log):
+        nodes[i] = seen.get(w)
+        seen[w] = i
+        if e[0] == "wait":
+            waits.append((i, e[1], phase))
+        elif e[0] == "arrive":
+            arrivals.setdefault((e[1], phase), []).append(i)
+    before = [0] * len(log)  # bit set of everything that comes before
+    by_wait = {i: (b, k) for i, b, k in waits}
+    for i in range(len(log)):
+        prev = nodes[i]
+        bits = 0 if prev is None else before[prev] | 1 << prev
+        if i in by_wait:
+            for a in arrivals.get(by_wait[i], []):
+                bits |= before[a] | 1 << a
+        before[i] = bits
+    return (lambda a, b: bool(before[b] >> a & 1)), nodes, waits, arrivals
+
+
+def skipped_or_early(kernel, shared=dict):
+    """Waits that a parity alone does not keep to their phase: the phase before may still be open when the wait
+    begins (it would be over at once), or the phase behind may be over before the wait has been (its parity would
+    not come round).  Barriers whose phases the loads complete count by the arrival that goes with the loads."""
+    log = nominal(kernel, shared)
+    follows, previous, waits, arrivals = order(log)
+    name = {v: k for k, v in reversed(list(kernel.names.items()))}
+    wrong = set()
+    for i, bar, phase in waits:
+        prev = previous[i]
+        if any(prev is None or not (a == prev or follows(a, prev)) for a in arrivals.get((bar, phase - 1), [])):
+            wrong.add((log[i][0], name[bar], "early"))
+        after = arrivals.get((bar, phase + 1), [])
+        complete = sum(log[a][1][2] for a in after) >= kernel.counts[bar]
+        if complete and not any(follows(i, a) for a in after):
+            wrong.add((log[i][0], name[bar], "skipped"))
+    return sorted(wrong)
+
+
+def forward(no_o=False, extra=False, lead=0, n_it=7, partial=False, tiled=1, text=None):
+    """The forward recurrence over n_it chunks, the first `lead` of them lead-in."""
+    n_chunks = n_it - lead
+    p = SimpleNamespace(h=extra, vnew=extra, tiled=tiled, o=not no_o, scale=1.0, Hv=1, N=1, lay=SimpleNamespace(
+        cu=SimpleNamespace(ptr=0)), ht=1, M=0, ht_row=0)
+    config = dict(NO_O=no_o, EXTRA=extra, STATE=no_o and not extra, PREP=12 if no_o else 16, p=p, n_it=n_it, lead=lead,
+                  n_chunks=n_chunks, sp=SimpleNamespace(len=64 * n_chunks - (10 if partial else 0), bos=0, chunk_base=0),
+                  CHUNK=64, tile_h=extra and tiled, tile_vn=extra and tiled, m_pass=False, hv=0, hq=0, n=0, D=128)
+    return Kernel("fwd_tc.cu", 512 if no_o else 640, config, text=text)
+
+
+def reverse(lead=0, n_it=7, partial=False, tiled=1, text=None):
+    """The reverse recurrence likewise."""
+    n_chunks = n_it - lead
+    p = SimpleNamespace(dh=1, du=1, tiled=tiled, scale=1.0, Hv=1, dh0=1, dh0_row=0)
+    config = dict(p=p, n_it=n_it, lead=lead, len_ext=64 * n_it - (10 if partial else 0), CHUNK=64, hv=0, hq=0, n=0, D=128,
+                  sp=SimpleNamespace(len=64 * n_chunks, bos=0, chunk_base=0))
+    return Kernel("bwd_dh_tc.cu", 512, config, text=text)
+
+
+CASES = [*itertools.chain(
+    (("forward", dict(lead=lead, extra=extra, partial=partial)) for lead, extra, partial in
+     itertools.product((0, 1, 2, 3), (False, True), (False, True))),
+    (("forward", dict(no_o=True, extra=extra, partial=partial)) for extra, partial in
+     itertools.product((False, True), (False, True))),
+    (("reverse", dict(lead=lead, partial=partial)) for lead, partial in itertools.product((0, 1, 2, 3), (False, True))))]
