@@ -639,8 +639,6 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       const float* sg = vec + (it & 3) * VEC_SLOT_FLOATS + V_SGAM * CHUNK;
       const long long row0 = sp.bos + (long long)c * CHUNK;
       const int valid = min(CHUNK, sp.len - c * CHUNK);
-      if (wq == 0 && elect_one()) tma_store_wait_read();  // the store of the chunk before has read the tile
-      asm volatile("bar.sync 1, 128;" ::: "memory");
       // The accumulators hold o transposed ([value index][token]).  Read with the 16-lane shape, a
       // lane gets mma-style fragments: rows l/4 and l/4 + 8 of a 16-row half, token pairs
       // 8 i + 2 (l%4), +1.  stmatrix with .trans writes each 8 x 8 fragment block transposed, i.e.
@@ -704,7 +702,9 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     for (int c = max(-lead, 0); c < n_it - lead && more(); ++c) {
       if (v == 0) { const int it = c + lead; FQLA_TRACE(2, 0); }
       WAIT(O_DONE, c & 1);
-      if (tries <= 0) break;  // nothing is stored of what is not complete
+      if (wq == 0 && elect_one()) tma_store_wait_read();  // the store of the chunk before has read the tile
+      // nothing is stored of what is not complete, and the four warps, which meet again behind this, go as one
+      if (!bar_all<1, 128>(tries > 0)) break;
       tc_fence_after();
       if (v == 0) { const int it = c + lead; FQLA_TRACE(2, 1); }
       epilogue(c);

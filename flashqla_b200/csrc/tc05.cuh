@@ -92,6 +92,22 @@ __device__ __forceinline__ void mbar_wait_uniform(uint64_t* bar, uint32_t parity
   while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity)) && --tries > 0) __nanosleep(20);
 }
 
+// Named barrier ID of N threads that tells all of them alike whether `ok` holds for each: a group that meets at
+// barriers leaves its loop as one, although each thread counts its own tries.
+template <int ID, int N>
+__device__ __forceinline__ bool bar_all(bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"((uint32_t)ok), "n"(ID), "n"(N)
+      : "memory");
+  return all != 0;
+}
+
 // Four 8 x 8 bf16 matrices from registers to shared memory, each stored TRANSPOSED: register i of
 // lane l carries the elements (row l/4, columns 2(l%4), +1) of matrix i - the layout of an
 // mma / 16x256b tensor-memory fragment - and lands at (row 2(l%4) + {0,1}, column l/4) of the

@@ -1,0 +1,24 @@
+"""What a block does when one of its bounded waits runs out, from the kernels' source (see wait_model.py): each
+wait of the first and the last warp of every role in turn, the waits that are then left open running out from either
+end.  Nothing is run on a device."""
+
+import pytest
+import wait_model
+
+FORMS = [("forward", dict(n_it=2)), ("forward", dict(n_it=2, lead=1, extra=True, partial=True)),
+         ("forward", dict(n_it=2, no_o=True, extra=True)), ("forward", dict(n_it=2, no_o=True)),
+         ("reverse", dict(n_it=2, partial=True))]
+
+
+@pytest.fixture(scope="module", params=FORMS, ids=lambda f: "-".join([f[0], *f[1]]))
+def plays(request):
+    """(warps left at a named barrier, what a warp signalled or issued behind its own wait) of every play"""
+    name, form = request.param
+    kernel = getattr(wait_model, name)(**form)
+    warps = [w for w in range(kernel.warps) if w < 4 or w % 4 in (0, 3)]
+    return [wait_model.given_up(kernel, w, nth, last_first) for w in warps
+            for nth in range(wait_model.waits_of(kernel, w)) for last_first in (False, True)]
+
+
+def test_every_warp_comes_to_the_end(plays):
+    assert [left for left, _ in plays if left] == []

@@ -4,8 +4,10 @@ who issues something asynchronous, read from the kernel's source and played on t
 ``Kernel`` takes the part of the source between the first bounded wait's count and the teardown, and walks it
 once per warp: control flow, integers and lambdas are followed, everything else is passed over (a condition
 that an event depends on and that cannot be evaluated is an error).  ``nominal`` plays the warps in turn,
-``skipped_or_early`` says which waits a parity alone does not keep to their phase."""
+``skipped_or_early`` says which waits a parity alone does not keep to their phase, ``given_up`` plays them with
+one wait that runs out."""
 
+import functools
 import itertools
 import os
 import re
@@ -73,6 +75,7 @@ def _parse(text):
     return nodes
 
 
+@functools.lru_cache(None)
 def _python(expr):
     """A C++ expression over integers as a Python one."""
     expr = re.sub(r"\((?:int|uint32_t|long long|bool)\)", "", expr.strip())
@@ -92,6 +95,15 @@ def _python(expr):
     return re.sub(r"!(?!=)", " not ", re.sub(r"\btrue\b", "True", re.sub(r"\bfalse\b", "False", expr))).strip()
 
 
+@functools.lru_cache(None)
+def _code(expr):
+    return compile(_python(expr), "<source>", "eval")
+
+
+def _eval(expr, env):
+    return eval(_code(expr), {}, env)
+
+
 class Kernel:
     """One block: `config` holds what the source's names stand for (template arguments, parameters)."""
 
@@ -107,15 +119,15 @@ class Kernel:
                 value = (self.names[same] if same in self.names else int(same)) if same else value + 1
                 self.names[name] = value
         self.config, self.warps = dict(config), threads // 32
-        self.counts = {}
+        self.counts, self.eventful, self.bodies = {}, {}, {}
         env = {**self.names, **self.config}
         for head, bar, count in re.findall(r"(for \([^)]*\) )?mbar_init\(&bars\[(\w+)\], ([^;]+)\);", src):
             if head:
                 first, last = re.search(r"= (\w+); i <= (\w+);", head).groups()
                 for b in range(self.names[first], self.names[last] + 1):
-                    self.counts[b] = eval(_python(count), {}, env)
+                    self.counts[b] = _eval(count, env)
             elif bar in self.names:
-                self.counts[self.names[bar]] = eval(_python(count), {}, env)
+                self.counts[self.names[bar]] = _eval(count, env)
         at = src.index("int tries = WAIT_TRIES;")
         self.nodes = _parse(src[at:src.index("tc_fence_before();\n  __syncthreads();\n  if (warp == 0) tmem_dealloc", at)])
 
@@ -131,7 +143,12 @@ class Kernel:
     def _has_event(self, node, lambdas):
         if node is None:
             return False
-        if node[0] in ("block",):
+        if id(node) not in self.eventful:  # (a lambda is known before the code that calls it)
+            self.eventful[id(node)] = self._find_event(node, lambdas)
+        return self.eventful[id(node)]
+
+    def _find_event(self, node, lambdas):
+        if node[0] == "block":
             return any(self._has_event(n, lambdas) for n in node[1])
         if node[0] == "label":
             return False
@@ -150,7 +167,7 @@ class Kernel:
             end = _close(expr, m.end() - 1)
             mine = yield from self._value(expr[m.end():end - 1], env, lambdas)
             result = yield "bar", int(m[1]), int(m[2]), bool(mine)
-            return eval(_python(expr[:m.start()] + str(result) + expr[end:]), {}, env)
+            return _eval(expr[:m.start()] + str(result) + expr[end:], env)
         for name in re.findall(r"\b(\w+)\(", expr):
             if name in lambdas and name not in env:
                 at = re.search(rf"\b{name}\(", expr)
@@ -158,7 +175,7 @@ class Kernel:
                 args = [a for a in _split(expr[at.end():end - 1]) if a]
                 result = yield from self._call(name, args, env, lambdas, False)
                 expr = expr[:at.start()] + repr(result) + expr[end:]
-        return eval(_python(expr), {}, env)
+        return _eval(expr, env)
 
     def _call(self, name, args, env, lambdas, one):
         params, body, _ = lambdas[name]
@@ -166,7 +183,7 @@ class Kernel:
         for a in args:
             m = BARRIER.match(a)
             try:
-                values.append(eval(_python(m[1] if m and m[1] else a), {}, env))
+                values.append(_eval(m[1] if m and m[1] else a, env))
             except NameError:  # an address
                 values.append(None)
         old = {p: env.get(p) for p in params}
@@ -188,7 +205,7 @@ class Kernel:
                         or EVENT.search(node[1])):
                     # an assignment under a condition counts if both can be followed
                     try:
-                        branch = node[2] if eval(_python(node[1]), {}, env) else node[3]
+                        branch = node[2] if _eval(node[1], env) else node[3]
                     except Exception:
                         continue
                     if branch:
@@ -251,7 +268,9 @@ class Kernel:
             return "return", (yield from self._value(m[1], env, lambdas)) if m[1].strip() else None
         if m := re.match(r"auto (\w+) = \[&\]\s*(?:\((.*?)\))?\s*(?=\{)", text, flags=re.S):
             params = [re.split(r"[\s&*]+", p)[-1] for p in _split(m[2] or "") if p]
-            body = _parse(text[m.end() + 1:_close(text, m.end()) - 1])
+            if text not in self.bodies:  # (parsed once: nodes are told apart by identity)
+                self.bodies[text] = _parse(text[m.end() + 1:_close(text, m.end()) - 1])
+            body = self.bodies[text]
             lambdas[m[1]] = (params, body, False)
             lambdas[m[1]] = (params, body, any(self._has_event(n, lambdas) for n in body))
             return None
@@ -261,14 +280,14 @@ class Kernel:
         if m := re.match(r"(\w+)(?:<.*?>)?\((.*)\)$", text, flags=re.S):
             name, args = m[1], [a for a in _split(m[2]) if a]
             if name.startswith("mbar_wait"):
-                bar = eval(_python(BARRIER.match(args[0])[1]), {}, env)
-                ok = yield "wait", bar, eval(_python(args[1]), {}, env) & 1
+                bar = _eval(BARRIER.match(args[0])[1], env)
+                ok = yield "wait", bar, _eval(args[1], env) & 1
                 if not ok:
                     env["tries"] = 0
                 return None
             if name in ("mbar_arrive", "mbar_arrive_expect_tx", "umma_commit"):
                 b = BARRIER.match(args[0])
-                bar = eval(_python(b[1] or b[2]), {}, env)
+                bar = _eval(b[1] or b[2], env)
                 yield "arrive", bar, 1 if one or name != "mbar_arrive" else 32
                 return None
             if EVENT.match(name):
@@ -279,7 +298,7 @@ class Kernel:
                     yield from self._call(name, args, env, lambdas, one)
                 return None
         if m := re.match(r"uint64_t\* (\w+) = &bars\[(.*)\]$", text, flags=re.S):
-            env[m[1]] = eval(_python(m[2]), {}, env)
+            env[m[1]] = _eval(m[2], env)
             return None
         m = re.match(r"(?:const |constexpr )?(?:int|bool|uint32_t|long long|Item) (.*)$", text, flags=re.S)
         for part in _split(m[1] if m else text):
@@ -406,6 +425,59 @@ def skipped_or_early(kernel, shared=dict):
         if complete and not any(follows(i, a) for a in after):
             wrong.add((log[i][0], name[bar], "skipped"))
     return sorted(wrong)
+
+
+def given_up(kernel, warp, nth, last_first, shared=dict):
+    """Plays the block with the `nth` wait of `warp` running out; whenever nobody can go on, the waits that are
+    open run out one at a time (from the highest or the lowest warp).  Returns (warps left at a named barrier,
+    [(warp, event)] that was signalled or issued by a warp behind a wait of its own that had run out)."""
+    block, named, late = _Block(kernel, shared), {}, []
+    out, count = set(), [0] * kernel.warps
+    while True:
+        moved = False
+        for w in range(kernel.warps):
+            while (e := block.at[w]) is not None:
+                if e[0] == "wait":
+                    ok = block.phase(e[1], e[2]) is not None
+                    if w == warp and count[w] == nth:
+                        out.add(w)
+                        ok = False
+                    if not ok and w not in out:
+                        break
+                    count[w] += 1
+                    block.go_on(w, ok)
+                elif e[0].startswith("bar"):
+                    here = named.setdefault(e[1], {})
+                    if w in here:
+                        break
+                    here[w] = e
+                    if e[0] == "bar_arrive":
+                        block.go_on(w)
+                    if 32 * len(here) == e[2]:
+                        named[e[1]] = {}
+                        for other, ev in here.items():
+                            if ev[0] == "bar":
+                                block.go_on(other, all(x[3] for x in here.values()))
+                    elif e[0] == "bar":
+                        moved = True
+                        break
+                else:
+                    if w in out:
+                        late.append((w, e))
+                    if e[0] == "arrive":
+                        block.arrive(e[1], e[2])
+                    block.go_on(w)
+                moved = True
+        if not moved:
+            open_ = [w for w, e in enumerate(block.at) if e is not None and e[0] == "wait"]
+            if not open_:
+                break
+            out.add(open_[-1] if last_first else open_[0])
+    return [(w, e) for w, e in enumerate(block.at) if e is not None], late
+
+
+def waits_of(kernel, warp, shared=dict):
+    return sum(1 for w, e, _ in nominal(kernel, shared) if w == warp and e[0] == "wait")
 
 
 def forward(no_o=False, extra=False, lead=0, n_it=7, partial=False, tiled=1, text=None):
