@@ -184,17 +184,13 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
-  int tries = WAIT_TRIES;  // see mbar_wait; `more`: none was given up, on to the next pass of a role's loop
+  // see mbar_wait; `more`: no lane of the warp has given a wait up, on to the next pass of its role's loop
+  int tries = WAIT_TRIES;
   auto WAIT = [&](int idx, uint32_t parity) { mbar_wait(&bars[idx], parity, tries); };
   // (of the issuing warps: see mbar_wait_uniform; 262144 tokens x 8 heads 584 us, 590 with the plain ones)
   auto WAITU = [&](int idx, uint32_t parity) { mbar_wait_uniform(&bars[idx], parity, tries); };
-  auto more_u = [&] {
-    const bool ok = __all_sync(0xffffffffu, tries > 0);
-    if (ok) tries = WAIT_TRIES;
-    return ok;
-  };
   auto more = [&] {
-    const bool ok = tries > 0;
+    const bool ok = __all_sync(0xffffffffu, tries > 0);
     if (ok) tries = WAIT_TRIES;
     return ok;
   };
@@ -304,9 +300,9 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       tc_fence_before();
       mbar_arrive(&bars[S_DEC]);
     }
-    if (tries > 0 && n_it > 0) WAIT(S_DONE, (n_it - 1) & 1);
+    if (n_it > 0) WAIT(S_DONE, (n_it - 1) & 1);
     const int dh0_row = p.dh0_row ? p.dh0_row[n] : n;
-    if (tries > 0 && p.dh0 && dh0_row >= 0) {
+    if (more() && p.dh0 && dh0_row >= 0) {
       float* dst = p.dh0 + ((long long)dh0_row * p.Hv + hv) * D * D;
       tc_fence_after();
 #pragma unroll 1
@@ -469,7 +465,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       const uint32_t st_lo = desc_lo_kmajor(smem + OFF_ST), dvt_lo = desc_lo_kmajor(smem + OFF_DVT);
       const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 8192), qmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE, 8192);
 #pragma unroll 1
-      for (int it = 0; it < n_it && more_u(); ++it) {
+      for (int it = 0; it < n_it && more(); ++it) {
         const int s = it & 1;
         const uint32_t so = s ? STAGE_LO : 0u;
         const int y_tile = (int)(((sp.chunk_base + (n_it - 1 - it)) * p.Hv + hv) * D);
@@ -512,7 +508,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE, 8192);
       const uint32_t app_lo = desc_lo_kmajor(smem + OFF_APP), pmn_lo = desc_lo_mnmajor(smem + OFF_P, 8192);
 #pragma unroll 1
-      for (int it = 0; it < n_it && more_u(); ++it) {
+      for (int it = 0; it < n_it && more(); ++it) {
         const int s = it & 1;
         const uint32_t so = s ? STAGE_LO : 0u;
         // (the Pg group has read P of the chunk before: P_READY was waited for)

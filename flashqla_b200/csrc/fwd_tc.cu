@@ -317,10 +317,11 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;  // this warp's lane quarter
-  int tries = WAIT_TRIES;  // see mbar_wait; `more`: none was given up, on to the next pass of a role's loop
+  // see mbar_wait; `more`: no lane of the warp has given a wait up, on to the next pass of its role's loop
+  int tries = WAIT_TRIES;
   auto WAIT = [&](int idx, uint32_t parity) { mbar_wait(&bars[idx], parity, tries); };
   auto more = [&] {
-    const bool ok = tries > 0;
+    const bool ok = __all_sync(0xffffffffu, tries > 0);
     if (ok) tries = WAIT_TRIES;
     return ok;
   };
@@ -455,10 +456,10 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       mbar_arrive(&bars[S_DEC]);
       if (v == 0) FQLA_TRACE(0, 4);
     }
-    if (tries > 0 && n_it > 0) WAIT(S_DONE, (n_it - 1) & 1);
+    if (n_it > 0) WAIT(S_DONE, (n_it - 1) & 1);
     const int ht_row = p.ht_row && !m_pass ? p.ht_row[n] : n;
     float* end = m_pass ? p.M : p.ht;
-    if (tries > 0 && end && ht_row >= 0) {
+    if (more() && end && ht_row >= 0) {
       float* dst = end + ((long long)ht_row * p.Hv + hv) * D * D;
       tc_fence_after();
 #pragma unroll 1

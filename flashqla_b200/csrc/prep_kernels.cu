@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(32 * kkt::MAX_WARPS, 3) kkt_solve_kernel(
   int tries = tc::WAIT_TRIES;
 
 #pragma unroll 1
-  for (int gi = warp; gi < G && tries > 0; gi += n_warps) {
+  for (int gi = warp; gi < G; gi += n_warps) {
     const int hv = hq * G + gi;
     {  // gates and beta of the rows lane, lane + 32
       float x[2];
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(32 * kkt::MAX_WARPS, 3) kkt_solve_kernel(
       sG[lane + 32] = x[1] * 1.4426950408889634f;
     }
     tc::mbar_wait(bar, 0, tries);
-    if (tries <= 0) break;
+    if (!__all_sync(0xffffffffu, tries > 0)) break;
     __syncwarp();
 
     // ---- 1. K K^T, lower blocks (rb, cb), index rb (rb + 1) / 2 + cb
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(32 * kkt::MAX_WARPS, 3) kkt_solve_kernel(
     }
   }  // value heads of this warp
   if (lane == 0) tc::tma_store_wait_read();  // shared memory outlives the stores' reads
-  if (tries <= 0 && lane == 0) atomicCAS(&g_kkt_status, 0, 1);
+  if (tries <= 0) atomicCAS(&g_kkt_status, 0, 1);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -2,6 +2,9 @@
 wait of the first and the last warp of every role in turn, the waits that are then left open running out from either
 end.  Nothing is run on a device."""
 
+import os
+import re
+
 import pytest
 import wait_model
 
@@ -22,3 +25,15 @@ def plays(request):
 
 def test_every_warp_comes_to_the_end(plays):
     assert [left for left, _ in plays if left] == []
+
+
+@pytest.mark.parametrize("file", ["fwd_tc.cu", "bwd_dh_tc.cu", "prep_kernels.cu"])
+def test_a_warp_goes_on_or_leaves_as_one(file):
+    """Each lane counts its own tries, and what stands behind a wait are instructions of whole warps: a look at the
+    count decides for the warp (a vote), for a group (a barrier's) or for what one lane does alone."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(wait_model.CSRC, file)).read())
+    alone = (r"__all_sync\(0xffffffffu, tries > 0\)", r"bar_all<\d+, \d+>\(tries > 0\)", r"elect_one\(\) && tries > 0",
+             r"if \(tries <= 0\) \*abort_flag = 1;", r"if \(tries <= 0\) atomicCAS\(", r"if \(tries > 0\) mbar_arrive\(")
+    looks = re.findall(r"[^\n]*\btries (?:>|<=) 0[^\n]*", text)
+    assert looks
+    assert [line.strip() for line in looks if not any(re.search(a, line) for a in alone)] == []
