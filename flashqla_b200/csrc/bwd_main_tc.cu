@@ -218,10 +218,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   int tries = WAIT_TRIES;  // see mbar_wait; filled up for each item
-  auto WAIT = [&](int idx, uint32_t parity) {
-    mbar_wait(&bars[idx], parity, tries);
-    return tries > 0;
-  };
+  auto WAIT = [&](int idx, uint32_t parity) { mbar_wait(&bars[idx], parity, tries); };
 
   if (warp == N_EPI / 32) {
     // ====================== issue warp: TMA loads and every tcgen05.mma ======================
@@ -423,7 +420,6 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         }
         cur = nxt;
       }
-      if (tries <= 0) *abort_flag = 1;
     }
   } else {
     // ====================== read-out warps ======================
@@ -608,6 +604,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         WAIT(L_D, ph);
         {
           tc_fence_after();
+          const int rows = tries > 0 ? valid : 0;  // (nothing is stored of what is not complete)
           float x[32];
           tmem_ld_16x64(tmem + lanes + T_DW + 64 * half, x);
           tmem_ld_wait();
@@ -642,7 +639,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
             const int row = 16 * qd + 4 * j + (lane >> 3);
             const uint4 w = *reinterpret_cast<const uint4*>(smem + OFF_V + half * 8192 + row * 128 +
                                                             (((lane & 7) ^ (row & 7)) << 4));
-            if (row < valid)
+            if (row < rows)
               *reinterpret_cast<uint4*>(p.dv + ((cur.row0 + row) * p.Hv + cur.hv) * D + 64 * half + 8 * (lane & 7)) = w;
           }
         }
@@ -821,6 +818,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         WAIT(C_5, ph);
         {
           tc_fence_after();
+          const int rows = tries > 0 ? valid : 0;
           bf16* out = hi ? p.dk : p.dq;
           const float f_y = hi ? -sBeta[row_w] * sGam[row_w] : 0.f;
           float s = 0.f;
@@ -851,7 +849,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
                 pc[2 * z + j] = pack8(x + 8 * j);
               }
             }
-            store_rows(out, out_q + 32 * pass, row_q, valid, pc);
+            store_rows(out, out_q + 32 * pass, row_q, rows, pc);
           }
           acc_w += f_y * s;
           if (hi) sRowDb[128 + half * 64 + row_w] = -sGam[row_w] * s;
@@ -866,17 +864,16 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       // ends an item with the wide read-outs, follows at most an item behind (R_E4) and finds the
       // chain group's contributions to dg, db and the vectors of the next item (other buffer)
       // behind R_CH.  (One barrier of all sixteen warps here held the chain group for the last
-      // wide read-out, 1600 of 14500 cycles per item.)  Each group has a stop flag of its own, by
-      // item parity, so that it is read by the whole group before it can be written again.
-      bool ok = tries > 0;
+      // wide read-out, 1600 of 14500 cycles per item.)  A thread that has given a wait up takes its group
+      // along: each group has a stop flag of its own, by item parity, so that it is read by the whole group before
+      // it can be written again, and behind the barrier all threads of a group go the same way.
+      const int stop = (chain ? 0 : 2) + (int)ph;
       if (chain) {
         if (nxt.valid > 0) write_vectors(nxt, ph ? sVec0 : sVec1);
       } else {
-        ok = ok && WAIT(R_CH, ph);
+        WAIT(R_CH, ph);
       }
-      if (!ok) *abort_flag = 1;
-      volatile int* stop = stop_flag + (chain ? 0 : 2) + ph;
-      if ((tid & 255) == 0) *stop = *abort_flag ? 1 : nxt.valid > 0 ? 0 : 2;
+      if (tries <= 0) stop_flag[stop] = 1;
       if (chain) {
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars[R_CH]);
@@ -887,13 +884,14 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       prev_first = cur.row0 * p.Hv + cur.hv;
       prev_rows = cur.valid;
       cur = nxt;
-      const int how = *stop;  // written before the barrier by one thread: uniform in the group
-      if (how) {
-        if (how == 2) combine(prev_first, prev_rows);  // (1: some wait was given up)
+      if (stop_flag[stop]) break;
+      if (nxt.valid == 0) {
+        combine(prev_first, prev_rows);
         break;
       }
     }
   }
+  if (tries <= 0) *abort_flag = 1;
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);

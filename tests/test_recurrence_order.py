@@ -1,4 +1,4 @@
-"""Barrier phases of the two recurrences, from their source (see wait_model.py).
+"""Barrier phases of the two recurrences and of the chunk-parallel backward, from their source (see wait_model.py).
 
 A wait on an mbarrier names a phase by its parity.  It is a wait for that phase only if the phase before is over
 when it begins and the phase behind it cannot be over before it has been passed, whatever the parts take: by program

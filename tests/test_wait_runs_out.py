@@ -1,6 +1,6 @@
 """What a block does when one of its bounded waits runs out, from the kernels' source (see wait_model.py): each
-wait of the first and the last warp of every role in turn, the waits that are then left open running out from either
-end.  Nothing is run on a device."""
+wait of the first and the last warp of every role in turn; of the waits that are then left open, the ones of the first
+or of the last warps run out first.  Nothing is run on a device."""
 
 import os
 import re
@@ -10,7 +10,8 @@ import wait_model
 
 FORMS = [("forward", dict(n_it=2)), ("forward", dict(n_it=2, lead=1, extra=True, partial=True)),
          ("forward", dict(n_it=2, no_o=True, extra=True)), ("forward", dict(n_it=2, no_o=True)),
-         ("reverse", dict(n_it=2, partial=True))]
+         ("reverse", dict(n_it=2, partial=True)), ("items", dict(n_items=2, partial=(1,))),
+         ("items", dict(n_items=2, clc=True))]
 
 
 @pytest.fixture(scope="module", params=FORMS, ids=lambda f: "-".join([f[0], *f[1]]))
@@ -18,13 +19,17 @@ def plays(request):
     """(warps left at a named barrier, what a warp signalled or issued behind its own wait) of every play"""
     name, form = request.param
     kernel = getattr(wait_model, name)(**form)
-    warps = [w for w in range(kernel.warps) if w < 4 or w % 4 in (0, 3)]
-    return [wait_model.given_up(kernel, w, nth, last_first) for w in warps
-            for nth in range(wait_model.waits_of(kernel, w)) for last_first in (False, True)]
+    warps = (0, 7, 8, 15, 16) if name == "items" else [w for w in range(kernel.warps) if w < 4 or w % 4 in (0, 3)]
+    return [wait_model.given_up(kernel, w, nth, bool(nth & 1)) for w in warps
+            for nth in range(wait_model.waits_of(kernel, w))]
 
 
 def test_every_warp_comes_to_the_end(plays):
     assert [left for left, _ in plays if left] == []
+
+
+def test_no_gradient_of_an_incomplete_item_is_stored(plays):
+    assert {(w, e) for _, late in plays for w, e in late if e[1] in ("dv", "store_rows")} == set()
 
 
 @pytest.mark.parametrize("file", ["fwd_tc.cu", "bwd_dh_tc.cu", "prep_kernels.cu"])

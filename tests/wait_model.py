@@ -7,6 +7,7 @@ that an event depends on and that cannot be evaluated is an error).  ``nominal``
 ``skipped_or_early`` says which waits a parity alone does not keep to their phase, ``given_up`` plays them with
 one wait that runs out."""
 
+import copy
 import functools
 import itertools
 import os
@@ -15,7 +16,7 @@ from types import SimpleNamespace
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "flashqla_b200", "csrc")
 EVENT = re.compile(r"\b(mbar_wait(?:_uniform)?|mbar_arrive(?:_expect_tx)?|umma_\w+|tma_(?:load|store)_2d|clc_try_cancel|"
-                   r"bar_all)\b|bar\.(?:sync|arrive)")
+                   r"bar_all|store_rows)\b|bar\.(?:sync|arrive)|uint4\*>\(p\.dv")
 BARRIER = re.compile(r"&bars\[(.*?)\]|^(\w+)$")
 
 
@@ -110,6 +111,7 @@ class Kernel:
     def __init__(self, file, threads, config, text=None):
         src = text if text is not None else open(os.path.join(CSRC, file)).read()
         src = re.sub(r"//[^\n]*|^[ \t]*#[^\n]*", "", src, flags=re.M)
+        src = re.sub(r"\b(pass|is|in|not)\b", r"\1_", src)  # names that Python has taken
         src = re.sub(r"(if \([^()]*\) )?(\{ const int it = [^;]*; )?FQLA_TRACE\([^;]*;( \})?", "", src)
         self.names = {}
         for body in re.findall(r"\benum \{(.*?)\}", src, flags=re.S):
@@ -119,6 +121,7 @@ class Kernel:
                 value = (self.names[same] if same in self.names else int(same)) if same else value + 1
                 self.names[name] = value
         self.config, self.warps = dict(config), threads // 32
+        self.shared = dict
         self.counts, self.eventful, self.bodies = {}, {}, {}
         env = {**self.names, **self.config}
         for head, bar, count in re.findall(r"(for \([^)]*\) )?mbar_init\(&bars\[(\w+)\], ([^;]+)\);", src):
@@ -129,7 +132,10 @@ class Kernel:
             elif bar in self.names:
                 self.counts[self.names[bar]] = _eval(count, env)
         at = src.index("int tries = WAIT_TRIES;")
-        self.nodes = _parse(src[at:src.index("tc_fence_before();\n  __syncthreads();\n  if (warp == 0) tmem_dealloc", at)])
+        self.nodes = _parse(src[at:src.index("\n  tc_fence_before();\n  __syncthreads();", at)])
+        # functions that are a named barrier
+        self.functions = {name: ([], [("do", barrier)], True) for name, barrier in re.findall(
+            r"void (\w+)\(\) \{\s*(asm volatile\(\"bar\.sync \d+, \d+;\"[^;]*);", src)}
 
     # ---- one warp ---------------------------------------------------------------------------------------
     def warp(self, index, shared):
@@ -137,29 +143,25 @@ class Kernel:
         env = {**self.names, **self.config, **shared, "warp": index, "lane": 0, "tid": 32 * index, "tries": 1,
                "WAIT_TRIES": 1, "elect_one": lambda: True, "__all_sync": lambda mask, x: x, "min": min, "max": max,
                "abs": abs, "__shfl_sync": lambda mask, x, lane: x, "INT_MAX": 2**31 - 1}
-        lambdas = {}
+        lambdas = dict(self.functions)
         yield from self._run(self.nodes, env, lambdas, False)
 
-    def _has_event(self, node, lambdas):
-        if node is None:
+    def _has_event(self, node, lambdas, leaves=True):
+        """whether an event, or (`leaves`) a way out of a loop or lambda, stands in the node"""
+        if node is None or node[0] == "label":
             return False
-        if id(node) not in self.eventful:  # (a lambda is known before the code that calls it)
-            self.eventful[id(node)] = self._find_event(node, lambdas)
-        return self.eventful[id(node)]
-
-    def _find_event(self, node, lambdas):
-        if node[0] == "block":
-            return any(self._has_event(n, lambdas) for n in node[1])
-        if node[0] == "label":
-            return False
-        text = node[1]
-        if EVENT.search(text) and "= [&]" not in text:
-            return True
-        if node[0] == "do" and re.fullmatch(r"break|return|continue", text):
-            return True
-        if any(n in lambdas and lambdas[n][2] for n in re.findall(r"\b(\w+)\(", text)):
-            return True
-        return any(self._has_event(n, lambdas) for n in node[2:])
+        key = id(node), leaves and node[0] != "for"  # (what leaves a loop without events is nothing)
+        if key not in self.eventful:  # (a lambda is known before the code that calls it)
+            text = node[1]
+            if node[0] == "block":
+                found = any(self._has_event(n, lambdas, leaves) for n in text)
+            else:
+                found = bool(EVENT.search(text) and "= [&]" not in text
+                             or key[1] and node[0] == "do" and re.match(r"(break|return|continue)\b", text)
+                             or any(n in lambdas and lambdas[n][2] for n in re.findall(r"\b(\w+)\(", text))
+                             or any(self._has_event(n, lambdas, key[1]) for n in node[2:]))
+            self.eventful[key] = found
+        return self.eventful[key]
 
     def _value(self, expr, env, lambdas):
         """(a generator: an expression may hold a vote or call a lambda)"""
@@ -257,7 +259,8 @@ class Kernel:
             return
         value = _python(m[4] if not m[3] else f"{m[2]} {m[3]} ({m[4]})")
         if re.fullmatch(r"\w+", m[2]):
-            env[m[2]] = eval(value, {}, env)
+            value = eval(value, {}, env)
+            env[m[2]] = copy.copy(value) if isinstance(value, SimpleNamespace) else value
         else:
             exec(f"{m[2]} = {value}", {}, env)
 
@@ -272,7 +275,7 @@ class Kernel:
                 self.bodies[text] = _parse(text[m.end() + 1:_close(text, m.end()) - 1])
             body = self.bodies[text]
             lambdas[m[1]] = (params, body, False)
-            lambdas[m[1]] = (params, body, any(self._has_event(n, lambdas) for n in body))
+            lambdas[m[1]] = (params, body, any(self._has_event(n, lambdas, False) for n in body))
             return None
         if m := re.match(r'asm volatile\("bar\.(sync|arrive) (\d+), (\d+);"', text):
             yield ("bar" if m[1] == "sync" else "bar_arrive"), int(m[2]), int(m[3]), True
@@ -291,7 +294,8 @@ class Kernel:
                 yield "arrive", bar, 1 if one or name != "mbar_arrive" else 32
                 return None
             if EVENT.match(name):
-                yield "issue", name, None
+                if name != "store_rows" or _eval(args[3], env) > 0:  # (rows to store)
+                    yield "issue", name, None
                 return None
             if name in lambdas and name not in env:
                 if lambdas[name][2]:
@@ -300,14 +304,18 @@ class Kernel:
         if m := re.match(r"uint64_t\* (\w+) = &bars\[(.*)\]$", text, flags=re.S):
             env[m[1]] = _eval(m[2], env)
             return None
+        if text.startswith("*reinterpret_cast<uint4*>(p.dv"):
+            yield "issue", "dv", None
+            return None
         m = re.match(r"(?:const |constexpr )?(?:int|bool|uint32_t|long long|Item) (.*)$", text, flags=re.S)
         for part in _split(m[1] if m else text):
+            if any(n in lambdas and lambdas[n][2] for n in re.findall(r"\b(\w+)\(", part)):
+                name, _, expr = part.partition(" = ")
+                env[name.strip()] = yield from self._value(expr.strip(), env, lambdas)
+                continue
+            assert not EVENT.search(part), part
             try:
-                if m and "=" in part and any(n in lambdas for n in re.findall(r"\b(\w+)\(", part)):
-                    name, _, expr = part.partition("=")
-                    env[name.strip()] = yield from self._value(expr.strip(), env, lambdas)
-                else:
-                    self._assign(part, env)
+                self._assign(part, env)
             except Exception:  # not an integer that can be followed
                 pass
         return None
@@ -317,9 +325,9 @@ class Kernel:
 class _Block:
     """The barriers of a block while its warps are played."""
 
-    def __init__(self, kernel, shared=dict):
+    def __init__(self, kernel):
         self.kernel, self.done, self.pending, self.arrived = kernel, {}, dict(kernel.counts), {}
-        shared = shared()
+        shared = kernel.shared()
         self.warps = [kernel.warp(w, shared) for w in range(kernel.warps)]
         self.at = [next(g, None) for g in self.warps]  # the event each warp stands at
 
@@ -344,9 +352,9 @@ class _Block:
             self.at[w] = None
 
 
-def nominal(kernel, shared=dict):
+def nominal(kernel):
     """[(warp, event, phase)] in an order in which the warps take turns; raises if they stop."""
-    block, log, named = _Block(kernel, shared), [], {}
+    block, log, named = _Block(kernel), [], {}
     while any(e is not None for e in block.at):
         moved = False
         for w, e in enumerate(block.at):
@@ -408,11 +416,11 @@ def order(log):
     return (lambda a, b: bool(before[b] >> a & 1)), nodes, waits, arrivals
 
 
-def skipped_or_early(kernel, shared=dict):
+def skipped_or_early(kernel):
     """Waits that a parity alone does not keep to their phase: the phase before may still be open when the wait
     begins (it would be over at once), or the phase behind may be over before the wait has been (its parity would
     not come round).  Barriers whose phases the loads complete count by the arrival that goes with the loads."""
-    log = nominal(kernel, shared)
+    log = nominal(kernel)
     follows, previous, waits, arrivals = order(log)
     name = {v: k for k, v in reversed(list(kernel.names.items()))}
     wrong = set()
@@ -427,11 +435,11 @@ def skipped_or_early(kernel, shared=dict):
     return sorted(wrong)
 
 
-def given_up(kernel, warp, nth, last_first, shared=dict):
+def given_up(kernel, warp, nth, last_first):
     """Plays the block with the `nth` wait of `warp` running out; whenever nobody can go on, the waits that are
     open run out one at a time (from the highest or the lowest warp).  Returns (warps left at a named barrier,
     [(warp, event)] that was signalled or issued by a warp behind a wait of its own that had run out)."""
-    block, named, late = _Block(kernel, shared), {}, []
+    block, named, late = _Block(kernel), {}, []
     out, count = set(), [0] * kernel.warps
     while True:
         moved = False
@@ -476,8 +484,8 @@ def given_up(kernel, warp, nth, last_first, shared=dict):
     return [(w, e) for w, e in enumerate(block.at) if e is not None], late
 
 
-def waits_of(kernel, warp, shared=dict):
-    return sum(1 for w, e, _ in nominal(kernel, shared) if w == warp and e[0] == "wait")
+def waits_of(kernel, warp):
+    return sum(1 for w, e, _ in nominal(kernel) if w == warp and e[0] == "wait")
 
 
 def forward(no_o=False, extra=False, lead=0, n_it=7, partial=False, tiled=1, text=None):
@@ -500,9 +508,27 @@ def reverse(lead=0, n_it=7, partial=False, tiled=1, text=None):
     return Kernel("bwd_dh_tc.cu", 512, config, text=text)
 
 
+def items(clc=False, tiled=True, partial=(), n_items=4, text=None):
+    """The chunk-parallel backward: one block that takes n_items items."""
+    config = dict(TILED=tiled, CLC=clc, N_EPI=512, D=128, CHUNK=64, p=SimpleNamespace(Hv=1000, next_item=0, dg_cumsum=0),
+                  total=n_items, raw=None, answers=0, blockIdx=SimpleNamespace(x=0), gridDim=SimpleNamespace(x=1))
+
+    def shared():
+        claims = itertools.count()
+        return dict(
+            ring=[None] * 4, stop_flag=[0] * 4, atomicAdd=lambda word, n: next(claims),
+            finish=lambda raw, w: SimpleNamespace(valid=40 if w in partial else 64, row0=0, hv=0, hq=0, chunk_id=0),
+            clc_block=lambda slot: next((w for w in [1 + next(claims)] if w < n_items), -1))
+
+    kernel = Kernel("bwd_main_tc.cu", 544, config, text=text)
+    kernel.shared = shared
+    return kernel
+
+
 CASES = [*itertools.chain(
     (("forward", dict(lead=lead, extra=extra, partial=partial)) for lead, extra, partial in
      itertools.product((0, 1, 2, 3), (False, True), (False, True))),
     (("forward", dict(no_o=True, extra=extra, partial=partial)) for extra, partial in
      itertools.product((False, True), (False, True))),
-    (("reverse", dict(lead=lead, partial=partial)) for lead, partial in itertools.product((0, 1, 2, 3), (False, True))))]
+    (("reverse", dict(lead=lead, partial=partial)) for lead, partial in itertools.product((0, 1, 2, 3), (False, True))),
+    (("items", dict(clc=clc, partial=partial)) for clc, partial in itertools.product((False, True), ((), (0, 2), (1, 3)))))]
