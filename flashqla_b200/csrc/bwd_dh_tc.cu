@@ -88,7 +88,9 @@ constexpr uint32_t TM_S = 0, TM_X1 = 128, TM_X2 = 192, TM_P = 256, TM_W = 384;
 enum { FULL0 = 0, FULL1, EMPTY0, EMPTY1, S_COPY, S_DEC, X1_DONE, X2_DONE, S_DONE, P_DONE, W_DONE,
        DV_READY, W_READY, P_READY, AP_READY, QS_READY, PRIV,
        // the A tile and the per-row vectors of a chunk travel one chunk ahead of q, k, dO
-       FULLA0, FULLA1, EMPTYA0, EMPTYA1, PRIVA };
+       FULLA0, FULLA1, EMPTYA0, EMPTYA1, PRIVA,
+       // all products have come to their end
+       SETTLED };
 enum { V_G = 0, V_BG = 1, V_RHO = 2, V_SGAM = 3, V_GL = 4 };
 }  // namespace bdtc
 
@@ -149,6 +151,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     mbar_init(&bars[EMPTYA0], 1);  // the scaling warp, the only reader of the raw A tile
     mbar_init(&bars[EMPTYA1], 1);
     mbar_init(&bars[PRIVA], 1);
+    mbar_init(&bars[SETTLED], 2);
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&map_q);
@@ -184,15 +187,19 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
-  // see mbar_wait; `more`: no lane of the warp has given a wait up, on to the next pass of its role's loop
-  int tries = WAIT_TRIES;
+  int tries = WAIT_TRIES;  // see mbar_wait; filled up for each pass of a role's loop
   auto WAIT = [&](int idx, uint32_t parity) { mbar_wait(&bars[idx], parity, tries); };
   // (of the issuing warps: see mbar_wait_uniform; 262144 tokens x 8 heads 584 us, 590 with the plain ones)
-  auto WAITU = [&](int idx, uint32_t parity) { mbar_wait_uniform(&bars[idx], parity, tries); };
-  auto more = [&] {
-    const bool ok = __all_sync(0xffffffffu, tries > 0);
-    if (ok) tries = WAIT_TRIES;
-    return ok;
+  auto WAITU = [&](int idx, uint32_t parity) { return mbar_wait_uniform(&bars[idx], parity, tries); };
+  auto fill = [&] { tries = tries > 0 ? WAIT_TRIES : tries; };
+  // A thread that has given a wait up issues, signals and stores nothing more: see fwd_tc.cu.
+  auto ARRIVE = [&](int idx) { mbar_arrive_if(&bars[idx], tries); };
+  auto issuing = [&] { return elect_one() && tries > 0; };  // of the producer
+  // At the end of a role that issues: a wait with a limit of its own.
+  auto settle = [&](int idx, uint32_t parity) {
+    int again = WAIT_TRIES;
+    mbar_wait(&bars[idx], parity, again);
+    if (again <= 0) tries = 0;
   };
 
   // End gradient -> tensor memory, dS^T[v][k]; zero without one and for a lead-out.  The three
@@ -247,7 +254,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
   case 1: {
     // =============================== state group ===============================
     const int v = tid - 128;
-    for (int it = 0; it < n_it && more(); ++it) {
+    for (int it = 0; it < n_it; ++it, fill()) {
       const int s = it & 1, c = n_it - 1 - it;
       if (it > 0) WAIT(S_DONE, (it - 1) & 1);
       tc_fence_after();
@@ -272,10 +279,10 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       }
       fence_proxy_async();
       tc_fence_before();
-      mbar_arrive(&bars[S_COPY]);
+      ARRIVE(S_COPY);
       if (hdst && !p.tiled) {  // row-major [k][v]: column v, from this thread's own row of the copy
 #pragma unroll 1
-        for (int k = 0; k < D; ++k)
+        for (int k = 0; k < (tries > 0 ? D : 0); ++k)
           hdst[(long long)k * D + v] =
               *reinterpret_cast<const bf16*>(smem + OFF_ST + (k >> 6) * 16384 + sw128_offset(v, k & 63));
       }
@@ -298,11 +305,11 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&bars[S_DEC]);
+      ARRIVE(S_DEC);
     }
     if (n_it > 0) WAIT(S_DONE, (n_it - 1) & 1);
     const int dh0_row = p.dh0_row ? p.dh0_row[n] : n;
-    if (more() && p.dh0 && dh0_row >= 0) {
+    if (__all_sync(0xffffffffu, tries > 0) && p.dh0 && dh0_row >= 0) {
       float* dst = p.dh0 + ((long long)dh0_row * p.Hv + hv) * D * D;
       tc_fence_after();
 #pragma unroll 1
@@ -348,10 +355,10 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       }
       fence_proxy_async();
       tc_fence_before();
-      mbar_arrive(&bars[W_READY]);
+      ARRIVE(W_READY);
     };
 #pragma unroll 1
-    for (int it = -1; it < n_it && more(); ++it) {  // it = -1: only w of the first iteration
+    for (int it = -1; it < n_it; ++it, fill()) {  // it = -1: only w of the first iteration
      if (it >= 0) {
       const int c = n_it - 1 - it;
       const long long row0 = sp.bos + (long long)c * CHUNK;
@@ -385,11 +392,11 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       // operand complete, accumulators read: hand over before the global stores
       fence_proxy_async();
       tc_fence_before();
-      mbar_arrive(&bars[DV_READY]);
+      ARRIVE(DV_READY);
       if (p.du && !p.tiled && it >= lead) {  // row-major: column v, from this thread's own row
         bf16* dst = p.du + (row0 * p.Hv + hv) * D + v;
 #pragma unroll 1
-        for (int j = 0; j < valid; ++j)
+        for (int j = 0; j < (tries > 0 ? valid : 0); ++j)
           dst[(long long)j * p.Hv * D] = *reinterpret_cast<const bf16*>(smem + OFF_DVT + sw128_offset(v, j));
       }
      }
@@ -405,7 +412,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
     const int row_a = 16 * wq + (lane >> 2), row_b = row_a + 8, cp = 2 * (lane & 3);
     const uint32_t lanes_p = (uint32_t)(wq * 32) << 16;
     const float log2_scale = log2f(p.scale);
-    for (int it = 0; it < n_it && more(); ++it) {
+    for (int it = 0; it < n_it; ++it, fill()) {
       const float* vs = vec + (it & 3) * VEC_SLOT_FLOATS;
       WAIT(FULL0 + (it & 1), (it >> 1) & 1);
       WAIT(P_DONE, it & 1);
@@ -433,7 +440,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       }
       fence_proxy_async();
       tc_fence_before();
-      mbar_arrive(&bars[P_READY]);
+      ARRIVE(P_READY);
       // (not before the update of the chunk before has been issued: its thread waits for that chunk's q)
       if (it > 0) WAIT(S_DONE, (it - 1) & 1);
       const float sg = vs[V_SGAM * CHUNK + qr];
@@ -445,7 +452,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         *x8 = make_uint4(scale2(a.x, sg, sg), scale2(a.y, sg, sg), scale2(a.z, sg, sg), scale2(a.w, sg, sg));
       }
       fence_proxy_async();
-      mbar_arrive(&bars[QS_READY]);
+      ARRIVE(QS_READY);
     }
   } break;
   default: if (warp == 0 || warp == 3) {
@@ -465,12 +472,11 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       const uint32_t st_lo = desc_lo_kmajor(smem + OFF_ST), dvt_lo = desc_lo_kmajor(smem + OFF_DVT);
       const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 8192), qmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE, 8192);
 #pragma unroll 1
-      for (int it = 0; it < n_it && more(); ++it) {
+      for (int it = 0; it < n_it; ++it, fill()) {
         const int s = it & 1;
         const uint32_t so = s ? STAGE_LO : 0u;
         const int y_tile = (int)(((sp.chunk_base + (n_it - 1 - it)) * p.Hv + hv) * D);
-        WAITU(FULL0 + s, (it >> 1) & 1);
-        WAITU(S_COPY, it & 1);
+        if (!(WAITU(FULL0 + s, (it >> 1) & 1) && WAITU(S_COPY, it & 1))) break;
         tc_fence_after();
         if (elect_one()) {
           // X1^T = dS^T K^T   (on the chain)
@@ -484,13 +490,11 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
           }
         }
         // dS^T <- dS^T + dO^T (scale gamma q) - dv^T w; the first product while dv is on its way
-        WAITU(QS_READY, it & 1);
-        WAITU(S_DEC, it & 1);
+        if (!(WAITU(QS_READY, it & 1) && WAITU(S_DEC, it & 1))) break;
         tc_fence_after();
         if (elect_one())
           umma_group<4, 128, 0, 128, 0, true>(tmem + TM_S, domn0_lo + so, qmn0_lo + so, ID_UPD_Q);
-        WAITU(W_READY, it & 1);
-        WAITU(DV_READY, it & 1);
+        if (!(WAITU(W_READY, it & 1) && WAITU(DV_READY, it & 1))) break;
         tc_fence_after();
         if (elect_one()) {
           umma_group<4, 2, 0, 128, 0, true>(tmem + TM_S, dvt_lo, wmn_lo, ID_UPD_W);
@@ -508,27 +512,25 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE, 8192);
       const uint32_t app_lo = desc_lo_kmajor(smem + OFF_APP), pmn_lo = desc_lo_mnmajor(smem + OFF_P, 8192);
 #pragma unroll 1
-      for (int it = 0; it < n_it && more(); ++it) {
+      for (int it = 0; it < n_it; ++it, fill()) {
         const int s = it & 1;
         const uint32_t so = s ? STAGE_LO : 0u;
         // (the Pg group has read P of the chunk before: P_READY was waited for)
-        WAITU(FULL0 + s, (it >> 1) & 1);
+        if (!WAITU(FULL0 + s, (it >> 1) & 1)) break;
         tc_fence_after();
         if (elect_one()) {
           umma_group<8, 2, 512, 2, 512, false>(tmem + TM_P, q0_lo + so, k0_lo + so, ID_P);
           umma_commit(&bars[P_DONE]);
         }
         // w, whose accumulator the dv / w group has read for the chunk before
-        WAITU(AP_READY, it & 1);
-        if (it > 0) WAITU(W_READY, (it - 1) & 1);
+        if (!(WAITU(AP_READY, it & 1) && (it == 0 || WAITU(W_READY, (it - 1) & 1)))) break;
         tc_fence_after();
         if (elect_one()) {
           umma_group<4, 2, 0, 128, 0, false>(tmem + TM_W, app_lo, kmn0_lo + so, ID_W);
           umma_commit(&bars[W_DONE]);
         }
         // X2^T = dO^T Pg, likewise
-        WAITU(P_READY, it & 1);
-        if (it > 0) WAITU(DV_READY, (it - 1) & 1);
+        if (!(WAITU(P_READY, it & 1) && (it == 0 || WAITU(DV_READY, (it - 1) & 1)))) break;
         tc_fence_after();
         if (elect_one()) {
           umma_group<4, 128, 0, 128, 0, false>(tmem + TM_X2, domn0_lo + so, pmn_lo, ID_X2);
@@ -537,6 +539,9 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         }
       }
     }
+    // no product is under way when the block goes, whoever gave up what
+    if (elect_one()) umma_commit(&bars[SETTLED]);
+    if (warp == 0) settle(SETTLED, 0);
   } else if (warp == 1) {
     // =============================== producer ===============================
     float g_r[2] = {0.f, 0.f}, b_r[2] = {0.f, 0.f}, gl_r = 0.f;
@@ -559,12 +564,13 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         if (((i >> 3) & 63) >= valid) *reinterpret_cast<uint4*>(base + i * 16) = make_uint4(0, 0, 0, 0);
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) mbar_arrive(full);
+      if (lane == 0 && tries > 0) mbar_arrive(full);
     };
     // As in fwd_tc.cu: q, k, dO of iteration it; vectors and A tile of iteration it + 1; the gates of
     // iteration it + 2 into registers.  Slot (it + 1) % 4 of the vectors was last read for iteration
     // it - 3, which the wait on the stage of iteration it - 2 has seen finished.
     // (A whole first chunk's q, k, dO go out at once, ahead of its gates, as in fwd_tc.cu.)
+    int loads = 0, a_loads = 0;  // q, k, dO and A tiles that have been asked for
     const bool early = n_it > 0 && len_ext >= n_it * CHUNK;
     auto load = [&](int it) {
       const int s = it & 1, c = n_it - 1 - it;
@@ -576,7 +582,7 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       }
       unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
       uint64_t* bar = &bars[partial ? PRIV : FULL0 + s];
-      if (elect_one()) {
+      if (issuing()) {
         mbar_expect_tx(bar, STAGE_BYTES - TILE_A);
         if (it > 0 || !early) mbar_arrive(bar);
         tma_load_2d(st + TILE, &map_k, hq * D, y, bar);
@@ -586,15 +592,16 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         tma_load_2d(st + 2 * TILE, &map_do, hv * D, y, bar);
         tma_load_2d(st + 2 * TILE + 8192, &map_do, hv * D + 64, y, bar);
       }
+      loads = tries > 0 ? it + 1 : loads;
       if (partial) {
         WAIT(PRIV, 0);
         zero_rows(st, 6, valid, &bars[FULL0 + s]);
       }
     };
 #pragma unroll 1
-    for (int it = -2; it < n_it && more(); ++it) {
+    for (int it = -2; it < n_it; ++it, fill()) {
       if (it > 0 || it == (early ? -2 : 0)) load(max(it, 0));
-      else if (it == 0 && lane == 0) mbar_arrive(&bars[FULL0]);
+      else if (it == 0 && lane == 0) ARRIVE(FULL0);
       const int j = it + 1;
       if (j >= 0 && j < n_it) {
         const int sj = j & 1, c = n_it - 1 - j;
@@ -618,10 +625,11 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
         __syncwarp();
         unsigned char* dst = smem + OFF_STAGE + sj * STAGE_BYTES + 3 * TILE;
         uint64_t* bar = &bars[partial ? PRIVA : FULLA0 + sj];
-        if (elect_one()) {
+        if (issuing()) {
           mbar_arrive_expect_tx(bar, TILE_A);
           tma_load_2d(dst, &map_a, hv * CHUNK, (int)(sp.bos + (long long)c * CHUNK), bar);
         }
+        a_loads = tries > 0 ? j + 1 : a_loads;
         if (partial) {
           // only the last chunk of a sequence (the first one walked) can be partial: used once
           WAIT(PRIVA, 0);
@@ -630,13 +638,19 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       }
       if (it + 2 < n_it) fetch(it + 2);
     }
+    // nor a load
+#pragma unroll 1
+    for (int i = 1; i <= 2; ++i) {
+      if (loads >= i) settle(FULL0 + ((loads - i) & 1), ((loads - i) >> 1) & 1);
+      if (a_loads >= i) settle(FULLA0 + ((a_loads - i) & 1), ((a_loads - i) >> 1) & 1);
+    }
   } else {
     // =============================== scaling warp (2) ===============================
     // A'' = A diag(beta gamma) (columns): thread t owns the 8 columns 8 (t%8) .. of the rows
     // t/8 + 4 i, its scale factors stay in registers and the eight threads of a row touch one
     // 128-byte line per access.
     const int c8 = lane & 7, r0 = lane >> 3;
-    for (int it = 0; it < n_it && more(); ++it) {
+    for (int it = 0; it < n_it; ++it, fill()) {
       const int s = it & 1;
       WAIT(FULLA0 + s, (it >> 1) & 1);
       if (it > 0) WAIT(W_DONE, (it - 1) & 1);  // w of the chunk before has been issued and is done
@@ -655,8 +669,8 @@ bwd_dh_tc_kernel(const BwdDhTcParams p, const __grid_constant__ CUtensorMap map_
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(&bars[AP_READY]);
-        mbar_arrive(&bars[EMPTYA0 + s]);  // the A tile of this stage is no longer read
+        ARRIVE(AP_READY);
+        ARRIVE(EMPTYA0 + s);  // the A tile of this stage is no longer read
       }
     }
   }

@@ -80,7 +80,7 @@ constexpr int OFF_DW = OFF_X + 8192;        // dW = A^T du
 // the chunk total (8) and what suffix_sum64 needs (2)
 constexpr int OFF_VEC = OFF_DW + ROW_TILE;
 constexpr int OFF_BAR = OFF_VEC + (2 * 256 + 128 + 3 * 256 + 18) * 4;
-constexpr int N_BARS = 20;
+constexpr int N_BARS = 22;
 constexpr int OFF_MISC = OFF_BAR + N_BARS * 8;
 constexpr int OFF_ITEM = OFF_MISC + 32;  // ring of four items, published by the issue warp
 constexpr int OFF_CLAIM = (OFF_ITEM + 4 * 32 + 15) / 16 * 16;  // CLC: two answers of 16 bytes
@@ -105,7 +105,8 @@ enum {
   R_CH,                                  // ... -> bulk group: item finished
   R_HD, R_E4, R_END,                     // the 8 warps of the bulk group -> issue warp
   I_NEXT,                                // issue warp -> read-out warps: the next item is in the ring
-  I_CLAIM                                // CLC: the answer with the next item has arrived
+  I_CLAIM,                               // CLC: the answer with the next item has arrived
+  SETTLED                                // all products have come to their end
 };
 }  // namespace bmtc
 
@@ -207,6 +208,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
     for (int i = R_DW; i <= R_END; ++i) mbar_init(&bars[i], N_EPI / 64);
     mbar_init(&bars[I_NEXT], 1);
     if (CLC) mbar_init(&bars[I_CLAIM], 1);
+    mbar_init(&bars[SETTLED], 1);
     *abort_flag = 0;
     for (int i = 0; i < 4; ++i) stop_flag[i] = 0;
     fence_mbar_init();
@@ -217,14 +219,14 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  int tries = WAIT_TRIES;  // see mbar_wait; filled up for each item
+  int tries = WAIT_TRIES;  // see mbar_wait; filled up for each item; used up, a thread signals and stores no more
   auto WAIT = [&](int idx, uint32_t parity) { mbar_wait(&bars[idx], parity, tries); };
 
   if (warp == N_EPI / 32) {
     // ====================== issue warp: TMA loads and every tcgen05.mma ======================
     // (the warp stays converged; see elect_one in tc05.cuh)
     {
-      auto WAIT = [&](int idx, uint32_t parity) { mbar_wait_uniform(&bars[idx], parity, tries); };
+      auto WAIT = [&](int idx, uint32_t parity) { return mbar_wait_uniform(&bars[idx], parity, tries); };
       // Four groups, in the order in which their buffers become free (A and du are dead after the first
       // product of an item, q only after the bulk group has read it).
       auto load_d = [&](const Item& t) {
@@ -298,7 +300,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       // read: what the chain group reads (dW, ds, qk, KK, D3) behind its own arrivals on the tiles it makes
       // of them, what the bulk group reads (dq, dk, Y) behind R_END of the item before.
 #pragma unroll 1
-      for (bool has_next = true; has_next && tries > 0; ++it) {
+      for (bool has_next = true; has_next; ++it) {
         tries = WAIT_TRIES;
         const uint32_t ph = it & 1;
         if (!CLC && lane == 0) claimed = (int)gridDim.x + atomicAdd(p.next_item, 1);
@@ -308,14 +310,13 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         const bool partial = cur.valid != CHUNK;
         if (partial) {
           if (it > 0) {  // q of this item, below for a full chunk
-            WAIT(C_2, ph ^ 1);
-            WAIT(R_E4, ph ^ 1);
+            if (!(WAIT(C_2, ph ^ 1) && WAIT(R_E4, ph ^ 1))) break;
             load_q(cur);
           }
-          WAIT(R_ZERO, zero_ph);
+          if (!WAIT(R_ZERO, zero_ph)) break;
           zero_ph ^= 1;
         } else {
-          WAIT(L_D, ph);
+          if (!WAIT(L_D, ph)) break;
         }
         tc_fence_after();
         // ---- dW = A^T du: needs nothing but A and du ----
@@ -331,12 +332,10 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         if (!partial) {
           if (it > 0) {
             // q of the item before is dead: its product is complete, the bulk group has used it
-            WAIT(C_2, ph ^ 1);
-            WAIT(R_E4, ph ^ 1);
+            if (!(WAIT(C_2, ph ^ 1) && WAIT(R_E4, ph ^ 1))) break;
             load_q(cur);
           }
-          WAIT(L_A, ph);
-          WAIT(L_Q, ph);
+          if (!(WAIT(L_A, ph) && WAIT(L_Q, ph))) break;
           tc_fence_after();
         }
         // ---- ds, q k^T, K K^T ----
@@ -348,7 +347,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           umma_group<8, 2, 512, 2, 512, false>(tmem + T_KK, k_lo, k_lo, ID_KK_64);
         }
         // ---- dW is an operand now: D3 = dW v_new^T ----
-        WAIT(R_DW, ph);
+        if (!WAIT(R_DW, ph)) break;
         tc_fence_after();
         if (elect_one()) {
           if constexpr (TILED) umma_group<8, 2, 512, 128, 512, false>(tmem + T_D3, dw_lo, vnT_lo, ID_KM_64);
@@ -357,8 +356,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         }
         int w_next;
         if constexpr (CLC) {
-          WAIT(I_CLAIM, ph);
-          if (tries <= 0) break;  // (no item to look up)
+          if (!WAIT(I_CLAIM, ph)) break;
           w_next = clc_block(answers + 16 * ph);
           fence_proxy_async();  // read before the request after the next one writes the slot
           has_next = w_next >= 0;
@@ -369,8 +367,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         const int h_next = has_next ? w_next % p.Hv : 0;
         if (has_next) load_index(w_next / p.Hv, raw);
         // ---- Y = dW h^T, dq1, dk1: off the chain ----
-        WAIT(L_H, ph);
-        if (it > 0) WAIT(R_END, ph ^ 1);
+        if (!(WAIT(L_H, ph) && (it == 0 || WAIT(R_END, ph ^ 1)))) break;
         tc_fence_after();
         if (elect_one()) {
           if constexpr (TILED) {
@@ -386,7 +383,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         }
         if (has_next) load_span(raw);
         // ---- ds is an operand now ----
-        WAIT(R_DS, ph);
+        if (!WAIT(R_DS, ph)) break;
         tc_fence_after();
         if (elect_one()) {
           umma_group<4, 2, 0, 128, 0, false>(tmem + T_DQ2, ds_lo, kmn_lo, ID_KM_128);
@@ -405,7 +402,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           mbar_arrive(&bars[I_NEXT]);
         }
         // ---- dk += (X + X^T) K with X = beta dL, onto ds^T q ----
-        WAIT(R_D3, ph);
+        if (!WAIT(R_D3, ph)) break;
         tc_fence_after();
         if (elect_one()) {
           umma_group<4, 2, 0, 128, 0, true>(tmem + T_DK2, x_lo, kmn_lo, ID_KM_128);
@@ -414,11 +411,23 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
         // h, dh, dO, v_new are dead once their products are complete and the h.dh sum is done; the other
         // k buffer belonged to the item before, which R_END above has seen finished
         if (has_next) {
-          WAIT(C_1B, ph);
-          WAIT(R_HD, ph);
+          if (!(WAIT(C_1B, ph) && WAIT(R_HD, ph))) break;
           load_a(nxt, (int)(ph ^ 1));
         }
         cur = nxt;
+      }
+      // No product is under way when the block goes, and no load: where this warp came through it has waited for
+      // all of them, else whichever phase of theirs is open is waited for.
+      if (elect_one()) umma_commit(&bars[SETTLED]);
+      int again = WAIT_TRIES;
+      mbar_wait(&bars[SETTLED], 0, again);
+      if (again <= 0) tries = 0;
+      if (tries <= 0) {
+#pragma unroll 1
+        for (int i = 0; i < (CLC ? 10 : 8); ++i) {
+          again = WAIT_TRIES / 64;
+          mbar_wait(&bars[i < 8 ? L_D + (i >> 1) : I_CLAIM], i & 1, again);
+        }
       }
     }
   } else {
@@ -487,7 +496,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       fence_proxy_async();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars[bar]);
+      if (lane == 0 && tries > 0) mbar_arrive(&bars[bar]);
     };
     auto zero_rows = [&](int off, int n_blocks, int valid) {
 #pragma unroll 1
@@ -772,7 +781,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
           acc_last += sGam[CHUNK - 1] * hd;
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[R_HD]);
+        if (lane == 0 && tries > 0) mbar_arrive(&bars[R_HD]);
         if (it > 0) combine(prev_first, prev_rows);  // fits into the wait for the first wide products
         const float f_w = hi ? sRho[row_w] : p.scale * sGam[row_w];
         const int row_q = row_w - (lane & 3);  // row of lane 0 of this quad
@@ -876,7 +885,7 @@ bwd_main_tc_kernel(const BwdMainTcParams p, const __grid_constant__ CUtensorMap 
       if (tries <= 0) stop_flag[stop] = 1;
       if (chain) {
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars[R_CH]);
+        if (lane == 0 && tries > 0) mbar_arrive(&bars[R_CH]);
         chain_barrier();
       } else {
         bulk_barrier();

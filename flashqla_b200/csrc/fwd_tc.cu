@@ -187,6 +187,8 @@ enum { FULL0 = 0, FULL1, EMPTY0, EMPTY1, S_COPY, S_DEC, VN_DONE, S_DONE, P_DONE,
        SB_FREE,
        // P has been read
        P_FREE,
+       // all products have come to their end
+       SETTLED,
        // state-only pass: W^T, made by the V and the O group, is there
        WB_READY = P_READY };
 // vectors inside a slot; V_GL holds gamma_last at [0], V_BG -beta gamma instead of beta gamma in
@@ -263,6 +265,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     mbar_init(&bars[EMPTY1], STATE ? 1 : NO_O ? 2 : 3);
     mbar_init(&bars[SB_FREE], 1);
     mbar_init(&bars[P_FREE], 128);
+    mbar_init(&bars[SETTLED], STATE ? 1 : NO_O ? 2 : 3);
     mbar_init(&bars[U_DONE], 1);
     mbar_init(&bars[FULLA0], 1);
     mbar_init(&bars[FULLA1], 1);
@@ -317,13 +320,21 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;  // this warp's lane quarter
-  // see mbar_wait; `more`: no lane of the warp has given a wait up, on to the next pass of its role's loop
-  int tries = WAIT_TRIES;
+  int tries = WAIT_TRIES;  // see mbar_wait; filled up for each pass of a role's loop
   auto WAIT = [&](int idx, uint32_t parity) { mbar_wait(&bars[idx], parity, tries); };
-  auto more = [&] {
-    const bool ok = __all_sync(0xffffffffu, tries > 0);
-    if (ok) tries = WAIT_TRIES;
-    return ok;
+  auto WAITU = [&](int idx, uint32_t parity) { return mbar_wait_uniform(&bars[idx], parity, tries); };
+  auto fill = [&] { tries = tries > 0 ? WAIT_TRIES : tries; };
+  // A thread that has given a wait up issues, signals and stores nothing more.  An issuing warp leaves its loop as one.
+  // The others walk theirs to the end, as their lanes each count for themselves and what follows are instructions of
+  // whole warps (a vote on the way out, once a chunk, cost 1 %: three prompts of 985 tokens x 64 heads 30.8 us
+  // instead of 30.5), one try a wait.
+  auto ARRIVE = [&](int idx) { mbar_arrive_if(&bars[idx], tries); };
+  auto issuing = [&] { return elect_one() && tries > 0; };  // of the producer
+  // At the end of a role that issues: a wait with a limit of its own.
+  auto settle = [&](int idx, uint32_t parity) {
+    int again = WAIT_TRIES;
+    mbar_wait(&bars[idx], parity, again);
+    if (again <= 0) tries = 0;
   };
 
   // Initial state -> tensor memory, S^T[v][k]; zero without one and for a lead-in.  The three
@@ -386,7 +397,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     // =============================== S group ===============================
     const int v = tid - 128;  // lane of tensor memory = value index
 #pragma unroll 1
-    for (int it = 0; it < n_it && more(); ++it) {
+    for (int it = 0; it < n_it; ++it, fill()) {
       const int s = it & 1;
       if (v == 0) FQLA_TRACE(0, 0);
       if (it > 0) WAIT(S_DONE, (it - 1) & 1);
@@ -410,7 +421,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&bars[S_COPY]);
+      ARRIVE(S_COPY);
       if (v == 0) FQLA_TRACE(0, 2);
       if constexpr (EXTRA) {
         // off the chain: the state entering this chunk as an output, from the operand copy
@@ -428,11 +439,11 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           }
           if (p.tiled) {
             fence_proxy_async();
-            mbar_arrive(&bars[ST_READY]);
+            ARRIVE(ST_READY);
           } else {  // row-major [k][v]: column v, from this thread's own row
             bf16* hdst = p.h + ((sp.chunk_base + (it - lead)) * p.Hv + hv) * (long long)D * D + v;
 #pragma unroll 1
-            for (int k = 0; k < D; ++k)
+            for (int k = 0; k < (tries > 0 ? D : 0); ++k)
               hdst[(long long)k * D] =
                   *reinterpret_cast<const bf16*>(smem + OFF_ST + (k >> 6) * 16384 + sw128_offset(v, k & 63));
           }
@@ -453,13 +464,13 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&bars[S_DEC]);
+      ARRIVE(S_DEC);
       if (v == 0) FQLA_TRACE(0, 4);
     }
     if (n_it > 0) WAIT(S_DONE, (n_it - 1) & 1);
     const int ht_row = p.ht_row && !m_pass ? p.ht_row[n] : n;
     float* end = m_pass ? p.M : p.ht;
-    if (more() && end && ht_row >= 0) {
+    if (__all_sync(0xffffffffu, tries > 0) && end && ht_row >= 0) {
       float* dst = end + ((long long)ht_row * p.Hv + hv) * D * D;
       tc_fence_after();
 #pragma unroll 1
@@ -485,7 +496,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     // operands in tensor memory.
     const int v = (warp & 3) * 32 + lane;  // tensor-memory lane = value index
     const int t0 = warp < 12 ? 0 : 32;
-    for (int it = 0; it < n_it && more(); ++it) {
+    for (int it = 0; it < n_it; ++it, fill()) {
       const int s = it & 1;
       WAIT(FULL0 + s, (it >> 1) & 1);
       const float* vs = vec + (it & 3) * VEC_SLOT_FLOATS + t0;
@@ -513,7 +524,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       tmem_st16(tmem + lane_sel + TM_WB + (t0 >> 1), pk);
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&bars[WB_READY]);
+      ARRIVE(WB_READY);
       // off the chain: rho, and rho times what the rounding of the operand left out
       load32(vs + V_RHO * CHUNK, f);
 #pragma unroll
@@ -531,7 +542,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       tmem_st16(tmem + lane_sel + TM_VRB + (t0 >> 1), pk);
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&bars[VB_READY]);
+      ARRIVE(VB_READY);
     }
   } break;
   case 2: if constexpr (!STATE) {
@@ -555,10 +566,10 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       }
       tc_fence_before();
       fence_proxy_async();
-      mbar_arrive(&bars[W_READY]);
+      ARRIVE(W_READY);
     };
 #pragma unroll 1
-    for (int it = -1; it < n_it && more(); ++it) {  // it = -1: only w^T of the first iteration
+    for (int it = -1; it < n_it; ++it, fill()) {  // it = -1: only w^T of the first iteration
      if (it >= 0) {
       const int c = it - lead;
       if (v == 0) FQLA_TRACE(1, 0);
@@ -592,7 +603,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&bars[VB_READY]);
+      ARRIVE(VB_READY);
       if (v == 0) FQLA_TRACE(1, 2);
       if constexpr (EXTRA) {
         // off the chain: v_new as an output, from the operand copy (the store of the chunk before has
@@ -608,10 +619,10 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
                 make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
           if (p.tiled) {
             fence_proxy_async();
-            mbar_arrive(&bars[VN_READY]);
+            ARRIVE(VN_READY);
           } else {  // row-major [row][v]: column v, from this thread's own row
             const long long row0 = sp.bos + (long long)c * CHUNK;
-            const int valid = min(CHUNK, sp.len - c * CHUNK);
+            const int valid = tries > 0 ? min(CHUNK, sp.len - c * CHUNK) : 0;
             bf16* dst = p.vnew + (row0 * p.Hv + hv) * D + v;
 #pragma unroll 1
             for (int j = 0; j < valid; ++j)
@@ -660,7 +671,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         tmem_ld_wait();
         if (h == 3) {  // all tensor-memory reads of this chunk's output are done
           tc_fence_before();
-          mbar_arrive(&bars[O_FREE]);
+          ARRIVE(O_FREE);
         }
         // this lane supplies the address of row r8 of matrix mtx of every store: matrices 0, 1 are
         // the two 8-row blocks of token block i, matrices 2, 3 those of token block i + 1
@@ -700,7 +711,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       }
     };
 #pragma unroll 1
-    for (int c = max(-lead, 0); c < n_it - lead && more(); ++c) {
+    for (int c = max(-lead, 0); c < n_it - lead; ++c, fill()) {
       if (v == 0) { const int it = c + lead; FQLA_TRACE(2, 0); }
       WAIT(O_DONE, c & 1);
       if (wq == 0 && elect_one()) tma_store_wait_read();  // the store of the chunk before has read the tile
@@ -735,7 +746,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     const uint32_t lanes_p = (uint32_t)(wq * 32) << 16;  // lanes 0-15 of the quarter
     const float log2_scale = log2f(p.scale);
 #pragma unroll 1
-    for (int it = -1; it < n_it && more(); ++it) {  // it = -1: only A of the first iteration
+    for (int it = -1; it < n_it; ++it, fill()) {  // it = -1: only A of the first iteration
       if (v == 0) FQLA_TRACE(2, 3);
       if (it + 1 < n_it) {
         const int j = it + 1, sj = j & 1;
@@ -762,8 +773,8 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
                          scale_bf16x2(a.z, g1.x, g1.y), scale_bf16x2(a.w, g1.z, g1.w));
         }
         fence_proxy_async();
-        mbar_arrive(&bars[AP_READY]);
-        mbar_arrive(&bars[EMPTYA0 + sj]);  // the A tile of this stage is no longer read here
+        ARRIVE(AP_READY);
+        ARRIVE(EMPTYA0 + sj);  // the A tile of this stage is no longer read here
       }
       if (v == 0) FQLA_TRACE(2, 4);
       if (!NO_O && it >= 0 && it >= lead) {
@@ -781,7 +792,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         tmem_ld_16x64(tmem + lanes_p + TM_P, x);
         tmem_ld_wait();
         tc_fence_before();
-        mbar_arrive(&bars[P_FREE]);
+        ARRIVE(P_FREE);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           if (i > 2 * wq + 1) continue;
@@ -797,7 +808,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           *reinterpret_cast<uint32_t*>(at + 1024) = pack_bf16(b0, b1);
         }
         fence_proxy_async();
-        mbar_arrive(&bars[P_READY]);
+        ARRIVE(P_READY);
         if (v == 96) FQLA_TRACE(2, 6);
       }
     }
@@ -814,24 +825,23 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     constexpr uint32_t ID_OT = idesc_bf16(128, 64, 0, 0);            // A from tensor memory
     constexpr uint32_t ID_S = idesc_bf16(128, 128, 0, 1);
     constexpr uint32_t STAGE_LO = STAGE_BYTES >> 4;
+    const bool idle = STATE ? warp != 0 : NO_O && warp == 1;
     if constexpr (STATE) {
       const uint32_t k0_lo = desc_lo_kmajor(smem + OFF_STAGE + TILE_QK);
       const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE_QK, 8192);
       const uint32_t a0_lo = desc_lo_kmajor(smem + OFF_STAGE + 2 * TILE_QK + TILE_V);
 #pragma unroll 1
-      for (int it = 0; it < n_it && warp == 0 && more(); ++it) {
+      for (int it = 0; it < n_it && warp == 0; ++it, fill()) {
         const int s = it & 1, ph = (it >> 1) & 1;
         const uint32_t so = s ? STAGE_LO : 0u;
-        WAIT(FULL0 + s, ph);
-        WAIT(S_COPY, it & 1);
+        if (!(WAITU(FULL0 + s, ph) && WAITU(S_COPY, it & 1))) break;
         tc_fence_after();
         if (elect_one()) {
           // U^T = S^T K^T   (A = packed S^T; B = K tile, K-major)
           umma_ts_group_kmajor_b<8>(tmem + TM_U, tmem + TM_SB, k0_lo + so, ID_OT);
           umma_commit(&bars[U_DONE]);
         }
-        WAIT(FULLA0 + s, ph);
-        WAIT(WB_READY, it & 1);
+        if (!(WAITU(FULLA0 + s, ph) && WAITU(WB_READY, it & 1))) break;
         tc_fence_after();
         if (elect_one()) {
           // Vn^T = W^T A^T   (A = packed W^T; B = A tile, K-major)
@@ -839,8 +849,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           umma_commit(&bars[VN_DONE]);
           umma_commit(&bars[EMPTYA0 + s]);
         }
-        WAIT(VB_READY, it & 1);
-        WAIT(S_DEC, it & 1);
+        if (!(WAITU(VB_READY, it & 1) && WAITU(S_DEC, it & 1))) break;
         tc_fence_after();
         if (elect_one()) {
           // S^T += (rho Vn)^T K
@@ -854,13 +863,11 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       const uint32_t wmn_lo = desc_lo_mnmajor(smem + OFF_W, 16384);
       const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE_QK, 8192);
 #pragma unroll 1
-      for (int it = 0; it < n_it && more(); ++it) {
+      for (int it = 0; it < n_it; ++it, fill()) {
         const int s = it & 1, c = it - lead;  // c < 0: lead-in chunk
         const uint32_t so = s ? STAGE_LO : 0u;
         if (lane == 0) FQLA_TRACE(3, 0);
-        WAIT(U_DONE, it & 1);
-        WAIT(W_READY, it & 1);
-        WAIT(S_COPY, it & 1);
+        if (!(WAITU(U_DONE, it & 1) && WAITU(W_READY, it & 1) && WAITU(S_COPY, it & 1))) break;
         tc_fence_after();
         if (lane == 0) FQLA_TRACE(3, 1);
         if (elect_one()) {
@@ -872,7 +879,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         if (lane == 0) FQLA_TRACE(3, 2);
         if constexpr (EXTRA) {
           if (tile_h && c >= 0) {  // the state entering this chunk, as an operand tile
-            WAIT(ST_READY, c & 1);
+            if (!WAITU(ST_READY, c & 1)) break;
             if (elect_one()) {
               const int y = (int)(((sp.chunk_base + c) * p.Hv + hv) * D);
               tma_store_2d(&map_h, 0, y, smem + OFF_ST);
@@ -882,8 +889,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           }
         }
         if (lane == 0) FQLA_TRACE(3, 3);
-        WAIT(VB_READY, it & 1);
-        WAIT(S_DEC, it & 1);
+        if (!(WAITU(VB_READY, it & 1) && WAITU(S_DEC, it & 1))) break;
         tc_fence_after();
         if (lane == 0) FQLA_TRACE(3, 4);
         if (elect_one()) {
@@ -896,7 +902,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         if (lane == 0) FQLA_TRACE(3, 5);
         if constexpr (EXTRA) {
           if (tile_vn && c >= 0) {
-            WAIT(VN_READY, c & 1);
+            if (!WAITU(VN_READY, c & 1)) break;
             if (elect_one()) {  // the v_new^T tile is complete
               tma_store_2d(&map_vn, 0, (int)(((sp.chunk_base + c) * p.Hv + hv) * D), smem + OFF_VNT);
               tma_store_commit();
@@ -918,14 +924,13 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       // and it waits only for VN_DONE, which that copy comes before (and which implies W_READY of the same chunk
       // and VB_READY of the one before).
 #pragma unroll 1
-      for (int it = 0; it < n_it && more(); ++it) {
+      for (int it = 0; it < n_it; ++it, fill()) {
         const int s = it & 1, c = it - lead;
         const uint32_t so = s ? STAGE_LO : 0u;
         if (lane == 0) FQLA_TRACE(4, 0);
         // P = Q K^T, over w^T; the prep group turns it into Pg
         if (c >= 0) {
-          WAIT(FULL0 + s, (it >> 1) & 1);
-          WAIT(W_READY, it & 1);
+          if (!(WAITU(FULL0 + s, (it >> 1) & 1) && WAITU(W_READY, it & 1))) break;
           tc_fence_after();
           if (lane == 0) FQLA_TRACE(4, 1);
           if (elect_one()) {
@@ -935,8 +940,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         }
         // O1^T = S^T Q^T   (A = packed S^T; B = q tile, K-major), behind Vn^T of the chain
         if (lane == 0) FQLA_TRACE(4, 2);
-        WAIT(VN_DONE, it & 1);
-        if (c > 0) WAIT(O_FREE, (c - 1) & 1);
+        if (!(WAITU(VN_DONE, it & 1) && (c <= 0 || WAITU(O_FREE, (c - 1) & 1)))) break;
         tc_fence_after();
         if (lane == 0) FQLA_TRACE(4, 3);
         if (elect_one()) {
@@ -947,8 +951,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         if (lane == 0) FQLA_TRACE(4, 4);
         // O2^T = Vn^T Pg^T   (A = packed Vn^T; B = Pg, K-major)
         if (c >= 0) {
-          WAIT(VB_READY, it & 1);
-          WAIT(P_READY, c & 1);
+          if (!(WAITU(VB_READY, it & 1) && WAITU(P_READY, c & 1))) break;
           tc_fence_after();
           if (lane == 0) FQLA_TRACE(4, 5);
           if (elect_one()) {
@@ -966,12 +969,11 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       const uint32_t vmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + 2 * TILE_QK, 8192);
       const uint32_t kmn0_lo = desc_lo_mnmajor(smem + OFF_STAGE + TILE_QK, 8192);
 #pragma unroll 1
-      for (int it = -1; it + 1 < n_it && more(); ++it) {
+      for (int it = -1; it + 1 < n_it; ++it, fill()) {
         const int s = (it + 1) & 1;
-        WAIT(FULL0 + s, ((it + 1) >> 1) & 1);
-        WAIT(AP_READY, (it + 1) & 1);
-        if (it >= 0) WAIT(VN_DONE, it & 1);
-        if (!NO_O && it >= 0 && it >= lead) WAIT(P_FREE, (it - lead) & 1);
+        if (!(WAITU(FULL0 + s, ((it + 1) >> 1) & 1) && WAITU(AP_READY, (it + 1) & 1))) break;
+        if (it >= 0 && !WAITU(VN_DONE, it & 1)) break;
+        if (!NO_O && it >= 0 && it >= lead && !WAITU(P_FREE, (it - lead) & 1)) break;
         tc_fence_after();
         if (lane == 0) FQLA_TRACE(5, 0);
         if (elect_one()) {
@@ -980,7 +982,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         }
         if (lane == 0) FQLA_TRACE(5, 1);
         // u^T over Vn^T, which has been read, behind the state update
-        if (it >= 0) WAIT(S_DONE, it & 1);
+        if (it >= 0 && !WAITU(S_DONE, it & 1)) break;
         tc_fence_after();
         if (lane == 0) FQLA_TRACE(5, 2);
         if (elect_one()) {
@@ -991,6 +993,9 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         if (lane == 0) FQLA_TRACE(5, 3);
       }
     }
+    // no product is under way when the block goes, whoever gave up what
+    if (!idle && elect_one()) umma_commit(&bars[SETTLED]);
+    if (warp == 0) settle(SETTLED, 0);
   } else {
     // =============================== producer ===============================
     // zero the rows past the sequence end in n 8 KB blocks of 64 rows (they belong to the next
@@ -1001,7 +1006,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         if (((i >> 3) & 63) >= valid) *reinterpret_cast<uint4*>(base + i * 16) = make_uint4(0, 0, 0, 0);
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) mbar_arrive(full);
+      if (lane == 0 && tries > 0) mbar_arrive(full);
     };
     // Iteration `it`: q, k, v of chunk it; vectors and A tile of chunk it + 1, a whole chunk before
     // its q, k, v (whose stage is still in use, but the prep warps can start on A early); the gates
@@ -1010,6 +1015,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     float g_r[2] = {0.f, 0.f}, b_r[2] = {0.f, 0.f}, gl_r = 0.f;
     // (A whole first chunk's q, k, v go out at once, ahead of its gates: it = -2.  The arrival on their barrier,
     // which stands for the vectors too, follows in its place.  100 tokens x 8 heads 13.1 -> 12.3 us.)
+    int loads = 0, a_loads = 0;  // q, k, v and A tiles that have been asked for
     const bool early = n_it > 0 && (lead > 0 || sp.len + lead * CHUNK >= CHUNK);
     auto load = [&](int it) {
       const int s = it & 1, c = it - lead;
@@ -1019,7 +1025,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       if (it >= 2) WAIT(EMPTY0 + s, ((it >> 1) - 1) & 1);
       unsigned char* st = smem + OFF_STAGE + s * STAGE_BYTES;
       uint64_t* bar = &bars[partial ? PRIV : FULL0 + s];
-      if (elect_one()) {
+      if (issuing()) {
         mbar_expect_tx(bar, STAGE_BYTES - TILE_A - (with_q ? 0 : TILE_QK) - (m_pass ? TILE_V : 0));
         if (it > 0 || !early) mbar_arrive(bar);
         tma_load_2d(st + TILE_QK, &map_k, hq * D, y, bar);
@@ -1033,15 +1039,16 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           tma_load_2d(st + 8192, &map_q, hq * D + 64, y, bar);
         }
       }
+      loads = tries > 0 ? it + 1 : loads;
       if (partial) {
         WAIT(PRIV, 0);
         zero_rows(st, 6, valid, &bars[FULL0 + s]);
       }
     };
 #pragma unroll 1
-    for (int it = -2; it < n_it && more(); ++it) {
+    for (int it = -2; it < n_it; ++it, fill()) {
       if (it > 0 || it == (early ? -2 : 0)) load(max(it, 0));
-      else if (it == 0 && lane == 0) mbar_arrive(&bars[FULL0]);
+      else if (it == 0 && lane == 0) ARRIVE(FULL0);
       const int j = it + 1;
       if (j >= 0 && j < n_it) {
         const int sj = j & 1, c = j - lead;
@@ -1063,10 +1070,11 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         __syncwarp();
         unsigned char* dst = smem + OFF_STAGE + sj * STAGE_BYTES + 2 * TILE_QK + TILE_V;
         uint64_t* bar = &bars[partial ? PRIVA : FULLA0 + sj];
-        if (elect_one()) {
+        if (issuing()) {
           mbar_arrive_expect_tx(bar, TILE_A);
           tma_load_2d(dst, &map_a, hv * CHUNK, (int)sp.bos + c * CHUNK, bar);
         }
+        a_loads = tries > 0 ? j + 1 : a_loads;
         if (partial) {
           // only the last chunk of a sequence can be partial: the private barrier is used once
           WAIT(PRIVA, 0);
@@ -1087,6 +1095,12 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
           if (r > last) b_r[z] = 0.f;
         }
       }
+    }
+    // nor a load
+#pragma unroll 1
+    for (int i = 1; i <= 2; ++i) {
+      if (loads >= i) settle(FULL0 + ((loads - i) & 1), ((loads - i) >> 1) & 1);
+      if (a_loads >= i) settle(FULLA0 + ((a_loads - i) & 1), ((a_loads - i) >> 1) & 1);
     }
   }
 

@@ -40,6 +40,13 @@ __device__ __forceinline__ void fence_mbar_init() {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s32(bar)) : "memory");
 }
+// ... of a thread that has given no wait up (see mbar_wait)
+__device__ __forceinline__ void mbar_arrive_if(uint64_t* bar, int tries) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(s32(bar)),
+      "r"(tries)
+      : "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {  // without an arrival
   asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(s32(bar)), "r"(bytes) : "memory");
 }
@@ -62,15 +69,16 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait.  `tries` is the thread's own count, WAIT_TRIES (about a second and more) at the start of each
-// pass of its loop; a wait that uses it up falls through, and so does every wait after it, until the loop looks
-// at the count and ends: one look a pass instead of a result at each of the dozens of wait sites, which were a
-// fifth of the kernels' code.  What a pass does after a wait was given up touches only the memory that it would
-// have touched anyway; its values are lost (the kernel sets its status word).  The thread is suspended by the
-// hardware meanwhile, but comes back early and often: trying again at once takes issue slots from the warps that
-// have work, hence the pause (chunk-parallel backward, 262144 tokens x 8 heads: 1510 us without it, 1260 with,
-// whether 20 or 400 ns; 1340 with a look at an abort flag in its place).  Polling with test_wait instead, or once
-// before it, costs more (forward recurrence 467 us, 484 with a test at the waits that are mostly over).
+// Bounded wait.  `tries` is the thread's own count, WAIT_TRIES at the start of each pass of its loop; a wait that
+// uses it up falls through, and every wait after it does so after one try: looks with a result at each of the dozens
+// of wait sites were a fifth of the kernels' code.  Such a thread issues, signals and stores nothing more, so that the
+// threads that wait for it run out too, and the block ends after two limits or so, with its values lost and the status
+// word set.  The lanes of a warp count each for themselves: only a vote may take a warp out of a loop.
+// The thread is suspended by the hardware meanwhile, but comes back early and often: trying again at once takes
+// issue slots from the warps that have work, hence the pause (chunk-parallel backward, 262144 tokens x 8 heads:
+// 1510 us without it, 1260 with, whether 20 or 400 ns; 1340 with a look at an abort flag in its place).  Polling with
+// test_wait instead, or once before it, costs more (forward recurrence 467 us, 484 with a test at the waits that are
+// mostly over).
 constexpr int WAIT_TRIES = 1 << 24;
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int& tries) {
   asm volatile(
@@ -86,10 +94,15 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int& t
 }
 
 // The same for a warp that issues products: it stays converged in the compiler's eyes, which keeps what is
-// computed between its waits in uniform registers.
-__device__ __forceinline__ void mbar_wait_uniform(uint64_t* bar, uint32_t parity, int& tries) {
+// computed between its waits in uniform registers, and may leave its loop right where a wait has been given up
+// (false), which costs nothing where it has not.
+__device__ __forceinline__ bool mbar_wait_uniform(uint64_t* bar, uint32_t parity, int& tries) {
 #pragma unroll 1
-  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity)) && --tries > 0) __nanosleep(20);
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if (--tries <= 0) return false;
+    __nanosleep(20);
+  }
+  return true;
 }
 
 // Named barrier ID of N threads that tells all of them alike whether `ok` holds for each: a group that meets at

@@ -16,20 +16,28 @@ FORMS = [("forward", dict(n_it=2)), ("forward", dict(n_it=2, lead=1, extra=True,
 
 @pytest.fixture(scope="module", params=FORMS, ids=lambda f: "-".join([f[0], *f[1]]))
 def plays(request):
-    """(warps left at a named barrier, what a warp signalled or issued behind its own wait) of every play"""
+    """the kernel, and of every play (warps left at a named barrier, what a warp signalled or issued behind its
+    own wait)"""
     name, form = request.param
     kernel = getattr(wait_model, name)(**form)
     warps = (0, 7, 8, 15, 16) if name == "items" else [w for w in range(kernel.warps) if w < 4 or w % 4 in (0, 3)]
-    return [wait_model.given_up(kernel, w, nth, bool(nth & 1)) for w in warps
-            for nth in range(wait_model.waits_of(kernel, w))]
+    return kernel, [wait_model.given_up(kernel, w, nth, bool(nth & 1)) for w in warps
+                    for nth in range(wait_model.waits_of(kernel, w))]
 
 
 def test_every_warp_comes_to_the_end(plays):
-    assert [left for left, _ in plays if left] == []
+    assert [left for left, _ in plays[1] if left] == []
 
 
 def test_no_gradient_of_an_incomplete_item_is_stored(plays):
-    assert {(w, e) for _, late in plays for w, e in late if e[1] in ("dv", "store_rows")} == set()
+    assert {(w, e) for _, late in plays[1] for w, e in late if e[1] in ("dv", "store_rows")} == set()
+
+
+def test_nothing_is_issued_or_signalled_behind_a_wait_that_ran_out(plays):
+    """...by the warp that waited: copies, products and arrivals may outlive the block or pass for the ones of
+    complete work (SETTLED is the end of what it had issued before)"""
+    kernel, results = plays
+    assert {(w, e) for _, late in results for w, e in late if e[1] != kernel.names["SETTLED"]} == set()
 
 
 @pytest.mark.parametrize("file", ["fwd_tc.cu", "bwd_dh_tc.cu", "prep_kernels.cu"])
@@ -38,7 +46,8 @@ def test_a_warp_goes_on_or_leaves_as_one(file):
     count decides for the warp (a vote), for a group (a barrier's) or for what one lane does alone."""
     text = re.sub(r"//[^\n]*", "", open(os.path.join(wait_model.CSRC, file)).read())
     alone = (r"__all_sync\(0xffffffffu, tries > 0\)", r"bar_all<\d+, \d+>\(tries > 0\)", r"elect_one\(\) && tries > 0",
-             r"if \(tries <= 0\) \*abort_flag = 1;", r"if \(tries <= 0\) atomicCAS\(", r"if \(tries > 0\) mbar_arrive\(")
+             r"if \(tries <= 0\) \*abort_flag = 1;", r"if \(tries <= 0\) atomicCAS\(", r"if \(tries > 0\) mbar_arrive\(",
+             r"lane == 0 && tries > 0\) mbar_arrive\(", r"tries > 0 \?")
     looks = re.findall(r"[^\n]*\btries (?:>|<=) 0[^\n]*", text)
     assert looks
     assert [line.strip() for line in looks if not any(re.search(a, line) for a in alone)] == []

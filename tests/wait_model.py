@@ -15,7 +15,7 @@ import re
 from types import SimpleNamespace
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "flashqla_b200", "csrc")
-EVENT = re.compile(r"\b(mbar_wait(?:_uniform)?|mbar_arrive(?:_expect_tx)?|umma_\w+|tma_(?:load|store)_2d|clc_try_cancel|"
+EVENT = re.compile(r"\b(mbar_wait(?:_uniform)?|mbar_arrive(?:_expect_tx|_if)?|umma_\w+|tma_(?:load|store)_2d|clc_try_cancel|"
                    r"bar_all|store_rows)\b|bar\.(?:sync|arrive)|uint4\*>\(p\.dv")
 BARRIER = re.compile(r"&bars\[(.*?)\]|^(\w+)$")
 
@@ -165,6 +165,18 @@ class Kernel:
 
     def _value(self, expr, env, lambdas):
         """(a generator: an expression may hold a vote or call a lambda)"""
+        if any(lambdas[n][2] for n in re.findall(r"\b(\w+)\(", expr) if n in lambdas):  # what waits, waits in order
+            expr = expr.strip()
+            for sign, ends in (("||", True), ("&&", False)):
+                parts = _split(expr.replace(sign, "\0"), "\0")
+                for part in parts if len(parts) > 1 else ():
+                    value = yield from self._value(part, env, lambdas)
+                    if bool(value) == ends or part is parts[-1]:
+                        return value
+            if expr[0] == "!":
+                return not (yield from self._value(expr[1:], env, lambdas))
+            if expr[0] == "(" and _close(expr, 0) == len(expr):
+                return (yield from self._value(expr[1:-1], env, lambdas))
         if m := re.search(r"bar_all<(\d+), (\d+)>\(", expr):
             end = _close(expr, m.end() - 1)
             mine = yield from self._value(expr[m.end():end - 1], env, lambdas)
@@ -232,8 +244,8 @@ class Kernel:
                         break
                     if out and out[0] != "continue":
                         return out
-                    if step:
-                        self._assign(step, env)
+                    for part in _split(step):
+                        self._assign(part, env)
             elif kind == "switch":
                 want = str((yield from self._value(node[1], env, lambdas)))
                 body = node[2][1]
@@ -267,6 +279,9 @@ class Kernel:
     def _do(self, text, env, lambdas, one):
         if text in ("break", "continue"):
             return (text,)
+        if m := re.match(r"return (mbar_wait\w*\(.*\))$", text):
+            yield from self._do(m[1], env, lambdas, one)
+            return "return", env["tries"] > 0
         if m := re.match(r"return\b(.*)", text, flags=re.S):
             return "return", (yield from self._value(m[1], env, lambdas)) if m[1].strip() else None
         if m := re.match(r"auto (\w+) = \[&\]\s*(?:\((.*?)\))?\s*(?=\{)", text, flags=re.S):
@@ -286,8 +301,12 @@ class Kernel:
                 bar = _eval(BARRIER.match(args[0])[1], env)
                 ok = yield "wait", bar, _eval(args[1], env) & 1
                 if not ok:
-                    env["tries"] = 0
+                    env[args[2]] = 0
                 return None
+            if name == "mbar_arrive_if":
+                name = "mbar_arrive"
+                if not env["tries"] > 0:
+                    return None
             if name in ("mbar_arrive", "mbar_arrive_expect_tx", "umma_commit"):
                 b = BARRIER.match(args[0])
                 bar = _eval(b[1] or b[2], env)
