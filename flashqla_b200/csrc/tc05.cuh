@@ -55,8 +55,8 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                "r"(bytes)
                : "memory");
 }
-// One try: the thread may be suspended by the hardware until the phase completes or a (short,
-// about 0.2 us on B200) system limit runs out; no instructions are issued meanwhile.
+// One try: the thread may be suspended by the hardware until the phase completes or a system limit runs out (4 us
+// in a block where nothing else happens, sooner in a busy one); no instructions are issued meanwhile.
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -74,12 +74,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // of wait sites were a fifth of the kernels' code.  Such a thread issues, signals and stores nothing more, so that the
 // threads that wait for it run out too, and the block ends after two limits or so, with its values lost and the status
 // word set.  The lanes of a warp count each for themselves: only a vote may take a warp out of a loop.
+// The limit: a try of a block that stands still takes 4.07 us with its pause (100 of them 408 us), so 2^18 a second.
+// (It was 2^24, more than a minute.)
 // The thread is suspended by the hardware meanwhile, but comes back early and often: trying again at once takes
 // issue slots from the warps that have work, hence the pause (chunk-parallel backward, 262144 tokens x 8 heads:
 // 1510 us without it, 1260 with, whether 20 or 400 ns; 1340 with a look at an abort flag in its place).  Polling with
 // test_wait instead, or once before it, costs more (forward recurrence 467 us, 484 with a test at the waits that are
 // mostly over).
-constexpr int WAIT_TRIES = 1 << 24;
+constexpr int WAIT_TRIES = 1 << 18;
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, int& tries) {
   asm volatile(
       "{\n\t.reg .pred p;\n"

@@ -1,6 +1,6 @@
 """What a block does when one of its bounded waits runs out, from the kernels' source (see wait_model.py): each
 wait of the first and the last warp of every role in turn; of the waits that are then left open, the ones of the first
-or of the last warps run out first.  Nothing is run on a device."""
+or of the last warps run out first.  Nothing of that is run on a device; the last test times a wait that runs out there."""
 
 import os
 import re
@@ -51,3 +51,26 @@ def test_a_warp_goes_on_or_leaves_as_one(file):
     looks = re.findall(r"[^\n]*\btries (?:>|<=) 0[^\n]*", text)
     assert looks
     assert [line.strip() for line in looks if not any(re.search(a, line) for a in alone)] == []
+
+
+@pytest.mark.gpu
+def test_a_wait_is_given_up_after_about_a_second():
+    """WAIT_TRIES times what a try takes where nobody arrives"""
+    import ctypes
+
+    import torch
+
+    from flashqla_b200 import _lib
+
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    tries = 1 << int(re.search(r"WAIT_TRIES = 1 << (\d+);", open(os.path.join(wait_model.CSRC, "tc05.cuh")).read())[1])
+    took = []
+    for n in (1, 50, 100):  # (the first launch loads the kernel)
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        assert lib.fqla_selftest_wait_timeout(n, stream) == 0
+        end.record()
+        torch.cuda.synchronize()
+        took.append(begin.elapsed_time(end))
+    assert lib.fqla_device_status(ctypes.byref(ctypes.c_int()), 1) == 0
+    assert 0.2 < (took[2] - took[1]) / 50 / 1000 * tries < 5
