@@ -20,7 +20,7 @@
 // and q and took longer over q than the chain over a chunk: 262144 tokens x 8 heads 674 -> 587 us, 32768 packed
 // x 32 heads 384 -> 360, 4096 x 8 heads 22.6 -> 21.7; with A scaled by the state group 618, 362 and 21.9.  With
 // waits that pause between two tries and row-major outputs made in rolled loops (69 -> 56 KB of code) 604 -> 584 and
-// 361 -> 353.)
+// 361 -> 353; with issuing warps that leave their loop where a wait is given up, 353 -> 348 to 351.)
 #include <cuda.h>
 
 #include <climits>

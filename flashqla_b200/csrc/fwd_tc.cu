@@ -34,19 +34,22 @@
 //                            w^T -> bf16 operand tile (shared memory)
 //     warps 12-15, O group : output epilogue o = s gamma O1 + O2
 //     warps 16-19, prep group : A', A'' of the next chunk, P -> Pg   (warps 12-15 where nothing is output)
-//     warp 0 issues the two products of the chain, warp 1 those of the output, warp 3 u^T and w^T
+//     warp 0 issues the two products of the chain, warp 1 those of the output (none where nothing is output),
+//     warp 3 u^T and w^T
 //     warp 2, producer: per-chunk gate vectors (fetched one chunk ahead), TMA loads of the q, k, v, A tiles
 //                       (2 stages), zero-fill of rows past the end of a partial chunk
 //
 // What bounds it: the chain of a chunk (3230 cycles on an idle chip: state copy 530, Vn^T 770, its read-out 780,
-// state update 700, and the arrivals between them) and, with all SMs at work, HBM: 262144 tokens x 8 heads 455 us,
+// state update 700, and the arrivals between them) and, with all SMs at work, HBM: 262144 tokens x 8 heads 454 us,
 // 5.3 TB/s.  Two things had made it 4830 and 516 us (4 x 8192 x 16 heads 151 -> 131 us, 32768 packed x 32 heads with
 // tiles 392 -> 353).  (1) Roles that waited for one another in a ring: one thread that issued everything off the
 // chain, and an output group that built Pg between two epilogues.  No role waits here for another one's work off the
 // chain, and w^T and P, which share their columns, are read out of them at once.  (2) Code: the instruction cache of
 // an SM holds some 28 KB (straight code of one warp per scheduler, measured: full speed up to there, 2.5 cycles an
 // instruction beyond, 10 with all SMs at it), and a chunk runs every role's loop once.  So loops are rolled to
-// rounds of one tensor-memory load, and a wait is six instructions (tc05.cuh): 57 -> 47 KB, with tiles 72 -> 52.
+// rounds of one tensor-memory load, and a wait is six instructions (tc05.cuh): 57 -> 49 KB, with tiles 72 -> 54.  (The
+// issuing warps wait as one instead, which lets them leave where a wait is given up: 55 and 61 KB, and no slower,
+// as this code is not on the way of the others: 262144 tokens x 8 heads 457 -> 454, 64 prompts of 135161 tokens 266 -> 264.5.)
 //
 // The state-only pass of the exact hand-off (end states and transition matrices of segments) is a
 // chain of its own, because its roundings go into every segment behind the hand-off: A diag(beta),
@@ -269,7 +272,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     mbar_init(&bars[U_DONE], 1);
     mbar_init(&bars[FULLA0], 1);
     mbar_init(&bars[FULLA1], 1);
-    // the only reader of the raw A tile: the state group, or (STATE) a product
+    // the only reader of the raw A tile: the prep group, or (STATE) a product
     mbar_init(&bars[EMPTYA0], STATE ? 1 : 128);
     mbar_init(&bars[EMPTYA1], STATE ? 1 : 128);
     mbar_init(&bars[PRIVA], 1);
@@ -295,7 +298,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
     tma_prefetch_desc(&map_v);
     tma_prefetch_desc(&map_a);
   }
-  // Pg is lower triangular: its tile is zeroed once, the O group only ever rewrites the column
+  // Pg is lower triangular: its tile is zeroed once, the prep group only ever rewrites the column
   // groups that can be non-zero for its rows
   for (int i = tid; i < 8192 / 16; i += NT)
     *reinterpret_cast<uint4*>(smem + OFF_P + i * 16) = make_uint4(0, 0, 0, 0);
@@ -406,9 +409,9 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       if (!NO_O && it > 0) WAIT(SB_FREE, (it - 1) & 1);
       tc_fence_after();
       if (v == 0) FQLA_TRACE(0, 1);
-      // on the chain: the bf16 operand copy of S^T, packed back into tensor memory.  (The products
-      // that read the copy of the chunk before were issued ahead of the state update whose
-      // completion was just waited for, and the tensor pipe runs in issue order.)
+      // on the chain: the bf16 operand copy of S^T, packed back into tensor memory.  (Of the products that read
+      // the copy of the chunk before, Vn^T came ahead of the state update, issued by the same thread; O1^T has
+      // signalled SB_FREE.)
 #pragma unroll 1
       for (int k0 = 0; k0 < D; k0 += 32) {
         float x[32];
@@ -711,7 +714,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
       }
     };
 #pragma unroll 1
-    for (int c = max(-lead, 0); c < n_it - lead; ++c, fill()) {
+    for (int c = 0; c < n_it - lead; ++c, fill()) {
       if (v == 0) { const int it = c + lead; FQLA_TRACE(2, 0); }
       WAIT(O_DONE, c & 1);
       if (wq == 0 && elect_one()) tma_store_wait_read();  // the store of the chunk before has read the tile
@@ -867,6 +870,7 @@ fwd_tc_kernel(const FwdTcParams p, const __grid_constant__ CUtensorMap map_q,
         const int s = it & 1, c = it - lead;  // c < 0: lead-in chunk
         const uint32_t so = s ? STAGE_LO : 0u;
         if (lane == 0) FQLA_TRACE(3, 0);
+        if (lane == 0 && it < 126) FQLA_CHUNK_CLOCK(it);
         if (!(WAITU(U_DONE, it & 1) && WAITU(W_READY, it & 1) && WAITU(S_COPY, it & 1))) break;
         tc_fence_after();
         if (lane == 0) FQLA_TRACE(3, 1);

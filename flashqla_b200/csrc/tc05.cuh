@@ -347,26 +347,6 @@ __device__ __forceinline__ void tmem_st_wait() {
 }
 
 // ---- descriptors -----------------------------------------------------------------------------
-// Shared-memory matrix descriptor for an SW128 tile (see the convention at the top).
-//   bits [0,14) start address >> 4, [16,30) leading byte offset >> 4, [32,46) stride byte offset
-//   >> 4, [46,48) version = 1, [61,64) layout type = 2 (128-byte swizzle).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes,
-                                              uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-__device__ __forceinline__ uint64_t desc_kmajor(const void* tile) {
-  return smem_desc(s32(tile), 16, 1024);
-}
-__device__ __forceinline__ uint64_t desc_mnmajor(const void* tile, uint32_t block_stride_bytes) {
-  return smem_desc(s32(tile), block_stride_bytes, 1024);
-}
-
 // Instruction descriptor for kind::f16 with bf16 inputs and fp32 accumulation.
 //   bits [4,6) D format (1 = f32), [7,10) A format (1 = bf16), [10,13) B format, 15 A major
 //   (0 = K, 1 = MN), 16 B major, [17,23) N >> 3, [24,29) M >> 4.
@@ -375,22 +355,13 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, int a_mn_major, 
          ((uint32_t)b_mn_major << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by one thread.
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                     uint32_t idesc, bool accumulate) {
-  uint32_t acc = accumulate ? 1u : 0u;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-// Lean issue form.  Every descriptor of an SW128 tile has the same high word (SBO = 1024,
-// version 1, 128-byte swizzle); the low word is (address >> 4) | (LBO >> 4) << 16, so a K step
-// is one 32-bit add on a per-tile base kept in a register.  Few, mutually independent
-// instructions per MMA matter: the issuing thread shares its scheduler with three busy warps
-// and pays a scheduling delay for every dependent instruction.
+// Shared-memory matrix descriptor for an SW128 tile (see the convention at the top):
+//   bits [0,14) start address >> 4, [16,30) leading byte offset >> 4, [32,46) stride byte offset
+//   >> 4, [46,48) version = 1, [61,64) layout type = 2 (128-byte swizzle).
+// All of them have the same high word (SBO = 1024, version 1, 128-byte swizzle); the low word is
+// (address >> 4) | (LBO >> 4) << 16, so a K step is one 32-bit add on a per-tile base kept in a register.
+// Few, mutually independent instructions per MMA matter: the issuing thread shares its scheduler with three busy
+// warps and pays a scheduling delay for every dependent instruction.
 constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo_kmajor(const void* tile) {
   return ((s32(tile) >> 4) & 0x3FFF) | (1u << 16);
@@ -398,6 +369,7 @@ __device__ __forceinline__ uint32_t desc_lo_kmajor(const void* tile) {
 __device__ __forceinline__ uint32_t desc_lo_mnmajor(const void* tile, uint32_t block_stride_bytes) {
   return ((s32(tile) >> 4) & 0x3FFF) | ((block_stride_bytes >> 4) << 16);
 }
+// D[tmem] (+)= A[smem] * B[smem]; issued by one thread.
 template <bool ACCUMULATE>
 __device__ __forceinline__ void umma_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,
                                         uint32_t idesc) {

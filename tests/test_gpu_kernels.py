@@ -265,7 +265,7 @@ def test_bounded_wait_runs_out_and_reports_through_the_status_word():
     status = ctypes.c_int(-1)
     assert lib.fqla_device_status(ctypes.byref(status), 0) == 0 and status.value == 0
     assert lib.fqla_selftest_wait_timeout(3, torch.cuda.current_stream().cuda_stream) == 0
-    torch.cuda.synchronize()  # the kernel comes back by itself after about 3 ms
+    torch.cuda.synchronize()  # the kernel comes back by itself after some 12 us
     assert lib.fqla_device_status(ctypes.byref(status), 1) == 0 and status.value == 1
     assert lib.fqla_device_status(ctypes.byref(status), 0) == 0 and status.value == 0
     after = run()
