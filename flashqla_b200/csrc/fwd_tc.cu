@@ -48,8 +48,9 @@
 // an SM holds some 28 KB (straight code of one warp per scheduler, measured: full speed up to there, 2.5 cycles an
 // instruction beyond, 10 with all SMs at it), and a chunk runs every role's loop once.  So loops are rolled to
 // rounds of one tensor-memory load, and a wait is six instructions (tc05.cuh): 57 -> 49 KB, with tiles 72 -> 54.  (The
-// issuing warps wait as one instead, which lets them leave where a wait is given up: 55 and 61 KB, and no slower,
-// as this code is not on the way of the others: 262144 tokens x 8 heads 457 -> 454, 64 prompts of 135161 tokens 266 -> 264.5.)
+// issuing warps wait as one instead, which lets them leave where a wait is given up: 55 and 61 KB, and no slower, as
+// this code is not on the way of the others: 262144 tokens x 8 heads 457 -> 454 us, 64 prompts of 135161 tokens
+// 266 -> 264.5.)
 //
 // The state-only pass of the exact hand-off (end states and transition matrices of segments) is a
 // chain of its own, because its roundings go into every segment behind the hand-off: A diag(beta),

@@ -1,6 +1,7 @@
 """What a block does when one of its bounded waits runs out, from the kernels' source (see wait_model.py): each
-wait of the first and the last warp of every role in turn; of the waits that are then left open, the ones of the first
-or of the last warps run out first.  Nothing of that is run on a device; the last test times a wait that runs out there."""
+wait of the first and the last warp of every role in turn; of the waits that are then left open, the ones of the
+first or of the last warps run out first.  Nothing of that is run on a device; the last test times a wait that runs
+out there."""
 
 import os
 import re

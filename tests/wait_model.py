@@ -15,8 +15,8 @@ import re
 from types import SimpleNamespace
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "flashqla_b200", "csrc")
-EVENT = re.compile(r"\b(mbar_wait(?:_uniform)?|mbar_arrive(?:_expect_tx|_if)?|umma_\w+|tma_(?:load|store)_2d|clc_try_cancel|"
-                   r"bar_all|store_rows)\b|bar\.(?:sync|arrive)|uint4\*>\(p\.dv")
+EVENT = re.compile(r"\b(mbar_wait(?:_uniform)?|mbar_arrive(?:_expect_tx|_if)?|umma_\w+|tma_(?:load|store)_2d|"
+                   r"clc_try_cancel|bar_all|store_rows)\b|bar\.(?:sync|arrive)|uint4\*>\(p\.dv")
 BARRIER = re.compile(r"&bars\[(.*?)\]|^(\w+)$")
 
 
@@ -529,8 +529,8 @@ def reverse(lead=0, n_it=7, partial=False, tiled=1, text=None):
 
 def items(clc=False, tiled=True, partial=(), n_items=4, text=None):
     """The chunk-parallel backward: one block that takes n_items items."""
-    config = dict(TILED=tiled, CLC=clc, N_EPI=512, D=128, CHUNK=64, p=SimpleNamespace(Hv=1000, next_item=0, dg_cumsum=0),
-                  total=n_items, raw=None, answers=0, blockIdx=SimpleNamespace(x=0), gridDim=SimpleNamespace(x=1))
+    config = dict(TILED=tiled, CLC=clc, N_EPI=512, D=128, CHUNK=64,
+                  p=SimpleNamespace(Hv=1000, next_item=0, dg_cumsum=0), total=n_items, raw=None, answers=0, blockIdx=SimpleNamespace(x=0), gridDim=SimpleNamespace(x=1))
 
     def shared():
         claims = itertools.count()
@@ -550,4 +550,5 @@ CASES = [*itertools.chain(
     (("forward", dict(no_o=True, extra=extra, partial=partial)) for extra, partial in
      itertools.product((False, True), (False, True))),
     (("reverse", dict(lead=lead, partial=partial)) for lead, partial in itertools.product((0, 1, 2, 3), (False, True))),
-    (("items", dict(clc=clc, partial=partial)) for clc, partial in itertools.product((False, True), ((), (0, 2), (1, 3)))))]
+    (("items", dict(clc=clc, partial=partial)) for clc, partial in
+     itertools.product((False, True), ((), (0, 2), (1, 3)))))]
